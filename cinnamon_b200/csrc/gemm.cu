@@ -15,7 +15,7 @@
 // Every wait is bounded: when one runs out the kernel records a code in a device status
 // word, every role leaves its loop, TMEM is freed and the kernel returns.
 #include "common.cuh"
-#include "tma.cuh"
+#include "tcgen05.cuh"
 #include <cuda.h>
 #include <mutex>
 #include <atomic>
@@ -54,23 +54,8 @@ struct GemmParams {
 // ---------------------------------------------------------------------------
 // bounded waits
 // ---------------------------------------------------------------------------
-constexpr long long WAIT_LIMIT_CYCLES = 4000000000LL;   // about two seconds
-
-// Bounded wait.  Returns false when the kernel is being abandoned.
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag, int code) {
-    if (mbar_try_wait(bar, parity)) return true;
-    const long long t0 = clock64();
-    for (uint32_t spin = 1;; ++spin) {
-        if (mbar_try_wait(bar, parity)) return true;
-        if ((spin & 255u) == 0) {
-            if (*abort_flag) return false;
-            if (clock64() - t0 > WAIT_LIMIT_CYCLES) {
-                *abort_flag = 1;
-                atomicCAS(&g_device_status, 0, code);
-                return false;
-            }
-        }
-    }
+    return mbar_wait_bounded(bar, parity, abort_flag, code, &g_device_status);
 }
 
 // The same wait taken by a whole warp, with one verdict for all its lanes: the promotion warps execute
@@ -87,13 +72,6 @@ __device__ __forceinline__ float ld_scale(const float* p) {
     return v;
 }
 
-__device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
-
-__device__ __forceinline__ void tc_commit(uint32_t bar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
-}
-
 // D[tmem] (+)= A[smem desc] * B[smem desc], e4m3 x e4m3 -> fp32
 __device__ __forceinline__ void tc_mma_f8(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
     asm volatile(
@@ -101,31 +79,6 @@ __device__ __forceinline__ void tc_mma_f8(uint32_t d_tmem, uint64_t a_desc, uint
         "setp.ne.b32 p, %4, 0;\n\t"
         "tcgen05.mma.cta_group::1.kind::f8f6f4 [%0], %1, %2, %3, p;\n\t}"
         ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate) : "memory");
-}
-
-// 32 lanes x 16 consecutive fp32 columns: thread i receives TMEM lane (base lane + i)
-__device__ __forceinline__ void tc_ld16(uint32_t taddr, float (&v)[16]) {
-    uint32_t r[16];
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
-        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
-          "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-        : "r"(taddr));
-    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-    for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]);
-}
-
-// Shared-memory matrix descriptor, 128-byte swizzle, Blackwell descriptor version 1.
-// lbo / sbo in bytes.
-__device__ __forceinline__ uint64_t make_smem_desc(uint32_t addr, uint32_t lbo, uint32_t sbo) {
-    uint64_t d = 0;
-    d |= (uint64_t)((addr >> 4) & 0x3FFF);
-    d |= (uint64_t)((lbo >> 4) & 0x3FFF) << 16;
-    d |= (uint64_t)((sbo >> 4) & 0x3FFF) << 32;
-    d |= (uint64_t)1 << 46;     // descriptor version
-    d |= (uint64_t)2 << 61;     // SWIZZLE_128B
-    return d;
 }
 
 // Instruction descriptor for kind::f8f6f4: fp32 accumulate, e4m3 x e4m3, A K-major.
@@ -972,10 +925,11 @@ int grouped_gemm_16bit(const void* A, const void* W, int in_dtype, const int64_t
 
 int read_quant_status(int* out, int reset);
 int read_moe_status(int* out, int reset);
+int read_indexer_status(int* out, int reset);
 
-// One word for the caller: the GEMM's code if it has one, else the quantisers', else the exchange kernels'.
+// One word for the caller: the GEMM's code if it has one, else the quantisers', the exchange kernels', the indexer's.
 int read_device_status(int* out, int reset) {
-    int v = 0, q = 0, m = 0;
+    int v = 0, q = 0, m = 0, x = 0;
     CINN_CHECK_CUDA(cudaMemcpyFromSymbol(&v, g_device_status, sizeof(int)));
     if (reset && v != 0) {
         int z = 0;
@@ -985,7 +939,9 @@ int read_device_status(int* out, int reset) {
     if (rc) return rc;
     rc = read_moe_status(&m, reset);
     if (rc) return rc;
-    *out = v != 0 ? v : (q != 0 ? q : m);
+    rc = read_indexer_status(&x, reset);
+    if (rc) return rc;
+    *out = v != 0 ? v : (q != 0 ? q : (m != 0 ? m : x));
     return CINN_OK;
 }
 

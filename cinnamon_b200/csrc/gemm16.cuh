@@ -15,21 +15,6 @@ namespace g16 {
 
 constexpr int GTHREADS = (EPI_WARPS + 2) * 32;
 
-// kind::f16 instruction descriptor: fp32 accumulate, A and B of the same 16-bit type, both K-major
-__host__ __device__ constexpr uint32_t make_idesc16(bool bf16) {
-    return (1u << 4)                                   // D format: fp32
-           | ((bf16 ? 1u : 0u) << 7) | ((bf16 ? 1u : 0u) << 10)   // A, B format: 0 = fp16, 1 = bf16
-           | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(BM >> 4) << 24);
-}
-
-__device__ __forceinline__ void tc_mma_f16(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-        ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate) : "memory");
-}
-
 template <bool BF16_IN, int OUT>
 __global__ void __launch_bounds__(GTHREADS, 1)
 grouped_gemm16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
@@ -122,7 +107,7 @@ grouped_gemm16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
     } else if (warp == EPI_WARPS + 1) {
         // ------------------------------ MMA issuer ------------------------------
         if (lane == 0) {
-            constexpr uint32_t idesc = make_idesc16(BF16_IN);
+            constexpr uint32_t idesc = make_idesc_f16(BF16_IN, BM, BN);
             uint32_t it = 0, tile_no = 0;
             bool alive = true;
             for (int t = blockIdx.x; t < n_total && alive; t += gridDim.x, ++tile_no) {

@@ -60,3 +60,19 @@ def test_kernel_views_and_sizes(dtype):
     k = kfull[:, :, 64:]                                                     # pitched rows
     got = K.lightning_indexer_fused(q.cuda(), kfull.cuda()[:, :, 64:], w.cuda())
     _close_fp16(got.cpu(), SO.lightning_indexer(q, k, w))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("shape", [(1, 1, 1, 1, 1), (2, 127, 129, 3, 20), (1, 128, 128, 4, 64), (1, 130, 257, 5, 72), (1, 40, 131, 3, 128),
+                                   (1, 17, 70, 2, 136)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_tile_edges(shape, dtype):
+    """Partial query and key tiles, padded widths, more heads than fit at once, and a row too wide for the tensor cores."""
+    from cinnamon_b200 import kernels as K
+    B, Lq, Lk, H, d = shape
+    g = torch.Generator().manual_seed(sum(shape))
+    q, k = torch.randn(B, Lq, H, d, generator=g).to(dtype), torch.randn(B, Lk, d, generator=g).to(dtype)
+    w = torch.rand(B, Lq, H, generator=g).to(dtype)
+    got = K.lightning_indexer_fused(q.cuda(), k.cuda(), w.cuda())
+    _close_fp16(got.cpu(), SO.lightning_indexer(q, k, w))
+    assert K.device_status() == 0
