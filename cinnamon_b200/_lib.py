@@ -8,7 +8,7 @@ from __future__ import annotations
 import ctypes
 import os
 
-from .build import LIB_PATH as _DEFAULT_LIB_PATH
+from .build import HOST_PATH, LIB_PATH as _DEFAULT_LIB_PATH
 
 OK, ERR_INVALID, ERR_CUDA, ERR_UNSUPPORTED, ERR_DEVICE = 0, 1, 2, 3, 4
 BF16, F32, F16, F32_BF16 = 0, 1, 2, 3
@@ -111,3 +111,19 @@ def check(status: int, what: str) -> None:
     if status == ERR_INVALID:
         raise AssertionError(msg)
     raise LibraryError(msg)
+
+
+def _load_host():
+    """The native host path (csrc/host), bound to the functions of the library loaded above."""
+    import importlib.util
+    import torch  # noqa: F401  (its libraries must be loaded before the extension that links to them)
+    if not os.path.exists(HOST_PATH):
+        raise LibraryError(f"{HOST_PATH} is missing: build it with `python -m cinnamon_b200.build`")
+    spec = importlib.util.spec_from_file_location("_host", HOST_PATH)
+    module = importlib.util.module_from_spec(spec)
+    spec.loader.exec_module(module)
+    module.bind({name: ctypes.cast(getattr(lib, name), ctypes.c_void_p).value for name in module.symbols()}, LibraryError)
+    return module
+
+
+host = _load_host()

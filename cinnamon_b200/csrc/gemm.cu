@@ -575,6 +575,19 @@ static size_t smem_bytes(int E) {
     return n;
 }
 
+// Lets a kernel use up to `bytes` of dynamic shared memory, once per device.  The limit belongs to the function, not to a
+// launch or a thread: it is set to the most any launch can ask for, so that no thread lowers it under another one.
+template <auto KERN>
+static int allow_smem_once(size_t bytes) {
+    static std::atomic<uint64_t> done{0};
+    int dev = 0;
+    CINN_CHECK_CUDA(cudaGetDevice(&dev));
+    if (dev >= 0 && dev < 64 && (done.load(std::memory_order_acquire) >> dev & 1)) return CINN_OK;
+    CINN_CHECK_CUDA(cudaFuncSetAttribute(KERN, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+    if (dev >= 0 && dev < 64) done.fetch_or(1ULL << dev, std::memory_order_release);
+    return CINN_OK;
+}
+
 // Output map for the TMA-store epilogue: (rows, N) of a 2-byte type, boxes of 64 columns x 128 rows, 128-byte swizzle.
 // Sets p.tma_out; when the output cannot go through TMA the (unused) operand map is passed in its place.
 static int make_out_map(CUtensorMap* tc, const CUtensorMap& fallback, GemmParams& p, int out_dtype, int64_t rows,
@@ -601,15 +614,10 @@ static int make_out_map(CUtensorMap* tc, const CUtensorMap& fallback, GemmParams
 template <bool B_MN, bool GROUPED, int OUT, bool SCATTER = false>
 static int launch(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& tc, const GemmParams& p, int grid,
                   cudaStream_t st) {
-    auto kern = fp8_gemm_kernel<B_MN, GROUPED, OUT, SCATTER>;
+    constexpr auto kern = fp8_gemm_kernel<B_MN, GROUPED, OUT, SCATTER>;
     const size_t smem = smem_bytes(GROUPED ? p.E : 0);
-    static thread_local size_t configured[64] = {};   // per instantiation, per thread, per device
-    int dev = 0;
-    CINN_CHECK_CUDA(cudaGetDevice(&dev));
-    if (dev < 0 || dev >= 64 || configured[dev] < smem) {
-        CINN_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        if (dev >= 0 && dev < 64) configured[dev] = smem;
-    }
+    int rc = allow_smem_once<kern>(smem_bytes(GROUPED ? MAX_EXPERTS : 0));
+    if (rc) return rc;
     kern<<<grid, THREADS, smem, st>>>(ta, tb, tc, p);
     CINN_CHECK_LAUNCH();
     return CINN_OK;
@@ -633,15 +641,10 @@ static int launch_out(const CUtensorMap& ta, const CUtensorMap& tb, GemmParams& 
 template <bool B_MN, int OUT>
 static int launch_pair(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& tc, const GemmParams& p, int clusters,
                        cudaStream_t st) {
-    auto kern = pair::fp8_gemm_pair_kernel<B_MN, OUT>;
+    constexpr auto kern = pair::fp8_gemm_pair_kernel<B_MN, OUT>;
     const size_t smem = pair::PSMEM_BYTES;
-    static thread_local bool configured[64] = {};
-    int dev = 0;
-    CINN_CHECK_CUDA(cudaGetDevice(&dev));
-    if (dev < 0 || dev >= 64 || !configured[dev]) {
-        CINN_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        if (dev >= 0 && dev < 64) configured[dev] = true;
-    }
+    int rc = allow_smem_once<kern>(smem);
+    if (rc) return rc;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(2 * clusters, 1, 1);
     cfg.blockDim = dim3(pair::PTHREADS, 1, 1);
@@ -803,15 +806,10 @@ int fp8_grouped_gemm_dgrad(const void* dY, const float* sdY, const void* W, cons
 template <int OUT>
 static int launch_pair_gk(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& tc, const GemmParams& p, int clusters,
                           cudaStream_t st) {
-    auto kern = pair::fp8_gemm_pair_kernel<false, OUT, true>;
+    constexpr auto kern = pair::fp8_gemm_pair_kernel<false, OUT, true>;
     const size_t smem = pair::PSMEM_BYTES;
-    static thread_local bool configured[64] = {};
-    int dev = 0;
-    CINN_CHECK_CUDA(cudaGetDevice(&dev));
-    if (dev < 0 || dev >= 64 || !configured[dev]) {
-        CINN_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        if (dev >= 0 && dev < 64) configured[dev] = true;
-    }
+    int rc = allow_smem_once<kern>(smem);
+    if (rc) return rc;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(2 * clusters, 1, 1);
     cfg.blockDim = dim3(pair::PTHREADS, 1, 1);
@@ -865,15 +863,10 @@ int fp8_gemm_grouped_k(const void* A, const float* sA, const void* B, const floa
 template <bool BF16_IN, int OUT>
 static int launch16(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& tc, const GemmParams& p, int grid,
                     cudaStream_t st) {
-    auto kern = g16::grouped_gemm16_kernel<BF16_IN, OUT>;
+    constexpr auto kern = g16::grouped_gemm16_kernel<BF16_IN, OUT>;
     const size_t smem = smem_bytes(p.E);
-    static thread_local size_t configured[64] = {};
-    int dev = 0;
-    CINN_CHECK_CUDA(cudaGetDevice(&dev));
-    if (dev < 0 || dev >= 64 || configured[dev] < smem) {
-        CINN_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        if (dev >= 0 && dev < 64) configured[dev] = smem;
-    }
+    int rc = allow_smem_once<kern>(smem_bytes(MAX_EXPERTS));
+    if (rc) return rc;
     kern<<<grid, g16::GTHREADS, smem, st>>>(ta, tb, tc, p);
     CINN_CHECK_LAUNCH();
     return CINN_OK;

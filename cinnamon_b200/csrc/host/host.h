@@ -1,0 +1,70 @@
+// Native host path: what kernels.py does between two Python calls - output allocation, argument checks, the sequence of
+// library calls - in C++.  A small FP8 layer is a handful of launches of a few microseconds each; done from Python, the
+// ctypes calls, device contexts and torch.empty calls around them cost four times the kernels (77 us against 15 us of
+// GPU time for 128 tokens through a 512 -> 1024 layer).
+//
+// The kernels stay behind the plain C ABI: this extension holds function pointers into the one loaded copy of
+// libcinnamon_b200.so, handed over by Python when it binds the library.
+#pragma once
+#include <torch/extension.h>
+#include <torch/csrc/Exceptions.h>
+#include <ATen/cuda/CUDAContext.h>
+#include <ATen/cuda/EmptyTensor.h>
+#include <c10/cuda/CUDAGuard.h>
+#include <atomic>
+#include <exception>
+#include <string>
+#include "../../../include/cinnamon_b200.h"
+
+namespace cinnhost {
+
+using at::Tensor;
+
+#define CINN_HOST_API(X)                                                                                            \
+    X(cinn_last_error) X(cinn_quant_rowwise) X(cinn_quant_rowwise_dual) X(cinn_quant_rowwise_with_block)             \
+    X(cinn_quant_rowwise_with_block_t) X(cinn_quant_blockwise) X(cinn_quant_blockwise_t) X(cinn_transpose_bytes)     \
+    X(cinn_requant_row_to_block) X(cinn_fp8_gemm)
+
+struct Api {
+#define CINN_DECL(name) decltype(&::name) name = nullptr;
+    CINN_HOST_API(CINN_DECL)
+#undef CINN_DECL
+};
+extern Api api;
+extern std::atomic<int64_t> launches;          // kernels of the library launched from here
+
+// A status of the library as an exception: `invalid` becomes Python's AssertionError, the rest LibraryError.
+struct CinnError : std::exception {
+    std::string msg;
+    bool invalid;
+    CinnError(std::string m, bool inv) : msg(std::move(m)), invalid(inv) {}
+    const char* what() const noexcept override { return msg.c_str(); }
+};
+
+inline void check(int status, const char* what) {
+    if (status == 0) return;
+    throw CinnError(std::string(what) + ": " + api.cinn_last_error() + " (status " + std::to_string(status) + ")", status == 1);
+}
+inline void require(bool ok, const char* what) {
+    if (!ok) throw CinnError(what, true);
+}
+
+constexpr int TAG_BF16 = 0, TAG_F32 = 1, TAG_F16 = 2, TAG_F32_BF16 = 3;
+inline int tag_of(at::ScalarType t) {           // -1: not a type the kernels read
+    switch (t) {
+        case at::kBFloat16: return TAG_BF16;
+        case at::kFloat: return TAG_F32;
+        case at::kHalf: return TAG_F16;
+        default: return -1;
+    }
+}
+inline Tensor readable(const Tensor& t) { return tag_of(t.scalar_type()) < 0 ? t.to(at::kFloat) : t; }
+
+inline Tensor empty(at::IntArrayRef size, at::ScalarType type, const at::Device& dev) {
+    return at::detail::empty_cuda(size, type, dev, std::nullopt);
+}
+inline int64_t up(int64_t a, int64_t b) { return (a + b - 1) / b; }
+inline void* stream() { return at::cuda::getCurrentCUDAStream().stream(); }
+inline float* f32(const Tensor& t) { return static_cast<float*>(t.data_ptr()); }
+
+}  // namespace cinnhost

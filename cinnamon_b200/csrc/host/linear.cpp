@@ -1,0 +1,199 @@
+// FP8 linear: forward and both gradients of FP8MatmulFunction (reference src/kernels.py:731-794) as one native call
+// each, and as a native autograd node.
+#include "host.h"
+
+namespace cinnhost {
+
+namespace {
+
+constexpr at::ScalarType F8 = at::kFloat8_e4m3fn;
+
+struct Linear {                                 // what the forward leaves for the backward
+    Tensor out, x, x_scale, w, w_scale, w_t;
+    bool x_is_block = false, x_is_block_t = false;
+};
+
+Tensor gemm(const Tensor& a, const Tensor& sa, const Tensor& b, int layout, const Tensor& sb, int64_t sbk, int64_t sbn, int64_t M,
+            int64_t N, int64_t K, at::ScalarType type, int tag) {
+    Tensor out = empty({M, N}, type, a.device());
+    check(api.cinn_fp8_gemm(a.data_ptr(), f32(sa), sa.stride(0), b.data_ptr(), f32(sb), sbk, sbn, out.data_ptr(), M, N, K, layout,
+                            tag, stream()), "cinn_fp8_gemm");
+    ++launches;
+    return out;
+}
+
+Linear forward(const Tensor& x, const Tensor& weight, bool round_scale, bool need_dgrad, bool need_wgrad, bool kmajor, int div,
+               const Tensor& w_q, const Tensor& w_s, const Tensor& w_qt) {
+    require(x.is_cuda(), "Input must be on CUDA");
+    c10::cuda::CUDAGuard guard(x.device());
+    const at::Device dev = x.device();
+    const int64_t K = x.size(-1), N = weight.size(0);
+    Tensor xf = readable(x.dim() == 2 ? x : x.reshape({-1, K}));
+    const int64_t M = xf.size(0), nkb = up(K, 128);
+    Linear r;
+    // When the weight will want a gradient, the block re-quantisation of the saved activations comes out of the same
+    // pass over x; it is written with the token axis contiguous where the token count allows, since the weight gradient
+    // reduces over tokens.
+    r.x_is_block = need_wgrad && K % 16 == 0;
+    r.x_is_block_t = r.x_is_block && M % 16 == 0 && kmajor;
+    Tensor xq = empty({M, K}, F8, dev), xs = empty({M, nkb}, at::kFloat, dev);
+    if (r.x_is_block) {
+        if (xf.stride(1) != 1) xf = xf.contiguous();
+        r.x = r.x_is_block_t ? empty({K, M}, F8, dev) : empty({M, K}, F8, dev);
+        r.x_scale = empty({up(M, 128), nkb}, at::kFloat, dev);
+        check((r.x_is_block_t ? api.cinn_quant_rowwise_with_block_t : api.cinn_quant_rowwise_with_block)(
+                  xf.data_ptr(), tag_of(xf.scalar_type()), M, K, xf.stride(0), xq.data_ptr(), f32(xs), r.x.data_ptr(), f32(r.x_scale),
+                  round_scale, div, stream()), "cinn_quant_rowwise_with_block");
+    } else {
+        check(api.cinn_quant_rowwise(xf.data_ptr(), tag_of(xf.scalar_type()), M, K, xf.stride(0), xf.stride(1), xq.data_ptr(), f32(xs),
+                                     128, round_scale, div, stream()), "cinn_quant_rowwise");
+        r.x = xq;
+        r.x_scale = xs;
+    }
+    ++launches;
+    if (w_q.defined()) {
+        r.w = w_q;
+        r.w_scale = w_s;
+        r.w_t = w_qt;
+    } else {
+        Tensor wf = readable(weight);
+        r.w = empty({N, K}, F8, dev);
+        r.w_scale = empty({up(N, 128), nkb}, at::kFloat, dev);
+        // the input gradient multiplies by the weight with N as the reduction axis: the byte-transposed copy it reads
+        // comes out of the same pass
+        if (kmajor && need_dgrad && N % 16 == 0 && K % 4 == 0 && wf.stride(1) == 1 && wf.stride(0) % 4 == 0) {
+            r.w_t = empty({K, N}, F8, dev);
+            check(api.cinn_quant_blockwise_t(wf.data_ptr(), tag_of(wf.scalar_type()), N, K, wf.stride(0), r.w.data_ptr(),
+                                             r.w_t.data_ptr(), f32(r.w_scale), 0, div, stream()), "cinn_quant_blockwise_t");
+        } else {
+            check(api.cinn_quant_blockwise(wf.data_ptr(), tag_of(wf.scalar_type()), N, K, wf.stride(0), wf.stride(1), r.w.data_ptr(),
+                                           f32(r.w_scale), 128, 128, 0, div, stream()), "cinn_quant_blockwise");
+        }
+        ++launches;
+    }
+    r.out = gemm(xq, xs, r.w, 0, r.w_scale, r.w_scale.stride(1), r.w_scale.stride(0), M, N, K, at::kBFloat16, TAG_BF16);
+    if (x.dim() != 2) {
+        auto shape = x.sizes().vec();
+        shape.back() = N;
+        r.out = r.out.view(shape);
+    }
+    return r;
+}
+
+std::tuple<Tensor, Tensor> backward(const Tensor& grad_out, Tensor x, Tensor x_scale, const Tensor& w, const Tensor& w_scale,
+                                    const Tensor& w_t, at::IntArrayRef x_shape, bool round_scale, bool x_is_block,
+                                    bool x_is_block_t, at::ScalarType weight_dtype, bool kmajor, int div, bool want_gx = true,
+                                    bool want_gw = true) {
+    c10::cuda::CUDAGuard guard(w.device());
+    const at::Device dev = w.device();
+    const int64_t N = w.size(0), K = w.size(1);
+    Tensor g = readable(grad_out.dim() == 2 ? grad_out : grad_out.reshape({-1, grad_out.size(-1)}));
+    if (g.stride(1) != 1) g = g.contiguous();
+    int64_t M = g.size(0);
+    const int64_t Mp = (M + 15) / 16 * 16;
+    // the token axis is the reduction axis of the weight gradient: a ragged count is padded with zero rows, which change
+    // neither an amax nor a sum (never with a transposed block copy: that needs a multiple of 16 tokens)
+    if (Mp != M) {
+        g = at::constant_pad_nd(g, {0, 0, 0, Mp - M});
+        x = at::constant_pad_nd(x.view(at::kByte), {0, 0, 0, Mp - M}).view(F8);
+        if (!x_is_block) x_scale = at::constant_pad_nd(x_scale, {0, 0, 0, Mp - M}, 1.0);
+    }
+    Tensor gq = empty({Mp, N}, F8, dev), gs = empty({Mp, up(N, 128)}, at::kFloat, dev);
+    Tensor gqt = empty({N, Mp}, F8, dev), gst = empty({N, up(Mp, 128)}, at::kFloat, dev);
+    check(api.cinn_quant_rowwise_dual(g.data_ptr(), tag_of(g.scalar_type()), Mp, N, g.stride(0), gq.data_ptr(), f32(gs),
+                                      gqt.data_ptr(), f32(gst), round_scale, div, stream()), "cinn_quant_rowwise_dual");
+    ++launches;
+    Tensor gx;
+    if (!want_gx) {
+    } else if (N % 16 == 0 && (kmajor || w_t.defined())) {
+        Tensor wt = w_t;
+        if (!wt.defined()) {
+            wt = empty({K, N}, F8, dev);
+            check(api.cinn_transpose_bytes(w.data_ptr(), w.stride(0), wt.data_ptr(), N, K, stream()), "cinn_transpose_bytes");
+            ++launches;
+        }
+        gx = gemm(gq, gs, wt, 0, w_scale, w_scale.stride(0), w_scale.stride(1), M, K, N, at::kBFloat16, TAG_BF16);
+    } else {
+        gx = gemm(gq, gs, w, 1, w_scale, w_scale.stride(0), w_scale.stride(1), M, K, N, at::kBFloat16, TAG_BF16);
+    }
+    if (gx.defined() && x_shape.size() != 2) gx = gx.reshape(x_shape);
+    if (!want_gw) return {gx, Tensor()};
+    if (!x_is_block) {
+        Tensor xb = empty({Mp, K}, F8, dev), xbs = empty({up(Mp, 128), up(K, 128)}, at::kFloat, dev);
+        x = x.contiguous();
+        x_scale = x_scale.contiguous();
+        check(api.cinn_requant_row_to_block(x.data_ptr(), f32(x_scale), Mp, K, xb.data_ptr(), f32(xbs), 0, div, stream()),
+              "cinn_requant_row_to_block");
+        ++launches;
+        x = xb;
+        x_scale = xbs;
+    }
+    // the reference returns a bf16 gradient that autograd casts to the master weight's type: the GEMM writes those values
+    const bool w32 = weight_dtype == at::kFloat;
+    Tensor gw = gemm(gqt, gst, x, x_is_block_t ? 0 : 1, x_scale, x_scale.stride(0), x_scale.stride(1), N, K, Mp,
+                     w32 ? at::kFloat : at::kBFloat16, w32 ? TAG_F32_BF16 : TAG_BF16);
+    return {gx, gw};
+}
+
+
+struct Quantised { Tensor q, s, q_t; };      // a weight already in e4m3 (undefined: quantise it here), handed around the node's tensors
+
+class LinearNode : public torch::autograd::Function<LinearNode> {
+public:
+    static Tensor forward(torch::autograd::AutogradContext* ctx, const Tensor& x, const Tensor& weight, bool round_scale, bool kmajor,
+                          int64_t div, const Quantised* wq) {
+        Linear r = cinnhost::forward(x, weight, round_scale, x.requires_grad(), weight.requires_grad(), kmajor, (int)div, wq->q, wq->s,
+                                     wq->q_t);
+        ctx->save_for_backward({r.x, r.x_scale, r.w, r.w_scale, r.w_t});
+        ctx->saved_data["x_shape"] = x.sizes().vec();
+        ctx->saved_data["flags"] = (int64_t)((round_scale ? 1 : 0) | (r.x_is_block ? 2 : 0) | (r.x_is_block_t ? 4 : 0) | (kmajor ? 8 : 0) |
+                                             ((int64_t)div << 4) | ((int64_t)weight.scalar_type() << 8));
+        return r.out;
+    }
+    static torch::autograd::variable_list backward(torch::autograd::AutogradContext* ctx, torch::autograd::variable_list grads) {
+        auto s = ctx->get_saved_variables();
+        const int64_t f = ctx->saved_data["flags"].toInt();
+        Tensor gx, gw;
+        try {
+            std::tie(gx, gw) = cinnhost::backward(grads[0], s[0], s[1], s[2], s[3], s[4], ctx->saved_data["x_shape"].toIntVector(), f & 1,
+                                                  f & 2, f & 4, (at::ScalarType)(f >> 8), f & 8, (f >> 4) & 15, ctx->needs_input_grad(0),
+                                                  ctx->needs_input_grad(1));
+        } catch (const CinnError& e) {
+            pybind11::gil_scoped_acquire gil;
+            PyErr_SetString(e.invalid ? PyExc_AssertionError : PyExc_RuntimeError, e.what());
+            python_error err;
+            err.persist();
+            throw err;
+        }
+        return {gx, gw, Tensor(), Tensor(), Tensor(), Tensor()};
+    }
+};
+
+Tensor or_none(const c10::optional<Tensor>& t) { return t.has_value() ? *t : Tensor(); }
+
+}  // namespace
+
+void bind_linear(pybind11::module_& m) {
+    using OptT = c10::optional<Tensor>;
+    // (out, x, x_scale, w, w_scale, w_t or None, x_is_block, x_is_block_t)
+    m.def("linear_forward", [](const Tensor& x, const Tensor& w, bool round_scale, bool need_dgrad, bool need_wgrad, bool kmajor, int div) {
+        Linear r = forward(x, w, round_scale, need_dgrad, need_wgrad, kmajor, div, Tensor(), Tensor(), Tensor());
+        return std::make_tuple(r.out, r.x, r.x_scale, r.w, r.w_scale, r.w_t.defined() ? OptT(r.w_t) : OptT(), r.x_is_block, r.x_is_block_t);
+    });
+    m.def("linear_backward", [](const Tensor& g, const Tensor& x, const Tensor& xs, const Tensor& w, const Tensor& ws, const OptT& wt,
+                                const std::vector<int64_t>& x_shape, bool round_scale, bool x_is_block, bool x_is_block_t, bool w_fp32,
+                                bool kmajor, int div) {
+        return backward(g, x, xs, w, ws, or_none(wt), x_shape, round_scale, x_is_block, x_is_block_t,
+                        w_fp32 ? at::kFloat : at::kBFloat16, kmajor, div);
+    });
+    // the differentiable call; without gradients to record nothing is saved and no gradient copies are made
+    m.def("linear", [](const Tensor& x, const Tensor& w, bool round_scale, bool kmajor, int div, const OptT& wq, const OptT& ws,
+                       const OptT& wqt) {
+        const Quantised cached{or_none(wq), or_none(ws), or_none(wqt)};
+        if (at::GradMode::is_enabled() && (x.requires_grad() || w.requires_grad()))
+            return LinearNode::apply(x, w, round_scale, kmajor, (int64_t)div, &cached);
+        return forward(x, w, round_scale, false, false, kmajor, div, cached.q, cached.s, cached.q_t).out;
+    });
+}
+
+}  // namespace cinnhost

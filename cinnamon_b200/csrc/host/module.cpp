@@ -1,0 +1,35 @@
+// Python module of the native host path: function pointers in, differentiable calls out.
+#include "host.h"
+
+namespace cinnhost {
+Api api;
+std::atomic<int64_t> launches{0};
+void bind_linear(pybind11::module_& m);
+}  // namespace cinnhost
+
+PYBIND11_MODULE(_host, m) {
+    using namespace cinnhost;
+    static pybind11::object library_error;
+    m.def("bind", [](const std::unordered_map<std::string, uintptr_t>& addr, pybind11::object error_type) {
+        library_error = std::move(error_type);
+#define CINN_BIND(name) api.name = reinterpret_cast<decltype(api.name)>(addr.at(#name));
+        CINN_HOST_API(CINN_BIND)
+#undef CINN_BIND
+    });
+    m.def("symbols", [] {
+        std::vector<std::string> names;
+#define CINN_NAME(name) names.push_back(#name);
+        CINN_HOST_API(CINN_NAME)
+#undef CINN_NAME
+        return names;
+    });
+    m.def("launches", [] { return launches.load(); });
+    pybind11::register_exception_translator([](std::exception_ptr p) {
+        try {
+            if (p) std::rethrow_exception(p);
+        } catch (const CinnError& e) {
+            PyErr_SetString(e.invalid ? PyExc_AssertionError : library_error.ptr(), e.what());
+        }
+    });
+    bind_linear(m);
+}

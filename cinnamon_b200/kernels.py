@@ -31,6 +31,7 @@ from . import _lib
 from .sparse_attention import SparseAttentionFunction, sparse_attention  # noqa: F401
 
 _L = _lib.lib
+_host = _lib.host
 FP8_E4M3_MAX = 448.0
 
 _DTYPE_TAG = {torch.bfloat16: _lib.BF16, torch.float32: _lib.F32, torch.float16: _lib.F16}
@@ -47,8 +48,9 @@ _KMAJOR_BACKWARD = os.environ.get("CINN_KMAJOR_BACKWARD", "1") != "0"
 _MOE_GROUPED_PRECISION = os.environ.get("CINN_MOE_GROUPED", "fp8")
 assert _MOE_GROUPED_PRECISION in ("fp8", "16bit"), "CINN_MOE_GROUPED must be fp8 or 16bit"
 
-# number of kernels of this library launched since import (the benchmark reports it)
-launch_count = 0
+# kernels of this library launched since import (the benchmark reports it): those launched from this file, to which
+# ``launch_count`` (a module attribute) adds those of the native host path
+_launches = 0
 # when set to a list, every GEMM launch appends a (start, end) pair of CUDA events to it
 gemm_events = None
 
@@ -82,8 +84,14 @@ def _ptr(t: torch.Tensor) -> ctypes.c_void_p:
 
 
 def _count(n: int = 1) -> None:
-    global launch_count
-    launch_count += n
+    global _launches
+    _launches += n
+
+
+def __getattr__(name: str):
+    if name == "launch_count":
+        return _launches + _host.launches()
+    raise AttributeError(f"module {__name__!r} has no attribute {name!r}")
 
 
 def device_status(reset: bool = True) -> int:
@@ -374,6 +382,14 @@ class FP8MatmulFunction(torch.autograd.Function):
         instead of once per call; the reference's three-argument call re-quantises every time (:747)."""
         assert x.is_cuda, "Input must be on CUDA"
         x_shape = x.shape
+        ctx.x_shape, ctx.round_scale, ctx.weight_dtype = x_shape, round_scale, weight.dtype
+        if weight_fp8 is None and gemm_events is None:
+            # the sequence below as one native call (csrc/host/linear.cpp)
+            out, *saved, ctx.w_fp8_t, ctx.x_is_block, ctx.x_is_block_t = _host.linear_forward(
+                x, weight, round_scale, ctx.needs_input_grad[0], ctx.needs_input_grad[1], _KMAJOR_BACKWARD, _DIV_MODE)
+            ctx.save_for_backward(*saved)
+            ctx.n_inputs = 3
+            return out
         x_flat = x.reshape(-1, x_shape[-1])
         M, K = x_flat.shape
         N = weight.shape[0]
@@ -411,9 +427,6 @@ class FP8MatmulFunction(torch.autograd.Function):
             ctx.save_for_backward(x_fp8, x_scale, w_fp8, w_scale)
         ctx.x_is_block = want_wgrad
         ctx.x_is_block_t = x_blk_t
-        ctx.x_shape = x_shape
-        ctx.round_scale = round_scale
-        ctx.weight_dtype = weight.dtype
         return out.reshape(*x_shape[:-1], -1)
 
     @staticmethod
@@ -421,6 +434,10 @@ class FP8MatmulFunction(torch.autograd.Function):
         x_fp8, x_scale, w_fp8, w_scale = ctx.saved_tensors
         x_shape = ctx.x_shape
         round_scale = ctx.round_scale
+        if gemm_events is None:
+            gx, gw = _host.linear_backward(grad_output, x_fp8, x_scale, w_fp8, w_scale, ctx.w_fp8_t, x_shape, round_scale, ctx.x_is_block,
+                                           ctx.x_is_block_t, ctx.weight_dtype == torch.float32, _KMAJOR_BACKWARD, _DIV_MODE)
+            return (gx, gw, None) + (None,) * (ctx.n_inputs - 3)
         N, K = w_fp8.shape
         grad_flat = grad_output.reshape(-1, grad_output.shape[-1])
         if grad_flat.stride(1) != 1:
@@ -496,17 +513,26 @@ class FP8Linear(torch.nn.Module):
                         self._w_cache = (key, (q, s, q_t))
                     else:
                         self._w_cache = (key, quantize_fp8_blockwise(wf, 128, 128))
-            out = FP8MatmulFunction.apply(x, w, self.round_scale, self._w_cache[1])
+            out = self._matmul(x, w, *self._w_cache[1])
         elif x.is_cuda and _ops is not None and torch.compiler.is_compiling():
             out = _ops.fp8_linear(x, self.weight, self.round_scale)       # one opaque graph node under torch.compile
         elif x.is_cuda:
-            out = FP8MatmulFunction.apply(x, self.weight, self.round_scale)
+            out = self._matmul(x, self.weight)
         else:
             # the reference does the same: an unquantised linear on CPU tensors (:823-824)
             out = torch.nn.functional.linear(x, self.weight, None)
         if self.bias is not None:
             out = out + self.bias
         return out
+
+    def _matmul(self, x, w, w_fp8=None, w_scale=None, w_fp8_t=None):
+        """``FP8MatmulFunction`` as a native autograd node (csrc/host/linear.cpp); as the Python one while the GEMMs are
+        being timed one by one."""
+        if gemm_events is not None:
+            if w_fp8 is None:
+                return FP8MatmulFunction.apply(x, w, self.round_scale)
+            return FP8MatmulFunction.apply(x, w, self.round_scale, (w_fp8, w_scale) if w_fp8_t is None else (w_fp8, w_scale, w_fp8_t))
+        return _host.linear(x, w, self.round_scale, _KMAJOR_BACKWARD, _DIV_MODE, w_fp8, w_scale, w_fp8_t)
 
     @classmethod
     def from_linear(cls, linear: torch.nn.Linear, round_scale: bool = False) -> "FP8Linear":
