@@ -35,6 +35,8 @@ SIGNATURES = {
     "cinn_swiglu_quant_rowwise_n": [_vp, _i32, _i64, _i64, _vp, _vp, _vp, _i32, _vp],
     "cinn_transpose_bytes": [_vp, _i64, _vp, _i64, _i64, _vp],
     "cinn_fp8_gemm": [_vp, _vp, _i64, _vp, _vp, _i64, _i64, _vp, _i64, _i64, _i64, _i32, _i32, _vp],
+    "cinn_fp8_gemm_workspace_bytes": [_i64, _i64, _i64, _i32],
+    "cinn_fp8_gemm_ws": [_vp, _vp, _i64, _vp, _vp, _i64, _i64, _vp, _i64, _i64, _i64, _i32, _i32, _vp, _i64, _vp],
     "cinn_grouped_gemm_16bit": [_vp, _vp, _i32, _vp, _vp, _i64, _i64, _i64, _i64, _vp, _i32, _vp],
     "cinn_fp8_grouped_gemm_dgrad": [_vp, _vp, _vp, _vp, _vp, _vp, _i64, _i64, _i64, _i64, _vp, _i32, _vp],
     "cinn_moe_combine": [_vp, _i32, _vp, _vp, _vp, _i64, _i64, _i32, _i64, _vp],
@@ -88,7 +90,7 @@ def _load() -> ctypes.CDLL:
         fn.argtypes = argtypes
         fn.restype = (ctypes.c_char_p if name == "cinn_last_error"
                       else ctypes.c_longlong if name == "cinn_set_wait_limit_cycles"
-                      else ctypes.c_int64 if name in ("cinn_moe_route_workspace_ints", "cinn_moe_route_static_max_ints",
+                      else ctypes.c_int64 if name in ("cinn_moe_route_workspace_ints", "cinn_moe_route_static_max_ints", "cinn_fp8_gemm_workspace_bytes",
                                                  "cinn_fp8_grouped_wgrad_scratch_bytes", "cinn_fp8_grouped_wgrad_fused_scratch_bytes")
                       else ctypes.c_int)
     return lib

@@ -41,7 +41,9 @@ int transpose_bytes(const void* in, int64_t ld_in, void* out, int64_t R, int64_t
 int swiglu_quant_rowwise(const void* h12, int dtype, int64_t T_rows, int64_t I, void* q, float* scales, int div_mode,
                          cudaStream_t st, const int64_t* n_rows_dev);
 int fp8_gemm(const void* A, const float* sA, int64_t ld_sa, const void* B, const float* sB, int64_t sbk, int64_t sbn,
-             void* C, int64_t M, int64_t N, int64_t K, int b_layout, int out_dtype, cudaStream_t st);
+             void* C, int64_t M, int64_t N, int64_t K, int b_layout, int out_dtype, cudaStream_t st, void* workspace,
+             int64_t workspace_bytes);
+int64_t fp8_gemm_workspace_bytes(int64_t M, int64_t N, int64_t K, int b_layout);
 int fp8_grouped_gemm(const void* A, const float* sA, const void* W, const float* sW, const int64_t* starts,
                      const int64_t* ends, int64_t E, int64_t T, int64_t d_in, int64_t d_out, void* C, int out_dtype,
                      cudaStream_t st, const long long* row_dst);
@@ -190,7 +192,18 @@ int cinn_fp8_gemm(const void* A, const float* sA, int64_t ld_sa, const void* B, 
                   int64_t sb_stride_n, void* C, int64_t M, int64_t N, int64_t K, int b_layout, int out_dtype,
                   void* stream) {
     return cinn::fp8_gemm(A, sA, ld_sa, B, sB, sb_stride_k, sb_stride_n, C, M, N, K, b_layout, out_dtype,
-                          (cudaStream_t)stream);
+                          (cudaStream_t)stream, nullptr, 0);
+}
+
+int64_t cinn_fp8_gemm_workspace_bytes(int64_t M, int64_t N, int64_t K, int b_layout) {
+    return cinn::fp8_gemm_workspace_bytes(M, N, K, b_layout);
+}
+
+int cinn_fp8_gemm_ws(const void* A, const float* sA, int64_t ld_sa, const void* B, const float* sB, int64_t sb_stride_k,
+                     int64_t sb_stride_n, void* C, int64_t M, int64_t N, int64_t K, int b_layout, int out_dtype,
+                     void* workspace, int64_t workspace_bytes, void* stream) {
+    return cinn::fp8_gemm(A, sA, ld_sa, B, sB, sb_stride_k, sb_stride_n, C, M, N, K, b_layout, out_dtype,
+                          (cudaStream_t)stream, workspace, workspace_bytes);
 }
 
 int cinn_fp8_grouped_gemm(const void* A, const float* sA, const void* W, const float* sW, const int64_t* starts,

@@ -48,6 +48,7 @@ struct GemmParams {
     void* C; int64_t ldc;          // scatter variant: C is a table of byte addresses, one per output row (0 = drop the row)
     int M, N, K;                   // dense: A is (M, K); grouped: M = total rows T
     const int64_t* starts; const int64_t* ends; int E; int b_rows_per_expert;
+    int splits;                    // SPLIT: pieces the reduction is cut into; C is then (splits, M, N) fp32 partial sums
     int tma_out;                   // 1: finished tiles leave through TMA stores (2-byte outputs, N % 8 == 0)
 };
 
@@ -243,7 +244,9 @@ __device__ __forceinline__ void store_rows_staged(const float* acc, uint8_t* sta
 // ---------------------------------------------------------------------------
 // the kernel
 // ---------------------------------------------------------------------------
-template <bool B_MN, bool GROUPED, int OUT, bool SCATTER = false>
+// SPLIT: a few tiles with a long reduction leave most SMs idle, so every tile is computed p.splits times over different
+// K blocks (tile t of n_total belongs to piece t / tiles) and the partial sums are added by split_sum_kernel.
+template <bool B_MN, bool GROUPED, int OUT, bool SCATTER = false, bool SPLIT = false>
 __global__ void __launch_bounds__(THREADS, 1)
 fp8_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                 const __grid_constant__ CUtensorMap tmC, const GemmParams p) {
@@ -305,8 +308,20 @@ fp8_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
 
-    const int KB = (p.K + BK - 1) / BK;
-    const int n_total = total_tiles<GROUPED>(p, cum);
+    const int KB_all = (p.K + BK - 1) / BK;
+    const int n_tiles_all = total_tiles<GROUPED>(p, cum);
+    const int n_total = SPLIT ? n_tiles_all * p.splits : n_tiles_all;
+    // tile t -> its K blocks [kb0, kb0 + KB) and its place in the output
+    auto blocks_of = [&](int t, int& kb0, int& KB) {
+        if constexpr (SPLIT) {
+            const int piece = t / n_tiles_all;
+            kb0 = (int)((int64_t)KB_all * piece / p.splits);
+            KB = (int)((int64_t)KB_all * (piece + 1) / p.splits) - kb0;
+        } else {
+            kb0 = 0; KB = KB_all;
+        }
+    };
+    auto tile_of = [&](int t) { return tile_info<GROUPED>(p, cum, SPLIT ? t % n_tiles_all : t); };
 
     if (warp >= EPI_WARPS) {
       if (warp == EPI_WARPS) {
@@ -315,7 +330,9 @@ fp8_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
             uint32_t it = 0;
             bool alive = true;
             for (int t = blockIdx.x; t < n_total && alive; t += gridDim.x) {
-                const TileInfo ti = tile_info<GROUPED>(p, cum, t);
+                const TileInfo ti = tile_of(t);
+                int kb0, KB;
+                blocks_of(t, kb0, KB);
                 const int b_row0 = GROUPED ? ti.expert * p.b_rows_per_expert : 0;
                 for (int kb = 0; kb < KB; ++kb, ++it) {
                     const int s = it % STAGES;
@@ -323,12 +340,13 @@ fp8_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
                     if (!mbar_wait(empty0 + 8 * s, ph ^ 1, abort_flag, (1 << 8) | 1)) { alive = false; break; }
                     const uint32_t fb = full0 + 8 * s;
                     mbar_expect_tx(fb, A_BYTES + B_BYTES);
-                    tma_load_2d(&tmA, fb, smem_u32(smem_a + s * A_BYTES), kb * BK, ti.m0);
+                    const int k = (kb0 + kb) * BK;
+                    tma_load_2d(&tmA, fb, smem_u32(smem_a + s * A_BYTES), k, ti.m0);
                     if constexpr (!B_MN) {
-                        tma_load_2d(&tmB, fb, smem_u32(smem_b + s * B_BYTES), kb * BK, b_row0 + ti.n0);
+                        tma_load_2d(&tmB, fb, smem_u32(smem_b + s * B_BYTES), k, b_row0 + ti.n0);
                     } else {
-                        tma_load_2d(&tmB, fb, smem_u32(smem_b + s * B_BYTES), ti.n0, b_row0 + kb * BK);
-                        tma_load_2d(&tmB, fb, smem_u32(smem_b + s * B_BYTES + B_BYTES / 2), ti.n0 + 128, b_row0 + kb * BK);
+                        tma_load_2d(&tmB, fb, smem_u32(smem_b + s * B_BYTES), ti.n0, b_row0 + k);
+                        tma_load_2d(&tmB, fb, smem_u32(smem_b + s * B_BYTES + B_BYTES / 2), ti.n0 + 128, b_row0 + k);
                     }
                 }
             }
@@ -354,6 +372,8 @@ fp8_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
             uint32_t it = 0, last = 0xffffffffu;
             bool alive = true;
             for (int t = blockIdx.x; t < n_total && alive; t += gridDim.x) {
+                int kb0, KB;
+                blocks_of(t, kb0, KB);
                 for (int kb = 0; kb < KB; ++kb, ++it) {
                     if ((it & 1u) != mine) continue;
                     last = it;
@@ -393,28 +413,38 @@ fp8_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
         // a tile does not start with an exposed round trip to L2 (it matters when K is only a few blocks).
         uint32_t n_rounds = 0;                   // staging rounds of this column group so far (two per TMA tile)
         float sa0 = 0.f, sb0 = 0.f, sa1 = 0.f, sb1 = 0.f, sa2 = 0.f, sb2 = 0.f;
-        auto scale_ptrs = [&](const TileInfo& ti, const float*& sa_ptr, const float*& sb_ptr) {
+        auto scale_ptrs = [&](const TileInfo& ti, int kb0, const float*& sa_ptr, const float*& sb_ptr) {
             const int row = ti.m0 + q * 32 + lane;
             const int col0 = ti.n0 + h * WCOLS;
             sa_ptr = p.sA + (int64_t)(row < ti.m_end ? row : ti.m0) * p.sa_stride_m;
             sb_ptr = p.sB + (int64_t)ti.expert * p.sb_stride_e + (int64_t)(col0 < p.N ? col0 / 128 : 0) * p.sb_stride_n;
+            if constexpr (SPLIT) {
+                sa_ptr += (int64_t)kb0 * p.sa_stride_k;
+                sb_ptr += (int64_t)kb0 * p.sb_stride_k;
+            }
         };
-        auto prefetch_scales = [&](const TileInfo& ti) {
+        auto prefetch_scales = [&](int t) {
+            const TileInfo ti = tile_of(t);
             const float *sa_ptr, *sb_ptr;
-            scale_ptrs(ti, sa_ptr, sb_ptr);
+            int kb0, KB;
+            blocks_of(t, kb0, KB);
+            scale_ptrs(ti, kb0, sa_ptr, sb_ptr);
             sa0 = ld_scale(sa_ptr); sb0 = ld_scale(sb_ptr);
             if (KB > 1) { sa1 = ld_scale(sa_ptr + p.sa_stride_k); sb1 = ld_scale(sb_ptr + p.sb_stride_k); }
             if (KB > 2) { sa2 = ld_scale(sa_ptr + 2 * p.sa_stride_k); sb2 = ld_scale(sb_ptr + 2 * p.sb_stride_k); }
         };
-        if ((int)blockIdx.x < n_total) prefetch_scales(tile_info<GROUPED>(p, cum, blockIdx.x));
+        if ((int)blockIdx.x < n_total) prefetch_scales(blockIdx.x);
         for (int t = blockIdx.x; t < n_total && alive; t += gridDim.x) {
-            const TileInfo ti = tile_info<GROUPED>(p, cum, t);
+            const TileInfo ti = tile_of(t);
+            int kb0, KB;
+            blocks_of(t, kb0, KB);
+            void* C = SPLIT ? (void*)(reinterpret_cast<float*>(p.C) + (int64_t)(t / n_tiles_all) * p.M * p.N) : p.C;
             const int row = ti.m0 + q * 32 + lane;
             const bool rvalid = row < ti.m_end;
             const int col0 = ti.n0 + h * WCOLS;
             const bool cvalid = col0 < p.N;
             const float *sa_ptr, *sb_ptr;
-            scale_ptrs(ti, sa_ptr, sb_ptr);
+            scale_ptrs(ti, kb0, sa_ptr, sb_ptr);
             float acc[WCOLS];
 #pragma unroll
             for (int i = 0; i < WCOLS; ++i) acc[i] = 0.0f;
@@ -453,7 +483,7 @@ fp8_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
                 __syncwarp();
                 if (lane == 0) mbar_arrive(tempty0 + 8 * b);
             }
-            if (alive && t + (int)gridDim.x < n_total) prefetch_scales(tile_info<GROUPED>(p, cum, t + gridDim.x));
+            if (alive && t + (int)gridDim.x < n_total) prefetch_scales(t + gridDim.x);
             constexpr bool TMA_OUT = (OUT == CINN_BF16 || OUT == CINN_F16);
             // A tile whose 128 rows all belong to it leaves through TMA stores.  Each column group of four
             // promotion warps owns one 16 KiB slot: its threads drop 64 columns of their rows into it (16-byte
@@ -495,13 +525,13 @@ fp8_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
                 if (!alive) break;
             } else if (alive && vec_ok && !(TMA_OUT && p.tma_out)) {
                 // warp-uniform: every lane takes part in the staging even if its own row is past the end
-                if (cvalid) store_rows_staged<OUT, WCOLS, SCATTER>(acc, store_stage + warp * 2048, p.C, p.ldc, ti.m0 + q * 32, ti.m_end, col0, p.N, lane);
+                if (cvalid) store_rows_staged<OUT, WCOLS, SCATTER>(acc, store_stage + warp * 2048, C, p.ldc, ti.m0 + q * 32, ti.m_end, col0, p.N, lane);
             } else if (alive && rvalid && cvalid) {
                 const int64_t base = (int64_t)row * p.ldc + col0;
 #pragma unroll
                 for (int j = 0; j < WCOLS / 8; ++j) {
                     const int ncols = p.N - (col0 + j * 8);
-                    if (ncols > 0) store8<OUT>(p.C, base + j * 8, &acc[j * 8], vec_ok, ncols);
+                    if (ncols > 0) store8<OUT>(C, base + j * 8, &acc[j * 8], vec_ok, ncols);
                 }
             }
         }
@@ -611,10 +641,10 @@ static int make_out_map(CUtensorMap* tc, const CUtensorMap& fallback, GemmParams
     return CINN_OK;
 }
 
-template <bool B_MN, bool GROUPED, int OUT, bool SCATTER = false>
+template <bool B_MN, bool GROUPED, int OUT, bool SCATTER = false, bool SPLIT = false>
 static int launch(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& tc, const GemmParams& p, int grid,
                   cudaStream_t st) {
-    constexpr auto kern = fp8_gemm_kernel<B_MN, GROUPED, OUT, SCATTER>;
+    constexpr auto kern = fp8_gemm_kernel<B_MN, GROUPED, OUT, SCATTER, SPLIT>;
     const size_t smem = smem_bytes(GROUPED ? p.E : 0);
     int rc = allow_smem_once<kern>(smem_bytes(GROUPED ? MAX_EXPERTS : 0));
     if (rc) return rc;
@@ -698,39 +728,136 @@ int set_gemm_sm_limit(int n) { return g_gemm_sm_limit.exchange(n < 0 ? 0 : n); }
 
 static inline bool al16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
 
+// ---------------------------------------------------------------------------
+// dense problems: which kernel, and into how many pieces the reduction is cut
+// ---------------------------------------------------------------------------
+// Sum of the `splits` partial results of every output element, in a fixed order (the result does not depend on which
+// piece finished first), rounded once.  Bound by reading the pieces, which were just written and mostly sit in L2.
+template <int OUT>
+__global__ void __launch_bounds__(256)
+split_sum_kernel(const float* __restrict__ part, void* __restrict__ out, int64_t n, int splits) {
+    using T = typename OutT<OUT>::type;
+    const int64_t i = ((int64_t)blockIdx.x * 256 + threadIdx.x) * 4;
+    if (i >= n) return;
+    float a[4] = {0.f, 0.f, 0.f, 0.f};
+    const bool vec = i + 4 <= n && (n & 3) == 0;
+    if (vec) {
+#pragma unroll 4
+        for (int s = 0; s < splits; ++s) {
+            const float4 v = __ldcs(reinterpret_cast<const float4*>(part + s * n + i));
+            a[0] += v.x; a[1] += v.y; a[2] += v.z; a[3] += v.w;
+        }
+    } else {
+        for (int s = 0; s < splits; ++s)
+            for (int j = 0; j < 4 && i + j < n; ++j) a[j] += part[s * n + i + j];
+    }
+    T* dst = reinterpret_cast<T*>(out) + i;
+    if constexpr (OUT == CINN_F32 || OUT == CINN_F32_BF16) {
+        if constexpr (OUT == CINN_F32_BF16)
+            for (int j = 0; j < 4; ++j) a[j] = __bfloat162float(__float2bfloat16_rn(a[j]));
+        if (vec) *reinterpret_cast<float4*>(dst) = make_float4(a[0], a[1], a[2], a[3]);
+        else for (int j = 0; j < 4 && i + j < n; ++j) dst[j] = a[j];
+    } else {
+        T h[4];
+        for (int j = 0; j < 4; ++j) {
+            if constexpr (OUT == CINN_BF16) h[j] = __float2bfloat16_rn(a[j]);
+            else h[j] = __float2half_rn(a[j]);
+        }
+        if (vec) *reinterpret_cast<uint2*>(dst) = *reinterpret_cast<const uint2*>(h);
+        else for (int j = 0; j < 4 && i + j < n; ++j) dst[j] = h[j];
+    }
+}
+
+static int launch_split_sum(const float* part, void* out, int64_t n, int splits, int out_dtype, cudaStream_t st) {
+    const unsigned grid = (unsigned)((n + 1023) / 1024);
+    switch (out_dtype) {
+        case CINN_BF16: split_sum_kernel<CINN_BF16><<<grid, 256, 0, st>>>(part, out, n, splits); break;
+        case CINN_F32: split_sum_kernel<CINN_F32><<<grid, 256, 0, st>>>(part, out, n, splits); break;
+        case CINN_F16: split_sum_kernel<CINN_F16><<<grid, 256, 0, st>>>(part, out, n, splits); break;
+        case CINN_F32_BF16: split_sum_kernel<CINN_F32_BF16><<<grid, 256, 0, st>>>(part, out, n, splits); break;
+        default: set_error("GEMM: unknown output dtype tag %d", out_dtype); return CINN_ERR_INVALID;
+    }
+    CINN_CHECK_LAUNCH();
+    return CINN_OK;
+}
+
+struct DensePlan { bool pair; int splits; };
+
+// A K block of a tile costs about 0.45 us in either kernel (a pair of SMs does twice the rows in it), a tile about 3 us
+// around its K blocks.  Splitting adds a pass over the partial sums: about 3 us of launch and the bytes at the rate L2
+// returns them.  The plan with the smallest sum of these wins; measured figures stand at the callers' cases.
+static DensePlan dense_plan(int64_t M, int64_t N, int64_t K, int b_layout, int64_t workspace_bytes) {
+    const int sms = gemm_sms();
+    const int64_t KB = (K + BK - 1) / BK;
+    auto waves = [](int64_t tiles, int64_t slots) { return (double)((tiles + slots - 1) / slots); };
+    const int64_t pair_tiles = ((M + pair::PM - 1) / pair::PM) * ((N + pair::PN - 1) / pair::PN);
+    const int64_t tiles = ((M + BM - 1) / BM) * ((N + BN - 1) / BN);
+    const double block_us = 0.45, tile_us = 3.0;
+    const int pm = pair_mode();
+    // the pair kernel wins with B K-major, the one-SM kernel with B MN-major
+    DensePlan best{false, 1};
+    double best_us = waves(tiles, sms) * (KB * block_us + tile_us);
+    if (pm == 2 ? pair_tiles >= sm_count() / 2 : (pm == 1 && b_layout == 0)) {
+        const double us = waves(pair_tiles, sms / 2) * (KB * block_us + tile_us);
+        if (us <= best_us * 1.02 || pm == 2) { best = {true, 1}; best_us = us; }
+    }
+    if (best_us < 12.0 || tiles >= sms) return best;
+    for (int s = 2; s <= 32 && s * 2 <= KB; ++s) {
+        const int64_t bytes = s * M * N * 4;
+        if (bytes > workspace_bytes) break;
+        const double us = waves(tiles * s, sms) * ((double)((KB + s - 1) / s) * block_us + tile_us) + 3.0 + bytes / 4e6;
+        if (us < 0.9 * best_us) { best = {false, s}; best_us = us; }
+    }
+    return best;
+}
+
+constexpr int64_t MAX_SPLIT_BYTES = 64LL << 20;
+
+int64_t fp8_gemm_workspace_bytes(int64_t M, int64_t N, int64_t K, int b_layout) {
+    if (M <= 0 || N <= 0 || K <= 0) return 0;
+    const DensePlan plan = dense_plan(M, N, K, b_layout, MAX_SPLIT_BYTES);
+    return plan.splits > 1 ? plan.splits * M * N * 4 : 0;
+}
+
 int fp8_gemm(const void* A, const float* sA, int64_t ld_sa, const void* B, const float* sB, int64_t sbk, int64_t sbn,
-             void* C, int64_t M, int64_t N, int64_t K, int b_layout, int out_dtype, cudaStream_t st) {
+             void* C, int64_t M, int64_t N, int64_t K, int b_layout, int out_dtype, cudaStream_t st, void* workspace,
+             int64_t workspace_bytes) {
     CINN_CHECK_ARG(M >= 0 && N >= 0 && K >= 0, "fp8_gemm: negative shape");
     if (M == 0 || N == 0) return CINN_OK;
     CINN_CHECK_ARG(A && sA && B && sB && C, "fp8_gemm: null pointer");
     CINN_CHECK_ARG(K > 0, "fp8_gemm: K must be positive");
     CINN_CHECK_ARG(M < (1LL << 31) && N < (1LL << 31) && K < (1LL << 31), "fp8_gemm: dimension too large");
     CINN_CHECK_ARG(K % 16 == 0, "fp8_gemm: K (%lld) must be a multiple of 16", (long long)K);
-    CINN_CHECK_ARG(al16(A) && al16(B) && al16(C), "fp8_gemm: A, B and C must be 16-byte aligned");
+    CINN_CHECK_ARG(al16(A) && al16(B) && al16(C) && al16(workspace), "fp8_gemm: A, B, C and the workspace must be 16-byte aligned");
     CINN_CHECK_ARG(b_layout == 0 || b_layout == 1, "fp8_gemm: unknown B layout %d", b_layout);
     CINN_CHECK_ARG(b_layout == 0 || N % 16 == 0, "fp8_gemm: B stored (K, N) needs N %% 16 == 0");
-    const int64_t pair_tiles = ((M + pair::PM - 1) / pair::PM) * ((N + pair::PN - 1) / pair::PN);
-    // measured on B200: the pair kernel wins with B K-major (forward), the one-SM kernel with B MN-major
-    const int pm = pair_mode();
-    const bool use_pair = pair_tiles >= sm_count() / 2 && (pm == 2 || (pm == 1 && b_layout == 0));
+    const DensePlan plan = dense_plan(M, N, K, b_layout, workspace ? workspace_bytes : 0);
     CUtensorMap ta, tb;
     int rc = make_map(&ta, A, (uint64_t)K, (uint64_t)M, (uint64_t)K, BK, BM);
     if (rc) return rc;
-    if (b_layout == 0) rc = make_map(&tb, B, (uint64_t)K, (uint64_t)N, (uint64_t)K, BK, use_pair ? 128 : BN);
+    if (b_layout == 0) rc = make_map(&tb, B, (uint64_t)K, (uint64_t)N, (uint64_t)K, BK, plan.pair ? 128 : BN);
     else rc = make_map(&tb, B, (uint64_t)N, (uint64_t)K, (uint64_t)N, 128, BK);
     if (rc) return rc;
     GemmParams p{};
     p.sA = sA; p.sa_stride_m = ld_sa; p.sa_stride_k = 1;
     p.sB = sB; p.sb_stride_k = sbk; p.sb_stride_n = sbn; p.sb_stride_e = 0;
     p.C = C; p.ldc = N; p.M = (int)M; p.N = (int)N; p.K = (int)K;
-    p.starts = nullptr; p.ends = nullptr; p.E = 1; p.b_rows_per_expert = 0;
-    if (use_pair) {
+    p.starts = nullptr; p.ends = nullptr; p.E = 1; p.b_rows_per_expert = 0; p.splits = 1;
+    if (plan.pair) {
+        const int64_t pair_tiles = ((M + pair::PM - 1) / pair::PM) * ((N + pair::PN - 1) / pair::PN);
         const int clusters = (int)(pair_tiles < gemm_sms() / 2 ? pair_tiles : gemm_sms() / 2);
         return b_layout == 0 ? launch_pair_out<false>(ta, tb, p, out_dtype, clusters, st)
                              : launch_pair_out<true>(ta, tb, p, out_dtype, clusters, st);
     }
-    const int64_t tiles = ((M + BM - 1) / BM) * ((N + BN - 1) / BN);
+    const int64_t tiles = ((M + BM - 1) / BM) * ((N + BN - 1) / BN) * plan.splits;
     const int grid = (int)(tiles < gemm_sms() ? tiles : gemm_sms());
+    if (plan.splits > 1) {
+        p.C = workspace; p.splits = plan.splits;
+        rc = b_layout == 0 ? launch<false, false, CINN_F32, false, true>(ta, tb, ta, p, grid, st)
+                           : launch<true, false, CINN_F32, false, true>(ta, tb, ta, p, grid, st);
+        if (rc) return rc;
+        return launch_split_sum(static_cast<const float*>(workspace), C, M * N, plan.splits, out_dtype, st);
+    }
     return b_layout == 0 ? launch_out<false, false>(ta, tb, p, out_dtype, grid, st)
                          : launch_out<true, false>(ta, tb, p, out_dtype, grid, st);
 }

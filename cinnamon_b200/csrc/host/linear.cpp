@@ -16,9 +16,11 @@ struct Linear {                                 // what the forward leaves for t
 Tensor gemm(const Tensor& a, const Tensor& sa, const Tensor& b, int layout, const Tensor& sb, int64_t sbk, int64_t sbn, int64_t M,
             int64_t N, int64_t K, at::ScalarType type, int tag) {
     Tensor out = empty({M, N}, type, a.device());
-    check(api.cinn_fp8_gemm(a.data_ptr(), f32(sa), sa.stride(0), b.data_ptr(), f32(sb), sbk, sbn, out.data_ptr(), M, N, K, layout,
-                            tag, stream()), "cinn_fp8_gemm");
-    ++launches;
+    const int64_t need = api.cinn_fp8_gemm_workspace_bytes(M, N, K, layout);       // few tiles, long reduction: cut along K
+    Tensor ws = need ? empty({need}, at::kByte, a.device()) : Tensor();
+    check(api.cinn_fp8_gemm_ws(a.data_ptr(), f32(sa), sa.stride(0), b.data_ptr(), f32(sb), sbk, sbn, out.data_ptr(), M, N, K, layout,
+                               tag, need ? ws.data_ptr() : nullptr, need, stream()), "cinn_fp8_gemm");
+    launches += need ? 2 : 1;
     return out;
 }
 

@@ -312,13 +312,15 @@ def _gemm(a, a_scales, b, b_layout, sb, sb_stride_k, sb_stride_n, M, N, K, out_d
         if gemm_events is not None:
             ev = (torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True))
             ev[0].record()
-        _lib.check(_L.cinn_fp8_gemm(_ptr(a), _ptr(a_scales), a_scales.stride(0), _ptr(b), _ptr(sb), sb_stride_k,
-                                    sb_stride_n, _ptr(out), M, N, K, b_layout, tag, _stream(a)),
+        need = int(_L.cinn_fp8_gemm_workspace_bytes(M, N, K, b_layout))      # few tiles, long reduction: cut along K
+        ws = torch.empty(need, dtype=torch.uint8, device=a.device) if need else None
+        _lib.check(_L.cinn_fp8_gemm_ws(_ptr(a), _ptr(a_scales), a_scales.stride(0), _ptr(b), _ptr(sb), sb_stride_k,
+                                       sb_stride_n, _ptr(out), M, N, K, b_layout, tag, _ptr(ws) if need else None, need, _stream(a)),
                    "cinn_fp8_gemm")
         if ev is not None:
             ev[1].record()
             gemm_events.append(ev)
-    _count()
+    _count(2 if need else 1)
     return out
 
 

@@ -140,6 +140,15 @@ int cinn_fp8_gemm(const void* A, const float* sA, int64_t ld_sa, const void* B, 
                   int64_t sb_stride_k, int64_t sb_stride_n, void* C, int64_t M, int64_t N, int64_t K,
                   int b_layout, int out_dtype, void* stream);
 
+/* The same product with a scratch buffer.  A problem with few output tiles and a long reduction (a weight gradient of a
+ * narrow layer, a few tokens through a wide one) is then cut along K over the whole GPU: fp32 partial sums go to the
+ * workspace and a second kernel adds them in a fixed order.  cinn_fp8_gemm_workspace_bytes says how much that takes
+ * (0: the problem fills the GPU as it is); a null or smaller workspace means fewer pieces, down to none. */
+int64_t cinn_fp8_gemm_workspace_bytes(int64_t M, int64_t N, int64_t K, int b_layout);
+int cinn_fp8_gemm_ws(const void* A, const float* sA, int64_t ld_sa, const void* B, const float* sB,
+                     int64_t sb_stride_k, int64_t sb_stride_n, void* C, int64_t M, int64_t N, int64_t K,
+                     int b_layout, int out_dtype, void* workspace, int64_t workspace_bytes, void* stream);
+
 /* Grouped (per-expert) block-scaled FP8 GEMM over ragged row ranges:
  * for each expert e:  C[starts[e]:ends[e], :] = A[starts[e]:ends[e], :] @ W[e]^T.
  * Replaces grouped_gemm_kernel + moe_grouped_gemm (src/kernels.py:440-523, 526-581); the reference runs it in

@@ -69,6 +69,25 @@ def test_gemm_layout_kn(K, M, N, Kd):
     assert err <= TOL and err <= 2e-5
 
 
+@pytest.mark.parametrize("M,N,Kd", [(128, 256, 8192), (1, 64, 7168), (130, 333, 6032), (1024, 512, 8208)])
+@pytest.mark.parametrize("kn", [False, True])
+def test_gemm_cut_along_k(K, M, N, Kd, kn):
+    """Few tiles, long reduction: partial sums over pieces of K (the last one short), added in a fixed order."""
+    if kn and N % 16:
+        pytest.skip("B stored (K, N) needs N % 16 == 0")
+    assert K._L.cinn_fp8_gemm_workspace_bytes(M, N, Kd, int(kn)) > 0
+    xq, xs, wq, ws = _operands(M, N, Kd, seed=M + N + Kd)
+    ref = O.fp8_matmul_f64(xq, wq.t(), xs, ws.t())
+    b = _f8(wq.t().contiguous()) if kn else _f8(wq).t()
+    for dtype in (torch.float32, torch.bfloat16):
+        out = K.fp8_matmul_dsv3(_f8(xq), b, xs.cuda(), ws.cuda().t(), out_dtype=dtype)
+        if dtype == torch.float32:
+            assert rel_fro(out, ref) <= 2e-5
+        else:
+            assert_bf16_close(out, ref, "bf16 output")
+        assert torch.equal(out, K.fp8_matmul_dsv3(_f8(xq), b, xs.cuda(), ws.cuda().t(), out_dtype=dtype))
+
+
 PAIR_SCRIPT = r"""
 import sys, torch
 sys.path.insert(0, sys.argv[1])
