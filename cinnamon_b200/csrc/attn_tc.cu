@@ -1,0 +1,1376 @@
+// Sparse attention on the tensor cores: see attn_tc.cuh for what it trades against the gather kernels.
+//
+// Scratch (from the caller, one block per call): what the queries picked (Picks), the bf16 parts of the inputs and one
+// flag word.  Everything is rebuilt on every call.
+//
+// What a dense tile cannot express falls back on the device, without the host knowing: a key picked more than 255 times
+// by one query, or results that are not finite (a NaN in a row nobody picked must not reach anyone, and 0 * NaN on a
+// tensor core would let it) set the flag, and the gather kernel, launched behind with that flag as its condition,
+// computes the whole call again.
+#include "attn_tc.cuh"
+#include <atomic>
+#include <cmath>
+
+namespace cinn {
+namespace atc {
+
+__device__ int g_attn_status = 0;          // 0, or (role << 8) | reason of a bounded wait that ran out
+
+// A bounded wait of a whole warp, with one verdict for all its lanes.
+__device__ __forceinline__ bool wait_warp(uint32_t bar, uint32_t parity, volatile int* abort_flag, int code) {
+    return __all_sync(0xffffffffu, mbar_wait_bounded(bar, parity, abort_flag, code, &g_attn_status));
+}
+
+// ---------------------------------------------------------------------------
+// what the queries picked
+// ---------------------------------------------------------------------------
+// One warp per query, in shared memory: the bits of its K indices, the running count of bits before every word, and from
+// these the rank of every slot's key.  Bound by reading the indices: 33 MB at 32 x 1024 queries x 128.
+__global__ void __launch_bounds__(128)
+picks_kernel(const int64_t* __restrict__ idx, uint32_t* __restrict__ bits, uint16_t* __restrict__ rank, uint8_t* __restrict__ count,
+             uint16_t* __restrict__ before_out, int* __restrict__ repeats, int* __restrict__ flag, int64_t n_rows, int L, int words, int K, int warps) {
+    extern __shared__ __align__(16) uint32_t sm[];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if (warp >= warps) return;
+    const int n_tiles = words / (T / 32);
+    uint32_t* b = sm + (size_t)warp * (2 * words + K);
+    uint32_t* before = b + words;
+    uint32_t* cnt = before + words;
+    for (int64_t w = (int64_t)blockIdx.x * warps + warp; w < n_rows; w += (int64_t)gridDim.x * warps) {
+        const int64_t bt = w / L;
+        const int t = (int)(w - bt * L);
+        const int64_t* row = idx + w * K;
+        for (int i = lane; i < words; i += 32) b[i] = 0u;
+        for (int i = lane; i < K; i += 32) cnt[i] = 0u;
+        __syncwarp();
+        for (int j = lane; j < K; j += 32) {
+            const int64_t i = row[j];
+            if (i >= 0 && i <= t) atomicOr(b + (i >> 5), 1u << (i & 31));
+        }
+        __syncwarp();
+        uint32_t carry = 0;
+        for (int i0 = 0; i0 < words; i0 += 32) {
+            const int i = i0 + lane;
+            const uint32_t n = i < words ? __popc(b[i]) : 0u;
+            uint32_t incl = n;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const uint32_t v = __shfl_up_sync(0xffffffffu, incl, o);
+                if (lane >= o) incl += v;
+            }
+            if (i < words) {
+                before[i] = carry + incl - n;
+                bits[w * words + i] = b[i];
+                before_out[w * words + i] = (uint16_t)before[i];
+            }
+            carry += __shfl_sync(0xffffffffu, incl, 31);
+        }
+        __syncwarp();
+        for (int j = lane; j < K; j += 32) {
+            const int64_t i = row[j];
+            uint32_t r = 0xffffu;
+            if (i >= 0 && i <= t) {
+                r = before[i >> 5] + __popc(b[i >> 5] & ((1u << (i & 31)) - 1u));
+                atomicAdd(cnt + r, 1u);
+            }
+            rank[w * K + j] = (uint16_t)r;
+        }
+        __syncwarp();
+        uint32_t most = 0;
+        for (int i = lane; i < K; i += 32) {
+            most = max(most, cnt[i]);
+            count[w * K + i] = (uint8_t)min(cnt[i], (uint32_t)MAX_COUNT);
+        }
+        if (most > 1) repeats[bt * n_tiles + t / T] = 1;
+        if (most > MAX_COUNT) *flag = 1;
+        __syncwarp();
+    }
+}
+
+// ---------------------------------------------------------------------------
+// bf16 parts of the inputs: (parts, rows, dpad), columns beyond d are zero
+// ---------------------------------------------------------------------------
+template <typename U> __device__ __forceinline__ float widen(U v);
+template <> __device__ __forceinline__ float widen<float>(float v) { return v; }
+template <> __device__ __forceinline__ float widen<__half>(__half v) { return __half2float(v); }
+template <> __device__ __forceinline__ float widen<__nv_bfloat16>(__nv_bfloat16 v) { return __bfloat162float(v); }
+
+struct SplitJob { const void* src; uint16_t* dst; int64_t rows; int d, dpad; };
+struct SplitJobs { SplitJob job[4]; int n; };
+
+// Bound by HBM: 4 bytes in and 6 out per fp32 element.
+template <typename U, int NS>
+__global__ void __launch_bounds__(256)
+split_parts_kernel(const SplitJobs jobs) {
+    for (int n = 0; n < jobs.n; ++n) {
+        const SplitJob jb = jobs.job[n];
+        const U* src = static_cast<const U*>(jb.src);
+        const int per_row = jb.dpad / 8;
+        const int64_t total = jb.rows * per_row, plane = jb.rows * jb.dpad;
+        const bool vec = jb.d % 8 == 0 && (reinterpret_cast<uintptr_t>(src) & 15) == 0;
+        for (int64_t e = (int64_t)blockIdx.x * 256 + threadIdx.x; e < total; e += (int64_t)gridDim.x * 256) {
+            const int64_t r = e / per_row;
+            const int c = (int)(e - r * per_row) * 8;
+            float v[8];
+            const U* p = src + r * jb.d + c;
+            if (vec && c < jb.d) {
+                if constexpr (sizeof(U) == 4) {
+                    const float4 a = __ldcs(reinterpret_cast<const float4*>(p)), b = __ldcs(reinterpret_cast<const float4*>(p) + 1);
+                    v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
+                } else {
+                    const uint4 raw = __ldcs(reinterpret_cast<const uint4*>(p));
+                    const U* u = reinterpret_cast<const U*>(&raw);
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) v[i] = widen<U>(u[i]);
+                }
+            } else {
+#pragma unroll
+                for (int i = 0; i < 8; ++i) v[i] = c + i < jb.d ? widen<U>(p[i]) : 0.0f;
+            }
+            uint32_t w[3][4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) split2(v[2 * i], v[2 * i + 1], w[0][i], w[1][i], w[2][i]);
+#pragma unroll
+            for (int s = 0; s < NS; ++s)
+                *reinterpret_cast<uint4*>(jb.dst + s * plane + r * jb.dpad + c) = make_uint4(w[s][0], w[s][1], w[s][2], w[s][3]);
+        }
+    }
+}
+
+// ---------------------------------------------------------------------------
+// forward
+// ---------------------------------------------------------------------------
+struct FwdArgs {
+    Picks picks;
+    float* out; void* out_cast; float* lse; float* attn; int* flag;
+    int H, L, words, K, Dv, BH, n_tiles, group;   // words: 32-key words per query
+    float scale;
+    int out_cast_tag;                      // CINN_BF16 / CINN_F16: the output once more in that type (out_cast)
+};
+
+// Blocks walk the heads in groups, within a group from the tiles with the most work to those with the least: the long
+// tiles of all its heads start first, and the heads in flight at a time (`group` of them, about three rounds of blocks)
+// keep their operands in L2.
+__device__ __forceinline__ void tile_of_block(int n_tiles, int BH, int group, int& tile, int& bh) {
+    const int g = blockIdx.x / (group * n_tiles), r = blockIdx.x - g * group * n_tiles;
+    const int heads = min(group, BH - g * group);
+    tile = n_tiles - 1 - r / heads;
+    bh = g * group + r % heads;
+}
+
+constexpr int FWD_THREADS = 10 * 32;       // two softmax warpgroups, TMA warp, MMA warp
+
+// Shared memory: queries [part][64-column panel] | ring of panels | barriers.
+template <int NS, int ND> struct FwdShape {
+    static constexpr int Q_PANELS = NS * ND;
+    static constexpr int RING = (Q_PANELS > 6 ? 4 : 6);
+    static constexpr int BAR_OFF = (Q_PANELS + RING) * PANEL;
+    static constexpr int BYTES = BAR_OFF + 256 + 1024 + T * 4;
+};
+
+// One CTA: 128 queries of one head and 64 value columns (blockIdx.z), over all key tiles up to the queries' own.  The two
+// softmax warpgroups take alternate key tiles, each with its own running maximum, sum and output accumulator, and merge
+// at the end: neither waits for the other, and while one turns scores into probabilities the tensor core works for the
+// other.  A thread owns a query.  It reads its 128 scores from tensor memory twice, 32 at a time: for the maximum of those
+// the query picked, whose raw values it leaves in the probabilities' output (by rank; permuted and normalised at the end),
+// and to write exp(score - max) back as three bf16 parts, the A operand of P V, in the columns it has just read and 64
+// beside them.  (Keeping the 128 scores in registers spilled, and with the operands in shared memory there is hardly an L1
+// for the spills: 1.3 ms where this takes 0.68, 32 x 8 x 1024 queries of 192 in fp32.)  256 of the 512 columns per warpgroup: 128 scores, 64 leading parts, 64 of
+// output.
+// NS: bf16 parts of q, k, v; ND: 64-column panels of q and k.
+template <int NS, int ND>
+__global__ void __launch_bounds__(FWD_THREADS, 1)
+attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
+                const __grid_constant__ CUtensorMap tmV, const FwdArgs a) {
+    using S = FwdShape<NS, ND>;
+    extern __shared__ uint8_t smem_raw[];
+    uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+    const uint32_t sq = smem_u32(smem), ring = sq + S::Q_PANELS * PANEL;
+    uint64_t* bars = reinterpret_cast<uint64_t*>(smem + S::BAR_OFF);
+    const uint32_t full0 = smem_u32(bars), empty0 = smem_u32(bars + S::RING), qfull = smem_u32(bars + 2 * S::RING);
+    const uint32_t sfull0 = qfull + 8, pready0 = qfull + 24, odone0 = qfull + 40;       // two each
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * S::RING + 7);
+    volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+    float* s_lse = reinterpret_cast<float*>(smem + S::BAR_OFF + 256);
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    int qt, bh;
+    tile_of_block(a.n_tiles, a.BH, a.group, qt, bh);
+    const int n_qt = a.n_tiles, half = blockIdx.z;
+    const int q0 = qt * T, n = qt + 1;                    // key tiles
+    if (tid == 0) {
+        *abort_flag = 0;
+        for (int i = 0; i < S::RING; ++i) { mbar_init(full0 + 8 * i, 1); mbar_init(empty0 + 8 * i, 1); }
+        mbar_init(qfull, 1);
+        for (int i = 0; i < 2; ++i) { mbar_init(sfull0 + 8 * i, 1); mbar_init(pready0 + 8 * i, 4); mbar_init(odone0 + 8 * i, 1); }
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == 9) tc_alloc(smem_u32(tmem_slot), 512);
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = *tmem_slot;
+
+    if (warp == 8) {
+        if (lane == 0) {
+            mbar_expect_tx(qfull, S::Q_PANELS * PANEL);
+            for (int p = 0; p < NS; ++p)
+                for (int c = 0; c < ND; ++c) tma_load_3d(&tmQ, qfull, sq + (p * ND + c) * PANEL, c * 64, q0, p * a.BH + bh);
+            uint32_t it = 0;
+            bool alive = true;
+            auto fetch = [&](const CUtensorMap* m, int x, int y, int z) {
+                const uint32_t s = it % S::RING, ph = (it / S::RING) & 1;
+                if (!alive || !mbar_wait_bounded(empty0 + 8 * s, ph ^ 1, abort_flag, (8 << 8) | 1, &g_attn_status)) { alive = false; return; }
+                mbar_expect_tx(full0 + 8 * s, PANEL);
+                tma_load_3d(m, full0 + 8 * s, ring + s * PANEL, x, y, z);
+                ++it;
+            };
+            for (int j = 0; j <= n && alive; ++j) {
+                if (j < n) {
+                    if constexpr (NS > 1)
+                        for (int c = 0; c < ND; ++c)
+                            for (int p = NS - 1; p >= 0; --p) fetch(&tmK, c * 64, j * T, p * a.BH + bh);
+                    for (int c = 0; c < ND; ++c) fetch(&tmK, c * 64, j * T, bh);
+                }
+                if (j > 0)
+                    for (int p = NS - 1; p >= 0; --p) fetch(&tmV, half * 64, (j - 1) * T, p * a.BH + bh);
+            }
+            if (!alive) {                                 // abandoned: let the copies in flight land
+                const long long t0 = clock64();
+                while (clock64() - t0 < 2000000LL) { }
+            }
+        }
+    } else if (warp == 9) {
+        if (wait_warp(qfull, 0, abort_flag, (8 << 8) | 2)) {
+            constexpr uint32_t id_s = make_idesc_f16(true, T, T), id_o = make_idesc_f16(true, T, 64, false, true);
+            uint32_t it = 0;
+            bool alive = true;
+            auto panel = [&](uint32_t& addr) {
+                const uint32_t s = it % S::RING;
+                if (!alive || !wait_warp(full0 + 8 * s, (it / S::RING) & 1, abort_flag, (8 << 8) | 3)) alive = false;
+                addr = ring + s * PANEL;
+                tc_fence_after();
+            };
+            for (int j = 0; j <= n && alive; ++j) {
+                if (j < n) {                              // scores of key tile j (over the probabilities of j - 2, whose product
+                    const uint32_t d = tmem + (j & 1) * 256;            // was issued before)
+                    bool first = true;
+                    // query parts [x_lo, x_hi] of column panel c against the ring's next key panel
+                    auto product = [&](int c, int x_hi, int x_lo) {
+                        uint32_t kp;
+                        panel(kp);
+                        if (!alive) return;
+                        const uint64_t kd = panel_desc(kp);
+                        uint64_t qd = panel_desc(sq + c * PANEL) + (uint64_t)(x_hi * ND * (PANEL >> 4));
+                        for (int x = x_hi; x >= x_lo; --x) {
+                            mma_panels(d, qd, kd, id_s, first);
+                            first = false;
+                            qd -= ND * (PANEL >> 4);
+                        }
+                        commit_elected(empty0 + 8 * (it % S::RING));
+                        ++it;
+                    };
+                    // The tensor core truncates the running sum at every step, so the small products go first and the
+                    // leading ones, for which the keys' leading parts are fetched again, last: ND x 4 truncations at full
+                    // size instead of six times as many.
+                    if constexpr (NS > 1)
+                        for (int c = 0; c < ND && alive; ++c)
+                            for (int p = NS - 1; p >= 0 && alive; --p) product(c, NS - 1 - p, p == 0 ? 1 : 0);
+                    for (int c = 0; c < ND && alive; ++c) product(c, 0, 0);
+                    commit_elected(sfull0 + 8 * (j & 1));
+                }
+                if (j > 0 && alive) {                     // output of key tile j - 1
+                    const int i = j - 1, w = i & 1;
+                    if (!wait_warp(pready0 + 8 * w, (i >> 1) & 1, abort_flag, (8 << 8) | 4)) { alive = false; break; }
+                    tc_fence_after();
+                    const uint32_t base = tmem + w * 256;
+                    bool first = NS > 1 || i < 2;
+                    for (int p = NS - 1; p >= 0 && alive; --p) {
+                        uint32_t vp;
+                        panel(vp);
+                        if (!alive) break;
+                        const uint64_t vd = panel_desc(vp);
+                        if (p == 0) { mma_part_at<2>(base + 192, base, base + 128, vd, id_o, first); first = false; }
+                        if (p <= 1) { mma_part_at<1>(base + 192, base, base + 128, vd, id_o, first); first = false; }
+                        mma_part_at<0>(base + 192, base, base + 128, vd, id_o, first);
+                        first = false;
+                        commit_elected(empty0 + 8 * (it % S::RING));
+                        ++it;
+                    }
+                    if (i + 2 >= n) commit_elected(odone0 + 8 * w);
+                }
+            }
+        }
+    } else {
+        const int wg = warp >> 2, quarter = warp & 3, r = quarter * 32 + lane;
+        const int t = q0 + r, b = bh / a.H;
+        const bool live = t < a.L;
+        const uint32_t base = tmem + ((uint32_t)(quarter * 32) << 16) + wg * 256;
+        const int64_t qrow = (int64_t)b * a.L + min(t, a.L - 1);
+        const uint4* bits = reinterpret_cast<const uint4*>(a.picks.bits + qrow * a.words);
+        const bool repeats = a.picks.repeats[b * n_qt + qt] != 0;
+        float* raw = a.attn + ((int64_t)bh * a.L + min(t, a.L - 1)) * a.K;          // the next picked key's raw score goes here
+        const uint8_t* count = a.picks.count + qrow * a.K;
+        const uint32_t push_mask = half == 0 ? ~0u : 0u;  // one of the column halves writes the scores
+        float m = -INFINITY, l = 0.0f;
+        // With three parts a tile's output is added up here, rounded to nearest: the tensor core truncates, and over a long
+        // row of tiles that would show in fp32.
+        constexpr bool KEEP = NS > 1;
+        float o_sum[KEEP ? 64 : 1];
+#pragma unroll
+        for (int i = 0; i < (KEEP ? 64 : 1); ++i) o_sum[i] = 0.0f;
+        auto add_output = [&] {
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+                float o[16];
+                tc_ld16(base + 192 + c * 16, o);
+#pragma unroll
+                for (int i = 0; i < 16; ++i) o_sum[(KEEP ? c * 16 + i : 0)] += o[i];
+            }
+        };
+        bool alive = true;
+        auto picked = [](const uint4& w) { return __popc(w.x) + __popc(w.y) + __popc(w.z) + __popc(w.w); };
+        const uint4 none = make_uint4(0u, 0u, 0u, 0u);
+        if (wg == 1 && live) {                            // the other warpgroup's tiles hold ranks as well
+            const int skip = picked(__ldg(bits));
+            raw += skip; count += skip;
+        }
+        uint4 mine = live && wg < n ? __ldg(bits + wg) : none;
+        for (int j = wg; j < n; j += 2) {
+            const uint4 cur = mine;
+            // bits of the next tile of either warpgroup, in flight during this one
+            const uint4 next = live && j + 1 < n ? __ldg(bits + j + 1) : none;
+            mine = live && j + 2 < n ? __ldg(bits + j + 2) : none;
+            if (!wait_warp(sfull0 + 8 * wg, (j >> 1) & 1, abort_flag, (8 << 8) | 5)) { alive = false; break; }
+            tc_fence_after();
+            if constexpr (KEEP)
+                if (j >= 2) add_output();                 // of tile j - 2, issued before these scores
+            // (one chunk of 32 columns per round and no further unrolling: unrolled, the two passes overran the
+            // instruction cache)
+            float mx[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+            uint4 w = cur;
+#pragma unroll 1
+            for (int c = 0; c < 4; ++c) {
+                uint32_t v[32];
+                ld32(base + c * 32, v);
+                ld_wait();
+                const uint32_t bit = w.x;
+                w = make_uint4(w.y, w.z, w.w, 0u);
+                const uint32_t push = bit & push_mask;
+                uint32_t at = 0;
+#pragma unroll
+                for (int i = 0; i < 32; ++i) {
+                    const float x = __uint_as_float(v[i]) * a.scale;
+                    mx[i & 3] = fmaxf(mx[i & 3], bit & (1u << i) ? x : -INFINITY);
+                    store_if(raw + at, x, push & (1u << i));
+                    at += (bit >> i) & 1u;
+                }
+                raw += at;
+            }
+            const float mt = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3]));
+            const uint8_t* count0 = count;
+            {
+                const int skip = picked(next);
+                raw += skip;
+                count += picked(cur) + skip;
+            }
+            // The reference point of the exponentials moves only when a score exceeds it by 5: sums stay below e^5 x K and
+            // nothing is lost, the output is rescaled once or twice in a row's life.
+            const bool move = mt > m + 5.0f || (m == -INFINITY && mt > -INFINITY);
+            if (__any_sync(0xffffffffu, move)) {
+                const float mn = move ? mt : m;
+                const float f = m == -INFINITY ? 0.0f : __expf(m - mn);
+                m = mn;
+                l *= f;
+                if constexpr (KEEP) {
+#pragma unroll
+                    for (int i = 0; i < 64; ++i) o_sum[i] *= f;
+                } else if (j >= 2) {
+#pragma unroll
+                    for (int c = 0; c < 4; ++c) {
+                        float o[16];
+                        uint32_t w[16];
+                        tc_ld16(base + 192 + c * 16, o);
+#pragma unroll
+                        for (int i = 0; i < 16; ++i) w[i] = __float_as_uint(o[i] * f);
+                        st16(base + 192 + c * 16, w);
+                    }
+                }
+            }
+            const float mu = m == -INFINITY ? 0.0f : m;
+            w = cur;
+#pragma unroll 1
+            for (int c = 0; c < 4; ++c) {
+                uint32_t v[32];
+                float p[32];
+                ld32(base + c * 32, v);
+                ld_wait();
+                const uint32_t bit = w.x;
+                w = make_uint4(w.y, w.z, w.w, 0u);
+#pragma unroll
+                for (int i = 0; i < 32; ++i) p[i] = exp_fast(bit & (1u << i) ? fmaf(__uint_as_float(v[i]), a.scale, -mu) : -INFINITY);
+                if (repeats) {                            // a key picked several times counts as often
+#pragma unroll
+                    for (int i = 0; i < 32; ++i)
+                        if (bit & (1u << i)) p[i] *= (float)*count0++;
+                }
+#pragma unroll
+                for (int i = 0; i < 32; i += 4) l += (p[i] + p[i + 1]) + (p[i + 2] + p[i + 3]);
+                // over the 32 scores just read go the second and third parts, the leading parts beside the scores
+                store_parts32(base + c * 32, base + 128 + c * 16, p);
+            }
+            st_wait();
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(pready0 + 8 * wg);
+        }
+        const bool ran = n > wg;
+        for (int i = 0; i < min(n, 2) && alive; ++i) {                  // every product has been added, no panel is read any more
+            alive = wait_warp(odone0 + 8 * i, 0, abort_flag, (8 << 8) | 6);
+        }
+        tc_fence_after();
+        if constexpr (KEEP)
+            if (ran && alive) add_output();
+        // merge: the second warpgroup leaves its state in the operand panels
+        float* merge = reinterpret_cast<float*>(smem);                   // [66][128], column r: conflict-free
+        if (wg == 1) {
+            merge[64 * T + r] = ran ? m : -INFINITY;
+            merge[65 * T + r] = l;
+            if (ran && alive) {
+#pragma unroll
+                for (int c = 0; c < 4; ++c) {
+                    float o[16];
+                    if constexpr (KEEP) {
+#pragma unroll
+                        for (int i = 0; i < 16; ++i) o[i] = o_sum[c * 16 + i];
+                    } else {
+                        tc_ld16(base + 192 + c * 16, o);
+                    }
+#pragma unroll
+                    for (int i = 0; i < 16; ++i) merge[(c * 16 + i) * T + r] = o[i];
+                }
+            }
+        }
+        asm volatile("bar.sync 1, 256;" ::: "memory");
+        if (wg == 0) {
+            const float m1 = merge[64 * T + r], l1 = merge[65 * T + r];
+            const float mm = fmaxf(m, m1);
+            const float f0 = m == -INFINITY ? 0.0f : __expf(m - mm), f1 = m1 == -INFINITY ? 0.0f : __expf(m1 - mm);
+            const float sum = l * f0 + l1 * f1;
+            const float inv = sum > 0.0f ? 1.0f / sum : 0.0f;
+            const float lse = sum > 0.0f ? mm + logf(sum) : 0.0f;
+            s_lse[r] = lse;
+            bool bad = false;
+            const int cols = min(64, a.Dv - half * 64);
+            float* orow = a.out + ((int64_t)bh * a.L + t) * a.Dv + half * 64;
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+                float o[16];
+                if constexpr (KEEP) {
+#pragma unroll
+                    for (int i = 0; i < 16; ++i) o[i] = o_sum[c * 16 + i];
+                } else {
+                    tc_ld16(base + 192 + c * 16, o);
+                }
+#pragma unroll
+                for (int i = 0; i < 16; ++i) {
+                    const float o1 = m1 == -INFINITY ? 0.0f : merge[(c * 16 + i) * T + r] * f1;
+                    o[i] = (o[i] * f0 + o1) * inv;
+                    bad |= !(fabsf(o[i]) <= 3.4e38f);
+                }
+                if (live && alive) {
+                    if (cols == 64 && (a.Dv & 3) == 0) {
+#pragma unroll
+                        for (int i = 0; i < 16; i += 4)
+                            *reinterpret_cast<float4*>(orow + c * 16 + i) = make_float4(o[i], o[i + 1], o[i + 2], o[i + 3]);
+                    } else {
+                        for (int i = 0; i < 16; ++i)
+                            if (c * 16 + i < cols) orow[c * 16 + i] = o[i];
+                    }
+                    if (a.out_cast) {
+                        uint16_t* crow = static_cast<uint16_t*>(a.out_cast) + ((int64_t)bh * a.L + t) * a.Dv + half * 64 + c * 16;
+                        uint32_t w[8];
+#pragma unroll
+                        for (int i = 0; i < 8; ++i) {
+                            if (a.out_cast_tag == CINN_BF16) {
+                                const __nv_bfloat162 h = __floats2bfloat162_rn(o[2 * i], o[2 * i + 1]);
+                                w[i] = *reinterpret_cast<const uint32_t*>(&h);
+                            } else {
+                                const __half2 h = __floats2half2_rn(o[2 * i], o[2 * i + 1]);
+                                w[i] = *reinterpret_cast<const uint32_t*>(&h);
+                            }
+                        }
+                        if (cols == 64 && (a.Dv & 7) == 0) {
+                            *reinterpret_cast<uint4*>(crow) = make_uint4(w[0], w[1], w[2], w[3]);
+                            *reinterpret_cast<uint4*>(crow + 8) = make_uint4(w[4], w[5], w[6], w[7]);
+                        } else {
+                            for (int i = 0; i < 16; ++i)
+                                if (c * 16 + i < cols) crow[i] = (uint16_t)(w[i >> 1] >> (16 * (i & 1)));
+                        }
+                    }
+                }
+            }
+            if (live && bad) *a.flag = 1;
+            if (live && half == 0) a.lse[(int64_t)bh * a.L + t] = lse;
+        }
+        asm volatile("bar.sync 1, 256;" ::: "memory");
+        // Raw scores by rank -> probabilities by slot.  A warp takes sixteen pieces of 32 slots at a time with all loads in
+        // flight, whole rows of them: every slot of a row is read before any is written.
+        if (half == 0 && alive) {
+            constexpr int U = MAX_SLOTS / 32;
+            const int chunks = (a.K + 31) / 32, per = U / chunks, rows = min(T, a.L - q0);
+            const uint16_t* rank = a.picks.rank + ((int64_t)b * a.L + q0) * a.K;
+            float* attn = a.attn + ((int64_t)bh * a.L + q0) * a.K;
+            for (int k0 = warp; k0 < rows; k0 += 8 * per) {              // rows k0, k0 + 8, ...
+                float v[U];
+                uint32_t c[U];
+                int rr = k0, j = lane;                    // piece u of the batch: its row and this lane's slot
+                auto advance = [&] { if ((j += 32) >= chunks * 32) { j = lane; rr += 8; } };
+                const int end = min(rows, k0 + 8 * per);
+#pragma unroll
+                for (int u = 0; u < U; ++u, advance()) {
+                    // (loads from clamped places and a choice afterwards: behind a condition they would go one by one)
+                    const uint32_t x = rank[min(rr, end - 1) * a.K + min(j, a.K - 1)];
+                    c[u] = rr < end && j < a.K ? x : 0xffffu;
+                }
+                rr = k0; j = lane;
+#pragma unroll
+                for (int u = 0; u < U; ++u, advance()) {
+                    const float x = attn[min(rr, end - 1) * a.K + min((int)c[u], a.K - 1)];
+                    v[u] = c[u] != 0xffffu ? x : -INFINITY;
+                }
+                __syncwarp();
+                rr = k0; j = lane;
+#pragma unroll
+                for (int u = 0; u < U; ++u, advance())
+                    if (rr < end && j < a.K) attn[rr * a.K + j] = exp_fast(v[u] - s_lse[rr]);
+            }
+        }
+    }
+    tc_fence_before();
+    __syncthreads();
+    if (warp == 9) {
+        tc_fence_after();
+        tc_dealloc(tmem, 512);
+    }
+}
+
+// ---------------------------------------------------------------------------
+// backward
+// ---------------------------------------------------------------------------
+// delta[row] = sum_d dO[row, d] * O[row, d]; one warp per row, bound by reading both
+template <typename U>
+__global__ void __launch_bounds__(256)
+delta_kernel(const U* __restrict__ d_out, const float* __restrict__ out, float* __restrict__ delta, int64_t rows, int Dv) {
+    const int lane = threadIdx.x & 31;
+    for (int64_t w = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5); w < rows; w += (int64_t)gridDim.x * 8) {
+        float s = 0.0f;
+        for (int d = lane; d < Dv; d += 32) s = fmaf(widen<U>(d_out[w * Dv + d]), out[w * Dv + d], s);
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+        if (lane == 0) delta[w] = s;
+    }
+}
+
+struct BwdArgs {
+    Picks picks;
+    const float* lse; const float* delta;
+    float* p; float* ds;                   // (B H, L, K) by rank: probability times count, and its score gradient
+    void* dq; void* dk; void* dv;          // in `tag`'s type
+    int* flag;
+    int H, L, words, K, Dqk, Dv, BH, n_tiles, group, tag;
+    float scale;
+};
+
+// 16 fp32 values of one row to `dst + col` (elements of `tag`'s type); the row has `width` columns
+__device__ __forceinline__ void store_row16(void* dst, int64_t row, int col, int width, int tag, const float (&o)[16]) {
+    if (tag == CINN_F32) {
+        float* d = static_cast<float*>(dst) + row * width + col;
+        if (col + 16 <= width && (width & 3) == 0) {
+#pragma unroll
+            for (int i = 0; i < 16; i += 4) *reinterpret_cast<float4*>(d + i) = make_float4(o[i], o[i + 1], o[i + 2], o[i + 3]);
+        } else {
+            for (int i = 0; i < 16; ++i)
+                if (col + i < width) d[i] = o[i];
+        }
+    } else {
+        uint16_t* d = static_cast<uint16_t*>(dst) + row * width + col;
+        uint32_t w[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            if (tag == CINN_BF16) {
+                const __nv_bfloat162 h = __floats2bfloat162_rn(o[2 * i], o[2 * i + 1]);
+                w[i] = *reinterpret_cast<const uint32_t*>(&h);
+            } else {
+                const __half2 h = __floats2half2_rn(o[2 * i], o[2 * i + 1]);
+                w[i] = *reinterpret_cast<const uint32_t*>(&h);
+            }
+        }
+        if (col + 16 <= width && (width & 7) == 0) {
+            *reinterpret_cast<uint4*>(d) = make_uint4(w[0], w[1], w[2], w[3]);
+            *reinterpret_cast<uint4*>(d + 8) = make_uint4(w[4], w[5], w[6], w[7]);
+        } else {
+            for (int i = 0; i < 16; ++i)
+                if (col + i < width) d[i] = (uint16_t)(w[i >> 1] >> (16 * (i & 1)));
+        }
+    }
+}
+
+// Adds pieces c0, c0 + STEP, ... < c1 of 16 accumulator columns to (or, the first time, writes them over) fp32 rows in
+// global memory, rounded to nearest.  The tensor core truncates its running sums at every step, which over thousands of
+// queries would show in an fp32 gradient; so the sums are taken out every few hundred steps and started afresh.  U pieces
+// are in flight at a time.
+template <int STEP, int U, typename ROW>
+__device__ __forceinline__ void flush_pieces(uint32_t taddr, int c0, int c1, bool live, bool add, bool& bad, ROW&& row_of) {
+#pragma unroll 1
+    for (int c = c0; c < c1; c += U * STEP) {
+        float o[U][16];
+        float4 old[U][4];
+        float* dst[U];
+        int n[U];
+        bool vec[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            n[u] = 0;
+            vec[u] = false;
+            if (c + STEP * u >= c1) continue;
+            dst[u] = row_of(c + STEP * u, n[u]);              // the piece's place and how many of its columns exist
+            n[u] = live ? n[u] : 0;
+            vec[u] = n[u] == 16 && (reinterpret_cast<uintptr_t>(dst[u]) & 15) == 0;
+            if (add && vec[u])
+#pragma unroll
+                for (int i = 0; i < 4; ++i) old[u][i] = reinterpret_cast<const float4*>(dst[u])[i];
+            tc_ld16(taddr + (c + STEP * u) * 16, o[u]);
+#pragma unroll
+            for (int i = 0; i < 16; ++i) bad |= live && !(fabsf(o[u][i]) <= 3.4e38f);
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            if (vec[u]) {
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    float4 x = make_float4(o[u][4 * i], o[u][4 * i + 1], o[u][4 * i + 2], o[u][4 * i + 3]);
+                    if (add) { x.x += old[u][i].x; x.y += old[u][i].y; x.z += old[u][i].z; x.w += old[u][i].w; }
+                    reinterpret_cast<float4*>(dst[u])[i] = x;
+                }
+            } else {
+#pragma unroll
+                for (int i = 0; i < 16; ++i)
+                    if (i < n[u]) dst[u][i] = (add ? dst[u][i] : 0.0f) + o[u][i];
+            }
+        }
+    }
+}
+
+// Shared memory of the query pass: queries and output gradients resident, a ring of key / value panels.  Of three parts
+// the smallest, which meets only the leading part of k and v, comes through the ring too: with everything resident two
+// panels were left, and the copies' latency bounded the pass (1.40 ms at 32 x 8 x 1024 queries of 192 in fp32).
+template <int NS, int ND, int NV> struct QPassShape {
+    static constexpr int KEPT = NS > 1 ? 2 : 1;            // resident parts
+    static constexpr int FIXED = KEPT * (ND + NV);
+    static constexpr int RING = FIXED > 8 ? 14 - FIXED : 6;
+    static constexpr int BAR_OFF = (FIXED + RING) * PANEL;
+    static constexpr int BYTES = BAR_OFF + 256 + 1024;
+};
+
+// Query pass: one CTA per 128 queries of a head, over their key tiles.  S = q k^T and dP = dO v^T in tensor memory; a
+// thread (a query, half of the tile's keys) turns them into p = exp(scale S - lse) and dS = p (dP - delta) scale, leaves
+// both by rank for the key pass, and writes dS back as an A operand for dq += dS k.  All of tensor memory: 128 columns of
+// S under the second and third parts of dS, 128 of dP, 64 of dS's leading parts, 192 of dq.
+template <int NS, int ND, int NV>
+__global__ void __launch_bounds__(FWD_THREADS, 1)
+attn_bwd_query_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
+                      const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmG, const BwdArgs a) {
+    using S = QPassShape<NS, ND, NV>;
+    extern __shared__ uint8_t smem_raw[];
+    uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+    const uint32_t sq = smem_u32(smem), sg = sq + S::KEPT * ND * PANEL, ring = sq + S::FIXED * PANEL;
+    uint64_t* bars = reinterpret_cast<uint64_t*>(smem + S::BAR_OFF);
+    const uint32_t full0 = smem_u32(bars), empty0 = smem_u32(bars + S::RING), qfull = smem_u32(bars + 2 * S::RING);
+    const uint32_t sfull = qfull + 8, dsready = qfull + 16, done = qfull + 24, taken = qfull + 32;
+    constexpr int EVERY = 2;                              // fp32 gradients: tiles between two flushes
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * S::RING + 5);
+    volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    int qt, bh;
+    tile_of_block(a.n_tiles, a.BH, a.group, qt, bh);
+    const int q0 = qt * T, n = qt + 1;
+    const bool flush = NS > 1 && a.tag == CINN_F32;
+    if (tid == 0) {
+        *abort_flag = 0;
+        for (int i = 0; i < S::RING; ++i) { mbar_init(full0 + 8 * i, 1); mbar_init(empty0 + 8 * i, 1); }
+        mbar_init(qfull, 1); mbar_init(sfull, 1); mbar_init(dsready, 8); mbar_init(done, 1); mbar_init(taken, 8);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == 9) tc_alloc(smem_u32(tmem_slot), 512);
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = *tmem_slot, t_s = tmem, t_dp = tmem + 128, t_lead = tmem + 256, t_dq = tmem + 320;
+
+    if (warp == 8) {
+        if (lane == 0) {
+            mbar_expect_tx(qfull, S::FIXED * PANEL);
+            for (int p = 0; p < S::KEPT; ++p) {
+                for (int c = 0; c < ND; ++c) tma_load_3d(&tmQ, qfull, sq + (p * ND + c) * PANEL, c * 64, q0, p * a.BH + bh);
+                for (int c = 0; c < NV; ++c) tma_load_3d(&tmG, qfull, sg + (p * NV + c) * PANEL, c * 64, q0, p * a.BH + bh);
+            }
+            uint32_t it = 0;
+            bool alive = true;
+            auto fetch = [&](const CUtensorMap* m, int x, int y, int z) {
+                const uint32_t s = it % S::RING, ph = (it / S::RING) & 1;
+                if (!alive || !mbar_wait_bounded(empty0 + 8 * s, ph ^ 1, abort_flag, (9 << 8) | 1, &g_attn_status)) { alive = false; return; }
+                mbar_expect_tx(full0 + 8 * s, PANEL);
+                tma_load_3d(m, full0 + 8 * s, ring + s * PANEL, x, y, z);
+                ++it;
+            };
+            for (int j = 0; j < n && alive; ++j) {
+                if constexpr (NS > 1)
+                    for (int c = 0; c < ND; ++c) {
+                        for (int p = NS - 1; p >= 0; --p) fetch(&tmK, c * 64, j * T, p * a.BH + bh);
+                        fetch(&tmQ, c * 64, q0, 2 * a.BH + bh);
+                    }
+                for (int c = 0; c < ND; ++c) fetch(&tmK, c * 64, j * T, bh);
+                for (int c = 0; c < NV; ++c) {
+                    for (int p = NS - 1; p >= 0; --p) fetch(&tmV, c * 64, j * T, p * a.BH + bh);
+                    if constexpr (NS > 1) fetch(&tmG, c * 64, q0, 2 * a.BH + bh);
+                }
+                for (int c = 0; c < ND; ++c)
+                    for (int p = NS - 1; p >= 0; --p) fetch(&tmK, c * 64, j * T, p * a.BH + bh);
+            }
+            if (!alive) {                                 // abandoned: let the copies in flight land
+                const long long t0 = clock64();
+                while (clock64() - t0 < 2000000LL) { }
+            }
+        }
+    } else if (warp == 9) {
+        if (wait_warp(qfull, 0, abort_flag, (9 << 8) | 2)) {
+            constexpr uint32_t id_s = make_idesc_f16(true, T, T), id_o = make_idesc_f16(true, T, 64, false, true);
+            uint32_t it = 0;
+            bool alive = true;
+            auto panel = [&](uint32_t& addr) {
+                const uint32_t s = it % S::RING;
+                if (!alive || !wait_warp(full0 + 8 * s, (it / S::RING) & 1, abort_flag, (9 << 8) | 3)) alive = false;
+                addr = ring + s * PANEL;
+                tc_fence_after();
+            };
+            auto release = [&] {
+                commit_elected(empty0 + 8 * (it % S::RING));
+                ++it;
+            };
+            // parts [x_lo, x_hi] of a resident panel (parts `stride` panels apart) against the ring's next panel; with
+            // `small`, the panel after it holds the third part, which goes first
+            auto product = [&](uint32_t d, uint32_t fixed, int stride, int x_hi, int x_lo, bool small, bool& first) {
+                uint32_t bp, ap;
+                panel(bp);
+                if (!alive) return;
+                const uint64_t bd = panel_desc(bp);
+                if (small) {
+                    const uint32_t held = it++;            // (released below, once every product with it has been issued)
+                    panel(ap);
+                    if (!alive) return;
+                    mma_panels(d, panel_desc(ap), bd, id_s, first);
+                    first = false;
+                    release();
+                    it = held;
+                }
+                uint64_t ad = panel_desc(fixed) + (uint64_t)(x_hi * stride * (PANEL >> 4));
+                for (int x = x_hi; x >= x_lo; --x) {
+                    mma_panels(d, ad, bd, id_s, first);
+                    first = false;
+                    ad -= stride * (PANEL >> 4);
+                }
+                release();
+                if (small) ++it;
+            };
+            for (int j = 0; j < n && alive; ++j) {
+                // (S overwrites the parts of dS that dq of tile j - 1 reads: issued after it, executed after it)
+                bool first = true;
+                if constexpr (NS > 1)
+                    for (int c = 0; c < ND && alive; ++c) {
+                        product(t_s, sq + c * PANEL, ND, 0, 0, false, first);                  // third part of k
+                        if (alive) product(t_s, sq + c * PANEL, ND, 1, 0, false, first);       // second
+                        if (alive) product(t_s, sq + c * PANEL, ND, 1, 1, true, first);        // leading, without q's leading part
+                    }
+                for (int c = 0; c < ND && alive; ++c) product(t_s, sq + c * PANEL, ND, 0, 0, false, first);
+                first = true;
+                for (int c = 0; c < NV && alive; ++c) {
+                    if constexpr (NS > 1) {
+                        product(t_dp, sg + c * PANEL, NV, 0, 0, false, first);
+                        if (alive) product(t_dp, sg + c * PANEL, NV, 1, 0, false, first);
+                        if (alive) product(t_dp, sg + c * PANEL, NV, 1, 0, true, first);
+                    } else {
+                        product(t_dp, sg + c * PANEL, NV, 0, 0, false, first);
+                    }
+                }
+                if (!alive) break;
+                commit_elected(sfull);
+                if (!wait_warp(dsready, j & 1, abort_flag, (9 << 8) | 4)) { alive = false; break; }
+                const bool fresh = j == 0 || (flush && j % EVERY == 0);
+                if (fresh && j > 0 && !wait_warp(taken, (j / EVERY - 1) & 1, abort_flag, (9 << 8) | 7)) { alive = false; break; }
+                tc_fence_after();
+                for (int c = 0; c < ND && alive; ++c) {
+                    first = fresh;
+                    for (int p = NS - 1; p >= 0 && alive; --p) {
+                        uint32_t kp;
+                        panel(kp);
+                        if (!alive) break;
+                        const uint64_t kd = panel_desc(kp);
+                        const uint32_t d = t_dq + c * 64;
+                        if (p == 0) { mma_part_at<2>(d, t_s, t_lead, kd, id_o, first); first = false; }
+                        if (p <= 1) { mma_part_at<1>(d, t_s, t_lead, kd, id_o, first); first = false; }
+                        mma_part_at<0>(d, t_s, t_lead, kd, id_o, first);
+                        first = false;
+                        commit_elected(empty0 + 8 * (it % S::RING));
+                        ++it;
+                    }
+                }
+                if (alive && (j + 1 == n || (flush && (j + 1) % EVERY == 0))) commit_elected(done);
+            }
+        }
+    } else {
+        const int h = warp >> 2, quarter = warp & 3, r = quarter * 32 + lane;
+        const int t = q0 + r, b = bh / a.H;
+        const bool live = t < a.L;
+        const uint32_t lanes = (uint32_t)(quarter * 32) << 16;
+        const int64_t qrow = (int64_t)b * a.L + min(t, a.L - 1), row = (int64_t)bh * a.L + min(t, a.L - 1);
+        const uint2* bits = reinterpret_cast<const uint2*>(a.picks.bits + qrow * a.words) + h;       // 64 keys of every tile
+        const uint16_t* before = a.picks.before + qrow * a.words + h * 2;
+        const bool repeats = a.picks.repeats[b * a.n_tiles + qt] != 0;
+        const uint8_t* count = a.picks.count + qrow * a.K;
+        const float lse = a.lse[row], delta = a.delta[row];
+        float* prow = a.p + row * a.K;
+        float* dsrow = a.ds + row * a.K;
+        bool alive = true;
+        uint2 mine = live ? __ldg(bits) : make_uint2(0u, 0u);
+        uint32_t rank = __ldg(before);
+        uint32_t rounds = 0;                              // sums of dq taken out so far
+        bool bad = false;
+        auto take = [&] {
+            if (!wait_warp(done, rounds & 1, abort_flag, (9 << 8) | 6)) return false;
+            tc_fence_after();
+            flush_pieces<2, 2>(t_dq + lanes, h, ND * 4, live, rounds > 0, bad, [&](int c, int& cols) {
+                cols = max(0, min(16, a.Dqk - c * 16));
+                return static_cast<float*>(a.dq) + row * a.Dqk + c * 16;
+            });
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(taken);
+            ++rounds;
+            return true;
+        };
+        for (int j = 0; j < n; ++j) {
+            if (flush && j > 0 && j % EVERY == 0 && !take()) { alive = false; break; }
+            const uint2 cur = mine;
+            uint32_t at0 = rank;
+            if (j + 1 < n) {
+                mine = live ? __ldg(bits + (j + 1) * 2) : make_uint2(0u, 0u);
+                rank = __ldg(before + (j + 1) * 4);
+            }
+            if (!wait_warp(sfull, j & 1, abort_flag, (9 << 8) | 5)) { alive = false; break; }
+            tc_fence_after();
+#pragma unroll 1
+            for (int c = 0; c < 2; ++c) {
+                uint32_t sv[32], dv[32];
+                ld32(t_s + lanes + h * 64 + c * 32, sv);
+                ld32(t_dp + lanes + h * 64 + c * 32, dv);
+                ld_wait();
+                const uint32_t bit = c == 0 ? cur.x : cur.y;
+                float p[32];
+#pragma unroll
+                for (int i = 0; i < 32; ++i) p[i] = exp_fast(bit & (1u << i) ? fmaf(__uint_as_float(sv[i]), a.scale, -lse) : -INFINITY);
+                if (repeats) {                            // a key picked several times counts as often
+                    const uint8_t* cnt = count + at0;
+#pragma unroll
+                    for (int i = 0; i < 32; ++i)
+                        if (bit & (1u << i)) p[i] *= (float)*cnt++;
+                }
+                float* pp = prow + at0;
+                float* dp = dsrow + at0;
+                uint32_t at = 0;
+#pragma unroll
+                for (int i = 0; i < 32; ++i) {
+                    const uint32_t pick = bit & (1u << i);
+                    const float ds = p[i] * (__uint_as_float(dv[i]) - delta) * a.scale;
+                    store_if(pp + at, p[i], pick);
+                    p[i] = pick ? ds : 0.0f;
+                    store_if(dp + at, p[i], pick);
+                    at += (bit >> i) & 1u;
+                }
+                at0 += at;
+                store_parts32(t_s + lanes + h * 64 + c * 32, t_lead + lanes + h * 32 + c * 16, p);
+            }
+            st_wait();
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(dsready);
+        }
+        if (alive && flush) {
+            take();
+        } else if (alive && wait_warp(done, 0, abort_flag, (9 << 8) | 6)) {
+            tc_fence_after();
+#pragma unroll 1
+            for (int c = h; c < ND * 4; c += 2) {
+                float o[16];
+                tc_ld16(t_dq + lanes + c * 16, o);
+#pragma unroll
+                for (int i = 0; i < 16; ++i) bad |= !(fabsf(o[i]) <= 3.4e38f);
+                if (live && c * 16 < a.Dqk) store_row16(a.dq, row, c * 16, a.Dqk, a.tag, o);
+            }
+        }
+        if (live && bad) *a.flag = 1;
+    }
+    tc_fence_before();
+    __syncthreads();
+    if (warp == 9) {
+        tc_fence_after();
+        tc_dealloc(tmem, 512);
+    }
+}
+
+// Shared memory of the key pass: a ring of stages, each 32 queries of every panel of q and dO.
+template <int NS, int ND, int NV> struct KPassShape {
+    static constexpr int SUB = 32 * 128;                   // 32 rows of a 64-column panel
+    static constexpr int PANELS = NS * (ND + NV), STAGE = PANELS * SUB;
+    static constexpr int STAGES = (14 * PANEL) / STAGE < 8 ? (14 * PANEL) / STAGE : 8;
+    static constexpr int BAR_OFF = STAGES * STAGE;
+    static constexpr int BYTES = BAR_OFF + 256 + 1024;
+};
+
+// Key pass: one CTA per 128 keys of a head, over the queries from the keys' own tile on, 32 at a time.  A thread owns a
+// key; for a warp's 32 keys the bits of a query are one word, and the ranks of the keys it picked are consecutive, so
+// that what the query pass left is read in short contiguous pieces: p by two warpgroups, dS by two others, chunk by chunk
+// in turn.  Each writes its 32 columns as an A operand (a buffer of 48 columns of its own), and the tensor core adds
+// dv += P^T dO, dk += dS^T q.
+constexpr int KEY_THREADS = 18 * 32;       // four producing warpgroups, TMA warp, MMA warp
+
+template <int NS, int ND, int NV>
+__global__ void __launch_bounds__(KEY_THREADS, 1)
+attn_bwd_key_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmG, const BwdArgs a) {
+    using S = KPassShape<NS, ND, NV>;
+    extern __shared__ uint8_t smem_raw[];
+    uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+    const uint32_t ring = smem_u32(smem);
+    uint64_t* bars = reinterpret_cast<uint64_t*>(smem + S::BAR_OFF);
+    const uint32_t full0 = smem_u32(bars), empty0 = smem_u32(bars + S::STAGES);
+    const uint32_t ready0 = smem_u32(bars + 2 * S::STAGES), free0 = ready0 + 32;        // [operand][buffer]
+    const uint32_t done = ready0 + 64, taken = ready0 + 72;
+    constexpr int EVERY = 8;                               // fp32 gradients: chunks between two flushes
+    const bool flush = NS > 1 && a.tag == CINN_F32;
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * S::STAGES + 10);
+    volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    int kt, bh;
+    tile_of_block(a.n_tiles, a.BH, a.group, kt, bh);
+    kt = a.n_tiles - 1 - kt;                               // the first keys have the most queries
+    const int k0 = kt * T, n = (a.n_tiles - kt) * 4;       // chunks of 32 queries
+    if (tid == 0) {
+        *abort_flag = 0;
+        for (int i = 0; i < S::STAGES; ++i) { mbar_init(full0 + 8 * i, 1); mbar_init(empty0 + 8 * i, 1); }
+        for (int i = 0; i < 4; ++i) { mbar_init(ready0 + 8 * i, 4); mbar_init(free0 + 8 * i, 1); }
+        mbar_init(done, 1); mbar_init(taken, 16);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == 17) tc_alloc(smem_u32(tmem_slot), 512);
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    // columns: dk | dv | [operand p, dS][buffer] 48
+    const uint32_t tmem = *tmem_slot, t_dk = tmem, t_dv = tmem + ND * 64, t_a = tmem + 320;
+
+    if (warp == 16) {
+        if (lane == 0) {
+            bool alive = true;
+            for (int i = 0; i < n && alive; ++i) {
+                const uint32_t s = i % S::STAGES, ph = (i / S::STAGES) & 1;
+                if (!mbar_wait_bounded(empty0 + 8 * s, ph ^ 1, abort_flag, (10 << 8) | 1, &g_attn_status)) { alive = false; break; }
+                mbar_expect_tx(full0 + 8 * s, S::STAGE);
+                uint32_t dst = ring + s * S::STAGE;
+                const int y = k0 + i * 32;
+                for (int p = 0; p < NS; ++p) {
+                    for (int c = 0; c < NV; ++c, dst += S::SUB) tma_load_3d(&tmG, full0 + 8 * s, dst, c * 64, y, p * a.BH + bh);
+                    for (int c = 0; c < ND; ++c, dst += S::SUB) tma_load_3d(&tmQ, full0 + 8 * s, dst, c * 64, y, p * a.BH + bh);
+                }
+            }
+            if (!alive) {                                 // abandoned: let the copies in flight land
+                const long long t0 = clock64();
+                while (clock64() - t0 < 2000000LL) { }
+            }
+        }
+    } else if (warp == 17) {
+        constexpr uint32_t id = make_idesc_f16(true, T, 64, false, true);
+        bool alive = true;
+        for (int i = 0; i < n && alive; ++i) {
+            const uint32_t s = i % S::STAGES, buf = i & 1;
+            if (!wait_warp(full0 + 8 * s, (i / S::STAGES) & 1, abort_flag, (10 << 8) | 2)) { alive = false; break; }
+            const uint32_t stage = ring + s * S::STAGE;
+            const bool fresh = i == 0 || (flush && i % EVERY == 0);
+            if (fresh && i > 0 && !wait_warp(taken, (i / EVERY - 1) & 1, abort_flag, (10 << 8) | 6)) { alive = false; break; }
+#pragma unroll
+            for (int op = 0; op < 2; ++op) {               // dv from p and dO, dk from dS and q
+                if (alive && !wait_warp(ready0 + 8 * (op * 2 + buf), (i >> 1) & 1, abort_flag, (10 << 8) | 3)) alive = false;
+                if (!alive) break;
+                tc_fence_after();
+                const uint32_t at = t_a + (op * 2 + buf) * 48;
+                for (int c = 0; c < (op ? ND : NV); ++c) {
+                    const uint32_t d = (op ? t_dk : t_dv) + c * 64;
+                    bool first = fresh;
+#pragma unroll
+                    for (int p = NS - 1; p >= 0; --p) {
+                        const uint64_t bd = panel_desc(stage + (p * (ND + NV) + (op ? NV : 0) + c) * S::SUB);
+                        if (p == 0) { mma_part_at<2, 2>(d, at, at + 32, bd, id, first); first = false; }
+                        if (p <= 1) { mma_part_at<1, 2>(d, at, at + 32, bd, id, first); first = false; }
+                        mma_part_at<0, 2>(d, at, at + 32, bd, id, first);
+                        first = false;
+                    }
+                }
+                commit_elected(free0 + 8 * (op * 2 + buf));
+            }
+            if (alive) commit_elected(empty0 + 8 * s);
+            if (alive && (i + 1 == n || (flush && (i + 1) % EVERY == 0))) commit_elected(done);
+        }
+    } else {
+        const int op = (warp >> 2) & 1, buf = warp >> 3, quarter = warp & 3, r = quarter * 32 + lane;
+        const int s = k0 + r, b = bh / a.H;
+        const uint32_t lanes = (uint32_t)(quarter * 32) << 16;
+        const int word = (k0 >> 5) + quarter;
+        const uint32_t* bits = a.picks.bits + ((int64_t)b * a.L) * a.words + word;
+        const uint16_t* before = a.picks.before + ((int64_t)b * a.L) * a.words + word;
+        const float* src = (op ? a.ds : a.p) + (int64_t)bh * a.L * a.K;
+        const uint32_t below = (1u << lane) - 1u;
+        bool alive = true;
+        // this lane's query of the next chunk: its word for the warp's keys, and where that word's picks begin
+        auto fetch = [&](int i, uint32_t& w, uint32_t& base) {
+            const int t = k0 + i * 32 + lane, tc = min(t, a.L - 1);
+            w = t < a.L ? __ldg(bits + (int64_t)tc * a.words) : 0u;
+            base = (uint32_t)tc * a.K + __ldg(before + (int64_t)tc * a.words);
+        };
+        const int64_t row = (int64_t)bh * a.L + min(s, a.L - 1);
+        uint32_t rounds = 0;                               // sums taken out so far
+        bool bad = false;
+        auto take = [&] {
+            if (!wait_warp(done, rounds & 1, abort_flag, (10 << 8) | 5)) return false;
+            tc_fence_after();
+            flush_pieces<4, 1>(t_dk + lanes, warp >> 2, (ND + NV) * 4, s < a.L, rounds > 0, bad, [&](int c, int& cols) {      // dk, then dv
+                const bool is_v = c >= ND * 4;
+                const int col = (is_v ? c - ND * 4 : c) * 16, width = is_v ? a.Dv : a.Dqk;
+                cols = max(0, min(16, width - col));
+                return static_cast<float*>(is_v ? a.dv : a.dk) + row * width + col;
+            });
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(taken);
+            ++rounds;
+            return true;
+        };
+        uint32_t w_next, base_next;
+        fetch(buf, w_next, base_next);
+        for (int i = buf; i < n; i += 2) {
+            if (flush && i >= EVERY && i % EVERY == buf && !take()) { alive = false; break; }
+            const uint32_t w = w_next, base = base_next;
+            if (i + 2 < n) fetch(i + 2, w_next, base_next);
+            float v[32];
+#pragma unroll
+            for (int u = 0; u < 32; ++u) {
+                const uint32_t wu = __shfl_sync(0xffffffffu, w, u), at = __shfl_sync(0xffffffffu, base, u) + __popc(wu & below);
+                const float x = __ldg(src + min(at, (uint32_t)a.L * a.K - 1u));       // a lane that was not picked reads its neighbour's
+                v[u] = wu >> lane & 1u ? x : 0.0f;
+            }
+            if (!wait_warp(free0 + 8 * (op * 2 + buf), ((i >> 1) & 1) ^ 1, abort_flag, (10 << 8) | 4)) { alive = false; break; }
+            tc_fence_after();
+            const uint32_t at = t_a + lanes + (op * 2 + buf) * 48;
+            store_parts32(at, at + 32, v);
+            st_wait();
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(ready0 + 8 * (op * 2 + buf));
+        }
+        if (alive && flush) {
+            take();
+        } else if (alive && wait_warp(done, 0, abort_flag, (10 << 8) | 5)) {
+            tc_fence_after();
+#pragma unroll 1
+            for (int c = warp >> 2; c < (ND + NV) * 4; c += 4) {       // 16-column pieces of dk, then dv
+                float o[16];
+                tc_ld16(t_dk + lanes + c * 16, o);
+#pragma unroll
+                for (int i = 0; i < 16; ++i) bad |= !(fabsf(o[i]) <= 3.4e38f);
+                const bool is_v = c >= ND * 4;
+                const int col = (is_v ? c - ND * 4 : c) * 16, width = is_v ? a.Dv : a.Dqk;
+                if (s < a.L && col < width) store_row16(is_v ? a.dv : a.dk, row, col, width, a.tag, o);
+            }
+        }
+        if (s < a.L && bad) *a.flag = 1;
+    }
+    tc_fence_before();
+    __syncthreads();
+    if (warp == 17) {
+        tc_fence_after();
+        tc_dealloc(tmem, 512);
+    }
+}
+
+// ---------------------------------------------------------------------------
+// host side
+// ---------------------------------------------------------------------------
+static inline int64_t up(int64_t v, int64_t a) { return (v + a - 1) / a * a; }
+
+// One call's shapes and where its scratch lies.
+struct Plan {
+    int64_t B, H, L, K, Dqk, Dv, BH, Lp;
+    int dtype, ns, nd, dp, nv;             // parts; panels, padded width of q and k; 64-column panels of v
+    bool direct;                           // bf16 rows TMA can read as they are: no copies
+    int64_t bits_off, rank_off, count_off, before_off, flag_off, q_off, k_off, v_off, g_off, delta_off, p_off, ds_off, grads_off, bytes;
+};
+
+static Plan make_plan(int64_t B, int64_t H, int64_t L, int64_t K, int64_t Dqk, int64_t Dv, int dtype, bool backward) {
+    Plan p{};
+    p.B = B; p.H = H; p.L = L; p.K = K; p.Dqk = Dqk; p.Dv = Dv; p.BH = B * H; p.Lp = up(L, T);
+    p.dtype = dtype;
+    p.ns = dtype == CINN_BF16 ? 1 : PARTS;
+    p.nd = (int)((Dqk + 63) / 64); p.dp = p.nd * 64; p.nv = (int)((Dv + 63) / 64);
+    p.direct = dtype == CINN_BF16 && Dqk % 8 == 0 && Dv % 8 == 0;
+    int64_t off = 0;
+    auto take = [&](int64_t bytes) { const int64_t o = off; off += up(bytes, 256); return o; };
+    p.flag_off = take(4 * (1 + B * (p.Lp / T)));          // the flag, then the tiles' `repeats`
+    p.bits_off = take(B * L * p.Lp / 8);
+    p.rank_off = take(B * L * K * 2);
+    p.count_off = take(B * L * K);
+    p.before_off = take(B * L * p.Lp / 32 * 2);
+    if (backward) {
+        p.delta_off = take(p.BH * L * 4);
+        p.p_off = take(p.BH * L * K * 4);
+        p.ds_off = take(p.BH * L * K * 4);
+        if (!p.direct) p.g_off = take(p.ns * p.BH * L * p.nv * 64 * 2);
+        // fp32 gradients for the fallback, where the caller's are not
+        if (dtype != CINN_F32) p.grads_off = take(p.BH * L * (2 * Dqk + Dv) * 4);
+    }
+    if (!p.direct) {
+        p.q_off = take(p.ns * p.BH * L * p.dp * 2);
+        p.k_off = take(p.ns * p.BH * L * p.dp * 2);
+        p.v_off = take(p.ns * p.BH * L * p.nv * 64 * 2);
+    }
+    p.bytes = off;
+    return p;
+}
+
+// Whether the dense tiles are worth it: their time (the causal half of the tiles is visited, a constant number of cycles
+// each that grows with the widths) against the gathers' (K rows of Dqk + Dv elements per query).  The constants are fitted
+// to measurements over L = 500 ... 4096, K = 32 ... 128, widths 64 ... 192; at 2 x 8 x 4096 queries the line lies between
+// K = 32 (gathers 0.21 ms, tiles 0.29 ms forward in bf16) and K = 128 (0.49 ms against 0.40 ms in fp32).
+static std::atomic<int> g_mode{-1};         // -1: by the estimate; 0 / 1: never / wherever the tiles can (tests, measurements)
+int set_mode(int mode) { return g_mode.exchange(mode); }
+
+static bool dense_pays(const Plan& p, bool backward) {
+    const int mode = g_mode.load(std::memory_order_relaxed);
+    if (mode >= 0) return mode != 0;
+    const double tiles = 0.5 * (double)(p.Lp / T) * (double)(p.Lp / T + 1) * (double)p.BH, q_tiles = (double)(p.Lp / T) * (double)p.BH;
+    const bool parts = p.ns > 1, wide = p.dtype == CINN_F32;
+    const double queries = (double)p.BH * p.L, row = (double)(p.Dqk + p.Dv), widths = p.dp + 64.0 * p.nv;
+    const double gathered = queries * p.K * row * (wide ? 4 : 2), split = parts ? queries * (row + p.Dqk) * (wide ? 10 : 8) / 6.2e6 : 0.0;
+    const double picks = 15.0 + 5.5e-6 * p.B * p.L * p.K;
+    double cycles, gather_us;
+    if (!backward) {
+        cycles = tiles * p.nv * (parts ? 8800.0 + 48.0 * p.dp : 7500.0 + 8.0 * p.dp) + q_tiles * p.nv * (6000.0 + 100.0 * p.K);
+        gather_us = 8.0 + gathered / (wide ? 9.5e6 : 5.3e6);
+    } else {
+        cycles = tiles * (parts ? 24000.0 + 190.0 * widths : 14000.0 + 66.0 * widths) + q_tiles * 20000.0;
+        gather_us = 30.0 + gathered / (wide ? 3.7e6 : 2.0e6);
+    }
+    return (picks + split + (backward ? 20.0 : 0.0) + cycles / (148.0 * 1900.0)) < 0.9 * gather_us;
+}
+
+static bool supported(int64_t B, int64_t H, int64_t L, int64_t K, int64_t Dqk, int64_t Dv) {
+    return B * H * L > 0 && K >= 1 && K <= MAX_SLOTS && Dqk <= 192 && Dv <= 128 && L <= 12000 && B * H <= 65535 && B * H * L < (1LL << 31) / 4;
+}
+
+static Picks picks_of(const Plan& p, const uint8_t* ws) {
+    return {reinterpret_cast<const uint32_t*>(ws + p.bits_off), reinterpret_cast<const uint16_t*>(ws + p.rank_off), ws + p.count_off,
+            reinterpret_cast<const uint16_t*>(ws + p.before_off), reinterpret_cast<const int*>(ws + p.flag_off) + 1};
+}
+
+// clears the flag and finds out what was picked
+static int make_picks(const Plan& p, const int64_t* idx, uint8_t* ws, cudaStream_t st) {
+    CINN_CHECK_CUDA(cudaMemsetAsync(ws + p.flag_off, 0, 4 * (1 + p.B * (p.Lp / T)), st));
+    const int words = (int)(p.Lp / 32), warps = 4;
+    const size_t smem = (size_t)warps * (2 * words + p.K) * 4;
+    const int64_t rows = p.B * p.L;
+    const int64_t want = (rows + warps - 1) / warps, cap = (int64_t)sm_count() * 16;
+    const unsigned grid = (unsigned)(want < cap ? want : cap);
+    int* flag = reinterpret_cast<int*>(ws + p.flag_off);
+    picks_kernel<<<grid, 32 * warps, smem, st>>>(idx, reinterpret_cast<uint32_t*>(ws + p.bits_off),
+                                                 reinterpret_cast<uint16_t*>(ws + p.rank_off), ws + p.count_off,
+                                                 reinterpret_cast<uint16_t*>(ws + p.before_off), flag + 1, flag, rows,
+                                                 (int)p.L, words, (int)p.K, warps);
+    CINN_CHECK_LAUNCH();
+    return CINN_OK;
+}
+
+static int split_parts(const SplitJobs& jobs, int dtype, cudaStream_t st) {
+    const unsigned grid = (unsigned)sm_count() * 16;
+    switch (dtype) {
+        case CINN_F32: split_parts_kernel<float, 3><<<grid, 256, 0, st>>>(jobs); break;
+        case CINN_F16: split_parts_kernel<__half, 3><<<grid, 256, 0, st>>>(jobs); break;
+        default: split_parts_kernel<__nv_bfloat16, 1><<<grid, 256, 0, st>>>(jobs); break;
+    }
+    CINN_CHECK_LAUNCH();
+    return CINN_OK;
+}
+
+// tensor maps of q, k, v (parts, heads, L, width), from the inputs themselves or from their parts
+static int operand_map(const Plan& p, CUtensorMap* m, const void* direct, const uint8_t* parts, int64_t d, int64_t padded,
+                       uint32_t box_rows = T) {
+    if (p.direct)
+        return encode_map_3d(m, direct, (uint64_t)d, (uint64_t)p.L, (uint64_t)p.BH, (uint64_t)d * 2, box_rows,
+                             CU_TENSOR_MAP_DATA_TYPE_BFLOAT16);
+    return encode_map_3d(m, parts, (uint64_t)padded, (uint64_t)p.L, (uint64_t)(p.ns * p.BH), (uint64_t)padded * 2, box_rows,
+                         CU_TENSOR_MAP_DATA_TYPE_BFLOAT16);
+}
+
+static int head_group(const Plan& p) {
+    const int64_t tiles = p.Lp / T, want = (3 * sm_count() + tiles - 1) / tiles;
+    return (int)(want < p.BH ? want : p.BH);
+}
+
+template <int NS, int ND>
+static int launch_fwd(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const FwdArgs& a, const Plan& p, cudaStream_t st) {
+    auto kern = attn_fwd_kernel<NS, ND>;
+    CINN_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, FwdShape<NS, ND>::BYTES));
+    dim3 grid((unsigned)(p.Lp / T * p.BH), 1, (unsigned)p.nv);
+    kern<<<grid, FWD_THREADS, FwdShape<NS, ND>::BYTES, st>>>(tq, tk, tv, a);
+    CINN_CHECK_LAUNCH();
+    return CINN_OK;
+}
+
+int64_t forward_workspace_bytes(int64_t B, int64_t H, int64_t L, int64_t K, int64_t Dqk, int64_t Dv, int dtype) {
+    if (!supported(B, H, L, K, Dqk, Dv)) return 0;
+    const Plan p = make_plan(B, H, L, K, Dqk, Dv, dtype, false);
+    return dense_pays(p, false) ? p.bytes : 0;
+}
+
+// Returns the flag's device address in *flag: the gather kernel behind it runs when it is set.
+int forward(const void* q, const void* k, const void* v, int dtype, const int64_t* idx, float* out, void* out_cast, float* lse,
+            float* attn, int64_t B, int64_t H, int64_t L, int64_t K, int64_t Dqk, int64_t Dv, float scale, uint8_t* ws,
+            const int** flag, cudaStream_t st) {
+    const Plan p = make_plan(B, H, L, K, Dqk, Dv, dtype, false);
+    auto al16 = [](const void* x) { return (reinterpret_cast<uintptr_t>(x) & 15) == 0; };
+    CINN_CHECK_ARG(!p.direct || (al16(q) && al16(k) && al16(v)), "sparse_attention: q, k and v must be 16-byte aligned");
+    *flag = reinterpret_cast<const int*>(ws + p.flag_off);
+    int rc = make_picks(p, idx, ws, st);
+    if (rc) return rc;
+    if (!p.direct) {
+        SplitJobs jobs{};
+        jobs.job[0] = {q, reinterpret_cast<uint16_t*>(ws + p.q_off), p.BH * L, (int)Dqk, p.dp};
+        jobs.job[1] = {k, reinterpret_cast<uint16_t*>(ws + p.k_off), p.BH * L, (int)Dqk, p.dp};
+        jobs.job[2] = {v, reinterpret_cast<uint16_t*>(ws + p.v_off), p.BH * L, (int)Dv, p.nv * 64};
+        jobs.n = 3;
+        rc = split_parts(jobs, dtype, st);
+        if (rc) return rc;
+    }
+    CUtensorMap tq, tk, tv;
+    if ((rc = operand_map(p, &tq, q, ws + p.q_off, Dqk, p.dp))) return rc;
+    if ((rc = operand_map(p, &tk, k, ws + p.k_off, Dqk, p.dp))) return rc;
+    if ((rc = operand_map(p, &tv, v, ws + p.v_off, Dv, p.nv * 64))) return rc;
+    FwdArgs a{};
+    a.picks = picks_of(p, ws);
+    a.out = out; a.out_cast = out_cast; a.lse = lse; a.attn = attn; a.flag = reinterpret_cast<int*>(ws + p.flag_off);
+    a.H = (int)H; a.L = (int)L; a.words = (int)(p.Lp / 32); a.K = (int)K; a.Dv = (int)Dv; a.BH = (int)p.BH; a.scale = scale;
+    a.n_tiles = (int)(p.Lp / T); a.group = head_group(p);
+    a.out_cast_tag = dtype;
+    if (p.ns == 1) {
+        switch (p.nd) {
+            case 1: return launch_fwd<1, 1>(tq, tk, tv, a, p, st);
+            case 2: return launch_fwd<1, 2>(tq, tk, tv, a, p, st);
+            default: return launch_fwd<1, 3>(tq, tk, tv, a, p, st);
+        }
+    }
+    switch (p.nd) {
+        case 1: return launch_fwd<3, 1>(tq, tk, tv, a, p, st);
+        case 2: return launch_fwd<3, 2>(tq, tk, tv, a, p, st);
+        default: return launch_fwd<3, 3>(tq, tk, tv, a, p, st);
+    }
+}
+
+template <int NS, int ND, int NV>
+static int launch_bwd(const CUtensorMap (&m)[6], const BwdArgs& a, const Plan& p, cudaStream_t st) {
+    auto qk = attn_bwd_query_kernel<NS, ND, NV>;
+    auto kk = attn_bwd_key_kernel<NS, ND, NV>;
+    const unsigned grid = (unsigned)(p.Lp / T * p.BH);
+    CINN_CHECK_CUDA(cudaFuncSetAttribute(qk, cudaFuncAttributeMaxDynamicSharedMemorySize, QPassShape<NS, ND, NV>::BYTES));
+    CINN_CHECK_CUDA(cudaFuncSetAttribute(kk, cudaFuncAttributeMaxDynamicSharedMemorySize, KPassShape<NS, ND, NV>::BYTES));
+    qk<<<grid, FWD_THREADS, QPassShape<NS, ND, NV>::BYTES, st>>>(m[0], m[1], m[2], m[3], a);
+    CINN_CHECK_LAUNCH();
+    kk<<<grid, KEY_THREADS, KPassShape<NS, ND, NV>::BYTES, st>>>(m[4], m[5], a);
+    CINN_CHECK_LAUNCH();
+    return CINN_OK;
+}
+
+int64_t backward_workspace_bytes(int64_t B, int64_t H, int64_t L, int64_t K, int64_t Dqk, int64_t Dv, int dtype) {
+    if (!supported(B, H, L, K, Dqk, Dv)) return 0;
+    const Plan p = make_plan(B, H, L, K, Dqk, Dv, dtype, true);
+    return dense_pays(p, true) ? p.bytes : 0;
+}
+
+// Gradients in `dtype` (dq, dk, dv written, not added to).  *flag as in forward; *fallback: fp32 buffers (dq | dk | dv) the
+// gather kernel may use when it has to run.
+int backward(const void* d_out, const float* out, const float* lse, const void* q, const void* k, const void* v, int dtype,
+             const int64_t* idx, void* dq, void* dk, void* dv, int64_t B, int64_t H, int64_t L, int64_t K, int64_t Dqk, int64_t Dv,
+             float scale, uint8_t* ws, const int** flag, float** fallback, cudaStream_t st) {
+    const Plan p = make_plan(B, H, L, K, Dqk, Dv, dtype, true);
+    *flag = reinterpret_cast<const int*>(ws + p.flag_off);
+    *fallback = dtype != CINN_F32 ? reinterpret_cast<float*>(ws + p.grads_off) : nullptr;
+    int rc = make_picks(p, idx, ws, st);
+    if (rc) return rc;
+    if (!p.direct) {
+        SplitJobs jobs{};
+        jobs.job[0] = {q, reinterpret_cast<uint16_t*>(ws + p.q_off), p.BH * L, (int)Dqk, p.dp};
+        jobs.job[1] = {k, reinterpret_cast<uint16_t*>(ws + p.k_off), p.BH * L, (int)Dqk, p.dp};
+        jobs.job[2] = {v, reinterpret_cast<uint16_t*>(ws + p.v_off), p.BH * L, (int)Dv, p.nv * 64};
+        jobs.job[3] = {d_out, reinterpret_cast<uint16_t*>(ws + p.g_off), p.BH * L, (int)Dv, p.nv * 64};
+        jobs.n = 4;
+        rc = split_parts(jobs, dtype, st);
+        if (rc) return rc;
+    }
+    float* delta = reinterpret_cast<float*>(ws + p.delta_off);
+    const int64_t rows = p.BH * L, want = (rows + 7) / 8, cap = (int64_t)sm_count() * 32;
+    const unsigned dgrid = (unsigned)(want < cap ? want : cap);
+    switch (dtype) {
+        case CINN_F32: delta_kernel<float><<<dgrid, 256, 0, st>>>((const float*)d_out, out, delta, rows, (int)Dv); break;
+        case CINN_F16: delta_kernel<__half><<<dgrid, 256, 0, st>>>((const __half*)d_out, out, delta, rows, (int)Dv); break;
+        default: delta_kernel<__nv_bfloat16><<<dgrid, 256, 0, st>>>((const __nv_bfloat16*)d_out, out, delta, rows, (int)Dv); break;
+    }
+    CINN_CHECK_LAUNCH();
+    CUtensorMap m[6];                                      // q, k, v, dO in boxes of 128 rows; q, dO in boxes of 32
+    if ((rc = operand_map(p, &m[0], q, ws + p.q_off, Dqk, p.dp))) return rc;
+    if ((rc = operand_map(p, &m[1], k, ws + p.k_off, Dqk, p.dp))) return rc;
+    if ((rc = operand_map(p, &m[2], v, ws + p.v_off, Dv, p.nv * 64))) return rc;
+    if ((rc = operand_map(p, &m[3], d_out, ws + p.g_off, Dv, p.nv * 64))) return rc;
+    if ((rc = operand_map(p, &m[4], q, ws + p.q_off, Dqk, p.dp, 32))) return rc;
+    if ((rc = operand_map(p, &m[5], d_out, ws + p.g_off, Dv, p.nv * 64, 32))) return rc;
+    BwdArgs a{};
+    a.picks = picks_of(p, ws);
+    a.lse = lse; a.delta = delta; a.p = reinterpret_cast<float*>(ws + p.p_off); a.ds = reinterpret_cast<float*>(ws + p.ds_off);
+    a.dq = dq; a.dk = dk; a.dv = dv; a.flag = reinterpret_cast<int*>(ws + p.flag_off);
+    a.H = (int)H; a.L = (int)L; a.words = (int)(p.Lp / 32); a.K = (int)K; a.Dqk = (int)Dqk; a.Dv = (int)Dv; a.BH = (int)p.BH;
+    a.n_tiles = (int)(p.Lp / T); a.group = head_group(p); a.tag = dtype; a.scale = scale;
+#define CINN_ATB(NS, ND, NV) if (p.ns == NS && p.nd == ND && p.nv == NV) return launch_bwd<NS, ND, NV>(m, a, p, st)
+    CINN_ATB(1, 1, 1); CINN_ATB(1, 2, 1); CINN_ATB(1, 3, 1); CINN_ATB(1, 1, 2); CINN_ATB(1, 2, 2); CINN_ATB(1, 3, 2);
+    CINN_ATB(3, 1, 1); CINN_ATB(3, 2, 1); CINN_ATB(3, 3, 1); CINN_ATB(3, 1, 2); CINN_ATB(3, 2, 2); CINN_ATB(3, 3, 2);
+#undef CINN_ATB
+    set_error("sparse_attention: no tile kernel for %d + %d column panels", p.nd, p.nv);
+    return CINN_ERR_INVALID;
+}
+
+}  // namespace atc
+
+int read_attn_status(int* out, int reset) {
+    int v = 0;
+    CINN_CHECK_CUDA(cudaMemcpyFromSymbol(&v, atc::g_attn_status, sizeof(int)));
+    if (reset && v != 0) {
+        int z = 0;
+        CINN_CHECK_CUDA(cudaMemcpyToSymbol(atc::g_attn_status, &z, sizeof(int)));
+    }
+    *out = v;
+    return CINN_OK;
+}
+
+}  // namespace cinn

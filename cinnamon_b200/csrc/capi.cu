@@ -56,12 +56,17 @@ int fp8_grouped_gemm_dgrad(const void* dY, const float* sdY, const void* W, cons
                            cudaStream_t st);
 int gather_rows(const void* q, const float* s, const int64_t* idx, void* out_q, float* out_s, int64_t n_out, int64_t n_src,
                 int64_t d, int64_t ns, cudaStream_t st);
-int sparse_attn_fwd(const void* q, const void* k, const void* v, int dtype, const int64_t* idx, float* out, float* lse,
-                    float* attn_w, int64_t B, int64_t H, int64_t L, int64_t K, int64_t Dqk, int64_t Dv, float scale,
-                    cudaStream_t st);
+namespace atc { int set_mode(int mode); }
+int64_t sparse_attn_workspace_bytes(int64_t B, int64_t H, int64_t L, int64_t K, int64_t Dqk, int64_t Dv, int dtype, int backward);
+int sparse_attn_fwd(const void* q, const void* k, const void* v, int dtype, const int64_t* idx, float* out, void* out_cast,
+                    float* lse, float* attn_w, int64_t B, int64_t H, int64_t L, int64_t K, int64_t Dqk, int64_t Dv, float scale,
+                    void* workspace, int64_t workspace_bytes, cudaStream_t st);
 int sparse_attn_bwd(const void* d_out, int grad_dtype, const float* out, const float* lse, const void* q, const void* k,
                     const void* v, int dtype, const int64_t* idx, float* dq, float* dk, float* dv, int64_t B, int64_t H,
-                    int64_t L, int64_t K, int64_t Dqk, int64_t Dv, float scale, cudaStream_t st);
+                    int64_t L, int64_t K, int64_t Dqk, int64_t Dv, float scale, const int* run_if, cudaStream_t st);
+int sparse_attn_bwd_tiles(const void* d_out, const float* out, const float* lse, const void* q, const void* k, const void* v, int dtype,
+                          const int64_t* idx, void* dq, void* dk, void* dv, int64_t B, int64_t H, int64_t L, int64_t K, int64_t Dqk,
+                          int64_t Dv, float scale, void* workspace, int64_t workspace_bytes, cudaStream_t st);
 int lightning_indexer(const void* q, const void* k, const void* w, int dtype, void* out, int64_t B, int64_t Lq, int64_t Lk,
                       int64_t H, int64_t d, const int64_t* q_strides, const int64_t* k_strides, const int64_t* w_strides,
                       cudaStream_t st);
@@ -237,7 +242,22 @@ int cinn_gather_rows(const void* q, const float* scales, const int64_t* idx, voi
 int cinn_sparse_attn_fwd(const void* q, const void* k, const void* v, int dtype, const int64_t* idx, float* out, float* lse,
                          float* attn_weights, int64_t B, int64_t H, int64_t L, int64_t K, int64_t d_qk, int64_t d_v,
                          float scale, void* stream) {
-    return cinn::sparse_attn_fwd(q, k, v, dtype, idx, out, lse, attn_weights, B, H, L, K, d_qk, d_v, scale, (cudaStream_t)stream);
+    return cinn::sparse_attn_fwd(q, k, v, dtype, idx, out, nullptr, lse, attn_weights, B, H, L, K, d_qk, d_v, scale, nullptr, 0,
+                                 (cudaStream_t)stream);
+}
+
+int cinn_set_sparse_attn_dense(int mode) { return cinn::atc::set_mode(mode < 0 ? -1 : mode); }
+
+int64_t cinn_sparse_attn_workspace_bytes(int64_t B, int64_t H, int64_t L, int64_t K, int64_t d_qk, int64_t d_v, int dtype,
+                                         int backward) {
+    return cinn::sparse_attn_workspace_bytes(B, H, L, K, d_qk, d_v, dtype, backward);
+}
+
+int cinn_sparse_attn_fwd_ws(const void* q, const void* k, const void* v, int dtype, const int64_t* idx, float* out,
+                            void* out_cast, float* lse, float* attn_weights, int64_t B, int64_t H, int64_t L, int64_t K,
+                            int64_t d_qk, int64_t d_v, float scale, void* workspace, int64_t workspace_bytes, void* stream) {
+    return cinn::sparse_attn_fwd(q, k, v, dtype, idx, out, out_cast, lse, attn_weights, B, H, L, K, d_qk, d_v, scale, workspace,
+                                 workspace_bytes, (cudaStream_t)stream);
 }
 
 int cinn_sparse_attn_bwd(const void* grad_out, int grad_dtype, const float* out, const float* lse, const void* q,
@@ -245,7 +265,14 @@ int cinn_sparse_attn_bwd(const void* grad_out, int grad_dtype, const float* out,
                          float* grad_v, int64_t B, int64_t H, int64_t L, int64_t K, int64_t d_qk, int64_t d_v, float scale,
                          void* stream) {
     return cinn::sparse_attn_bwd(grad_out, grad_dtype, out, lse, q, k, v, dtype, idx, grad_q, grad_k, grad_v, B, H, L, K, d_qk,
-                                 d_v, scale, (cudaStream_t)stream);
+                                 d_v, scale, nullptr, (cudaStream_t)stream);
+}
+
+int cinn_sparse_attn_bwd_ws(const void* grad_out, const float* out, const float* lse, const void* q, const void* k, const void* v,
+                            int dtype, const int64_t* idx, void* grad_q, void* grad_k, void* grad_v, int64_t B, int64_t H, int64_t L,
+                            int64_t K, int64_t d_qk, int64_t d_v, float scale, void* workspace, int64_t workspace_bytes, void* stream) {
+    return cinn::sparse_attn_bwd_tiles(grad_out, out, lse, q, k, v, dtype, idx, grad_q, grad_k, grad_v, B, H, L, K, d_qk, d_v, scale,
+                                       workspace, workspace_bytes, (cudaStream_t)stream);
 }
 
 int cinn_lightning_indexer(const void* q, const void* k, const void* w, int dtype, void* out, int64_t B, int64_t Lq,

@@ -594,6 +594,30 @@ int encode_map_2d(CUtensorMap* map, const void* base, uint64_t inner, uint64_t r
     return CINN_OK;
 }
 
+// 3-D map of 2-byte elements: `planes` matrices of (rows, inner), boxes of 64 columns x box_rows of one matrix, 128-byte
+// swizzle; rows past a matrix's end read as zeros instead of its neighbour's
+int encode_map_3d(CUtensorMap* map, const void* base, uint64_t inner, uint64_t rows, uint64_t planes, uint64_t pitch_bytes,
+                  uint32_t box_rows, CUtensorMapDataType dtype) {
+    EncodeFn enc = get_encode();
+    if (!enc) { set_error("cuTensorMapEncodeTiled is not available from the CUDA driver"); return CINN_ERR_CUDA; }
+    cuuint64_t dims[3] = {inner, rows, planes};
+    cuuint64_t strides[2] = {pitch_bytes, pitch_bytes * rows};
+    cuuint32_t box[3] = {64, box_rows, 1};
+    cuuint32_t estr[3] = {1, 1, 1};
+    auto go = [&] {
+        return enc(map, dtype, 3, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                   CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    };
+    CUresult r = go();
+    if (r == CUDA_ERROR_INVALID_CONTEXT || r == CUDA_ERROR_NOT_INITIALIZED) { cudaFree(nullptr); r = go(); }
+    if (r != CUDA_SUCCESS) {
+        set_error("cuTensorMapEncodeTiled failed with CUresult %d (base %p inner %llu rows %llu planes %llu)", (int)r, base,
+                  (unsigned long long)inner, (unsigned long long)rows, (unsigned long long)planes);
+        return CINN_ERR_CUDA;
+    }
+    return CINN_OK;
+}
+
 // GEMM operands and outputs: 128-byte swizzle; `pitch` in BYTES
 static int make_map(CUtensorMap* map, const void* base, uint64_t inner, uint64_t rows, uint64_t pitch, uint32_t box_inner,
                     uint32_t box_rows, CUtensorMapDataType dtype = CU_TENSOR_MAP_DATA_TYPE_UINT8) {
@@ -1046,10 +1070,12 @@ int grouped_gemm_16bit(const void* A, const void* W, int in_dtype, const int64_t
 int read_quant_status(int* out, int reset);
 int read_moe_status(int* out, int reset);
 int read_indexer_status(int* out, int reset);
+int read_attn_status(int* out, int reset);
 
-// One word for the caller: the GEMM's code if it has one, else the quantisers', the exchange kernels', the indexer's.
+// One word for the caller: the GEMM's code if it has one, else the quantisers', the exchange kernels', the indexer's,
+// the attention's.
 int read_device_status(int* out, int reset) {
-    int v = 0, q = 0, m = 0, x = 0;
+    int v = 0, q = 0, m = 0, x = 0, a = 0;
     CINN_CHECK_CUDA(cudaMemcpyFromSymbol(&v, g_device_status, sizeof(int)));
     if (reset && v != 0) {
         int z = 0;
@@ -1061,7 +1087,9 @@ int read_device_status(int* out, int reset) {
     if (rc) return rc;
     rc = read_indexer_status(&x, reset);
     if (rc) return rc;
-    *out = v != 0 ? v : (q != 0 ? q : (m != 0 ? m : x));
+    rc = read_attn_status(&a, reset);
+    if (rc) return rc;
+    *out = v != 0 ? v : (q != 0 ? q : (m != 0 ? m : (x != 0 ? x : a)));
     return CINN_OK;
 }
 

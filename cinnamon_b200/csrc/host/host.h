@@ -23,7 +23,8 @@ using at::Tensor;
 #define CINN_HOST_API(X)                                                                                            \
     X(cinn_last_error) X(cinn_quant_rowwise) X(cinn_quant_rowwise_dual) X(cinn_quant_rowwise_with_block)             \
     X(cinn_quant_rowwise_with_block_t) X(cinn_quant_blockwise) X(cinn_quant_blockwise_t) X(cinn_transpose_bytes)     \
-    X(cinn_requant_row_to_block) X(cinn_fp8_gemm_ws) X(cinn_fp8_gemm_workspace_bytes)
+    X(cinn_requant_row_to_block) X(cinn_fp8_gemm_ws) X(cinn_fp8_gemm_workspace_bytes) \
+    X(cinn_sparse_attn_workspace_bytes) X(cinn_sparse_attn_fwd_ws) X(cinn_sparse_attn_bwd) X(cinn_sparse_attn_bwd_ws)
 
 struct Api {
 #define CINN_DECL(name) decltype(&::name) name = nullptr;
@@ -47,6 +48,21 @@ inline void check(int status, const char* what) {
 }
 inline void require(bool ok, const char* what) {
     if (!ok) throw CinnError(what, true);
+}
+
+// Runs the body of a native backward: a CinnError in an autograd worker travels to the caller's thread as the Python
+// exception it stands for.
+template <typename F>
+void as_python_error(F&& body) {
+    try {
+        body();
+    } catch (const CinnError& e) {
+        pybind11::gil_scoped_acquire gil;
+        PyErr_SetString(e.invalid ? PyExc_AssertionError : PyExc_RuntimeError, e.what());
+        python_error err;
+        err.persist();
+        throw err;
+    }
 }
 
 constexpr int TAG_BF16 = 0, TAG_F32 = 1, TAG_F16 = 2, TAG_F32_BF16 = 3;

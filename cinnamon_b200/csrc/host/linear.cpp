@@ -156,17 +156,11 @@ public:
         auto s = ctx->get_saved_variables();
         const int64_t f = ctx->saved_data["flags"].toInt();
         Tensor gx, gw;
-        try {
+        as_python_error([&] {
             std::tie(gx, gw) = cinnhost::backward(grads[0], s[0], s[1], s[2], s[3], s[4], ctx->saved_data["x_shape"].toIntVector(), f & 1,
                                                   f & 2, f & 4, (at::ScalarType)(f >> 8), f & 8, (f >> 4) & 15, ctx->needs_input_grad(0),
                                                   ctx->needs_input_grad(1));
-        } catch (const CinnError& e) {
-            pybind11::gil_scoped_acquire gil;
-            PyErr_SetString(e.invalid ? PyExc_AssertionError : PyExc_RuntimeError, e.what());
-            python_error err;
-            err.persist();
-            throw err;
-        }
+        });
         return {gx, gw, Tensor(), Tensor(), Tensor(), Tensor()};
     }
 };

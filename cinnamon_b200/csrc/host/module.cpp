@@ -5,6 +5,7 @@ namespace cinnhost {
 Api api;
 std::atomic<int64_t> launches{0};
 void bind_linear(pybind11::module_& m);
+void bind_attention(pybind11::module_& m);
 }  // namespace cinnhost
 
 PYBIND11_MODULE(_host, m) {
@@ -32,4 +33,5 @@ PYBIND11_MODULE(_host, m) {
         }
     });
     bind_linear(m);
+    bind_attention(m);
 }

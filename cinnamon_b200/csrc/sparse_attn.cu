@@ -7,6 +7,9 @@
 // Backward: delta = dO.O, dp_j = p_j (dO.v_j - delta), dq = scale * sum_j dp_j k_j,
 // dk[idx_j] += scale * dp_j q, dv[idx_j] += p_j dO (fp32 atomics, as in the reference).
 //
+// Sequences of which the queries pick a fair share go through dense tiles on the tensor cores (attn_tc.cu); these are
+// the kernels for the rest - long sequences with short lists, wide rows - and what the dense path falls back to.
+//
 // One warp per (b, h, t).  The index list, the scores and the fp32 query live in the warp's slice of shared
 // memory.  Scores: one lane per key, the key row read with 16-byte loads (rows of one (b, h) are a few hundred
 // KiB and stay in L1/L2).  Output and gradients: one lane per pair of feature columns, so every gathered value
@@ -22,6 +25,11 @@ template <typename T> __device__ __forceinline__ float to_float(T v);
 template <> __device__ __forceinline__ float to_float<float>(float v) { return v; }
 template <> __device__ __forceinline__ float to_float<__nv_bfloat16>(__nv_bfloat16 v) { return __bfloat162float(v); }
 template <> __device__ __forceinline__ float to_float<__half>(__half v) { return __half2float(v); }
+
+template <typename T> __device__ __forceinline__ T from_float(float v);
+template <> __device__ __forceinline__ float from_float<float>(float v) { return v; }
+template <> __device__ __forceinline__ __nv_bfloat16 from_float<__nv_bfloat16>(float v) { return __float2bfloat16_rn(v); }
+template <> __device__ __forceinline__ __half from_float<__half>(float v) { return __float2half_rn(v); }
 
 // Part of the dot product of an fp32 vector in shared memory with a row of T in global memory: eight lanes share a
 // row, lane l8 of them takes the 16-byte chunks l8, l8 + 8, ... (so the eight lanes read 128 contiguous bytes per
@@ -90,12 +98,14 @@ __host__ __device__ inline size_t warp_smem_floats(int K, int Dqk, int Dv, bool 
 
 }  // namespace
 
+// out_cast: the output once more in the inputs' type, where that is not fp32.  run_if: do nothing when it points to zero.
 template <typename T>
 __global__ void __launch_bounds__(256)
 sparse_attn_fwd_kernel(const T* __restrict__ q, const T* __restrict__ k, const T* __restrict__ v,
                        const int64_t* __restrict__ idx, float* __restrict__ out, float* __restrict__ lse,
-                       float* __restrict__ attn_w, int B, int H, int L, int K, int Dqk, int Dv, float scale,
-                       int warps_per_cta, bool vec_qk) {
+                       float* __restrict__ attn_w, T* __restrict__ out_cast, int B, int H, int L, int K, int Dqk, int Dv, float scale,
+                       int warps_per_cta, bool vec_qk, const int* __restrict__ run_if) {
+    if (run_if && *run_if == 0) return;
     extern __shared__ __align__(16) float sm[];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     if (warp >= warps_per_cta) return;
@@ -162,6 +172,10 @@ sparse_attn_fwd_kernel(const T* __restrict__ q, const T* __restrict__ k, const T
             }
             orow[d0] = a0;
             if (two) orow[d0 + 1] = a1;
+            if (out_cast) {
+                out_cast[w * Dv + d0] = from_float<T>(a0);
+                if (two) out_cast[w * Dv + d0 + 1] = from_float<T>(a1);
+            }
         }
         __syncwarp();
     }
@@ -173,7 +187,8 @@ sparse_attn_bwd_kernel(const TG* __restrict__ d_out, const float* __restrict__ o
                        const T* __restrict__ q, const T* __restrict__ k, const T* __restrict__ v,
                        const int64_t* __restrict__ idx, float* __restrict__ dq, float* __restrict__ dk,
                        float* __restrict__ dv, int B, int H, int L, int K, int Dqk, int Dv, float scale,
-                       int warps_per_cta, bool vec_qk, bool vec_v, int atom_qk, int atom_v) {
+                       int warps_per_cta, bool vec_qk, bool vec_v, int atom_qk, int atom_v, const int* __restrict__ run_if) {
+    if (run_if && *run_if == 0) return;
     // atom_qk / atom_v: widest vector (4, 2 or 1 floats) the gradient buffers' widths AND addresses allow
     extern __shared__ __align__(16) float sm[];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -332,38 +347,70 @@ static int check_sparse_args(int64_t B, int64_t H, int64_t L, int64_t K, int64_t
 }
 
 template <typename T>
-static int sparse_fwd_typed(const T* q, const T* k, const T* v, const int64_t* idx, float* out, float* lse, float* attn_w,
-                            int B, int H, int L, int K, int Dqk, int Dv, float scale, cudaStream_t st) {
+static int sparse_fwd_typed(const T* q, const T* k, const T* v, const int64_t* idx, float* out, float* lse, float* attn_w, T* out_cast,
+                            int B, int H, int L, int K, int Dqk, int Dv, float scale, const int* run_if, cudaStream_t st) {
     int warps; unsigned grid; size_t smem;
     int rc = sparse_launch_shape(K, Dqk, Dv, false, (int64_t)B * H * L, &warps, &grid, &smem);
     if (rc) return rc;
     rc = allow_smem(sparse_attn_fwd_kernel<T>);
     if (rc) return rc;
     const bool vec_qk = (Dqk * sizeof(T)) % 16 == 0 && (reinterpret_cast<uintptr_t>(k) & 15) == 0;
-    sparse_attn_fwd_kernel<T><<<grid, 256, smem, st>>>(q, k, v, idx, out, lse, attn_w, B, H, L, K, Dqk, Dv, scale, warps, vec_qk);
+    sparse_attn_fwd_kernel<T><<<grid, 256, smem, st>>>(q, k, v, idx, out, lse, attn_w, out_cast, B, H, L, K, Dqk, Dv, scale, warps, vec_qk,
+                                                          run_if);
     CINN_CHECK_LAUNCH();
     return CINN_OK;
 }
 
-int sparse_attn_fwd(const void* q, const void* k, const void* v, int dtype, const int64_t* idx, float* out, float* lse,
-                    float* attn_w, int64_t B, int64_t H, int64_t L, int64_t K, int64_t Dqk, int64_t Dv, float scale,
-                    cudaStream_t st) {
+namespace atc {                          // attn_tc.cu
+int64_t forward_workspace_bytes(int64_t B, int64_t H, int64_t L, int64_t K, int64_t Dqk, int64_t Dv, int dtype);
+int forward(const void* q, const void* k, const void* v, int dtype, const int64_t* idx, float* out, void* out_cast, float* lse,
+            float* attn, int64_t B, int64_t H, int64_t L, int64_t K, int64_t Dqk, int64_t Dv, float scale, uint8_t* ws,
+            const int** flag, cudaStream_t st);
+int64_t backward_workspace_bytes(int64_t B, int64_t H, int64_t L, int64_t K, int64_t Dqk, int64_t Dv, int dtype);
+int backward(const void* d_out, const float* out, const float* lse, const void* q, const void* k, const void* v, int dtype,
+             const int64_t* idx, void* dq, void* dk, void* dv, int64_t B, int64_t H, int64_t L, int64_t K, int64_t Dqk, int64_t Dv,
+             float scale, uint8_t* ws, const int** flag, float** fallback, cudaStream_t st);
+}  // namespace atc
+
+int64_t sparse_attn_workspace_bytes(int64_t B, int64_t H, int64_t L, int64_t K, int64_t Dqk, int64_t Dv, int dtype, int backward) {
+    if (B < 0 || H < 0 || L < 0 || K < 0 || Dqk < 1 || Dv < 1) return 0;
+    if (backward) return atc::backward_workspace_bytes(B, H, L, K, Dqk, Dv, dtype);
+    return atc::forward_workspace_bytes(B, H, L, K, Dqk, Dv, dtype);
+}
+
+// With a workspace of sparse_attn_workspace_bytes the dense tiles compute the call where they pay and the gather kernel
+// stands behind them for what they cannot express; without one it computes the call.
+int sparse_attn_fwd(const void* q, const void* k, const void* v, int dtype, const int64_t* idx, float* out, void* out_cast,
+                    float* lse, float* attn_w, int64_t B, int64_t H, int64_t L, int64_t K, int64_t Dqk, int64_t Dv, float scale,
+                    void* workspace, int64_t workspace_bytes, cudaStream_t st) {
     int rc = check_sparse_args(B, H, L, K, Dqk, Dv);
     if (rc) return rc;
     if (B * H * L == 0) return CINN_OK;
     CINN_CHECK_ARG(q && k && v && out && lse && (K == 0 || (idx && attn_w)), "sparse_attention: null pointer");
-    switch (dtype) {
-        case CINN_BF16: return sparse_fwd_typed((const __nv_bfloat16*)q, (const __nv_bfloat16*)k, (const __nv_bfloat16*)v, idx, out, lse, attn_w, (int)B, (int)H, (int)L, (int)K, (int)Dqk, (int)Dv, scale, st);
-        case CINN_F16: return sparse_fwd_typed((const __half*)q, (const __half*)k, (const __half*)v, idx, out, lse, attn_w, (int)B, (int)H, (int)L, (int)K, (int)Dqk, (int)Dv, scale, st);
-        case CINN_F32: return sparse_fwd_typed((const float*)q, (const float*)k, (const float*)v, idx, out, lse, attn_w, (int)B, (int)H, (int)L, (int)K, (int)Dqk, (int)Dv, scale, st);
-        default: set_error("sparse_attention: unknown dtype tag %d", dtype); return CINN_ERR_INVALID;
+    CINN_CHECK_ARG(dtype == CINN_BF16 || dtype == CINN_F16 || dtype == CINN_F32, "sparse_attention: unknown dtype tag %d", dtype);
+    const int* run_if = nullptr;
+    const int64_t need = workspace ? atc::forward_workspace_bytes(B, H, L, K, Dqk, Dv, dtype) : 0;
+    const bool aligned = ((reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(k) | reinterpret_cast<uintptr_t>(v) |
+                           reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(out_cast) | reinterpret_cast<uintptr_t>(workspace)) & 15) == 0;
+    if (need > 0 && workspace_bytes >= need && aligned) {
+        rc = atc::forward(q, k, v, dtype, idx, out, out_cast, lse, attn_w, B, H, L, K, Dqk, Dv, scale, static_cast<uint8_t*>(workspace),
+                          &run_if, st);
+        if (rc) return rc;
     }
+#define CINN_SF(T) sparse_fwd_typed((const T*)q, (const T*)k, (const T*)v, idx, out, lse, attn_w, (T*)out_cast, (int)B, (int)H, (int)L, \
+                                    (int)K, (int)Dqk, (int)Dv, scale, run_if, st)
+    switch (dtype) {
+        case CINN_BF16: return CINN_SF(__nv_bfloat16);
+        case CINN_F16: return CINN_SF(__half);
+        default: return CINN_SF(float);
+    }
+#undef CINN_SF
 }
 
 template <typename T, typename TG>
 static int sparse_bwd_typed(const TG* d_out, const float* out, const float* lse, const T* q, const T* k, const T* v,
                             const int64_t* idx, float* dq, float* dk, float* dv, int B, int H, int L, int K, int Dqk, int Dv,
-                            float scale, cudaStream_t st) {
+                            float scale, const int* run_if, cudaStream_t st) {
     int warps; unsigned grid; size_t smem;
     int rc = sparse_launch_shape(K, Dqk, Dv, true, (int64_t)B * H * L, &warps, &grid, &smem);
     if (rc) return rc;
@@ -379,7 +426,7 @@ static int sparse_bwd_typed(const TG* d_out, const float* out, const float* lse,
         return 1;
     };
     sparse_attn_bwd_kernel<T, TG><<<grid, 256, smem, st>>>(d_out, out, lse, q, k, v, idx, dq, dk, dv, B, H, L, K, Dqk, Dv, scale,
-                                                         warps, vec_qk, vec_v, widest(Dqk, dk, dq), widest(Dv, dv, dv));
+                                                         warps, vec_qk, vec_v, widest(Dqk, dk, dq), widest(Dv, dv, dv), run_if);
     CINN_CHECK_LAUNCH();
     return CINN_OK;
 }
@@ -387,7 +434,7 @@ static int sparse_bwd_typed(const TG* d_out, const float* out, const float* lse,
 // dq is written; dk and dv are ACCUMULATED into (the caller zeroes them, as the reference does, :1257-1259)
 int sparse_attn_bwd(const void* d_out, int grad_dtype, const float* out, const float* lse, const void* q, const void* k,
                     const void* v, int dtype, const int64_t* idx, float* dq, float* dk, float* dv, int64_t B, int64_t H,
-                    int64_t L, int64_t K, int64_t Dqk, int64_t Dv, float scale, cudaStream_t st) {
+                    int64_t L, int64_t K, int64_t Dqk, int64_t Dv, float scale, const int* run_if, cudaStream_t st) {
     int rc = check_sparse_args(B, H, L, K, Dqk, Dv);
     if (rc) return rc;
     if (B * H * L == 0) return CINN_OK;
@@ -395,7 +442,7 @@ int sparse_attn_bwd(const void* d_out, int grad_dtype, const float* out, const f
     CINN_CHECK_ARG(grad_dtype == dtype || grad_dtype == CINN_F32, "sparse_attention: the output gradient must have the inputs' "
                    "type or be fp32 (tags %d, %d)", grad_dtype, dtype);
 #define CINN_SB(T, TG) sparse_bwd_typed((const TG*)d_out, out, lse, (const T*)q, (const T*)k, (const T*)v, idx, dq, dk, dv, (int)B, \
-                                        (int)H, (int)L, (int)K, (int)Dqk, (int)Dv, scale, st)
+                                        (int)H, (int)L, (int)K, (int)Dqk, (int)Dv, scale, run_if, st)
     switch (dtype) {
         case CINN_BF16: return grad_dtype == CINN_F32 ? CINN_SB(__nv_bfloat16, float) : CINN_SB(__nv_bfloat16, __nv_bfloat16);
         case CINN_F16: return grad_dtype == CINN_F32 ? CINN_SB(__half, float) : CINN_SB(__half, __half);
@@ -403,6 +450,59 @@ int sparse_attn_bwd(const void* d_out, int grad_dtype, const float* out, const f
         default: set_error("sparse_attention: unknown dtype tag %d", dtype); return CINN_ERR_INVALID;
     }
 #undef CINN_SB
+}
+
+// The fallback of the tiles' backward around the gather kernel: zeroes before it, the gradients' own type after it.
+__global__ void zero_if_kernel(const int* __restrict__ run_if, float* __restrict__ p, int64_t n) {
+    if (*run_if == 0) return;
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) p[i] = 0.0f;
+}
+template <typename T>
+__global__ void cast_if_kernel(const int* __restrict__ run_if, const float* __restrict__ src, T* __restrict__ dst, int64_t n) {
+    if (*run_if == 0) return;
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) dst[i] = from_float<T>(src[i]);
+}
+
+// Gradients written (not added) in `dtype`, through the tiles; needs the workspace that sparse_attn_workspace_bytes asks for.
+int sparse_attn_bwd_tiles(const void* d_out, const float* out, const float* lse, const void* q, const void* k, const void* v, int dtype,
+                          const int64_t* idx, void* dq, void* dk, void* dv, int64_t B, int64_t H, int64_t L, int64_t K, int64_t Dqk,
+                          int64_t Dv, float scale, void* workspace, int64_t workspace_bytes, cudaStream_t st) {
+    int rc = check_sparse_args(B, H, L, K, Dqk, Dv);
+    if (rc) return rc;
+    CINN_CHECK_ARG(dtype == CINN_BF16 || dtype == CINN_F16 || dtype == CINN_F32, "sparse_attention: unknown dtype tag %d", dtype);
+    const int64_t need = atc::backward_workspace_bytes(B, H, L, K, Dqk, Dv, dtype);
+    const uintptr_t bits = reinterpret_cast<uintptr_t>(d_out) | reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(k) |
+                           reinterpret_cast<uintptr_t>(v) | reinterpret_cast<uintptr_t>(dq) | reinterpret_cast<uintptr_t>(dk) |
+                           reinterpret_cast<uintptr_t>(dv) | reinterpret_cast<uintptr_t>(workspace);
+    CINN_CHECK_ARG(d_out && out && lse && q && k && v && dq && dk && dv && idx && workspace, "sparse_attention: null pointer");
+    CINN_CHECK_ARG(need > 0 && workspace_bytes >= need && (bits & 15) == 0,
+                   "sparse_attention: the tiled backward needs %lld bytes of workspace and 16-byte aligned tensors", (long long)need);
+    const int* run_if = nullptr;
+    float* fb = nullptr;
+    rc = atc::backward(d_out, out, lse, q, k, v, dtype, idx, dq, dk, dv, B, H, L, K, Dqk, Dv, scale, static_cast<uint8_t*>(workspace),
+                       &run_if, &fb, st);
+    if (rc) return rc;
+    const int64_t nqk = B * H * L * Dqk, nv = B * H * L * Dv;
+    float* gq = fb ? fb : static_cast<float*>(dq);
+    float* gk = fb ? fb + nqk : static_cast<float*>(dk);
+    float* gv = fb ? fb + 2 * nqk : static_cast<float*>(dv);
+    const unsigned grid = (unsigned)sm_count() * 4;
+    if (fb) {
+        zero_if_kernel<<<grid, 256, 0, st>>>(run_if, gk, nqk + nv);
+    } else {
+        zero_if_kernel<<<grid, 256, 0, st>>>(run_if, gk, nqk);
+        zero_if_kernel<<<grid, 256, 0, st>>>(run_if, gv, nv);
+    }
+    CINN_CHECK_LAUNCH();
+    rc = sparse_attn_bwd(d_out, dtype, out, lse, q, k, v, dtype, idx, gq, gk, gv, B, H, L, K, Dqk, Dv, scale, run_if, st);
+    if (rc || !fb) return rc;
+    const struct { const float* src; void* dst; int64_t n; } casts[3] = {{gq, dq, nqk}, {gk, dk, nqk}, {gv, dv, nv}};
+    for (const auto& c : casts) {
+        if (dtype == CINN_BF16) cast_if_kernel<<<grid, 256, 0, st>>>(run_if, c.src, static_cast<__nv_bfloat16*>(c.dst), c.n);
+        else cast_if_kernel<<<grid, 256, 0, st>>>(run_if, c.src, static_cast<__half*>(c.dst), c.n);
+    }
+    CINN_CHECK_LAUNCH();
+    return CINN_OK;
 }
 
 }  // namespace cinn

@@ -48,4 +48,7 @@ __device__ __forceinline__ void fence_async_smem() { asm volatile("fence.proxy.a
 int encode_map_2d(CUtensorMap* map, const void* base, uint64_t inner, uint64_t rows, uint64_t pitch_bytes,
                   uint32_t box_inner, uint32_t box_rows, CUtensorMapDataType dtype, CUtensorMapSwizzle swizzle);
 
+int encode_map_3d(CUtensorMap* map, const void* base, uint64_t inner, uint64_t rows, uint64_t planes, uint64_t pitch_bytes,
+                  uint32_t box_rows, CUtensorMapDataType dtype);
+
 }  // namespace cinn

@@ -246,7 +246,19 @@ int cinn_sparse_attn_fwd(const void* q, const void* k, const void* v, int dtype,
                          float* attn_weights, int64_t B, int64_t H, int64_t L, int64_t K, int64_t d_qk, int64_t d_v,
                          float scale, void* stream);
 
-/* Backward of the above.  Replaces sparse_attention_bwd_kernel + SparseAttentionFunction.backward
+/* The same with a scratch buffer (256-byte aligned), by which a sequence of which the queries pick a fair share goes
+ * through dense tiles on the tensor cores instead of row gathers.  cinn_sparse_attn_workspace_bytes (backward: 0 / 1) says
+ * how much that takes, 0 where the gathers are the better choice; a null or smaller workspace selects them.
+ * out_cast: null, or the output once more in `dtype`. */
+int cinn_set_sparse_attn_dense(int mode); /* -1: choose by shape (default), 0: gathers, 1: dense tiles where they can;
+                                             returns the previous mode */
+int64_t cinn_sparse_attn_workspace_bytes(int64_t B, int64_t H, int64_t L, int64_t K, int64_t d_qk, int64_t d_v, int dtype,
+                                         int backward);
+int cinn_sparse_attn_fwd_ws(const void* q, const void* k, const void* v, int dtype, const int64_t* idx, float* out,
+                            void* out_cast, float* lse, float* attn_weights, int64_t B, int64_t H, int64_t L, int64_t K,
+                            int64_t d_qk, int64_t d_v, float scale, void* workspace, int64_t workspace_bytes, void* stream);
+
+/* Backward of cinn_sparse_attn_fwd.  Replaces sparse_attention_bwd_kernel + SparseAttentionFunction.backward
  * (src/kernels.py:1055-1186, 1247-1289).  grad_out: (B, H, L, d_v) of `grad_dtype` (the inputs' type or fp32);
  * out, lse: as saved by the forward.  grad_q is written; grad_k and grad_v (fp32, same shapes as k and v) are
  * ACCUMULATED into with fp32 atomics, so the caller zeroes them first, as the reference does (:1257-1259). */
@@ -255,6 +267,12 @@ int cinn_sparse_attn_bwd(const void* grad_out, int grad_dtype, const float* out,
                          float* grad_v, int64_t B, int64_t H, int64_t L, int64_t K, int64_t d_qk, int64_t d_v, float scale,
                          void* stream);
 
+
+/* The backward through dense tiles, for shapes where cinn_sparse_attn_workspace_bytes(..., 1) is not zero: grad_out is of
+ * `dtype`, and grad_q, grad_k and grad_v are WRITTEN in `dtype`.  All tensors 16-byte aligned. */
+int cinn_sparse_attn_bwd_ws(const void* grad_out, const float* out, const float* lse, const void* q, const void* k, const void* v,
+                            int dtype, const int64_t* idx, void* grad_q, void* grad_k, void* grad_v, int64_t B, int64_t H, int64_t L,
+                            int64_t K, int64_t d_qk, int64_t d_v, float scale, void* workspace, int64_t workspace_bytes, void* stream);
 
 /* Lightning indexer logits: out[b, t, s] = sum_h relu(q[b, t, h, :] . k[b, s, :]) * w[b, t, h], fp16.
  * Replaces lightning_indexer_kernel + lightning_indexer_fused (src/kernels.py:321-433): dot-product operands

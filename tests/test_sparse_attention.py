@@ -158,3 +158,67 @@ def test_backward_with_gradient_buffers_at_odd_addresses():
     for a, b in zip(*grads):
         torch.testing.assert_close(a, b, rtol=1e-5, atol=1e-6)
     assert K.device_status() == 0
+
+
+@pytest.fixture(params=["dense", "gather"])
+def attention_path(request):
+    """Every shape the tiles can take through the tiles, and through the gathers."""
+    from cinnamon_b200 import kernels as K
+    before = K._L.cinn_set_sparse_attn_dense(1 if request.param == "dense" else 0)
+    yield request.param
+    K._L.cinn_set_sparse_attn_dense(before)
+    assert K.device_status() == 0
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32, torch.float16])
+@pytest.mark.parametrize("shape", [(1, 2, 1, 1, 64, 64), (1, 2, 127, 33, 64, 64), (2, 1, 129, 32, 192, 64), (1, 2, 300, 40, 72, 100),
+                                   (1, 1, 385, 70, 128, 128), (1, 1, 260, 7, 20, 6)])
+def test_tiles_and_gathers(dtype, shape, attention_path):
+    """Partial tiles, one to four key tiles, padded and split widths, duplicates, queries without a valid key, indices
+    outside the sequence.  The same bounds for both paths: fp32 arithmetic on the given inputs."""
+    from cinnamon_b200 import kernels as K
+    B, H, L, Ks, Dqk, Dv = shape
+    g = torch.Generator().manual_seed(sum(shape))
+    q, k, go = (torch.randn(B, H, L, d, generator=g).to(dtype) for d in (Dqk, Dqk, Dv))
+    v = torch.randn(B, H, L, Dv, generator=g).to(dtype)
+    idx = torch.randint(-2, L + 2, (B, L, Ks), generator=g)
+    idx[:, L // 2] = L + 1                                # a query without any valid key
+    scale = Dqk ** -0.5
+    ref_out, ref_attn, _ = SO.forward(q, k, v, idx, scale)
+    qc, kc, vc = (t.cuda().requires_grad_(True) for t in (q, k, v))
+    out, attn = K.sparse_attention(qc, kc, vc, idx.cuda(), scale)
+    tol = {torch.float32: 1e-5, torch.bfloat16: 8e-3, torch.float16: 1e-3}[dtype]       # rounding of the returned output
+    torch.testing.assert_close(out.float().cpu().double(), ref_out, rtol=tol, atol=tol)
+    torch.testing.assert_close(attn.cpu().double(), ref_attn, rtol=2e-5, atol=1e-7)
+    out.backward(go.cuda())
+    for name, got, want in zip(("dq", "dk", "dv"), (qc.grad, kc.grad, vc.grad), SO.backward(q, k, v, idx, scale, go)):
+        assert got.dtype == dtype
+        err = (got.float().cpu().double() - want).norm() / want.norm().clamp(min=1e-30)
+        assert err < {torch.float32: 2e-6, torch.bfloat16: 4e-3, torch.float16: 5e-4}[dtype], (name, float(err))
+
+
+@pytest.mark.gpu
+def test_tiles_fall_back_on_the_device(attention_path):
+    """What the tiles cannot express: a key picked more than 255 times, and rows nobody picked that hold NaN or infinity."""
+    from cinnamon_b200 import kernels as K
+    g = torch.Generator().manual_seed(3)
+    q, k, v = (torch.randn(1, 1, 140, 64, generator=g) for _ in range(3))
+    idx = torch.randint(0, 140, (1, 140, 300), generator=g)
+    idx[idx == 17] = 18
+    idx[0, 100] = 5
+    ref_out, ref_attn, _ = SO.forward(q, k, v, idx, 0.2)
+    go = torch.randn(1, 1, 140, 64, generator=g)
+    ref = SO.backward(q, k, v, idx, 0.2, go)
+    k[0, 0, 17], v[0, 0, 17] = float("nan"), float("inf")
+    for _ in range(2):
+        qc, kc, vc = (t.cuda().requires_grad_(True) for t in (q, k, v))
+        out, attn = K.sparse_attention(qc, kc, vc, idx.cuda(), 0.2)
+        out.backward(go.cuda())
+        for got, want in zip((qc.grad, kc.grad, vc.grad), ref):
+            assert float((got.cpu().double() - want).norm() / want.norm()) < 2e-6
+        torch.testing.assert_close(out.cpu().double(), ref_out, rtol=1e-5, atol=1e-6)
+        torch.testing.assert_close(attn.cpu().double(), ref_attn, rtol=2e-5, atol=1e-7)
+        idx[0, 100, ::2] = 6                              # now only the rows that nobody picked
+        clean = (q, torch.nan_to_num(k), torch.nan_to_num(v, posinf=0.0), idx, 0.2)
+        (ref_out, ref_attn, _), ref = SO.forward(*clean), SO.backward(*clean, go)
