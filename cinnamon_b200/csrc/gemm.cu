@@ -140,6 +140,30 @@ __device__ __forceinline__ TileInfo tile_info(const GemmParams& p, const int* cu
     return ti;
 }
 
+// grouped: cum[e] = row tiles (of `rows`) of the experts before e, cum[E] = all of them; by one warp
+__device__ __forceinline__ void tile_prefix_sum(const GemmParams& p, int* cum, int rows, int lane) {
+    int carry = 0;
+    for (int base = 0; base < p.E; base += 32) {
+        const int e = base + lane;
+        int cnt = 0;
+        if (e < p.E) {
+            long long s = p.starts[e], t = p.ends[e];
+            if (t > (long long)p.M) t = p.M;
+            if (s < 0) s = 0;
+            if (t > s) cnt = (int)((t - s + rows - 1) / rows);
+        }
+        int incl = cnt;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int v = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= o) incl += v;
+        }
+        if (e < p.E) cum[e] = carry + incl - cnt;
+        carry += __shfl_sync(0xffffffffu, incl, 31);
+    }
+    if (lane == 0) cum[p.E] = carry;
+}
+
 template <int OUT> struct OutT;
 template <> struct OutT<CINN_BF16> { using type = __nv_bfloat16; };
 template <> struct OutT<CINN_F16> { using type = __half; };
@@ -280,28 +304,7 @@ fp8_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
     if constexpr (GROUPED) {
-        if (warp == 0) {                           // prefix sum of per-expert m-tile counts
-            int carry = 0;
-            for (int base = 0; base < p.E; base += 32) {
-                const int e = base + lane;
-                int cnt = 0;
-                if (e < p.E) {
-                    long long s = p.starts[e], t = p.ends[e];
-                    if (t > (long long)p.M) t = p.M;
-                    if (s < 0) s = 0;
-                    if (t > s) cnt = (int)((t - s + BM - 1) / BM);
-                }
-                int incl = cnt;
-#pragma unroll
-                for (int o = 1; o < 32; o <<= 1) {
-                    const int v = __shfl_up_sync(0xffffffffu, incl, o);
-                    if (lane >= o) incl += v;
-                }
-                if (e < p.E) cum[e] = carry + incl - cnt;
-                carry += __shfl_sync(0xffffffffu, incl, 31);
-            }
-            if (lane == 0) cum[p.E] = carry;
-        }
+        if (warp == 0) tile_prefix_sum(p, cum, BM, lane);
     }
     tc_fence_before();
     __syncthreads();
@@ -692,12 +695,12 @@ static int launch_out(const CUtensorMap& ta, const CUtensorMap& tb, GemmParams& 
     }
 }
 
-template <bool B_MN, int OUT>
+template <bool B_MN, int OUT, bool GK = false, bool GR = false>
 static int launch_pair(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& tc, const GemmParams& p, int clusters,
                        cudaStream_t st) {
-    constexpr auto kern = pair::fp8_gemm_pair_kernel<B_MN, OUT>;
-    const size_t smem = pair::PSMEM_BYTES;
-    int rc = allow_smem_once<kern>(smem);
+    constexpr auto kern = pair::fp8_gemm_pair_kernel<B_MN, OUT, GK, GR>;
+    const size_t smem = pair::PSMEM_BYTES + (GR ? 4 * (size_t)(p.E + 2) : 0);
+    int rc = allow_smem_once<kern>(pair::PSMEM_BYTES + (GR ? 4 * (size_t)(MAX_EXPERTS + 2) : 0));
     if (rc) return rc;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(2 * clusters, 1, 1);
@@ -902,7 +905,11 @@ int fp8_grouped_gemm(const void* A, const float* sA, const void* W, const float*
     CUtensorMap ta, tb;
     int rc = make_map(&ta, A, (uint64_t)d_in, (uint64_t)T, (uint64_t)d_in, BK, BM);
     if (rc) return rc;
-    rc = make_map(&tb, W, (uint64_t)d_in, (uint64_t)(E * d_out), (uint64_t)d_in, BK, BN);
+    // Pairs of SMs on 256-row tiles from 256 rows per expert on average (how the rows are really spread only the device
+    // knows): below that the half-empty tiles cost more than the pair saves.
+    const bool use_pair = row_dst == nullptr && pair_mode() != 0 && T >= pair::PM * E &&
+                          (T + pair::PM - 1) / pair::PM * ((d_out + pair::PN - 1) / pair::PN) >= gemm_sms() / 2;
+    rc = make_map(&tb, W, (uint64_t)d_in, (uint64_t)(E * d_out), (uint64_t)d_in, BK, use_pair ? 128 : BN);
     if (rc) return rc;
     const int64_t nkb = (d_in + 127) / 128, nnb = (d_out + 127) / 128;
     GemmParams p{};
@@ -916,6 +923,19 @@ int fp8_grouped_gemm(const void* A, const float* sA, const void* W, const float*
         p.tma_out = 0;
         return out_dtype == CINN_BF16 ? launch<false, true, CINN_BF16, true>(ta, tb, ta, p, gemm_sms(), st)
                                       : launch<false, true, CINN_F16, true>(ta, tb, ta, p, gemm_sms(), st);
+    }
+    if (use_pair) {
+        CUtensorMap tc;
+        rc = make_out_map(&tc, ta, p, out_dtype, T, true);
+        if (rc) return rc;
+        const int clusters = gemm_sms() / 2;
+        switch (out_dtype) {
+            case CINN_BF16: return launch_pair<false, CINN_BF16, false, true>(ta, tb, tc, p, clusters, st);
+            case CINN_F16: return launch_pair<false, CINN_F16, false, true>(ta, tb, tc, p, clusters, st);
+            case CINN_F32: return launch_pair<false, CINN_F32, false, true>(ta, tb, tc, p, clusters, st);
+            case CINN_F32_BF16: return launch_pair<false, CINN_F32_BF16, false, true>(ta, tb, tc, p, clusters, st);
+            default: set_error("GEMM: unknown output dtype tag %d", out_dtype); return CINN_ERR_INVALID;
+        }
     }
     return launch_out<false, true>(ta, tb, p, out_dtype, gemm_sms(), st);
 }
@@ -954,29 +974,6 @@ int fp8_grouped_gemm_dgrad(const void* dY, const float* sdY, const void* W, cons
 // Weight gradients of all experts in one launch (the GK instantiation of the pair kernel): dW (E, d_out, d_in) with
 // A = dY^T quantised per expert segment, (d_out, max_tiles * 128), and B = x block-quantised per segment and
 // transposed, (d_in, max_tiles * 128); kb_start (E + 1 ints, device) gives every expert's K blocks.
-template <int OUT>
-static int launch_pair_gk(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& tc, const GemmParams& p, int clusters,
-                          cudaStream_t st) {
-    constexpr auto kern = pair::fp8_gemm_pair_kernel<false, OUT, true>;
-    const size_t smem = pair::PSMEM_BYTES;
-    int rc = allow_smem_once<kern>(smem);
-    if (rc) return rc;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(2 * clusters, 1, 1);
-    cfg.blockDim = dim3(pair::PTHREADS, 1, 1);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = st;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = 2;
-    attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    CINN_CHECK_CUDA(cudaLaunchKernelEx(&cfg, kern, ta, tb, tc, p));
-    return CINN_OK;
-}
-
 int fp8_gemm_grouped_k(const void* A, const float* sA, const void* B, const float* sB, const int* kb_start, int64_t E,
                        int64_t M, int64_t N, int64_t max_tiles, void* C, int out_dtype, cudaStream_t st) {
     CINN_CHECK_ARG(E >= 1 && M > 0 && N > 0 && max_tiles >= 1, "grouped-K GEMM: bad shape");
@@ -1002,9 +999,9 @@ int fp8_gemm_grouped_k(const void* A, const float* sA, const void* B, const floa
     const int64_t tiles = E * (M / pair::PM) * (N / pair::PN);
     const int clusters = (int)(tiles < gemm_sms() / 2 ? tiles : gemm_sms() / 2);
     switch (out_dtype) {
-        case CINN_BF16: return launch_pair_gk<CINN_BF16>(ta, tb, tc, p, clusters, st);
-        case CINN_F32: return launch_pair_gk<CINN_F32>(ta, tb, tc, p, clusters, st);
-        case CINN_F32_BF16: return launch_pair_gk<CINN_F32_BF16>(ta, tb, tc, p, clusters, st);
+        case CINN_BF16: return launch_pair<false, CINN_BF16, true>(ta, tb, tc, p, clusters, st);
+        case CINN_F32: return launch_pair<false, CINN_F32, true>(ta, tb, tc, p, clusters, st);
+        case CINN_F32_BF16: return launch_pair<false, CINN_F32_BF16, true>(ta, tb, tc, p, clusters, st);
         default: set_error("grouped-K GEMM: the gradient is fp32 (optionally holding bf16-rounded values) or bf16"); return CINN_ERR_INVALID;
     }
 }

@@ -98,7 +98,12 @@ __device__ __forceinline__ PairTile pair_tile(const GemmParams& p, int t) {
 // which expert e owns the K blocks [kb_start[e], kb_start[e + 1]) (p.starts holds that int array, p.E = E); tile t
 // belongs to expert t / (tiles per expert) and is stored at rows e * M + ... of the (E * M, N) output.  An expert
 // without rows gets zeros.  M and N are multiples of 256 here, so every tile is whole.
-template <bool B_MN, int OUT, bool GK = false>
+//
+// GR ("grouped rows"): E independent problems of the same N x K over the ragged row ranges [starts[e], ends[e]) of A and C
+// (device arrays), B stacked (E * b_rows_per_expert rows).  The tiles of all experts are one list, found through a prefix sum
+// of their tile counts in shared memory behind the barriers; a CTA whose 128 rows are not all its expert's stores them with
+// row predicates.  Worth it from a few tiles of rows per expert on: see fp8_grouped_gemm.
+template <bool B_MN, int OUT, bool GK = false, bool GR = false>
 __global__ void __launch_bounds__(PTHREADS, 1)
 fp8_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                      const __grid_constant__ CUtensorMap tmC, const GemmParams p) {
@@ -112,6 +117,7 @@ fp8_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * PSTAGES + 8);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
     uint8_t* store_stage = c_stage;                                             // 2 KiB per promotion warp (non-TMA path)
+    int* cum = reinterpret_cast<int*>(reinterpret_cast<uint8_t*>(bars) + 256);  // GR: E + 1 prefix counts of row tiles
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t rank = cluster_ctarank();           // 0 = leader
@@ -130,6 +136,9 @@ fp8_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
         asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(TMEM_COLS) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
     }
+    if constexpr (GR) {
+        if (warp == 0) tile_prefix_sum(p, cum, PM, lane);
+    }
     tc_fence_before();
     __syncthreads();
     cluster_sync();                                    // both CTAs' barriers exist before anyone signals them
@@ -138,12 +147,27 @@ fp8_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
 
     const int KB_dense = (p.K + BK - 1) / BK;
     const int per_expert = pair_total(p);
-    const int n_total = GK ? per_expert * p.E : per_expert;
+    const int n_tiles = (p.N + PN - 1) / PN;
+    const int n_total = GR ? cum[p.E] * n_tiles : (GK ? per_expert * p.E : per_expert);
     const int cluster_id = blockIdx.x >> 1, n_clusters = gridDim.x >> 1;
     const int* kb_start = reinterpret_cast<const int*>(p.starts);
-    // tile t -> its coordinates inside one problem, the expert it belongs to, its K blocks
-    auto locate = [&](int t, PairTile& ti, int& e, int& kb0, int& KB) {
-        if constexpr (GK) {
+    // tile t -> its coordinates inside one problem (GR: among all rows), the expert it belongs to, its K blocks, and one past
+    // the last row it may write
+    auto locate = [&](int t, PairTile& ti, int& e, int& kb0, int& KB, int& m_end) {
+        m_end = p.M;
+        if constexpr (GR) {
+            const int mt = t / n_tiles;
+            int lo = 0, hi = p.E;                      // largest e with cum[e] <= mt
+            while (hi - lo > 1) {
+                const int mid = (lo + hi) >> 1;
+                if (cum[mid] <= mt) lo = mid; else hi = mid;
+            }
+            e = lo; kb0 = 0; KB = KB_dense;
+            const long long first = p.starts[lo], last = p.ends[lo];
+            ti.m0 = (int)first + (mt - cum[lo]) * PM;
+            ti.n0 = (t - mt * n_tiles) * PN;
+            m_end = (int)(last < (long long)p.M ? last : (long long)p.M);
+        } else if constexpr (GK) {
             e = t / per_expert;
             ti = pair_tile(p, t - e * per_expert);
             kb0 = kb_start[e];
@@ -161,8 +185,9 @@ fp8_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
             uint32_t it = 0;
             bool alive = true;
             for (int t = cluster_id; t < n_total && alive; t += n_clusters) {
-                PairTile ti; int e, kb0, KB;
-                locate(t, ti, e, kb0, KB);
+                PairTile ti; int e, kb0, KB, m_end;
+                locate(t, ti, e, kb0, KB, m_end);
+                const int b_row0 = GR ? e * p.b_rows_per_expert : 0;
                 for (int kb = 0; kb < KB; ++kb, ++it) {
                     const int s = it % PSTAGES;
                     const uint32_t ph = (it / PSTAGES) & 1;
@@ -170,8 +195,8 @@ fp8_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
                     if (rank == 0) mbar_expect_tx(full0 + 8 * s, 2 * (PA_BYTES + PB_BYTES));
                     const uint32_t fb = full_leader + 8 * s;
                     tma_load_2d_pair(&tmA, fb, smem_u32(smem_a + s * PA_BYTES), (kb0 + kb) * BK, ti.m0 + 128 * (int)rank);
-                    if constexpr (!B_MN) tma_load_2d_pair(&tmB, fb, smem_u32(smem_b + s * PB_BYTES), (kb0 + kb) * BK, ti.n0 + 128 * (int)rank);
-                    else tma_load_2d_pair(&tmB, fb, smem_u32(smem_b + s * PB_BYTES), ti.n0 + 128 * (int)rank, (kb0 + kb) * BK);
+                    if constexpr (!B_MN) tma_load_2d_pair(&tmB, fb, smem_u32(smem_b + s * PB_BYTES), (kb0 + kb) * BK, b_row0 + ti.n0 + 128 * (int)rank);
+                    else tma_load_2d_pair(&tmB, fb, smem_u32(smem_b + s * PB_BYTES), ti.n0 + 128 * (int)rank, b_row0 + (kb0 + kb) * BK);
                 }
             }
             if (!alive) {
@@ -189,8 +214,11 @@ fp8_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
             uint32_t it = 0, last = 0xffffffffu;
             bool alive = true;
             for (int t = cluster_id; t < n_total && alive; t += n_clusters) {
-                PairTile ti_; int e_, kb0_, KB;
-                locate(t, ti_, e_, kb0_, KB);
+                int KB = KB_dense;
+                if constexpr (GK) {
+                    PairTile ti_; int e_, kb0_, end_;
+                    locate(t, ti_, e_, kb0_, KB, end_);
+                }
                 for (int kb = 0; kb < KB; ++kb, ++it) {
                     if ((it & 1u) != mine) continue;
                     last = it;
@@ -224,15 +252,16 @@ fp8_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
         bool alive = true;
         const bool vec_ok = (OUT == CINN_F32 || OUT == CINN_F32_BF16) ? (p.ldc % 4 == 0) : (p.ldc % 8 == 0);
         for (int t = cluster_id; t < n_total && alive; t += n_clusters) {
-            PairTile ti; int e, kb0, KB;
-            locate(t, ti, e, kb0, KB);
+            PairTile ti; int e, kb0, KB, m_end;
+            locate(t, ti, e, kb0, KB, m_end);
             const int row = ti.m0 + 128 * (int)rank + q * 32 + lane;
-            const bool rvalid = row < p.M;
+            const bool rvalid = row < m_end;
             const int col0 = ti.n0 + h * 128;
             const bool cvalid = col0 < p.N;
-            const float* sa_ptr = p.sA + (int64_t)(rvalid ? row : 0) * p.sa_stride_m + (int64_t)kb0 * p.sa_stride_k;
-            const float* sb_ptr = p.sB + (int64_t)(cvalid ? col0 / 128 : 0) * p.sb_stride_n + (int64_t)kb0 * p.sb_stride_k;
-            const int out_row0 = e * p.M;                      // GK: the expert's slice of the (E * M, N) output
+            const float* sa_ptr = p.sA + (int64_t)(rvalid ? row : (GR ? ti.m0 : 0)) * p.sa_stride_m + (int64_t)kb0 * p.sa_stride_k;
+            const float* sb_ptr = p.sB + (int64_t)(cvalid ? col0 / 128 : 0) * p.sb_stride_n + (int64_t)kb0 * p.sb_stride_k
+                                  + (GR ? (int64_t)e * p.sb_stride_e : 0);
+            const int out_row0 = GR ? 0 : e * p.M;                      // GK: the expert's slice of the (E * M, N) output
             float acc[128];
 #pragma unroll
             for (int i = 0; i < 128; ++i) acc[i] = 0.0f;
@@ -271,7 +300,23 @@ fp8_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
                 __syncwarp();
                 if (lane == 0) mbar_arrive_remote(tempty_leader + 8 * b);
             }
-            if (alive && p.tma_out) {
+            const bool whole = !GR || ti.m0 + 128 * (int)rank + 128 <= m_end;
+            if (alive && p.tma_out && !whole) {
+                // ragged tail: staged 16-byte stores through the group's slots, once the TMA unit has read them
+                const uint32_t par = n_rounds & 1u;
+                const bool elected = (warp == h * 4) && lane == 0;
+                if (elected) tma_store_wait_read();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(gfree0 + 8 * h);
+                if (!mbar_wait_warp(gfree0 + 8 * h, par, abort_flag, (3 << 8) | 2)) { alive = false; break; }
+                if (cvalid && vec_ok)
+                    store_rows_staged<OUT, 128>(acc, c_stage + h * 2 * C_SLOT_BYTES + q * 2048, p.C, p.ldc,
+                                                ti.m0 + 128 * (int)rank + q * 32, m_end, col0, p.N, lane);
+                if (lane == 0) mbar_arrive(gfull0 + 8 * h);
+                if (elected) mbar_wait(gfull0 + 8 * h, par, abort_flag, (3 << 8) | 3);
+                __syncwarp();
+                ++n_rounds;
+            } else if (alive && p.tma_out) {
                 // The tile leaves through TMA stores.  Each column group of four promotion warps owns two 16 KiB slots
                 // (boxes of 128 rows x 128 bytes, 128-byte swizzle): its threads drop their rows into them in 16-byte
                 // chunks and one thread hands the boxes to the TMA unit.  A 2-byte output fits the group's 128 columns
@@ -317,7 +362,7 @@ fp8_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
                 if (!alive) break;
             } else if (alive && vec_ok) {
                 if (cvalid) store_rows_staged<OUT, 128>(acc, store_stage + warp * 2048, p.C, p.ldc,
-                                                        out_row0 + ti.m0 + 128 * (int)rank + q * 32, out_row0 + p.M, col0, p.N, lane);
+                                                        out_row0 + ti.m0 + 128 * (int)rank + q * 32, out_row0 + m_end, col0, p.N, lane);
             } else if (alive && rvalid && cvalid) {
                 const int64_t base = (int64_t)(out_row0 + row) * p.ldc + col0;
 #pragma unroll

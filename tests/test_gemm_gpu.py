@@ -299,6 +299,27 @@ def test_grouped_gemm(K, name):
     assert rel.median().item() < 0.08
 
 
+@pytest.mark.parametrize("case", [(3, 384, 4096, [700, 0, 900]), (2, 256, 9480, [257, 511]), (2, 144, 4872, [1, 1280]), (1, 128, 5000, [1152])])
+def test_grouped_gemm_on_sm_pairs(K, case):
+    """Enough rows per expert for the two-SM kernel: tiles whose second half is empty, full or cut anywhere, an expert
+    without rows, columns that are no multiple of a tile, every way out (TMA boxes, staged tails, 2- and 4-byte types)."""
+    E, d_in, d_out, counts = case
+    x, w, starts, ends = _grouped_case(E, d_in, d_out, counts, seed=d_out, gap=9)
+    ref = O.grouped_gemm_fp8_f64(x, w, starts, ends)
+    xq, xs = K.quantize_fp8_rowwise(x.cuda())
+    wq, ws = K.quantize_expert_weights(w.cuda())
+    T, used = x.shape[0], int(ends[-1])
+    covered = torch.zeros(T, dtype=torch.bool)
+    for s, e in zip(starts.tolist(), ends.tolist()):
+        covered[s:e] = True
+    for dtype in (torch.float32, torch.bfloat16, torch.float16):
+        out = torch.full((T, d_out), 777.0, dtype=dtype, device="cuda")
+        K.fp8_grouped_gemm(xq, xs, wq, ws, starts.cuda(), ends.cuda(), out=out)
+        got = out.cpu()
+        assert torch.all(got[~covered] == 777.0), "rows outside every expert's range were written"
+        assert rel_fro(got[covered].float(), ref[covered]) <= {torch.float32: 2e-5, torch.bfloat16: 2e-3, torch.float16: 3e-4}[dtype]
+
+
 @pytest.mark.parametrize("name", list(GROUPED))
 @pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
 def test_grouped_gemm_16bit(K, name, dtype):
