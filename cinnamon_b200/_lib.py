@@ -44,6 +44,8 @@ SIGNATURES = {
     "cinn_moe_combine_backward": [_vp, _i32, _vp, _vp, _vp, _vp, _vp, _i64, _i64, _i32, _i64, _vp],
     "cinn_moe_route_workspace_ints": [_i64, _i32],
     "cinn_moe_route": [_vp, _vp, _i64, _i32, _i32, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp],
+    "cinn_moe_route_ranges": [_vp, _i32, _vp, _i64, _i32, _i32] + [_vp] * 12,
+    "cinn_spread_rows": [_vp, _vp, _vp, _vp, _vp, _i64, _i64, _i32, _i64, _i64, _vp],
     "cinn_moe_route_static_max_ints": [],
     "cinn_moe_route_static": [_vp, _vp, _i64, _i32, _i32, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp],
     "cinn_gather_rows": [_vp, _vp, _vp, _vp, _vp, _i64, _i64, _i64, _i64, _vp],

@@ -19,7 +19,7 @@ LIB_PATH = os.path.join(LIB_DIR, "libcinnamon_b200.so")
 SOURCES = ["quant.cu", "gemm.cu", "moe.cu", "route.cu", "sparse_attn.cu", "attn_tc.cu", "indexer.cu", "wgrad.cu", "capi.cu"]
 HOST_DIR = os.path.join(CSRC, "host")
 HOST_PATH = os.path.join(LIB_DIR, "_host.so")
-HOST_SOURCES = ["linear.cpp", "attention.cpp", "module.cpp"]
+HOST_SOURCES = ["linear.cpp", "attention.cpp", "moe.cpp", "module.cpp"]
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
     "-Xcompiler", "-fPIC", "--expt-relaxed-constexpr",

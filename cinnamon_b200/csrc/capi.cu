@@ -113,9 +113,11 @@ int quantize_block_t(const void* x, int dtype, int64_t M, int64_t N, int64_t ld,
                      int round_scale, int div_mode, cudaStream_t st);
 int swiglu(const void* h12, const void* dh, void* out, int dtype, int64_t T_rows, int64_t I, int backward, cudaStream_t st);
 int64_t moe_route_workspace_ints(int64_t T, int E);
-int moe_route(const float* logits, const float* bias, int64_t T, int E, int top_k, int* workspace, int* top_experts,
+int moe_route(const void* logits, int logits_dtype, const float* bias, int64_t T, int E, int top_k, int* workspace, int* top_experts,
               float* top_gates, int64_t* token_indices, float* sorted_scores, int64_t* sorted_experts, int64_t* counts,
-              int64_t* pair_pos, float* pair_gate, cudaStream_t st);
+              int64_t* starts, int64_t* ends, int64_t* pair_pos, float* pair_gate, cudaStream_t st);
+int spread_rows(const void* q, const float* s, const int64_t* pos, void* out_q, float* out_s, int64_t n_tokens, int64_t n_rows,
+                int top_k, int64_t d, int64_t ns, cudaStream_t st);
 int64_t moe_route_static_max_ints();
 int moe_route_static(const float* logits, const float* bias, int64_t T, int E, int top_k, int* top_experts, float* top_gates,
                      int64_t* token_indices, float* sorted_scores, int64_t* sorted_experts, int64_t* counts,
@@ -402,8 +404,21 @@ int64_t cinn_moe_route_workspace_ints(int64_t n_tokens, int n_experts) {
 int cinn_moe_route(const float* logits, const float* bias, int64_t n_tokens, int n_experts, int top_k, int* workspace,
                    int* top_experts, float* top_gates, int64_t* token_indices, float* sorted_scores,
                    int64_t* sorted_experts, int64_t* counts, int64_t* pair_pos, float* pair_gate, void* stream) {
-    return cinn::moe_route(logits, bias, n_tokens, n_experts, top_k, workspace, top_experts, top_gates, token_indices,
-                           sorted_scores, sorted_experts, counts, pair_pos, pair_gate, (cudaStream_t)stream);
+    return cinn::moe_route(logits, CINN_F32, bias, n_tokens, n_experts, top_k, workspace, top_experts, top_gates, token_indices,
+                           sorted_scores, sorted_experts, counts, nullptr, nullptr, pair_pos, pair_gate, (cudaStream_t)stream);
+}
+
+int cinn_moe_route_ranges(const void* logits, int logits_dtype, const float* bias, int64_t n_tokens, int n_experts, int top_k,
+                          int* workspace, int* top_experts, float* top_gates, int64_t* token_indices, float* sorted_scores,
+                          int64_t* sorted_experts, int64_t* counts, int64_t* starts, int64_t* ends, int64_t* pair_pos,
+                          float* pair_gate, void* stream) {
+    return cinn::moe_route(logits, logits_dtype, bias, n_tokens, n_experts, top_k, workspace, top_experts, top_gates, token_indices,
+                           sorted_scores, sorted_experts, counts, starts, ends, pair_pos, pair_gate, (cudaStream_t)stream);
+}
+
+int cinn_spread_rows(const void* q, const float* scales, const int64_t* pos, void* out_q, float* out_scales, int64_t n_tokens,
+                     int64_t n_rows, int top_k, int64_t d, int64_t n_scales, void* stream) {
+    return cinn::spread_rows(q, scales, pos, out_q, out_scales, n_tokens, n_rows, top_k, d, n_scales, (cudaStream_t)stream);
 }
 
 int64_t cinn_moe_route_static_max_ints(void) { return cinn::moe_route_static_max_ints(); }

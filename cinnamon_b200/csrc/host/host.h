@@ -24,7 +24,9 @@ using at::Tensor;
     X(cinn_last_error) X(cinn_quant_rowwise) X(cinn_quant_rowwise_dual) X(cinn_quant_rowwise_with_block)             \
     X(cinn_quant_rowwise_with_block_t) X(cinn_quant_blockwise) X(cinn_quant_blockwise_t) X(cinn_transpose_bytes)     \
     X(cinn_requant_row_to_block) X(cinn_fp8_gemm_ws) X(cinn_fp8_gemm_workspace_bytes) \
-    X(cinn_sparse_attn_workspace_bytes) X(cinn_sparse_attn_fwd_ws) X(cinn_sparse_attn_bwd) X(cinn_sparse_attn_bwd_ws)
+    X(cinn_sparse_attn_workspace_bytes) X(cinn_sparse_attn_fwd_ws) X(cinn_sparse_attn_bwd) X(cinn_sparse_attn_bwd_ws)                  \
+    X(cinn_moe_route_workspace_ints) X(cinn_moe_route_ranges) X(cinn_spread_rows) X(cinn_fp8_grouped_gemm)                \
+    X(cinn_swiglu_quant_rowwise) X(cinn_moe_combine) X(cinn_moe_combine_add)
 
 struct Api {
 #define CINN_DECL(name) decltype(&::name) name = nullptr;
@@ -65,6 +67,7 @@ void as_python_error(F&& body) {
     }
 }
 
+constexpr at::ScalarType F8 = at::kFloat8_e4m3fn;
 constexpr int TAG_BF16 = 0, TAG_F32 = 1, TAG_F16 = 2, TAG_F32_BF16 = 3;
 inline int tag_of(at::ScalarType t) {           // -1: not a type the kernels read
     switch (t) {
@@ -81,6 +84,9 @@ inline Tensor empty(at::IntArrayRef size, at::ScalarType type, const at::Device&
 }
 inline int64_t up(int64_t a, int64_t b) { return (a + b - 1) / b; }
 inline void* stream() { return at::cuda::getCurrentCUDAStream().stream(); }
+inline float* f32(const Tensor& t);
+Tensor gemm(const Tensor& a, const Tensor& sa, const Tensor& b, int layout, const Tensor& sb, int64_t sbk, int64_t sbn, int64_t M,
+            int64_t N, int64_t K, at::ScalarType type, int tag);               // linear.cpp
 inline float* f32(const Tensor& t) { return static_cast<float*>(t.data_ptr()); }
 
 }  // namespace cinnhost

@@ -4,15 +4,6 @@
 
 namespace cinnhost {
 
-namespace {
-
-constexpr at::ScalarType F8 = at::kFloat8_e4m3fn;
-
-struct Linear {                                 // what the forward leaves for the backward
-    Tensor out, x, x_scale, w, w_scale, w_t;
-    bool x_is_block = false, x_is_block_t = false;
-};
-
 Tensor gemm(const Tensor& a, const Tensor& sa, const Tensor& b, int layout, const Tensor& sb, int64_t sbk, int64_t sbn, int64_t M,
             int64_t N, int64_t K, at::ScalarType type, int tag) {
     Tensor out = empty({M, N}, type, a.device());
@@ -23,6 +14,13 @@ Tensor gemm(const Tensor& a, const Tensor& sa, const Tensor& b, int layout, cons
     launches += need ? 2 : 1;
     return out;
 }
+
+namespace {
+
+struct Linear {                                 // what the forward leaves for the backward
+    Tensor out, x, x_scale, w, w_scale, w_t;
+    bool x_is_block = false, x_is_block_t = false;
+};
 
 Linear forward(const Tensor& x, const Tensor& weight, bool round_scale, bool need_dgrad, bool need_wgrad, bool kmajor, int div,
                const Tensor& w_q, const Tensor& w_s, const Tensor& w_qt) {

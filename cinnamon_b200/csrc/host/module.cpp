@@ -6,6 +6,7 @@ Api api;
 std::atomic<int64_t> launches{0};
 void bind_linear(pybind11::module_& m);
 void bind_attention(pybind11::module_& m);
+void bind_moe(pybind11::module_& m);
 }  // namespace cinnhost
 
 PYBIND11_MODULE(_host, m) {
@@ -34,4 +35,5 @@ PYBIND11_MODULE(_host, m) {
     });
     bind_linear(m);
     bind_attention(m);
+    bind_moe(m);
 }

@@ -1,38 +1,54 @@
 // MoE routing on the device: top-k selection and the stable sort of (token, expert) pairs by expert.
 //
 // Replaces the chain of torch calls at the head of cinnamon's MoE.forward (src/layers.py:122-148):
-// sigmoid, + expert_bias, topk, gather, normalise, sort by expert, token_indices, bincount.  Three launches:
+// sigmoid, + expert_bias, topk, gather, normalise, sort by expert, token_indices, bincount.  Two or three launches:
 //
 //   route_topk_kernel     one warp per token: sigmoid scores, the k largest of score + bias (ties: the lower
-//                         expert id), gates = score / (sum of the k scores + 1e-9); every CTA of 128 tokens also
-//                         leaves a histogram of the experts it selected in the workspace
-//   route_scan_kernel     one CTA: per expert, the running sum of those histograms over the CTAs (the
-//                         histograms become offsets) -> counts; exclusive scan over experts -> first row
-//   route_scatter_kernel  the same CTAs again: every pair gets the next free row of its expert, pairs taken in
-//                         (token, slot) order, so the order is that of a stable sort and the same on every
-//                         run; writes token_indices / sorted_scores / sorted_experts, and per token its k rows
-//                         in ascending order with their gates (what the combine pass reads)
+//                         expert id), gates = score / (sum of the k scores + 1e-9); every CTA also leaves a histogram
+//                         of the experts its tokens selected in the workspace
+//   route_scan_kernel     one warp per expert: the running sum of those histograms over the CTAs (the histograms
+//                         become offsets) -> counts.  With 32 CTAs or fewer the scatter kernel does this itself.
+//   route_scatter_kernel  the same CTAs again: an exclusive scan of the counts gives every expert's first row, and every
+//                         pair gets the next free row of its expert, pairs taken in (token, slot) order, so the order is
+//                         that of a stable sort and the same on every run; writes token_indices / sorted_scores /
+//                         sorted_experts, the experts' row ranges, and per token its k rows in ascending order with their
+//                         gates (what the combine pass reads)
 //
-// The workspace (ceil(T / 128) * E ints) is the only memory beyond inputs and outputs.
+// Tokens per CTA: 8 (one per warp) as long as the histograms stay below 131072 counters, then 32 up to 262144, then 128.  Selecting the top k is a
+// serial chain of shuffles per token, so what counts is how many warps there are: 64 tokens in one CTA took 38 us.
+//
+// The workspace (one int per CTA and expert, and one more per expert) is the only memory beyond inputs and outputs.
 #include "common.cuh"
 #include <mutex>
 
 namespace cinn {
 
-constexpr int ROUTE_TOKENS_PER_CTA = 128;
+constexpr int ROUTE_MAX_TOKENS_PER_CTA = 128;
+constexpr int ROUTE_FEW_CTAS = 32;             // up to here the scatter kernel sums the histograms itself
+static inline int route_tokens_per_cta(int64_t T, int E) {
+    if (T <= 8 * 1024 && (T + 7) / 8 * E <= 131072) return 8;
+    if (T <= 32 * 1024 && (T + 31) / 32 * E <= 262144) return 32;
+    return 128;
+}
+
+template <typename L> __device__ __forceinline__ float logit(L v);
+template <> __device__ __forceinline__ float logit<float>(float v) { return v; }
+template <> __device__ __forceinline__ float logit<__nv_bfloat16>(__nv_bfloat16 v) { return __bfloat162float(v); }
+template <> __device__ __forceinline__ float logit<__half>(__half v) { return __half2float(v); }
+
 constexpr int ROUTE_MAX_EXPERTS = 1024;
 constexpr int ROUTE_MAX_TOPK = 32;
 
-template <int VPL>      // expert values per lane, E <= 32 * VPL
+template <int VPL, typename L>      // expert values per lane, E <= 32 * VPL
 __global__ void __launch_bounds__(256)
-route_topk_kernel(const float* __restrict__ logits, const float* __restrict__ bias, int T, int E, int top_k,
+route_topk_kernel(const L* __restrict__ logits, const float* __restrict__ bias, int T, int E, int top_k, int tokens_per_cta,
                   int* __restrict__ top_experts, float* __restrict__ top_gates, int* __restrict__ hist) {
     __shared__ int s_hist[ROUTE_MAX_EXPERTS];
     for (int e = threadIdx.x; e < E; e += 256) s_hist[e] = 0;
     __syncthreads();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int t_begin = blockIdx.x * ROUTE_TOKENS_PER_CTA;
-    const int t_end = min(t_begin + ROUTE_TOKENS_PER_CTA, T);
+    const int t_begin = blockIdx.x * tokens_per_cta;
+    const int t_end = min(t_begin + tokens_per_cta, T);
     float b[VPL];
 #pragma unroll
     for (int i = 0; i < VPL; ++i) b[i] = (lane + 32 * i < E) ? bias[lane + 32 * i] : 0.0f;
@@ -42,7 +58,7 @@ route_topk_kernel(const float* __restrict__ logits, const float* __restrict__ bi
         for (int i = 0; i < VPL; ++i) {
             const int e = lane + 32 * i;
             if (e < E) {
-                const float x = logits[(int64_t)t * E + e];
+                const float x = logit<L>(logits[(int64_t)t * E + e]);
                 s[i] = __fdiv_rn(1.0f, 1.0f + expf(-x));                  // torch.sigmoid in fp32
                 sel[i] = s[i] + b[i];
                 if (sel[i] != sel[i]) sel[i] = -INFINITY;                  // a NaN is never selected
@@ -88,50 +104,101 @@ route_topk_kernel(const float* __restrict__ logits, const float* __restrict__ bi
     for (int e = threadIdx.x; e < E; e += 256) hist[(int64_t)blockIdx.x * E + e] = s_hist[e];
 }
 
-__global__ void __launch_bounds__(1024)
-route_scan_kernel(int* __restrict__ hist, int n_ctas, int E, int64_t* __restrict__ counts, int* __restrict__ first_row) {
-    __shared__ int s_scan[ROUTE_MAX_EXPERTS];
-    const int e = threadIdx.x;
-    int total = 0;
-    if (e < E) {
-        for (int b = 0; b < n_ctas; ++b) {
-            const int v = hist[(int64_t)b * E + e];
-            hist[(int64_t)b * E + e] = total;
-            total += v;
+__global__ void __launch_bounds__(256)
+route_scan_kernel(int* __restrict__ hist, int n_ctas, int E, int* __restrict__ totals) {
+    const int lane = threadIdx.x & 31, e = blockIdx.x * 8 + (threadIdx.x >> 5);
+    if (e >= E) return;
+    int carry = 0;
+    for (int b0 = 0; b0 < n_ctas; b0 += 128) {               // four histograms per lane in flight
+        int v[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            const int b = b0 + u * 32 + lane;
+            v[u] = b < n_ctas ? hist[(int64_t)b * E + e] : 0;
         }
-        counts[e] = total;
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            const int b = b0 + u * 32 + lane;
+            int incl = v[u];
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int x = __shfl_up_sync(0xffffffffu, incl, o);
+                if (lane >= o) incl += x;
+            }
+            if (b < n_ctas) hist[(int64_t)b * E + e] = carry + incl - v[u];
+            carry += __shfl_sync(0xffffffffu, incl, 31);
+        }
     }
-    s_scan[e] = e < E ? total : 0;
-    __syncthreads();
-    // inclusive scan over experts (Hillis-Steele; E <= 1024 = blockDim)
-    for (int o = 1; o < 1024; o <<= 1) {
-        const int v = e >= o ? s_scan[e - o] : 0;
-        __syncthreads();
-        s_scan[e] += v;
-        __syncthreads();
-    }
-    if (e < E) first_row[e] = s_scan[e] - total;
+    if (lane == 0) totals[e] = carry;
 }
 
+// totals: per-expert counts from route_scan_kernel, with `hist` turned into offsets; null: hist still holds counts
 __global__ void __launch_bounds__(256)
 route_scatter_kernel(const int* __restrict__ top_experts, const float* __restrict__ top_gates, const int* __restrict__ hist,
-                     const int* __restrict__ first_row, int T, int E, int top_k, int64_t* __restrict__ token_indices,
-                     float* __restrict__ sorted_scores, int64_t* __restrict__ sorted_experts,
-                     int64_t* __restrict__ pair_pos, float* __restrict__ pair_gate) {
+                     const int* __restrict__ totals, int T, int E, int top_k, int tokens_per_cta, int64_t* __restrict__ token_indices,
+                     float* __restrict__ sorted_scores, int64_t* __restrict__ sorted_experts, int64_t* __restrict__ counts,
+                     int64_t* __restrict__ starts, int64_t* __restrict__ ends, int64_t* __restrict__ pair_pos,
+                     float* __restrict__ pair_gate) {
     __shared__ int s_next[ROUTE_MAX_EXPERTS];                                  // next free row of every expert
-    __shared__ int s_pos[ROUTE_TOKENS_PER_CTA * ROUTE_MAX_TOPK];
-    for (int e = threadIdx.x; e < E; e += 256) s_next[e] = first_row[e] + hist[(int64_t)blockIdx.x * E + e];
+    __shared__ int s_warp[8];
+    __shared__ int s_pos[ROUTE_MAX_TOKENS_PER_CTA * ROUTE_MAX_TOPK];
+    {
+        // thread i: experts 4 i .. 4 i + 3; their counts, the rows of earlier CTAs, and a scan of the counts
+        int cnt[4], mine[4], sum = 0;
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            const int e = threadIdx.x * 4 + u;
+            cnt[u] = 0; mine[u] = 0;
+            if (e < E) {
+                if (totals) {
+                    cnt[u] = totals[e];
+                    mine[u] = hist[(int64_t)blockIdx.x * E + e];
+                } else {
+                    for (int b = 0; b < (int)gridDim.x; ++b) {
+                        const int v = hist[(int64_t)b * E + e];
+                        if (b < (int)blockIdx.x) mine[u] += v;
+                        cnt[u] += v;
+                    }
+                }
+            }
+            sum += cnt[u];
+        }
+        const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+        int incl = sum;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int x = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= o) incl += x;
+        }
+        if (lane == 31) s_warp[warp] = incl;
+        __syncthreads();
+        int first = incl - sum;
+        for (int w = 0; w < warp; ++w) first += s_warp[w];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            const int e = threadIdx.x * 4 + u;
+            if (e < E) {
+                s_next[e] = first + mine[u];
+                if (blockIdx.x == 0) {
+                    counts[e] = cnt[u];
+                    if (starts) { starts[e] = first; ends[e] = first + cnt[u]; }
+                }
+                first += cnt[u];
+            }
+        }
+    }
     __syncthreads();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int t_begin = blockIdx.x * ROUTE_TOKENS_PER_CTA;
-    const int n_tok = min(ROUTE_TOKENS_PER_CTA, T - t_begin);
+    const int t_begin = blockIdx.x * tokens_per_cta;
+    const int n_tok = min(tokens_per_cta, T - t_begin);
     const int n_pairs = n_tok * top_k;
     const int64_t pair0 = (int64_t)t_begin * top_k;
     for (int base = 0; base < n_pairs; base += 256) {
         const int p = base + threadIdx.x;
         const bool live = p < n_pairs;
         const int e = live ? top_experts[pair0 + p] : -1 - lane;              // dead lanes match nobody
-        for (int w = 0; w < 8; ++w) {                                          // warps take their turn: (token, slot) order
+        const int turns = min(8, (n_pairs - base + 31) / 32);
+        for (int w = 0; w < turns; ++w) {                                      // warps take their turn: (token, slot) order
             if (warp == w) {
                 const unsigned peers = __match_any_sync(0xffffffffu, e);
                 const int leader = __ffs(peers) - 1;
@@ -171,27 +238,14 @@ route_scatter_kernel(const int* __restrict__ top_experts, const float* __restric
 }
 
 int64_t moe_route_workspace_ints(int64_t T, int E) {
-    return ((T + ROUTE_TOKENS_PER_CTA - 1) / ROUTE_TOKENS_PER_CTA) * (int64_t)E + E;
+    const int per = route_tokens_per_cta(T, E);
+    return ((T + per - 1) / per) * (int64_t)E + E;
 }
 
-int moe_route(const float* logits, const float* bias, int64_t T, int E, int top_k, int* workspace, int* top_experts,
-              float* top_gates, int64_t* token_indices, float* sorted_scores, int64_t* sorted_experts, int64_t* counts,
-              int64_t* pair_pos, float* pair_gate, cudaStream_t st) {
-    CINN_CHECK_ARG(T >= 0 && E >= 1 && E <= ROUTE_MAX_EXPERTS, "moe_route: 1 <= E <= %d experts (got %d)", ROUTE_MAX_EXPERTS, E);
-    CINN_CHECK_ARG(top_k >= 1 && top_k <= ROUTE_MAX_TOPK && top_k <= E, "moe_route: 1 <= top_k <= min(E, %d) (got %d)",
-                   ROUTE_MAX_TOPK, top_k);
-    CINN_CHECK_ARG(T * (int64_t)top_k < (1LL << 31), "moe_route: too many (token, expert) pairs");
-    CINN_CHECK_ARG(counts != nullptr, "moe_route: null pointer");
-    if (T == 0) {
-        CINN_CHECK_CUDA(cudaMemsetAsync(counts, 0, sizeof(int64_t) * E, st));
-        return CINN_OK;
-    }
-    CINN_CHECK_ARG(logits && bias && workspace && top_experts && top_gates && token_indices && sorted_scores &&
-                   sorted_experts && pair_pos && pair_gate, "moe_route: null pointer");
-    const int n_ctas = (int)((T + ROUTE_TOKENS_PER_CTA - 1) / ROUTE_TOKENS_PER_CTA);
-    int* hist = workspace;
-    int* first_row = workspace + (int64_t)n_ctas * E;
-#define CINN_TOPK(V) route_topk_kernel<V><<<n_ctas, 256, 0, st>>>(logits, bias, (int)T, E, top_k, top_experts, top_gates, hist)
+template <typename L>
+static void launch_topk(const L* logits, const float* bias, int T, int E, int top_k, int per, int n_ctas, int* top_experts,
+                        float* top_gates, int* hist, cudaStream_t st) {
+#define CINN_TOPK(V) route_topk_kernel<V, L><<<n_ctas, 256, 0, st>>>(logits, bias, T, E, top_k, per, top_experts, top_gates, hist)
     if (E <= 32) CINN_TOPK(1);
     else if (E <= 64) CINN_TOPK(2);
     else if (E <= 128) CINN_TOPK(4);
@@ -199,11 +253,42 @@ int moe_route(const float* logits, const float* bias, int64_t T, int E, int top_
     else if (E <= 512) CINN_TOPK(16);
     else CINN_TOPK(32);
 #undef CINN_TOPK
+}
+
+// logits_dtype: CINN_F32, or a 16-bit type that is widened on load.  starts / ends (E each): null, or every expert's rows.
+int moe_route(const void* logits, int logits_dtype, const float* bias, int64_t T, int E, int top_k, int* workspace, int* top_experts,
+              float* top_gates, int64_t* token_indices, float* sorted_scores, int64_t* sorted_experts, int64_t* counts,
+              int64_t* starts, int64_t* ends, int64_t* pair_pos, float* pair_gate, cudaStream_t st) {
+    CINN_CHECK_ARG(T >= 0 && E >= 1 && E <= ROUTE_MAX_EXPERTS, "moe_route: 1 <= E <= %d experts (got %d)", ROUTE_MAX_EXPERTS, E);
+    CINN_CHECK_ARG(top_k >= 1 && top_k <= ROUTE_MAX_TOPK && top_k <= E, "moe_route: 1 <= top_k <= min(E, %d) (got %d)",
+                   ROUTE_MAX_TOPK, top_k);
+    CINN_CHECK_ARG(T * (int64_t)top_k < (1LL << 31), "moe_route: too many (token, expert) pairs");
+    CINN_CHECK_ARG(counts != nullptr && (starts == nullptr) == (ends == nullptr), "moe_route: null pointer");
+    CINN_CHECK_ARG(logits_dtype == CINN_F32 || logits_dtype == CINN_BF16 || logits_dtype == CINN_F16, "moe_route: unknown dtype tag %d",
+                   logits_dtype);
+    if (T == 0) {
+        CINN_CHECK_CUDA(cudaMemsetAsync(counts, 0, sizeof(int64_t) * E, st));
+        if (starts) {
+            CINN_CHECK_CUDA(cudaMemsetAsync(starts, 0, sizeof(int64_t) * E, st));
+            CINN_CHECK_CUDA(cudaMemsetAsync(ends, 0, sizeof(int64_t) * E, st));
+        }
+        return CINN_OK;
+    }
+    CINN_CHECK_ARG(logits && bias && workspace && top_experts && top_gates && token_indices && sorted_scores &&
+                   sorted_experts && pair_pos && pair_gate, "moe_route: null pointer");
+    const int per = route_tokens_per_cta(T, E), n_ctas = (int)((T + per - 1) / per);
+    int* hist = workspace;
+    int* totals = n_ctas > ROUTE_FEW_CTAS ? workspace + (int64_t)n_ctas * E : nullptr;
+    if (logits_dtype == CINN_F32) launch_topk((const float*)logits, bias, (int)T, E, top_k, per, n_ctas, top_experts, top_gates, hist, st);
+    else if (logits_dtype == CINN_BF16) launch_topk((const __nv_bfloat16*)logits, bias, (int)T, E, top_k, per, n_ctas, top_experts, top_gates, hist, st);
+    else launch_topk((const __half*)logits, bias, (int)T, E, top_k, per, n_ctas, top_experts, top_gates, hist, st);
     CINN_CHECK_LAUNCH();
-    route_scan_kernel<<<1, 1024, 0, st>>>(hist, n_ctas, E, counts, first_row);
-    CINN_CHECK_LAUNCH();
-    route_scatter_kernel<<<n_ctas, 256, 0, st>>>(top_experts, top_gates, hist, first_row, (int)T, E, top_k, token_indices,
-                                                 sorted_scores, sorted_experts, pair_pos, pair_gate);
+    if (totals) {
+        route_scan_kernel<<<(E + 7) / 8, 256, 0, st>>>(hist, n_ctas, E, totals);
+        CINN_CHECK_LAUNCH();
+    }
+    route_scatter_kernel<<<n_ctas, 256, 0, st>>>(top_experts, top_gates, hist, totals, (int)T, E, top_k, per, token_indices, sorted_scores,
+                                                 sorted_experts, counts, starts, ends, pair_pos, pair_gate);
     CINN_CHECK_LAUNCH();
     return CINN_OK;
 }
@@ -253,8 +338,8 @@ int moe_route_static(const float* logits, const float* bias, int64_t T, int E, i
     int* scratch = nullptr;
     int rc = route_scratch_address(&scratch);
     if (rc) return rc;
-    return moe_route(logits, bias, T, E, top_k, scratch, top_experts, top_gates, token_indices, sorted_scores,
-                     sorted_experts, counts, pair_pos, pair_gate, st);
+    return moe_route(logits, CINN_F32, bias, T, E, top_k, scratch, top_experts, top_gates, token_indices, sorted_scores,
+                     sorted_experts, counts, nullptr, nullptr, pair_pos, pair_gate, st);
 }
 
 }  // namespace cinn

@@ -930,14 +930,14 @@ def p2p_return(rows, seg_start, home_base, peer_home, n_ranks: int, capacity_row
 
 
 def moe_route(logits: torch.Tensor, bias: torch.Tensor, top_k: int):
-    """Routing of ``MoE.forward`` (reference src/layers.py:122-148) from the router's fp32 logits, on the
+    """Routing of ``MoE.forward`` (reference src/layers.py:122-148) from the router's logits (evaluated in fp32), on the
     device and without a host synchronisation: sigmoid scores, top-k of score + bias, normalised gates, and the
     (token, expert) pairs in the order of a stable sort by expert.  Returns a dict of tensors:
     ``top_experts`` (T, k) int32, ``top_gates`` (T, k), ``token_indices`` / ``sorted_scores`` /
-    ``sorted_experts`` (T*k), ``counts`` (E) int64, ``pair_pos`` / ``pair_gate`` (T, k)."""
+    ``sorted_experts`` (T*k), ``counts`` and the row ranges ``starts`` / ``ends`` (E) int64, ``pair_pos`` / ``pair_gate`` (T, k)."""
     assert logits.is_cuda and bias.is_cuda, "Inputs must be on CUDA"
     assert logits.ndim == 2, "logits must be (tokens, experts)"
-    logits = logits.float().contiguous()
+    logits = (logits if logits.dtype in _DTYPE_TAG else logits.float()).contiguous()
     bias = bias.float().contiguous()
     T, E = logits.shape
     dev = logits.device
@@ -950,13 +950,16 @@ def moe_route(logits: torch.Tensor, bias: torch.Tensor, top_k: int):
             "sorted_scores": torch.empty(T * top_k, dtype=torch.float32, device=dev),
             "sorted_experts": torch.empty(T * top_k, dtype=torch.int64, device=dev),
             "counts": torch.empty(E, dtype=torch.int64, device=dev),
+            "starts": torch.empty(E, dtype=torch.int64, device=dev),
+            "ends": torch.empty(E, dtype=torch.int64, device=dev),
             "pair_pos": torch.empty((T, top_k), dtype=torch.int64, device=dev),
             "pair_gate": torch.empty((T, top_k), dtype=torch.float32, device=dev),
         }
-        _lib.check(_L.cinn_moe_route(_ptr(logits), _ptr(bias), T, E, top_k, _ptr(ws), _ptr(out["top_experts"]),
-                                     _ptr(out["top_gates"]), _ptr(out["token_indices"]), _ptr(out["sorted_scores"]),
-                                     _ptr(out["sorted_experts"]), _ptr(out["counts"]), _ptr(out["pair_pos"]),
-                                     _ptr(out["pair_gate"]), _stream(logits)), "cinn_moe_route")
+        _lib.check(_L.cinn_moe_route_ranges(_ptr(logits), _DTYPE_TAG[logits.dtype], _ptr(bias), T, E, top_k, _ptr(ws),
+                                            _ptr(out["top_experts"]), _ptr(out["top_gates"]), _ptr(out["token_indices"]),
+                                            _ptr(out["sorted_scores"]), _ptr(out["sorted_experts"]), _ptr(out["counts"]),
+                                            _ptr(out["starts"]), _ptr(out["ends"]), _ptr(out["pair_pos"]), _ptr(out["pair_gate"]),
+                                            _stream(logits)), "cinn_moe_route")
     _count(3)
     return out
 

@@ -44,7 +44,8 @@ def router_logits(x: torch.Tensor, router_weight: torch.Tensor) -> torch.Tensor:
     activations, scores in fp32 afterwards."""
     if x.dtype in (torch.bfloat16, torch.float16):
         w = router_weight if router_weight.dtype == x.dtype else router_weight.to(x.dtype)
-        return torch.nn.functional.linear(x, w).float()
+        logits = torch.nn.functional.linear(x, w)
+        return logits if logits.is_cuda else logits.float()         # (the routing kernel widens them itself)
     return torch.nn.functional.linear(x.float(), router_weight.float())
 
 
@@ -724,6 +725,15 @@ class ExpertParallelMoE(torch.nn.Module):
     def forward(self, x: torch.Tensor) -> torch.Tensor:
         flat = x.reshape(-1, x.shape[-1])
         router = self._router_as(flat.dtype)
+        if (flat.is_cuda and self.trace is None and self.K.gemm_events is None and flat.shape[1] % 16 == 0
+                and flat.dtype in self.K._DTYPE_TAG and isinstance(self.shared, (FP8SwiGLU, type(None)))
+                and isinstance(self.experts, FP8Experts) and (not dist.is_initialized() or dist.get_world_size(self.group) == 1)):
+            # one GPU: the sequence below as one native call (csrc/host/moe.cpp)
+            e, sh = self.experts, self.shared
+            shared = (None,) * 4 if sh is None else (sh.w12_q, sh.w12_s, sh.w3_q, sh.w3_s)
+            y = self.K._host.moe_forward(flat.contiguous(), router, self.expert_bias, self.top_k, e.w12_q, e.w12_s, e.w3_q, e.w3_s,
+                                         *shared, sh is not None and sh.round_scale, self.K._DIV_MODE)
+            return y.reshape(x.shape)
         world = dist.get_world_size(self.group) if dist.is_initialized() else 1
         sh, join = None, None
         if self.trace is not None and flat.is_cuda:

@@ -296,6 +296,11 @@ int cinn_swiglu_backward(const void* h12, const void* grad_h, void* grad_h12, in
 int cinn_gather_rows(const void* q, const float* scales, const int64_t* idx, void* out_q, float* out_scales, int64_t n_out,
                      int64_t n_src, int64_t d, int64_t n_scales, void* stream);
 
+/* The same dispatch from the tokens' side: token t's bytes and scales are written to rows pos[t, j], j < top_k (n_rows rows;
+ * places outside are skipped).  Every token is read once. */
+int cinn_spread_rows(const void* q, const float* scales, const int64_t* pos, void* out_q, float* out_scales, int64_t n_tokens,
+                     int64_t n_rows, int top_k, int64_t d, int64_t n_scales, void* stream);
+
 /* Row scatter: out[idx[r], :] = in[r, :] for r < n_rows; rows of row_bytes bytes (a multiple of 16), out has
  * n_dst rows, entries of idx outside [0, n_dst) are skipped.  Brings the expert outputs of an expert-parallel
  * rank from the expert-grouped order back to the order in which the rows arrived, before they travel home
@@ -409,6 +414,13 @@ int64_t cinn_moe_route_workspace_ints(int64_t n_tokens, int n_experts);
 int cinn_moe_route(const float* logits, const float* bias, int64_t n_tokens, int n_experts, int top_k, int* workspace,
                    int* top_experts, float* top_gates, int64_t* token_indices, float* sorted_scores,
                    int64_t* sorted_experts, int64_t* counts, int64_t* pair_pos, float* pair_gate, void* stream);
+
+/* The same from logits of any float type (`logits_dtype`; 16-bit logits are widened on load), which also leaves every
+ * expert's range of sorted rows in starts / ends (n_experts each, or both null): what the grouped GEMMs read. */
+int cinn_moe_route_ranges(const void* logits, int logits_dtype, const float* bias, int64_t n_tokens, int n_experts, int top_k,
+                          int* workspace, int* top_experts, float* top_gates, int64_t* token_indices, float* sorted_scores,
+                          int64_t* sorted_experts, int64_t* counts, int64_t* starts, int64_t* ends, int64_t* pair_pos,
+                          float* pair_gate, void* stream);
 
 /* cinn_moe_route for callers that have no device memory to give as a workspace and may not allocate any: a
  * serving process that handed all of HBM to its own arena at start-up, a job running at the memory limit, a

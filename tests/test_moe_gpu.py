@@ -134,6 +134,35 @@ def test_route_kernel_matches_torch(K, T, E, k):
         assert torch.equal(got[key], again[key]), key
 
 
+@pytest.mark.parametrize("T,E,k", [(8, 256, 8), (256, 33, 2), (257, 256, 8), (5000, 64, 3), (8300, 1024, 4), (40000, 16, 2)])
+def test_route_cta_sizes_and_row_ranges(K, T, E, k):
+    """8, 32 and 128 tokens per CTA, with and without the scan launch; 16-bit logits as their fp32 values; row ranges."""
+    g = torch.Generator(device="cuda").manual_seed(T + E + k)
+    logits = torch.randn(T, E, generator=g, device="cuda").bfloat16()
+    bias = torch.randn(E, generator=g, device="cuda") * 0.3
+    got, ref = K.moe_route(logits, bias, k), K.moe_route(logits.float(), bias, k)
+    assert all(torch.equal(got[n], ref[n]) for n in got)
+    order = got["top_experts"].reshape(-1).long().sort(stable=True)
+    assert torch.equal(got["sorted_experts"], order.values) and torch.equal(got["token_indices"], order.indices // k)
+    assert torch.equal(got["ends"], got["counts"].cumsum(0)) and torch.equal(got["starts"], got["ends"] - got["counts"])
+
+
+@pytest.mark.parametrize("T,d,shared,rs", [(1, 256, True, False), (70, 272, True, True), (300, 512, False, False)])
+def test_native_layer_matches_its_parts(K, T, d, shared, rs):
+    """The one-GPU layer as one native call against the same layer run part by part (what a traced call does)."""
+    from cinnamon_b200 import moe
+    g = torch.Generator().manual_seed(T + d)
+    E, I, k = 8, 128, 3
+    w = lambda *s: (torch.randn(*s, generator=g) * 0.05).bfloat16().cuda()                       # noqa: E731
+    sh = moe.FP8SwiGLU(w(I, d), w(I, d), w(d, I), round_scale=rs) if shared else None
+    layer = moe.ExpertParallelMoE(w(E, d).float(), torch.randn(E, generator=g).cuda() * 0.1, w(E, 2 * I, d), w(E, d, I), k, shared=sh)
+    x = torch.randn(T, d, generator=g).bfloat16().cuda()
+    y = layer(x)
+    layer.trace = []
+    assert torch.equal(y, layer(x)) and len(layer.trace) > 3
+    assert layer(x[:0]).shape == (0, d)
+
+
 def test_gather_quantized_rows(K):
     g = torch.Generator().manual_seed(5)
     q = torch.randint(0, 256, (300, 512), generator=g, dtype=torch.uint8).cuda().view(torch.float8_e4m3fn)
