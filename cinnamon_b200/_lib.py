@@ -45,6 +45,12 @@ SIGNATURES = {
     "cinn_moe_route_workspace_ints": [_i64, _i32],
     "cinn_moe_route": [_vp, _vp, _i64, _i32, _i32, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp],
     "cinn_moe_route_ranges": [_vp, _i32, _vp, _i64, _i32, _i32] + [_vp] * 12,
+    "cinn_swiglu_rounded": [_vp, _vp, _i32, _i64, _i64, _vp],
+    "cinn_swiglu_rounded_backward": [_vp, _vp, _vp, _i32, _i64, _i64, _vp],
+    "cinn_moe_balance_workspace_bytes": [_i64, _i64, _i32],
+    "cinn_moe_balance_loss": [_vp, _i32, _vp, _i64, _i64, _i32, _i32, ctypes.c_float, _vp, _vp, _vp, _vp],
+    "cinn_moe_gates_backward": [_vp, _i32, _vp, _vp, _vp, _vp, _vp, ctypes.c_float, _i64, _i64, _i32, _i32, _vp, _vp],
+    "cinn_moe_update_bias": [_vp, _vp, _i32, ctypes.c_float, ctypes.c_float, _vp],
     "cinn_spread_rows": [_vp, _vp, _vp, _vp, _vp, _i64, _i64, _i32, _i64, _i64, _vp],
     "cinn_moe_route_static_max_ints": [],
     "cinn_moe_route_static": [_vp, _vp, _i64, _i32, _i32, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp],
@@ -98,7 +104,7 @@ def _load() -> ctypes.CDLL:
         fn.argtypes = argtypes
         fn.restype = (ctypes.c_char_p if name == "cinn_last_error"
                       else ctypes.c_longlong if name == "cinn_set_wait_limit_cycles"
-                      else ctypes.c_int64 if name in ("cinn_moe_route_workspace_ints", "cinn_moe_route_static_max_ints", "cinn_fp8_gemm_workspace_bytes",
+                      else ctypes.c_int64 if name in ("cinn_moe_route_workspace_ints", "cinn_moe_route_static_max_ints", "cinn_fp8_gemm_workspace_bytes", "cinn_moe_balance_workspace_bytes",
                                                  "cinn_sparse_attn_workspace_bytes",
                                                  "cinn_fp8_grouped_wgrad_scratch_bytes", "cinn_fp8_grouped_wgrad_fused_scratch_bytes")
                       else ctypes.c_int)

@@ -16,10 +16,10 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 LIB_DIR = os.path.join(HERE, "lib")
 LIB_PATH = os.path.join(LIB_DIR, "libcinnamon_b200.so")
-SOURCES = ["quant.cu", "gemm.cu", "moe.cu", "route.cu", "sparse_attn.cu", "attn_tc.cu", "indexer.cu", "wgrad.cu", "capi.cu"]
+SOURCES = ["quant.cu", "gemm.cu", "moe.cu", "moe_train.cu", "route.cu", "sparse_attn.cu", "attn_tc.cu", "indexer.cu", "wgrad.cu", "capi.cu"]
 HOST_DIR = os.path.join(CSRC, "host")
 HOST_PATH = os.path.join(LIB_DIR, "_host.so")
-HOST_SOURCES = ["linear.cpp", "attention.cpp", "moe.cpp", "module.cpp"]
+HOST_SOURCES = ["linear.cpp", "attention.cpp", "moe.cpp", "moe_train.cpp", "module.cpp"]
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
     "-Xcompiler", "-fPIC", "--expt-relaxed-constexpr",

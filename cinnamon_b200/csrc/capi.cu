@@ -111,7 +111,14 @@ int quantize_row_block(const void* x, int dtype, int64_t M, int64_t N, int64_t l
                        float* s_blk, int round_scale, int div_mode, cudaStream_t st, int transpose_block);
 int quantize_block_t(const void* x, int dtype, int64_t M, int64_t N, int64_t ld, void* q, void* q_t, float* scales,
                      int round_scale, int div_mode, cudaStream_t st);
-int swiglu(const void* h12, const void* dh, void* out, int dtype, int64_t T_rows, int64_t I, int backward, cudaStream_t st);
+int swiglu(const void* h12, const void* dh, void* out, int dtype, int64_t T_rows, int64_t I, int backward, int round, cudaStream_t st);
+int64_t balance_workspace_bytes(int64_t batch, int64_t seq, int E);
+int balance_loss(const void* logits, int dtype, const int* top_experts, int64_t batch, int64_t seq, int E, int top_k, float alpha,
+                 void* workspace, float* share, float* loss, cudaStream_t st);
+int gates_backward(const void* logits, int dtype, const int64_t* sorted_experts, const int64_t* pair_pos, const float* d_gates,
+                   const float* share, const float* d_loss, float alpha, int64_t batch, int64_t seq, int E, int top_k, void* d_logits,
+                   cudaStream_t st);
+int update_bias(const int64_t* counts, float* bias, int E, float expected, float gamma, cudaStream_t st);
 int64_t moe_route_workspace_ints(int64_t T, int E);
 int moe_route(const void* logits, int logits_dtype, const float* bias, int64_t T, int E, int top_k, int* workspace, int* top_experts,
               float* top_gates, int64_t* token_indices, float* sorted_scores, int64_t* sorted_experts, int64_t* counts,
@@ -329,11 +336,40 @@ int cinn_fp8_grouped_wgrad(const void* dY, int dy_dtype, const void* x_q, const 
 }
 
 int cinn_swiglu(const void* h12, void* h, int dtype, int64_t T, int64_t I, void* stream) {
-    return cinn::swiglu(h12, nullptr, h, dtype, T, I, 0, (cudaStream_t)stream);
+    return cinn::swiglu(h12, nullptr, h, dtype, T, I, 0, 0, (cudaStream_t)stream);
 }
 
 int cinn_swiglu_backward(const void* h12, const void* grad_h, void* grad_h12, int dtype, int64_t T, int64_t I, void* stream) {
-    return cinn::swiglu(h12, grad_h, grad_h12, dtype, T, I, 1, (cudaStream_t)stream);
+    return cinn::swiglu(h12, grad_h, grad_h12, dtype, T, I, 1, 0, (cudaStream_t)stream);
+}
+
+int cinn_swiglu_rounded(const void* h12, void* h, int dtype, int64_t T, int64_t I, void* stream) {
+    return cinn::swiglu(h12, nullptr, h, dtype, T, I, 0, 1, (cudaStream_t)stream);
+}
+
+int cinn_swiglu_rounded_backward(const void* h12, const void* grad_h, void* grad_h12, int dtype, int64_t T, int64_t I, void* stream) {
+    return cinn::swiglu(h12, grad_h, grad_h12, dtype, T, I, 1, 1, (cudaStream_t)stream);
+}
+
+int64_t cinn_moe_balance_workspace_bytes(int64_t batch, int64_t seq, int n_experts) {
+    return cinn::balance_workspace_bytes(batch, seq, n_experts);
+}
+
+int cinn_moe_balance_loss(const void* logits, int logits_dtype, const int* top_experts, int64_t batch, int64_t seq, int n_experts,
+                          int top_k, float alpha, void* workspace, float* share, float* loss, void* stream) {
+    return cinn::balance_loss(logits, logits_dtype, top_experts, batch, seq, n_experts, top_k, alpha, workspace, share, loss,
+                              (cudaStream_t)stream);
+}
+
+int cinn_moe_gates_backward(const void* logits, int logits_dtype, const int64_t* sorted_experts, const int64_t* pair_pos,
+                            const float* d_gates, const float* share, const float* d_loss, float alpha, int64_t batch, int64_t seq,
+                            int n_experts, int top_k, void* d_logits, void* stream) {
+    return cinn::gates_backward(logits, logits_dtype, sorted_experts, pair_pos, d_gates, share, d_loss, alpha, batch, seq, n_experts,
+                                top_k, d_logits, (cudaStream_t)stream);
+}
+
+int cinn_moe_update_bias(const int64_t* counts, float* bias, int n_experts, float expected, float gamma, void* stream) {
+    return cinn::update_bias(counts, bias, n_experts, expected, gamma, (cudaStream_t)stream);
 }
 
 int cinn_p2p_barrier(const int64_t* peer_flags, int rank, int n_ranks, unsigned epoch, void* stream) {

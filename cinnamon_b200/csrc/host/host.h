@@ -8,6 +8,7 @@
 #pragma once
 #include <torch/extension.h>
 #include <torch/csrc/Exceptions.h>
+#include <ATen/autocast_mode.h>
 #include <ATen/cuda/CUDAContext.h>
 #include <ATen/cuda/EmptyTensor.h>
 #include <c10/cuda/CUDAGuard.h>
@@ -26,7 +27,10 @@ using at::Tensor;
     X(cinn_requant_row_to_block) X(cinn_fp8_gemm_ws) X(cinn_fp8_gemm_workspace_bytes) \
     X(cinn_sparse_attn_workspace_bytes) X(cinn_sparse_attn_fwd_ws) X(cinn_sparse_attn_bwd) X(cinn_sparse_attn_bwd_ws)                  \
     X(cinn_moe_route_workspace_ints) X(cinn_moe_route_ranges) X(cinn_spread_rows) X(cinn_fp8_grouped_gemm)                \
-    X(cinn_swiglu_quant_rowwise) X(cinn_moe_combine) X(cinn_moe_combine_add)
+    X(cinn_swiglu_quant_rowwise) X(cinn_moe_combine) X(cinn_moe_combine_add)                \
+    X(cinn_swiglu_rounded) X(cinn_swiglu_rounded_backward) X(cinn_moe_balance_workspace_bytes) X(cinn_moe_balance_loss)     \
+    X(cinn_moe_gates_backward) X(cinn_moe_update_bias) X(cinn_moe_combine_backward) X(cinn_swiglu_backward)                 \
+    X(cinn_fp8_grouped_wgrad_fused_scratch_bytes) X(cinn_fp8_grouped_wgrad_fused) X(cinn_fp8_grouped_gemm_dgrad)
 
 struct Api {
 #define CINN_DECL(name) decltype(&::name) name = nullptr;
@@ -87,6 +91,36 @@ inline void* stream() { return at::cuda::getCurrentCUDAStream().stream(); }
 inline float* f32(const Tensor& t);
 Tensor gemm(const Tensor& a, const Tensor& sa, const Tensor& b, int layout, const Tensor& sb, int64_t sbk, int64_t sbn, int64_t M,
             int64_t N, int64_t K, at::ScalarType type, int tag);               // linear.cpp
+
+struct Linear {                                 // what an FP8 linear's forward leaves for its backward
+    Tensor out, x, x_scale, w, w_scale, w_t;
+    bool x_is_block = false, x_is_block_t = false;
+};
+Linear linear_forward(const Tensor& x, const Tensor& weight, bool round_scale, bool need_dgrad, bool need_wgrad, bool kmajor, int div,
+                      const Tensor& w_q, const Tensor& w_s, const Tensor& w_qt);
+std::tuple<Tensor, Tensor> linear_backward(const Tensor& grad_out, Tensor x, Tensor x_scale, const Tensor& w, const Tensor& w_scale,
+                                           const Tensor& w_t, at::IntArrayRef x_shape, bool round_scale, bool x_is_block,
+                                           bool x_is_block_t, at::ScalarType weight_dtype, bool kmajor, int div, bool want_gx,
+                                           bool want_gw, at::ScalarType gx_type);
+
+struct Quantised { Tensor q, s; };
+Quantised rowwise(const Tensor& x, bool round_scale, int div);                 // moe.cpp
+Quantised swiglu_quantised(const Tensor& h12, int div);
+Tensor grouped(const Quantised& x, const Quantised& w, const Tensor& starts, const Tensor& ends);
+struct Routes {                                 // moe_route's outputs, in three tensors
+    Tensor longs, floats, top;                  // token_indices | sorted_experts | pair_pos | counts | starts | ends; scores | pair_gate
+    int64_t pairs = 0, E = 0;
+    int64_t* part(int64_t at) const { return longs.data_ptr<int64_t>() + at; }
+    int64_t* token_indices() const { return part(0); }
+    int64_t* sorted_experts() const { return part(pairs); }
+    int64_t* pos() const { return part(2 * pairs); }
+    Tensor counts() const { return longs.narrow(0, 3 * pairs, E); }
+    Tensor starts() const { return longs.narrow(0, 3 * pairs + E, E); }
+    Tensor ends() const { return longs.narrow(0, 3 * pairs + 2 * E, E); }
+    float* gates() const { return static_cast<float*>(floats.data_ptr()) + pairs; }
+};
+Routes route(const Tensor& logits, const Tensor& bias, int64_t top_k);
+Quantised spread(const Quantised& x, const Routes& r, int64_t top_k);
 inline float* f32(const Tensor& t) { return static_cast<float*>(t.data_ptr()); }
 
 }  // namespace cinnhost

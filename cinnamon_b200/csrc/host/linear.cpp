@@ -15,14 +15,7 @@ Tensor gemm(const Tensor& a, const Tensor& sa, const Tensor& b, int layout, cons
     return out;
 }
 
-namespace {
-
-struct Linear {                                 // what the forward leaves for the backward
-    Tensor out, x, x_scale, w, w_scale, w_t;
-    bool x_is_block = false, x_is_block_t = false;
-};
-
-Linear forward(const Tensor& x, const Tensor& weight, bool round_scale, bool need_dgrad, bool need_wgrad, bool kmajor, int div,
+Linear linear_forward(const Tensor& x, const Tensor& weight, bool round_scale, bool need_dgrad, bool need_wgrad, bool kmajor, int div,
                const Tensor& w_q, const Tensor& w_s, const Tensor& w_qt) {
     require(x.is_cuda(), "Input must be on CUDA");
     c10::cuda::CUDAGuard guard(x.device());
@@ -80,10 +73,10 @@ Linear forward(const Tensor& x, const Tensor& weight, bool round_scale, bool nee
     return r;
 }
 
-std::tuple<Tensor, Tensor> backward(const Tensor& grad_out, Tensor x, Tensor x_scale, const Tensor& w, const Tensor& w_scale,
+std::tuple<Tensor, Tensor> linear_backward(const Tensor& grad_out, Tensor x, Tensor x_scale, const Tensor& w, const Tensor& w_scale,
                                     const Tensor& w_t, at::IntArrayRef x_shape, bool round_scale, bool x_is_block,
-                                    bool x_is_block_t, at::ScalarType weight_dtype, bool kmajor, int div, bool want_gx = true,
-                                    bool want_gw = true) {
+                                    bool x_is_block_t, at::ScalarType weight_dtype, bool kmajor, int div, bool want_gx,
+                                           bool want_gw, at::ScalarType gx_type) {
     c10::cuda::CUDAGuard guard(w.device());
     const at::Device dev = w.device();
     const int64_t N = w.size(0), K = w.size(1);
@@ -103,6 +96,8 @@ std::tuple<Tensor, Tensor> backward(const Tensor& grad_out, Tensor x, Tensor x_s
     check(api.cinn_quant_rowwise_dual(g.data_ptr(), tag_of(g.scalar_type()), Mp, N, g.stride(0), gq.data_ptr(), f32(gs),
                                       gqt.data_ptr(), f32(gst), round_scale, div, stream()), "cinn_quant_rowwise_dual");
     ++launches;
+    // (the reference's input gradient is bf16 and autograd casts it to the input's type: fp32 holds those values)
+    const int gx_tag = gx_type == at::kFloat ? TAG_F32_BF16 : TAG_BF16;
     Tensor gx;
     if (!want_gx) {
     } else if (N % 16 == 0 && (kmajor || w_t.defined())) {
@@ -112,9 +107,9 @@ std::tuple<Tensor, Tensor> backward(const Tensor& grad_out, Tensor x, Tensor x_s
             check(api.cinn_transpose_bytes(w.data_ptr(), w.stride(0), wt.data_ptr(), N, K, stream()), "cinn_transpose_bytes");
             ++launches;
         }
-        gx = gemm(gq, gs, wt, 0, w_scale, w_scale.stride(0), w_scale.stride(1), M, K, N, at::kBFloat16, TAG_BF16);
+        gx = gemm(gq, gs, wt, 0, w_scale, w_scale.stride(0), w_scale.stride(1), M, K, N, gx_type, gx_tag);
     } else {
-        gx = gemm(gq, gs, w, 1, w_scale, w_scale.stride(0), w_scale.stride(1), M, K, N, at::kBFloat16, TAG_BF16);
+        gx = gemm(gq, gs, w, 1, w_scale, w_scale.stride(0), w_scale.stride(1), M, K, N, gx_type, gx_tag);
     }
     if (gx.defined() && x_shape.size() != 2) gx = gx.reshape(x_shape);
     if (!want_gw) return {gx, Tensor()};
@@ -136,18 +131,21 @@ std::tuple<Tensor, Tensor> backward(const Tensor& grad_out, Tensor x, Tensor x_s
 }
 
 
-struct Quantised { Tensor q, s, q_t; };      // a weight already in e4m3 (undefined: quantise it here), handed around the node's tensors
+namespace {
+
+struct CachedWeight { Tensor q, s, q_t; };      // a weight already in e4m3 (undefined: quantise it here), handed around the node's tensors
 
 class LinearNode : public torch::autograd::Function<LinearNode> {
 public:
     static Tensor forward(torch::autograd::AutogradContext* ctx, const Tensor& x, const Tensor& weight, bool round_scale, bool kmajor,
-                          int64_t div, const Quantised* wq) {
-        Linear r = cinnhost::forward(x, weight, round_scale, x.requires_grad(), weight.requires_grad(), kmajor, (int)div, wq->q, wq->s,
+                          int64_t div, const CachedWeight* wq) {
+        Linear r = linear_forward(x, weight, round_scale, x.requires_grad(), weight.requires_grad(), kmajor, (int)div, wq->q, wq->s,
                                      wq->q_t);
         ctx->save_for_backward({r.x, r.x_scale, r.w, r.w_scale, r.w_t});
         ctx->saved_data["x_shape"] = x.sizes().vec();
         ctx->saved_data["flags"] = (int64_t)((round_scale ? 1 : 0) | (r.x_is_block ? 2 : 0) | (r.x_is_block_t ? 4 : 0) | (kmajor ? 8 : 0) |
-                                             ((int64_t)div << 4) | ((int64_t)weight.scalar_type() << 8));
+                                             ((int64_t)div << 4) | ((int64_t)weight.scalar_type() << 8) |
+                                             (x.scalar_type() == at::kFloat ? 1 << 16 : 0));
         return r.out;
     }
     static torch::autograd::variable_list backward(torch::autograd::AutogradContext* ctx, torch::autograd::variable_list grads) {
@@ -155,9 +153,9 @@ public:
         const int64_t f = ctx->saved_data["flags"].toInt();
         Tensor gx, gw;
         as_python_error([&] {
-            std::tie(gx, gw) = cinnhost::backward(grads[0], s[0], s[1], s[2], s[3], s[4], ctx->saved_data["x_shape"].toIntVector(), f & 1,
-                                                  f & 2, f & 4, (at::ScalarType)(f >> 8), f & 8, (f >> 4) & 15, ctx->needs_input_grad(0),
-                                                  ctx->needs_input_grad(1));
+            std::tie(gx, gw) = linear_backward(grads[0], s[0], s[1], s[2], s[3], s[4], ctx->saved_data["x_shape"].toIntVector(), f & 1,
+                                                  f & 2, f & 4, (at::ScalarType)(f >> 8 & 255), f & 8, (f >> 4) & 15, ctx->needs_input_grad(0),
+                                                  ctx->needs_input_grad(1), f >> 16 & 1 ? at::kFloat : at::kBFloat16);
         });
         return {gx, gw, Tensor(), Tensor(), Tensor(), Tensor()};
     }
@@ -171,22 +169,22 @@ void bind_linear(pybind11::module_& m) {
     using OptT = c10::optional<Tensor>;
     // (out, x, x_scale, w, w_scale, w_t or None, x_is_block, x_is_block_t)
     m.def("linear_forward", [](const Tensor& x, const Tensor& w, bool round_scale, bool need_dgrad, bool need_wgrad, bool kmajor, int div) {
-        Linear r = forward(x, w, round_scale, need_dgrad, need_wgrad, kmajor, div, Tensor(), Tensor(), Tensor());
+        Linear r = linear_forward(x, w, round_scale, need_dgrad, need_wgrad, kmajor, div, Tensor(), Tensor(), Tensor());
         return std::make_tuple(r.out, r.x, r.x_scale, r.w, r.w_scale, r.w_t.defined() ? OptT(r.w_t) : OptT(), r.x_is_block, r.x_is_block_t);
     });
     m.def("linear_backward", [](const Tensor& g, const Tensor& x, const Tensor& xs, const Tensor& w, const Tensor& ws, const OptT& wt,
                                 const std::vector<int64_t>& x_shape, bool round_scale, bool x_is_block, bool x_is_block_t, bool w_fp32,
                                 bool kmajor, int div) {
-        return backward(g, x, xs, w, ws, or_none(wt), x_shape, round_scale, x_is_block, x_is_block_t,
-                        w_fp32 ? at::kFloat : at::kBFloat16, kmajor, div);
+        return linear_backward(g, x, xs, w, ws, or_none(wt), x_shape, round_scale, x_is_block, x_is_block_t,
+                        w_fp32 ? at::kFloat : at::kBFloat16, kmajor, div, true, true, at::kBFloat16);
     });
     // the differentiable call; without gradients to record nothing is saved and no gradient copies are made
     m.def("linear", [](const Tensor& x, const Tensor& w, bool round_scale, bool kmajor, int div, const OptT& wq, const OptT& ws,
                        const OptT& wqt) {
-        const Quantised cached{or_none(wq), or_none(ws), or_none(wqt)};
+        const CachedWeight cached{or_none(wq), or_none(ws), or_none(wqt)};
         if (at::GradMode::is_enabled() && (x.requires_grad() || w.requires_grad()))
             return LinearNode::apply(x, w, round_scale, kmajor, (int64_t)div, &cached);
-        return forward(x, w, round_scale, false, false, kmajor, div, cached.q, cached.s, cached.q_t).out;
+        return linear_forward(x, w, round_scale, false, false, kmajor, div, cached.q, cached.s, cached.q_t).out;
     });
 }
 

@@ -7,6 +7,7 @@ std::atomic<int64_t> launches{0};
 void bind_linear(pybind11::module_& m);
 void bind_attention(pybind11::module_& m);
 void bind_moe(pybind11::module_& m);
+void bind_moe_train(pybind11::module_& m);
 }  // namespace cinnhost
 
 PYBIND11_MODULE(_host, m) {
@@ -36,4 +37,5 @@ PYBIND11_MODULE(_host, m) {
     bind_linear(m);
     bind_attention(m);
     bind_moe(m);
+    bind_moe_train(m);
 }

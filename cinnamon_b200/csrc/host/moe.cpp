@@ -5,10 +5,6 @@
 
 namespace cinnhost {
 
-namespace {
-
-struct Quantised { Tensor q, s; };
-
 Quantised rowwise(const Tensor& x, bool round_scale, int div) {
     const int64_t M = x.size(0), K = x.size(1);
     Quantised r{empty({M, K}, F8, x.device()), empty({M, up(K, 128)}, at::kFloat, x.device())};
@@ -18,7 +14,7 @@ Quantised rowwise(const Tensor& x, bool round_scale, int div) {
     return r;
 }
 
-Quantised swiglu(const Tensor& h12, int div) {
+Quantised swiglu_quantised(const Tensor& h12, int div) {
     const int64_t T = h12.size(0), I = h12.size(1) / 2;
     Quantised r{empty({T, I}, F8, h12.device()), empty({T, up(I, 128)}, at::kFloat, h12.device())};
     check(api.cinn_swiglu_quant_rowwise(h12.data_ptr(), tag_of(h12.scalar_type()), T, I, r.q.data_ptr(), f32(r.s), div, stream()),
@@ -37,6 +33,38 @@ Tensor grouped(const Quantised& x, const Quantised& w, const Tensor& starts, con
     return out;
 }
 
+Routes route(const Tensor& logits_in, const Tensor& bias, int64_t top_k) {
+    const Tensor logits = readable(logits_in).contiguous(), b = bias.to(at::kFloat).contiguous();
+    const int64_t T = logits.size(0), E = logits.size(1);
+    const at::Device dev = logits.device();
+    Routes r;
+    r.pairs = T * top_k;
+    r.E = E;
+    r.longs = empty({3 * r.pairs + 3 * E}, at::kLong, dev);
+    r.floats = empty({2 * r.pairs}, at::kFloat, dev);
+    r.top = empty({r.pairs}, at::kInt, dev);
+    Tensor ws = empty({std::max<int64_t>(1, api.cinn_moe_route_workspace_ints(T, (int)E))}, at::kInt, dev);
+    Tensor top_gates = empty({r.pairs}, at::kFloat, dev);
+    check(api.cinn_moe_route_ranges(logits.data_ptr(), tag_of(logits.scalar_type()), f32(b), T, (int)E, (int)top_k, ws.data_ptr<int>(),
+                                    r.top.data_ptr<int>(), f32(top_gates), r.token_indices(), f32(r.floats), r.sorted_experts(),
+                                    r.part(3 * r.pairs), r.part(3 * r.pairs + E), r.part(3 * r.pairs + 2 * E), r.pos(), r.gates(),
+                                    stream()), "cinn_moe_route");
+    launches += 3;
+    return r;
+}
+
+// quantised tokens to the rows of their pairs
+Quantised spread(const Quantised& x, const Routes& r, int64_t top_k) {
+    const int64_t T = x.q.size(0), d = x.q.size(1), ns = x.s.size(1);
+    Quantised rows{empty({r.pairs, d}, F8, x.q.device()), empty({r.pairs, ns}, at::kFloat, x.q.device())};
+    check(api.cinn_spread_rows(x.q.data_ptr(), f32(x.s), r.pos(), rows.q.data_ptr(), f32(rows.s), T, r.pairs, (int)top_k, d, ns, stream()),
+          "cinn_spread_rows");
+    ++launches;
+    return rows;
+}
+
+namespace {
+
 // x (T, d), contiguous; router (E, d) in the type the logits are computed in; the weights as FP8Experts and FP8SwiGLU hold
 // them.  Returns (T, d) fp32.
 Tensor forward(const Tensor& x, const Tensor& router, const Tensor& bias, int64_t top_k, const Quantised& w12, const Quantised& w3,
@@ -51,40 +79,26 @@ Tensor forward(const Tensor& x, const Tensor& router, const Tensor& bias, int64_
     if (sw12.q.defined()) {
         const Quantised xs = shared_round ? rowwise(x, true, div) : xq;
         const int64_t I2 = sw12.q.size(0);
-        const Quantised h = swiglu(gemm(xs.q, xs.s, sw12.q, 0, sw12.s, sw12.s.stride(1), sw12.s.stride(0), T, I2, d, at::kBFloat16,
+        const Quantised h = swiglu_quantised(gemm(xs.q, xs.s, sw12.q, 0, sw12.s, sw12.s.stride(1), sw12.s.stride(0), T, I2, d, at::kBFloat16,
                                         TAG_BF16), div);
         shared = gemm(h.q, h.s, sw3.q, 0, sw3.s, sw3.s.stride(1), sw3.s.stride(0), T, d, I2 / 2, at::kBFloat16, TAG_BF16);
     }
     Tensor logits = at::mm(x, router.to(x.scalar_type()).t());
-    logits = readable(logits).contiguous();
-    const int64_t pairs = T * top_k;
-    Tensor ws = empty({std::max<int64_t>(1, api.cinn_moe_route_workspace_ints(T, (int)E))}, at::kInt, dev);
-    Tensor top_e = empty({pairs}, at::kInt, dev), top_g = empty({pairs}, at::kFloat, dev);
-    Tensor longs = empty({3 * pairs + 3 * E}, at::kLong, dev), floats = empty({2 * pairs}, at::kFloat, dev);
-    int64_t* l = longs.data_ptr<int64_t>();
-    const Tensor starts = longs.narrow(0, 3 * pairs + E, E), ends = longs.narrow(0, 3 * pairs + 2 * E, E);
-    const Tensor b = bias.to(at::kFloat).contiguous();
-    check(api.cinn_moe_route_ranges(logits.data_ptr(), tag_of(logits.scalar_type()), f32(b), T, (int)E, (int)top_k, ws.data_ptr<int>(),
-                                    top_e.data_ptr<int>(), f32(top_g), l, f32(floats), l + pairs, l + 3 * pairs,
-                                    starts.data_ptr<int64_t>(), ends.data_ptr<int64_t>(), l + 2 * pairs, f32(floats) + pairs, stream()),
-          "cinn_moe_route");
-    launches += 3;
-    const int64_t* pos = l + 2 * pairs;
-    Quantised rows{empty({pairs, d}, F8, dev), empty({pairs, up(d, 128)}, at::kFloat, dev)};
-    check(api.cinn_spread_rows(xq.q.data_ptr(), f32(xq.s), pos, rows.q.data_ptr(), f32(rows.s), T, pairs, (int)top_k, d, up(d, 128),
-                               stream()), "cinn_spread_rows");
-    ++launches;
+    const Routes r = route(logits, bias, top_k);
+    const Tensor starts = r.starts(), ends = r.ends();
+    const int64_t pairs = r.pairs, *pos = r.pos();
+    Quantised rows = spread(xq, r, top_k);
     Tensor h12 = grouped(rows, w12, starts, ends);
     rows = Quantised{};
-    const Quantised h = swiglu(h12, div);
+    const Quantised h = swiglu_quantised(h12, div);
     h12.reset();
     const Tensor out = grouped(h, w3, starts, ends);
     Tensor y = empty({T, d}, at::kFloat, dev);
     if (shared.defined())
-        check(api.cinn_moe_combine_add(out.data_ptr(), TAG_BF16, pos, f32(floats) + pairs, shared.data_ptr(), TAG_BF16, f32(y), T, pairs,
+        check(api.cinn_moe_combine_add(out.data_ptr(), TAG_BF16, pos, r.gates(), shared.data_ptr(), TAG_BF16, f32(y), T, pairs,
                                        (int)top_k, d, stream()), "cinn_moe_combine_add");
     else
-        check(api.cinn_moe_combine(out.data_ptr(), TAG_BF16, pos, f32(floats) + pairs, f32(y), T, pairs, (int)top_k, d, stream()),
+        check(api.cinn_moe_combine(out.data_ptr(), TAG_BF16, pos, r.gates(), f32(y), T, pairs, (int)top_k, d, stream()),
               "cinn_moe_combine");
     ++launches;
     return y;

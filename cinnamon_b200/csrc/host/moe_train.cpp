@@ -1,0 +1,256 @@
+// The trainable MoE block (layers.MoE, layers.SwiGLU) as two native autograd nodes: the shared expert, and router + routed
+// experts + combine.  Written as modules and torch calls the block was 128 launches and 2.7 ms of host time per step at 32 x
+// 1024 tokens of 512; as nodes it also stops converting and copying between its parts:
+//   - w1 and w2 of a shared expert are one GEMM on x quantised once, forward and backward
+//   - tokens are quantised once and their bytes spread to the experts' rows (forward); the rows' gradients come home as one
+//     gather pass with the router's part added in it (backward), where autograd's index_select needed an atomic index_add
+//   - expert outputs stay in bf16 up to the combine pass, their gradients likewise
+//   - gates and balance loss have a kernel for their derivative (csrc/moe_train.cu)
+#include "host.h"
+
+namespace cinnhost {
+
+namespace {
+
+using torch::autograd::AutogradContext;
+using torch::autograd::variable_list;
+
+// ---------------------------------------------------------------------------------------------------------------------
+// shared expert: w3(silu(w1 x) * w2 x) on FP8 linears (reference src/layers.py:15-31 after convert_to_fp8)
+// ---------------------------------------------------------------------------------------------------------------------
+struct SwiGLUOptions { bool round12, round3, kmajor; int div; };
+
+Tensor swiglu_rounded(const Tensor& h12) {
+    const int64_t T = h12.size(0), I = h12.size(1) / 2;
+    Tensor h = empty({T, I}, h12.scalar_type(), h12.device());
+    check(api.cinn_swiglu_rounded(h12.data_ptr(), h.data_ptr(), tag_of(h12.scalar_type()), T, I, stream()), "cinn_swiglu");
+    ++launches;
+    return h;
+}
+
+struct SwiGLUNode : public torch::autograd::Function<SwiGLUNode> {
+    static Tensor forward(AutogradContext* ctx, const Tensor& x, const Tensor& w1, const Tensor& w2, const Tensor& w3, const SwiGLUOptions* o) {
+        c10::cuda::CUDAGuard guard(x.device());
+        const bool gx = x.requires_grad(), g12 = w1.requires_grad() || w2.requires_grad(), g3 = w3.requires_grad(), any = gx || g12;
+        const Linear a = linear_forward(x, at::cat({w1, w2}), o->round12, gx, g12, o->kmajor, o->div, Tensor(), Tensor(), Tensor());
+        const Tensor h12 = a.out.view({-1, a.out.size(-1)});
+        const Linear b = linear_forward(swiglu_rounded(h12), w3, o->round3, any, g3, o->kmajor, o->div, Tensor(), Tensor(), Tensor());
+        if (any || g3) {
+            ctx->save_for_backward({a.x, a.x_scale, a.w, a.w_scale, a.w_t, h12, b.x, b.x_scale, b.w, b.w_scale, b.w_t});
+            ctx->saved_data["x_shape"] = x.sizes().vec();
+            auto flags = [&](bool round, const Linear& l, const Tensor& w) {
+                return (int64_t)((round ? 1 : 0) | (l.x_is_block ? 2 : 0) | (l.x_is_block_t ? 4 : 0) | (o->kmajor ? 8 : 0) | (o->div << 4) |
+                                 ((int)w.scalar_type() << 8));
+            };
+            ctx->saved_data["a"] = flags(o->round12, a, w1);
+            ctx->saved_data["b"] = flags(o->round3, b, w3);
+            ctx->saved_data["x32"] = x.scalar_type() == at::kFloat;
+        }
+        auto shape = x.sizes().vec();
+        shape.back() = w3.size(0);
+        return b.out.view(shape);
+    }
+
+    static variable_list backward(AutogradContext* ctx, variable_list grads) {
+        auto s = ctx->get_saved_variables();
+        const bool gx = ctx->needs_input_grad(0), g12 = ctx->needs_input_grad(1) || ctx->needs_input_grad(2), g3 = ctx->needs_input_grad(3);
+        Tensor dx, d1, d2, d3;
+        as_python_error([&] {
+            auto back = [&](int64_t f, const Tensor& g, int at, at::IntArrayRef shape, bool want_x, bool want_w, at::ScalarType type) {
+                return linear_backward(g, s[at], s[at + 1], s[at + 2], s[at + 3], s[at + 4], shape, f & 1, f & 2, f & 4,
+                                       (at::ScalarType)(f >> 8 & 255), f & 8, (int)(f >> 4 & 15), want_x, want_w, type);
+            };
+            const Tensor& h12 = s[5];
+            const int64_t T = h12.size(0), I = h12.size(1) / 2;
+            Tensor dh;
+            std::tie(dh, d3) = back(ctx->saved_data["b"].toInt(), grads[0], 6, {T, I}, gx || g12, g3, at::kBFloat16);
+            if (!(gx || g12)) return;
+            c10::cuda::CUDAGuard guard(h12.device());
+            Tensor dh12 = empty({T, 2 * I}, h12.scalar_type(), h12.device()), d12;
+            check(api.cinn_swiglu_rounded_backward(h12.data_ptr(), dh.data_ptr(), dh12.data_ptr(), tag_of(h12.scalar_type()), T, I, stream()),
+                  "cinn_swiglu_backward");
+            ++launches;
+            std::tie(dx, d12) = back(ctx->saved_data["a"].toInt(), dh12, 0, ctx->saved_data["x_shape"].toIntVector(), gx, g12,
+                                     ctx->saved_data["x32"].toBool() ? at::kFloat : at::kBFloat16);
+            if (g12) {
+                d1 = d12.narrow(0, 0, I);
+                d2 = d12.narrow(0, I, I);
+            }
+        });
+        return {dx, d1, d2, d3, Tensor()};
+    }
+};
+
+// ---------------------------------------------------------------------------------------------------------------------
+// router, routed experts, combine (reference src/layers.py:56-87, 118-179)
+// ---------------------------------------------------------------------------------------------------------------------
+struct BlockOptions {
+    Tensor bias;                               // (E,) fp32
+    Quantised w12, w3;                         // the expert weights in e4m3
+    int64_t top_k, batch;
+    double alpha;                              // balance loss, 0 = none
+    at::ScalarType router_type;                // what the router multiplies in (autocast's type, or x's)
+    int div;
+    Tensor counts;                             // out: rows per expert
+};
+
+// gradients of grouped(x, w) given dy, rows of every expert contiguous and all rows covered
+std::tuple<Tensor, Tensor> grouped_backward(const Tensor& dy, const Tensor& xq, const Tensor& xs, const Tensor& wq, const Tensor& ws,
+                                            const Tensor& starts, const Tensor& ends, at::ScalarType w_type, bool want_x,
+                                            at::ScalarType x_type, int div) {
+    const int64_t R = dy.size(0), E = wq.size(0), d_out = wq.size(1), d_in = wq.size(2);
+    const at::Device dev = dy.device();
+    const int64_t *st = starts.data_ptr<int64_t>(), *en = ends.data_ptr<int64_t>();
+    const int64_t need = api.cinn_fp8_grouped_wgrad_fused_scratch_bytes(R, E, d_in, d_out);
+    Tensor scratch = empty({need}, at::kByte, dev), dw = empty({E, d_out, d_in}, w_type, dev);
+    Tensor gq = empty({R, d_out}, F8, dev), gs = empty({R, d_out / 128}, at::kFloat, dev);
+    check(api.cinn_fp8_grouped_wgrad_fused(dy.data_ptr(), tag_of(dy.scalar_type()), xq.data_ptr(), f32(xs), st, en, E, R, d_in, d_out,
+                                           scratch.data_ptr(), need, dw.data_ptr(), w_type == at::kFloat ? TAG_F32_BF16 : TAG_BF16, div,
+                                           gq.data_ptr(), f32(gs), stream()), "cinn_fp8_grouped_wgrad_fused");
+    launches += 4;
+    Tensor dx;
+    if (want_x) {
+        dx = empty({R, d_in}, x_type, dev);
+        check(api.cinn_fp8_grouped_gemm_dgrad(gq.data_ptr(), f32(gs), wq.data_ptr(), f32(ws), st, en, E, R, d_in, d_out, dx.data_ptr(),
+                                              tag_of(x_type), stream()), "cinn_fp8_grouped_gemm_dgrad");
+        ++launches;
+    }
+    return {dx, dw};
+}
+
+struct BlockNode : public torch::autograd::Function<BlockNode> {
+    static variable_list forward(AutogradContext* ctx, const Tensor& x, const Tensor& router, const Tensor& w12, const Tensor& w3,
+                                 const Tensor& addend, BlockOptions* o) {
+        c10::cuda::CUDAGuard guard(x.device());
+        at::AutoDispatchBelowAutograd below;
+        const at::Device dev = x.device();
+        const int64_t T = x.size(0), d = x.size(1), E = router.size(0), k = o->top_k, seq = T / o->batch;
+        const Tensor xr = x.to(o->router_type), wr = router.to(o->router_type);
+        const Tensor logits = at::mm(xr, wr.t());
+        const Routes r = route(logits, o->bias, k);
+        const Tensor starts = r.starts(), ends = r.ends();
+        const Quantised rows = spread(rowwise(x, false, o->div), r, k);
+        const Tensor h12 = grouped(rows, o->w12, starts, ends);
+        const Quantised h = swiglu_quantised(h12, o->div);
+        const Tensor out = grouped(h, o->w3, starts, ends);
+        Tensor y = empty({T, d}, at::kFloat, dev);
+        check(api.cinn_moe_combine_add(out.data_ptr(), TAG_BF16, r.pos(), r.gates(), addend.data_ptr(), tag_of(addend.scalar_type()), f32(y),
+                                       T, r.pairs, (int)k, d, stream()), "cinn_moe_combine_add");
+        ++launches;
+        Tensor share, loss;
+        if (o->alpha > 0) {
+            share = empty({o->batch, E}, at::kFloat, dev);
+            loss = empty({}, at::kFloat, dev);
+            Tensor ws = empty({api.cinn_moe_balance_workspace_bytes(o->batch, seq, (int)E)}, at::kByte, dev);
+            check(api.cinn_moe_balance_loss(logits.data_ptr(), tag_of(logits.scalar_type()), r.top.data_ptr<int>(), o->batch, seq, (int)E,
+                                            (int)k, (float)o->alpha, ws.data_ptr(), f32(share), f32(loss), stream()), "cinn_moe_balance_loss");
+            launches += 2;
+        }
+        o->counts = r.counts();
+        ctx->save_for_backward({xr, wr, logits, r.longs, r.floats, rows.q, rows.s, h12, h.q, h.s, out, o->w12.q, o->w12.s, o->w3.q, o->w3.s,
+                                share});
+        ctx->saved_data["n"] = std::vector<int64_t>{k, o->batch, o->div, (int64_t)x.scalar_type(), (int64_t)router.scalar_type(),
+                                                    (int64_t)w12.scalar_type(), (int64_t)w3.scalar_type(), (int64_t)addend.scalar_type()};
+        ctx->saved_data["alpha"] = o->alpha;
+        ctx->set_materialize_grads(false);
+        if (loss.defined()) return {y, loss};
+        return {y};
+    }
+
+    static variable_list backward(AutogradContext* ctx, variable_list grads) {
+        auto s = ctx->get_saved_variables();
+        const auto n = ctx->saved_data["n"].toIntVector();
+        const int64_t k = n[0], batch = n[1];
+        const int div = (int)n[2];
+        const auto type = [&](int i) { return (at::ScalarType)n[i]; };
+        const float alpha = (float)ctx->saved_data["alpha"].toDouble();
+        Tensor dx, d_router, dw12, dw3, d_add;
+        as_python_error([&] {
+            const Tensor &xr = s[0], &wr = s[1], &logits = s[2], &h12 = s[7], &out = s[10];
+            c10::cuda::CUDAGuard guard(xr.device());
+            const at::Device dev = xr.device();
+            const int64_t T = xr.size(0), d = xr.size(1), E = wr.size(0), seq = T / batch;
+            Routes r;
+            r.longs = s[3]; r.floats = s[4]; r.pairs = T * k; r.E = E;
+            const Tensor starts = r.starts(), ends = r.ends();
+            const bool want_x = ctx->needs_input_grad(0), want_r = ctx->needs_input_grad(1), want_12 = ctx->needs_input_grad(2);
+            const bool want_3 = ctx->needs_input_grad(3);
+            Tensor d_gates, d_rows;
+            if (grads[0].defined()) {
+                const Tensor dy = grads[0].to(at::kFloat).contiguous();
+                if (ctx->needs_input_grad(4)) d_add = dy.to(type(7));
+                if (want_x || want_r || want_12 || want_3) {
+                    Tensor d_out = empty({r.pairs, d}, at::kBFloat16, dev);
+                    d_gates = empty({T, k}, at::kFloat, dev);
+                    check(api.cinn_moe_combine_backward(out.data_ptr(), TAG_BF16, r.pos(), r.gates(), f32(dy), d_out.data_ptr(), f32(d_gates),
+                                                        T, r.pairs, (int)k, d, stream()), "cinn_moe_combine_backward");
+                    ++launches;
+                    const bool below = want_x || want_12;
+                    Tensor dh;
+                    std::tie(dh, dw3) = grouped_backward(d_out, s[8], s[9], s[13], s[14], starts, ends, type(6), below, at::kBFloat16, div);
+                    d_out.reset();
+                    if (below) {
+                        const int64_t I = h12.size(1) / 2;
+                        Tensor dh12 = empty({r.pairs, 2 * I}, at::kBFloat16, dev);
+                        check(api.cinn_swiglu_backward(h12.data_ptr(), dh.data_ptr(), dh12.data_ptr(), TAG_BF16, r.pairs, I, stream()),
+                              "cinn_swiglu_backward");
+                        ++launches;
+                        std::tie(d_rows, dw12) = grouped_backward(dh12, s[5], s[6], s[11], s[12], starts, ends, type(5), want_x,
+                                                                  type(3), div);
+                    }
+                }
+            }
+            const bool loss = grads.size() > 1 && grads[1].defined();
+            Tensor dxr;
+            if ((want_x || want_r) && (loss || d_gates.defined())) {
+                Tensor d_logits = empty({T, E}, logits.scalar_type(), dev);
+                const Tensor dl = loss ? grads[1].to(at::kFloat) : Tensor();
+                check(api.cinn_moe_gates_backward(logits.data_ptr(), tag_of(logits.scalar_type()), r.sorted_experts(), r.pos(),
+                                                  d_gates.defined() ? f32(d_gates) : nullptr, loss ? f32(s[15]) : nullptr,
+                                                  loss ? f32(dl) : nullptr, alpha, batch, seq, (int)E, (int)k, d_logits.data_ptr(), stream()),
+                      "cinn_moe_gates_backward");
+                ++launches;
+                if (want_r) d_router = at::mm(d_logits.t(), xr).to(type(4));
+                if (want_x) dxr = at::mm(d_logits, wr);
+            }
+            if (want_x && d_rows.defined()) {
+                dx = empty({T, d}, at::kFloat, dev);
+                check(api.cinn_moe_combine_add(d_rows.data_ptr(), tag_of(d_rows.scalar_type()), r.pos(), nullptr, dxr.data_ptr(),
+                                               tag_of(dxr.scalar_type()), f32(dx), T, r.pairs, (int)k, d, stream()), "cinn_moe_combine_add");
+                ++launches;
+            } else {
+                dx = dxr;
+            }
+            if (dx.defined()) dx = dx.to(type(3));
+        });
+        return {dx, d_router, dw12, dw3, d_add, Tensor()};
+    }
+};
+
+}  // namespace
+
+void bind_moe_train(pybind11::module_& m) {
+    m.def("swiglu_block", [](const Tensor& x, const Tensor& w1, const Tensor& w2, const Tensor& w3, bool round12, bool round3, bool kmajor,
+                             int div) {
+        const SwiGLUOptions o{round12, round3, kmajor, div};
+        return SwiGLUNode::apply(x, w1, w2, w3, &o);
+    });
+    // (y, balance loss or None, rows per expert)
+    m.def("moe_block", [](const Tensor& x, const Tensor& router, const Tensor& w12, const Tensor& w3, const Tensor& addend,
+                          const Tensor& bias, const Tensor& w12_q, const Tensor& w12_s, const Tensor& w3_q, const Tensor& w3_s, int64_t top_k,
+                          int64_t batch, double alpha, bool cast_router, int div) {
+        BlockOptions o{bias, {w12_q, w12_s}, {w3_q, w3_s}, top_k, batch, alpha,
+                       cast_router ? at::autocast::get_autocast_dtype(at::kCUDA) : x.scalar_type(), div, Tensor()};
+        auto r = BlockNode::apply(x, router, w12, w3, addend, &o);
+        return std::make_tuple(r[0], r.size() > 1 ? c10::optional<Tensor>(r[1]) : c10::optional<Tensor>(), o.counts);
+    });
+    m.def("moe_update_bias", [](Tensor bias, const Tensor& counts, double expected, double gamma) {
+        c10::cuda::CUDAGuard guard(bias.device());
+        check(api.cinn_moe_update_bias(counts.data_ptr<int64_t>(), f32(bias), (int)bias.numel(), (float)expected, (float)gamma, stream()),
+              "cinn_moe_update_bias");
+        ++launches;
+        bias.unsafeGetTensorImpl()->bump_version();
+    });
+}
+
+}  // namespace cinnhost

@@ -62,7 +62,7 @@ moe_combine_kernel(const T* __restrict__ rows, const int64_t* __restrict__ pos, 
         int64_t p = -1;
         if (threadIdx.x < top_k) {
             p = pos[t * top_k + threadIdx.x];
-            s_gate[threadIdx.x] = gates[t * top_k + threadIdx.x];
+            s_gate[threadIdx.x] = gates ? gates[t * top_k + threadIdx.x] : 1.0f;      // null: plain sum
         }
         s_pos[threadIdx.x] = (p >= 0 && p < n_rows) ? p : -1;
     }
@@ -103,7 +103,7 @@ int moe_combine(const void* rows, int dtype, const int64_t* pos, const float* ga
                 void* y, int64_t n_tokens, int64_t n_rows, int top_k, int64_t d, cudaStream_t st) {
     CINN_CHECK_ARG(n_tokens >= 0 && n_rows >= 0 && d >= 0, "moe_combine: negative shape");
     if (n_tokens == 0 || d == 0) return CINN_OK;
-    CINN_CHECK_ARG(pos && gates && y && (rows || n_rows == 0), "moe_combine: null pointer");
+    CINN_CHECK_ARG(pos && y && (rows || n_rows == 0), "moe_combine: null pointer");
     CINN_CHECK_ARG(top_k >= 1 && top_k <= kMaxTopK, "moe_combine: top_k must be in [1, %d]", kMaxTopK);
     CINN_CHECK_ARG(d % 8 == 0 && d < (1LL << 31), "moe_combine: the row width (%lld) must be a multiple of 8", (long long)d);
     CINN_CHECK_ARG((reinterpret_cast<uintptr_t>(rows) & 15) == 0 && (reinterpret_cast<uintptr_t>(y) & 15) == 0,
@@ -133,6 +133,10 @@ template <typename T> __device__ __forceinline__ T from_float(float v);
 template <> __device__ __forceinline__ float from_float<float>(float v) { return v; }
 template <> __device__ __forceinline__ __nv_bfloat16 from_float<__nv_bfloat16>(float v) { return __float2bfloat16_rn(v); }
 template <> __device__ __forceinline__ __half from_float<__half>(float v) { return __float2half_rn(v); }
+
+__device__ __forceinline__ float to_float(float v) { return v; }
+__device__ __forceinline__ float to_float(__nv_bfloat16 v) { return __bfloat162float(v); }
+__device__ __forceinline__ float to_float(__half v) { return __half2float(v); }
 
 template <typename T>
 __device__ __forceinline__ void store8f(T* p, const float (&v)[8]) {
@@ -182,7 +186,9 @@ moe_combine_backward_kernel(const T* __restrict__ rows, const int64_t* __restric
     }
 }
 
-template <typename T, bool BACKWARD>
+// ROUND: silu(h1) is rounded to the activation type before the product, forward and backward, as `F.silu(w1(x)) * w2(x)`
+// on 16-bit tensors does (the shared experts, src/layers.py:27-31).
+template <typename T, bool BACKWARD, bool ROUND = false>
 __global__ void __launch_bounds__(256)
 swiglu_kernel(const T* __restrict__ h12, const T* __restrict__ dh, T* __restrict__ out, int64_t T_rows, int I) {
     const int per_row = I >> 3;
@@ -196,7 +202,11 @@ swiglu_kernel(const T* __restrict__ h12, const T* __restrict__ dh, T* __restrict
         if constexpr (!BACKWARD) {
             float h[8];
 #pragma unroll
-            for (int j = 0; j < 8; ++j) h[j] = (a[j] / (1.0f + expf(-a[j]))) * b[j];
+            for (int j = 0; j < 8; ++j) {
+                float s = a[j] / (1.0f + expf(-a[j]));
+                if constexpr (ROUND) s = to_float(from_float<T>(s));
+                h[j] = s * b[j];
+            }
             store8f<T>(out + row * (int64_t)I + col, h);
         } else {
             float g[8], d1[8], d2[8];
@@ -204,8 +214,13 @@ swiglu_kernel(const T* __restrict__ h12, const T* __restrict__ dh, T* __restrict
 #pragma unroll
             for (int j = 0; j < 8; ++j) {
                 const float sig = 1.0f / (1.0f + expf(-a[j]));
-                d1[j] = g[j] * b[j] * sig * (1.0f + a[j] * (1.0f - sig));
-                d2[j] = g[j] * a[j] * sig;
+                if constexpr (ROUND) {
+                    d1[j] = to_float(from_float<T>(g[j] * b[j])) * sig * (1.0f + a[j] * (1.0f - sig));
+                    d2[j] = g[j] * to_float(from_float<T>(a[j] * sig));
+                } else {
+                    d1[j] = g[j] * b[j] * sig * (1.0f + a[j] * (1.0f - sig));
+                    d2[j] = g[j] * a[j] * sig;
+                }
             }
             store8f<T>(out + row * 2 * (int64_t)I + col, d1);
             store8f<T>(out + row * 2 * (int64_t)I + I + col, d2);
@@ -214,18 +229,20 @@ swiglu_kernel(const T* __restrict__ h12, const T* __restrict__ dh, T* __restrict
 }
 
 template <typename T>
-static int swiglu_typed(const T* h12, const T* dh, T* out, int64_t T_rows, int64_t I, bool backward, cudaStream_t st) {
+static int swiglu_typed(const T* h12, const T* dh, T* out, int64_t T_rows, int64_t I, bool backward, bool round, cudaStream_t st) {
     int64_t blocks = (T_rows * (I / 8) + 255) / 256;
     const int64_t cap = (int64_t)sm_count() * 16;
     if (blocks > cap) blocks = cap;
-    if (backward) swiglu_kernel<T, true><<<(unsigned)blocks, 256, 0, st>>>(h12, dh, out, T_rows, (int)I);
+    if (backward && round) swiglu_kernel<T, true, true><<<(unsigned)blocks, 256, 0, st>>>(h12, dh, out, T_rows, (int)I);
+    else if (backward) swiglu_kernel<T, true><<<(unsigned)blocks, 256, 0, st>>>(h12, dh, out, T_rows, (int)I);
+    else if (round) swiglu_kernel<T, false, true><<<(unsigned)blocks, 256, 0, st>>>(h12, dh, out, T_rows, (int)I);
     else swiglu_kernel<T, false><<<(unsigned)blocks, 256, 0, st>>>(h12, dh, out, T_rows, (int)I);
     CINN_CHECK_LAUNCH();
     return CINN_OK;
 }
 
 // forward: out (T, I) = silu(h12[:, :I]) * h12[:, I:];  backward: out (T, 2I) = d h12 given dh (T, I)
-int swiglu(const void* h12, const void* dh, void* out, int dtype, int64_t T_rows, int64_t I, int backward, cudaStream_t st) {
+int swiglu(const void* h12, const void* dh, void* out, int dtype, int64_t T_rows, int64_t I, int backward, int round, cudaStream_t st) {
     CINN_CHECK_ARG(T_rows >= 0 && I >= 0, "swiglu: negative shape");
     if (T_rows == 0 || I == 0) return CINN_OK;
     CINN_CHECK_ARG(h12 && out && (!backward || dh), "swiglu: null pointer");
@@ -233,9 +250,9 @@ int swiglu(const void* h12, const void* dh, void* out, int dtype, int64_t T_rows
     CINN_CHECK_ARG((reinterpret_cast<uintptr_t>(h12) & 15) == 0 && (reinterpret_cast<uintptr_t>(out) & 15) == 0 &&
                    (reinterpret_cast<uintptr_t>(dh) & 15) == 0, "swiglu: buffers must be 16-byte aligned");
     switch (dtype) {
-        case CINN_BF16: return swiglu_typed((const __nv_bfloat16*)h12, (const __nv_bfloat16*)dh, (__nv_bfloat16*)out, T_rows, I, backward != 0, st);
-        case CINN_F16: return swiglu_typed((const __half*)h12, (const __half*)dh, (__half*)out, T_rows, I, backward != 0, st);
-        case CINN_F32: return swiglu_typed((const float*)h12, (const float*)dh, (float*)out, T_rows, I, backward != 0, st);
+        case CINN_BF16: return swiglu_typed((const __nv_bfloat16*)h12, (const __nv_bfloat16*)dh, (__nv_bfloat16*)out, T_rows, I, backward != 0, round != 0, st);
+        case CINN_F16: return swiglu_typed((const __half*)h12, (const __half*)dh, (__half*)out, T_rows, I, backward != 0, round != 0, st);
+        case CINN_F32: return swiglu_typed((const float*)h12, (const float*)dh, (float*)out, T_rows, I, backward != 0, round != 0, st);
         default: set_error("swiglu: unknown dtype tag %d", dtype); return CINN_ERR_INVALID;
     }
 }

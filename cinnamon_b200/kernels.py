@@ -546,6 +546,25 @@ class FP8Linear(torch.nn.Module):
         return fp8_linear
 
 
+def has_hooks(module: torch.nn.Module) -> bool:
+    return bool(module._forward_hooks or module._forward_pre_hooks or module._backward_hooks or module._backward_pre_hooks)
+
+
+def swiglu_block_ready(x, w1, w2, w3) -> bool:
+    """Whether ``w3(silu(w1(x)) * w2(x))`` can run as one native node: three plain ``FP8Linear`` layers, the first two alike."""
+    layers = (w1, w2, w3)
+    return (all(type(m) is FP8Linear and m.bias is None and not m.cache_quantized_weight and not has_hooks(m)
+                and m.weight.dtype in _DTYPE_TAG and m.weight.is_cuda for m in layers)
+            and gemm_events is None and w1.round_scale == w2.round_scale and w1.weight.shape == w2.weight.shape
+            and w1.weight.dtype == w2.weight.dtype and w1.weight.shape[0] % 128 == 0 and x.shape[-1] == w1.weight.shape[1]
+            and w3.weight.shape[1] == w1.weight.shape[0] and x.numel() > 0 and x.shape[-1] % 16 == 0)
+
+
+def swiglu_block(x, w1, w2, w3) -> torch.Tensor:
+    """``w3(silu(w1(x)) * w2(x))`` of three FP8 linears with x quantised once and w1, w2 as one GEMM (csrc/host/moe_train.cpp)."""
+    return _host.swiglu_block(x, w1.weight, w2.weight, w3.weight, w1.round_scale, w3.round_scale, _KMAJOR_BACKWARD, _DIV_MODE)
+
+
 def convert_to_fp8(model: torch.nn.Module, exclude_names: list = None) -> torch.nn.Module:
     """Swap eligible ``nn.Linear`` modules for ``FP8Linear`` in place (reference
     src/kernels.py:843-905): names containing embedding / lm_head / router / norm /

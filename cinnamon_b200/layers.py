@@ -39,6 +39,10 @@ class SwiGLU(nn.Module):
         self.w3 = nn.Linear(hidden_dim, d_model, bias=False)
 
     def forward(self, x):
+        if x.is_cuda and not torch.compiler.is_compiling():
+            from . import kernels as K
+            if K.swiglu_block_ready(x, self.w1, self.w2, self.w3):
+                return K.swiglu_block(x, self.w1, self.w2, self.w3)
         return self.w3(F.silu(self.w1(x)) * self.w2(x))
 
 
@@ -130,15 +134,41 @@ class MoE(nn.Module):
                              "by the first call")
         return self._peer
 
+    def _native_ready(self, flat, shared_out):
+        """Whether the routed part can run as one native autograd node (``_forward_native``): every expert on this GPU, plain
+        modules without hooks, e4m3 experts of widths the fused weight gradient takes."""
+        from . import kernels as K
+        ex, r = self.routed_experts, self.router
+        plain = (type(ex) is GroupedExperts and type(r) is nn.Linear and r.bias is None and not K.has_hooks(ex) and not K.has_hooks(r))
+        return (plain and not self.sharded and flat.shape[0] > 0 and not torch.compiler.is_compiling() and K.gemm_events is None
+                and K._MOE_GROUPED_PRECISION == "fp8" and ex.d_model % 256 == 0 and ex.hidden_dim % 256 == 0
+                and all(w.dtype in (torch.float32, torch.bfloat16) and w.is_contiguous() for w in (ex.w12, ex.w3))
+                and flat.dtype in K._DTYPE_TAG and shared_out.dtype in K._DTYPE_TAG and self.expert_bias.dtype == torch.float32
+                and (torch.is_autocast_enabled("cuda") or flat.dtype == r.weight.dtype))
+
+    def _forward_native(self, flat, shared_out, batch, seq):
+        """Router, routed experts and combine as one native autograd node (csrc/host/moe_train.cpp)."""
+        from . import kernels as K
+        ex = self.routed_experts
+        y, balance, counts = K._host.moe_block(flat.contiguous(), self.router.weight, ex.w12, ex.w3,
+                                               shared_out.reshape(flat.shape).contiguous(), self.expert_bias, *K.cached_expert_weights(ex.w12),
+                                               *K.cached_expert_weights(ex.w3), self.top_k, batch, float(self.balance_alpha),
+                                               torch.is_autocast_enabled("cuda"), K._DIV_MODE)
+        if self.training:
+            K._host.moe_update_bias(self.expert_bias, counts, flat.shape[0] * self.top_k / self.n_routed, self.gamma)
+        return y.view(batch, seq, -1), balance
+
     def forward(self, x):
         batch, seq, d = x.shape
         shared_out = self.shared_experts[0](x) if len(self.shared_experts) == 1 else sum(e(x) for e in self.shared_experts)
         flat = x.reshape(-1, d)
+        if flat.is_cuda and self._native_ready(flat, shared_out):
+            return self._forward_native(flat, shared_out, batch, seq)
         logits = self.router(flat)
         scores = torch.sigmoid(logits.float())
         if flat.is_cuda:
             from . import kernels as K
-            r = K.moe_route(logits.detach().float(), self.expert_bias, self.top_k)
+            r = K.moe_route(logits.detach(), self.expert_bias, self.top_k)
             routing = _moe.Routing(token_indices=r["token_indices"], sorted_scores=r["sorted_scores"],
                                    sorted_experts=r["sorted_experts"], counts=r["counts"], pair_pos=r["pair_pos"],
                                    pair_gate=r["pair_gate"])

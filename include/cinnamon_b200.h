@@ -289,6 +289,27 @@ int cinn_lightning_indexer(const void* q, const void* k, const void* w, int dtyp
 int cinn_swiglu(const void* h12, void* h, int dtype, int64_t T, int64_t I, void* stream);
 int cinn_swiglu_backward(const void* h12, const void* grad_h, void* grad_h12, int dtype, int64_t T, int64_t I, void* stream);
 
+/* The same with silu(h1) rounded to the activation type before the product, forward and backward: `F.silu(w1(x)) * w2(x)`
+ * on 16-bit tensors (the shared experts, src/layers.py:27-31). */
+int cinn_swiglu_rounded(const void* h12, void* h, int dtype, int64_t T, int64_t I, void* stream);
+int cinn_swiglu_rounded_backward(const void* h12, const void* grad_h, void* grad_h12, int dtype, int64_t T, int64_t I, void* stream);
+
+/* Sequence-wise balance loss (src/layers.py:167-177) from the router's logits (batch * seq, n_experts) and the selection
+ * top_experts (batch * seq, top_k): share (batch, n_experts) = selections * n_experts / (top_k * seq), and
+ * *loss = alpha * mean over sequences of sum_e share * mean normalised score. */
+int64_t cinn_moe_balance_workspace_bytes(int64_t batch, int64_t seq, int n_experts);
+int cinn_moe_balance_loss(const void* logits, int logits_dtype, const int* top_experts, int64_t batch, int64_t seq, int n_experts,
+                          int top_k, float alpha, void* workspace, float* share, float* loss, void* stream);
+
+/* Gradient of the logits from those of the normalised gates (d_gates (batch * seq, top_k) in the order of pair_pos; null:
+ * zero) and of the balance loss (share as left by the forward and the device scalar d_loss; null: no such loss). */
+int cinn_moe_gates_backward(const void* logits, int logits_dtype, const int64_t* sorted_experts, const int64_t* pair_pos,
+                            const float* d_gates, const float* share, const float* d_loss, float alpha, int64_t batch, int64_t seq,
+                            int n_experts, int top_k, void* d_logits, void* stream);
+
+/* bias[e] += counts[e] > expected ? -gamma : gamma, clamped to [-1, 1] (src/layers.py:111-116) */
+int cinn_moe_update_bias(const int64_t* counts, float* bias, int n_experts, float expected, float gamma, void* stream);
+
 /* Dispatch gather of quantised tokens: out_q[r, :] = q[idx[r], :], out_scales[r, :] = scales[idx[r], :] for
  * r < n_out, in one pass (the `flat_x[token_indices]` of MoE.forward, src/layers.py:140, on tokens that were
  * quantised once before the gather).  q: (n_src, d) e4m3 bytes, d a multiple of 16; scales: (n_src, n_scales)

@@ -140,3 +140,38 @@ def test_sharded_moe_block_trains_like_the_unsharded_one_on_gpus(K, tmp_path, ex
     for rank in range(2):
         text = (tmp_path / f"ok_{rank}").read_text()
         assert text == "[True, True, True, True, True, True, True] status 0", f"rank {rank}: {text}"
+
+
+@pytest.mark.parametrize("case", [(2, 40, 8, 2, 256, 512, 0.01), (1, 129, 33, 3, 256, 1024, 0.0), (3, 64, 300, 6, 512, 512, 0.02)])
+@pytest.mark.parametrize("autocast", [True, False])
+def test_native_block_matches_the_module_path(K, case, autocast):
+    """The block as native autograd nodes against the same block run through its modules (a forward hook on an inner module
+    selects that path): outputs, balance loss, bias update and every gradient.  The two differ where bf16 or e4m3 rounding
+    meets sums in another order (x's gradient adds its parts before one rounding instead of after several)."""
+    from cinnamon_b200 import layers
+    B, L, E, k, d, h, alpha = case
+    torch.manual_seed(E)
+    with torch.device("cuda"):
+        a = layers.MoE(E, 1, k, d, h, 2, 0.01, alpha)
+        b = layers.MoE(E, 1, k, d, h, 2, 0.01, alpha)
+    b.load_state_dict(a.state_dict())
+    a, b = K.convert_to_fp8(a).train(), K.convert_to_fp8(b).train()
+    for m in (b.shared_experts[0].w1, b.router):
+        m.register_forward_hook(lambda *args: None)
+    x = torch.randn(B, L, d, device="cuda")
+    dy = torch.randn(B, L, d, device="cuda")
+    got = []
+    for block in (a, b):
+        xi = x.clone().requires_grad_(True)
+        with torch.autocast("cuda", dtype=torch.bfloat16, enabled=autocast):
+            y, bal = block(xi)
+        ((y.float() * dy).sum() + (bal * 3.0 if bal is not None else 0.0)).backward()
+        got.append((y, bal, xi.grad, dict(block.named_parameters()), block.expert_bias))
+    (y0, b0, gx0, p0, eb0), (y1, b1, gx1, p1, eb1) = got
+    rel = lambda u, v: float((u.float() - v.float()).norm() / v.float().norm())                   # noqa: E731
+    assert rel(y0, y1) < 1e-3 and torch.equal(eb0, eb1) and (b0 is None) == (b1 is None)
+    if b0 is not None:
+        assert abs(float(b0) - float(b1)) < 1e-5 * abs(float(b1)) + 1e-9
+    assert gx0.dtype == gx1.dtype and rel(gx0, gx1) < 1e-2
+    for name, p in p0.items():
+        assert p.grad.dtype == p1[name].grad.dtype and rel(p.grad, p1[name].grad) < 1e-2, name
