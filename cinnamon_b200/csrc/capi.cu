@@ -43,6 +43,8 @@ int swiglu_quant_rowwise(const void* h12, int dtype, int64_t T_rows, int64_t I, 
 int fp8_gemm(const void* A, const float* sA, int64_t ld_sa, const void* B, const float* sB, int64_t sbk, int64_t sbn,
              void* C, int64_t M, int64_t N, int64_t K, int b_layout, int out_dtype, cudaStream_t st, void* workspace,
              int64_t workspace_bytes);
+int quantize_block_beside(const void* x, int dtype, int64_t M, int64_t N, int64_t ld_m, int64_t ld_n, void* q, void* q_t, float* scales,
+                          int round_scale, int div_mode, cudaStream_t st);
 int64_t fp8_gemm_workspace_bytes(int64_t M, int64_t N, int64_t K, int b_layout);
 int fp8_grouped_gemm(const void* A, const float* sA, const void* W, const float* sW, const int64_t* starts,
                      const int64_t* ends, int64_t E, int64_t T, int64_t d_in, int64_t d_out, void* C, int out_dtype,
@@ -155,6 +157,11 @@ int cinn_quant_blockwise(const void* x, int x_dtype, int64_t M, int64_t N, int64
 int cinn_quant_blockwise_t(const void* x, int x_dtype, int64_t M, int64_t N, int64_t ld, void* q, void* q_t, float* scales,
                            int round_scale, int div_mode, void* stream) {
     return cinn::quantize_block_t(x, x_dtype, M, N, ld, q, q_t, scales, round_scale, div_mode, (cudaStream_t)stream);
+}
+
+int cinn_quant_block_beside(const void* x, int x_dtype, int64_t M, int64_t N, int64_t ld_m, int64_t ld_n, void* q, void* q_t,
+                            float* scales, int round_scale, int div_mode, void* stream) {
+    return cinn::quantize_block_beside(x, x_dtype, M, N, ld_m, ld_n, q, q_t, scales, round_scale, div_mode, (cudaStream_t)stream);
 }
 
 int cinn_quant_rowwise_dual(const void* x, int x_dtype, int64_t M, int64_t N, int64_t ld, void* q_row, float* s_row,

@@ -48,6 +48,24 @@ void set_error(const char* fmt, ...);
 
 #define CINN_CHECK_LAUNCH()  CINN_CHECK_CUDA(cudaGetLastError())
 
+// Programmatic dependent launch.  A kernel launched by launch_dependent may start while the one before it on the stream is
+// still running, as soon as every block of that one has called pdl_trigger (or has ended); nothing it reads or writes in
+// global memory may come before its pdl_wait, which returns when the kernel before has finished and its writes are visible.
+// What is won is the launch latency and the prologue, which between kernels of 3 - 10 us are a quarter of the time.
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+template <typename... P, typename... A>
+inline cudaError_t launch_dependent(void (*kern)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A&&... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid; cfg.blockDim = block; cfg.dynamicSmemBytes = smem; cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr; cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...);
+}
+
 int sm_count();   // SMs of the current device (cached per device)
 
 // ---- arithmetic shared by every quantiser ---------------------------------

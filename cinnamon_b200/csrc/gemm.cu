@@ -303,6 +303,8 @@ fp8_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(TMEM_COLS) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
+    pdl_wait();                                    // (all of the above is this block's own; from here on, memory is read)
+    pdl_trigger();
     if constexpr (GROUPED) {
         if (warp == 0) tile_prefix_sum(p, cum, BM, lane);
     }
@@ -675,8 +677,7 @@ static int launch(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMa
     const size_t smem = smem_bytes(GROUPED ? p.E : 0);
     int rc = allow_smem_once<kern>(smem_bytes(GROUPED ? MAX_EXPERTS : 0));
     if (rc) return rc;
-    kern<<<grid, THREADS, smem, st>>>(ta, tb, tc, p);
-    CINN_CHECK_LAUNCH();
+    CINN_CHECK_CUDA(launch_dependent(kern, grid, THREADS, smem, st, ta, tb, tc, p));
     return CINN_OK;
 }
 
@@ -707,13 +708,15 @@ static int launch_pair(const CUtensorMap& ta, const CUtensorMap& tb, const CUten
     cfg.blockDim = dim3(pair::PTHREADS, 1, 1);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
-    cudaLaunchAttribute attr[1];
+    cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = 2;
     attr[0].val.clusterDim.y = 1;
     attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = 2;
     CINN_CHECK_CUDA(cudaLaunchKernelEx(&cfg, kern, ta, tb, tc, p));
     return CINN_OK;
 }
@@ -764,6 +767,7 @@ template <int OUT>
 __global__ void __launch_bounds__(256)
 split_sum_kernel(const float* __restrict__ part, void* __restrict__ out, int64_t n, int splits) {
     using T = typename OutT<OUT>::type;
+    pdl_wait();
     const int64_t i = ((int64_t)blockIdx.x * 256 + threadIdx.x) * 4;
     if (i >= n) return;
     float a[4] = {0.f, 0.f, 0.f, 0.f};
@@ -798,10 +802,10 @@ split_sum_kernel(const float* __restrict__ part, void* __restrict__ out, int64_t
 static int launch_split_sum(const float* part, void* out, int64_t n, int splits, int out_dtype, cudaStream_t st) {
     const unsigned grid = (unsigned)((n + 1023) / 1024);
     switch (out_dtype) {
-        case CINN_BF16: split_sum_kernel<CINN_BF16><<<grid, 256, 0, st>>>(part, out, n, splits); break;
-        case CINN_F32: split_sum_kernel<CINN_F32><<<grid, 256, 0, st>>>(part, out, n, splits); break;
-        case CINN_F16: split_sum_kernel<CINN_F16><<<grid, 256, 0, st>>>(part, out, n, splits); break;
-        case CINN_F32_BF16: split_sum_kernel<CINN_F32_BF16><<<grid, 256, 0, st>>>(part, out, n, splits); break;
+        case CINN_BF16: CINN_CHECK_CUDA(launch_dependent(split_sum_kernel<CINN_BF16>, grid, 256, 0, st, part, out, n, splits)); break;
+        case CINN_F32: CINN_CHECK_CUDA(launch_dependent(split_sum_kernel<CINN_F32>, grid, 256, 0, st, part, out, n, splits)); break;
+        case CINN_F16: CINN_CHECK_CUDA(launch_dependent(split_sum_kernel<CINN_F16>, grid, 256, 0, st, part, out, n, splits)); break;
+        case CINN_F32_BF16: CINN_CHECK_CUDA(launch_dependent(split_sum_kernel<CINN_F32_BF16>, grid, 256, 0, st, part, out, n, splits)); break;
         default: set_error("GEMM: unknown output dtype tag %d", out_dtype); return CINN_ERR_INVALID;
     }
     CINN_CHECK_LAUNCH();

@@ -23,7 +23,7 @@ using at::Tensor;
 
 #define CINN_HOST_API(X)                                                                                            \
     X(cinn_last_error) X(cinn_quant_rowwise) X(cinn_quant_rowwise_dual) X(cinn_quant_rowwise_with_block)             \
-    X(cinn_quant_rowwise_with_block_t) X(cinn_quant_blockwise) X(cinn_quant_blockwise_t) X(cinn_transpose_bytes)     \
+    X(cinn_quant_rowwise_with_block_t) X(cinn_quant_blockwise) X(cinn_quant_block_beside) X(cinn_transpose_bytes)     \
     X(cinn_requant_row_to_block) X(cinn_fp8_gemm_ws) X(cinn_fp8_gemm_workspace_bytes) \
     X(cinn_sparse_attn_workspace_bytes) X(cinn_sparse_attn_fwd_ws) X(cinn_sparse_attn_bwd) X(cinn_sparse_attn_bwd_ws)                  \
     X(cinn_moe_route_workspace_ints) X(cinn_moe_route_ranges) X(cinn_spread_rows) X(cinn_fp8_grouped_gemm)                \

@@ -56,12 +56,14 @@ Linear linear_forward(const Tensor& x, const Tensor& weight, bool round_scale, b
         // comes out of the same pass
         if (kmajor && need_dgrad && N % 16 == 0 && K % 4 == 0 && wf.stride(1) == 1 && wf.stride(0) % 4 == 0) {
             r.w_t = empty({K, N}, F8, dev);
-            check(api.cinn_quant_blockwise_t(wf.data_ptr(), tag_of(wf.scalar_type()), N, K, wf.stride(0), r.w.data_ptr(),
-                                             r.w_t.data_ptr(), f32(r.w_scale), 0, div, stream()), "cinn_quant_blockwise_t");
-        } else {
+        }
+        if (M > 0)                              // beside the activations' quantiser just enqueued
+            check(api.cinn_quant_block_beside(wf.data_ptr(), tag_of(wf.scalar_type()), N, K, wf.stride(0), wf.stride(1), r.w.data_ptr(),
+                                              r.w_t.defined() ? r.w_t.data_ptr() : nullptr, f32(r.w_scale), 0, div, stream()),
+                  "cinn_quant_blockwise");
+        else                                    // (no token: nobody reads the transposed copy)
             check(api.cinn_quant_blockwise(wf.data_ptr(), tag_of(wf.scalar_type()), N, K, wf.stride(0), wf.stride(1), r.w.data_ptr(),
                                            f32(r.w_scale), 128, 128, 0, div, stream()), "cinn_quant_blockwise");
-        }
         ++launches;
     }
     r.out = gemm(xq, xs, r.w, 0, r.w_scale, r.w_scale.stride(1), r.w_scale.stride(0), M, N, K, at::kBFloat16, TAG_BF16);

@@ -48,39 +48,46 @@ __device__ __forceinline__ Raw8c<T> load_raw8c(const T* p) {
     return r;
 }
 
-// One CTA per token; for few tokens the columns are spread over blockIdx.y as well.  The vectors of four rows are fetched, as
-// stored, before any is added: bound by reading the rows once (32768 tokens x 8 rows of 7168: 5.2 GB in 0.77 ms; 1.04 ms with one row at a time).
-template <typename T>
+// per_token threads (a power of two) per token; for few tokens the columns are spread over blockIdx.y as well.  The vectors of
+// U rows are fetched, as stored, before any is added: bound by reading the rows once (32768 tokens x 8 rows of 7168: 5.2 GB in
+// 0.77 ms; 1.04 ms with one row at a time).
+template <typename T, int U>
 __global__ void __launch_bounds__(256)
 moe_combine_kernel(const T* __restrict__ rows, const int64_t* __restrict__ pos, const float* __restrict__ gates,
-                   const void* __restrict__ addend, int addend_dtype, float* __restrict__ y, int64_t n_rows, int top_k,
-                   int d) {
-    __shared__ int64_t s_pos[kMaxTopK + 4];
-    __shared__ float s_gate[kMaxTopK + 4];
-    const int64_t t = blockIdx.x;
-    if (threadIdx.x < kMaxTopK + 4) {
+                   const void* __restrict__ addend, int addend_dtype, float* __restrict__ y, int64_t n_tokens, int64_t n_rows,
+                   int top_k, int d, int per_token) {
+    constexpr int SLOTS = 256;                         // (token, slot) pairs of a CTA kept in shared memory
+    __shared__ int64_t s_pos[SLOTS];
+    __shared__ float s_gate[SLOTS];
+    const int tokens = 256 / per_token, slots = (top_k + U - 1) / U * U;
+    const int tl = threadIdx.x / per_token, x = threadIdx.x - tl * per_token;
+    const int64_t t0 = (int64_t)blockIdx.x * tokens, t = t0 + tl;
+    for (int i = threadIdx.x; i < tokens * slots; i += 256) {
+        const int a = i / slots, j = i - a * slots;
         int64_t p = -1;
-        if (threadIdx.x < top_k) {
-            p = pos[t * top_k + threadIdx.x];
-            s_gate[threadIdx.x] = gates ? gates[t * top_k + threadIdx.x] : 1.0f;      // null: plain sum
+        if (j < top_k && t0 + a < n_tokens) {
+            p = pos[(t0 + a) * top_k + j];
+            s_gate[i] = gates ? gates[(t0 + a) * top_k + j] : 1.0f;      // null: plain sum
         }
-        s_pos[threadIdx.x] = (p >= 0 && p < n_rows) ? p : -1;
+        s_pos[i] = (p >= 0 && p < n_rows) ? p : -1;
     }
     __syncthreads();
-    for (int c = (blockIdx.y * 256 + threadIdx.x) * 8; c < d; c += gridDim.y * 256 * 8) {
+    if (t >= n_tokens) return;
+    const int64_t* my_pos = s_pos + tl * slots;
+    const float* my_gate = s_gate + tl * slots;
+    for (int c = (blockIdx.y * per_token + x) * 8; c < d; c += gridDim.y * per_token * 8) {
         float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-        for (int j0 = 0; j0 < top_k; j0 += 4) {
-            Raw8c<T> raw[4];
+        for (int j0 = 0; j0 < top_k; j0 += U) {
+            Raw8c<T> raw[U];
 #pragma unroll
-            for (int u = 0; u < 4; ++u) {          // (a slot without a row reads the first one, whose value goes nowhere)
-                if (n_rows > 0) raw[u] = load_raw8c<T>(rows + (s_pos[j0 + u] < 0 ? 0 : s_pos[j0 + u]) * d + c);
-            }
+            for (int u = 0; u < U; ++u)            // (a slot without a row reads the first one, whose value goes nowhere)
+                if (n_rows > 0) raw[u] = load_raw8c<T>(rows + (my_pos[j0 + u] < 0 ? 0 : my_pos[j0 + u]) * d + c);
 #pragma unroll
-            for (int u = 0; u < 4; ++u) {
-                if (s_pos[j0 + u] < 0) continue;
+            for (int u = 0; u < U; ++u) {
+                if (my_pos[j0 + u] < 0) continue;
                 float v[8];
                 load8f<T>(reinterpret_cast<const T*>(&raw[u]), v);
-                const float g = s_gate[j0 + u];
+                const float g = my_gate[j0 + u];
 #pragma unroll
                 for (int i = 0; i < 8; ++i) acc[i] = __fadd_rn(acc[i], __fmul_rn(v[i], g));   // product then sum, as the reference
             }
@@ -99,6 +106,18 @@ moe_combine_kernel(const T* __restrict__ rows, const int64_t* __restrict__ pos, 
     }
 }
 
+template <typename T>
+static void launch_combine(const T* rows, const int64_t* pos, const float* gates, const void* addend, int addend_dtype, float* y,
+                           int64_t n_tokens, int64_t n_rows, int top_k, int d, cudaStream_t st) {
+    int per = 256;                                     // a narrow row needs fewer threads (512 columns: 64)
+    while (per > 32 && per / 2 * 8 >= d) per /= 2;
+    const int64_t tokens = 256 / per;
+    const bool few = n_tokens < 4 * sm_count() && d <= 32768;
+    const dim3 grid((unsigned)((n_tokens + tokens - 1) / tokens), few ? (unsigned)((d + per * 8 - 1) / (per * 8)) : 1u);
+    if (top_k <= 2) moe_combine_kernel<T, 2><<<grid, 256, 0, st>>>(rows, pos, gates, addend, addend_dtype, y, n_tokens, n_rows, top_k, d, per);
+    else moe_combine_kernel<T, 4><<<grid, 256, 0, st>>>(rows, pos, gates, addend, addend_dtype, y, n_tokens, n_rows, top_k, d, per);
+}
+
 int moe_combine(const void* rows, int dtype, const int64_t* pos, const float* gates, const void* addend, int addend_dtype,
                 void* y, int64_t n_tokens, int64_t n_rows, int top_k, int64_t d, cudaStream_t st) {
     CINN_CHECK_ARG(n_tokens >= 0 && n_rows >= 0 && d >= 0, "moe_combine: negative shape");
@@ -112,11 +131,10 @@ int moe_combine(const void* rows, int dtype, const int64_t* pos, const float* ga
     CINN_CHECK_ARG(addend == nullptr || addend_dtype == CINN_BF16 || addend_dtype == CINN_F16 || addend_dtype == CINN_F32,
                    "moe_combine: unknown addend dtype tag %d", addend_dtype);
     CINN_CHECK_ARG((reinterpret_cast<uintptr_t>(addend) & 15) == 0, "moe_combine: the addend must be 16-byte aligned");
-    const dim3 grid((unsigned)n_tokens, n_tokens >= 4 * sm_count() || d > 32768 ? 1u : (unsigned)((d + 2047) / 2048));
     switch (dtype) {
-        case CINN_BF16: moe_combine_kernel<__nv_bfloat16><<<grid, 256, 0, st>>>((const __nv_bfloat16*)rows, pos, gates, addend, addend_dtype, (float*)y, n_rows, top_k, (int)d); break;
-        case CINN_F16: moe_combine_kernel<__half><<<grid, 256, 0, st>>>((const __half*)rows, pos, gates, addend, addend_dtype, (float*)y, n_rows, top_k, (int)d); break;
-        case CINN_F32: moe_combine_kernel<float><<<grid, 256, 0, st>>>((const float*)rows, pos, gates, addend, addend_dtype, (float*)y, n_rows, top_k, (int)d); break;
+        case CINN_BF16: launch_combine((const __nv_bfloat16*)rows, pos, gates, addend, addend_dtype, (float*)y, n_tokens, n_rows, top_k, (int)d, st); break;
+        case CINN_F16: launch_combine((const __half*)rows, pos, gates, addend, addend_dtype, (float*)y, n_tokens, n_rows, top_k, (int)d, st); break;
+        case CINN_F32: launch_combine((const float*)rows, pos, gates, addend, addend_dtype, (float*)y, n_tokens, n_rows, top_k, (int)d, st); break;
         default: set_error("moe_combine: unknown dtype tag %d", dtype); return CINN_ERR_INVALID;
     }
     CINN_CHECK_LAUNCH();

@@ -112,6 +112,7 @@ template <typename T, int DIV, bool ROUND, int UNROLL>
 __global__ void __launch_bounds__(256)
 quant_row_vec_kernel(const T* __restrict__ x, int64_t ld, uint8_t* __restrict__ q, float* __restrict__ scales,
                      int N, int nb, int64_t total_tiles, int step_rows, int step_cols) {
+    pdl_trigger();
     // the n-th tile of this half-warp is hw + n * n_hw; (step_rows, step_cols) = divmod(n_hw, nb)
     const int sub = threadIdx.x & 15;
     const int64_t hw = (int64_t)blockIdx.x * 16 + (threadIdx.x >> 4);
@@ -543,6 +544,7 @@ quant_row_dual_kernel(const T* __restrict__ x, int64_t ld, uint8_t* __restrict__
                       uint8_t* __restrict__ q_col, float* __restrict__ s_col, int M, int N, int nb_n, int nb_m) {
     __shared__ __align__(16) float s_amax[8][128];
     __shared__ __align__(16) uint8_t s_out[128 * 128];
+    pdl_trigger();
     const int sub = threadIdx.x & 15, hw = threadIdx.x >> 4;
     const int n = blockIdx.x * 128 + sub * 8;
     const int mt = blockIdx.y * 128 + hw * 8;
@@ -597,6 +599,7 @@ quant_row_dual_tma_kernel(const __grid_constant__ CUtensorMap tmX, uint8_t* __re
     const int sub = threadIdx.x & 15, hw = threadIdx.x >> 4;
     const int stride = gridDim.x;
 
+    pdl_trigger();
     if (threadIdx.x == 0) {
         for (int s = 0; s < DUAL_STAGES; ++s) mbar_init(full0 + 8 * s, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -730,8 +733,9 @@ quant_row_dual_seg_kernel(const __grid_constant__ CUtensorMap tmX, uint8_t* __re
 template <typename T, int DIV, bool ROUND>
 __global__ void __launch_bounds__(256)
 quant_block_vec_kernel(const T* __restrict__ x, int64_t ld, uint8_t* __restrict__ q, float* __restrict__ scales,
-                       int M, int N, int nb) {
+                       int M, int N, int nb, int beside) {
     __shared__ float s_red[8];
+    pdl_trigger();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int r0 = blockIdx.y * 128, c = blockIdx.x * 128 + lane * 4;
     float v[16][4];
@@ -767,6 +771,7 @@ quant_block_vec_kernel(const T* __restrict__ x, int64_t ld, uint8_t* __restrict_
             *reinterpret_cast<uint32_t*>(q + (int64_t)r * N + c) = o;
         }
     }
+    if (beside) pdl_wait();
 }
 
 // 4 x 4 byte transpose in registers: r[i] holds bytes (row i, columns 0..3); c[j] receives (rows 0..3, column j).
@@ -807,9 +812,10 @@ __device__ __forceinline__ void store_tile_transposed(const uint32_t (&blk)[4][4
 template <typename T, int DIV, bool ROUND>
 __global__ void __launch_bounds__(256)
 quant_block_vec_t_kernel(const T* __restrict__ x, int64_t ld, uint8_t* __restrict__ q, uint8_t* __restrict__ q_t,
-                         float* __restrict__ scales, int M, int N, int nb) {
+                         float* __restrict__ scales, int M, int N, int nb, int beside) {
     __shared__ float s_red[8];
     __shared__ uint32_t s_t[128 * 32];
+    pdl_trigger();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int r0 = blockIdx.y * 128, c = blockIdx.x * 128 + lane * 4;
     float v[16][4];
@@ -850,6 +856,7 @@ quant_block_vec_t_kernel(const T* __restrict__ x, int64_t ld, uint8_t* __restric
         transpose4x4_bytes(rows, blk[a]);
     }
     store_tile_transposed(blk, s_t, q_t, M, r0, blockIdx.x * 128, M, N);
+    if (beside) pdl_wait();
 }
 
 // Block-wise, arbitrary strides / block sizes: one CTA per block, two passes.
@@ -1091,6 +1098,7 @@ swiglu_quant_row_kernel(const T* __restrict__ h12, uint8_t* __restrict__ q, floa
                         const int64_t* __restrict__ n_rows_dev) {
     // optional row count that only the device knows (an expert-parallel rank's received rows): rows past it are skipped
     if (n_rows_dev != nullptr) total_tiles = min(total_tiles, max(n_rows_dev[0], (int64_t)0) * nb);
+    pdl_trigger();
     // the n-th tile of this half-warp is hw + n * n_hw; (step_rows, step_cols) = divmod(n_hw, nb): tile
     // coordinates advance without a division in the loop
     const int sub = threadIdx.x & 15;
@@ -1228,6 +1236,15 @@ transpose_bytes_vec_kernel(const uint8_t* __restrict__ in, int64_t ld_in, uint8_
 // ---------------------------------------------------------------------------
 // host-side dispatch
 // ---------------------------------------------------------------------------
+// The weight's quantiser runs beside the activations' (quantize_block_beside): its blocks start with the other kernel still at
+// work, read and write nothing that one touches, and wait for it only before they end, so that whatever is launched next and
+// waits for this kernel has waited for both.
+static thread_local bool t_beside = false;
+struct BesidePrevious {
+    BesidePrevious() { t_beside = true; }
+    ~BesidePrevious() { t_beside = false; }
+};
+
 static inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
 
 template <typename T, int DIV, bool ROUND>
@@ -1273,7 +1290,8 @@ static int launch_blockwise(const T* x, int64_t M, int64_t N, int64_t ld_m, int6
     dim3 grid((unsigned)nb, (unsigned)mb);
     const bool a = sizeof(T) == 4 ? aligned16(x) : ((reinterpret_cast<uintptr_t>(x) & 7) == 0);
     if (bm == 128 && bn == 128 && ld_n == 1 && N % 4 == 0 && ld_m % 4 == 0 && a && (reinterpret_cast<uintptr_t>(q) & 3) == 0) {
-        quant_block_vec_kernel<T, DIV, ROUND><<<grid, 256, 0, st>>>(x, ld_m, q, scales, (int)M, (int)N, nb);
+        if (t_beside) CINN_CHECK_CUDA(launch_dependent(quant_block_vec_kernel<T, DIV, ROUND>, grid, 256, 0, st, x, ld_m, q, scales, (int)M, (int)N, nb, 1));
+        else quant_block_vec_kernel<T, DIV, ROUND><<<grid, 256, 0, st>>>(x, ld_m, q, scales, (int)M, (int)N, nb, 0);
     } else {
         quant_block_generic_kernel<T, DIV, ROUND><<<grid, 256, 0, st>>>(x, ld_m, ld_n, q, scales, (int)M, (int)N, bm, bn, nb);
     }
@@ -1287,7 +1305,11 @@ static int dispatch_block_t(const T* x, int64_t M, int64_t N, int64_t ld, uint8_
     const int mb = (int)((M + 127) / 128), nb = (int)((N + 127) / 128);
     CINN_CHECK_ARG(mb <= 65535, "block-wise quantiser: more than 65535 row blocks (%d)", mb);
     dim3 grid((unsigned)nb, (unsigned)mb);
-#define CINN_B(DIV, RND) quant_block_vec_t_kernel<T, DIV, RND><<<grid, 256, 0, st>>>(x, ld, q, q_t, scales, (int)M, (int)N, nb)
+#define CINN_B(DIV, RND) \
+    do { \
+        if (t_beside) CINN_CHECK_CUDA(launch_dependent(quant_block_vec_t_kernel<T, DIV, RND>, grid, 256, 0, st, x, ld, q, q_t, scales, (int)M, (int)N, nb, 1)); \
+        else quant_block_vec_t_kernel<T, DIV, RND><<<grid, 256, 0, st>>>(x, ld, q, q_t, scales, (int)M, (int)N, nb, 0); \
+    } while (0)
     if (div_mode == CINN_DIV_FULL) { if (round_scale) CINN_B(CINN_DIV_FULL, true); else CINN_B(CINN_DIV_FULL, false); }
     else                           { if (round_scale) CINN_B(CINN_DIV_RN, true);   else CINN_B(CINN_DIV_RN, false); }
 #undef CINN_B
@@ -1312,6 +1334,18 @@ int quantize_block_t(const void* x, int dtype, int64_t M, int64_t N, int64_t ld,
         case CINN_F32:  return dispatch_block_t((const float*)x, M, N, ld, (uint8_t*)q, (uint8_t*)q_t, scales, round_scale, div_mode, st);
         default: set_error("block quantiser (+ transposed copy): unknown dtype tag %d", dtype); return CINN_ERR_INVALID;
     }
+}
+
+// quantize (128 x 128 blocks) or, with q_t, quantize_block_t, beside the kernel enqueued last on the stream: a quantiser of
+// this library that shares no memory with this one's inputs and outputs.
+int quantize(bool blockwise, const void* x, int dtype, int64_t M, int64_t N, int64_t ld_m, int64_t ld_n, void* q,
+             float* scales, int bm, int bn, int round_scale, int div_mode, cudaStream_t st);
+int quantize_block_beside(const void* x, int dtype, int64_t M, int64_t N, int64_t ld_m, int64_t ld_n, void* q, void* q_t, float* scales,
+                          int round_scale, int div_mode, cudaStream_t st) {
+    BesidePrevious scope;
+    CINN_CHECK_ARG(q_t == nullptr || ld_n == 1, "block quantiser (+ transposed copy): rows must be contiguous");
+    return q_t ? quantize_block_t(x, dtype, M, N, ld_m, q, q_t, scales, round_scale, div_mode, st)
+               : quantize(true, x, dtype, M, N, ld_m, ld_n, q, scales, 128, 128, round_scale, div_mode, st);
 }
 
 template <typename T>

@@ -130,6 +130,12 @@ int cinn_swiglu_quant_rowwise_n(const void* h12, int dtype, int64_t T, int64_t I
  * e4m3 operands (src/kernels.py:748). */
 int cinn_transpose_bytes(const void* in, int64_t ld_in, void* out, int64_t R, int64_t C, void* stream);
 
+/* The 128 x 128 block quantiser (q_t not null: with the byte-transposed copy, as cinn_quant_blockwise_t) for a matrix that
+ * shares no memory with the call enqueued last on this stream, which must have been a quantiser of this library that had
+ * something to do: the two run side by side.  What is enqueued next is ordered after both. */
+int cinn_quant_block_beside(const void* x, int x_dtype, int64_t M, int64_t N, int64_t ld_m, int64_t ld_n, void* q, void* q_t,
+                            float* scales, int round_scale, int div_mode, void* stream);
+
 /* Block-scaled FP8 GEMM:  C[M, N] = sum_kb (A[:, kb] * sA[:, kb]) @ (B[kb, :] * sB[kb, nb]).
  * Replaces fp8_gemm_kernel + fp8_matmul_dsv3 (src/kernels.py:588-664, 667-702).
  * A: (M, K) e4m3, K contiguous.  sA: (M, ceil(K/128)) fp32, row pitch ld_sa.
