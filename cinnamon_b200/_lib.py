@@ -28,6 +28,7 @@ SIGNATURES = {
     "cinn_quant_rowwise_with_block_t": [_vp, _i32, _i64, _i64, _i64, _vp, _vp, _vp, _vp, _i32, _i32, _vp],
     "cinn_set_wait_limit_cycles": [ctypes.c_longlong],
     "cinn_quant_blockwise_t": [_vp, _i32, _i64, _i64, _i64, _vp, _vp, _vp, _i32, _i32, _vp],
+    "cinn_quant_linear": [_vp, _i32, _i64, _i64, _vp, _vp, _i32, _vp, _i32, _i64, _i64, _vp, _vp, _i64, _i64, _i64, _i32, _vp],
     "cinn_quant_block_beside": [_vp, _i32, _i64, _i64, _i64, _i64, _vp, _vp, _vp, _i32, _i32, _vp],
     "cinn_quant_blockwise": [_vp, _i32, _i64, _i64, _i64, _i64, _vp, _vp, _i32, _i32, _i32, _i32, _vp],
     "cinn_requant_row_to_block": [_vp, _vp, _i64, _i64, _vp, _vp, _i32, _i32, _vp],

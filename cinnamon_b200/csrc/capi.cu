@@ -43,6 +43,9 @@ int swiglu_quant_rowwise(const void* h12, int dtype, int64_t T_rows, int64_t I, 
 int fp8_gemm(const void* A, const float* sA, int64_t ld_sa, const void* B, const float* sB, int64_t sbk, int64_t sbn,
              void* C, int64_t M, int64_t N, int64_t K, int b_layout, int out_dtype, cudaStream_t st, void* workspace,
              int64_t workspace_bytes);
+int quantize_linear(const void* x, int x_dtype, int64_t ldx_m, int64_t ldx_k, void* xq, float* xs, int round_scale, const void* w,
+                    int w_dtype, int64_t ldw_n, int64_t ldw_k, void* wq, float* ws, int64_t M, int64_t N, int64_t K, int div_mode,
+                    cudaStream_t st);
 int quantize_block_beside(const void* x, int dtype, int64_t M, int64_t N, int64_t ld_m, int64_t ld_n, void* q, void* q_t, float* scales,
                           int round_scale, int div_mode, cudaStream_t st);
 int64_t fp8_gemm_workspace_bytes(int64_t M, int64_t N, int64_t K, int b_layout);
@@ -157,6 +160,13 @@ int cinn_quant_blockwise(const void* x, int x_dtype, int64_t M, int64_t N, int64
 int cinn_quant_blockwise_t(const void* x, int x_dtype, int64_t M, int64_t N, int64_t ld, void* q, void* q_t, float* scales,
                            int round_scale, int div_mode, void* stream) {
     return cinn::quantize_block_t(x, x_dtype, M, N, ld, q, q_t, scales, round_scale, div_mode, (cudaStream_t)stream);
+}
+
+int cinn_quant_linear(const void* x, int x_dtype, int64_t ldx_m, int64_t ldx_k, void* xq, float* xs, int round_scale, const void* w,
+                      int w_dtype, int64_t ldw_n, int64_t ldw_k, void* wq, float* ws, int64_t M, int64_t N, int64_t K, int div_mode,
+                      void* stream) {
+    return cinn::quantize_linear(x, x_dtype, ldx_m, ldx_k, xq, xs, round_scale, w, w_dtype, ldw_n, ldw_k, wq, ws, M, N, K, div_mode,
+                                 (cudaStream_t)stream);
 }
 
 int cinn_quant_block_beside(const void* x, int x_dtype, int64_t M, int64_t N, int64_t ld_m, int64_t ld_n, void* q, void* q_t,

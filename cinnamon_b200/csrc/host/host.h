@@ -23,14 +23,14 @@ using at::Tensor;
 
 #define CINN_HOST_API(X)                                                                                            \
     X(cinn_last_error) X(cinn_quant_rowwise) X(cinn_quant_rowwise_dual) X(cinn_quant_rowwise_with_block)             \
-    X(cinn_quant_rowwise_with_block_t) X(cinn_quant_blockwise) X(cinn_quant_block_beside) X(cinn_transpose_bytes)     \
+    X(cinn_quant_rowwise_with_block_t) X(cinn_quant_blockwise) X(cinn_quant_block_beside) X(cinn_quant_linear) X(cinn_transpose_bytes)     \
     X(cinn_requant_row_to_block) X(cinn_fp8_gemm_ws) X(cinn_fp8_gemm_workspace_bytes) \
     X(cinn_sparse_attn_workspace_bytes) X(cinn_sparse_attn_fwd_ws) X(cinn_sparse_attn_bwd) X(cinn_sparse_attn_bwd_ws)                  \
     X(cinn_moe_route_workspace_ints) X(cinn_moe_route_ranges) X(cinn_spread_rows) X(cinn_fp8_grouped_gemm)                \
     X(cinn_swiglu_quant_rowwise) X(cinn_moe_combine) X(cinn_moe_combine_add)                \
     X(cinn_swiglu_rounded) X(cinn_swiglu_rounded_backward) X(cinn_moe_balance_workspace_bytes) X(cinn_moe_balance_loss)     \
     X(cinn_moe_gates_backward) X(cinn_moe_update_bias) X(cinn_moe_combine_backward) X(cinn_swiglu_backward)                 \
-    X(cinn_fp8_grouped_wgrad_fused_scratch_bytes) X(cinn_fp8_grouped_wgrad_fused) X(cinn_fp8_grouped_gemm_dgrad)
+    X(cinn_fp8_grouped_wgrad_fused_scratch_bytes) X(cinn_fp8_grouped_wgrad_fused) X(cinn_fp8_grouped_gemm_dgrad) X(cinn_zero_rows_outside)
 
 struct Api {
 #define CINN_DECL(name) decltype(&::name) name = nullptr;
@@ -106,7 +106,7 @@ std::tuple<Tensor, Tensor> linear_backward(const Tensor& grad_out, Tensor x, Ten
 struct Quantised { Tensor q, s; };
 Quantised rowwise(const Tensor& x, bool round_scale, int div);                 // moe.cpp
 Quantised swiglu_quantised(const Tensor& h12, int div);
-Tensor grouped(const Quantised& x, const Quantised& w, const Tensor& starts, const Tensor& ends);
+Tensor grouped(const Quantised& x, const Quantised& w, const Tensor& starts, const Tensor& ends, at::ScalarType type = at::kBFloat16);
 struct Routes {                                 // moe_route's outputs, in three tensors
     Tensor longs, floats, top;                  // token_indices | sorted_experts | pair_pos | counts | starts | ends; scores | pair_gate
     int64_t pairs = 0, E = 0;

@@ -133,6 +133,31 @@ std::tuple<Tensor, Tensor> linear_backward(const Tensor& grad_out, Tensor x, Ten
 }
 
 
+// Without gradients nothing but the result outlives the call: one scratch buffer, one launch for both quantisers.
+static Tensor linear_inference(const Tensor& x, const Tensor& weight, bool round_scale, int div) {
+    require(x.is_cuda(), "Input must be on CUDA");
+    c10::cuda::CUDAGuard guard(x.device());
+    const int64_t K = x.size(-1), N = weight.size(0), nkb = up(K, 128);
+    const Tensor xf = readable(x.dim() == 2 ? x : x.reshape({-1, K})), wf = readable(weight);
+    const int64_t M = xf.size(0);
+    auto shape = x.sizes().vec();
+    shape.back() = N;
+    Tensor out = empty(shape, at::kBFloat16, x.device());
+    const auto room = [](int64_t bytes) { return (bytes + 255) / 256 * 256; };
+    const int64_t o_xs = room(M * K), o_wq = o_xs + room(4 * M * nkb), o_ws = o_wq + room(N * K), o_part = o_ws + room(4 * up(N, 128) * nkb);
+    const int64_t need = api.cinn_fp8_gemm_workspace_bytes(M, N, K, 0);            // few tiles, long reduction: cut along K
+    Tensor buf = empty({o_part + need}, at::kByte, x.device());
+    uint8_t* b = buf.data_ptr<uint8_t>();
+    float *xs = reinterpret_cast<float*>(b + o_xs), *ws = reinterpret_cast<float*>(b + o_ws);
+    check(api.cinn_quant_linear(xf.data_ptr(), tag_of(xf.scalar_type()), xf.stride(0), xf.stride(1), b, xs, round_scale, wf.data_ptr(),
+                                tag_of(wf.scalar_type()), wf.stride(0), wf.stride(1), b + o_wq, ws, M, N, K, div, stream()),
+          "cinn_quant_linear");
+    check(api.cinn_fp8_gemm_ws(b, xs, nkb, b + o_wq, ws, 1, nkb, out.data_ptr(), M, N, K, 0, TAG_BF16, need ? b + o_part : nullptr, need,
+                               stream()), "cinn_fp8_gemm");
+    launches += need ? 3 : 2;
+    return out;
+}
+
 namespace {
 
 struct CachedWeight { Tensor q, s, q_t; };      // a weight already in e4m3 (undefined: quantise it here), handed around the node's tensors
@@ -186,6 +211,7 @@ void bind_linear(pybind11::module_& m) {
         const CachedWeight cached{or_none(wq), or_none(ws), or_none(wqt)};
         if (at::GradMode::is_enabled() && (x.requires_grad() || w.requires_grad()))
             return LinearNode::apply(x, w, round_scale, kmajor, (int64_t)div, &cached);
+        if (!cached.q.defined()) return linear_inference(x, w, round_scale, div);
         return linear_forward(x, w, round_scale, false, false, kmajor, div, cached.q, cached.s, cached.q_t).out;
     });
 }

@@ -23,11 +23,11 @@ Quantised swiglu_quantised(const Tensor& h12, int div) {
     return r;
 }
 
-Tensor grouped(const Quantised& x, const Quantised& w, const Tensor& starts, const Tensor& ends) {
+Tensor grouped(const Quantised& x, const Quantised& w, const Tensor& starts, const Tensor& ends, at::ScalarType type) {
     const int64_t T = x.q.size(0), E = w.q.size(0), d_out = w.q.size(1), d_in = w.q.size(2);
-    Tensor out = empty({T, d_out}, at::kBFloat16, x.q.device());
+    Tensor out = empty({T, d_out}, type, x.q.device());
     check(api.cinn_fp8_grouped_gemm(x.q.data_ptr(), f32(x.s), w.q.data_ptr(), f32(w.s), starts.data_ptr<int64_t>(),
-                                    ends.data_ptr<int64_t>(), E, T, d_in, d_out, out.data_ptr(), TAG_BF16, stream()),
+                                    ends.data_ptr<int64_t>(), E, T, d_in, d_out, out.data_ptr(), tag_of(type), stream()),
           "cinn_fp8_grouped_gemm");
     ++launches;
     return out;

@@ -94,23 +94,33 @@ struct BlockOptions {
     Tensor counts;                             // out: rows per expert
 };
 
-// gradients of grouped(x, w) given dy, rows of every expert contiguous and all rows covered
+// gradients of grouped(x, w) given dy; `covered`: the experts' ranges cover every row (else the others' gradients are zero)
 std::tuple<Tensor, Tensor> grouped_backward(const Tensor& dy, const Tensor& xq, const Tensor& xs, const Tensor& wq, const Tensor& ws,
                                             const Tensor& starts, const Tensor& ends, at::ScalarType w_type, bool want_x,
-                                            at::ScalarType x_type, int div) {
+                                            at::ScalarType x_type, int div, bool covered = true) {
     const int64_t R = dy.size(0), E = wq.size(0), d_out = wq.size(1), d_in = wq.size(2);
     const at::Device dev = dy.device();
     const int64_t *st = starts.data_ptr<int64_t>(), *en = ends.data_ptr<int64_t>();
     const int64_t need = api.cinn_fp8_grouped_wgrad_fused_scratch_bytes(R, E, d_in, d_out);
     Tensor scratch = empty({need}, at::kByte, dev), dw = empty({E, d_out, d_in}, w_type, dev);
     Tensor gq = empty({R, d_out}, F8, dev), gs = empty({R, d_out / 128}, at::kFloat, dev);
+    const bool one_pass = dy.scalar_type() != at::kFloat;          // both quantisations of dy from one pass: 2-byte gradients
     check(api.cinn_fp8_grouped_wgrad_fused(dy.data_ptr(), tag_of(dy.scalar_type()), xq.data_ptr(), f32(xs), st, en, E, R, d_in, d_out,
                                            scratch.data_ptr(), need, dw.data_ptr(), w_type == at::kFloat ? TAG_F32_BF16 : TAG_BF16, div,
-                                           gq.data_ptr(), f32(gs), stream()), "cinn_fp8_grouped_wgrad_fused");
+                                           one_pass ? gq.data_ptr() : nullptr, one_pass ? f32(gs) : nullptr, stream()), "cinn_fp8_grouped_wgrad_fused");
     launches += 4;
     Tensor dx;
     if (want_x) {
+        if (!one_pass) {
+            const Quantised g = rowwise(dy, false, div);
+            gq = g.q;
+            gs = g.s;
+        }
         dx = empty({R, d_in}, x_type, dev);
+        if (!covered) {
+            check(api.cinn_zero_rows_outside(dx.data_ptr(), R, d_in * dx.element_size(), st, en, E, stream()), "cinn_zero_rows_outside");
+            ++launches;
+        }
         check(api.cinn_fp8_grouped_gemm_dgrad(gq.data_ptr(), f32(gs), wq.data_ptr(), f32(ws), st, en, E, R, d_in, d_out, dx.data_ptr(),
                                               tag_of(x_type), stream()), "cinn_fp8_grouped_gemm_dgrad");
         ++launches;
@@ -227,6 +237,39 @@ struct BlockNode : public torch::autograd::Function<BlockNode> {
     }
 };
 
+// ---------------------------------------------------------------------------------------------------------------------
+// moe_grouped_gemm (reference src/kernels.py:526-581) with its gradients
+// ---------------------------------------------------------------------------------------------------------------------
+struct GroupedNode : public torch::autograd::Function<GroupedNode> {
+    static Tensor forward(AutogradContext* ctx, const Tensor& x_in, const Tensor& w, const Tensor& starts_in, const Tensor& ends_in,
+                          const Quantised* wq, at::ScalarType type, int64_t div) {
+        c10::cuda::CUDAGuard guard(x_in.device());
+        at::AutoDispatchBelowAutograd below;
+        const Tensor x = readable(x_in), starts = starts_in.to(at::kLong).contiguous(), ends = ends_in.to(at::kLong).contiguous();
+        const Quantised xq = rowwise(x, false, (int)div);
+        ctx->save_for_backward({xq.q, xq.s, wq->q, wq->s, starts, ends});
+        ctx->saved_data["n"] = std::vector<int64_t>{(int64_t)x_in.scalar_type(), (int64_t)w.scalar_type(), div};
+        return grouped(xq, *wq, starts, ends, type);
+    }
+    static variable_list backward(AutogradContext* ctx, variable_list grads) {
+        auto s = ctx->get_saved_variables();
+        const auto n = ctx->saved_data["n"].toIntVector();
+        Tensor dx, dw;
+        as_python_error([&] {
+            c10::cuda::CUDAGuard guard(s[0].device());
+            const Tensor dy = readable(grads[0]).contiguous();
+            const auto x_type = (at::ScalarType)n[0], w_type = (at::ScalarType)n[1];
+            const auto dx_type = tag_of(x_type) < 0 ? at::kFloat : x_type;
+            const auto dw_type = w_type == at::kBFloat16 ? at::kBFloat16 : at::kFloat;
+            std::tie(dx, dw) = grouped_backward(dy, s[0], s[1], s[2], s[3], s[4], s[5], dw_type, ctx->needs_input_grad(0), dx_type, (int)n[2],
+                                                false);
+            if (dx.defined()) dx = dx.to(x_type);
+            dw = dw.to(w_type);
+        });
+        return {dx, dw, Tensor(), Tensor(), Tensor(), Tensor(), Tensor()};
+    }
+};
+
 }  // namespace
 
 void bind_moe_train(pybind11::module_& m) {
@@ -234,6 +277,15 @@ void bind_moe_train(pybind11::module_& m) {
                              int div) {
         const SwiGLUOptions o{round12, round3, kmajor, div};
         return SwiGLUNode::apply(x, w1, w2, w3, &o);
+    });
+    m.def("grouped_gemm", [](const Tensor& x, const Tensor& w, const Tensor& starts, const Tensor& ends, const Tensor& w_q, const Tensor& w_s,
+                             int tag, int div) {
+        const Quantised q{w_q, w_s};
+        const auto type = tag == TAG_BF16 ? at::kBFloat16 : (tag == TAG_F16 ? at::kHalf : at::kFloat);
+        if (at::GradMode::is_enabled() && (x.requires_grad() || w.requires_grad()))
+            return GroupedNode::apply(x, w, starts, ends, &q, type, (int64_t)div);
+        c10::cuda::CUDAGuard guard(x.device());
+        return grouped(rowwise(readable(x), false, div), q, starts.to(at::kLong).contiguous(), ends.to(at::kLong).contiguous(), type);
     });
     // (y, balance loss or None, rows per expert)
     m.def("moe_block", [](const Tensor& x, const Tensor& router, const Tensor& w12, const Tensor& w3, const Tensor& addend,

@@ -109,14 +109,12 @@ __device__ __forceinline__ void unpack_raw8(const Raw8<T>& r, float (&v)[8]) {
 }
 
 template <typename T, int DIV, bool ROUND, int UNROLL>
-__global__ void __launch_bounds__(256)
-quant_row_vec_kernel(const T* __restrict__ x, int64_t ld, uint8_t* __restrict__ q, float* __restrict__ scales,
-                     int N, int nb, int64_t total_tiles, int step_rows, int step_cols) {
-    pdl_trigger();
+__device__ __forceinline__ void quant_rows(const T* __restrict__ x, int64_t ld, uint8_t* __restrict__ q, float* __restrict__ scales,
+                                           int N, int nb, int64_t total_tiles, int step_rows, int step_cols, int block, int n_blocks) {
     // the n-th tile of this half-warp is hw + n * n_hw; (step_rows, step_cols) = divmod(n_hw, nb)
     const int sub = threadIdx.x & 15;
-    const int64_t hw = (int64_t)blockIdx.x * 16 + (threadIdx.x >> 4);
-    const int64_t n_hw = (int64_t)gridDim.x * 16;
+    const int64_t hw = (int64_t)block * 16 + (threadIdx.x >> 4);
+    const int64_t n_hw = (int64_t)n_blocks * 16;
     int64_t t = hw;                                  // this half-warp's next tile to FETCH
     int row = (int)(hw / nb);
     int cb = (int)(hw - (int64_t)row * nb);
@@ -170,6 +168,14 @@ quant_row_vec_kernel(const T* __restrict__ x, int64_t ld, uint8_t* __restrict__ 
             if (sub == 0 && tile[u] >= 0) scales[tile[u]] = s;
         }
     }
+}
+
+template <typename T, int DIV, bool ROUND, int UNROLL>
+__global__ void __launch_bounds__(256)
+quant_row_vec_kernel(const T* __restrict__ x, int64_t ld, uint8_t* __restrict__ q, float* __restrict__ scales,
+                     int N, int nb, int64_t total_tiles, int step_rows, int step_cols) {
+    pdl_trigger();
+    quant_rows<T, DIV, ROUND, UNROLL>(x, ld, q, scales, N, nb, total_tiles, step_rows, step_cols, blockIdx.x, gridDim.x);
 }
 
 // ---------------------------------------------------------------------------
@@ -731,13 +737,11 @@ quant_row_dual_seg_kernel(const __grid_constant__ CUtensorMap tmX, uint8_t* __re
 // the amax and the cast, so the input is read exactly once.
 // ---------------------------------------------------------------------------
 template <typename T, int DIV, bool ROUND>
-__global__ void __launch_bounds__(256)
-quant_block_vec_kernel(const T* __restrict__ x, int64_t ld, uint8_t* __restrict__ q, float* __restrict__ scales,
-                       int M, int N, int nb, int beside) {
+__device__ __forceinline__ void quant_block(const T* __restrict__ x, int64_t ld, uint8_t* __restrict__ q, float* __restrict__ scales,
+                                            int M, int N, int nb, int bx, int by) {
     __shared__ float s_red[8];
-    pdl_trigger();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int r0 = blockIdx.y * 128, c = blockIdx.x * 128 + lane * 4;
+    const int r0 = by * 128, c = bx * 128 + lane * 4;
     float v[16][4];
 #pragma unroll
     for (int i = 0; i < 16; ++i) {
@@ -761,7 +765,7 @@ quant_block_vec_kernel(const T* __restrict__ x, int64_t ld, uint8_t* __restrict_
     for (int w = 1; w < 8; ++w) amax = fmaxf(amax, s_red[w]);
     const float s = scale_from_amax<DIV, ROUND>(amax);
     const float d = divisor_of<DIV>(s);
-    if (threadIdx.x == 0) scales[(int64_t)blockIdx.y * nb + blockIdx.x] = s;
+    if (threadIdx.x == 0) scales[(int64_t)by * nb + bx] = s;
 #pragma unroll
     for (int i = 0; i < 16; ++i) {
         const int r = r0 + warp + i * 8;
@@ -771,7 +775,30 @@ quant_block_vec_kernel(const T* __restrict__ x, int64_t ld, uint8_t* __restrict_
             *reinterpret_cast<uint32_t*>(q + (int64_t)r * N + c) = o;
         }
     }
+}
+
+template <typename T, int DIV, bool ROUND>
+__global__ void __launch_bounds__(256)
+quant_block_vec_kernel(const T* __restrict__ x, int64_t ld, uint8_t* __restrict__ q, float* __restrict__ scales,
+                       int M, int N, int nb, int beside) {
+    pdl_trigger();
+    quant_block<T, DIV, ROUND>(x, ld, q, scales, M, N, nb, blockIdx.x, blockIdx.y);
     if (beside) pdl_wait();
+}
+
+// Both quantisations of a linear without gradients in one launch: the first nb_n x nb_k blocks take the weight's 128 x 128
+// blocks, the rest the activations' rows.  For a few hundred tokens the launch is what a quantiser costs.
+template <typename TX, typename TW, int DIV, bool ROUND>
+__global__ void __launch_bounds__(256)
+quant_linear_kernel(const TX* __restrict__ x, int64_t ldx, uint8_t* __restrict__ xq, float* __restrict__ xs, int64_t total_tiles,
+                    int step_rows, int step_cols, const TW* __restrict__ w, int64_t ldw, uint8_t* __restrict__ wq,
+                    float* __restrict__ ws, int N, int K, int nb_k, int w_blocks) {
+    pdl_trigger();
+    if ((int)blockIdx.x < w_blocks)
+        quant_block<TW, DIV, false>(w, ldw, wq, ws, N, K, nb_k, blockIdx.x % nb_k, blockIdx.x / nb_k);
+    else
+        quant_rows<TX, DIV, ROUND, 2>(x, ldx, xq, xs, K, nb_k, total_tiles, step_rows, step_cols, blockIdx.x - w_blocks,
+                                      gridDim.x - w_blocks);
 }
 
 // 4 x 4 byte transpose in registers: r[i] holds bytes (row i, columns 0..3); c[j] receives (rows 0..3, column j).
@@ -1334,6 +1361,51 @@ int quantize_block_t(const void* x, int dtype, int64_t M, int64_t N, int64_t ld,
         case CINN_F32:  return dispatch_block_t((const float*)x, M, N, ld, (uint8_t*)q, (uint8_t*)q_t, scales, round_scale, div_mode, st);
         default: set_error("block quantiser (+ transposed copy): unknown dtype tag %d", dtype); return CINN_ERR_INVALID;
     }
+}
+
+template <typename TX, typename TW>
+static int launch_quant_linear(const TX* x, int64_t ldx, uint8_t* xq, float* xs, int round_scale, const TW* w, int64_t ldw, uint8_t* wq,
+                               float* ws, int64_t M, int64_t N, int64_t K, int div_mode, cudaStream_t st) {
+    const int nb = (int)((K + 127) / 128);
+    const int64_t tiles = M * nb, w_blocks = (N + 127) / 128 * nb;
+    int64_t blocks = (tiles + 31) / 32;
+    const int64_t cap = (int64_t)sm_count() * 8;
+    if (blocks > cap) blocks = cap;
+    const int64_t n_hw = blocks * 16;
+    const unsigned grid = (unsigned)(w_blocks + blocks);
+#define CINN_Q(DIV, RND) quant_linear_kernel<TX, TW, DIV, RND><<<grid, 256, 0, st>>>(x, ldx, xq, xs, tiles, (int)(n_hw / nb), (int)(n_hw % nb), w, ldw, wq, ws, (int)N, (int)K, nb, (int)w_blocks)
+    if (div_mode == CINN_DIV_FULL) { if (round_scale) CINN_Q(CINN_DIV_FULL, true); else CINN_Q(CINN_DIV_FULL, false); }
+    else                           { if (round_scale) CINN_Q(CINN_DIV_RN, true);   else CINN_Q(CINN_DIV_RN, false); }
+#undef CINN_Q
+    CINN_CHECK_LAUNCH();
+    return CINN_OK;
+}
+
+int quantize(bool blockwise, const void* x, int dtype, int64_t M, int64_t N, int64_t ld_m, int64_t ld_n, void* q,
+             float* scales, int bm, int bn, int round_scale, int div_mode, cudaStream_t st);
+// x (M, K) in 1 x 128 tiles and w (N, K) in 128 x 128 blocks: one launch where both can be read in whole vectors, else two
+int quantize_linear(const void* x, int x_dtype, int64_t ldx_m, int64_t ldx_k, void* xq, float* xs, int round_scale, const void* w,
+                    int w_dtype, int64_t ldw_n, int64_t ldw_k, void* wq, float* ws, int64_t M, int64_t N, int64_t K, int div_mode,
+                    cudaStream_t st) {
+    const bool fits = M > 0 && N > 0 && K > 0 && x && w && xq && xs && wq && ws && (div_mode == CINN_DIV_FULL || div_mode == CINN_DIV_RN) &&
+                      M < (1LL << 31) && N < (1LL << 31) && K < (1LL << 31) && (N + 127) / 128 * ((K + 127) / 128) < (1LL << 30) &&
+                      ldx_k == 1 && ldw_k == 1 && ldx_m >= 0 && ldw_n >= 0 && K % 8 == 0 && ldx_m % 8 == 0 && ldw_n % 4 == 0 &&
+                      aligned16(x) && aligned16(xq) && aligned16(w) && aligned16(wq) &&
+                      (x_dtype == CINN_BF16 || x_dtype == CINN_F16 || x_dtype == CINN_F32) && (w_dtype == CINN_F32 || w_dtype == CINN_BF16);
+    if (!fits) {
+        int rc = quantize(false, x, x_dtype, M, K, ldx_m, ldx_k, xq, xs, 1, 128, round_scale, div_mode, st);
+        return rc ? rc : quantize(true, w, w_dtype, N, K, ldw_n, ldw_k, wq, ws, 128, 128, 0, div_mode, st);
+    }
+#define CINN_QL(TX, TW) return launch_quant_linear((const TX*)x, ldx_m, (uint8_t*)xq, xs, round_scale, (const TW*)w, ldw_n, (uint8_t*)wq, ws, M, N, K, div_mode, st)
+    if (w_dtype == CINN_F32) {
+        if (x_dtype == CINN_BF16) CINN_QL(__nv_bfloat16, float);
+        if (x_dtype == CINN_F16) CINN_QL(__half, float);
+        CINN_QL(float, float);
+    }
+    if (x_dtype == CINN_BF16) CINN_QL(__nv_bfloat16, __nv_bfloat16);
+    if (x_dtype == CINN_F16) CINN_QL(__half, __nv_bfloat16);
+    CINN_QL(float, __nv_bfloat16);
+#undef CINN_QL
 }
 
 // quantize (128 x 128 blocks) or, with q_t, quantize_block_t, beside the kernel enqueued last on the stream: a quantiser of

@@ -1181,7 +1181,15 @@ def moe_grouped_gemm(sorted_x: torch.Tensor, weights: torch.Tensor, expert_start
         return grouped_gemm_16bit(sorted_x.to(torch.float16), _expert_weights_fp16(weights), expert_starts, expert_ends, dtype)
     if _ops is not None and torch.compiler.is_compiling():
         return _ops.grouped_gemm(sorted_x, weights, expert_starts, expert_ends, dtype)
-    if torch.is_grad_enabled() and (sorted_x.requires_grad or weights.requires_grad):
+    grad = torch.is_grad_enabled() and (sorted_x.requires_grad or weights.requires_grad)
+    E, d_out, d_in = weights.shape
+    if (gemm_events is None and sorted_x.ndim == 2 and sorted_x.shape[0] > 0 and sorted_x.shape[1] == d_in and dtype in _DTYPE_TAG
+            and expert_starts.numel() == E == expert_ends.numel() and E > 0 and min(sorted_x.stride()) >= 0
+            and (not grad or (d_in % 256 == 0 and d_out % 256 == 0 and E <= 1024))):
+        # quantiser, GEMM and both gradients behind one native autograd node (csrc/host/moe_train.cpp)
+        return _host.grouped_gemm(sorted_x, weights, expert_starts, expert_ends, *cached_expert_weights(weights), _DTYPE_TAG[dtype],
+                                  _DIV_MODE)
+    if grad:
         return MoEGroupedGemmFunction.apply(sorted_x, weights, expert_starts, expert_ends, dtype)
     x = sorted_x if sorted_x.stride(-1) == 1 else sorted_x.contiguous()
     x_fp8, x_scale = quantize_fp8_rowwise(x, block_size=128)

@@ -130,6 +130,12 @@ int cinn_swiglu_quant_rowwise_n(const void* h12, int dtype, int64_t T, int64_t I
  * e4m3 operands (src/kernels.py:748). */
 int cinn_transpose_bytes(const void* in, int64_t ld_in, void* out, int64_t R, int64_t C, void* stream);
 
+/* What a linear without gradients quantises, in one launch where the layouts allow: x (M, K) in 1 x 128 tiles (round_scale as
+ * in cinn_quant_rowwise), w (N, K) in 128 x 128 blocks. */
+int cinn_quant_linear(const void* x, int x_dtype, int64_t ldx_m, int64_t ldx_k, void* xq, float* xs, int round_scale, const void* w,
+                      int w_dtype, int64_t ldw_n, int64_t ldw_k, void* wq, float* ws, int64_t M, int64_t N, int64_t K, int div_mode,
+                      void* stream);
+
 /* The 128 x 128 block quantiser (q_t not null: with the byte-transposed copy, as cinn_quant_blockwise_t) for a matrix that
  * shares no memory with the call enqueued last on this stream, which must have been a quantiser of this library that had
  * something to do: the two run side by side.  What is enqueued next is ordered after both. */
