@@ -828,7 +828,7 @@ static DensePlan dense_plan(int64_t M, int64_t N, int64_t K, int b_layout, int64
     // the pair kernel wins with B K-major, the one-SM kernel with B MN-major
     DensePlan best{false, 1};
     double best_us = waves(tiles, sms) * (KB * block_us + tile_us);
-    if (pm == 2 ? pair_tiles >= sm_count() / 2 : (pm == 1 && b_layout == 0)) {
+    if (pm == 2 ? pair_tiles >= sm_count() / 2 : (pm == 1 && b_layout == 0 && M > BM)) {       // (128 rows would leave a CTA idle)
         const double us = waves(pair_tiles, sms / 2) * (KB * block_us + tile_us);
         if (us <= best_us * 1.02 || pm == 2) { best = {true, 1}; best_us = us; }
     }
