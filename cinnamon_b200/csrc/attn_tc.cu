@@ -21,6 +21,18 @@ __device__ __forceinline__ bool wait_warp(uint32_t bar, uint32_t parity, volatil
     return __all_sync(0xffffffffu, mbar_wait_bounded(bar, parity, abort_flag, code, &g_attn_status));
 }
 
+// The four warps of a warpgroup meet at a barrier in shared memory (four arrivals): bounded, so that a warp that gave up
+// leaves nobody behind.
+struct WarpgroupBarrier {
+    uint32_t bar, phase;
+    volatile int* abort_flag;
+    __device__ __forceinline__ bool sync(int code) {
+        __syncwarp();
+        if ((threadIdx.x & 31) == 0) mbar_arrive(bar);
+        return wait_warp(bar, phase++ & 1u, abort_flag, code);
+    }
+};
+
 // ---------------------------------------------------------------------------
 // what the queries picked
 // ---------------------------------------------------------------------------
@@ -615,50 +627,49 @@ __device__ __forceinline__ void store_row16(void* dst, int64_t row, int col, int
     }
 }
 
-// Adds pieces c0, c0 + STEP, ... < c1 of 16 accumulator columns to (or, the first time, writes them over) fp32 rows in
-// global memory, rounded to nearest.  The tensor core truncates its running sums at every step, which over thousands of
-// queries would show in an fp32 gradient; so the sums are taken out every few hundred steps and started afresh.  U pieces
-// are in flight at a time.
-template <int STEP, int U, typename ROW>
-__device__ __forceinline__ void flush_pieces(uint32_t taddr, int c0, int c1, bool live, bool add, bool& bad, ROW&& row_of) {
+// fp32 gradients leave tensor memory every few hundred steps and are added up in global memory, rounded to nearest: the tensor
+// core truncates its running sums at every step, which over thousands of queries would show in fp32.  A warpgroup takes
+// pieces of 16 columns x 128 rows: registers, a slot of 8 KiB (64-byte swizzle), and a TMA store (the first time) or reduce;
+// nobody reads the old values back.  (As loads, adds and stores of every thread's own row a flush took 20 000 cycles.)  Only
+// this block touches these rows and a flush waits for the one before, so the sums are the same on every run.
+constexpr int SLOT_COLS = 16, SLOT_BYTES = T * SLOT_COLS * 4;
+
+// where(c): the map and first column of piece c.  All four warps of a warpgroup call it; slots: this warpgroup's.  False: given up.
+template <int SLOTS, typename WHERE>
+__device__ __forceinline__ bool flush_tma(uint32_t taddr, WarpgroupBarrier& all, int code, int c0, int c1, int step, uint32_t slots, int row, int plane, bool first,
+                                          bool live, bool& bad, WHERE&& where) {
+    const int quarter = (threadIdx.x >> 5) & 3, lane = threadIdx.x & 31, r = quarter * 32 + lane;
+    const bool elected = quarter == 0 && lane == 0;
+    if (elected && !first) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");      // the flush before has been added
+    int n = 0;
 #pragma unroll 1
-    for (int c = c0; c < c1; c += U * STEP) {
-        float o[U][16];
-        float4 old[U][4];
-        float* dst[U];
-        int n[U];
-        bool vec[U];
+    for (int c = c0; c < c1; c += step, ++n) {
+        float o[16];
+        tc_ld16(taddr + c * 16, o);
+        const uint32_t slot = slots + (n % SLOTS) * SLOT_BYTES;
+        if (elected && n >= SLOTS) asm volatile("cp.async.bulk.wait_group.read %0;" ::"n"(SLOTS - 1) : "memory");
+        if (!all.sync(code)) return false;
 #pragma unroll
-        for (int u = 0; u < U; ++u) {
-            n[u] = 0;
-            vec[u] = false;
-            if (c + STEP * u >= c1) continue;
-            dst[u] = row_of(c + STEP * u, n[u]);              // the piece's place and how many of its columns exist
-            n[u] = live ? n[u] : 0;
-            vec[u] = n[u] == 16 && (reinterpret_cast<uintptr_t>(dst[u]) & 15) == 0;
-            if (add && vec[u])
-#pragma unroll
-                for (int i = 0; i < 4; ++i) old[u][i] = reinterpret_cast<const float4*>(dst[u])[i];
-            tc_ld16(taddr + (c + STEP * u) * 16, o[u]);
-#pragma unroll
-            for (int i = 0; i < 16; ++i) bad |= live && !(fabsf(o[u][i]) <= 3.4e38f);
+        for (int i = 0; i < 4; ++i) {
+            bad |= live && !(fabsf(o[4 * i]) <= 3.4e38f && fabsf(o[4 * i + 1]) <= 3.4e38f && fabsf(o[4 * i + 2]) <= 3.4e38f &&
+                             fabsf(o[4 * i + 3]) <= 3.4e38f);
+            asm volatile("st.shared.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(slot + r * 64 + ((i ^ ((r >> 1) & 3)) << 4)), "f"(o[4 * i]),
+                         "f"(o[4 * i + 1]), "f"(o[4 * i + 2]), "f"(o[4 * i + 3]) : "memory");
         }
-#pragma unroll
-        for (int u = 0; u < U; ++u) {
-            if (vec[u]) {
-#pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                    float4 x = make_float4(o[u][4 * i], o[u][4 * i + 1], o[u][4 * i + 2], o[u][4 * i + 3]);
-                    if (add) { x.x += old[u][i].x; x.y += old[u][i].y; x.z += old[u][i].z; x.w += old[u][i].w; }
-                    reinterpret_cast<float4*>(dst[u])[i] = x;
-                }
-            } else {
-#pragma unroll
-                for (int i = 0; i < 16; ++i)
-                    if (i < n[u]) dst[u][i] = (add ? dst[u][i] : 0.0f) + o[u][i];
+        fence_async_smem();
+        if (!all.sync(code)) return false;
+        if (elected) {
+            int x;
+            const CUtensorMap* m = where(c, x);
+            if (m) {
+                if (first) tma_store_3d(m, slot, x, row, plane);
+                else tma_add_3d(m, slot, x, row, plane);
             }
+            tma_store_commit();
         }
     }
+    if (elected) tma_store_wait_read();                    // the slots are free again
+    return all.sync(code);
 }
 
 // Shared memory of the query pass: queries and output gradients resident, a ring of key / value panels.  Of three parts
@@ -667,19 +678,22 @@ __device__ __forceinline__ void flush_pieces(uint32_t taddr, int c0, int c1, boo
 template <int NS, int ND, int NV> struct QPassShape {
     static constexpr int KEPT = NS > 1 ? 2 : 1;            // resident parts
     static constexpr int FIXED = KEPT * (ND + NV);
-    static constexpr int RING = FIXED > 8 ? 14 - FIXED : 6;
-    static constexpr int BAR_OFF = (FIXED + RING) * PANEL;
+    static constexpr int RING = FIXED > 7 ? 13 - FIXED : 6;
+    static constexpr int SLOT_OFF = (FIXED + RING) * PANEL;        // one slot per warpgroup
+    static constexpr int BAR_OFF = SLOT_OFF + 2 * SLOT_BYTES;
     static constexpr int BYTES = BAR_OFF + 256 + 1024;
 };
 
 // Query pass: one CTA per 128 queries of a head, over their key tiles.  S = q k^T and dP = dO v^T in tensor memory; a
 // thread (a query, half of the tile's keys) turns them into p = exp(scale S - lse) and dS = p (dP - delta) scale, leaves
-// both by rank for the key pass, and writes dS back as an A operand for dq += dS k.  All of tensor memory: 128 columns of
+// both by rank for the key pass, and writes dS back as an A operand for dq += dS k.  (Collecting a row's values in shared
+// memory to store them together took twice as long as these scattered stores.)  All of tensor memory: 128 columns of
 // S under the second and third parts of dS, 128 of dP, 64 of dS's leading parts, 192 of dq.
 template <int NS, int ND, int NV>
 __global__ void __launch_bounds__(FWD_THREADS, 1)
 attn_bwd_query_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
-                      const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmG, const BwdArgs a) {
+                      const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmG,
+                      const __grid_constant__ CUtensorMap tmDQ, const BwdArgs a) {
     using S = QPassShape<NS, ND, NV>;
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
@@ -687,8 +701,9 @@ attn_bwd_query_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
     uint64_t* bars = reinterpret_cast<uint64_t*>(smem + S::BAR_OFF);
     const uint32_t full0 = smem_u32(bars), empty0 = smem_u32(bars + S::RING), qfull = smem_u32(bars + 2 * S::RING);
     const uint32_t sfull = qfull + 8, dsready = qfull + 16, done = qfull + 24, taken = qfull + 32;
-    constexpr int EVERY = 2;                              // fp32 gradients: tiles between two flushes
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * S::RING + 5);
+    constexpr int EVERY = 1;                              // fp32 gradients: tiles between two flushes
+    const uint32_t group0 = qfull + 40;                   // the two warpgroups' own barriers
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * S::RING + 7);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     int qt, bh;
@@ -699,6 +714,7 @@ attn_bwd_query_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
         *abort_flag = 0;
         for (int i = 0; i < S::RING; ++i) { mbar_init(full0 + 8 * i, 1); mbar_init(empty0 + 8 * i, 1); }
         mbar_init(qfull, 1); mbar_init(sfull, 1); mbar_init(dsready, 8); mbar_init(done, 1); mbar_init(taken, 8);
+        for (int i = 0; i < 2; ++i) mbar_init(group0 + 8 * i, 4);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 9) tc_alloc(smem_u32(tmem_slot), 512);
@@ -845,13 +861,13 @@ attn_bwd_query_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
         uint32_t rank = __ldg(before);
         uint32_t rounds = 0;                              // sums of dq taken out so far
         bool bad = false;
+        const uint32_t slots = smem_u32(smem + S::SLOT_OFF) + h * SLOT_BYTES;
+        WarpgroupBarrier group{group0 + 8 * h, 0, abort_flag};
         auto take = [&] {
             if (!wait_warp(done, rounds & 1, abort_flag, (9 << 8) | 6)) return false;
             tc_fence_after();
-            flush_pieces<2, 2>(t_dq + lanes, h, ND * 4, live, rounds > 0, bad, [&](int c, int& cols) {
-                cols = max(0, min(16, a.Dqk - c * 16));
-                return static_cast<float*>(a.dq) + row * a.Dqk + c * 16;
-            });
+            if (!flush_tma<1>(t_dq + lanes, group, (9 << 8) | 8, h, ND * 4, 2, slots, q0, bh, rounds == 0, live, bad,
+                                        [&](int c, int& x) { x = c * 16; return x < a.Dqk ? &tmDQ : nullptr; })) return false;
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive(taken);
@@ -918,6 +934,7 @@ attn_bwd_query_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
             }
         }
         if (live && bad) *a.flag = 1;
+        if (quarter == 0 && lane == 0) tma_store_wait_all();
     }
     tc_fence_before();
     __syncthreads();
@@ -931,8 +948,9 @@ attn_bwd_query_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
 template <int NS, int ND, int NV> struct KPassShape {
     static constexpr int SUB = 32 * 128;                   // 32 rows of a 64-column panel
     static constexpr int PANELS = NS * (ND + NV), STAGE = PANELS * SUB;
-    static constexpr int STAGES = (14 * PANEL) / STAGE < 8 ? (14 * PANEL) / STAGE : 8;
-    static constexpr int BAR_OFF = STAGES * STAGE;
+    static constexpr int STAGES = (12 * PANEL) / STAGE < 8 ? (12 * PANEL) / STAGE : 8;
+    static constexpr int SLOT_OFF = STAGES * STAGE;
+    static constexpr int BAR_OFF = SLOT_OFF + 4 * SLOT_BYTES;
     static constexpr int BYTES = BAR_OFF + 256 + 1024;
 };
 
@@ -945,7 +963,8 @@ constexpr int KEY_THREADS = 18 * 32;       // four producing warpgroups, TMA war
 
 template <int NS, int ND, int NV>
 __global__ void __launch_bounds__(KEY_THREADS, 1)
-attn_bwd_key_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmG, const BwdArgs a) {
+attn_bwd_key_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmG,
+                    const __grid_constant__ CUtensorMap tmDK, const __grid_constant__ CUtensorMap tmDV, const BwdArgs a) {
     using S = KPassShape<NS, ND, NV>;
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
@@ -954,9 +973,10 @@ attn_bwd_key_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
     const uint32_t full0 = smem_u32(bars), empty0 = smem_u32(bars + S::STAGES);
     const uint32_t ready0 = smem_u32(bars + 2 * S::STAGES), free0 = ready0 + 32;        // [operand][buffer]
     const uint32_t done = ready0 + 64, taken = ready0 + 72;
-    constexpr int EVERY = 8;                               // fp32 gradients: chunks between two flushes
+    constexpr int EVERY = 4;                               // fp32 gradients: chunks between two flushes
     const bool flush = NS > 1 && a.tag == CINN_F32;
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * S::STAGES + 10);
+    const uint32_t group0 = ready0 + 80;                   // the four warpgroups' own barriers
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * S::STAGES + 14);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     int kt, bh;
@@ -968,6 +988,7 @@ attn_bwd_key_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
         for (int i = 0; i < S::STAGES; ++i) { mbar_init(full0 + 8 * i, 1); mbar_init(empty0 + 8 * i, 1); }
         for (int i = 0; i < 4; ++i) { mbar_init(ready0 + 8 * i, 4); mbar_init(free0 + 8 * i, 1); }
         mbar_init(done, 1); mbar_init(taken, 16);
+        for (int i = 0; i < 4; ++i) mbar_init(group0 + 8 * i, 4);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 17) tc_alloc(smem_u32(tmem_slot), 512);
@@ -1046,16 +1067,21 @@ attn_bwd_key_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
         };
         const int64_t row = (int64_t)bh * a.L + min(s, a.L - 1);
         uint32_t rounds = 0;                               // sums taken out so far
+        WarpgroupBarrier group{group0 + 8 * (warp >> 2), 0, abort_flag};
         bool bad = false;
         auto take = [&] {
             if (!wait_warp(done, rounds & 1, abort_flag, (10 << 8) | 5)) return false;
             tc_fence_after();
-            flush_pieces<4, 1>(t_dk + lanes, warp >> 2, (ND + NV) * 4, s < a.L, rounds > 0, bad, [&](int c, int& cols) {      // dk, then dv
+            const int wg = warp >> 2;
+            const bool ok = flush_tma<1>(t_dk + lanes, group, (10 << 8) | 7, wg, (ND + NV) * 4, 4,
+                                                   smem_u32(smem + S::SLOT_OFF) + wg * SLOT_BYTES, k0, bh, rounds == 0, s < a.L, bad,
+                                                   [&](int c, int& x) -> const CUtensorMap* {                // dk, then dv
                 const bool is_v = c >= ND * 4;
-                const int col = (is_v ? c - ND * 4 : c) * 16, width = is_v ? a.Dv : a.Dqk;
-                cols = max(0, min(16, width - col));
-                return static_cast<float*>(is_v ? a.dv : a.dk) + row * width + col;
+                x = (is_v ? c - ND * 4 : c) * 16;
+                if (x >= (is_v ? a.Dv : a.Dqk)) return nullptr;
+                return is_v ? &tmDV : &tmDK;
             });
+            if (!ok) return false;
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive(taken);
@@ -1100,6 +1126,7 @@ attn_bwd_key_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
             }
         }
         if (s < a.L && bad) *a.flag = 1;
+        if (quarter == 0 && lane == 0) tma_store_wait_all();
     }
     tc_fence_before();
     __syncthreads();
@@ -1291,21 +1318,22 @@ int forward(const void* q, const void* k, const void* v, int dtype, const int64_
 }
 
 template <int NS, int ND, int NV>
-static int launch_bwd(const CUtensorMap (&m)[6], const BwdArgs& a, const Plan& p, cudaStream_t st) {
+static int launch_bwd(const CUtensorMap (&m)[9], const BwdArgs& a, const Plan& p, cudaStream_t st) {
     auto qk = attn_bwd_query_kernel<NS, ND, NV>;
     auto kk = attn_bwd_key_kernel<NS, ND, NV>;
     const unsigned grid = (unsigned)(p.Lp / T * p.BH);
     CINN_CHECK_CUDA(cudaFuncSetAttribute(qk, cudaFuncAttributeMaxDynamicSharedMemorySize, QPassShape<NS, ND, NV>::BYTES));
     CINN_CHECK_CUDA(cudaFuncSetAttribute(kk, cudaFuncAttributeMaxDynamicSharedMemorySize, KPassShape<NS, ND, NV>::BYTES));
-    qk<<<grid, FWD_THREADS, QPassShape<NS, ND, NV>::BYTES, st>>>(m[0], m[1], m[2], m[3], a);
+    qk<<<grid, FWD_THREADS, QPassShape<NS, ND, NV>::BYTES, st>>>(m[0], m[1], m[2], m[3], m[6], a);
     CINN_CHECK_LAUNCH();
-    kk<<<grid, KEY_THREADS, KPassShape<NS, ND, NV>::BYTES, st>>>(m[4], m[5], a);
+    kk<<<grid, KEY_THREADS, KPassShape<NS, ND, NV>::BYTES, st>>>(m[4], m[5], m[7], m[8], a);
     CINN_CHECK_LAUNCH();
     return CINN_OK;
 }
 
 int64_t backward_workspace_bytes(int64_t B, int64_t H, int64_t L, int64_t K, int64_t Dqk, int64_t Dv, int dtype) {
     if (!supported(B, H, L, K, Dqk, Dv)) return 0;
+    if (dtype == CINN_F32 && (Dqk % 4 != 0 || Dv % 4 != 0)) return 0;                // rows a TMA box cannot address
     const Plan p = make_plan(B, H, L, K, Dqk, Dv, dtype, true);
     return dense_pays(p, true) ? p.bytes : 0;
 }
@@ -1339,13 +1367,20 @@ int backward(const void* d_out, const float* out, const float* lse, const void* 
         default: delta_kernel<__nv_bfloat16><<<dgrid, 256, 0, st>>>((const __nv_bfloat16*)d_out, out, delta, rows, (int)Dv); break;
     }
     CINN_CHECK_LAUNCH();
-    CUtensorMap m[6];                                      // q, k, v, dO in boxes of 128 rows; q, dO in boxes of 32
+    CUtensorMap m[9];                                      // q, k, v, dO in boxes of 128 rows; q, dO in boxes of 32; dq, dk, dv
     if ((rc = operand_map(p, &m[0], q, ws + p.q_off, Dqk, p.dp))) return rc;
     if ((rc = operand_map(p, &m[1], k, ws + p.k_off, Dqk, p.dp))) return rc;
     if ((rc = operand_map(p, &m[2], v, ws + p.v_off, Dv, p.nv * 64))) return rc;
     if ((rc = operand_map(p, &m[3], d_out, ws + p.g_off, Dv, p.nv * 64))) return rc;
     if ((rc = operand_map(p, &m[4], q, ws + p.q_off, Dqk, p.dp, 32))) return rc;
     if ((rc = operand_map(p, &m[5], d_out, ws + p.g_off, Dv, p.nv * 64, 32))) return rc;
+    m[6] = m[7] = m[8] = m[0];
+    if (dtype == CINN_F32) {
+        const struct { void* p; int64_t d; } outs[3] = {{dq, Dqk}, {dk, Dqk}, {dv, Dv}};
+        for (int i = 0; i < 3; ++i)
+            if ((rc = encode_map_3d(&m[6 + i], outs[i].p, (uint64_t)outs[i].d, (uint64_t)L, (uint64_t)p.BH, (uint64_t)outs[i].d * 4, T,
+                                    CU_TENSOR_MAP_DATA_TYPE_FLOAT32, SLOT_COLS, CU_TENSOR_MAP_SWIZZLE_64B))) return rc;
+    }
     BwdArgs a{};
     a.picks = picks_of(p, ws);
     a.lse = lse; a.delta = delta; a.p = reinterpret_cast<float*>(ws + p.p_off); a.ds = reinterpret_cast<float*>(ws + p.ds_off);

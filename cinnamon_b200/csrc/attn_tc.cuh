@@ -86,6 +86,20 @@ __device__ __forceinline__ void tma_load_3d(const CUtensorMap* map, uint32_t bar
         ::"r"(dst), "l"(map), "r"(bar), "r"(x), "r"(y), "r"(z) : "memory");
 }
 
+// a box of shared memory to global memory, written or added (fp32, rounded to nearest, in L2)
+__device__ __forceinline__ void tma_store_3d(const CUtensorMap* map, uint32_t src, int x, int y, int z) {
+    asm volatile("cp.async.bulk.tensor.3d.global.shared::cta.bulk_group [%0, {%2, %3, %4}], [%1];"
+                 ::"l"(map), "r"(src), "r"(x), "r"(y), "r"(z) : "memory");
+}
+__device__ __forceinline__ void tma_add_3d(const CUtensorMap* map, uint32_t src, int x, int y, int z) {
+    asm volatile("cp.reduce.async.bulk.tensor.3d.global.shared::cta.add.bulk_group [%0, {%2, %3, %4}], [%1];"
+                 ::"l"(map), "r"(src), "r"(x), "r"(y), "r"(z) : "memory");
+}
+// *(smem float at addr) = x if take is not zero, as a predicated instruction
+__device__ __forceinline__ void store_shared_if(uint32_t addr, float x, uint32_t take) {
+    asm volatile("{\n\t.reg .pred t;\n\tsetp.ne.u32 t, %2, 0;\n\t@t st.shared.f32 [%0], %1;\n\t}" ::"r"(addr), "f"(x), "r"(take) : "memory");
+}
+
 // two fp32 values as three packed bf16 pairs whose sum they are
 __device__ __forceinline__ void split2(float a, float b, uint32_t& hi, uint32_t& mid, uint32_t& lo) {
     auto pack = [](float x, float y) {

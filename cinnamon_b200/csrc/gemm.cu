@@ -599,19 +599,19 @@ int encode_map_2d(CUtensorMap* map, const void* base, uint64_t inner, uint64_t r
     return CINN_OK;
 }
 
-// 3-D map of 2-byte elements: `planes` matrices of (rows, inner), boxes of 64 columns x box_rows of one matrix, 128-byte
-// swizzle; rows past a matrix's end read as zeros instead of its neighbour's
+// 3-D map: `planes` matrices of (rows, inner), boxes of box_inner columns x box_rows of one matrix; rows past a matrix's end
+// read as zeros instead of its neighbour's, and are not written
 int encode_map_3d(CUtensorMap* map, const void* base, uint64_t inner, uint64_t rows, uint64_t planes, uint64_t pitch_bytes,
-                  uint32_t box_rows, CUtensorMapDataType dtype) {
+                  uint32_t box_rows, CUtensorMapDataType dtype, uint32_t box_inner, CUtensorMapSwizzle swizzle) {
     EncodeFn enc = get_encode();
     if (!enc) { set_error("cuTensorMapEncodeTiled is not available from the CUDA driver"); return CINN_ERR_CUDA; }
     cuuint64_t dims[3] = {inner, rows, planes};
     cuuint64_t strides[2] = {pitch_bytes, pitch_bytes * rows};
-    cuuint32_t box[3] = {64, box_rows, 1};
+    cuuint32_t box[3] = {box_inner, box_rows, 1};
     cuuint32_t estr[3] = {1, 1, 1};
     auto go = [&] {
         return enc(map, dtype, 3, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                   CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+                   swizzle, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     };
     CUresult r = go();
     if (r == CUDA_ERROR_INVALID_CONTEXT || r == CUDA_ERROR_NOT_INITIALIZED) { cudaFree(nullptr); r = go(); }

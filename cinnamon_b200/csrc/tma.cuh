@@ -49,6 +49,7 @@ int encode_map_2d(CUtensorMap* map, const void* base, uint64_t inner, uint64_t r
                   uint32_t box_inner, uint32_t box_rows, CUtensorMapDataType dtype, CUtensorMapSwizzle swizzle);
 
 int encode_map_3d(CUtensorMap* map, const void* base, uint64_t inner, uint64_t rows, uint64_t planes, uint64_t pitch_bytes,
-                  uint32_t box_rows, CUtensorMapDataType dtype);
+                  uint32_t box_rows, CUtensorMapDataType dtype, uint32_t box_inner = 64,
+                  CUtensorMapSwizzle swizzle = CU_TENSOR_MAP_SWIZZLE_128B);
 
 }  // namespace cinn
