@@ -586,7 +586,7 @@ delta_kernel(const U* __restrict__ d_out, const float* __restrict__ out, float* 
 struct BwdArgs {
     Picks picks;
     const float* lse; const float* delta;
-    float* p; float* ds;                   // (B H, L, K) by rank: probability times count, and its score gradient
+    float2* pd;                            // (B H, L, K) by rank: probability times count, and its score gradient
     void* dq; void* dk; void* dv;          // in `tag`'s type
     int* flag;
     int H, L, words, K, Dqk, Dv, BH, n_tiles, group, tag;
@@ -854,8 +854,7 @@ attn_bwd_query_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
         const bool repeats = a.picks.repeats[b * a.n_tiles + qt] != 0;
         const uint8_t* count = a.picks.count + qrow * a.K;
         const float lse = a.lse[row], delta = a.delta[row];
-        float* prow = a.p + row * a.K;
-        float* dsrow = a.ds + row * a.K;
+        float2* pdrow = a.pd + row * a.K;
         bool alive = true;
         uint2 mine = live ? __ldg(bits) : make_uint2(0u, 0u);
         uint32_t rank = __ldg(before);
@@ -900,16 +899,15 @@ attn_bwd_query_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
                     for (int i = 0; i < 32; ++i)
                         if (bit & (1u << i)) p[i] *= (float)*cnt++;
                 }
-                float* pp = prow + at0;
-                float* dp = dsrow + at0;
+                // (one 8-byte store for both: the store unit takes a line per lane and instruction, and that bounds this phase)
+                float2* pd = pdrow + at0;
                 uint32_t at = 0;
 #pragma unroll
                 for (int i = 0; i < 32; ++i) {
                     const uint32_t pick = bit & (1u << i);
                     const float ds = p[i] * (__uint_as_float(dv[i]) - delta) * a.scale;
-                    store_if(pp + at, p[i], pick);
+                    store2_if(pd + at, p[i], ds, pick);
                     p[i] = pick ? ds : 0.0f;
-                    store_if(dp + at, p[i], pick);
                     at += (bit >> i) & 1u;
                 }
                 at0 += at;
@@ -956,9 +954,10 @@ template <int NS, int ND, int NV> struct KPassShape {
 
 // Key pass: one CTA per 128 keys of a head, over the queries from the keys' own tile on, 32 at a time.  A thread owns a
 // key; for a warp's 32 keys the bits of a query are one word, and the ranks of the keys it picked are consecutive, so
-// that what the query pass left is read in short contiguous pieces: p by two warpgroups, dS by two others, chunk by chunk
-// in turn.  Each writes its 32 columns as an A operand (a buffer of 48 columns of its own), and the tensor core adds
-// dv += P^T dO, dk += dS^T q.
+// that what the query pass left is read in short contiguous pieces, p and dS together.  Two warpgroups take half of a
+// chunk's queries each and write them as A operands (48 columns for p, 48 for dS), two others the next chunk's; the tensor
+// core adds dv += P^T dO, dk += dS^T q.  (p and dS apart, a warpgroup reading one of them for all 32 queries, and the flush
+// before the gather: 859 us at 32 x 8 x 1024 queries of 192 in fp32, where this takes 716.)
 constexpr int KEY_THREADS = 18 * 32;       // four producing warpgroups, TMA warp, MMA warp
 
 template <int NS, int ND, int NV>
@@ -986,7 +985,7 @@ attn_bwd_key_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
     if (tid == 0) {
         *abort_flag = 0;
         for (int i = 0; i < S::STAGES; ++i) { mbar_init(full0 + 8 * i, 1); mbar_init(empty0 + 8 * i, 1); }
-        for (int i = 0; i < 4; ++i) { mbar_init(ready0 + 8 * i, 4); mbar_init(free0 + 8 * i, 1); }
+        for (int i = 0; i < 4; ++i) { mbar_init(ready0 + 8 * i, 8); mbar_init(free0 + 8 * i, 1); }
         mbar_init(done, 1); mbar_init(taken, 16);
         for (int i = 0; i < 4; ++i) mbar_init(group0 + 8 * i, 4);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -1050,13 +1049,13 @@ attn_bwd_key_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
             if (alive && (i + 1 == n || (flush && (i + 1) % EVERY == 0))) commit_elected(done);
         }
     } else {
-        const int op = (warp >> 2) & 1, buf = warp >> 3, quarter = warp & 3, r = quarter * 32 + lane;
+        const int half = (warp >> 2) & 1, buf = warp >> 3, quarter = warp & 3, r = quarter * 32 + lane;
         const int s = k0 + r, b = bh / a.H;
         const uint32_t lanes = (uint32_t)(quarter * 32) << 16;
         const int word = (k0 >> 5) + quarter;
         const uint32_t* bits = a.picks.bits + ((int64_t)b * a.L) * a.words + word;
         const uint16_t* before = a.picks.before + ((int64_t)b * a.L) * a.words + word;
-        const float* src = (op ? a.ds : a.p) + (int64_t)bh * a.L * a.K;
+        const float2* src = a.pd + (int64_t)bh * a.L * a.K;
         const uint32_t below = (1u << lane) - 1u;
         bool alive = true;
         // this lane's query of the next chunk: its word for the warp's keys, and where that word's picks begin
@@ -1091,24 +1090,31 @@ attn_bwd_key_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
         uint32_t w_next, base_next;
         fetch(buf, w_next, base_next);
         for (int i = buf; i < n; i += 2) {
-            if (flush && i >= EVERY && i % EVERY == buf && !take()) { alive = false; break; }
             const uint32_t w = w_next, base = base_next;
             if (i + 2 < n) fetch(i + 2, w_next, base_next);
-            float v[32];
+            float vp[16], vd[16];
 #pragma unroll
-            for (int u = 0; u < 32; ++u) {
-                const uint32_t wu = __shfl_sync(0xffffffffu, w, u), at = __shfl_sync(0xffffffffu, base, u) + __popc(wu & below);
-                const float x = __ldg(src + min(at, (uint32_t)a.L * a.K - 1u));       // a lane that was not picked reads its neighbour's
-                v[u] = wu >> lane & 1u ? x : 0.0f;
+            for (int u = 0; u < 16; ++u) {
+                const uint32_t wu = __shfl_sync(0xffffffffu, w, half * 16 + u);
+                const uint32_t at = __shfl_sync(0xffffffffu, base, half * 16 + u) + __popc(wu & below);
+                const float2 x = __ldg(src + min(at, (uint32_t)a.L * a.K - 1u));      // a lane that was not picked reads its neighbour's
+                vp[u] = wu >> lane & 1u ? x.x : 0.0f;
+                vd[u] = wu >> lane & 1u ? x.y : 0.0f;
             }
-            if (!wait_warp(free0 + 8 * (op * 2 + buf), ((i >> 1) & 1) ^ 1, abort_flag, (10 << 8) | 4)) { alive = false; break; }
+            // (with this chunk's values already here, the flush costs the tensor core its own time only)
+            if (flush && i >= EVERY && i % EVERY == buf && !take()) { alive = false; break; }
+            if (!wait_warp(free0 + 8 * buf, ((i >> 1) & 1) ^ 1, abort_flag, (10 << 8) | 4)) { alive = false; break; }
+            if (!wait_warp(free0 + 8 * (2 + buf), ((i >> 1) & 1) ^ 1, abort_flag, (10 << 8) | 4)) { alive = false; break; }
             tc_fence_after();
-            const uint32_t at = t_a + lanes + (op * 2 + buf) * 48;
-            store_parts32(at, at + 32, v);
+            store_parts16(t_a + lanes + buf * 48, t_a + lanes + buf * 48 + 32, half, vp);
+            store_parts16(t_a + lanes + (2 + buf) * 48, t_a + lanes + (2 + buf) * 48 + 32, half, vd);
             st_wait();
             tc_fence_before();
             __syncwarp();
-            if (lane == 0) mbar_arrive(ready0 + 8 * (op * 2 + buf));
+            if (lane == 0) {
+                mbar_arrive(ready0 + 8 * buf);
+                mbar_arrive(ready0 + 8 * (2 + buf));
+            }
         }
         if (alive && flush) {
             take();
@@ -1146,7 +1152,7 @@ struct Plan {
     int64_t B, H, L, K, Dqk, Dv, BH, Lp;
     int dtype, ns, nd, dp, nv;             // parts; panels, padded width of q and k; 64-column panels of v
     bool direct;                           // bf16 rows TMA can read as they are: no copies
-    int64_t bits_off, rank_off, count_off, before_off, flag_off, q_off, k_off, v_off, g_off, delta_off, p_off, ds_off, grads_off, bytes;
+    int64_t bits_off, rank_off, count_off, before_off, flag_off, q_off, k_off, v_off, g_off, delta_off, pd_off, grads_off, bytes;
 };
 
 static Plan make_plan(int64_t B, int64_t H, int64_t L, int64_t K, int64_t Dqk, int64_t Dv, int dtype, bool backward) {
@@ -1165,8 +1171,7 @@ static Plan make_plan(int64_t B, int64_t H, int64_t L, int64_t K, int64_t Dqk, i
     p.before_off = take(B * L * p.Lp / 32 * 2);
     if (backward) {
         p.delta_off = take(p.BH * L * 4);
-        p.p_off = take(p.BH * L * K * 4);
-        p.ds_off = take(p.BH * L * K * 4);
+        p.pd_off = take(p.BH * L * K * 8);
         if (!p.direct) p.g_off = take(p.ns * p.BH * L * p.nv * 64 * 2);
         // fp32 gradients for the fallback, where the caller's are not
         if (dtype != CINN_F32) p.grads_off = take(p.BH * L * (2 * Dqk + Dv) * 4);
@@ -1200,7 +1205,7 @@ static bool dense_pays(const Plan& p, bool backward) {
         cycles = tiles * p.nv * (parts ? 8800.0 + 48.0 * p.dp : 7500.0 + 8.0 * p.dp) + q_tiles * p.nv * (6000.0 + 100.0 * p.K);
         gather_us = 8.0 + gathered / (wide ? 9.5e6 : 5.3e6);
     } else {
-        cycles = tiles * (parts ? 24000.0 + 190.0 * widths : 14000.0 + 66.0 * widths) + q_tiles * 20000.0;
+        cycles = tiles * (parts ? 27000.0 + 130.0 * widths : 12000.0 + 55.0 * widths) + q_tiles * 20000.0;
         gather_us = 30.0 + gathered / (wide ? 3.7e6 : 2.0e6);
     }
     return (picks + split + (backward ? 20.0 : 0.0) + cycles / (148.0 * 1900.0)) < 0.9 * gather_us;
@@ -1383,7 +1388,7 @@ int backward(const void* d_out, const float* out, const float* lse, const void* 
     }
     BwdArgs a{};
     a.picks = picks_of(p, ws);
-    a.lse = lse; a.delta = delta; a.p = reinterpret_cast<float*>(ws + p.p_off); a.ds = reinterpret_cast<float*>(ws + p.ds_off);
+    a.lse = lse; a.delta = delta; a.pd = reinterpret_cast<float2*>(ws + p.pd_off);
     a.dq = dq; a.dk = dk; a.dv = dv; a.flag = reinterpret_cast<int*>(ws + p.flag_off);
     a.H = (int)H; a.L = (int)L; a.words = (int)(p.Lp / 32); a.K = (int)K; a.Dqk = (int)Dqk; a.Dv = (int)Dv; a.BH = (int)p.BH;
     a.n_tiles = (int)(p.Lp / T); a.group = head_group(p); a.tag = dtype; a.scale = scale;

@@ -95,11 +95,6 @@ __device__ __forceinline__ void tma_add_3d(const CUtensorMap* map, uint32_t src,
     asm volatile("cp.reduce.async.bulk.tensor.3d.global.shared::cta.add.bulk_group [%0, {%2, %3, %4}], [%1];"
                  ::"l"(map), "r"(src), "r"(x), "r"(y), "r"(z) : "memory");
 }
-// *(smem float at addr) = x if take is not zero, as a predicated instruction
-__device__ __forceinline__ void store_shared_if(uint32_t addr, float x, uint32_t take) {
-    asm volatile("{\n\t.reg .pred t;\n\tsetp.ne.u32 t, %2, 0;\n\t@t st.shared.f32 [%0], %1;\n\t}" ::"r"(addr), "f"(x), "r"(take) : "memory");
-}
-
 // two fp32 values as three packed bf16 pairs whose sum they are
 __device__ __forceinline__ void split2(float a, float b, uint32_t& hi, uint32_t& mid, uint32_t& lo) {
     auto pack = [](float x, float y) {
@@ -129,6 +124,18 @@ __device__ __forceinline__ void store_if(float* p, float x, uint32_t take) {
         ::"l"(p), "f"(x), "r"(take) : "memory");
 }
 
+// *p = (x, y) if take is not zero, as one predicated instruction
+__device__ __forceinline__ void store2_if(float2* p, float x, float y, uint32_t take) {
+    asm volatile(
+        "{\n\t.reg .pred t;\n\t"
+        "setp.ne.u32 t, %3, 0;\n\t"
+        "@t st.global.v2.f32 [%0], {%1, %2};\n\t}"
+        ::"l"(p), "f"(x), "f"(y), "r"(take) : "memory");
+}
+__device__ __forceinline__ void st8(uint32_t taddr, const uint32_t (&r)[8]) {
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%8], {%0, %1, %2, %3, %4, %5, %6, %7};"
+                 ::"r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(taddr) : "memory");
+}
 // Writes 32 consecutive reduction positions (keys or queries) of this lane's row as an A operand in tensor memory: the
 // leading parts in 16 columns at `lead`, the second and third in 32 columns at `rest`.
 __device__ __forceinline__ void store_parts32(uint32_t rest, uint32_t lead, const float (&v)[32]) {
@@ -150,6 +157,16 @@ __device__ __forceinline__ void mma_panels(uint32_t d, uint64_t a, uint64_t b, u
     mma_ss(d, a, b, idesc, fresh ? 0u : 1u);
 #pragma unroll
     for (int s = 1; s < 4; ++s) mma_ss(d, a + s * K_STEP, b + s * K_STEP, idesc, 1u);
+}
+
+// the same for one half (0 or 1) of the 32 positions
+__device__ __forceinline__ void store_parts16(uint32_t rest, uint32_t lead, int half, const float (&v)[16]) {
+    uint32_t hi[8], mid[8], lo[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) split2(v[2 * i], v[2 * i + 1], hi[i], mid[i], lo[i]);
+    st8(lead + half * 8, hi);
+    st8(rest + half * 8, mid);
+    st8(rest + 16 + half * 8, lo);
 }
 
 // D (+)= part X of a tensor-memory operand of 16 STEPS positions (store_parts32) times an MN-major panel
