@@ -30,6 +30,7 @@ constexpr int STAGES = 4;             // even: each of the two MMA issuers then 
                                       // sees every phase of their barriers (a parity wait cannot skip a phase)
 constexpr int C_SLOT_BYTES = BM * 128;   // one TMA-store box: 128 rows x 64 columns of a 2-byte type
 constexpr int C_STAGE_BYTES = 2 * C_SLOT_BYTES;   // one slot per column group of promotion warps
+constexpr int STORE_ROWS = 32;           // rows of the FP8 kernels' TMA-store boxes: those of one promotion warp
 constexpr int A_BYTES = BM * BK;   // 16 KiB
 constexpr int B_BYTES = BN * BK;   // 32 KiB
 constexpr int EPI_WARPS = 8;                    // four TMEM lane quarters x two column groups
@@ -73,12 +74,13 @@ __device__ __forceinline__ float ld_scale(const float* p) {
     return v;
 }
 
-// D[tmem] (+)= A[smem desc] * B[smem desc], e4m3 x e4m3 -> fp32
+// D[tmem] (+)= A[smem desc] * B[smem desc], e4m3 x e4m3 -> fp32.  Called by a whole warp, issued by one elected lane.
 __device__ __forceinline__ void tc_mma_f8(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
     asm volatile(
-        "{\n\t.reg .pred p;\n\t"
+        "{\n\t.reg .pred p, e;\n\t"
+        "elect.sync _|e, 0xffffffff;\n\t"
         "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f8f6f4 [%0], %1, %2, %3, p;\n\t}"
+        "@e tcgen05.mma.cta_group::1.kind::f8f6f4 [%0], %1, %2, %3, p;\n\t}"
         ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate) : "memory");
 }
 
@@ -281,7 +283,7 @@ fp8_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
     uint8_t* smem_b = smem + STAGES * A_BYTES;
     uint8_t* c_stage = smem + STAGES * (A_BYTES + B_BYTES);
     uint64_t* bars = reinterpret_cast<uint64_t*>(c_stage + C_STAGE_BYTES);
-    // bars[0..S) full, [S..2S) empty, [2S..2S+2) tmem full, [2S+2..2S+4) tmem empty, then slot free / slot full x 2
+    // bars[0..S) full, [S..2S) empty, [2S..2S+2) tmem full, [2S+2..2S+4) tmem empty
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * STAGES + 8);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
     uint8_t* store_stage = c_stage;                                        // 2 KiB per promotion warp (non-TMA path)
@@ -290,13 +292,11 @@ fp8_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t full0 = smem_u32(bars), empty0 = smem_u32(bars + STAGES);
     const uint32_t tfull0 = smem_u32(bars + 2 * STAGES), tempty0 = smem_u32(bars + 2 * STAGES + 2);
-    const uint32_t gfree0 = smem_u32(bars + 2 * STAGES + 4), gfull0 = smem_u32(bars + 2 * STAGES + 6);
 
     if (threadIdx.x == 0) *abort_flag = 0;
     if (warp == EPI_WARPS && lane == 0) {
         for (int s = 0; s < STAGES; ++s) { mbar_init(full0 + 8 * s, 1); mbar_init(empty0 + 8 * s, 1); }
         for (int b = 0; b < 2; ++b) { mbar_init(tfull0 + 8 * b, 1); mbar_init(tempty0 + 8 * b, EPI_WARPS); }
-        for (int g = 0; g < 2; ++g) { mbar_init(gfree0 + 8 * g, 4); mbar_init(gfull0 + 8 * g, 4); }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == EPI_WARPS + 1) {
@@ -368,10 +368,11 @@ fp8_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
         }
     } else {
         // ------------------------------ MMA issuers ------------------------------
-        // Two warps take alternate K blocks (one TMEM buffer each).  Issuing a block's MMAs blocks the
-        // issuing thread for about as long as they execute, and every barrier probe costs a few
-        // hundred cycles next to a busy tensor pipe; with two issuers one probes while the other feeds.
-        if (lane == 0) {
+        // Two warps take alternate K blocks (one TMEM buffer each), each as a whole with one elected lane issuing: with
+        // warp-uniform control flow the descriptors live in uniform registers.  Issued from a branch of one lane, a K block's
+        // four MMAs and its commits took their issuer 600 cycles, more than the 512 of the arithmetic, and with the probes
+        // around them that (and not the promotion) set the pace.
+        {
             constexpr uint32_t idesc = make_idesc(B_MN);
             const uint32_t mine = (uint32_t)(warp - (EPI_WARPS + 1));
             uint32_t it = 0, last = 0xffffffffu;
@@ -387,8 +388,8 @@ fp8_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
                     const uint32_t b = it & 1, bph = (it >> 1) & 1;
                     // operands first (they landed long ago: this costs one barrier probe, taken while
                     // the epilogue still works on the buffer), then the TMEM buffer
-                    if (!mbar_wait(full0 + 8 * s, ph, abort_flag, (2 << 8) | 1)) { alive = false; break; }
-                    if (!mbar_wait(tempty0 + 8 * b, bph ^ 1, abort_flag, (2 << 8) | 2)) { alive = false; break; }
+                    if (!mbar_wait_warp(full0 + 8 * s, ph, abort_flag, (2 << 8) | 1)) { alive = false; break; }
+                    if (!mbar_wait_warp(tempty0 + 8 * b, bph ^ 1, abort_flag, (2 << 8) | 2)) { alive = false; break; }
                     tc_fence_after();
                     const uint32_t a_addr = smem_u32(smem_a + s * A_BYTES);
                     const uint32_t b_addr = smem_u32(smem_b + s * B_BYTES);
@@ -400,8 +401,8 @@ fp8_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
                                                  : make_smem_desc(b_addr + k * 32, 16, 1024);
                         tc_mma_f8(d, ad, bd, idesc, k > 0 ? 1u : 0u);
                     }
-                    tc_commit(empty0 + 8 * s);      // the stage may be refilled once these MMAs retire
-                    tc_commit(tfull0 + 8 * b);      // and the partial tile is ready for promotion
+                    tc_commit_elected(tfull0 + 8 * b);      // the partial tile is ready for promotion once these MMAs retire
+                    tc_commit_elected(empty0 + 8 * s);      // and the stage may be refilled
                 }
             }
             // every MMA issued above must have retired before tensor memory is freed
@@ -416,7 +417,6 @@ fp8_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
         const bool vec_ok = (OUT == CINN_F32 || OUT == CINN_F32_BF16) ? (p.ldc % 4 == 0) : (p.ldc % 8 == 0);
         // The first three scale pairs of a tile are fetched while the previous tile is being stored, so that
         // a tile does not start with an exposed round trip to L2 (it matters when K is only a few blocks).
-        uint32_t n_rounds = 0;                   // staging rounds of this column group so far (two per TMA tile)
         float sa0 = 0.f, sb0 = 0.f, sa1 = 0.f, sb1 = 0.f, sa2 = 0.f, sb2 = 0.f;
         auto scale_ptrs = [&](const TileInfo& ti, int kb0, const float*& sa_ptr, const float*& sb_ptr) {
             const int row = ti.m0 + q * 32 + lane;
@@ -490,44 +490,33 @@ fp8_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
             }
             if (alive && t + (int)gridDim.x < n_total) prefetch_scales(t + gridDim.x);
             constexpr bool TMA_OUT = (OUT == CINN_BF16 || OUT == CINN_F16);
-            // A tile whose 128 rows all belong to it leaves through TMA stores.  Each column group of four
-            // promotion warps owns one 16 KiB slot: its threads drop 64 columns of their rows into it (16-byte
-            // chunks, 128-byte swizzle), one thread hands the box to the TMA unit, and the group repeats for its
-            // other 64 columns once the unit has read the slot.  Storing one row per thread straight from
-            // registers costs thousands of cycles per tile, and so do shared-memory round trips next to a busy
-            // tensor pipe.
-            const bool whole = !GROUPED || ti.m0 + BM <= ti.m_end;
+            // Rows that all belong to the tile leave through TMA stores.  Every promotion warp owns a 4 KiB box: its lanes
+            // drop 64 columns of their rows into it (16-byte chunks, 128-byte swizzle), one lane hands the box to the TMA
+            // unit, and the warp repeats for its other 64 columns once the unit has read the box.  (No warp waits for
+            // another: see the two-SM kernel.)  Storing one row per thread straight from registers costs thousands of
+            // cycles per tile, and so do shared-memory round trips next to a busy tensor pipe.
+            const bool whole = !GROUPED || row - lane + STORE_ROWS <= ti.m_end;
             if (TMA_OUT && alive && p.tma_out && whole) {
-                const bool elected = (warp == h * 4) && lane == 0;
-                const uint32_t slot = smem_u32(c_stage) + h * C_SLOT_BYTES;
-                const int rl = q * 32 + lane;
+                const uint32_t slot = smem_u32(c_stage) + warp * STORE_ROWS * 128;
 #pragma unroll
                 for (int r = 0; r < 2; ++r) {
-                    const uint32_t par = n_rounds & 1u;
-                    if (elected) tma_store_wait_read();               // the unit has finished reading this slot
+                    if (lane == 0) tma_store_wait_read();             // the unit has finished reading this box
                     __syncwarp();
-                    if (lane == 0) mbar_arrive(gfree0 + 8 * h);
-                    if (!mbar_wait_warp(gfree0 + 8 * h, par, abort_flag, (3 << 8) | 2)) { alive = false; break; }
 #pragma unroll
                     for (int j = 0; j < 8; ++j) {
                         const uint4 v = pack16<OUT>(&acc[r * 64 + j * 8]);
-                        asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(slot + rl * 128 + ((j ^ (rl & 7)) << 4)),
+                        asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(slot + lane * 128 + ((j ^ (lane & 7)) << 4)),
                                      "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
                     }
                     fence_async_smem();
                     __syncwarp();
-                    if (lane == 0) mbar_arrive(gfull0 + 8 * h);
-                    if (elected) {
+                    if (lane == 0) {
                         const int col = col0 + r * 64;
-                        if (mbar_wait(gfull0 + 8 * h, par, abort_flag, (3 << 8) | 3)) {
-                            if (col < p.N) tma_store_2d(&tmC, slot, col, ti.m0);
-                            tma_store_commit();
-                        }
+                        if (col < p.N) tma_store_2d(&tmC, slot, col, row);
+                        tma_store_commit();
                     }
-                    __syncwarp();   // the elected lane rejoins its warp before the next warp-collective instruction
-                    ++n_rounds;
+                    __syncwarp();   // the lane rejoins its warp before the next warp-collective instruction
                 }
-                if (!alive) break;
             } else if (alive && vec_ok && !(TMA_OUT && p.tma_out)) {
                 // warp-uniform: every lane takes part in the staging even if its own row is past the end
                 if (cvalid) store_rows_staged<OUT, WCOLS, SCATTER>(acc, store_stage + warp * 2048, C, p.ldc, ti.m0 + q * 32, ti.m_end, col0, p.N, lane);
@@ -540,7 +529,7 @@ fp8_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
                 }
             }
         }
-        if (lane == 0 && (warp & 3) == 0) tma_store_wait_all();      // this group's boxes have reached global memory
+        if (lane == 0) tma_store_wait_all();                // this warp's boxes have reached global memory
     }
 
     tc_fence_before();
@@ -650,19 +639,19 @@ static int allow_smem_once(size_t bytes) {
 // Output map for the TMA-store epilogue: (rows, N) of a 2-byte type, boxes of 64 columns x 128 rows, 128-byte swizzle.
 // Sets p.tma_out; when the output cannot go through TMA the (unused) operand map is passed in its place.
 static int make_out_map(CUtensorMap* tc, const CUtensorMap& fallback, GemmParams& p, int out_dtype, int64_t rows,
-                        bool fp32_boxes = false) {
+                        int box_rows, bool fp32_boxes = false) {
     p.tma_out = 0;
     *tc = fallback;
     if (((uintptr_t)p.C & 15) != 0) return CINN_OK;               // TMA wants a 16-byte aligned base; plain stores otherwise
     if (fp32_boxes && (out_dtype == CINN_F32 || out_dtype == CINN_F32_BF16) && p.N % 4 == 0) {
-        // the two-SM kernel also sends 4-byte outputs through TMA: boxes of 32 columns x 128 rows
-        int rc = make_map(tc, p.C, (uint64_t)p.N, (uint64_t)rows, (uint64_t)p.ldc * 4, 32, BM, CU_TENSOR_MAP_DATA_TYPE_FLOAT32);
+        // the two-SM kernel also sends 4-byte outputs through TMA: boxes of 32 columns
+        int rc = make_map(tc, p.C, (uint64_t)p.N, (uint64_t)rows, (uint64_t)p.ldc * 4, 32, box_rows, CU_TENSOR_MAP_DATA_TYPE_FLOAT32);
         if (rc) return rc;
         p.tma_out = 1;
         return CINN_OK;
     }
     if ((out_dtype == CINN_BF16 || out_dtype == CINN_F16) && p.N % 8 == 0) {
-        int rc = make_map(tc, p.C, (uint64_t)p.N, (uint64_t)rows, (uint64_t)p.ldc * 2, 64, BM,
+        int rc = make_map(tc, p.C, (uint64_t)p.N, (uint64_t)rows, (uint64_t)p.ldc * 2, 64, box_rows,
                           out_dtype == CINN_BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16);
         if (rc) return rc;
         p.tma_out = 1;
@@ -685,7 +674,7 @@ template <bool B_MN, bool GROUPED>
 static int launch_out(const CUtensorMap& ta, const CUtensorMap& tb, GemmParams& p, int out_dtype, int grid,
                       cudaStream_t st) {
     CUtensorMap tc;
-    int rc = make_out_map(&tc, ta, p, out_dtype, p.M);
+    int rc = make_out_map(&tc, ta, p, out_dtype, p.M, STORE_ROWS);
     if (rc) return rc;
     switch (out_dtype) {
         case CINN_BF16: return launch<B_MN, GROUPED, CINN_BF16>(ta, tb, tc, p, grid, st);
@@ -725,7 +714,7 @@ template <bool B_MN>
 static int launch_pair_out(const CUtensorMap& ta, const CUtensorMap& tb, GemmParams& p, int out_dtype, int clusters,
                            cudaStream_t st) {
     CUtensorMap tc;
-    int rc = make_out_map(&tc, ta, p, out_dtype, p.M, true);
+    int rc = make_out_map(&tc, ta, p, out_dtype, p.M, STORE_ROWS, true);
     if (rc) return rc;
     switch (out_dtype) {
         case CINN_BF16: return launch_pair<B_MN, CINN_BF16>(ta, tb, tc, p, clusters, st);
@@ -930,7 +919,7 @@ int fp8_grouped_gemm(const void* A, const float* sA, const void* W, const float*
     }
     if (use_pair) {
         CUtensorMap tc;
-        rc = make_out_map(&tc, ta, p, out_dtype, T, true);
+        rc = make_out_map(&tc, ta, p, out_dtype, T, STORE_ROWS, true);
         if (rc) return rc;
         const int clusters = gemm_sms() / 2;
         switch (out_dtype) {
@@ -998,7 +987,7 @@ int fp8_gemm_grouped_k(const void* A, const float* sA, const void* B, const floa
     p.C = C; p.ldc = N; p.M = (int)M; p.N = (int)N; p.K = 0;
     p.starts = reinterpret_cast<const int64_t*>(kb_start); p.ends = nullptr; p.E = (int)E; p.b_rows_per_expert = 0;
     CUtensorMap tc;
-    rc = make_out_map(&tc, ta, p, out_dtype, E * M, true);
+    rc = make_out_map(&tc, ta, p, out_dtype, E * M, STORE_ROWS, true);
     if (rc) return rc;
     const int64_t tiles = E * (M / pair::PM) * (N / pair::PN);
     const int clusters = (int)(tiles < gemm_sms() / 2 ? tiles : gemm_sms() / 2);
@@ -1046,7 +1035,7 @@ int grouped_gemm_16bit(const void* A, const void* W, int in_dtype, const int64_t
     p.C = C; p.ldc = d_out; p.M = (int)T; p.N = (int)d_out; p.K = (int)d_in;
     p.starts = starts; p.ends = ends; p.E = (int)E; p.b_rows_per_expert = (int)d_out;
     CUtensorMap tc;
-    rc = make_out_map(&tc, ta, p, out_dtype, p.M);
+    rc = make_out_map(&tc, ta, p, out_dtype, p.M, BM);
     if (rc) return rc;
     const int grid = gemm_sms();
 #define CINN_G16(BF, O) return launch16<BF, O>(ta, tb, tc, p, grid, st)

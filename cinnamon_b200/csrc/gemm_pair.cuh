@@ -21,11 +21,12 @@ constexpr int PSTAGES = 4;               // even (see the one-SM kernel); leaves
 constexpr int PA_BYTES = 128 * BK;      // A rows of this CTA: 16 KiB
 constexpr int PB_BYTES = 128 * BK;      // B columns of this CTA: 16 KiB
 constexpr int PTHREADS = 11 * 32;
-// dynamic shared memory: operand stages | four 16 KiB output slots = the CTA's whole 128 x 256 tile of a 2-byte type
-// (TMA-store boxes; also the 2 KiB-per-warp staging of the non-TMA path) | 256 B of barriers and flags, plus 1 KiB of
+// dynamic shared memory: operand stages | two 4 KiB output boxes per promotion warp = the CTA's whole 128 x 256 tile of a
+// 2-byte type (TMA-store boxes; also the 2 KiB-per-warp staging of the non-TMA path) | 256 B of barriers and flags, plus 1 KiB of
 // slack to align the stages to 1024 bytes
 constexpr int PSTAGE_OFF = PSTAGES * (PA_BYTES + PB_BYTES);
-constexpr int PC_BYTES = 4 * C_SLOT_BYTES;
+constexpr int PBOX_BYTES = STORE_ROWS * 128;  // one TMA-store box
+constexpr int PC_BYTES = 8 * 2 * PBOX_BYTES;
 constexpr size_t PSMEM_BYTES = (size_t)PSTAGE_OFF + PC_BYTES + 256 + 1024;
 
 __device__ __forceinline__ uint32_t cluster_ctarank() {
@@ -56,18 +57,23 @@ __device__ __forceinline__ void tma_load_2d_pair(const CUtensorMap* map, uint32_
         "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
         ::"r"(dst), "l"(map), "r"(bar_cluster), "r"(x), "r"(y) : "memory");
 }
+// Both are called by a whole warp and issued by the lane that elect.sync chooses.
 // Completion of the pair's MMAs issued so far is reported to the barrier at the same offset in BOTH CTAs:
 // one commit per CTA, each naming that CTA's barrier by its cluster address.
-__device__ __forceinline__ void tc_commit_pair(uint32_t bar) {
-    const uint32_t own = mapa(bar, 0), peer = mapa(bar, 1);
-    asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(own) : "memory");
-    asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(peer) : "memory");
+__device__ __forceinline__ void tc_commit_pair(uint32_t own, uint32_t peer) {
+    asm volatile(
+        "{\n\t.reg .pred e;\n\t"
+        "elect.sync _|e, 0xffffffff;\n\t"
+        "@e tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t"
+        "@e tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64 [%1];\n\t}"
+        ::"r"(own), "r"(peer) : "memory");
 }
 __device__ __forceinline__ void tc_mma_f8_pair(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
     asm volatile(
-        "{\n\t.reg .pred p;\n\t"
+        "{\n\t.reg .pred p, e;\n\t"
+        "elect.sync _|e, 0xffffffff;\n\t"
         "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::2.kind::f8f6f4 [%0], %1, %2, %3, p;\n\t}"
+        "@e tcgen05.mma.cta_group::2.kind::f8f6f4 [%0], %1, %2, %3, p;\n\t}"
         ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate) : "memory");
 }
 __host__ __device__ constexpr uint32_t make_idesc_pair(bool b_mn_major) {
@@ -116,20 +122,17 @@ fp8_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
     // [0, S) full (used in the leader), [S, 2S) empty, [2S, 2S+2) tmem full, [2S+2, 2S+4) tmem empty (leader)
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * PSTAGES + 8);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
-    uint8_t* store_stage = c_stage;                                             // 2 KiB per promotion warp (non-TMA path)
     int* cum = reinterpret_cast<int*>(reinterpret_cast<uint8_t*>(bars) + 256);  // GR: E + 1 prefix counts of row tiles
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t rank = cluster_ctarank();           // 0 = leader
     const uint32_t full0 = smem_u32(bars), empty0 = smem_u32(bars + PSTAGES);
     const uint32_t tfull0 = smem_u32(bars + 2 * PSTAGES), tempty0 = smem_u32(bars + 2 * PSTAGES + 2);
-    const uint32_t gfree0 = smem_u32(bars + 2 * PSTAGES + 4), gfull0 = smem_u32(bars + 2 * PSTAGES + 6);
 
     if (threadIdx.x == 0) *abort_flag = 0;
     if (warp == 8 && lane == 0) {
         for (int s = 0; s < PSTAGES; ++s) { mbar_init(full0 + 8 * s, 1); mbar_init(empty0 + 8 * s, 1); }
         for (int b = 0; b < 2; ++b) { mbar_init(tfull0 + 8 * b, 1); mbar_init(tempty0 + 8 * b, 16); }
-        for (int g = 0; g < 2; ++g) { mbar_init(gfree0 + 8 * g, 4); mbar_init(gfull0 + 8 * g, 4); }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 9) {
@@ -209,9 +212,11 @@ fp8_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
             }
         }
     } else if (warp >= 9) {
-        // ------------------------------ MMA issuers (leader only) ------------------------------
-        if (lane == 0 && rank == 0) {
+        // ------------------ MMA issuers (leader only; whole warps, as in the one-SM kernel) ------------------
+        if (rank == 0) {
             constexpr uint32_t idesc = make_idesc_pair(B_MN);
+            const uint32_t tfull_own = mapa(tfull0, 0), tfull_peer = mapa(tfull0, 1);
+            const uint32_t empty_own = mapa(empty0, 0), empty_peer = mapa(empty0, 1);
             const uint32_t mine = (uint32_t)(warp - 9);
             uint32_t it = 0, last = 0xffffffffu;
             bool alive = true;
@@ -227,8 +232,8 @@ fp8_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
                     const int s = it % PSTAGES;
                     const uint32_t ph = (it / PSTAGES) & 1;
                     const uint32_t b = it & 1, bph = (it >> 1) & 1;
-                    if (!mbar_wait(full0 + 8 * s, ph, abort_flag, (2 << 8) | 1)) { alive = false; break; }
-                    if (!mbar_wait(tempty0 + 8 * b, bph ^ 1, abort_flag, (2 << 8) | 2)) { alive = false; break; }
+                    if (!mbar_wait_warp(full0 + 8 * s, ph, abort_flag, (2 << 8) | 1)) { alive = false; break; }
+                    if (!mbar_wait_warp(tempty0 + 8 * b, bph ^ 1, abort_flag, (2 << 8) | 2)) { alive = false; break; }
                     tc_fence_after();
                     const uint32_t a_addr = smem_u32(smem_a + s * PA_BYTES);
                     const uint32_t b_addr = smem_u32(smem_b + s * PB_BYTES);
@@ -240,8 +245,8 @@ fp8_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
                                                  : make_smem_desc(b_addr + k * 32, 16, 1024);
                         tc_mma_f8_pair(d, ad, bd, idesc, k > 0 ? 1u : 0u);
                     }
-                    tc_commit_pair(empty0 + 8 * s);
-                    tc_commit_pair(tfull0 + 8 * b);
+                    tc_commit_pair(tfull_own + 8 * b, tfull_peer + 8 * b);
+                    tc_commit_pair(empty_own + 8 * s, empty_peer + 8 * s);
                 }
             }
             if (alive && last != 0xffffffffu) mbar_wait(tfull0 + 8 * (last & 1), (last >> 1) & 1, abort_flag, (2 << 8) | 3);
@@ -250,7 +255,7 @@ fp8_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
         // ------------------------------ promotion / epilogue (both CTAs) ------------------------------
         const int q = warp & 3, h = warp >> 2;
         const uint32_t tempty_leader = mapa(tempty0, 0);
-        uint32_t it = 0, n_rounds = 0;
+        uint32_t it = 0;
         bool alive = true;
         const bool vec_ok = (OUT == CINN_F32 || OUT == CINN_F32_BF16) ? (p.ldc % 4 == 0) : (p.ldc % 8 == 0);
         for (int t = cluster_id; t < n_total && alive; t += n_clusters) {
@@ -302,68 +307,48 @@ fp8_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
                 __syncwarp();
                 if (lane == 0) mbar_arrive_remote(tempty_leader + 8 * b);
             }
-            const bool whole = !GR || ti.m0 + 128 * (int)rank + 128 <= m_end;
-            if (alive && p.tma_out && !whole) {
-                // ragged tail: staged 16-byte stores through the group's slots, once the TMA unit has read them
-                const uint32_t par = n_rounds & 1u;
-                const bool elected = (warp == h * 4) && lane == 0;
-                if (elected) tma_store_wait_read();
-                __syncwarp();
-                if (lane == 0) mbar_arrive(gfree0 + 8 * h);
-                if (!mbar_wait_warp(gfree0 + 8 * h, par, abort_flag, (3 << 8) | 2)) { alive = false; break; }
-                if (cvalid && vec_ok)
-                    store_rows_staged<OUT, 128>(acc, c_stage + h * 2 * C_SLOT_BYTES + q * 2048, p.C, p.ldc,
-                                                ti.m0 + 128 * (int)rank + q * 32, m_end, col0, p.N, lane);
-                if (lane == 0) mbar_arrive(gfull0 + 8 * h);
-                if (elected) mbar_wait(gfull0 + 8 * h, par, abort_flag, (3 << 8) | 3);
-                __syncwarp();
-                ++n_rounds;
-            } else if (alive && p.tma_out) {
-                // The tile leaves through TMA stores.  Each column group of four promotion warps owns two 16 KiB slots
-                // (boxes of 128 rows x 128 bytes, 128-byte swizzle): its threads drop their rows into them in 16-byte
-                // chunks and one thread hands the boxes to the TMA unit.  A 2-byte output fits the group's 128 columns
-                // in one round; a 4-byte output takes two rounds of 64 columns.  Nobody waits for the unit until the
-                // slots are needed again.
+            if (alive && p.tma_out && (!GR || row - lane + 32 <= m_end)) {
+                // The tile leaves through TMA stores.  Every promotion warp owns 8 KiB of the staging area, two boxes of 32 rows
+                // x 128 bytes (128-byte swizzle): its lanes drop their rows in 16-byte chunks and one lane hands the boxes to
+                // the TMA unit.  A 2-byte output fits the warp's 128 columns in one round; a 4-byte output takes two rounds of
+                // 64 columns.  Nobody waits for the unit until the boxes are needed again, and no warp for another: with boxes
+                // of 128 rows, four warps met at two barriers for each (16384 x 7168 -> 2048: 211 us, where this takes 195;
+                // 32768 x 512 -> 1024: 29.8 and 27.4).
                 using T = typename OutT<OUT>::type;
                 constexpr int EPR = 128 / (int)sizeof(T);          // elements per 128-byte box row
                 constexpr int PER16 = 16 / (int)sizeof(T);
                 constexpr int ROUNDS = 128 / (2 * EPR);
-                const bool elected = (warp == h * 4) && lane == 0;
-                const uint32_t slot = smem_u32(c_stage) + h * 2 * C_SLOT_BYTES;
-                const int rl = q * 32 + lane;
+                const uint32_t slot = smem_u32(c_stage) + warp * 2 * PBOX_BYTES;
 #pragma unroll
                 for (int r = 0; r < ROUNDS; ++r) {
-                    const uint32_t par = n_rounds & 1u;
-                    if (elected) tma_store_wait_read();               // the previous boxes have left the slots
+                    if (lane == 0) tma_store_wait_read();             // the previous boxes have left the slots
                     __syncwarp();
-                    if (lane == 0) mbar_arrive(gfree0 + 8 * h);
-                    if (!mbar_wait_warp(gfree0 + 8 * h, par, abort_flag, (3 << 8) | 2)) { alive = false; break; }
 #pragma unroll
                     for (int j = 0; j < 16; ++j) {
                         const uint4 v = pack16<OUT>(&acc[r * 2 * EPR + (j >> 3) * EPR + (j & 7) * PER16]);
                         asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};"
-                                     ::"r"(slot + (j >> 3) * C_SLOT_BYTES + rl * 128 + (((j & 7) ^ (rl & 7)) << 4)),
+                                     ::"r"(slot + (j >> 3) * PBOX_BYTES + lane * 128 + (((j & 7) ^ (lane & 7)) << 4)),
                                        "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
                     }
                     fence_async_smem();
                     __syncwarp();
-                    if (lane == 0) mbar_arrive(gfull0 + 8 * h);
-                    if (elected) {
-                        if (mbar_wait(gfull0 + 8 * h, par, abort_flag, (3 << 8) | 3)) {
+                    if (lane == 0) {
 #pragma unroll
-                            for (int sl = 0; sl < 2; ++sl) {
-                                const int col = col0 + r * 2 * EPR + sl * EPR;
-                                if (col < p.N) tma_store_2d(&tmC, slot + sl * C_SLOT_BYTES, col, out_row0 + ti.m0 + 128 * (int)rank);
-                            }
-                            tma_store_commit();
+                        for (int sl = 0; sl < 2; ++sl) {
+                            const int col = col0 + r * 2 * EPR + sl * EPR;
+                            if (col < p.N) tma_store_2d(&tmC, slot + sl * PBOX_BYTES, col, out_row0 + row);
                         }
+                        tma_store_commit();
                     }
-                    __syncwarp();       // the elected lane rejoins its warp before the next warp-collective instruction
-                    ++n_rounds;
+                    __syncwarp();       // the lane rejoins its warp before the next warp-collective instruction
                 }
-                if (!alive) break;
             } else if (alive && vec_ok) {
-                if (cvalid) store_rows_staged<OUT, 128>(acc, store_stage + warp * 2048, p.C, p.ldc,
+                // rows of two owners, or an output that TMA cannot write: staged 16-byte stores
+                if (p.tma_out) {
+                    if (lane == 0) tma_store_wait_read();
+                    __syncwarp();
+                }
+                if (cvalid) store_rows_staged<OUT, 128>(acc, c_stage + warp * 2 * PBOX_BYTES, p.C, p.ldc,
                                                         out_row0 + ti.m0 + 128 * (int)rank + q * 32, out_row0 + m_end, col0, p.N, lane);
             } else if (alive && rvalid && cvalid) {
                 const int64_t base = (int64_t)(out_row0 + row) * p.ldc + col0;
@@ -374,7 +359,7 @@ fp8_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
                 }
             }
         }
-        if (lane == 0 && (warp & 3) == 0) tma_store_wait_all();      // this group's boxes have reached global memory
+        if (lane == 0) tma_store_wait_all();                // this warp's boxes have reached global memory
     }
 
     // nobody leaves while the other CTA may still read this CTA's shared memory or signal its barriers
