@@ -278,7 +278,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
                             first = false;
                             qd -= ND * (PANEL >> 4);
                         }
-                        tc_commit_elected(empty0 + 8 * (it % S::RING));
+                        tc_commit(empty0 + 8 * (it % S::RING));
                         ++it;
                     };
                     // The tensor core truncates the running sum at every step, so the small products go first and the
@@ -288,7 +288,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
                         for (int c = 0; c < ND && alive; ++c)
                             for (int p = NS - 1; p >= 0 && alive; --p) product(c, NS - 1 - p, p == 0 ? 1 : 0);
                     for (int c = 0; c < ND && alive; ++c) product(c, 0, 0);
-                    tc_commit_elected(sfull0 + 8 * (j & 1));
+                    tc_commit(sfull0 + 8 * (j & 1));
                 }
                 if (j > 0 && alive) {                     // output of key tile j - 1
                     const int i = j - 1, w = i & 1;
@@ -305,10 +305,10 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
                         if (p <= 1) { mma_part_at<1>(base + 192, base, base + 128, vd, id_o, first); first = false; }
                         mma_part_at<0>(base + 192, base, base + 128, vd, id_o, first);
                         first = false;
-                        tc_commit_elected(empty0 + 8 * (it % S::RING));
+                        tc_commit(empty0 + 8 * (it % S::RING));
                         ++it;
                     }
-                    if (i + 2 >= n) tc_commit_elected(odone0 + 8 * w);
+                    if (i + 2 >= n) tc_commit(odone0 + 8 * w);
                 }
             }
         }
@@ -770,7 +770,7 @@ attn_bwd_query_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
                 tc_fence_after();
             };
             auto release = [&] {
-                tc_commit_elected(empty0 + 8 * (it % S::RING));
+                tc_commit(empty0 + 8 * (it % S::RING));
                 ++it;
             };
             // parts [x_lo, x_hi] of a resident panel (parts `stride` panels apart) against the ring's next panel; with
@@ -819,7 +819,7 @@ attn_bwd_query_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
                     }
                 }
                 if (!alive) break;
-                tc_commit_elected(sfull);
+                tc_commit(sfull);
                 if (!wait_warp(dsready, j & 1, abort_flag, (9 << 8) | 4)) { alive = false; break; }
                 const bool fresh = j == 0 || (flush && j % EVERY == 0);
                 if (fresh && j > 0 && !wait_warp(taken, (j / EVERY - 1) & 1, abort_flag, (9 << 8) | 7)) { alive = false; break; }
@@ -836,11 +836,11 @@ attn_bwd_query_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
                         if (p <= 1) { mma_part_at<1>(d, t_s, t_lead, kd, id_o, first); first = false; }
                         mma_part_at<0>(d, t_s, t_lead, kd, id_o, first);
                         first = false;
-                        tc_commit_elected(empty0 + 8 * (it % S::RING));
+                        tc_commit(empty0 + 8 * (it % S::RING));
                         ++it;
                     }
                 }
-                if (alive && (j + 1 == n || (flush && (j + 1) % EVERY == 0))) tc_commit_elected(done);
+                if (alive && (j + 1 == n || (flush && (j + 1) % EVERY == 0))) tc_commit(done);
             }
         }
     } else {
@@ -1043,10 +1043,10 @@ attn_bwd_key_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
                         first = false;
                     }
                 }
-                tc_commit_elected(free0 + 8 * (op * 2 + buf));
+                tc_commit(free0 + 8 * (op * 2 + buf));
             }
-            if (alive) tc_commit_elected(empty0 + 8 * s);
-            if (alive && (i + 1 == n || (flush && (i + 1) % EVERY == 0))) tc_commit_elected(done);
+            if (alive) tc_commit(empty0 + 8 * s);
+            if (alive && (i + 1 == n || (flush && (i + 1) % EVERY == 0))) tc_commit(done);
         }
     } else {
         const int half = (warp >> 2) & 1, buf = warp >> 3, quarter = warp & 3, r = quarter * 32 + lane;

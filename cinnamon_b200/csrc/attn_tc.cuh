@@ -31,18 +31,6 @@ struct Picks {
     const int* repeats;                    // (B, tiles): whether a query of the tile picked a key more than once
 };
 
-// The MMA warp runs as a whole and one elected lane issues: with warp-uniform control flow the descriptors live in
-// uniform registers.  Issued from a branch that one lane takes, an MMA cost its issuer 70 to 130 cycles of moves, more
-// than the MMA itself.
-// D[tmem] (+)= A[smem desc] * B[smem desc], 16-bit operands, fp32 accumulation
-__device__ __forceinline__ void mma_ss(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
-    asm volatile(
-        "{\n\t.reg .pred p, e;\n\t"
-        "elect.sync _|e, 0xffffffff;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "@e tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-        ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate) : "memory");
-}
 // D[tmem] (+)= A[tmem] * B[smem desc]
 __device__ __forceinline__ void mma_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
     asm volatile(
@@ -146,9 +134,9 @@ __device__ __forceinline__ uint64_t panel_desc(uint32_t panel) { return make_sme
 
 // D (+)= A B over the 64 columns of two K-major panels; the first step overwrites D when `fresh`
 __device__ __forceinline__ void mma_panels(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, bool fresh) {
-    mma_ss(d, a, b, idesc, fresh ? 0u : 1u);
+    tc_mma_f16(d, a, b, idesc, fresh ? 0u : 1u);
 #pragma unroll
-    for (int s = 1; s < 4; ++s) mma_ss(d, a + s * K_STEP, b + s * K_STEP, idesc, 1u);
+    for (int s = 1; s < 4; ++s) tc_mma_f16(d, a + s * K_STEP, b + s * K_STEP, idesc, 1u);
 }
 
 // the same for one half (0 or 1) of the 32 positions

@@ -401,8 +401,8 @@ fp8_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
                                                  : make_smem_desc(b_addr + k * 32, 16, 1024);
                         tc_mma_f8(d, ad, bd, idesc, k > 0 ? 1u : 0u);
                     }
-                    tc_commit_elected(tfull0 + 8 * b);      // the partial tile is ready for promotion once these MMAs retire
-                    tc_commit_elected(empty0 + 8 * s);      // and the stage may be refilled
+                    tc_commit(tfull0 + 8 * b);      // the partial tile is ready for promotion once these MMAs retire
+                    tc_commit(empty0 + 8 * s);      // and the stage may be refilled
                 }
             }
             // every MMA issued above must have retired before tensor memory is freed

@@ -105,20 +105,20 @@ grouped_gemm16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
             }
         }
     } else if (warp == EPI_WARPS + 1) {
-        // ------------------------------ MMA issuer ------------------------------
-        if (lane == 0) {
+        // ------------------------------ MMA issuer (whole warp, one elected lane) ------------------------------
+        {
             constexpr uint32_t idesc = make_idesc_f16(BF16_IN, BM, BN);
             uint32_t it = 0, tile_no = 0;
             bool alive = true;
             for (int t = blockIdx.x; t < n_total && alive; t += gridDim.x, ++tile_no) {
                 const uint32_t b = tile_no & 1, bph = (tile_no >> 1) & 1;
-                if (!mbar_wait(tempty0 + 8 * b, bph ^ 1, abort_flag, (2 << 8) | 2)) { alive = false; break; }
+                if (!mbar_wait_warp(tempty0 + 8 * b, bph ^ 1, abort_flag, (2 << 8) | 2)) { alive = false; break; }
                 tc_fence_after();
                 const uint32_t d = tmem_base + b * BN;
                 for (int kb = 0; kb < KB; ++kb, ++it) {
                     const int s = it % STAGES;
                     const uint32_t ph = (it / STAGES) & 1;
-                    if (!mbar_wait(full0 + 8 * s, ph, abort_flag, (2 << 8) | 1)) { alive = false; break; }
+                    if (!mbar_wait_warp(full0 + 8 * s, ph, abort_flag, (2 << 8) | 1)) { alive = false; break; }
                     tc_fence_after();
                     const uint32_t a_addr = smem_u32(smem_a + s * A_BYTES);
                     const uint32_t b_addr = smem_u32(smem_b + s * B_BYTES);

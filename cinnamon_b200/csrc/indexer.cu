@@ -86,7 +86,7 @@ indexer_kernel(const T* __restrict__ q, const T* __restrict__ k, const T* __rest
 __device__ int g_indexer_status = 0;       // 0, or (role << 8) | reason of a bounded wait that ran out
 
 constexpr int ITC_T = 128;                 // queries and keys per tile
-constexpr int ITC_THREADS = 256;           // eight warps load, then fold; thread 0 issues the MMAs as well
+constexpr int ITC_THREADS = 256;           // eight warps load, then fold; warp 0 issues the MMAs as well
 constexpr int ITC_PANEL = ITC_T * 128;     // bytes of 128 rows x 64 fp16 columns: one swizzle panel
 constexpr int ITC_MAX_D = 128;
 constexpr int ITC_Q_BYTES = 64 * 1024;     // resident queries
@@ -210,10 +210,11 @@ indexer_tc_kernel(const T* __restrict__ q, const T* __restrict__ k, const T* __r
         __syncthreads();
         tc_fence_after();
         tmem = *tmem_slot;
-        // head h of the chunk: issued by thread 0 once the buffer's previous dot products have been read
+        // head h of the chunk: issued by warp 0 once the buffer's previous dot products have been read
         auto issue = [&](int h) {
             const uint32_t n = it0 + h, buf = n & 1;
-            if (!mbar_wait_bounded(free0 + 8 * buf, ((n >> 1) & 1) ^ 1, abort_flag, (7 << 8) | 1, &g_indexer_status)) return;
+            const bool ok = mbar_wait_bounded(free0 + 8 * buf, ((n >> 1) & 1) ^ 1, abort_flag, (7 << 8) | 1, &g_indexer_status);
+            if (!__all_sync(0xffffffffu, ok)) return;
             tc_fence_after();
             for (int s = 0; s < a.dpad / 16; ++s) {
                 const uint32_t off = (s >> 2) * ITC_PANEL + (s & 3) * 32;
@@ -222,11 +223,10 @@ indexer_tc_kernel(const T* __restrict__ q, const T* __restrict__ k, const T* __r
             }
             tc_commit(full0 + 8 * buf);
         };
-        if (tid == 0) {
+        if (warp == 0) {
             issue(0);
             if (nh > 1) issue(1);
         }
-        __syncwarp();
         for (int h = 0; h < nh && alive; ++h) {
             const uint32_t n = it0 + h, buf = n & 1;
             const float wh = t < a.Lq ? w_to_float<T>(w[b * a.swb + t * a.swq + (h0 + h) * a.swh]) : 0.0f;
@@ -244,8 +244,8 @@ indexer_tc_kernel(const T* __restrict__ q, const T* __restrict__ k, const T* __r
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive(free0 + 8 * buf);
-            if (tid == 0 && h + 2 < nh) issue(h + 2);
             __syncwarp();
+            if (warp == 0 && h + 2 < nh) issue(h + 2);
         }
         it0 += nh;
         __syncthreads();              // every MMA of these heads has been read, hence has finished: the queries may go

@@ -27,12 +27,9 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint32_t bar, uint32_t parity,
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 
+// Arrival on the barrier once the MMAs issued so far have retired; called by a whole warp and issued by the lane that
+// elect.sync chooses, the one that issued the MMAs.
 __device__ __forceinline__ void tc_commit(uint32_t bar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
-}
-
-// the same, called by a whole warp and issued by the lane that elect.sync chooses (the one that issued the MMAs)
-__device__ __forceinline__ void tc_commit_elected(uint32_t bar) {
     asm volatile(
         "{\n\t.reg .pred e;\n\t"
         "elect.sync _|e, 0xffffffff;\n\t"
@@ -49,12 +46,16 @@ __device__ __forceinline__ void tc_dealloc(uint32_t base, uint32_t cols) {
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(base), "r"(cols) : "memory");
 }
 
+// The MMA warp runs as a whole and one elected lane issues: with warp-uniform control flow the descriptors live in
+// uniform registers.  Issued from a branch that one lane takes, an MMA cost its issuer 70 to 130 cycles of moves, more
+// than the MMA itself.
 // 16-bit operands of one type: D[tmem] (+)= A[smem desc] * B[smem desc], fp32 accumulation
 __device__ __forceinline__ void tc_mma_f16(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
     asm volatile(
-        "{\n\t.reg .pred p;\n\t"
+        "{\n\t.reg .pred p, e;\n\t"
+        "elect.sync _|e, 0xffffffff;\n\t"
         "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+        "@e tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
         ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate) : "memory");
 }
 
