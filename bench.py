@@ -658,7 +658,9 @@ def bench_moe(Kmod, dev, rank, world, steps, warmup, bias_scale, label, chunks=1
         q_s, s_s = Kmod.quantize_fp8_rowwise(x_s)
         gq, gsc = Kmod.gather_quantized_rows(q_s, s_s, r_s["token_indices"])
         rows_out = full(gq, gsc, starts_s, ends_s)
-        y_ref = Kmod.moe_combine(rows_out, r_s["pair_pos"], r_s["pair_gate"], module.shared(x_s))
+        # (the shared expert on all tokens, then the sampled ones: alone, a few hundred tokens are cut along K, which adds the
+        # same products in another order)
+        y_ref = Kmod.moe_combine(rows_out, r_s["pair_pos"], r_s["pair_gate"], module.shared(x)[idx].contiguous())
         y_got = y.reshape(T_local, c["d"])[idx]
         err = float((y_got - y_ref).norm() / y_ref.norm())
         bit_equal = bool(torch.equal(y_got, y_ref))

@@ -1134,9 +1134,10 @@ class MoEGroupedGemmFunction(torch.autograd.Function):
     ``FP8MatmulFunction`` (src/kernels.py:763-794) expert by expert:
 
       dX[e rows] = rowwise(dY[e rows]) @ W_q[e]                                 one grouped launch
-      dW[e]      = rowwise(dY[e rows]^T) @ blockwise(dequant_rowwise(x_q[e rows]))   per non-empty expert
+      dW[e]      = rowwise(dY[e rows]^T) @ blockwise(dequant_rowwise(x_q[e rows]))
 
-    The weight gradient walks the experts on the host (their row counts are read back once per backward)."""
+    Widths that are multiples of 256: all experts' weight gradients in four launches; other widths: expert by expert, after
+    one read-back of the row ranges."""
 
     @staticmethod
     def forward(ctx, sorted_x, weights, expert_starts, expert_ends, out_dtype):
