@@ -39,6 +39,7 @@ SIGNATURES = {
     "cinn_fp8_gemm": [_vp, _vp, _i64, _vp, _vp, _i64, _i64, _vp, _i64, _i64, _i64, _i32, _i32, _vp],
     "cinn_fp8_gemm_workspace_bytes": [_i64, _i64, _i64, _i32],
     "cinn_fp8_gemm_ws": [_vp, _vp, _i64, _vp, _vp, _i64, _i64, _vp, _i64, _i64, _i64, _i32, _i32, _vp, _i64, _vp],
+    "cinn_fp8_gemm_pitched": [_vp, _i64, _vp, _i64, _vp, _i64, _vp, _i64, _i64, _vp, _i64, _i64, _i64, _i32, _i32, _vp, _i64, _vp],
     "cinn_grouped_gemm_16bit": [_vp, _vp, _i32, _vp, _vp, _i64, _i64, _i64, _i64, _vp, _i32, _vp],
     "cinn_fp8_grouped_gemm_dgrad": [_vp, _vp, _vp, _vp, _vp, _vp, _i64, _i64, _i64, _i64, _vp, _i32, _vp],
     "cinn_moe_combine": [_vp, _i32, _vp, _vp, _vp, _i64, _i64, _i32, _i64, _vp],

@@ -40,8 +40,8 @@ int dequantize(const void* q, const float* scales, void* out, int out_dtype, int
 int transpose_bytes(const void* in, int64_t ld_in, void* out, int64_t R, int64_t C, cudaStream_t st);
 int swiglu_quant_rowwise(const void* h12, int dtype, int64_t T_rows, int64_t I, void* q, float* scales, int div_mode,
                          cudaStream_t st, const int64_t* n_rows_dev);
-int fp8_gemm(const void* A, const float* sA, int64_t ld_sa, const void* B, const float* sB, int64_t sbk, int64_t sbn,
-             void* C, int64_t M, int64_t N, int64_t K, int b_layout, int out_dtype, cudaStream_t st, void* workspace,
+int fp8_gemm(const void* A, int64_t lda, const float* sA, int64_t ld_sa, const void* B, int64_t ldb, const float* sB, int64_t sbk,
+             int64_t sbn, void* C, int64_t M, int64_t N, int64_t K, int b_layout, int out_dtype, cudaStream_t st, void* workspace,
              int64_t workspace_bytes);
 int quantize_linear(const void* x, int x_dtype, int64_t ldx_m, int64_t ldx_k, void* xq, float* xs, int round_scale, const void* w,
                     int w_dtype, int64_t ldw_n, int64_t ldw_k, void* wq, float* ws, int64_t M, int64_t N, int64_t K, int div_mode,
@@ -222,7 +222,7 @@ int cinn_transpose_bytes(const void* in, int64_t ld_in, void* out, int64_t R, in
 int cinn_fp8_gemm(const void* A, const float* sA, int64_t ld_sa, const void* B, const float* sB, int64_t sb_stride_k,
                   int64_t sb_stride_n, void* C, int64_t M, int64_t N, int64_t K, int b_layout, int out_dtype,
                   void* stream) {
-    return cinn::fp8_gemm(A, sA, ld_sa, B, sB, sb_stride_k, sb_stride_n, C, M, N, K, b_layout, out_dtype,
+    return cinn::fp8_gemm(A, K, sA, ld_sa, B, b_layout == 0 ? K : N, sB, sb_stride_k, sb_stride_n, C, M, N, K, b_layout, out_dtype,
                           (cudaStream_t)stream, nullptr, 0);
 }
 
@@ -233,8 +233,15 @@ int64_t cinn_fp8_gemm_workspace_bytes(int64_t M, int64_t N, int64_t K, int b_lay
 int cinn_fp8_gemm_ws(const void* A, const float* sA, int64_t ld_sa, const void* B, const float* sB, int64_t sb_stride_k,
                      int64_t sb_stride_n, void* C, int64_t M, int64_t N, int64_t K, int b_layout, int out_dtype,
                      void* workspace, int64_t workspace_bytes, void* stream) {
-    return cinn::fp8_gemm(A, sA, ld_sa, B, sB, sb_stride_k, sb_stride_n, C, M, N, K, b_layout, out_dtype,
+    return cinn::fp8_gemm(A, K, sA, ld_sa, B, b_layout == 0 ? K : N, sB, sb_stride_k, sb_stride_n, C, M, N, K, b_layout, out_dtype,
                           (cudaStream_t)stream, workspace, workspace_bytes);
+}
+
+int cinn_fp8_gemm_pitched(const void* A, int64_t lda, const float* sA, int64_t ld_sa, const void* B, int64_t ldb, const float* sB,
+                          int64_t sb_stride_k, int64_t sb_stride_n, void* C, int64_t M, int64_t N, int64_t K, int b_layout,
+                          int out_dtype, void* workspace, int64_t workspace_bytes, void* stream) {
+    return cinn::fp8_gemm(A, lda, sA, ld_sa, B, ldb, sB, sb_stride_k, sb_stride_n, C, M, N, K, b_layout, out_dtype, (cudaStream_t)stream,
+                          workspace, workspace_bytes);
 }
 
 int cinn_fp8_grouped_gemm(const void* A, const float* sA, const void* W, const float* sW, const int64_t* starts,

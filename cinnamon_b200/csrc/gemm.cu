@@ -839,8 +839,9 @@ int64_t fp8_gemm_workspace_bytes(int64_t M, int64_t N, int64_t K, int b_layout) 
     return plan.splits > 1 ? plan.splits * M * N * 4 : 0;
 }
 
-int fp8_gemm(const void* A, const float* sA, int64_t ld_sa, const void* B, const float* sB, int64_t sbk, int64_t sbn,
-             void* C, int64_t M, int64_t N, int64_t K, int b_layout, int out_dtype, cudaStream_t st, void* workspace,
+// lda, ldb: bytes from one stored row of A and B to the next (a column range of a wider matrix is read in place)
+int fp8_gemm(const void* A, int64_t lda, const float* sA, int64_t ld_sa, const void* B, int64_t ldb, const float* sB, int64_t sbk,
+             int64_t sbn, void* C, int64_t M, int64_t N, int64_t K, int b_layout, int out_dtype, cudaStream_t st, void* workspace,
              int64_t workspace_bytes) {
     CINN_CHECK_ARG(M >= 0 && N >= 0 && K >= 0, "fp8_gemm: negative shape");
     if (M == 0 || N == 0) return CINN_OK;
@@ -851,12 +852,14 @@ int fp8_gemm(const void* A, const float* sA, int64_t ld_sa, const void* B, const
     CINN_CHECK_ARG(al16(A) && al16(B) && al16(C) && al16(workspace), "fp8_gemm: A, B, C and the workspace must be 16-byte aligned");
     CINN_CHECK_ARG(b_layout == 0 || b_layout == 1, "fp8_gemm: unknown B layout %d", b_layout);
     CINN_CHECK_ARG(b_layout == 0 || N % 16 == 0, "fp8_gemm: B stored (K, N) needs N %% 16 == 0");
+    CINN_CHECK_ARG(lda >= K && ldb >= (b_layout == 0 ? K : N) && lda % 16 == 0 && ldb % 16 == 0,
+                   "fp8_gemm: row pitches (%lld, %lld) must be multiples of 16 and no shorter than a row", (long long)lda, (long long)ldb);
     const DensePlan plan = dense_plan(M, N, K, b_layout, workspace ? workspace_bytes : 0);
     CUtensorMap ta, tb;
-    int rc = make_map(&ta, A, (uint64_t)K, (uint64_t)M, (uint64_t)K, BK, BM);
+    int rc = make_map(&ta, A, (uint64_t)K, (uint64_t)M, (uint64_t)lda, BK, BM);
     if (rc) return rc;
-    if (b_layout == 0) rc = make_map(&tb, B, (uint64_t)K, (uint64_t)N, (uint64_t)K, BK, plan.pair ? 128 : BN);
-    else rc = make_map(&tb, B, (uint64_t)N, (uint64_t)K, (uint64_t)N, 128, BK);
+    if (b_layout == 0) rc = make_map(&tb, B, (uint64_t)K, (uint64_t)N, (uint64_t)ldb, BK, plan.pair ? 128 : BN);
+    else rc = make_map(&tb, B, (uint64_t)N, (uint64_t)K, (uint64_t)ldb, 128, BK);
     if (rc) return rc;
     GemmParams p{};
     p.sA = sA; p.sa_stride_m = ld_sa; p.sa_stride_k = 1;

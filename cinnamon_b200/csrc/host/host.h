@@ -24,7 +24,7 @@ using at::Tensor;
 #define CINN_HOST_API(X)                                                                                            \
     X(cinn_last_error) X(cinn_quant_rowwise) X(cinn_quant_rowwise_dual) X(cinn_quant_rowwise_with_block)             \
     X(cinn_quant_rowwise_with_block_t) X(cinn_quant_blockwise) X(cinn_quant_block_beside) X(cinn_quant_linear) X(cinn_transpose_bytes)     \
-    X(cinn_requant_row_to_block) X(cinn_fp8_gemm_ws) X(cinn_fp8_gemm_workspace_bytes) \
+    X(cinn_requant_row_to_block) X(cinn_fp8_gemm_ws) X(cinn_fp8_gemm_pitched) X(cinn_fp8_gemm_workspace_bytes) \
     X(cinn_sparse_attn_workspace_bytes) X(cinn_sparse_attn_fwd_ws) X(cinn_sparse_attn_bwd) X(cinn_sparse_attn_bwd_ws)                  \
     X(cinn_moe_route_workspace_ints) X(cinn_moe_route_ranges) X(cinn_spread_rows) X(cinn_fp8_grouped_gemm)                \
     X(cinn_swiglu_quant_rowwise) X(cinn_moe_combine) X(cinn_moe_combine_add)                \
@@ -98,10 +98,13 @@ struct Linear {                                 // what an FP8 linear's forward 
 };
 Linear linear_forward(const Tensor& x, const Tensor& weight, bool round_scale, bool need_dgrad, bool need_wgrad, bool kmajor, int div,
                       const Tensor& w_q, const Tensor& w_s, const Tensor& w_qt);
-std::tuple<Tensor, Tensor> linear_backward(const Tensor& grad_out, Tensor x, Tensor x_scale, const Tensor& w, const Tensor& w_scale,
-                                           const Tensor& w_t, at::IntArrayRef x_shape, bool round_scale, bool x_is_block,
-                                           bool x_is_block_t, at::ScalarType weight_dtype, bool kmajor, int div, bool want_gx,
-                                           bool want_gw, at::ScalarType gx_type);
+// (input gradients, weight gradient).  `parts` > 1: the weight is that many layers of equally many rows (a multiple of 128)
+// stacked, and every layer's input gradient is returned by itself.
+std::tuple<std::vector<Tensor>, Tensor> linear_backward(const Tensor& grad_out, Tensor x, Tensor x_scale, const Tensor& w,
+                                                        const Tensor& w_scale, const Tensor& w_t, at::IntArrayRef x_shape,
+                                                        bool round_scale, bool x_is_block, bool x_is_block_t,
+                                                        at::ScalarType weight_dtype, bool kmajor, int div, bool want_gx,
+                                                        bool want_gw, at::ScalarType gx_type, int parts = 1);
 
 struct Quantised { Tensor q, s; };
 Quantised rowwise(const Tensor& x, bool round_scale, int div);                 // moe.cpp

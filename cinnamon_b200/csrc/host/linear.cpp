@@ -75,10 +75,11 @@ Linear linear_forward(const Tensor& x, const Tensor& weight, bool round_scale, b
     return r;
 }
 
-std::tuple<Tensor, Tensor> linear_backward(const Tensor& grad_out, Tensor x, Tensor x_scale, const Tensor& w, const Tensor& w_scale,
-                                    const Tensor& w_t, at::IntArrayRef x_shape, bool round_scale, bool x_is_block,
-                                    bool x_is_block_t, at::ScalarType weight_dtype, bool kmajor, int div, bool want_gx,
-                                           bool want_gw, at::ScalarType gx_type) {
+std::tuple<std::vector<Tensor>, Tensor> linear_backward(const Tensor& grad_out, Tensor x, Tensor x_scale, const Tensor& w,
+                                                        const Tensor& w_scale, const Tensor& w_t, at::IntArrayRef x_shape,
+                                                        bool round_scale, bool x_is_block, bool x_is_block_t,
+                                                        at::ScalarType weight_dtype, bool kmajor, int div, bool want_gx,
+                                                        bool want_gw, at::ScalarType gx_type, int parts) {
     c10::cuda::CUDAGuard guard(w.device());
     const at::Device dev = w.device();
     const int64_t N = w.size(0), K = w.size(1);
@@ -100,20 +101,29 @@ std::tuple<Tensor, Tensor> linear_backward(const Tensor& grad_out, Tensor x, Ten
     ++launches;
     // (the reference's input gradient is bf16 and autograd casts it to the input's type: fp32 holds those values)
     const int gx_tag = gx_type == at::kFloat ? TAG_F32_BF16 : TAG_BF16;
-    Tensor gx;
-    if (!want_gx) {
-    } else if (N % 16 == 0 && (kmajor || w_t.defined())) {
+    std::vector<Tensor> gx(parts);
+    if (want_gx) {
+        const bool k_major = N % 16 == 0 && (kmajor || w_t.defined());
         Tensor wt = w_t;
-        if (!wt.defined()) {
+        if (k_major && !wt.defined()) {
             wt = empty({K, N}, F8, dev);
             check(api.cinn_transpose_bytes(w.data_ptr(), w.stride(0), wt.data_ptr(), N, K, stream()), "cinn_transpose_bytes");
             ++launches;
         }
-        gx = gemm(gq, gs, wt, 0, w_scale, w_scale.stride(0), w_scale.stride(1), M, K, N, gx_type, gx_tag);
-    } else {
-        gx = gemm(gq, gs, w, 1, w_scale, w_scale.stride(0), w_scale.stride(1), M, K, N, gx_type, gx_tag);
+        const int64_t n = N / parts;                // reduction length of a part: columns of gq and wt, rows of w
+        const int64_t need = api.cinn_fp8_gemm_workspace_bytes(M, K, n, k_major ? 0 : 1);
+        Tensor ws = need ? empty({need}, at::kByte, dev) : Tensor();
+        for (int p = 0; p < parts; ++p) {
+            Tensor out = empty({M, K}, gx_type, dev);
+            const uint8_t* b = static_cast<const uint8_t*>(k_major ? wt.data_ptr() : w.data_ptr()) + p * n * (k_major ? 1 : K);
+            check(api.cinn_fp8_gemm_pitched(static_cast<const uint8_t*>(gq.data_ptr()) + p * n, N, f32(gs) + p * (n / 128), gs.stride(0), b,
+                                            k_major ? N : K, f32(w_scale) + p * (n / 128) * w_scale.stride(0), w_scale.stride(0),
+                                            w_scale.stride(1), out.data_ptr(), M, K, n, k_major ? 0 : 1, gx_tag,
+                                            need ? ws.data_ptr() : nullptr, need, stream()), "cinn_fp8_gemm");
+            launches += need ? 2 : 1;
+            gx[p] = x_shape.size() != 2 ? out.reshape(x_shape) : out;
+        }
     }
-    if (gx.defined() && x_shape.size() != 2) gx = gx.reshape(x_shape);
     if (!want_gw) return {gx, Tensor()};
     if (!x_is_block) {
         Tensor xb = empty({Mp, K}, F8, dev), xbs = empty({up(Mp, 128), up(K, 128)}, at::kFloat, dev);
@@ -178,13 +188,14 @@ public:
     static torch::autograd::variable_list backward(torch::autograd::AutogradContext* ctx, torch::autograd::variable_list grads) {
         auto s = ctx->get_saved_variables();
         const int64_t f = ctx->saved_data["flags"].toInt();
-        Tensor gx, gw;
+        std::vector<Tensor> gx(1);
+        Tensor gw;
         as_python_error([&] {
             std::tie(gx, gw) = linear_backward(grads[0], s[0], s[1], s[2], s[3], s[4], ctx->saved_data["x_shape"].toIntVector(), f & 1,
                                                   f & 2, f & 4, (at::ScalarType)(f >> 8 & 255), f & 8, (f >> 4) & 15, ctx->needs_input_grad(0),
                                                   ctx->needs_input_grad(1), f >> 16 & 1 ? at::kFloat : at::kBFloat16);
         });
-        return {gx, gw, Tensor(), Tensor(), Tensor(), Tensor()};
+        return {gx[0], gw, Tensor(), Tensor(), Tensor(), Tensor()};
     }
 };
 
@@ -202,8 +213,9 @@ void bind_linear(pybind11::module_& m) {
     m.def("linear_backward", [](const Tensor& g, const Tensor& x, const Tensor& xs, const Tensor& w, const Tensor& ws, const OptT& wt,
                                 const std::vector<int64_t>& x_shape, bool round_scale, bool x_is_block, bool x_is_block_t, bool w_fp32,
                                 bool kmajor, int div) {
-        return linear_backward(g, x, xs, w, ws, or_none(wt), x_shape, round_scale, x_is_block, x_is_block_t,
-                        w_fp32 ? at::kFloat : at::kBFloat16, kmajor, div, true, true, at::kBFloat16);
+        auto [gx, gw] = linear_backward(g, x, xs, w, ws, or_none(wt), x_shape, round_scale, x_is_block, x_is_block_t,
+                                        w_fp32 ? at::kFloat : at::kBFloat16, kmajor, div, true, true, at::kBFloat16);
+        return std::make_tuple(gx[0], gw);
     });
     // the differentiable call; without gradients to record nothing is saved and no gradient copies are made
     m.def("linear", [](const Tensor& x, const Tensor& w, bool round_scale, bool kmajor, int div, const OptT& wq, const OptT& ws,

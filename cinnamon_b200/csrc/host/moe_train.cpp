@@ -1,7 +1,8 @@
 // The trainable MoE block (layers.MoE, layers.SwiGLU) as two native autograd nodes: the shared expert, and router + routed
 // experts + combine.  Written as modules and torch calls the block was 128 launches and 2.7 ms of host time per step at 32 x
 // 1024 tokens of 512; as nodes it also stops converting and copying between its parts:
-//   - w1 and w2 of a shared expert are one GEMM on x quantised once, forward and backward
+//   - w1 and w2 of a shared expert share one quantisation of x and one of their output gradients, and one GEMM forward and
+//     for the weight gradients
 //   - tokens are quantised once and their bytes spread to the experts' rows (forward); the rows' gradients come home as one
 //     gather pass with the router's part added in it (backward), where autograd's index_select needed an atomic index_add
 //   - expert outputs stay in bf16 up to the combine pass, their gradients likewise
@@ -28,8 +29,13 @@ Tensor swiglu_rounded(const Tensor& h12) {
     return h;
 }
 
+// x comes in twice, once for w2 and once for w1: each of the two layers returns an input gradient of its own, rounded to bf16
+// as the layer by itself rounds it, and autograd adds them up in the order in which it would for two layers.  (One product over
+// [dh1 dh2] [w1; w2] rounds once and is 20 us faster at 32768 tokens, but then the block's gradient depends on whether a
+// hook, a traced call or a compiled one takes it through its layers: 2e-3 of the gradient.)
 struct SwiGLUNode : public torch::autograd::Function<SwiGLUNode> {
-    static Tensor forward(AutogradContext* ctx, const Tensor& x, const Tensor& w1, const Tensor& w2, const Tensor& w3, const SwiGLUOptions* o) {
+    static Tensor forward(AutogradContext* ctx, const Tensor& x, const Tensor&, const Tensor& w1, const Tensor& w2, const Tensor& w3,
+                          const SwiGLUOptions* o) {
         c10::cuda::CUDAGuard guard(x.device());
         const bool gx = x.requires_grad(), g12 = w1.requires_grad() || w2.requires_grad(), g3 = w3.requires_grad(), any = gx || g12;
         const Linear a = linear_forward(x, at::cat({w1, w2}), o->round12, gx, g12, o->kmajor, o->div, Tensor(), Tensor(), Tensor());
@@ -53,31 +59,33 @@ struct SwiGLUNode : public torch::autograd::Function<SwiGLUNode> {
 
     static variable_list backward(AutogradContext* ctx, variable_list grads) {
         auto s = ctx->get_saved_variables();
-        const bool gx = ctx->needs_input_grad(0), g12 = ctx->needs_input_grad(1) || ctx->needs_input_grad(2), g3 = ctx->needs_input_grad(3);
-        Tensor dx, d1, d2, d3;
+        const bool gx = ctx->needs_input_grad(0), g12 = ctx->needs_input_grad(2) || ctx->needs_input_grad(3), g3 = ctx->needs_input_grad(4);
+        std::vector<Tensor> dx(2), dh(1);
+        Tensor d1, d2, d3;
         as_python_error([&] {
-            auto back = [&](int64_t f, const Tensor& g, int at, at::IntArrayRef shape, bool want_x, bool want_w, at::ScalarType type) {
+            auto back = [&](int64_t f, const Tensor& g, int at, at::IntArrayRef shape, bool want_x, bool want_w, at::ScalarType type,
+                            int parts) {
                 return linear_backward(g, s[at], s[at + 1], s[at + 2], s[at + 3], s[at + 4], shape, f & 1, f & 2, f & 4,
-                                       (at::ScalarType)(f >> 8 & 255), f & 8, (int)(f >> 4 & 15), want_x, want_w, type);
+                                       (at::ScalarType)(f >> 8 & 255), f & 8, (int)(f >> 4 & 15), want_x, want_w, type, parts);
             };
             const Tensor& h12 = s[5];
             const int64_t T = h12.size(0), I = h12.size(1) / 2;
-            Tensor dh;
-            std::tie(dh, d3) = back(ctx->saved_data["b"].toInt(), grads[0], 6, {T, I}, gx || g12, g3, at::kBFloat16);
+            std::tie(dh, d3) = back(ctx->saved_data["b"].toInt(), grads[0], 6, {T, I}, gx || g12, g3, at::kBFloat16, 1);
             if (!(gx || g12)) return;
             c10::cuda::CUDAGuard guard(h12.device());
             Tensor dh12 = empty({T, 2 * I}, h12.scalar_type(), h12.device()), d12;
-            check(api.cinn_swiglu_rounded_backward(h12.data_ptr(), dh.data_ptr(), dh12.data_ptr(), tag_of(h12.scalar_type()), T, I, stream()),
+            check(api.cinn_swiglu_rounded_backward(h12.data_ptr(), dh[0].data_ptr(), dh12.data_ptr(), tag_of(h12.scalar_type()), T, I, stream()),
                   "cinn_swiglu_backward");
             ++launches;
             std::tie(dx, d12) = back(ctx->saved_data["a"].toInt(), dh12, 0, ctx->saved_data["x_shape"].toIntVector(), gx, g12,
-                                     ctx->saved_data["x32"].toBool() ? at::kFloat : at::kBFloat16);
+                                     ctx->saved_data["x32"].toBool() ? at::kFloat : at::kBFloat16, 2);
             if (g12) {
-                d1 = d12.narrow(0, 0, I);
-                d2 = d12.narrow(0, I, I);
+                const auto halves = at::unsafe_split(d12, I, 0);
+                d1 = halves[0];
+                d2 = halves[1];
             }
         });
-        return {dx, d1, d2, d3, Tensor()};
+        return {dx[1], dx[0], d1, d2, d3, Tensor()};
     }
 };
 
@@ -276,7 +284,7 @@ void bind_moe_train(pybind11::module_& m) {
     m.def("swiglu_block", [](const Tensor& x, const Tensor& w1, const Tensor& w2, const Tensor& w3, bool round12, bool round3, bool kmajor,
                              int div) {
         const SwiGLUOptions o{round12, round3, kmajor, div};
-        return SwiGLUNode::apply(x, w1, w2, w3, &o);
+        return SwiGLUNode::apply(x, x, w1, w2, w3, &o);
     });
     m.def("grouped_gemm", [](const Tensor& x, const Tensor& w, const Tensor& starts, const Tensor& ends, const Tensor& w_q, const Tensor& w_s,
                              int tag, int div) {

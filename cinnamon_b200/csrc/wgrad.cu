@@ -16,8 +16,8 @@ int quantize_transposed_padded(const void* x, int dtype, int64_t M, int64_t N_in
                                float* scales, int div_mode, cudaStream_t st);
 int requant_row_to_block_padded(const void* xq, const float* xs, int64_t M_in, int64_t M, int64_t K, void* out, float* scales,
                                 int div_mode, cudaStream_t st);
-int fp8_gemm(const void* A, const float* sA, int64_t ld_sa, const void* B, const float* sB, int64_t sbk, int64_t sbn,
-             void* C, int64_t M, int64_t N, int64_t K, int b_layout, int out_dtype, cudaStream_t st, void* workspace,
+int fp8_gemm(const void* A, int64_t lda, const float* sA, int64_t ld_sa, const void* B, int64_t ldb, const float* sB, int64_t sbk,
+             int64_t sbn, void* C, int64_t M, int64_t N, int64_t K, int b_layout, int out_dtype, cudaStream_t st, void* workspace,
              int64_t workspace_bytes);
 
 static inline int64_t up(int64_t v, int64_t a) { return (v + a - 1) / a * a; }
@@ -72,7 +72,7 @@ int fp8_grouped_wgrad(const void* dY, int dy_dtype, const void* x_q, const float
         rc = requant_row_to_block_padded(static_cast<const uint8_t*>(x_q) + s * d_in, x_s + s * nkb, n, n_pad, d_in, xb_q, xb_s,
                                          div_mode, st);
         if (rc) return rc;
-        rc = fp8_gemm(gt_q, gt_s, nt, xb_q, xb_s, nkb, 1, dw_e, d_out, d_in, n_pad, 1 /* B stored (K, N) */, out_dtype, st, nullptr, 0);
+        rc = fp8_gemm(gt_q, n_pad, gt_s, nt, xb_q, d_in, xb_s, nkb, 1, dw_e, d_out, d_in, n_pad, 1 /* B stored (K, N) */, out_dtype, st, nullptr, 0);
         if (rc) return rc;
     }
     return CINN_OK;

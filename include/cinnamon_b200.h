@@ -161,6 +161,12 @@ int cinn_fp8_gemm_ws(const void* A, const float* sA, int64_t ld_sa, const void* 
                      int64_t sb_stride_k, int64_t sb_stride_n, void* C, int64_t M, int64_t N, int64_t K,
                      int b_layout, int out_dtype, void* workspace, int64_t workspace_bytes, void* stream);
 
+/* The same with row pitches: stored rows of A and B lie lda and ldb bytes apart (multiples of 16), so that a range of columns
+ * of a wider matrix is multiplied where it lies. */
+int cinn_fp8_gemm_pitched(const void* A, int64_t lda, const float* sA, int64_t ld_sa, const void* B, int64_t ldb, const float* sB,
+                          int64_t sb_stride_k, int64_t sb_stride_n, void* C, int64_t M, int64_t N, int64_t K, int b_layout,
+                          int out_dtype, void* workspace, int64_t workspace_bytes, void* stream);
+
 /* Grouped (per-expert) block-scaled FP8 GEMM over ragged row ranges:
  * for each expert e:  C[starts[e]:ends[e], :] = A[starts[e]:ends[e], :] @ W[e]^T.
  * Replaces grouped_gemm_kernel + moe_grouped_gemm (src/kernels.py:440-523, 526-581); the reference runs it in

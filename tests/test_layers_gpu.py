@@ -175,3 +175,27 @@ def test_native_block_matches_the_module_path(K, case, autocast):
     assert gx0.dtype == gx1.dtype and rel(gx0, gx1) < 1e-2
     for name, p in p0.items():
         assert p.grad.dtype == p1[name].grad.dtype and rel(p.grad, p1[name].grad) < 1e-2, name
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("tokens,d,hidden", [(48, 256, 512), (131, 384, 128)])
+def test_native_swiglu_is_its_layers_bit_for_bit(K, dtype, tokens, d, hidden):
+    """The shared expert as one node against the same three layers (a hook on one of them selects that path): every output
+    and gradient is the same number, x's too, whose two parts are rounded by layer and added up in autograd's order.
+    (Reductions of fewer than 20 blocks of 128 are never cut, so no sum is taken in another order.)"""
+    from cinnamon_b200 import layers
+    torch.manual_seed(tokens)
+    with torch.device("cuda"):
+        block = layers.SwiGLU(d, hidden)
+    block = K.convert_to_fp8(block)
+    x = torch.randn(tokens, d, device="cuda").to(dtype)
+    dy = torch.randn(tokens, d, device="cuda").bfloat16()
+    base = torch.randn(tokens, d, device="cuda").to(dtype)                     # a third gradient of x, from elsewhere
+    got = []
+    for _ in range(2):
+        xi = x.clone().requires_grad_(True)
+        y = block(xi)
+        got.append([y, *torch.autograd.grad([y, xi * base], [xi, *block.parameters()], [dy, torch.ones_like(xi)])])
+        block.w1.register_forward_hook(lambda *args: None)
+    for a, b in zip(*got):
+        assert a.dtype == b.dtype and torch.equal(a, b)
