@@ -199,3 +199,22 @@ def test_native_swiglu_is_its_layers_bit_for_bit(K, dtype, tokens, d, hidden):
         block.w1.register_forward_hook(lambda *args: None)
     for a, b in zip(*got):
         assert a.dtype == b.dtype and torch.equal(a, b)
+
+
+def test_native_routed_experts_compute_the_module_paths_silu(K):
+    """Forward of the block on widely spread activations (two experts per token, whose gates both paths add up alike): the
+    node quantises silu(h1) * h2 in the pass that computes it, the module path from a bf16 copy; the output is the same, bit
+    for bit."""
+    from cinnamon_b200 import layers
+    torch.manual_seed(7)
+    with torch.device("cuda"):
+        block = layers.MoE(4, 1, 2, 256, 1024, 2, 0.0, 0.0)
+    block = K.convert_to_fp8(block).eval()
+    with torch.no_grad():
+        block.routed_experts.w12.mul_(12.0)
+    x = torch.randn(1, 8192, 256, device="cuda")
+    with torch.autocast("cuda", dtype=torch.bfloat16):
+        native, _ = block(x)
+        block.router.register_forward_hook(lambda *args: None)
+        modules, _ = block(x)
+    assert torch.equal(native, modules)
