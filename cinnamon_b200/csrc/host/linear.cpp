@@ -15,9 +15,23 @@ Tensor gemm(const Tensor& a, const Tensor& sa, const Tensor& b, int layout, cons
     return out;
 }
 
+// What the kernels take for granted, refused on the host before anything is launched.  w_q, w_s: the weight's e4m3 copy, or
+// undefined.
+static void check_operands(const Tensor& x, const Tensor& weight, const Tensor& w_q, const Tensor& w_s) {
+    require(x.is_cuda() && weight.is_cuda(), "Input must be on CUDA");
+    require(weight.device() == x.device(), "FP8 linear: input and weight must be on the same device");
+    require(x.dim() >= 1 && weight.dim() == 2 && weight.size(1) == x.size(-1),
+            "FP8 linear: the weight must be a matrix as wide as the input's last dimension");
+    TORCH_CHECK(x.numel() > 0, "FP8 linear: the input has no rows");
+    if (!w_q.defined()) return;
+    require(w_s.defined() && w_q.device() == x.device() && w_s.device() == x.device() && w_q.sizes() == weight.sizes() && w_q.is_contiguous() &&
+                w_q.scalar_type() == F8 && w_s.scalar_type() == at::kFloat && w_s.dim() == 2 && w_s.size(0) == up(weight.size(0), 128) &&
+                w_s.size(1) == up(weight.size(1), 128), "FP8 linear: the quantised copy does not belong to the weight");
+}
+
 Linear linear_forward(const Tensor& x, const Tensor& weight, bool round_scale, bool need_dgrad, bool need_wgrad, bool kmajor, int div,
                const Tensor& w_q, const Tensor& w_s, const Tensor& w_qt) {
-    require(x.is_cuda(), "Input must be on CUDA");
+    check_operands(x, weight, w_q, w_s);
     c10::cuda::CUDAGuard guard(x.device());
     const at::Device dev = x.device();
     const int64_t K = x.size(-1), N = weight.size(0);
@@ -57,13 +71,10 @@ Linear linear_forward(const Tensor& x, const Tensor& weight, bool round_scale, b
         if (kmajor && need_dgrad && N % 16 == 0 && K % 4 == 0 && wf.stride(1) == 1 && wf.stride(0) % 4 == 0) {
             r.w_t = empty({K, N}, F8, dev);
         }
-        if (M > 0)                              // beside the activations' quantiser just enqueued
-            check(api.cinn_quant_block_beside(wf.data_ptr(), tag_of(wf.scalar_type()), N, K, wf.stride(0), wf.stride(1), r.w.data_ptr(),
-                                              r.w_t.defined() ? r.w_t.data_ptr() : nullptr, f32(r.w_scale), 0, div, stream()),
-                  "cinn_quant_blockwise");
-        else                                    // (no token: nobody reads the transposed copy)
-            check(api.cinn_quant_blockwise(wf.data_ptr(), tag_of(wf.scalar_type()), N, K, wf.stride(0), wf.stride(1), r.w.data_ptr(),
-                                           f32(r.w_scale), 128, 128, 0, div, stream()), "cinn_quant_blockwise");
+        // beside the activations' quantiser just enqueued
+        check(api.cinn_quant_block_beside(wf.data_ptr(), tag_of(wf.scalar_type()), N, K, wf.stride(0), wf.stride(1), r.w.data_ptr(),
+                                          r.w_t.defined() ? r.w_t.data_ptr() : nullptr, f32(r.w_scale), 0, div, stream()),
+              "cinn_quant_blockwise");
         ++launches;
     }
     r.out = gemm(xq, xs, r.w, 0, r.w_scale, r.w_scale.stride(1), r.w_scale.stride(0), M, N, K, at::kBFloat16, TAG_BF16);
@@ -145,7 +156,7 @@ std::tuple<std::vector<Tensor>, Tensor> linear_backward(const Tensor& grad_out, 
 
 // Without gradients nothing but the result outlives the call: one scratch buffer, one launch for both quantisers.
 static Tensor linear_inference(const Tensor& x, const Tensor& weight, bool round_scale, int div) {
-    require(x.is_cuda(), "Input must be on CUDA");
+    check_operands(x, weight, Tensor(), Tensor());
     c10::cuda::CUDAGuard guard(x.device());
     const int64_t K = x.size(-1), N = weight.size(0), nkb = up(K, 128);
     const Tensor xf = readable(x.dim() == 2 ? x : x.reshape({-1, K})), wf = readable(weight);

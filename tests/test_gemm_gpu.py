@@ -226,6 +226,30 @@ def test_fp8_linear_module(K):
     assert lin.weight.grad is not None and lin.weight.grad.dtype == torch.float32
 
 
+@pytest.mark.parametrize("grad", [True, False])
+def test_fp8_linear_refuses_operands_that_do_not_fit(K, grad):
+    """A weight left on the host, a weight of another width and an input without rows raise before anything is launched."""
+    with torch.device("cuda"):
+        lin = K.FP8Linear(256, 384)
+    x = torch.randn(32, 256, device="cuda", requires_grad=grad)
+    lin(x)
+    torch.cuda.synchronize()
+    launched = K.launch_count
+    with torch.set_grad_enabled(grad):
+        with pytest.raises(AssertionError, match="CUDA"):
+            K.FP8Linear(256, 384)(x)
+        for width in (128, 272):
+            with pytest.raises(AssertionError, match="wide"):
+                lin(torch.randn(32, width, device="cuda", requires_grad=grad))
+        with pytest.raises(RuntimeError, match="no rows"):
+            lin(x[:0])
+        w_q, w_s = K.quantize_fp8_blockwise(torch.randn(384, 128, device="cuda"))
+        launched += 1
+        with pytest.raises(AssertionError, match="quantised copy"):
+            K._host.linear(x, lin.weight, False, True, K._DIV_MODE, w_q, w_s, None)
+    assert K.launch_count == launched
+
+
 def test_weight_caches_and_updates_through_data(K):
     """The e4m3 copies follow every update that goes through the tensor (version counter); an update through
     ``.data`` leaves them stale until ``invalidate_weight_cache`` is called - the documented behaviour."""
