@@ -37,6 +37,9 @@ Linear linear_forward(const Tensor& x, const Tensor& weight, bool round_scale, b
     const int64_t K = x.size(-1), N = weight.size(0);
     Tensor xf = readable(x.dim() == 2 ? x : x.reshape({-1, K}));
     const int64_t M = xf.size(0), nkb = up(K, 128);
+    // A weight of another type is converted here, before the activations' quantiser is enqueued: the weight's quantiser runs
+    // beside that one and waits for nothing it reads.
+    const Tensor wf = w_q.defined() ? Tensor() : readable(weight);
     Linear r;
     // When the weight will want a gradient, the block re-quantisation of the saved activations comes out of the same
     // pass over x; it is written with the token axis contiguous where the token count allows, since the weight gradient
@@ -63,7 +66,6 @@ Linear linear_forward(const Tensor& x, const Tensor& weight, bool round_scale, b
         r.w_scale = w_s;
         r.w_t = w_qt;
     } else {
-        Tensor wf = readable(weight);
         r.w = empty({N, K}, F8, dev);
         r.w_scale = empty({up(N, 128), nkb}, at::kFloat, dev);
         // the input gradient multiplies by the weight with N as the reduction axis: the byte-transposed copy it reads

@@ -250,6 +250,29 @@ def test_fp8_linear_refuses_operands_that_do_not_fit(K, grad):
     assert K.launch_count == launched
 
 
+def test_fp8_linear_converts_its_weight_before_the_quantisers(K):
+    """A float64 weight in training: the same numbers as its fp32 copy.  The weight's quantiser starts beside the
+    activations', so the conversion it reads has to be enqueued ahead of both: seen in the order of the launches."""
+    from torch.profiler import ProfilerActivity, profile
+    with torch.device("cuda"):
+        lin = K.FP8Linear(512, 1024)
+    wide = K.FP8Linear(512, 1024)
+    wide.weight = torch.nn.Parameter(lin.weight.detach().double())
+    got = []
+    for layer in (lin, wide):
+        x = torch.randn(256, 512, device="cuda", generator=torch.Generator(device="cuda").manual_seed(3)).requires_grad_(True)
+        layer(x)
+        with profile(activities=[ProfilerActivity.CPU, ProfilerActivity.CUDA]) as prof:
+            y = layer(x)
+            torch.cuda.synchronize()
+        names = [e.name for e in sorted((e for e in prof.events() if e.device_type.name == "CUDA"), key=lambda e: e.time_range.start)]
+        got.append([y, *torch.autograd.grad(y, [x, layer.weight], torch.ones_like(y))])
+    for a, b in zip(*got):
+        assert torch.equal(a, b.to(a.dtype))
+    quantisers = [i for i, n in enumerate(names) if "quant_" in n]
+    assert len(quantisers) == 2 and quantisers[1] == quantisers[0] + 1, names          # nothing between the two
+
+
 def test_weight_caches_and_updates_through_data(K):
     """The e4m3 copies follow every update that goes through the tensor (version counter); an update through
     ``.data`` leaves them stale until ``invalidate_weight_cache`` is called - the documented behaviour."""
