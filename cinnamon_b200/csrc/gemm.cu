@@ -737,7 +737,8 @@ static int pair_mode() {
 }
 
 // The persistent GEMM kernels normally take every SM.  A caller that wants other kernels to run beside them
-// (the send/receive kernels of an all-to-all on another stream) can cap the number of SMs they occupy.
+// (the send/receive kernels of an all-to-all on another stream) can cap the number of SMs they occupy.  Read once per call:
+// another thread may change it meanwhile.
 static std::atomic<int> g_gemm_sm_limit{0};
 static inline int gemm_sms() {
     const int lim = g_gemm_sm_limit.load(std::memory_order_relaxed), all = sm_count();
@@ -806,8 +807,7 @@ struct DensePlan { bool pair; int splits; };
 // A K block of a tile costs about 0.45 us in either kernel (a pair of SMs does twice the rows in it), a tile about 3 us
 // around its K blocks.  Splitting adds a pass over the partial sums: about 3 us of launch and the bytes at the rate L2
 // returns them.  The plan with the smallest sum of these wins; measured figures stand at the callers' cases.
-static DensePlan dense_plan(int64_t M, int64_t N, int64_t K, int b_layout, int64_t workspace_bytes) {
-    const int sms = gemm_sms();
+static DensePlan dense_plan(int64_t M, int64_t N, int64_t K, int b_layout, int64_t workspace_bytes, int sms) {
     const int64_t KB = (K + BK - 1) / BK;
     auto waves = [](int64_t tiles, int64_t slots) { return (double)((tiles + slots - 1) / slots); };
     const int64_t pair_tiles = ((M + pair::PM - 1) / pair::PM) * ((N + pair::PN - 1) / pair::PN);
@@ -817,7 +817,8 @@ static DensePlan dense_plan(int64_t M, int64_t N, int64_t K, int b_layout, int64
     // the pair kernel wins with B K-major, the one-SM kernel with B MN-major
     DensePlan best{false, 1};
     double best_us = waves(tiles, sms) * (KB * block_us + tile_us);
-    if (pm == 2 ? pair_tiles >= sm_count() / 2 : (pm == 1 && b_layout == 0 && M > BM)) {       // (128 rows would leave a CTA idle)
+    // (128 rows would leave a CTA idle; a pair takes two SMs)
+    if (sms >= 2 && (pm == 2 ? pair_tiles >= sm_count() / 2 : (pm == 1 && b_layout == 0 && M > BM))) {
         const double us = waves(pair_tiles, sms / 2) * (KB * block_us + tile_us);
         if (us <= best_us * 1.02 || pm == 2) { best = {true, 1}; best_us = us; }
     }
@@ -835,7 +836,7 @@ constexpr int64_t MAX_SPLIT_BYTES = 64LL << 20;
 
 int64_t fp8_gemm_workspace_bytes(int64_t M, int64_t N, int64_t K, int b_layout) {
     if (M <= 0 || N <= 0 || K <= 0) return 0;
-    const DensePlan plan = dense_plan(M, N, K, b_layout, MAX_SPLIT_BYTES);
+    const DensePlan plan = dense_plan(M, N, K, b_layout, MAX_SPLIT_BYTES, gemm_sms());
     return plan.splits > 1 ? plan.splits * M * N * 4 : 0;
 }
 
@@ -854,7 +855,8 @@ int fp8_gemm(const void* A, int64_t lda, const float* sA, int64_t ld_sa, const v
     CINN_CHECK_ARG(b_layout == 0 || N % 16 == 0, "fp8_gemm: B stored (K, N) needs N %% 16 == 0");
     CINN_CHECK_ARG(lda >= K && ldb >= (b_layout == 0 ? K : N) && lda % 16 == 0 && ldb % 16 == 0,
                    "fp8_gemm: row pitches (%lld, %lld) must be multiples of 16 and no shorter than a row", (long long)lda, (long long)ldb);
-    const DensePlan plan = dense_plan(M, N, K, b_layout, workspace ? workspace_bytes : 0);
+    const int sms = gemm_sms();
+    const DensePlan plan = dense_plan(M, N, K, b_layout, workspace ? workspace_bytes : 0, sms);
     CUtensorMap ta, tb;
     int rc = make_map(&ta, A, (uint64_t)K, (uint64_t)M, (uint64_t)lda, BK, BM);
     if (rc) return rc;
@@ -868,12 +870,12 @@ int fp8_gemm(const void* A, int64_t lda, const float* sA, int64_t ld_sa, const v
     p.starts = nullptr; p.ends = nullptr; p.E = 1; p.b_rows_per_expert = 0; p.splits = 1;
     if (plan.pair) {
         const int64_t pair_tiles = ((M + pair::PM - 1) / pair::PM) * ((N + pair::PN - 1) / pair::PN);
-        const int clusters = (int)(pair_tiles < gemm_sms() / 2 ? pair_tiles : gemm_sms() / 2);
+        const int clusters = (int)(pair_tiles < sms / 2 ? pair_tiles : sms / 2);
         return b_layout == 0 ? launch_pair_out<false>(ta, tb, p, out_dtype, clusters, st)
                              : launch_pair_out<true>(ta, tb, p, out_dtype, clusters, st);
     }
     const int64_t tiles = ((M + BM - 1) / BM) * ((N + BN - 1) / BN) * plan.splits;
-    const int grid = (int)(tiles < gemm_sms() ? tiles : gemm_sms());
+    const int grid = (int)(tiles < sms ? tiles : sms);
     if (plan.splits > 1) {
         p.C = workspace; p.splits = plan.splits;
         rc = b_layout == 0 ? launch<false, false, CINN_F32, false, true>(ta, tb, ta, p, grid, st)
@@ -903,8 +905,9 @@ int fp8_grouped_gemm(const void* A, const float* sA, const void* W, const float*
     if (rc) return rc;
     // Pairs of SMs on 256-row tiles from 256 rows per expert on average (how the rows are really spread only the device
     // knows): below that the half-empty tiles cost more than the pair saves.
-    const bool use_pair = row_dst == nullptr && pair_mode() != 0 && T >= pair::PM * E &&
-                          (T + pair::PM - 1) / pair::PM * ((d_out + pair::PN - 1) / pair::PN) >= gemm_sms() / 2;
+    const int sms = gemm_sms();
+    const bool use_pair = row_dst == nullptr && pair_mode() != 0 && sms >= 2 && T >= pair::PM * E &&
+                          (T + pair::PM - 1) / pair::PM * ((d_out + pair::PN - 1) / pair::PN) >= sms / 2;
     rc = make_map(&tb, W, (uint64_t)d_in, (uint64_t)(E * d_out), (uint64_t)d_in, BK, use_pair ? 128 : BN);
     if (rc) return rc;
     const int64_t nkb = (d_in + 127) / 128, nnb = (d_out + 127) / 128;
@@ -917,14 +920,14 @@ int fp8_grouped_gemm(const void* A, const float* sA, const void* W, const float*
         // scattered rows: the table travels in the C slot of the parameters, tiles leave through staged 16-byte stores
         p.C = const_cast<long long*>(row_dst);
         p.tma_out = 0;
-        return out_dtype == CINN_BF16 ? launch<false, true, CINN_BF16, true>(ta, tb, ta, p, gemm_sms(), st)
-                                      : launch<false, true, CINN_F16, true>(ta, tb, ta, p, gemm_sms(), st);
+        return out_dtype == CINN_BF16 ? launch<false, true, CINN_BF16, true>(ta, tb, ta, p, sms, st)
+                                      : launch<false, true, CINN_F16, true>(ta, tb, ta, p, sms, st);
     }
     if (use_pair) {
         CUtensorMap tc;
         rc = make_out_map(&tc, ta, p, out_dtype, T, STORE_ROWS, true);
         if (rc) return rc;
-        const int clusters = gemm_sms() / 2;
+        const int clusters = sms / 2;
         switch (out_dtype) {
             case CINN_BF16: return launch_pair<false, CINN_BF16, false, true>(ta, tb, tc, p, clusters, st);
             case CINN_F16: return launch_pair<false, CINN_F16, false, true>(ta, tb, tc, p, clusters, st);
@@ -933,7 +936,7 @@ int fp8_grouped_gemm(const void* A, const float* sA, const void* W, const float*
             default: set_error("GEMM: unknown output dtype tag %d", out_dtype); return CINN_ERR_INVALID;
         }
     }
-    return launch_out<false, true>(ta, tb, p, out_dtype, gemm_sms(), st);
+    return launch_out<false, true>(ta, tb, p, out_dtype, sms, st);
 }
 
 // Input gradient of the grouped GEMM: dX[starts[e]:ends[e], :] = dY[starts[e]:ends[e], :] @ W[e]
@@ -993,7 +996,8 @@ int fp8_gemm_grouped_k(const void* A, const float* sA, const void* B, const floa
     rc = make_out_map(&tc, ta, p, out_dtype, E * M, STORE_ROWS, true);
     if (rc) return rc;
     const int64_t tiles = E * (M / pair::PM) * (N / pair::PN);
-    const int clusters = (int)(tiles < gemm_sms() / 2 ? tiles : gemm_sms() / 2);
+    const int sms = gemm_sms(), pairs = sms >= 2 ? sms / 2 : 1;              // (only the two-SM kernel does this: a cap of one SM counts as two)
+    const int clusters = (int)(tiles < pairs ? tiles : pairs);
     switch (out_dtype) {
         case CINN_BF16: return launch_pair<false, CINN_BF16, true>(ta, tb, tc, p, clusters, st);
         case CINN_F32: return launch_pair<false, CINN_F32, true>(ta, tb, tc, p, clusters, st);

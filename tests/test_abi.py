@@ -52,6 +52,20 @@ def test_bad_arguments_are_reported_not_crashed(built):
     assert L.cinn_fp8_gemm(None, None, 1, None, None, 1, 1, None, 0, 128, 128, 0, 0, None) == 0
 
 
+def test_gemm_plans_under_a_cap_of_one_sm(built):
+    """Planning divides tiles by SM pairs: with a cap below two SMs there are none (in a process of its own: this once ended it)."""
+    import subprocess
+    import sys
+    code = ("from cinnamon_b200 import kernels as K\n"
+            "for cap in (1, 2, 3):\n"
+            "    K.set_gemm_sm_limit(cap)\n"
+            "    for M, N, Kd in ((512, 512, 512), (64, 512, 7168), (4096, 4096, 4096)):\n"
+            "        for layout in (0, 1):\n"
+            "            assert K._L.cinn_fp8_gemm_workspace_bytes(M, N, Kd, layout) >= 0\n")
+    p = subprocess.run([sys.executable, "-c", code], cwd=ROOT, capture_output=True, text=True, timeout=300)
+    assert p.returncode == 0, (p.returncode, p.stderr)
+
+
 def test_cpu_tensors_assert_like_the_reference(built):
     import torch
     from cinnamon_b200 import kernels as K

@@ -367,6 +367,26 @@ def test_grouped_gemm_on_sm_pairs(K, case):
         assert rel_fro(got[covered].float(), ref[covered]) <= {torch.float32: 2e-5, torch.bfloat16: 2e-3, torch.float16: 3e-4}[dtype]
 
 
+def test_gemms_under_a_cap_of_one_sm(K):
+    """Dense (also more than 128 rows), grouped (enough rows for pairs) and grouped weight gradient: the same bits as uncapped."""
+    xq, xs, wq, ws = _operands(300, 320, 512, seed=1)
+    x, w, starts, ends = _grouped_case(2, 256, 512, [300, 500], seed=2)
+
+    def run():
+        dense = K.fp8_matmul_dsv3(_f8(xq), _f8(wq).t(), xs.cuda(), ws.cuda().t())
+        xg, wg = x.cuda().float().requires_grad_(True), w.cuda().float().requires_grad_(True)
+        y = K.moe_grouped_gemm(xg, wg, starts.cuda(), ends.cuda(), dtype=torch.bfloat16)
+        return dense, y, *torch.autograd.grad(y, [xg, wg], torch.ones_like(y))
+    want = run()
+    before = K.set_gemm_sm_limit(1)
+    try:
+        got = run()
+    finally:
+        K.set_gemm_sm_limit(before)
+    for a, b in zip(got, want):
+        assert torch.equal(a, b)
+
+
 @pytest.mark.parametrize("name", list(GROUPED))
 @pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
 def test_grouped_gemm_16bit(K, name, dtype):
