@@ -471,7 +471,9 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
             const float inv = sum > 0.0f ? 1.0f / sum : 0.0f;
             const float lse = sum > 0.0f ? mm + logf(sum) : 0.0f;
             s_lse[r] = lse;
-            bool bad = false;
+            // (no finite result can hide a sum that is not a number: with NaN scores only, the second warpgroup's maximum stays
+            // at -inf and its output is left out below)
+            bool bad = sum != sum;
             const int cols = min(64, a.Dv - half * 64);
             float* orow = a.out + ((int64_t)bh * a.L + t) * a.Dv + half * 64;
 #pragma unroll

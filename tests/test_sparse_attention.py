@@ -222,3 +222,30 @@ def test_tiles_fall_back_on_the_device(attention_path):
         idx[0, 100, ::2] = 6                              # now only the rows that nobody picked
         clean = (q, torch.nan_to_num(k), torch.nan_to_num(v, posinf=0.0), idx, 0.2)
         (ref_out, ref_attn, _), ref = SO.forward(*clean), SO.backward(*clean, go)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("key", [17, 200, 300])
+def test_a_nan_key_reaches_the_queries_that_picked_it(dtype, key):
+    """A picked key that holds NaN, in the first, second or third key tile, the only one picked there: tiles and gathers give
+    the same numbers and the same NaNs."""
+    from cinnamon_b200 import kernels as K
+    g = torch.Generator().manual_seed(key)
+    q, k, v = (torch.randn(1, 2, 400, 64, generator=g).to(dtype) for _ in range(3))
+    idx = torch.randint(0, 100, (1, 400, 24), generator=g)
+    idx[idx == 17] = 18
+    idx[0, 301:340, 5] = key
+    k[0, 0, key, 3] = float("nan")
+    got = []
+    for mode in (1, 0):
+        before = K._L.cinn_set_sparse_attn_dense(mode)
+        try:
+            out, attn = K.sparse_attention(q.cuda(), k.cuda(), v.cuda(), idx.cuda())
+            got.append((out.cpu(), attn.cpu()))
+        finally:
+            K._L.cinn_set_sparse_attn_dense(before)
+    assert torch.isnan(got[0][0][0, 0, 301:340]).all() and not torch.isnan(got[0][0][0, 1]).any()
+    for a, b in zip(*got):
+        torch.testing.assert_close(a, b, rtol=1e-5 if dtype == torch.float32 else 8e-3, atol=1e-6, equal_nan=True)
+    assert K.device_status() == 0
