@@ -99,7 +99,7 @@ void bind_attention(pybind11::module_& m) {
         return backward(g, q, k, v, idx, out32, lse, scale, like.scalar_type());
     });
     m.def("attention", [](const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& idx, double scale) {
-        if (at::GradMode::is_enabled() && (q.requires_grad() || k.requires_grad() || v.requires_grad())) {
+        if (takes_node(q, k, v)) {
             auto r = AttentionNode::apply(q, k, v, idx, scale);
             return std::make_tuple(r[0], r[1]);
         }

@@ -86,6 +86,12 @@ inline Tensor readable(const Tensor& t) { return tag_of(t.scalar_type()) < 0 ? t
 inline Tensor empty(at::IntArrayRef size, at::ScalarType type, const at::Device& dev) {
     return at::detail::empty_cuda(size, type, dev, std::nullopt);
 }
+// Whether a call goes through its autograd node: a gradient will be recorded, or an input carries a forward-mode tangent, which
+// the node refuses (computed without it, the tangent would be dropped in silence).
+template <typename... T>
+bool takes_node(const T&... t) {
+    return (at::GradMode::is_enabled() && (t.requires_grad() || ...)) || (t._fw_grad(/*level=*/0).defined() || ...);
+}
 inline int64_t up(int64_t a, int64_t b) { return (a + b - 1) / b; }
 inline void* stream() { return at::cuda::getCurrentCUDAStream().stream(); }
 inline float* f32(const Tensor& t);

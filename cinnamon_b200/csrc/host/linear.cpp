@@ -234,7 +234,7 @@ void bind_linear(pybind11::module_& m) {
     m.def("linear", [](const Tensor& x, const Tensor& w, bool round_scale, bool kmajor, int div, const OptT& wq, const OptT& ws,
                        const OptT& wqt) {
         const CachedWeight cached{or_none(wq), or_none(ws), or_none(wqt)};
-        if (at::GradMode::is_enabled() && (x.requires_grad() || w.requires_grad()))
+        if (takes_node(x, w))
             return LinearNode::apply(x, w, round_scale, kmajor, (int64_t)div, &cached);
         if (!cached.q.defined()) return linear_inference(x, w, round_scale, div);
         return linear_forward(x, w, round_scale, false, false, kmajor, div, cached.q, cached.s, cached.q_t).out;

@@ -218,3 +218,23 @@ def test_native_routed_experts_compute_the_module_paths_silu(K):
         block.router.register_forward_hook(lambda *args: None)
         modules, _ = block(x)
     assert torch.equal(native, modules)
+
+
+@pytest.mark.parametrize("grad", [True, False])
+def test_forward_mode_tangents_are_refused_not_dropped(K, grad):
+    """Neither the FP8 linear nor the attention has a forward-mode derivative: a dual input raises, with frozen weights and
+    without a gradient to record too, where the calls take a path without an autograd node."""
+    import torch.autograd.forward_ad as fw
+    from cinnamon_b200 import layers
+    with torch.device("cuda"):
+        lin = K.FP8Linear(256, 384).requires_grad_(False)
+        swiglu = K.convert_to_fp8(torch.nn.Sequential(layers.SwiGLU(256, 512))).requires_grad_(False)
+        x, tangent = torch.randn(2, 32, 256).unbind(0)
+        q, k, v = torch.randn(3, 1, 2, 32, 64).unbind(0)
+        idx = torch.zeros(1, 32, 4, dtype=torch.long)
+    with torch.set_grad_enabled(grad), fw.dual_level():
+        for call in (lambda: lin(fw.make_dual(x, tangent)), lambda: swiglu(fw.make_dual(x, tangent)),
+                     lambda: K.sparse_attention(fw.make_dual(q, torch.ones_like(q)), k, v, idx),
+                     lambda: K.sparse_attention(q, k, fw.make_dual(v, torch.ones_like(v)), idx)):
+            with pytest.raises(RuntimeError, match="jvp"):
+                call()
