@@ -104,6 +104,7 @@ struct Linear {                                 // what an FP8 linear's forward 
 };
 Linear linear_forward(const Tensor& x, const Tensor& weight, bool round_scale, bool need_dgrad, bool need_wgrad, bool kmajor, int div,
                       const Tensor& w_q, const Tensor& w_s, const Tensor& w_qt);
+Tensor linear_inference(const Tensor& x, const Tensor& weight, bool round_scale, int div);
 // (input gradients, weight gradient).  `parts` > 1: the weight is that many layers of equally many rows (a multiple of 128)
 // stacked, and every layer's input gradient is returned by itself.
 std::tuple<std::vector<Tensor>, Tensor> linear_backward(const Tensor& grad_out, Tensor x, Tensor x_scale, const Tensor& w,

@@ -157,7 +157,7 @@ std::tuple<std::vector<Tensor>, Tensor> linear_backward(const Tensor& grad_out, 
 
 
 // Without gradients nothing but the result outlives the call: one scratch buffer, one launch for both quantisers.
-static Tensor linear_inference(const Tensor& x, const Tensor& weight, bool round_scale, int div) {
+Tensor linear_inference(const Tensor& x, const Tensor& weight, bool round_scale, int div) {
     check_operands(x, weight, Tensor(), Tensor());
     c10::cuda::CUDAGuard guard(x.device());
     const int64_t K = x.size(-1), N = weight.size(0), nkb = up(K, 128);

@@ -238,3 +238,19 @@ def test_forward_mode_tangents_are_refused_not_dropped(K, grad):
                      lambda: K.sparse_attention(q, k, fw.make_dual(v, torch.ones_like(v)), idx)):
             with pytest.raises(RuntimeError, match="jvp"):
                 call()
+
+
+def test_swiglu_without_gradients_keeps_nothing_for_a_backward(K):
+    """Evaluation: one launch quantises a layer's input and weight (no block copies, no transposed weight); same numbers."""
+    from cinnamon_b200 import layers
+    with torch.device("cuda"):
+        block = K.convert_to_fp8(layers.SwiGLU(256, 512))
+    x = torch.randn(3, 40, 256, device="cuda")
+    want = block(x)
+    n = K.launch_count
+    with torch.no_grad():
+        got = block(x)
+    assert K.launch_count - n == 5                # quantise, multiply; silu; quantise, multiply
+    assert torch.equal(got, want) and not got.requires_grad
+    block.requires_grad_(False)
+    assert torch.equal(block(x), want)
