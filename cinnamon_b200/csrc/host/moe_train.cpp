@@ -41,6 +41,7 @@ struct SwiGLUNode : public torch::autograd::Function<SwiGLUNode> {
         const Linear a = linear_forward(x, at::cat({w1, w2}), o->round12, gx, g12, o->kmajor, o->div, Tensor(), Tensor(), Tensor());
         const Tensor h12 = a.out.view({-1, a.out.size(-1)});
         const Linear b = linear_forward(swiglu_rounded(h12), w3, o->round3, any, g3, o->kmajor, o->div, Tensor(), Tensor(), Tensor());
+        ctx->set_materialize_grads(false);
         if (any || g3) {
             ctx->save_for_backward({a.x, a.x_scale, a.w, a.w_scale, a.w_t, h12, b.x, b.x_scale, b.w, b.w_scale, b.w_t});
             ctx->saved_data["x_shape"] = x.sizes().vec();
@@ -62,6 +63,8 @@ struct SwiGLUNode : public torch::autograd::Function<SwiGLUNode> {
         const bool gx = ctx->needs_input_grad(0), g12 = ctx->needs_input_grad(2) || ctx->needs_input_grad(3), g3 = ctx->needs_input_grad(4);
         std::vector<Tensor> dx(2), dh(1);
         Tensor d1, d2, d3;
+        // (the block's output is not part of what is differentiated, its balance loss alone is: no gradient, not a zero one)
+        if (!grads[0].defined()) return {Tensor(), Tensor(), Tensor(), Tensor(), Tensor(), Tensor()};
         as_python_error([&] {
             auto back = [&](int64_t f, const Tensor& g, int at, at::IntArrayRef shape, bool want_x, bool want_w, at::ScalarType type,
                             int parts) {

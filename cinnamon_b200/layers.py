@@ -134,12 +134,17 @@ class MoE(nn.Module):
                              "by the first call")
         return self._peer
 
-    def _native_ready(self, flat, shared_out):
+    def _native_ready(self, x, flat, shared_out):
         """Whether the routed part can run as one native autograd node (``_forward_native``): every expert on this GPU, plain
-        modules without hooks, e4m3 experts of widths the fused weight gradient takes."""
+        modules without hooks, e4m3 experts of widths the fused weight gradient takes.  The node has the balance loss as a
+        second output: differentiated alone it must leave the shared experts without a gradient, which theirs do as native
+        nodes."""
         from . import kernels as K
         ex, r = self.routed_experts, self.router
         plain = (type(ex) is GroupedExperts and type(r) is nn.Linear and r.bias is None and not K.has_hooks(ex) and not K.has_hooks(r))
+        if self.balance_alpha > 0 and shared_out.requires_grad:
+            plain = plain and all(type(e) is SwiGLU and not K.has_hooks(e) and K.swiglu_block_ready(x, e.w1, e.w2, e.w3)
+                                  for e in self.shared_experts)
         return (plain and not self.sharded and flat.shape[0] > 0 and not torch.compiler.is_compiling() and K.gemm_events is None
                 and K._MOE_GROUPED_PRECISION == "fp8" and ex.d_model % 256 == 0 and ex.hidden_dim % 256 == 0
                 and all(w.dtype in (torch.float32, torch.bfloat16) and w.is_contiguous() for w in (ex.w12, ex.w3))
@@ -162,7 +167,7 @@ class MoE(nn.Module):
         batch, seq, d = x.shape
         shared_out = self.shared_experts[0](x) if len(self.shared_experts) == 1 else sum(e(x) for e in self.shared_experts)
         flat = x.reshape(-1, d)
-        if flat.is_cuda and self._native_ready(flat, shared_out):
+        if flat.is_cuda and self._native_ready(x, flat, shared_out):
             return self._forward_native(flat, shared_out, batch, seq)
         logits = self.router(flat)
         scores = torch.sigmoid(logits.float())

@@ -254,3 +254,20 @@ def test_swiglu_without_gradients_keeps_nothing_for_a_backward(K):
     assert torch.equal(got, want) and not got.requires_grad
     block.requires_grad_(False)
     assert torch.equal(block(x), want)
+
+
+@pytest.mark.parametrize("hooked", [False, True])
+def test_balance_loss_alone_leaves_the_experts_without_gradients(K, hooked):
+    """Differentiating only the balance loss: the router and x get a gradient, no expert gets one (None, not zeros, which an
+    optimiser with weight decay or momentum would act on)."""
+    from cinnamon_b200 import layers
+    with torch.device("cuda"):
+        block = K.convert_to_fp8(layers.MoE(8, 1, 2, 256, 1024, 2, 0.01, 0.01))
+    if hooked:
+        block.shared_experts[0].w1.register_forward_hook(lambda *args: None)
+    x = torch.randn(2, 40, 256, device="cuda", requires_grad=True)
+    with torch.autocast("cuda", dtype=torch.bfloat16):
+        _, balance = block(x)
+    balance.backward()
+    assert block.router.weight.grad is not None and x.grad is not None
+    assert [n for n, p in block.named_parameters() if p.grad is not None] == ["router.weight"]
