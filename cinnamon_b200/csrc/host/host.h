@@ -130,6 +130,8 @@ struct Routes {                                 // moe_route's outputs, in three
     float* gates() const { return static_cast<float*>(floats.data_ptr()) + pairs; }
 };
 Routes route(const Tensor& logits, const Tensor& bias, int64_t top_k);
+// refuses operands on other devices or of other widths, before anything is launched
+void check_layer(const Tensor& x, const Tensor& router, const Tensor& bias, const Quantised& w12, const Quantised& w3);
 Quantised spread(const Quantised& x, const Routes& r, int64_t top_k);
 inline float* f32(const Tensor& t) { return static_cast<float*>(t.data_ptr()); }
 

@@ -33,6 +33,16 @@ Tensor grouped(const Quantised& x, const Quantised& w, const Tensor& starts, con
     return out;
 }
 
+void check_layer(const Tensor& x, const Tensor& router, const Tensor& bias, const Quantised& w12, const Quantised& w3) {
+    const auto dev = x.device();
+    require(x.is_cuda() && router.is_cuda() && bias.is_cuda(), "Inputs must be on CUDA");
+    require(router.device() == dev && bias.device() == dev && w12.q.device() == dev && w3.q.device() == dev && w12.s.device() == dev &&
+                w3.s.device() == dev, "MoE: input, router and experts must be on the same device");
+    const int64_t E = router.size(0), d = x.size(1);
+    require(router.size(1) == d && bias.numel() == E && w12.q.size(0) == E && w3.q.size(0) == E && w12.q.size(2) == d &&
+                w3.q.size(1) == d && w12.q.size(1) == 2 * w3.q.size(2), "MoE: the widths of input, router and experts do not fit together");
+}
+
 Routes route(const Tensor& logits_in, const Tensor& bias, int64_t top_k) {
     const Tensor logits = readable(logits_in).contiguous(), b = bias.to(at::kFloat).contiguous();
     const int64_t T = logits.size(0), E = logits.size(1);
@@ -69,7 +79,9 @@ namespace {
 // them.  Returns (T, d) fp32.
 Tensor forward(const Tensor& x, const Tensor& router, const Tensor& bias, int64_t top_k, const Quantised& w12, const Quantised& w3,
                const Quantised& sw12, const Quantised& sw3, bool shared_round, int div) {
-    require(x.is_cuda() && router.is_cuda() && bias.is_cuda(), "Inputs must be on CUDA");
+    check_layer(x, router, bias, w12, w3);
+    require(!sw12.q.defined() || (sw12.q.device() == x.device() && sw12.q.size(1) == x.size(1) && sw3.q.size(0) == x.size(1) &&
+                                  sw12.q.size(0) == 2 * sw3.q.size(1)), "MoE: the shared expert does not fit the input");
     c10::cuda::CUDAGuard guard(x.device());
     at::NoGradGuard no_grad;
     const at::Device dev = x.device();

@@ -310,6 +310,8 @@ void bind_moe_train(pybind11::module_& m) {
     m.def("moe_block", [](const Tensor& x, const Tensor& router, const Tensor& w12, const Tensor& w3, const Tensor& addend,
                           const Tensor& bias, const Tensor& w12_q, const Tensor& w12_s, const Tensor& w3_q, const Tensor& w3_s, int64_t top_k,
                           int64_t batch, double alpha, bool cast_router, int div) {
+        check_layer(x, router, bias, {w12_q, w12_s}, {w3_q, w3_s});
+        require(addend.device() == x.device() && addend.sizes() == x.sizes(), "MoE: the shared experts' output does not fit the input");
         BlockOptions o{bias, {w12_q, w12_s}, {w3_q, w3_s}, top_k, batch, alpha,
                        cast_router ? at::autocast::get_autocast_dtype(at::kCUDA) : x.scalar_type(), div, Tensor()};
         auto r = BlockNode::apply(x, router, w12, w3, addend, &o);

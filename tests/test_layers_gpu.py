@@ -271,3 +271,28 @@ def test_balance_loss_alone_leaves_the_experts_without_gradients(K, hooked):
     balance.backward()
     assert block.router.weight.grad is not None and x.grad is not None
     assert [n for n, p in block.named_parameters() if p.grad is not None] == ["router.weight"]
+
+
+def test_moe_layers_refuse_a_bias_left_on_the_host(K):
+    """The routing bias on the CPU and an input of another width raise before anything is launched."""
+    from cinnamon_b200 import layers, moe
+    with torch.device("cuda"):
+        block = K.convert_to_fp8(layers.MoE(8, 1, 2, 256, 1024, 2, 0.01, 0.01))
+        w = lambda *s: torch.randn(*s).bfloat16()                                             # noqa: E731
+        serve = moe.ExpertParallelMoE(w(8, 256).float(), torch.zeros(8), w(8, 256, 256), w(8, 256, 128), 2,
+                                      shared=moe.FP8SwiGLU(w(128, 256), w(128, 256), w(256, 128)))
+        x = torch.randn(1, 40, 256)
+        wide = torch.randn(40, 272).bfloat16()
+    with torch.no_grad(), torch.autocast("cuda", dtype=torch.bfloat16):
+        block(x), serve(x[0].bfloat16())
+        torch.cuda.synchronize()
+        with pytest.raises(AssertionError, match="widths"):
+            serve(wide)
+        block.expert_bias = block.expert_bias.cpu()
+        serve.expert_bias = serve.expert_bias.cpu()
+        with pytest.raises(AssertionError, match="CUDA"):
+            block(x)
+        n = K.launch_count
+        with pytest.raises(AssertionError, match="CUDA"):
+            serve(x[0].bfloat16())
+        assert K.launch_count == n
