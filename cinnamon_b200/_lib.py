@@ -86,6 +86,7 @@ SIGNATURES = {
     "cinn_swiglu": [_vp, _vp, _i32, _i64, _i64, _vp],
     "cinn_swiglu_backward": [_vp, _vp, _vp, _i32, _i64, _i64, _vp],
     "cinn_moe_combine_add": [_vp, _i32, _vp, _vp, _vp, _i32, _vp, _i64, _i64, _i32, _i64, _vp],
+    "cinn_moe_sum_add": [_vp, _i32, _vp, _vp, _i32, _vp, _i64, _i64, _i32, _i64, _vp],
     "cinn_device_status": [ctypes.POINTER(ctypes.c_int), _i32],
     "cinn_fp8_grouped_gemm": [_vp, _vp, _vp, _vp, _vp, _vp, _i64, _i64, _i64, _i64, _vp, _i32, _vp],
 }

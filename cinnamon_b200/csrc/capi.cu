@@ -258,13 +258,22 @@ int cinn_fp8_grouped_gemm_dgrad(const void* dY, const float* sdY, const void* W,
 
 int cinn_moe_combine(const void* rows, int dtype, const int64_t* pos, const float* gates, void* y, int64_t n_tokens,
                      int64_t n_rows, int top_k, int64_t d, void* stream) {
+    using namespace cinn;
+    CINN_CHECK_ARG(gates || n_tokens <= 0 || d <= 0, "moe_combine: null pointer");
     return cinn::moe_combine(rows, dtype, pos, gates, nullptr, 0, y, n_tokens, n_rows, top_k, d, (cudaStream_t)stream);
 }
 
 int cinn_moe_combine_add(const void* rows, int dtype, const int64_t* pos, const float* gates, const void* addend,
                          int addend_dtype, void* y, int64_t n_tokens, int64_t n_rows, int top_k, int64_t d, void* stream) {
+    using namespace cinn;
+    CINN_CHECK_ARG(gates || n_tokens <= 0 || d <= 0, "moe_combine: null pointer");
     return cinn::moe_combine(rows, dtype, pos, gates, addend, addend_dtype, y, n_tokens, n_rows, top_k, d,
                              (cudaStream_t)stream);
+}
+
+int cinn_moe_sum_add(const void* rows, int dtype, const int64_t* pos, const void* addend, int addend_dtype, void* y, int64_t n_tokens,
+                     int64_t n_rows, int top_k, int64_t d, void* stream) {
+    return cinn::moe_combine(rows, dtype, pos, nullptr, addend, addend_dtype, y, n_tokens, n_rows, top_k, d, (cudaStream_t)stream);
 }
 
 int cinn_gather_rows(const void* q, const float* scales, const int64_t* idx, void* out_q, float* out_scales, int64_t n_out,

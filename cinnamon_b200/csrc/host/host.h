@@ -27,7 +27,7 @@ using at::Tensor;
     X(cinn_requant_row_to_block) X(cinn_fp8_gemm_ws) X(cinn_fp8_gemm_pitched) X(cinn_fp8_gemm_workspace_bytes) \
     X(cinn_sparse_attn_workspace_bytes) X(cinn_sparse_attn_fwd_ws) X(cinn_sparse_attn_bwd) X(cinn_sparse_attn_bwd_ws)                  \
     X(cinn_moe_route_workspace_ints) X(cinn_moe_route_ranges) X(cinn_spread_rows) X(cinn_fp8_grouped_gemm)                \
-    X(cinn_swiglu_quant_rowwise) X(cinn_moe_combine) X(cinn_moe_combine_add)                \
+    X(cinn_swiglu_quant_rowwise) X(cinn_moe_combine) X(cinn_moe_combine_add) X(cinn_moe_sum_add)                \
     X(cinn_swiglu_rounded) X(cinn_swiglu_rounded_backward) X(cinn_moe_balance_workspace_bytes) X(cinn_moe_balance_loss)     \
     X(cinn_moe_gates_backward) X(cinn_moe_update_bias) X(cinn_moe_combine_backward) X(cinn_swiglu_backward)                 \
     X(cinn_fp8_grouped_wgrad_fused_scratch_bytes) X(cinn_fp8_grouped_wgrad_fused) X(cinn_fp8_grouped_gemm_dgrad) X(cinn_zero_rows_outside)

@@ -236,8 +236,8 @@ struct BlockNode : public torch::autograd::Function<BlockNode> {
             }
             if (want_x && d_rows.defined()) {
                 dx = empty({T, d}, at::kFloat, dev);
-                check(api.cinn_moe_combine_add(d_rows.data_ptr(), tag_of(d_rows.scalar_type()), r.pos(), nullptr, dxr.data_ptr(),
-                                               tag_of(dxr.scalar_type()), f32(dx), T, r.pairs, (int)k, d, stream()), "cinn_moe_combine_add");
+                check(api.cinn_moe_sum_add(d_rows.data_ptr(), tag_of(d_rows.scalar_type()), r.pos(), dxr.data_ptr(), tag_of(dxr.scalar_type()),
+                                           f32(dx), T, r.pairs, (int)k, d, stream()), "cinn_moe_sum_add");
                 ++launches;
             } else {
                 dx = dxr;

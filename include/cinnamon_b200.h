@@ -241,6 +241,11 @@ int cinn_moe_combine(const void* rows, int dtype, const int64_t* pos, const floa
 int cinn_moe_combine_add(const void* rows, int dtype, const int64_t* pos, const float* gates, const void* addend,
                          int addend_dtype, void* y, int64_t n_tokens, int64_t n_rows, int top_k, int64_t d, void* stream);
 
+/* The plain sum of a token's rows, y[t, :] = addend[t, :] + sum_j rows[pos[t, j], :] (addend as above): how the gradients of a
+ * token's rows come home. */
+int cinn_moe_sum_add(const void* rows, int dtype, const int64_t* pos, const void* addend, int addend_dtype, void* y, int64_t n_tokens,
+                     int64_t n_rows, int top_k, int64_t d, void* stream);
+
 /* Zero the rows of buf (n_rows x row_bytes) that no range [starts[r], ends[r]) covers (device-side int64 ranges,
  * clamped to the buffer).  The backward of the grouped GEMM uses it so that rows of no expert get a zero input
  * gradient without a fill of the whole buffer.  No reference counterpart (the reference's grouped GEMM,

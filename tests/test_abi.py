@@ -47,6 +47,10 @@ def test_bad_arguments_are_reported_not_crashed(built):
     assert st == _lib.ERR_INVALID and "multiple of 16" in _lib.last_error()
     with pytest.raises(AssertionError):
         _lib.check(st, "cinn_fp8_gemm")
+    # a combine without gates is refused, with and without an addend
+    p = ctypes.c_void_p(256)
+    assert L.cinn_moe_combine(p, 0, p, None, p, 4, 8, 2, 64, None) == _lib.ERR_INVALID
+    assert L.cinn_moe_combine_add(p, 0, p, None, p, 0, p, 4, 8, 2, 64, None) == _lib.ERR_INVALID and "null" in _lib.last_error()
     # empty problems are a successful no-op
     assert L.cinn_quant_rowwise(None, 0, 0, 128, 128, 1, None, None, 128, 0, 0, None) == 0
     assert L.cinn_fp8_gemm(None, None, 1, None, None, 1, 1, None, 0, 128, 128, 0, 0, None) == 0
