@@ -547,7 +547,10 @@ class FP8Linear(torch.nn.Module):
 
 
 def has_hooks(module: torch.nn.Module) -> bool:
-    return bool(module._forward_hooks or module._forward_pre_hooks or module._backward_hooks or module._backward_pre_hooks)
+    """Whether anything but the class's ``forward`` would run in a call of ``module``: hooks of its own, hooks for every module
+    (a profiler's or an offloader's), or a ``forward`` replaced on the instance."""
+    return bool(module._forward_hooks or module._forward_pre_hooks or module._backward_hooks or module._backward_pre_hooks
+                or "forward" in module.__dict__ or torch.nn.modules.module._has_any_global_hook())
 
 
 def swiglu_block_ready(x, w1, w2, w3) -> bool:

@@ -726,8 +726,8 @@ class ExpertParallelMoE(torch.nn.Module):
         flat = x.reshape(-1, x.shape[-1])
         router = self._router_as(flat.dtype)
         if (flat.is_cuda and self.trace is None and self.K.gemm_events is None and flat.shape[1] % 16 == 0
-                and flat.dtype in self.K._DTYPE_TAG and isinstance(self.shared, (FP8SwiGLU, type(None)))
-                and isinstance(self.experts, FP8Experts) and (not dist.is_initialized() or dist.get_world_size(self.group) == 1)):
+                and flat.dtype in self.K._DTYPE_TAG and type(self.shared) in (FP8SwiGLU, type(None))
+                and type(self.experts) is FP8Experts and (not dist.is_initialized() or dist.get_world_size(self.group) == 1)):
             # one GPU: the sequence below as one native call (csrc/host/moe.cpp)
             e, sh = self.experts, self.shared
             shared = (None,) * 4 if sh is None else (sh.w12_q, sh.w12_s, sh.w3_q, sh.w3_s)

@@ -106,3 +106,19 @@ def test_sharded_moe_block_trains_like_the_unsharded_one(tmp_path):
                           timeout=300, env=dict(os.environ, OMP_NUM_THREADS="2"))
     for rank in range(2):
         assert (tmp_path / f"ok_{rank}").read_text() == "1", f"rank {rank}: sharded and unsharded layers disagree"
+
+
+def test_what_counts_as_a_plain_module():
+    """The native block skips the calls of its inner modules only where nothing listens to them."""
+    from cinnamon_b200 import kernels as K
+    from torch.nn.modules.module import register_module_forward_hook, register_module_forward_pre_hook
+    lin = torch.nn.Linear(4, 4)
+    assert not K.has_hooks(lin)
+    for add in (lin.register_forward_hook, lin.register_forward_pre_hook, lin.register_full_backward_hook,
+                register_module_forward_hook, register_module_forward_pre_hook):
+        handle = add(lambda *args: None)
+        assert K.has_hooks(lin)
+        handle.remove()
+        assert not K.has_hooks(lin)
+    lin.forward = lambda x: x                                                  # as an offloading wrapper does
+    assert K.has_hooks(lin)

@@ -163,6 +163,32 @@ def test_native_layer_matches_its_parts(K, T, d, shared, rs):
     assert layer(x[:0]).shape == (0, d)
 
 
+def test_subclassed_experts_are_called(K):
+    """Experts or a shared expert of a class of their own are called, not replaced by the native layer's sequence."""
+    from cinnamon_b200 import moe
+    calls = []
+
+    class Experts(moe.FP8Experts):
+        def __call__(self, *args, **kw):
+            calls.append("experts")
+            return super().__call__(*args, **kw)
+
+    class Shared(moe.FP8SwiGLU):
+        def __call__(self, *args, **kw):
+            calls.append("shared")
+            return super().__call__(*args, **kw)
+    g = torch.Generator().manual_seed(1)
+    w = lambda *s: (torch.randn(*s, generator=g) * 0.05).bfloat16().cuda()                       # noqa: E731
+    w12, w3, sh = w(8, 256, 256), w(8, 256, 128), (w(128, 256), w(128, 256), w(256, 128))
+    layer = moe.ExpertParallelMoE(w(8, 256).float(), torch.zeros(8, device="cuda"), w12, w3, 2, shared=moe.FP8SwiGLU(*sh))
+    x = w(40, 256)
+    want = layer(x)
+    layer.experts = Experts(w12, w3)
+    assert torch.equal(layer(x), want) and calls == ["experts"]
+    layer.shared = Shared(*sh)
+    assert torch.equal(layer(x), want) and sorted(calls[1:]) == ["experts", "shared"]
+
+
 def test_gather_quantized_rows(K):
     g = torch.Generator().manual_seed(5)
     q = torch.randint(0, 256, (300, 512), generator=g, dtype=torch.uint8).cuda().view(torch.float8_e4m3fn)
