@@ -38,6 +38,7 @@ struct Api {
 #undef CINN_DECL
 };
 extern Api api;
+extern PyObject* library_error;                // _lib.LibraryError
 extern std::atomic<int64_t> launches;          // kernels of the library launched from here
 
 // A status of the library as an exception: `invalid` becomes Python's AssertionError, the rest LibraryError.
@@ -64,7 +65,7 @@ void as_python_error(F&& body) {
         body();
     } catch (const CinnError& e) {
         pybind11::gil_scoped_acquire gil;
-        PyErr_SetString(e.invalid ? PyExc_AssertionError : PyExc_RuntimeError, e.what());
+        PyErr_SetString(e.invalid ? PyExc_AssertionError : library_error, e.what());
         python_error err;
         err.persist();
         throw err;

@@ -3,6 +3,7 @@
 
 namespace cinnhost {
 Api api;
+PyObject* library_error = PyExc_RuntimeError;
 std::atomic<int64_t> launches{0};
 void bind_linear(pybind11::module_& m);
 void bind_attention(pybind11::module_& m);
@@ -12,9 +13,8 @@ void bind_moe_train(pybind11::module_& m);
 
 PYBIND11_MODULE(_host, m) {
     using namespace cinnhost;
-    static pybind11::object library_error;
     m.def("bind", [](const std::unordered_map<std::string, uintptr_t>& addr, pybind11::object error_type) {
-        library_error = std::move(error_type);
+        library_error = error_type.release().ptr();        // (bound once, kept for the life of the process)
 #define CINN_BIND(name) api.name = reinterpret_cast<decltype(api.name)>(addr.at(#name));
         CINN_HOST_API(CINN_BIND)
 #undef CINN_BIND
@@ -31,7 +31,7 @@ PYBIND11_MODULE(_host, m) {
         try {
             if (p) std::rethrow_exception(p);
         } catch (const CinnError& e) {
-            PyErr_SetString(e.invalid ? PyExc_AssertionError : library_error.ptr(), e.what());
+            PyErr_SetString(e.invalid ? PyExc_AssertionError : library_error, e.what());
         }
     });
     bind_linear(m);

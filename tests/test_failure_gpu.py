@@ -103,3 +103,24 @@ def test_return_and_row_table_with_destinations_out_of_range(K):
     expect = [home.data_ptr() + i * d * 2 for i in range(cap)] + [0] * (n - cap)
     assert table.tolist() == expect
     _gemm_still_works(K)
+
+
+def test_a_failing_call_raises_the_librarys_exception_in_both_directions(K):
+    """An error status of the library (from a stand-in for one of its functions) is a LibraryError, in the forward and in a
+    native backward, which runs on autograd's own thread."""
+    import ctypes
+    from cinnamon_b200 import _lib
+    lin = K.FP8Linear(256, 384).cuda()
+    x = torch.randn(32, 256, device="cuda", requires_grad=True)
+    address = {n: ctypes.cast(getattr(_lib.lib, n), ctypes.c_void_p).value for n in _lib.host.symbols()}
+    stand_in = ctypes.CFUNCTYPE(ctypes.c_int)(lambda: _lib.ERR_CUDA)
+    try:
+        for name in ("cinn_quant_rowwise_with_block_t", "cinn_quant_rowwise_dual"):
+            y = lin(x)
+            _lib.host.bind({**address, name: ctypes.cast(stand_in, ctypes.c_void_p).value}, _lib.LibraryError)
+            with pytest.raises(_lib.LibraryError, match="status 2"):
+                y.sum().backward() if "dual" in name else lin(x)
+            _lib.host.bind(address, _lib.LibraryError)
+    finally:
+        _lib.host.bind(address, _lib.LibraryError)
+    lin(x).sum().backward()
