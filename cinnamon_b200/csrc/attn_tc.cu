@@ -1,7 +1,8 @@
 // Sparse attention on the tensor cores: see attn_tc.cuh for what it trades against the gather kernels.
 //
 // Scratch (from the caller, one block per call): what the queries picked (Picks), the bf16 parts of the inputs and one
-// flag word.  Everything is rebuilt on every call.
+// flag word.  Everything is rebuilt on every call.  It is about as large as the tensors (32 x 8 x 1024 queries of 192 / 64 in
+// fp32, 128 picks: 0.70 GB forward, 1.07 GB backward); a call that would need more than MAX_SCRATCH_BYTES takes the gathers.
 //
 // What a dense tile cannot express falls back on the device, without the host knowing: a key picked more than 255 times
 // by one query, or results that are not finite (a NaN in a row nobody picked must not reach anyone, and 0 * NaN on a
@@ -1217,6 +1218,10 @@ static bool supported(int64_t B, int64_t H, int64_t L, int64_t K, int64_t Dqk, i
     return B * H * L > 0 && K >= 1 && K <= MAX_SLOTS && Dqk <= 192 && Dv <= 128 && L <= 12000 && B * H <= 65535 && B * H * L < (1LL << 31) / 4;
 }
 
+// a tenth of the memory: what a call may add to its tensors for the sake of speed
+constexpr int64_t MAX_SCRATCH_BYTES = 16LL << 30;
+static int64_t scratch_bytes(const Plan& p, bool backward) { return p.bytes <= MAX_SCRATCH_BYTES && dense_pays(p, backward) ? p.bytes : 0; }
+
 static Picks picks_of(const Plan& p, const uint8_t* ws) {
     return {reinterpret_cast<const uint32_t*>(ws + p.bits_off), reinterpret_cast<const uint16_t*>(ws + p.rank_off), ws + p.count_off,
             reinterpret_cast<const uint16_t*>(ws + p.before_off), reinterpret_cast<const int*>(ws + p.flag_off) + 1};
@@ -1278,7 +1283,7 @@ static int launch_fwd(const CUtensorMap& tq, const CUtensorMap& tk, const CUtens
 int64_t forward_workspace_bytes(int64_t B, int64_t H, int64_t L, int64_t K, int64_t Dqk, int64_t Dv, int dtype) {
     if (!supported(B, H, L, K, Dqk, Dv)) return 0;
     const Plan p = make_plan(B, H, L, K, Dqk, Dv, dtype, false);
-    return dense_pays(p, false) ? p.bytes : 0;
+    return scratch_bytes(p, false);
 }
 
 // Returns the flag's device address in *flag: the gather kernel behind it runs when it is set.
@@ -1342,7 +1347,7 @@ int64_t backward_workspace_bytes(int64_t B, int64_t H, int64_t L, int64_t K, int
     if (!supported(B, H, L, K, Dqk, Dv)) return 0;
     if (dtype == CINN_F32 && (Dqk % 4 != 0 || Dv % 4 != 0)) return 0;                // rows a TMA box cannot address
     const Plan p = make_plan(B, H, L, K, Dqk, Dv, dtype, true);
-    return dense_pays(p, true) ? p.bytes : 0;
+    return scratch_bytes(p, true);
 }
 
 // Gradients in `dtype` (dq, dk, dv written, not added to).  *flag as in forward; *fallback: fp32 buffers (dq | dk | dv) the

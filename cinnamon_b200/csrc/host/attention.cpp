@@ -6,6 +6,17 @@ namespace cinnhost {
 
 namespace {
 
+// The tiles' scratch; undefined where they need none, or where there is no room for it: the gather kernels, which need none,
+// compute the call then.
+Tensor scratch(int64_t bytes, const at::Device& dev) {
+    if (!bytes) return Tensor();
+    try {
+        return empty({bytes}, at::kByte, dev);
+    } catch (const c10::OutOfMemoryError&) {
+        return Tensor();
+    }
+}
+
 struct Attention { Tensor out, attn, q, k, v, idx, out32, lse; };
 
 Attention forward(const Tensor& q_in, const Tensor& k_in, const Tensor& v_in, const Tensor& idx_in, double scale) {
@@ -24,8 +35,9 @@ Attention forward(const Tensor& q_in, const Tensor& k_in, const Tensor& v_in, co
     r.attn = empty({B, H, L, K}, at::kFloat, dev);
     const bool cast = work != at::kFloat;
     r.out = cast ? empty({B, H, L, Dv}, work, dev) : r.out32;
-    const int64_t need = api.cinn_sparse_attn_workspace_bytes(B, H, L, K, Dqk, Dv, tag_of(work), 0);
-    Tensor ws = need ? empty({need}, at::kByte, dev) : Tensor();
+    int64_t need = api.cinn_sparse_attn_workspace_bytes(B, H, L, K, Dqk, Dv, tag_of(work), 0);
+    const Tensor ws = scratch(need, dev);
+    if (!ws.defined()) need = 0;
     check(api.cinn_sparse_attn_fwd_ws(r.q.data_ptr(), r.k.data_ptr(), r.v.data_ptr(), tag_of(work), r.idx.data_ptr<int64_t>(), f32(r.out32),
                                       cast ? r.out.data_ptr() : nullptr, f32(r.lse), f32(r.attn), B, H, L, K, Dqk, Dv, (float)scale,
                                       need ? ws.data_ptr() : nullptr, need, stream()), "cinn_sparse_attn_fwd");
@@ -42,8 +54,8 @@ std::tuple<Tensor, Tensor, Tensor> backward(const Tensor& grad_out, const Tensor
     const int tag = tag_of(q.scalar_type());
     const int64_t need = api.cinn_sparse_attn_workspace_bytes(B, H, L, K, Dqk, Dv, tag, 1);
     const auto odd = [](const Tensor& t) { return (reinterpret_cast<uintptr_t>(t.data_ptr()) & 15) != 0; };
-    if (need && g.scalar_type() == q.scalar_type() && !(odd(q) || odd(k) || odd(v) || odd(g))) {
-        Tensor ws = empty({need}, at::kByte, q.device());
+    const bool tiles = need && g.scalar_type() == q.scalar_type() && !(odd(q) || odd(k) || odd(v) || odd(g));
+    if (const Tensor ws = scratch(tiles ? need : 0, q.device()); ws.defined()) {
         Tensor gq = empty({B, H, L, Dqk}, q.scalar_type(), q.device()), gk = empty({B, H, L, Dqk}, q.scalar_type(), q.device());
         Tensor gv = empty({B, H, L, Dv}, q.scalar_type(), q.device());
         check(api.cinn_sparse_attn_bwd_ws(g.data_ptr(), f32(out32), f32(lse), q.data_ptr(), k.data_ptr(), v.data_ptr(), tag,

@@ -271,7 +271,7 @@ int cinn_sparse_attn_fwd(const void* q, const void* k, const void* v, int dtype,
 
 /* The same with a scratch buffer (256-byte aligned), by which a sequence of which the queries pick a fair share goes
  * through dense tiles on the tensor cores instead of row gathers.  cinn_sparse_attn_workspace_bytes (backward: 0 / 1) says
- * how much that takes, 0 where the gathers are the better choice; a null or smaller workspace selects them.
+ * how much that takes (about as much as the tensors, 16 GiB at most), 0 where the gathers are the better choice; a null or smaller workspace selects them.
  * out_cast: null, or the output once more in `dtype`. */
 int cinn_set_sparse_attn_dense(int mode); /* -1: choose by shape (default), 0: gathers, 1: dense tiles where they can;
                                              returns the previous mode */

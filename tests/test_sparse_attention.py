@@ -249,3 +249,42 @@ def test_a_nan_key_reaches_the_queries_that_picked_it(dtype, key):
     for a, b in zip(*got):
         torch.testing.assert_close(a, b, rtol=1e-5 if dtype == torch.float32 else 8e-3, atol=1e-6, equal_nan=True)
     assert K.device_status() == 0
+
+
+def test_scratch_of_the_tiles_is_bounded():
+    """No shape asks for more than 16 GiB, and the listed training shape for what its documentation says."""
+    from cinnamon_b200 import _lib
+    need = _lib.lib.cinn_sparse_attn_workspace_bytes
+    assert 0 < need(32, 8, 1024, 128, 192, 64, _lib.F32, 0) < 0.8e9 and 0 < need(32, 8, 1024, 128, 192, 64, _lib.F32, 1) < 1.2e9
+    for B, H, L, K in ((512, 8, 1024, 512), (64, 64, 4096, 512), (16, 64, 12000, 512), (4096, 16, 512, 256)):
+        for dtype in (_lib.F32, _lib.BF16, _lib.F16):
+            for backward in (0, 1):
+                assert 0 <= need(B, H, L, K, 192, 128, dtype, backward) <= 16 << 30
+
+
+@pytest.mark.gpu
+def test_without_room_for_the_scratch_the_gathers_compute_the_call():
+    """Memory for the tensors but not for the tiles' scratch: the call succeeds, with the gathers' numbers."""
+    from cinnamon_b200 import kernels as K
+    g = torch.Generator(device="cuda").manual_seed(9)
+    B, H, L, k, dq, dv = 4, 8, 1024, 128, 192, 64
+    q, kk, v = (torch.randn(B, H, L, d, generator=g, device="cuda").requires_grad_(True) for d in (dq, dq, dv))
+    idx = torch.randint(0, L, (B, L, k), generator=g, device="cuda")
+    need = K._L.cinn_sparse_attn_workspace_bytes(B, H, L, k, dq, dv, 1, 0)
+    outputs = 4 * B * H * L * (dv + 1 + k)
+    assert need > 1.3 * outputs
+    before = K._L.cinn_set_sparse_attn_dense(0)
+    want = [t.detach().clone() for t in K.sparse_attention(q, kk, v, idx)]
+    K._L.cinn_set_sparse_attn_dense(before)
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    limit = torch.cuda.memory_reserved() + int(1.1 * outputs) + (24 << 20)
+    try:
+        torch.cuda.set_per_process_memory_fraction(limit / torch.cuda.get_device_properties(0).total_memory)
+        out, attn = K.sparse_attention(q, kk, v, idx)
+    finally:
+        torch.cuda.set_per_process_memory_fraction(1.0)
+    assert torch.equal(out, want[0]) and torch.equal(attn, want[1])
+    tiles, _ = K.sparse_attention(q, kk, v, idx)
+    assert not torch.equal(tiles, out)                            # (with room it is the tiles that compute it)
+    torch.testing.assert_close(tiles, out, rtol=1e-5, atol=1e-5)
