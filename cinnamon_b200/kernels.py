@@ -299,9 +299,10 @@ def transpose_fp8(x_fp8: torch.Tensor) -> torch.Tensor:
 # -----------------------------------------------------------------------------
 # GEMM (reference: src/kernels.py:667-702)
 # -----------------------------------------------------------------------------
-def _gemm(a, a_scales, b, b_layout, sb, sb_stride_k, sb_stride_n, M, N, K, out_dtype, bf16_rounded=False, out=None):
+def _gemm(a, a_scales, b, b_layout, sb, sb_stride_k, sb_stride_n, M, N, K, out_dtype, bf16_rounded=False, out=None, whole=False):
     """``bf16_rounded`` (fp32 output only): store the result rounded to bf16, i.e. exactly what a
-    bf16 result cast to fp32 would hold.  ``out``: a contiguous (M, N) tensor of ``out_dtype`` to write into."""
+    bf16 result cast to fp32 would hold.  ``out``: a contiguous (M, N) tensor of ``out_dtype`` to write into.
+    ``whole``: never cut along K, so that a row's bits do not depend on how many rows the call has."""
     with torch.cuda.device(a.device):
         if out is None:
             out = torch.empty((M, N), dtype=out_dtype, device=a.device)
@@ -312,7 +313,8 @@ def _gemm(a, a_scales, b, b_layout, sb, sb_stride_k, sb_stride_n, M, N, K, out_d
         if gemm_events is not None:
             ev = (torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True))
             ev[0].record()
-        need = int(_L.cinn_fp8_gemm_workspace_bytes(M, N, K, b_layout))      # few tiles, long reduction: cut along K
+        # few tiles, long reduction: cut along K
+        need = 0 if whole else int(_L.cinn_fp8_gemm_workspace_bytes(M, N, K, b_layout))
         ws = torch.empty(need, dtype=torch.uint8, device=a.device) if need else None
         _lib.check(_L.cinn_fp8_gemm_ws(_ptr(a), _ptr(a_scales), a_scales.stride(0), _ptr(b), _ptr(sb), sb_stride_k,
                                        sb_stride_n, _ptr(out), M, N, K, b_layout, tag, _ptr(ws) if need else None, need, _stream(a)),

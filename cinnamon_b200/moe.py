@@ -148,7 +148,9 @@ class FP8SwiGLU:
         (the layout ``GroupedExperts`` uses for the routed experts, src/layers.py:47-49);
       * SiLU, the product and the quantisation of w3's input are one pass over that GEMM's output.
 
-    ``round_scale`` is the power-of-two scale option of w1 / w2's input quantisation."""
+    ``round_scale`` is the power-of-two scale option of w1 / w2's input quantisation.  A token's result does not depend on
+    the other tokens of the call: the GEMMs are never cut along K, so that a rank's share of the tokens gives the bits that one
+    GPU with all of them gives."""
 
     def __init__(self, w1: torch.Tensor, w2: torch.Tensor, w3: torch.Tensor, round_scale: bool = False):
         from . import kernels as K
@@ -172,10 +174,10 @@ class FP8SwiGLU:
         if x_q is None:
             x_q, x_s = K.quantize_fp8_rowwise(x, 128, self.round_scale)
         h12 = K._gemm(x_q, x_s, self.w12_q, K._lib.B_NK, self.w12_s, self.w12_s.stride(1), self.w12_s.stride(0), T,
-                      2 * self.hidden, self.d_model, torch.bfloat16)
+                      2 * self.hidden, self.d_model, torch.bfloat16, whole=True)
         h_q, h_s = K.swiglu_quantize_rowwise(h12)
         return K._gemm(h_q, h_s, self.w3_q, K._lib.B_NK, self.w3_s, self.w3_s.stride(1), self.w3_s.stride(0), T,
-                       self.d_model, self.hidden, torch.bfloat16)
+                       self.d_model, self.hidden, torch.bfloat16, whole=True)
 
 
 # ---------------------------------------------------------------------------------------

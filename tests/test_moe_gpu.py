@@ -163,6 +163,22 @@ def test_native_layer_matches_its_parts(K, T, d, shared, rs):
     assert layer(x[:0]).shape == (0, d)
 
 
+@pytest.mark.parametrize("tokens", [1, 40, 130])
+def test_shared_expert_of_a_share_of_the_tokens(K, tokens):
+    """Wide enough that few tokens would be cut along K: a rank's tokens get the bits that all tokens on one GPU give them, by
+    the shared expert itself (several ranks) and in the native layer (one GPU)."""
+    from cinnamon_b200 import moe
+    g = torch.Generator().manual_seed(tokens)
+    w = lambda *s: (torch.randn(*s, generator=g) * 0.05).bfloat16().cuda()                       # noqa: E731
+    d, I, E = 7168, 2048, 2
+    sh = moe.FP8SwiGLU(w(I, d), w(I, d), w(d, I))
+    x = w(2048, d) * 20
+    assert K._L.cinn_fp8_gemm_workspace_bytes(tokens, 2 * I, d, 0) > 0 == K._L.cinn_fp8_gemm_workspace_bytes(2048, 2 * I, d, 0)
+    assert torch.equal(sh(x[:tokens]), sh(x)[:tokens])
+    layer = moe.ExpertParallelMoE(w(E, d).float(), torch.zeros(E, device="cuda"), w(E, 256, d) * 0, w(E, d, 128), 1, shared=sh)
+    assert torch.equal(layer(x[:tokens]), sh(x)[:tokens].float())      # (routed experts of zeros: the shared expert's output)
+
+
 def test_subclassed_experts_are_called(K):
     """Experts or a shared expert of a class of their own are called, not replaced by the native layer's sequence."""
     from cinnamon_b200 import moe
