@@ -87,6 +87,7 @@ SIGNATURES = {
     "cinn_swiglu_backward": [_vp, _vp, _vp, _i32, _i64, _i64, _vp],
     "cinn_moe_combine_add": [_vp, _i32, _vp, _vp, _vp, _i32, _vp, _i64, _i64, _i32, _i64, _vp],
     "cinn_moe_sum_add": [_vp, _i32, _vp, _vp, _i32, _vp, _i64, _i64, _i32, _i64, _vp],
+    "cinn_launch_count": [],
     "cinn_device_status": [ctypes.POINTER(ctypes.c_int), _i32],
     "cinn_fp8_grouped_gemm": [_vp, _vp, _vp, _vp, _vp, _vp, _i64, _i64, _i64, _i64, _vp, _i32, _vp],
 }
@@ -109,7 +110,7 @@ def _load() -> ctypes.CDLL:
         fn.restype = (ctypes.c_char_p if name == "cinn_last_error"
                       else ctypes.c_longlong if name == "cinn_set_wait_limit_cycles"
                       else ctypes.c_int64 if name in ("cinn_moe_route_workspace_ints", "cinn_moe_route_static_max_ints", "cinn_fp8_gemm_workspace_bytes", "cinn_moe_balance_workspace_bytes",
-                                                 "cinn_sparse_attn_workspace_bytes",
+                                                 "cinn_sparse_attn_workspace_bytes", "cinn_launch_count",
                                                  "cinn_fp8_grouped_wgrad_scratch_bytes", "cinn_fp8_grouped_wgrad_fused_scratch_bytes")
                       else ctypes.c_int)
     return lib

@@ -14,6 +14,8 @@ void set_error(const char* fmt, ...) {
     va_end(ap);
 }
 
+std::atomic<int64_t> g_launches{0};
+
 int sm_count() {
     static int cached[64];
     static std::mutex mu;
@@ -489,6 +491,8 @@ int cinn_spread_rows(const void* q, const float* scales, const int64_t* pos, voi
                      int64_t n_rows, int top_k, int64_t d, int64_t n_scales, void* stream) {
     return cinn::spread_rows(q, scales, pos, out_q, out_scales, n_tokens, n_rows, top_k, d, n_scales, (cudaStream_t)stream);
 }
+
+int64_t cinn_launch_count(void) { return cinn::g_launches.load(std::memory_order_relaxed); }
 
 int64_t cinn_moe_route_static_max_ints(void) { return cinn::moe_route_static_max_ints(); }
 

@@ -1,5 +1,6 @@
 // Shared helpers for the cinnamon_b200 CUDA library (sm_100a only).
 #pragma once
+#include <atomic>
 #include <cuda_runtime.h>
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
@@ -46,7 +47,13 @@ void set_error(const char* fmt, ...);
         }                                                                              \
     } while (0)
 
-#define CINN_CHECK_LAUNCH()  CINN_CHECK_CUDA(cudaGetLastError())
+// after every launch, and after nothing else: it also counts it (cinn_launch_count)
+extern std::atomic<int64_t> g_launches;
+#define CINN_CHECK_LAUNCH()                                          \
+    do {                                                             \
+        CINN_CHECK_CUDA(cudaGetLastError());                         \
+        cinn::g_launches.fetch_add(1, std::memory_order_relaxed);    \
+    } while (0)
 
 // Programmatic dependent launch.  A kernel launched by launch_dependent may start while the one before it on the stream is
 // still running, as soon as every block of that one has called pdl_trigger (or has ended); nothing it reads or writes in

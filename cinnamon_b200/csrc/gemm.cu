@@ -667,6 +667,7 @@ static int launch(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMa
     int rc = allow_smem_once<kern>(smem_bytes(GROUPED ? MAX_EXPERTS : 0));
     if (rc) return rc;
     CINN_CHECK_CUDA(launch_dependent(kern, grid, THREADS, smem, st, ta, tb, tc, p));
+    CINN_CHECK_LAUNCH();
     return CINN_OK;
 }
 
@@ -707,6 +708,7 @@ static int launch_pair(const CUtensorMap& ta, const CUtensorMap& tb, const CUten
     cfg.attrs = attr;
     cfg.numAttrs = 2;
     CINN_CHECK_CUDA(cudaLaunchKernelEx(&cfg, kern, ta, tb, tc, p));
+    CINN_CHECK_LAUNCH();
     return CINN_OK;
 }
 

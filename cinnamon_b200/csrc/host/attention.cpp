@@ -41,7 +41,6 @@ Attention forward(const Tensor& q_in, const Tensor& k_in, const Tensor& v_in, co
     check(api.cinn_sparse_attn_fwd_ws(r.q.data_ptr(), r.k.data_ptr(), r.v.data_ptr(), tag_of(work), r.idx.data_ptr<int64_t>(), f32(r.out32),
                                       cast ? r.out.data_ptr() : nullptr, f32(r.lse), f32(r.attn), B, H, L, K, Dqk, Dv, (float)scale,
                                       need ? ws.data_ptr() : nullptr, need, stream()), "cinn_sparse_attn_fwd");
-    launches += need ? (cast ? 3 : 4) : 1;
     if (in != work) r.out = r.out32.to(in);
     return r;
 }
@@ -61,7 +60,6 @@ std::tuple<Tensor, Tensor, Tensor> backward(const Tensor& grad_out, const Tensor
         check(api.cinn_sparse_attn_bwd_ws(g.data_ptr(), f32(out32), f32(lse), q.data_ptr(), k.data_ptr(), v.data_ptr(), tag,
                                           idx.data_ptr<int64_t>(), gq.data_ptr(), gk.data_ptr(), gv.data_ptr(), B, H, L, K, Dqk, Dv,
                                           (float)scale, ws.data_ptr(), need, stream()), "cinn_sparse_attn_bwd");
-        launches += 7;
         if (in == q.scalar_type()) return {gq, gk, gv};
         return {gq.to(in), gk.to(in), gv.to(in)};
     }
@@ -72,7 +70,6 @@ std::tuple<Tensor, Tensor, Tensor> backward(const Tensor& grad_out, const Tensor
     check(api.cinn_sparse_attn_bwd(g.data_ptr(), tag_of(g.scalar_type()), f32(out32), f32(lse), q.data_ptr(), k.data_ptr(), v.data_ptr(),
                                    tag_of(q.scalar_type()), idx.data_ptr<int64_t>(), f32(gq), f32(gk), f32(gv), B, H, L, K, Dqk, Dv,
                                    (float)scale, stream()), "cinn_sparse_attn_bwd");
-    ++launches;
     return {gq.to(in), gk.to(in), gv.to(in)};
 }
 

@@ -12,7 +12,6 @@
 #include <ATen/cuda/CUDAContext.h>
 #include <ATen/cuda/EmptyTensor.h>
 #include <c10/cuda/CUDAGuard.h>
-#include <atomic>
 #include <exception>
 #include <string>
 #include "../../../include/cinnamon_b200.h"
@@ -39,7 +38,6 @@ struct Api {
 };
 extern Api api;
 extern PyObject* library_error;                // _lib.LibraryError
-extern std::atomic<int64_t> launches;          // kernels of the library launched from here
 
 // A status of the library as an exception: `invalid` becomes Python's AssertionError, the rest LibraryError.
 struct CinnError : std::exception {

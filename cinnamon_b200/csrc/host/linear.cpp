@@ -11,7 +11,6 @@ Tensor gemm(const Tensor& a, const Tensor& sa, const Tensor& b, int layout, cons
     Tensor ws = need ? empty({need}, at::kByte, a.device()) : Tensor();
     check(api.cinn_fp8_gemm_ws(a.data_ptr(), f32(sa), sa.stride(0), b.data_ptr(), f32(sb), sbk, sbn, out.data_ptr(), M, N, K, layout,
                                tag, need ? ws.data_ptr() : nullptr, need, stream()), "cinn_fp8_gemm");
-    launches += need ? 2 : 1;
     return out;
 }
 
@@ -60,7 +59,6 @@ Linear linear_forward(const Tensor& x, const Tensor& weight, bool round_scale, b
         r.x = xq;
         r.x_scale = xs;
     }
-    ++launches;
     if (w_q.defined()) {
         r.w = w_q;
         r.w_scale = w_s;
@@ -77,7 +75,6 @@ Linear linear_forward(const Tensor& x, const Tensor& weight, bool round_scale, b
         check(api.cinn_quant_block_beside(wf.data_ptr(), tag_of(wf.scalar_type()), N, K, wf.stride(0), wf.stride(1), r.w.data_ptr(),
                                           r.w_t.defined() ? r.w_t.data_ptr() : nullptr, f32(r.w_scale), 0, div, stream()),
               "cinn_quant_blockwise");
-        ++launches;
     }
     r.out = gemm(xq, xs, r.w, 0, r.w_scale, r.w_scale.stride(1), r.w_scale.stride(0), M, N, K, at::kBFloat16, TAG_BF16);
     if (x.dim() != 2) {
@@ -111,7 +108,6 @@ std::tuple<std::vector<Tensor>, Tensor> linear_backward(const Tensor& grad_out, 
     Tensor gqt = empty({N, Mp}, F8, dev), gst = empty({N, up(Mp, 128)}, at::kFloat, dev);
     check(api.cinn_quant_rowwise_dual(g.data_ptr(), tag_of(g.scalar_type()), Mp, N, g.stride(0), gq.data_ptr(), f32(gs),
                                       gqt.data_ptr(), f32(gst), round_scale, div, stream()), "cinn_quant_rowwise_dual");
-    ++launches;
     // (the reference's input gradient is bf16 and autograd casts it to the input's type: fp32 holds those values)
     const int gx_tag = gx_type == at::kFloat ? TAG_F32_BF16 : TAG_BF16;
     std::vector<Tensor> gx(parts);
@@ -121,7 +117,6 @@ std::tuple<std::vector<Tensor>, Tensor> linear_backward(const Tensor& grad_out, 
         if (k_major && !wt.defined()) {
             wt = empty({K, N}, F8, dev);
             check(api.cinn_transpose_bytes(w.data_ptr(), w.stride(0), wt.data_ptr(), N, K, stream()), "cinn_transpose_bytes");
-            ++launches;
         }
         const int64_t n = N / parts;                // reduction length of a part: columns of gq and wt, rows of w
         const int64_t need = api.cinn_fp8_gemm_workspace_bytes(M, K, n, k_major ? 0 : 1);
@@ -133,7 +128,6 @@ std::tuple<std::vector<Tensor>, Tensor> linear_backward(const Tensor& grad_out, 
                                             k_major ? N : K, f32(w_scale) + p * (n / 128) * w_scale.stride(0), w_scale.stride(0),
                                             w_scale.stride(1), out.data_ptr(), M, K, n, k_major ? 0 : 1, gx_tag,
                                             need ? ws.data_ptr() : nullptr, need, stream()), "cinn_fp8_gemm");
-            launches += need ? 2 : 1;
             gx[p] = x_shape.size() != 2 ? out.reshape(x_shape) : out;
         }
     }
@@ -144,7 +138,6 @@ std::tuple<std::vector<Tensor>, Tensor> linear_backward(const Tensor& grad_out, 
         x_scale = x_scale.contiguous();
         check(api.cinn_requant_row_to_block(x.data_ptr(), f32(x_scale), Mp, K, xb.data_ptr(), f32(xbs), 0, div, stream()),
               "cinn_requant_row_to_block");
-        ++launches;
         x = xb;
         x_scale = xbs;
     }
@@ -177,7 +170,6 @@ Tensor linear_inference(const Tensor& x, const Tensor& weight, bool round_scale,
           "cinn_quant_linear");
     check(api.cinn_fp8_gemm_ws(b, xs, nkb, b + o_wq, ws, 1, nkb, out.data_ptr(), M, N, K, 0, TAG_BF16, need ? b + o_part : nullptr, need,
                                stream()), "cinn_fp8_gemm");
-    launches += need ? 3 : 2;
     return out;
 }
 

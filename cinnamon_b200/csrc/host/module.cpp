@@ -4,7 +4,6 @@
 namespace cinnhost {
 Api api;
 PyObject* library_error = PyExc_RuntimeError;
-std::atomic<int64_t> launches{0};
 void bind_linear(pybind11::module_& m);
 void bind_attention(pybind11::module_& m);
 void bind_moe(pybind11::module_& m);
@@ -26,7 +25,6 @@ PYBIND11_MODULE(_host, m) {
 #undef CINN_NAME
         return names;
     });
-    m.def("launches", [] { return launches.load(); });
     pybind11::register_exception_translator([](std::exception_ptr p) {
         try {
             if (p) std::rethrow_exception(p);

@@ -10,7 +10,6 @@ Quantised rowwise(const Tensor& x, bool round_scale, int div) {
     Quantised r{empty({M, K}, F8, x.device()), empty({M, up(K, 128)}, at::kFloat, x.device())};
     check(api.cinn_quant_rowwise(x.data_ptr(), tag_of(x.scalar_type()), M, K, x.stride(0), x.stride(1), r.q.data_ptr(), f32(r.s), 128,
                                  round_scale, div, stream()), "cinn_quant_rowwise");
-    ++launches;
     return r;
 }
 
@@ -19,7 +18,6 @@ Quantised swiglu_quantised(const Tensor& h12, int div) {
     Quantised r{empty({T, I}, F8, h12.device()), empty({T, up(I, 128)}, at::kFloat, h12.device())};
     check(api.cinn_swiglu_quant_rowwise(h12.data_ptr(), tag_of(h12.scalar_type()), T, I, r.q.data_ptr(), f32(r.s), div, stream()),
           "cinn_swiglu_quant_rowwise");
-    ++launches;
     return r;
 }
 
@@ -29,7 +27,6 @@ Tensor grouped(const Quantised& x, const Quantised& w, const Tensor& starts, con
     check(api.cinn_fp8_grouped_gemm(x.q.data_ptr(), f32(x.s), w.q.data_ptr(), f32(w.s), starts.data_ptr<int64_t>(),
                                     ends.data_ptr<int64_t>(), E, T, d_in, d_out, out.data_ptr(), tag_of(type), stream()),
           "cinn_fp8_grouped_gemm");
-    ++launches;
     return out;
 }
 
@@ -59,7 +56,6 @@ Routes route(const Tensor& logits_in, const Tensor& bias, int64_t top_k) {
                                     r.top.data_ptr<int>(), f32(top_gates), r.token_indices(), f32(r.floats), r.sorted_experts(),
                                     r.part(3 * r.pairs), r.part(3 * r.pairs + E), r.part(3 * r.pairs + 2 * E), r.pos(), r.gates(),
                                     stream()), "cinn_moe_route");
-    launches += 3;
     return r;
 }
 
@@ -69,7 +65,6 @@ Quantised spread(const Quantised& x, const Routes& r, int64_t top_k) {
     Quantised rows{empty({r.pairs, d}, F8, x.q.device()), empty({r.pairs, ns}, at::kFloat, x.q.device())};
     check(api.cinn_spread_rows(x.q.data_ptr(), f32(x.s), r.pos(), rows.q.data_ptr(), f32(rows.s), T, r.pairs, (int)top_k, d, ns, stream()),
           "cinn_spread_rows");
-    ++launches;
     return rows;
 }
 
@@ -82,7 +77,6 @@ Tensor gemm_whole(const Tensor& a, const Tensor& sa, const Tensor& b, const Tens
     Tensor out = empty({M, N}, at::kBFloat16, a.device());
     check(api.cinn_fp8_gemm_ws(a.data_ptr(), f32(sa), sa.stride(0), b.data_ptr(), f32(sb), sb.stride(1), sb.stride(0), out.data_ptr(), M, N, K, 0,
                                TAG_BF16, nullptr, 0, stream()), "cinn_fp8_gemm");
-    ++launches;
     return out;
 }
 
@@ -122,7 +116,6 @@ Tensor forward(const Tensor& x, const Tensor& router, const Tensor& bias, int64_
     else
         check(api.cinn_moe_combine(out.data_ptr(), TAG_BF16, pos, r.gates(), f32(y), T, pairs, (int)top_k, d, stream()),
               "cinn_moe_combine");
-    ++launches;
     return y;
 }
 

@@ -25,7 +25,6 @@ Tensor swiglu_rounded(const Tensor& h12) {
     const int64_t T = h12.size(0), I = h12.size(1) / 2;
     Tensor h = empty({T, I}, h12.scalar_type(), h12.device());
     check(api.cinn_swiglu_rounded(h12.data_ptr(), h.data_ptr(), tag_of(h12.scalar_type()), T, I, stream()), "cinn_swiglu");
-    ++launches;
     return h;
 }
 
@@ -79,7 +78,6 @@ struct SwiGLUNode : public torch::autograd::Function<SwiGLUNode> {
             Tensor dh12 = empty({T, 2 * I}, h12.scalar_type(), h12.device()), d12;
             check(api.cinn_swiglu_rounded_backward(h12.data_ptr(), dh[0].data_ptr(), dh12.data_ptr(), tag_of(h12.scalar_type()), T, I, stream()),
                   "cinn_swiglu_backward");
-            ++launches;
             std::tie(dx, d12) = back(ctx->saved_data["a"].toInt(), dh12, 0, ctx->saved_data["x_shape"].toIntVector(), gx, g12,
                                      ctx->saved_data["x32"].toBool() ? at::kFloat : at::kBFloat16, 2);
             if (g12) {
@@ -119,7 +117,6 @@ std::tuple<Tensor, Tensor> grouped_backward(const Tensor& dy, const Tensor& xq, 
     check(api.cinn_fp8_grouped_wgrad_fused(dy.data_ptr(), tag_of(dy.scalar_type()), xq.data_ptr(), f32(xs), st, en, E, R, d_in, d_out,
                                            scratch.data_ptr(), need, dw.data_ptr(), w_type == at::kFloat ? TAG_F32_BF16 : TAG_BF16, div,
                                            one_pass ? gq.data_ptr() : nullptr, one_pass ? f32(gs) : nullptr, stream()), "cinn_fp8_grouped_wgrad_fused");
-    launches += 4;
     Tensor dx;
     if (want_x) {
         if (!one_pass) {
@@ -130,11 +127,9 @@ std::tuple<Tensor, Tensor> grouped_backward(const Tensor& dy, const Tensor& xq, 
         dx = empty({R, d_in}, x_type, dev);
         if (!covered) {
             check(api.cinn_zero_rows_outside(dx.data_ptr(), R, d_in * dx.element_size(), st, en, E, stream()), "cinn_zero_rows_outside");
-            ++launches;
         }
         check(api.cinn_fp8_grouped_gemm_dgrad(gq.data_ptr(), f32(gs), wq.data_ptr(), f32(ws), st, en, E, R, d_in, d_out, dx.data_ptr(),
                                               tag_of(x_type), stream()), "cinn_fp8_grouped_gemm_dgrad");
-        ++launches;
     }
     return {dx, dw};
 }
@@ -157,7 +152,6 @@ struct BlockNode : public torch::autograd::Function<BlockNode> {
         Tensor y = empty({T, d}, at::kFloat, dev);
         check(api.cinn_moe_combine_add(out.data_ptr(), TAG_BF16, r.pos(), r.gates(), addend.data_ptr(), tag_of(addend.scalar_type()), f32(y),
                                        T, r.pairs, (int)k, d, stream()), "cinn_moe_combine_add");
-        ++launches;
         Tensor share, loss;
         if (o->alpha > 0) {
             share = empty({o->batch, E}, at::kFloat, dev);
@@ -165,7 +159,6 @@ struct BlockNode : public torch::autograd::Function<BlockNode> {
             Tensor ws = empty({api.cinn_moe_balance_workspace_bytes(o->batch, seq, (int)E)}, at::kByte, dev);
             check(api.cinn_moe_balance_loss(logits.data_ptr(), tag_of(logits.scalar_type()), r.top.data_ptr<int>(), o->batch, seq, (int)E,
                                             (int)k, (float)o->alpha, ws.data_ptr(), f32(share), f32(loss), stream()), "cinn_moe_balance_loss");
-            launches += 2;
         }
         o->counts = r.counts();
         ctx->save_for_backward({xr, wr, logits, r.longs, r.floats, rows.q, rows.s, h12, h.q, h.s, out, o->w12.q, o->w12.s, o->w3.q, o->w3.s,
@@ -205,7 +198,6 @@ struct BlockNode : public torch::autograd::Function<BlockNode> {
                     d_gates = empty({T, k}, at::kFloat, dev);
                     check(api.cinn_moe_combine_backward(out.data_ptr(), TAG_BF16, r.pos(), r.gates(), f32(dy), d_out.data_ptr(), f32(d_gates),
                                                         T, r.pairs, (int)k, d, stream()), "cinn_moe_combine_backward");
-                    ++launches;
                     const bool below = want_x || want_12;
                     Tensor dh;
                     std::tie(dh, dw3) = grouped_backward(d_out, s[8], s[9], s[13], s[14], starts, ends, type(6), below, at::kBFloat16, div);
@@ -215,7 +207,6 @@ struct BlockNode : public torch::autograd::Function<BlockNode> {
                         Tensor dh12 = empty({r.pairs, 2 * I}, at::kBFloat16, dev);
                         check(api.cinn_swiglu_backward(h12.data_ptr(), dh.data_ptr(), dh12.data_ptr(), TAG_BF16, r.pairs, I, stream()),
                               "cinn_swiglu_backward");
-                        ++launches;
                         std::tie(d_rows, dw12) = grouped_backward(dh12, s[5], s[6], s[11], s[12], starts, ends, type(5), want_x,
                                                                   type(3), div);
                     }
@@ -230,7 +221,6 @@ struct BlockNode : public torch::autograd::Function<BlockNode> {
                                                   d_gates.defined() ? f32(d_gates) : nullptr, loss ? f32(s[15]) : nullptr,
                                                   loss ? f32(dl) : nullptr, alpha, batch, seq, (int)E, (int)k, d_logits.data_ptr(), stream()),
                       "cinn_moe_gates_backward");
-                ++launches;
                 if (want_r) d_router = at::mm(d_logits.t(), xr).to(type(4));
                 if (want_x) dxr = at::mm(d_logits, wr);
             }
@@ -238,7 +228,6 @@ struct BlockNode : public torch::autograd::Function<BlockNode> {
                 dx = empty({T, d}, at::kFloat, dev);
                 check(api.cinn_moe_sum_add(d_rows.data_ptr(), tag_of(d_rows.scalar_type()), r.pos(), dxr.data_ptr(), tag_of(dxr.scalar_type()),
                                            f32(dx), T, r.pairs, (int)k, d, stream()), "cinn_moe_sum_add");
-                ++launches;
             } else {
                 dx = dxr;
             }
@@ -321,7 +310,6 @@ void bind_moe_train(pybind11::module_& m) {
         c10::cuda::CUDAGuard guard(bias.device());
         check(api.cinn_moe_update_bias(counts.data_ptr<int64_t>(), f32(bias), (int)bias.numel(), (float)expected, (float)gamma, stream()),
               "cinn_moe_update_bias");
-        ++launches;
         bias.unsafeGetTensorImpl()->bump_version();
     });
 }

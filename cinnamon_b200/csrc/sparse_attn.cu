@@ -491,6 +491,7 @@ int sparse_attn_bwd_tiles(const void* d_out, const float* out, const float* lse,
         zero_if_kernel<<<grid, 256, 0, st>>>(run_if, gk, nqk + nv);
     } else {
         zero_if_kernel<<<grid, 256, 0, st>>>(run_if, gk, nqk);
+        CINN_CHECK_LAUNCH();
         zero_if_kernel<<<grid, 256, 0, st>>>(run_if, gv, nv);
     }
     CINN_CHECK_LAUNCH();
@@ -500,8 +501,8 @@ int sparse_attn_bwd_tiles(const void* d_out, const float* out, const float* lse,
     for (const auto& c : casts) {
         if (dtype == CINN_BF16) cast_if_kernel<<<grid, 256, 0, st>>>(run_if, c.src, static_cast<__nv_bfloat16*>(c.dst), c.n);
         else cast_if_kernel<<<grid, 256, 0, st>>>(run_if, c.src, static_cast<__half*>(c.dst), c.n);
+        CINN_CHECK_LAUNCH();
     }
-    CINN_CHECK_LAUNCH();
     return CINN_OK;
 }
 

@@ -48,9 +48,6 @@ _KMAJOR_BACKWARD = os.environ.get("CINN_KMAJOR_BACKWARD", "1") != "0"
 _MOE_GROUPED_PRECISION = os.environ.get("CINN_MOE_GROUPED", "fp8")
 assert _MOE_GROUPED_PRECISION in ("fp8", "16bit"), "CINN_MOE_GROUPED must be fp8 or 16bit"
 
-# kernels of this library launched since import (the benchmark reports it): those launched from this file, to which
-# ``launch_count`` (a module attribute) adds those of the native host path
-_launches = 0
 # when set to a list, every GEMM launch appends a (start, end) pair of CUDA events to it
 gemm_events = None
 
@@ -83,14 +80,9 @@ def _ptr(t: torch.Tensor) -> ctypes.c_void_p:
     return ctypes.c_void_p(t.data_ptr())
 
 
-def _count(n: int = 1) -> None:
-    global _launches
-    _launches += n
-
-
 def __getattr__(name: str):
-    if name == "launch_count":
-        return _launches + _host.launches()
+    if name == "launch_count":                      # kernels launched by the library so far (the benchmark reports it)
+        return int(_L.cinn_launch_count())
     raise AttributeError(f"module {__name__!r} has no attribute {name!r}")
 
 
@@ -110,7 +102,6 @@ def selfcheck_division(device=None) -> int:
     with torch.cuda.device(device if device is not None else torch.cuda.current_device()):
         stream = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
         _lib.check(_L.cinn_selfcheck_division(ctypes.byref(n), stream), "cinn_selfcheck_division")
-    _count(2)
     return int(n.value)
 
 
@@ -142,7 +133,6 @@ def quantize_fp8_rowwise(x: torch.Tensor, block_size: int = 128, round_scale: bo
         _lib.check(_L.cinn_quant_rowwise(_ptr(x), _DTYPE_TAG[x.dtype], M, N, x.stride(0), x.stride(1), _ptr(q),
                                          _ptr(s), block_size, int(bool(round_scale)), _DIV_MODE, _stream(x)),
                    "cinn_quant_rowwise")
-    _count()
     return q, s
 
 
@@ -165,7 +155,6 @@ def quantize_fp8_rowwise_dual(x: torch.Tensor, round_scale: bool = False):
         _lib.check(_L.cinn_quant_rowwise_dual(_ptr(x), _DTYPE_TAG[x.dtype], M, N, x.stride(0), _ptr(q_row), _ptr(s_row),
                                               _ptr(q_col), _ptr(s_col), int(bool(round_scale)), _DIV_MODE, _stream(x)),
                    "cinn_quant_rowwise_dual")
-    _count()
     return q_row, s_row, q_col, s_col
 
 
@@ -192,7 +181,6 @@ def quantize_fp8_rowwise_with_block(x: torch.Tensor, round_scale: bool = False, 
         _lib.check(fn(_ptr(x), _DTYPE_TAG[x.dtype], M, N, x.stride(0), _ptr(q_row), _ptr(s_row),
                       _ptr(q_blk), _ptr(s_blk), int(bool(round_scale)), _DIV_MODE, _stream(x)),
                    "cinn_quant_rowwise_with_block")
-    _count()
     return q_row, s_row, q_blk, s_blk
 
 
@@ -211,7 +199,6 @@ def quantize_fp8_blockwise(x: torch.Tensor, block_m: int = 128, block_n: int = 1
         _lib.check(_L.cinn_quant_blockwise(_ptr(x), _DTYPE_TAG[x.dtype], M, N, x.stride(0), x.stride(1), _ptr(q),
                                            _ptr(s), block_m, block_n, int(bool(round_scale)), _DIV_MODE, _stream(x)),
                    "cinn_quant_blockwise")
-    _count()
     return q, s
 
 
@@ -232,7 +219,6 @@ def quantize_fp8_blockwise_t(x: torch.Tensor, round_scale: bool = False):
         s = torch.empty(((M + 127) // 128, (N + 127) // 128), dtype=torch.float32, device=x.device)
         _lib.check(_L.cinn_quant_blockwise_t(_ptr(x), _DTYPE_TAG[x.dtype], M, N, x.stride(0), _ptr(q), _ptr(q_t), _ptr(s),
                                              int(bool(round_scale)), _DIV_MODE, _stream(x)), "cinn_quant_blockwise_t")
-    _count()
     return q, s, q_t
 
 
@@ -244,7 +230,6 @@ def _dequant(x_fp8, scales, block_m, block_n, out_dtype):
         out = torch.empty((M, N), dtype=out_dtype, device=x_fp8.device)
         _lib.check(_L.cinn_dequant(_ptr(x_fp8), _ptr(scales), _ptr(out), _DTYPE_TAG[out_dtype], M, N, block_m, block_n,
                                    _stream(x_fp8)), "cinn_dequant")
-    _count()
     return out
 
 
@@ -276,7 +261,6 @@ def requantize_rowwise_to_blockwise(x_fp8: torch.Tensor, x_scale: torch.Tensor, 
         _lib.check(_L.cinn_requant_row_to_block(_ptr(x_fp8), _ptr(x_scale), M, K, _ptr(out), _ptr(s),
                                                 int(transpose_out), _DIV_MODE, _stream(x_fp8)),
                    "cinn_requant_row_to_block")
-    _count()
     return out, s
 
 
@@ -292,7 +276,6 @@ def transpose_fp8(x_fp8: torch.Tensor) -> torch.Tensor:
         out = torch.empty((C, R), dtype=x_fp8.dtype, device=x_fp8.device)
         _lib.check(_L.cinn_transpose_bytes(_ptr(x_fp8), x_fp8.stride(0), _ptr(out), R, C, _stream(x_fp8)),
                    "cinn_transpose_bytes")
-    _count()
     return out
 
 
@@ -322,7 +305,6 @@ def _gemm(a, a_scales, b, b_layout, sb, sb_stride_k, sb_stride_n, M, N, K, out_d
         if ev is not None:
             ev[1].record()
             gemm_events.append(ev)
-    _count(2 if need else 1)
     return out
 
 
@@ -667,7 +649,6 @@ def fp8_grouped_gemm(x_fp8, x_scale, w_fp8, w_scale, expert_starts, expert_ends,
         _lib.check(_L.cinn_fp8_grouped_gemm(_ptr(x_fp8), _ptr(x_scale), _ptr(w_fp8), _ptr(w_scale), _ptr(starts),
                                             _ptr(ends), E, T, d_in, d_out, _ptr(out), _DTYPE_TAG[out.dtype],
                                             _stream(x_fp8)), "cinn_fp8_grouped_gemm")
-    _count()
     return out
 
 
@@ -684,7 +665,6 @@ def fp8_grouped_gemm_scatter(x_fp8, x_scale, w_fp8, w_scale, expert_starts, expe
         _lib.check(_L.cinn_fp8_grouped_gemm_scatter(_ptr(x_fp8), _ptr(x_scale), _ptr(w_fp8), _ptr(w_scale), _ptr(starts),
                                                     _ptr(ends), E, T, d_in, d_out, _ptr(row_dst), _DTYPE_TAG[out_dtype],
                                                     _stream(x_fp8)), "cinn_fp8_grouped_gemm_scatter")
-    _count()
 
 
 def p2p_row_table(seg_start, home_base, peer_home, n_rows: int, row_bytes: int, n_ranks: int, capacity_rows: int) -> torch.Tensor:
@@ -695,7 +675,6 @@ def p2p_row_table(seg_start, home_base, peer_home, n_rows: int, row_bytes: int, 
         _lib.check(_L.cinn_p2p_row_table(_ptr(seg_start), _ptr(home_base), _ptr(peer_home), n_rows, row_bytes,
                                          home_base.numel(), n_ranks, capacity_rows, _ptr(table), _stream(seg_start)),
                    "cinn_p2p_row_table")
-    _count()
     return table
 
 
@@ -718,7 +697,6 @@ def swiglu_quantize_rowwise(h12: torch.Tensor, n_rows_dev: torch.Tensor = None):
             assert n_rows_dev.dtype == torch.int64 and n_rows_dev.is_cuda
             _lib.check(_L.cinn_swiglu_quant_rowwise_n(_ptr(h12), _DTYPE_TAG[h12.dtype], T, I, _ptr(n_rows_dev), _ptr(q),
                                                       _ptr(s), _DIV_MODE, _stream(h12)), "cinn_swiglu_quant_rowwise_n")
-    _count()
     return q, s
 
 
@@ -737,7 +715,6 @@ class SwiGLUFunction(torch.autograd.Function):
         with torch.cuda.device(flat.device):
             h = torch.empty((T, I), dtype=flat.dtype, device=flat.device)
             _lib.check(_L.cinn_swiglu(_ptr(flat), _ptr(h), _DTYPE_TAG[flat.dtype], T, I, _stream(flat)), "cinn_swiglu")
-        _count()
         ctx.save_for_backward(flat)
         ctx.shape, ctx.in_dtype = shape, h12.dtype
         return h.reshape(*shape[:-1], I).to(h12.dtype)
@@ -751,7 +728,6 @@ class SwiGLUFunction(torch.autograd.Function):
             grad = torch.empty_like(flat)
             _lib.check(_L.cinn_swiglu_backward(_ptr(flat), _ptr(g), _ptr(grad), _DTYPE_TAG[flat.dtype], T, I, _stream(flat)),
                        "cinn_swiglu_backward")
-        _count()
         return grad.reshape(ctx.shape).to(ctx.in_dtype)
 
 
@@ -785,7 +761,6 @@ def moe_combine(rows: torch.Tensor, pos: torch.Tensor, gates: torch.Tensor, adde
             _lib.check(_L.cinn_moe_combine_add(_ptr(rows), _DTYPE_TAG[rows.dtype], _ptr(pos), _ptr(gates), _ptr(addend),
                                                _DTYPE_TAG[addend.dtype], _ptr(y), T, rows.shape[0], k, d, _stream(rows)),
                        "cinn_moe_combine_add")
-    _count()
     return y
 
 
@@ -814,7 +789,6 @@ class MoECombineFunction(torch.autograd.Function):
             _lib.check(_L.cinn_moe_combine_backward(_ptr(rows_c), _DTYPE_TAG[rows_c.dtype], _ptr(pos_c), _ptr(gates_c), _ptr(dy),
                                                     _ptr(d_rows), _ptr(d_gates), T, rows_c.shape[0], k, rows_c.shape[1],
                                                     _stream(rows_c)), "cinn_moe_combine_backward")
-        _count()
         d_add = None if ctx.addend_dtype is None else dy.to(ctx.addend_dtype)
         return d_rows, None, d_gates.to(gates.dtype), d_add
 
@@ -840,7 +814,6 @@ def lightning_indexer_fused(q: torch.Tensor, k: torch.Tensor, w: torch.Tensor) -
         sw = (ctypes.c_int64 * 3)(*w.stride())
         _lib.check(_L.cinn_lightning_indexer(_ptr(q), _ptr(k), _ptr(w), _DTYPE_TAG[work], _ptr(out), B, Lq, Lk, H, d,
                                              sq, sk, sw, _stream(q)), "cinn_lightning_indexer")
-    _count()
     return out
 
 
@@ -859,7 +832,6 @@ def gather_quantized_rows(x_fp8: torch.Tensor, x_scale: torch.Tensor, idx: torch
         out_s = torch.empty((n_out, ns), dtype=torch.float32, device=x_fp8.device)
         _lib.check(_L.cinn_gather_rows(_ptr(x_fp8), _ptr(x_scale), _ptr(idx), _ptr(out_q), _ptr(out_s), n_out, n_src, d, ns,
                                        _stream(x_fp8)), "cinn_gather_rows")
-    _count()
     return out_q, out_s
 
 
@@ -883,7 +855,6 @@ def scatter_rows(rows: torch.Tensor, idx: torch.Tensor, n_out: int = None) -> to
         out = torch.empty((n_out, d), dtype=rows.dtype, device=rows.device)
         _lib.check(_L.cinn_scatter_rows(_ptr(rows), _ptr(idx), _ptr(out), n, n_out, row_bytes, _stream(rows)),
                    "cinn_scatter_rows")
-    _count()
     return out
 
 
@@ -899,7 +870,6 @@ def p2p_dispatch(x_fp8, x_scale, token_indices, sorted_experts, base_send, my_st
                                         _ptr(my_start), _ptr(peer_q), _ptr(peer_s), token_indices.numel(), n_tokens, d,
                                         x_scale.shape[1], experts_per_rank, n_ranks, capacity_rows, _stream(x_fp8)),
                    "cinn_p2p_dispatch")
-    _count()
 
 
 def p2p_dispatch_signal(x_fp8, x_scale, token_indices, sorted_experts, tables, buffers, e_lo: int = 0, e_hi: int = None,
@@ -921,7 +891,6 @@ def p2p_dispatch_signal(x_fp8, x_scale, token_indices, sorted_experts, tables, b
                                                b.LANDED_SLOT if flag_slot is None else flag_slot,
                                                b._call & 0x7FFFFFFF, _ptr(b.done), e_lo, e_local if e_hi is None else e_hi,
                                                int(n_sms), _stream(x_fp8)), "cinn_p2p_dispatch_signal")
-    _count()
 
 
 def p2p_row_table_wait(tables, buffers, n_rows: int, row_bytes: int, flag_slot: int = None) -> torch.Tensor:
@@ -937,7 +906,6 @@ def p2p_row_table_wait(tables, buffers, n_rows: int, row_bytes: int, flag_slot: 
                                               b._call & 0x7FFFFFFF,
                                               ctypes.c_void_p(torch.cuda.current_stream(dev).cuda_stream)),
                    "cinn_p2p_row_table_wait")
-    _count()
     return table
 
 
@@ -950,7 +918,6 @@ def p2p_return(rows, seg_start, home_base, peer_home, n_ranks: int, capacity_row
         _lib.check(_L.cinn_p2p_return(_ptr(rows), _ptr(seg_start), _ptr(home_base), _ptr(peer_home), rows.shape[0],
                                       rows.shape[1] * rows.element_size(), home_base.numel(), n_ranks, capacity_rows,
                                       _stream(rows)), "cinn_p2p_return")
-    _count()
 
 
 def moe_route(logits: torch.Tensor, bias: torch.Tensor, top_k: int):
@@ -984,7 +951,6 @@ def moe_route(logits: torch.Tensor, bias: torch.Tensor, top_k: int):
                                             _ptr(out["sorted_scores"]), _ptr(out["sorted_experts"]), _ptr(out["counts"]),
                                             _ptr(out["starts"]), _ptr(out["ends"]), _ptr(out["pair_pos"]), _ptr(out["pair_gate"]),
                                             _stream(logits)), "cinn_moe_route")
-    _count(3)
     return out
 
 
@@ -1002,7 +968,6 @@ def fp8_grouped_gemm_dgrad(dy_fp8, dy_scale, w_fp8, w_scale, expert_starts, expe
         _lib.check(_L.cinn_fp8_grouped_gemm_dgrad(_ptr(dy_fp8), _ptr(dy_scale), _ptr(w_fp8), _ptr(w_scale), _ptr(starts),
                                                   _ptr(ends), E, T, d_in, d_out, _ptr(dx), _DTYPE_TAG[out_dtype],
                                                   _stream(dy_fp8)), "cinn_fp8_grouped_gemm_dgrad")
-    _count(2)
     return dx
 
 
@@ -1042,7 +1007,6 @@ def fp8_grouped_wgrad(grad_out: torch.Tensor, x_fp8: torch.Tensor, x_scale: torc
                                                        out_tag, _DIV_MODE, _ptr(g_q) if one_pass else None,
                                                        _ptr(g_s) if one_pass else None, _stream(g)),
                        "cinn_fp8_grouped_wgrad_fused")
-        _count(4)
         if with_row_quant:
             return (grad_w, g_q, g_s) if one_pass else (grad_w, *quantize_fp8_rowwise(g, block_size=128))
         return grad_w
@@ -1057,7 +1021,6 @@ def fp8_grouped_wgrad(grad_out: torch.Tensor, x_fp8: torch.Tensor, x_scale: torc
                                              ctypes.c_void_p(starts_h.data_ptr()), ctypes.c_void_p(ends_h.data_ptr()), n_experts,
                                              T, d_in, d_out, _ptr(scratch), scratch.numel(), _ptr(grad_w), out_tag, _DIV_MODE,
                                              _stream(g)), "cinn_fp8_grouped_wgrad")
-    _count(3 * n_experts)
     if with_row_quant:
         return (grad_w, *quantize_fp8_rowwise(g, block_size=128))
     return grad_w
@@ -1100,7 +1063,6 @@ def grouped_gemm_16bit(sorted_x: torch.Tensor, weights: torch.Tensor, expert_sta
             out = torch.empty((T, d_out), dtype=out_dtype, device=x.device)
         _lib.check(_L.cinn_grouped_gemm_16bit(_ptr(x), _ptr(w), _DTYPE_TAG[x.dtype], _ptr(starts), _ptr(ends), E, T, d_in, d_out,
                                               _ptr(out), _DTYPE_TAG[out.dtype], _stream(x)), "cinn_grouped_gemm_16bit")
-    _count()
     return out
 
 

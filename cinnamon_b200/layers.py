@@ -6,7 +6,7 @@ Same constructors, parameter and buffer names (``routed_experts.w12`` / ``.w3``,
 moves between the two (with one rank; with expert parallelism ``routed_experts`` holds this rank's slice).  What
 differs is how the work is done:
 
-  * routing after the router GEMM is three launches on the device (``kernels.moe_route``): no sort / bincount / cumsum
+  * routing after the router GEMM is two or three launches on the device (``kernels.moe_route``): no sort / bincount / cumsum
     chain and no ``.item()`` synchronisation (the reference reads ``expert_counts.max()`` back, src/layers.py:151);
   * the routed experts are two differentiable grouped GEMMs on e4m3 operands with a one-kernel SwiGLU between them
     (the reference's grouped GEMM has no backward, so its routed experts receive no gradient on a GPU);

@@ -52,7 +52,7 @@ def router_logits(x: torch.Tensor, router_weight: torch.Tensor) -> torch.Tensor:
 def route(x: torch.Tensor, router_weight: torch.Tensor, expert_bias: torch.Tensor, top_k: int) -> Routing:
     """Router of ``MoE.forward`` (src/layers.py:122-148): sigmoid scores, top-k on
     scores + bias, gates normalised over the selected experts, pairs sorted by expert.
-    On a GPU everything after the router GEMM is three kernel launches (``kernels.moe_route``) with no host
+    On a GPU everything after the router GEMM is two or three kernel launches (``kernels.moe_route``) with no host
     synchronisation; on the CPU (host-logic tests) it is the reference's chain of torch calls."""
     n_experts = router_weight.shape[0]
     logits = router_logits(x, router_weight)

@@ -490,6 +490,9 @@ int cinn_moe_route_static(const float* logits, const float* bias, int64_t n_toke
  * until a GEMM has let go of an SM.  No reference counterpart (the reference's kernels are not persistent). */
 int cinn_set_gemm_sm_limit(int n_sms);
 
+/* Kernels this library has launched in this process so far (all threads and devices). */
+int64_t cinn_launch_count(void);
+
 /* Reads (and with reset != 0 clears) the device-side status word of the current device into the HOST int
  * *out.  0 means no kernel of this library has given up on a bounded wait since the last reset; any other
  * value is (role << 8) | reason.  This call synchronises with the device.  No counterpart in the reference,

@@ -296,3 +296,42 @@ def test_moe_layers_refuse_a_bias_left_on_the_host(K):
         with pytest.raises(AssertionError, match="CUDA"):
             serve(x[0].bfloat16())
         assert K.launch_count == n
+
+
+def test_launch_count_is_what_the_profiler_sees(K):
+    """``K.launch_count`` against the library's kernels in a profile: linears, routing with and without its scan, attention of
+    every type through tiles and gathers, the serving layer, a training step of the block."""
+    from torch.profiler import ProfilerActivity, profile
+    from cinnamon_b200 import layers, moe
+    with torch.device("cuda"):
+        lin = K.FP8Linear(512, 384)
+        block = K.convert_to_fp8(layers.MoE(8, 1, 2, 256, 1024, 2, 0.01, 0.01))
+        w = lambda *s: torch.randn(*s).bfloat16()                                             # noqa: E731
+        serve = moe.ExpertParallelMoE(w(8, 256).float(), torch.zeros(8), w(8, 256, 256), w(8, 256, 128), 2,
+                                      shared=moe.FP8SwiGLU(w(128, 256), w(128, 256), w(256, 128)))
+        x = torch.randn(2, 40, 256, requires_grad=True)
+        bias = torch.zeros(8)
+
+    def attention(dtype, d, mode):
+        before = K._L.cinn_set_sparse_attn_dense(mode)
+        q, k, v = (torch.randn(1, 2, 300, d, device="cuda", dtype=dtype, requires_grad=True) for _ in range(3))
+        out, _ = K.sparse_attention(q, k, v, torch.randint(0, 300, (1, 300, 16), device="cuda"))
+        out.sum().backward()
+        K._L.cinn_set_sparse_attn_dense(before)
+    calls = [lambda: lin(torch.randn(48, 512, device="cuda")).sum().backward(), lambda: block(x)[0].sum().backward(),
+             lambda: serve(x[0].detach().bfloat16()), lambda: K.moe_route(torch.randn(200, 8, device="cuda"), bias, 2),
+             lambda: K.moe_route(torch.randn(3000, 8, device="cuda"), bias, 2),
+             lambda: K.fp8_matmul_dsv3(K.quantize_fp8_rowwise(torch.randn(64, 8192, device="cuda"))[0],               # cut along K
+                                       K.quantize_fp8_blockwise(torch.randn(256, 8192, device="cuda"))[0].t(),
+                                       torch.ones(64, 64, device="cuda"), torch.ones(64, 2, device="cuda"))]
+    calls += [lambda dt=dt, d=d, mode=mode: attention(dt, d, mode) for dt in (torch.bfloat16, torch.float16, torch.float32)
+              for d in (64, 20) for mode in (0, 1)]
+    for i, call in enumerate(calls):
+        call()
+        torch.cuda.synchronize()
+        n = K.launch_count
+        with profile(activities=[ProfilerActivity.CPU, ProfilerActivity.CUDA]) as prof:
+            call()
+            torch.cuda.synchronize()
+        seen = [e.name for e in prof.events() if e.device_type.name == "CUDA" and "cinn::" in e.name]
+        assert K.launch_count - n == len(seen), (i, seen)
