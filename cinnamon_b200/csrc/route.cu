@@ -14,9 +14,6 @@
 //                         sorted_experts, the experts' row ranges, and per token its k rows in ascending order with their
 //                         gates (what the combine pass reads)
 //
-// Tokens per CTA: 8 (one per warp) as long as the histograms stay below 131072 counters, then 32 up to 262144, then 128.  Selecting the top k is a
-// serial chain of shuffles per token, so what counts is how many warps there are: 64 tokens in one CTA took 38 us.
-//
 // The workspace (one int per CTA and expert, and one more per expert) is the only memory beyond inputs and outputs.
 #include "common.cuh"
 #include <mutex>
@@ -25,10 +22,20 @@ namespace cinn {
 
 constexpr int ROUTE_MAX_TOKENS_PER_CTA = 128;
 constexpr int ROUTE_FEW_CTAS = 32;             // up to here the scatter kernel sums the histograms itself
+constexpr int64_t ROUTE_STATIC_MAX_INTS = 1 << 19;                     // 2 MiB: the built-in scratch (moe_route_static)
+
+// Tokens per CTA, a power of two: as few as one per warp while that is at most five CTAs per SM, more for more tokens.  Selecting
+// the top k is a serial chain of shuffles per token, so what counts is how many warps there are, until the histograms of every
+// CTA cost more than the chains save; five per SM is where the measured lines cross (us at 8 / 16 / 32 / 64 / 128 tokens per CTA:
+// 2048 tokens x 256 experts 27 / 29 / 41 / 66 / 116, 8192 x 64 37 / 31 / 31 / 39 / 64, 16384 x 256 82 / 67 / 64 / 78 / 121,
+// 32768 x 256 150 / 117 / 104 / 107 / 137, 131072 x 256 539 / 414 / 346 / 322 / 330).  (Any multiple of 8 instead: 24 and 72 tokens
+// are up to 11 % slower than 32 and 128 with 8 pairs a token, which the scatter takes 256 at a time.)  Fewer CTAs where their
+// histograms would not fit the built-in scratch, so that it serves what it serves at 128 tokens per CTA.
 static inline int route_tokens_per_cta(int64_t T, int E) {
-    if (T <= 8 * 1024 && (T + 7) / 8 * E <= 131072) return 8;
-    if (T <= 32 * 1024 && (T + 31) / 32 * E <= 262144) return 32;
-    return 128;
+    int64_t per = 8;
+    while (per < ROUTE_MAX_TOKENS_PER_CTA &&
+           (T > per * 5 * sm_count() || ((T + per - 1) / per + 1) * E > ROUTE_STATIC_MAX_INTS)) per *= 2;
+    return (int)per;
 }
 
 template <typename L> __device__ __forceinline__ float logit(L v);
@@ -299,7 +306,6 @@ int moe_route(const void* logits, int logits_dtype, const float* bias, int64_t T
 // a device share it, so two calls that overlap on that GPU (different streams, different threads) race; the
 // routing kernels overwrite every word they later read, so nothing has to be cleared between calls.
 // ---------------------------------------------------------------------------
-constexpr int64_t ROUTE_STATIC_MAX_INTS = 1 << 19;                     // 2 MiB
 static __device__ __align__(256) int g_route_scratch[ROUTE_STATIC_MAX_INTS];
 
 constexpr int ROUTE_MAX_DEVICES = 64;

@@ -70,6 +70,22 @@ def test_gemm_plans_under_a_cap_of_one_sm(built):
     assert p.returncode == 0, (p.returncode, p.stderr)
 
 
+def test_routing_workspace_keeps_what_the_built_in_scratch_serves(built):
+    """Tokens per CTA grow with the tokens, and the workspace fits the built-in scratch wherever it does at
+    the most tokens per CTA."""
+    from cinnamon_b200 import _lib
+    ints, limit = _lib.lib.cinn_moe_route_workspace_ints, _lib.lib.cinn_moe_route_static_max_ints()
+    for E in (1, 8, 33, 256, 511, 1024):
+        last = 0
+        for T in sorted({int(1.07 ** i) for i in range(1, 200)} | {8192, 8193, 32768, 32769, 65536, 65537}):
+            ctas = ints(T, E) // E - 1
+            per = -(-T // ctas)
+            assert ctas >= -(-T // 128) and per >= 0.9 * last, (T, E, ctas)
+            last = per if per > 8 else 0
+            if -(-T // 128) * E + E <= limit:
+                assert ints(T, E) <= limit, (T, E)
+
+
 def test_cpu_tensors_assert_like_the_reference(built):
     import torch
     from cinnamon_b200 import kernels as K

@@ -134,9 +134,9 @@ def test_route_kernel_matches_torch(K, T, E, k):
         assert torch.equal(got[key], again[key]), key
 
 
-@pytest.mark.parametrize("T,E,k", [(8, 256, 8), (256, 33, 2), (257, 256, 8), (5000, 64, 3), (8300, 1024, 4), (40000, 16, 2)])
+@pytest.mark.parametrize("T,E,k", [(8, 256, 8), (256, 33, 2), (257, 256, 8), (5000, 64, 3), (8300, 1024, 4), (40000, 16, 2), (131077, 8, 2)])
 def test_route_cta_sizes_and_row_ranges(K, T, E, k):
-    """8, 32 and 128 tokens per CTA, with and without the scan launch; 16-bit logits as their fp32 values; row ranges."""
+    """8, 16, 64 and 128 tokens per CTA, with and without the scan launch; 16-bit logits as their fp32 values; row ranges."""
     g = torch.Generator(device="cuda").manual_seed(T + E + k)
     logits = torch.randn(T, E, generator=g, device="cuda").bfloat16()
     bias = torch.randn(E, generator=g, device="cuda") * 0.3
