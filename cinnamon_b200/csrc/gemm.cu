@@ -727,8 +727,8 @@ static int launch_pair_out(const CUtensorMap& ta, const CUtensorMap& tb, GemmPar
     }
 }
 
-// Two-SM pairs serve dense problems with at least one 256 x 256 tile per pair of SMs (about 4 % faster than
-// the one-SM kernel there); CINN_GEMM_PAIR=0 keeps every problem on the one-SM kernel.
+// Two-SM pairs serve dense problems whose waves of 256 x 256 tiles cost no more than the one-SM kernel's (dense_plan), and
+// grouped ones with enough rows per expert; CINN_GEMM_PAIR=0 keeps every problem on the one-SM kernel.
 static int pair_mode() {
     static int mode = -1;
     if (mode < 0) {
@@ -808,7 +808,11 @@ struct DensePlan { bool pair; int splits; };
 
 // A K block of a tile costs about 0.45 us in either kernel (a pair of SMs does twice the rows in it), a tile about 3 us
 // around its K blocks.  Splitting adds a pass over the partial sums: about 3 us of launch and the bytes at the rate L2
-// returns them.  The plan with the smallest sum of these wins; measured figures stand at the callers' cases.
+// returns them.  The plan with the smallest sum of these wins.  Measured with cold operands, launch included: one tile alone 7.2 /
+// 12.3 / 34.3 us for 4 / 16 / 64 K blocks, a full wave of pairs 9.2 / 15.4 / 43.0, two waves 12.3 / 24.1 / 71.2; whole -> as
+// planned (M x N x K): 64 x 4096 x 7168 29.7 -> 16.3, 300 x 576 x 7168 29.7 -> 15.4 (B MN-major), 512 x 1024 x 32768 117 -> 31,
+// 16 x 18432 x 7168 38.9 -> 34.3, 128 x 512 x 2560 14.3 -> 12.8.  The demands (12 us, a gain of a tenth) leave the problems whole
+// where the second launch eats what is won: 1024 x 4096 x 4096 (22 us), 64 x 7168 x 2048 (12.8).
 static DensePlan dense_plan(int64_t M, int64_t N, int64_t K, int b_layout, int64_t workspace_bytes, int sms) {
     const int64_t KB = (K + BK - 1) / BK;
     auto waves = [](int64_t tiles, int64_t slots) { return (double)((tiles + slots - 1) / slots); };
