@@ -22,6 +22,28 @@ __device__ __forceinline__ bool wait_warp(uint32_t bar, uint32_t parity, volatil
     return __all_sync(0xffffffffu, mbar_wait_bounded(bar, parity, abort_flag, code, &g_attn_status));
 }
 
+// The MMA warp's end of a ring of panels.  (Asking for the next panel before this one's MMAs, so as to wait only if it is not
+// there, delays the MMAs: 320 to 350 cycles per panel of four where the plain wait takes the MMAs' own 256.)
+template <int RING> struct PanelRing {
+    uint32_t full0, empty0, base;
+    volatile int* abort_flag;
+    int code;
+    uint32_t slot, phase;
+    bool alive;
+    __device__ __forceinline__ PanelRing(uint32_t full, uint32_t empty, uint32_t panels, volatile int* flag, int reason)
+        : full0(full), empty0(empty), base(panels), abort_flag(flag), code(reason), slot(0), phase(0), alive(true) {}
+    // the next panel's address, and the slot to release once the MMAs that read it are issued
+    __device__ __forceinline__ bool next(uint32_t& addr, uint32_t& taken) {
+        if (!alive || !wait_warp(full0 + 8 * slot, phase, abort_flag, code)) return alive = false;
+        tc_fence_after();
+        addr = base + slot * PANEL;
+        taken = slot;
+        if (++slot == RING) { slot = 0; phase ^= 1u; }
+        return true;
+    }
+    __device__ __forceinline__ void release(uint32_t taken) { tc_commit(empty0 + 8 * taken); }
+};
+
 // The four warps of a warpgroup meet at a barrier in shared memory (four arrivals): bounded, so that a warp that gave up
 // leaves nobody behind.
 struct WarpgroupBarrier {
@@ -171,40 +193,139 @@ __device__ __forceinline__ void tile_of_block(int n_tiles, int BH, int group, in
     bh = g * group + r % heads;
 }
 
-constexpr int FWD_THREADS = 10 * 32;       // two softmax warpgroups, TMA warp, MMA warp
-
-// Shared memory: queries [part][64-column panel] | ring of panels | barriers.
+// Shared memory: queries [part][64-column panel] | ring of panels | barriers | row maxima on their way between two warps.
+// With one part two CTAs share an SM, each with one pair of softmax warpgroups: the first loads, the merge and the permutation of
+// one run under the other's tiles (a CTA of two pairs spent 20 000 of its 55 000 cycles on them, at 8 x 8 x 1531 queries of
+// 192).  Three parts of 192 columns need most of an SM's shared memory for the queries alone.
 template <int NS, int ND> struct FwdShape {
+    static constexpr int PAIRS = NS > 1 ? 2 : 1;           // of softmax warpgroups
+    static constexpr int THREADS = (8 * PAIRS + 2) * 32;   // and a TMA warp, an MMA warp
     static constexpr int Q_PANELS = NS * ND;
-    static constexpr int RING = (Q_PANELS > 6 ? 4 : 6);
+    static constexpr int RING = NS > 1 ? (Q_PANELS > 6 ? 4 : 6) : 6 - Q_PANELS;
     static constexpr int BAR_OFF = (Q_PANELS + RING) * PANEL;
-    static constexpr int BYTES = BAR_OFF + 256 + 1024 + T * 4;
+    static constexpr int PAIR_OFF = BAR_OFF + 512;         // [round & 1][pair][half][row]
+    static constexpr int LSE_OFF = PAIR_OFF + 4 * PAIRS * T * 4;
+    static constexpr int BYTES = LSE_OFF + T * 4 + 1024;
 };
 
-// One CTA: 128 queries of one head and 64 value columns (blockIdx.z), over all key tiles up to the queries' own.  The two
-// softmax warpgroups take alternate key tiles, each with its own running maximum, sum and output accumulator, and merge
-// at the end: neither waits for the other, and while one turns scores into probabilities the tensor core works for the
-// other.  A thread owns a query.  It reads its 128 scores from tensor memory twice, 32 at a time: for the maximum of those
-// the query picked, whose raw values it leaves in the probabilities' output (by rank; permuted and normalised at the end),
-// and to write exp(score - max) back as three bf16 parts, the A operand of P V, in the columns it has just read and 64
-// beside them.  (Keeping the 128 scores in registers spilled, and with the operands in shared memory there is hardly an L1
-// for the spills: 1.3 ms where this takes 0.68, 32 x 8 x 1024 queries of 192 in fp32.)  256 of the 512 columns per warpgroup: 128 scores, 64 leading parts, 64 of
-// output.
+// 16 columns of a thread's row: scores to probabilities relative to `m`, left as parts over the scores and beside them.  The
+// picked raw scores go to rows + at (bytes) in passing when PUSH.  (32 columns at a time spilled.)
+template <bool PUSH>
+__device__ __forceinline__ void softmax_chunk(uint32_t t_s, uint32_t t_lead, uint32_t bit, float scale, float m, bool repeats,
+                                              const uint8_t*& count, float* rows, uint32_t& at, uint64_t (&l)[2]) {
+    uint32_t v[16];
+    float p[16];
+    ld16(t_s, v);
+    ld_wait();
+    const uint64_t sc = pair2(scale, scale), off = pair2(-m, -m), l2e = pair2(1.4426950408889634f, 1.4426950408889634f);
+#pragma unroll
+    for (int i = 0; i < 16; i += 2) {
+        unpair2(mul2(fma2(pair2(__uint_as_float(v[i]), __uint_as_float(v[i + 1])), sc, off), l2e), p[i], p[i + 1]);
+#pragma unroll
+        for (int e = i; e < i + 2; ++e) {
+            p[e] = exp2_fast(p[e]);
+            if constexpr (PUSH) push_if(bit, 1u << e, rows, at, __uint_as_float(v[e]), p[e]);
+            else p[e] = bit & (1u << e) ? p[e] : 0.0f;
+        }
+    }
+    if (repeats) {                                        // a key picked several times counts as often
+#pragma unroll
+        for (int i = 0; i < 16; ++i)
+            if (bit & (1u << i)) p[i] *= (float)*count++;
+    }
+#pragma unroll
+    for (int i = 0; i < 16; i += 2) l[(i >> 1) & 1] = add2(l[(i >> 1) & 1], pair2(p[i], p[i + 1]));
+    store_parts16(t_s, t_lead, p);
+}
+
+// Raw scores by rank -> probabilities by slot, in place: rows of K slots, one warp of WARPS.  Every slot of a row is read
+// before any of it is written.
+template <int WARPS>
+__device__ __forceinline__ void by_slot(const uint16_t* rank, float* attn, const float* lse, int rows, int K, float scale, int warp, int lane) {
+    if (K >= 4 && K <= 512 && (K & (K - 1)) == 0) {
+        // whole rows in batches of 512 slots, four in a row per lane and load
+        const int log_k = 31 - __clz(K), end = rows << log_k;
+#pragma unroll 1
+        for (int e0 = warp * 512; e0 < end; e0 += WARPS * 512) {
+            uint2 c[4];
+            float4 x[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) c[u] = __ldg(reinterpret_cast<const uint2*>(rank + min(e0 + u * 128 + lane * 4, end - 4)));
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                const int e = min(e0 + u * 128 + lane * 4, end - 4), row = e >> log_k;
+                const float* from = attn + (row << log_k);
+                const float z = lse[row];
+                auto one = [&](uint32_t at) {
+                    const float s = from[min((int)at, K - 1)];
+                    return at == 0xffffu ? 0.0f : exp_fast(s * scale - z);
+                };
+                x[u] = make_float4(one(c[u].x & 0xffffu), one(c[u].x >> 16), one(c[u].y & 0xffffu), one(c[u].y >> 16));
+            }
+            __syncwarp();
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                const int e = e0 + u * 128 + lane * 4;
+                if (e < end) *reinterpret_cast<float4*>(attn + e) = x[u];
+            }
+        }
+        return;
+    }
+    // a warp takes sixteen pieces of 32 slots at a time with all loads in flight
+    constexpr int U = MAX_SLOTS / 32;
+    const int chunks = (K + 31) / 32, per = U / chunks;
+    for (int k0 = warp; k0 < rows; k0 += WARPS * per) {                     // rows k0, k0 + WARPS, ...
+        float v[U];
+        uint32_t c[U];
+        int rr = k0, j = lane;                            // piece u of the batch: its row and this lane's slot
+        auto advance = [&] { if ((j += 32) >= chunks * 32) { j = lane; rr += WARPS; } };
+        const int end = min(rows, k0 + WARPS * per);
+#pragma unroll
+        for (int u = 0; u < U; ++u, advance()) {
+            // (loads from clamped places and a choice afterwards: behind a condition they would go one by one)
+            const uint32_t x = rank[min(rr, end - 1) * K + min(j, K - 1)];
+            c[u] = rr < end && j < K ? x : 0xffffu;
+        }
+        rr = k0; j = lane;
+#pragma unroll
+        for (int u = 0; u < U; ++u, advance()) {
+            const float x = attn[min(rr, end - 1) * K + min((int)c[u], K - 1)] * scale;
+            v[u] = c[u] != 0xffffu ? x : -INFINITY;
+        }
+        __syncwarp();
+        rr = k0; j = lane;
+#pragma unroll
+        for (int u = 0; u < U; ++u, advance())
+            if (rr < end && j < K) attn[rr * K + j] = exp_fast(v[u] - lse[rr]);
+    }
+}
+
+// One CTA: 128 queries of one head and 64 value columns (blockIdx.z), over all key tiles up to the queries' own.  A pair of
+// softmax warpgroups takes a key tile, a thread a query and half of the tile's keys; two pairs (of one CTA, which merge their
+// maxima, sums and outputs at the end, or of two) keep out of each other's way, and while one turns scores into probabilities the
+// tensor core works for the other.  A thread reads its 64 scores from tensor memory twice: for the maximum,
+// which it exchanges with the thread of the other half, and to write exp(score - max) back as three bf16 parts, the A operand
+// of P V, in the columns it has just read and 32 beside them, leaving the raw scores of the picked keys in the probabilities'
+// output (by rank; permuted and normalised at the end).  256 columns per pair: 128 scores, 64 leading parts, 64 of output.
+// Bound by the instructions per score and what hides their latency: FIG
 // NS: bf16 parts of q, k, v; ND: 64-column panels of q and k.
 template <int NS, int ND>
-__global__ void __launch_bounds__(FWD_THREADS, 1)
+__global__ void __launch_bounds__(FwdShape<NS, ND>::THREADS, 3 - FwdShape<NS, ND>::PAIRS)
 attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                 const __grid_constant__ CUtensorMap tmV, const FwdArgs a) {
     using S = FwdShape<NS, ND>;
+    constexpr int PAIRS = S::PAIRS, TMA_WARP = 8 * PAIRS, MMA_WARP = TMA_WARP + 1;
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
     const uint32_t sq = smem_u32(smem), ring = sq + S::Q_PANELS * PANEL;
     uint64_t* bars = reinterpret_cast<uint64_t*>(smem + S::BAR_OFF);
     const uint32_t full0 = smem_u32(bars), empty0 = smem_u32(bars + S::RING), qfull = smem_u32(bars + 2 * S::RING);
     const uint32_t sfull0 = qfull + 8, pready0 = qfull + 24, odone0 = qfull + 40;       // two each
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * S::RING + 7);
+    const uint32_t pair0 = odone0 + 16;                   // eight, one per two warps that share rows
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * S::RING + 15);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
-    float* s_lse = reinterpret_cast<float*>(smem + S::BAR_OFF + 256);
+    float* s_pair = reinterpret_cast<float*>(smem + S::PAIR_OFF);
+    float* s_lse = reinterpret_cast<float*>(smem + S::LSE_OFF);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     int qt, bh;
     tile_of_block(a.n_tiles, a.BH, a.group, qt, bh);
@@ -214,16 +335,17 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         *abort_flag = 0;
         for (int i = 0; i < S::RING; ++i) { mbar_init(full0 + 8 * i, 1); mbar_init(empty0 + 8 * i, 1); }
         mbar_init(qfull, 1);
-        for (int i = 0; i < 2; ++i) { mbar_init(sfull0 + 8 * i, 1); mbar_init(pready0 + 8 * i, 4); mbar_init(odone0 + 8 * i, 1); }
+        for (int i = 0; i < 2; ++i) { mbar_init(sfull0 + 8 * i, 1); mbar_init(pready0 + 8 * i, 8); mbar_init(odone0 + 8 * i, 1); }
+        for (int i = 0; i < 8; ++i) mbar_init(pair0 + 8 * i, 2);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    if (warp == 9) tc_alloc(smem_u32(tmem_slot), 512);
+    if (warp == MMA_WARP) tc_alloc(smem_u32(tmem_slot), 256 * PAIRS);
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
 
-    if (warp == 8) {
+    if (warp == TMA_WARP) {
         if (lane == 0) {
             mbar_expect_tx(qfull, S::Q_PANELS * PANEL);
             for (int p = 0; p < NS; ++p)
@@ -237,335 +359,313 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
                 tma_load_3d(m, full0 + 8 * s, ring + s * PANEL, x, y, z);
                 ++it;
             };
-            for (int j = 0; j <= n && alive; ++j) {
-                if (j < n) {
-                    if constexpr (NS > 1)
-                        for (int c = 0; c < ND; ++c)
-                            for (int p = NS - 1; p >= 0; --p) fetch(&tmK, c * 64, j * T, p * a.BH + bh);
-                    for (int c = 0; c < ND; ++c) fetch(&tmK, c * 64, j * T, bh);
-                }
+            auto keys = [&](int j) {
+                if constexpr (NS > 1)
+                    for (int c = 0; c < ND; ++c)
+                        for (int p = NS - 1; p >= 0; --p) fetch(&tmK, c * 64, j * T, p * a.BH + bh);
+                for (int c = 0; c < ND; ++c) fetch(&tmK, c * 64, j * T, bh);
+            };
+            for (int j = 0; j <= n && alive; ++j) {       // in the order in which the MMA warp takes them
+                if (PAIRS > 1 && j < n) keys(j);
                 if (j > 0)
                     for (int p = NS - 1; p >= 0; --p) fetch(&tmV, half * 64, (j - 1) * T, p * a.BH + bh);
+                if (PAIRS == 1 && j < n) keys(j);
             }
             if (!alive) {                                 // abandoned: let the copies in flight land
                 const long long t0 = clock64();
                 while (clock64() - t0 < 2000000LL) { }
             }
         }
-    } else if (warp == 9) {
+    } else if (warp == MMA_WARP) {
         if (wait_warp(qfull, 0, abort_flag, (8 << 8) | 2)) {
             constexpr uint32_t id_s = make_idesc_f16(true, T, T), id_o = make_idesc_f16(true, T, 64, false, true);
-            uint32_t it = 0;
-            bool alive = true;
-            auto panel = [&](uint32_t& addr) {
-                const uint32_t s = it % S::RING;
-                if (!alive || !wait_warp(full0 + 8 * s, (it / S::RING) & 1, abort_flag, (8 << 8) | 3)) alive = false;
-                addr = ring + s * PANEL;
-                tc_fence_after();
+            PanelRing<S::RING> panels(full0, empty0, ring, abort_flag, (8 << 8) | 3);
+            // scores of key tile j, over the probabilities of the pair's tile before, whose product was issued before
+            auto scores = [&](int j) {
+                const uint32_t d = tmem + j % PAIRS * 256;
+                bool first = true;
+                // query parts [x_lo, x_hi] of column panel c against the ring's next key panel
+                auto product = [&](int c, int x_hi, int x_lo) {
+                    uint32_t kp, slot;
+                    if (!panels.next(kp, slot)) return;
+                    const uint32_t kd = panel_desc(kp);
+                    uint32_t qd = panel_desc(sq + c * PANEL) + x_hi * ND * (PANEL >> 4);
+                    for (int x = x_hi; x >= x_lo; --x) {
+                        mma_panels(d, qd, kd, id_s, first);
+                        first = false;
+                        qd -= ND * (PANEL >> 4);
+                    }
+                    panels.release(slot);
+                };
+                // The tensor core truncates the running sum at every step, so the small products go first and the leading
+                // ones, for which the keys' leading parts are fetched again, last: ND x 4 truncations at full size instead of
+                // six times as many.
+                if constexpr (NS > 1)
+                    for (int c = 0; c < ND; ++c)
+                        for (int p = NS - 1; p >= 0; --p) product(c, NS - 1 - p, p == 0 ? 1 : 0);
+                for (int c = 0; c < ND; ++c) product(c, 0, 0);
+                tc_commit(sfull0 + 8 * (j % PAIRS));
             };
-            for (int j = 0; j <= n && alive; ++j) {
-                if (j < n) {                              // scores of key tile j (over the probabilities of j - 2, whose product
-                    const uint32_t d = tmem + (j & 1) * 256;            // was issued before)
-                    bool first = true;
-                    // query parts [x_lo, x_hi] of column panel c against the ring's next key panel
-                    auto product = [&](int c, int x_hi, int x_lo) {
-                        uint32_t kp;
-                        panel(kp);
-                        if (!alive) return;
-                        const uint64_t kd = panel_desc(kp);
-                        uint64_t qd = panel_desc(sq + c * PANEL) + (uint64_t)(x_hi * ND * (PANEL >> 4));
-                        for (int x = x_hi; x >= x_lo; --x) {
-                            mma_panels(d, qd, kd, id_s, first);
-                            first = false;
-                            qd -= ND * (PANEL >> 4);
-                        }
-                        tc_commit(empty0 + 8 * (it % S::RING));
-                        ++it;
-                    };
-                    // The tensor core truncates the running sum at every step, so the small products go first and the
-                    // leading ones, for which the keys' leading parts are fetched again, last: ND x 4 truncations at full
-                    // size instead of six times as many.
-                    if constexpr (NS > 1)
-                        for (int c = 0; c < ND && alive; ++c)
-                            for (int p = NS - 1; p >= 0 && alive; --p) product(c, NS - 1 - p, p == 0 ? 1 : 0);
-                    for (int c = 0; c < ND && alive; ++c) product(c, 0, 0);
-                    tc_commit(sfull0 + 8 * (j & 1));
-                }
-                if (j > 0 && alive) {                     // output of key tile j - 1
-                    const int i = j - 1, w = i & 1;
-                    if (!wait_warp(pready0 + 8 * w, (i >> 1) & 1, abort_flag, (8 << 8) | 4)) { alive = false; break; }
+            for (int j = 0; j <= n && panels.alive; ++j) {
+                if (PAIRS > 1 && j < n) scores(j);
+                if (j > 0 && panels.alive) {              // output of key tile j - 1
+                    const int i = j - 1, w = i % PAIRS;
+                    if (!wait_warp(pready0 + 8 * w, (i / PAIRS) & 1, abort_flag, (8 << 8) | 4)) break;
                     tc_fence_after();
                     const uint32_t base = tmem + w * 256;
-                    bool first = NS > 1 || i < 2;
-                    for (int p = NS - 1; p >= 0 && alive; --p) {
-                        uint32_t vp;
-                        panel(vp);
-                        if (!alive) break;
-                        const uint64_t vd = panel_desc(vp);
+                    bool first = NS > 1 || i < PAIRS;
+                    for (int p = NS - 1; p >= 0; --p) {
+                        uint32_t vp, slot;
+                        if (!panels.next(vp, slot)) break;
+                        const uint32_t vd = panel_desc(vp);
                         if (p == 0) { mma_part_at<2>(base + 192, base, base + 128, vd, id_o, first); first = false; }
                         if (p <= 1) { mma_part_at<1>(base + 192, base, base + 128, vd, id_o, first); first = false; }
                         mma_part_at<0>(base + 192, base, base + 128, vd, id_o, first);
                         first = false;
-                        tc_commit(empty0 + 8 * (it % S::RING));
-                        ++it;
+                        panels.release(slot);
                     }
-                    if (i + 2 >= n) tc_commit(odone0 + 8 * w);
+                    if (i + PAIRS >= n) tc_commit(odone0 + 8 * w);
                 }
+                if (PAIRS == 1 && j < n) scores(j);
             }
         }
     } else {
-        const int wg = warp >> 2, quarter = warp & 3, r = quarter * 32 + lane;
+        const int pair = warp >> 3, h = (warp >> 2) & 1, quarter = warp & 3, r = quarter * 32 + lane;
         const int t = q0 + r, b = bh / a.H;
         const bool live = t < a.L;
-        const uint32_t base = tmem + ((uint32_t)(quarter * 32) << 16) + wg * 256;
+        const uint32_t base = tmem + ((uint32_t)(quarter * 32) << 16) + pair * 256;
+        const uint32_t t_s = base + h * 64, t_lead = base + 128 + h * 32, t_o = base + 192 + h * 32;      // this half's
         const int64_t qrow = (int64_t)b * a.L + min(t, a.L - 1);
         const uint4* bits = reinterpret_cast<const uint4*>(a.picks.bits + qrow * a.words);
+        const uint16_t* before = a.picks.before + qrow * a.words + h * 2;
         const bool repeats = a.picks.repeats[b * n_qt + qt] != 0;
-        float* raw = a.attn + ((int64_t)bh * a.L + min(t, a.L - 1)) * a.K;          // the next picked key's raw score goes here
-        const uint8_t* count = a.picks.count + qrow * a.K;
-        const uint32_t push_mask = half == 0 ? ~0u : 0u;  // one of the column halves writes the scores
-        float m = -INFINITY, l = 0.0f;
+        float* rows = a.attn + (int64_t)bh * a.L * a.K;
+        const uint32_t row_at = (uint32_t)min(t, a.L - 1) * (uint32_t)a.K;
+        const uint8_t* counts = a.picks.count + qrow * a.K;
+        float m = -INFINITY;
+        uint64_t l2[2] = {0u, 0u};                        // (0, 0) each
         // With three parts a tile's output is added up here, rounded to nearest: the tensor core truncates, and over a long
         // row of tiles that would show in fp32.
         constexpr bool KEEP = NS > 1;
-        float o_sum[KEEP ? 64 : 1];
+        uint64_t o_sum[KEEP ? 16 : 1];
 #pragma unroll
-        for (int i = 0; i < (KEEP ? 64 : 1); ++i) o_sum[i] = 0.0f;
+        for (int i = 0; i < (KEEP ? 16 : 1); ++i) o_sum[i] = 0u;
         auto add_output = [&] {
 #pragma unroll
-            for (int c = 0; c < 4; ++c) {
+            for (int c = 0; c < 2; ++c) {
                 float o[16];
-                tc_ld16(base + 192 + c * 16, o);
+                tc_ld16(t_o + c * 16, o);
 #pragma unroll
-                for (int i = 0; i < 16; ++i) o_sum[(KEEP ? c * 16 + i : 0)] += o[i];
+                for (int i = 0; i < 8; ++i) {
+                    uint64_t& sum = o_sum[KEEP ? c * 8 + i : 0];
+                    sum = add2(sum, pair2(o[2 * i], o[2 * i + 1]));
+                }
             }
         };
         bool alive = true;
-        auto picked = [](const uint4& w) { return __popc(w.x) + __popc(w.y) + __popc(w.z) + __popc(w.w); };
+        // the larger of both halves' values, in both
+        uint32_t rounds = 0;
+        const uint32_t pair_bar = pair0 + 8 * (pair * 4 + quarter);
+        auto exchange = [&](float& x) {
+            float* slot = s_pair + ((rounds & 1) * PAIRS + pair) * 2 * T + r;
+            slot[h * T] = x;
+            __syncwarp();
+            if (lane == 0) mbar_arrive(pair_bar);
+            if (!wait_warp(pair_bar, rounds & 1, abort_flag, (8 << 8) | 7)) return false;
+            x = fmaxf(x, slot[(h ^ 1) * T]);
+            ++rounds;
+            return true;
+        };
         const uint4 none = make_uint4(0u, 0u, 0u, 0u);
-        if (wg == 1 && live) {                            // the other warpgroup's tiles hold ranks as well
-            const int skip = picked(__ldg(bits));
-            raw += skip; count += skip;
-        }
-        uint4 mine = live && wg < n ? __ldg(bits + wg) : none;
-        for (int j = wg; j < n; j += 2) {
+        uint4 mine = live && pair < n ? __ldg(bits + pair) : none;
+        uint32_t rank = pair < n ? __ldg(before + pair * 4) : 0u;
+        const uint64_t scale2 = pair2(a.scale, a.scale);
+        for (int j = pair; j < n; j += PAIRS) {
             const uint4 cur = mine;
-            // bits of the next tile of either warpgroup, in flight during this one
-            const uint4 next = live && j + 1 < n ? __ldg(bits + j + 1) : none;
-            mine = live && j + 2 < n ? __ldg(bits + j + 2) : none;
-            if (!wait_warp(sfull0 + 8 * wg, (j >> 1) & 1, abort_flag, (8 << 8) | 5)) { alive = false; break; }
+            uint32_t at = (row_at + rank) * 4;
+            const uint8_t* count = counts + rank;
+            if (j + PAIRS < n) {                          // the next tile's, in flight during this one
+                mine = live ? __ldg(bits + j + PAIRS) : none;
+                rank = __ldg(before + (j + PAIRS) * 4);
+            }
+            if (!wait_warp(sfull0 + 8 * pair, (j / PAIRS) & 1, abort_flag, (8 << 8) | 5)) { alive = false; break; }
             tc_fence_after();
             if constexpr (KEEP)
-                if (j >= 2) add_output();                 // of tile j - 2, issued before these scores
-            // (one chunk of 32 columns per round and no further unrolling: unrolled, the two passes overran the
-            // instruction cache)
-            float mx[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
-            uint4 w = cur;
+                if (j >= PAIRS) add_output();             // of the pair's tile before, issued before these scores
+            // The reference point of the exponentials moves only when a picked score exceeds it by 5: sums stay below e^5 x K
+            // and nothing is lost, the output is rescaled once or twice in a row's life.  The maximum of all the tile's scores
+            // is cheaper than that of the picked ones (one instruction per score, not three) and says most times that no
+            // row's point has to move.
+            bool look = j < PAIRS;
+            if (!look) {
+                float mx[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
 #pragma unroll 1
-            for (int c = 0; c < 4; ++c) {
-                uint32_t v[32];
-                ld32(base + c * 32, v);
-                ld_wait();
-                const uint32_t bit = w.x;
-                w = make_uint4(w.y, w.z, w.w, 0u);
-                const uint32_t push = bit & push_mask;
-                uint32_t at = 0;
+                for (int c = 0; c < 2; ++c) {
+                    uint32_t v[32];
+                    ld32(t_s + c * 32, v);
+                    ld_wait();
 #pragma unroll
-                for (int i = 0; i < 32; ++i) {
-                    const float x = __uint_as_float(v[i]) * a.scale;
-                    mx[i & 3] = fmaxf(mx[i & 3], bit & (1u << i) ? x : -INFINITY);
-                    store_if(raw + at, x, push & (1u << i));
-                    at += (bit >> i) & 1u;
+                    for (int i = 0; i < 32; i += 2) {
+                        float x, y;
+                        unpair2(mul2(pair2(__uint_as_float(v[i]), __uint_as_float(v[i + 1])), scale2), x, y);
+                        mx[(i >> 1) & 3] = fmaxf(mx[(i >> 1) & 3], fmaxf(x, y));
+                    }
                 }
-                raw += at;
+                float top = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3]));
+                if (!exchange(top)) { alive = false; break; }
+                look = __any_sync(0xffffffffu, (cur.x | cur.y | cur.z | cur.w) != 0u && !(top <= m + 5.0f));
             }
-            const float mt = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3]));
-            const uint8_t* count0 = count;
-            {
-                const int skip = picked(next);
-                raw += skip;
-                count += picked(cur) + skip;
-            }
-            // The reference point of the exponentials moves only when a score exceeds it by 5: sums stay below e^5 x K and
-            // nothing is lost, the output is rescaled once or twice in a row's life.
-            const bool move = mt > m + 5.0f || (m == -INFINITY && mt > -INFINITY);
-            if (__any_sync(0xffffffffu, move)) {
-                const float mn = move ? mt : m;
-                const float f = m == -INFINITY ? 0.0f : __expf(m - mn);
-                m = mn;
-                l *= f;
-                if constexpr (KEEP) {
+            if (look) {
+                float mx[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+#pragma unroll 1
+                for (int c = 0; c < 2; ++c) {
+                    uint32_t v[32];
+                    ld32(t_s + c * 32, v);
+                    ld_wait();
+                    const uint32_t bit = c == 0 ? (h ? cur.z : cur.x) : (h ? cur.w : cur.y);
 #pragma unroll
-                    for (int i = 0; i < 64; ++i) o_sum[i] *= f;
-                } else if (j >= 2) {
+                    for (int i = 0; i < 32; ++i) mx[i & 3] = fmaxf(mx[i & 3], bit & (1u << i) ? __uint_as_float(v[i]) * a.scale : -INFINITY);
+                }
+                float mt = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3]));
+                if (!exchange(mt)) { alive = false; break; }
+                const bool move = mt > m + 5.0f || (m == -INFINITY && mt > -INFINITY);
+                if (__any_sync(0xffffffffu, move)) {
+                    const float mn = move ? mt : m;
+                    const float f = m == -INFINITY ? 0.0f : __expf(m - mn);
+                    const uint64_t f2 = pair2(f, f);
+                    m = mn;
+                    l2[0] = mul2(l2[0], f2);
+                    l2[1] = mul2(l2[1], f2);
+                    if constexpr (KEEP) {
 #pragma unroll
-                    for (int c = 0; c < 4; ++c) {
-                        float o[16];
-                        uint32_t w[16];
-                        tc_ld16(base + 192 + c * 16, o);
+                        for (int i = 0; i < 16; ++i) o_sum[i] = mul2(o_sum[i], f2);
+                    } else if (j >= PAIRS) {
 #pragma unroll
-                        for (int i = 0; i < 16; ++i) w[i] = __float_as_uint(o[i] * f);
-                        st16(base + 192 + c * 16, w);
+                        for (int c = 0; c < 2; ++c) {
+                            float o[16];
+                            uint32_t w[16];
+                            tc_ld16(t_o + c * 16, o);
+#pragma unroll
+                            for (int i = 0; i < 16; ++i) w[i] = __float_as_uint(o[i] * f);
+                            st16(t_o + c * 16, w);
+                        }
                     }
                 }
             }
             const float mu = m == -INFINITY ? 0.0f : m;
-            w = cur;
 #pragma unroll 1
             for (int c = 0; c < 4; ++c) {
-                uint32_t v[32];
-                float p[32];
-                ld32(base + c * 32, v);
-                ld_wait();
-                const uint32_t bit = w.x;
-                w = make_uint4(w.y, w.z, w.w, 0u);
-#pragma unroll
-                for (int i = 0; i < 32; ++i) p[i] = exp_fast(bit & (1u << i) ? fmaf(__uint_as_float(v[i]), a.scale, -mu) : -INFINITY);
-                if (repeats) {                            // a key picked several times counts as often
-#pragma unroll
-                    for (int i = 0; i < 32; ++i)
-                        if (bit & (1u << i)) p[i] *= (float)*count0++;
-                }
-#pragma unroll
-                for (int i = 0; i < 32; i += 4) l += (p[i] + p[i + 1]) + (p[i + 2] + p[i + 3]);
-                // over the 32 scores just read go the second and third parts, the leading parts beside the scores
-                store_parts32(base + c * 32, base + 128 + c * 16, p);
+                const uint32_t bit = (c < 2 ? (h ? cur.z : cur.x) : (h ? cur.w : cur.y)) >> (c & 1) * 16;
+                if (half == 0) softmax_chunk<true>(t_s + c * 16, t_lead + c * 8, bit, a.scale, mu, repeats, count, rows, at, l2);
+                else softmax_chunk<false>(t_s + c * 16, t_lead + c * 8, bit, a.scale, mu, repeats, count, rows, at, l2);
             }
             st_wait();
             tc_fence_before();
             __syncwarp();
-            if (lane == 0) mbar_arrive(pready0 + 8 * wg);
+            if (lane == 0) mbar_arrive(pready0 + 8 * pair);
         }
-        const bool ran = n > wg;
-        for (int i = 0; i < min(n, 2) && alive; ++i) {                  // every product has been added, no panel is read any more
+        const bool ran = n > pair;
+        for (int i = 0; i < min(n, PAIRS) && alive; ++i) {                  // every product has been added, no panel is read any more
             alive = wait_warp(odone0 + 8 * i, 0, abort_flag, (8 << 8) | 6);
         }
         tc_fence_after();
-        if constexpr (KEEP)
+        float o[32];
+        if constexpr (KEEP) {
             if (ran && alive) add_output();
-        // merge: the second warpgroup leaves its state in the operand panels
-        float* merge = reinterpret_cast<float*>(smem);                   // [66][128], column r: conflict-free
-        if (wg == 1) {
-            merge[64 * T + r] = ran ? m : -INFINITY;
-            merge[65 * T + r] = l;
+#pragma unroll
+            for (int i = 0; i < 16; ++i) unpair2(o_sum[i], o[2 * i], o[2 * i + 1]);
+        } else {
+            uint32_t v[32];
+            ld32(t_o, v);
+            ld_wait();
+#pragma unroll
+            for (int i = 0; i < 32; ++i) o[i] = __uint_as_float(v[i]);
+        }
+        float l;
+        {
+            float x, y;
+            unpair2(add2(l2[0], l2[1]), x, y);
+            l = x + y;
+        }
+        // merge: each half leaves its sum in the operand panels, a second pair all its state
+        float* merge = reinterpret_cast<float*>(smem);                   // [69][128], column r: conflict-free
+        merge[(65 + pair * 2 + h) * T + r] = l;
+        if (PAIRS > 1 && pair == 1) {
+            if (h == 0) merge[64 * T + r] = ran ? m : -INFINITY;
             if (ran && alive) {
 #pragma unroll
-                for (int c = 0; c < 4; ++c) {
-                    float o[16];
-                    if constexpr (KEEP) {
-#pragma unroll
-                        for (int i = 0; i < 16; ++i) o[i] = o_sum[c * 16 + i];
-                    } else {
-                        tc_ld16(base + 192 + c * 16, o);
-                    }
-#pragma unroll
-                    for (int i = 0; i < 16; ++i) merge[(c * 16 + i) * T + r] = o[i];
-                }
+                for (int i = 0; i < 32; ++i) merge[(h * 32 + i) * T + r] = o[i];
             }
         }
-        asm volatile("bar.sync 1, 256;" ::: "memory");
-        if (wg == 0) {
-            const float m1 = merge[64 * T + r], l1 = merge[65 * T + r];
+        asm volatile("bar.sync 1, %0;" ::"n"(256 * PAIRS) : "memory");
+        if (pair == 0) {
+            const float l0 = merge[65 * T + r] + merge[66 * T + r];
+            const float m1 = PAIRS > 1 ? merge[64 * T + r] : -INFINITY, l1 = PAIRS > 1 ? merge[67 * T + r] + merge[68 * T + r] : 0.0f;
             const float mm = fmaxf(m, m1);
             const float f0 = m == -INFINITY ? 0.0f : __expf(m - mm), f1 = m1 == -INFINITY ? 0.0f : __expf(m1 - mm);
-            const float sum = l * f0 + l1 * f1;
+            const float sum = l0 * f0 + l1 * f1;
             const float inv = sum > 0.0f ? 1.0f / sum : 0.0f;
             const float lse = sum > 0.0f ? mm + logf(sum) : 0.0f;
-            s_lse[r] = lse;
-            // (no finite result can hide a sum that is not a number: with NaN scores only, the second warpgroup's maximum stays
+            // (no finite result can hide a sum that is not a number: with NaN scores only, the second pair's maximum stays
             // at -inf and its output is left out below)
             bool bad = sum != sum;
-            const int cols = min(64, a.Dv - half * 64);
-            float* orow = a.out + ((int64_t)bh * a.L + t) * a.Dv + half * 64;
+            const int col0 = half * 64 + h * 32, cols = min(32, a.Dv - col0);
+            const int64_t orow = ((int64_t)bh * a.L + t) * a.Dv + col0;
 #pragma unroll
-            for (int c = 0; c < 4; ++c) {
-                float o[16];
-                if constexpr (KEEP) {
+            for (int i = 0; i < 32; ++i) {
+                const float o1 = m1 == -INFINITY ? 0.0f : merge[(h * 32 + i) * T + r] * f1;
+                o[i] = (o[i] * f0 + o1) * inv;
+                bad |= !(fabsf(o[i]) <= 3.4e38f);
+            }
+            if (live && alive && cols > 0) {
+                if (cols == 32 && (a.Dv & 3) == 0) {
 #pragma unroll
-                    for (int i = 0; i < 16; ++i) o[i] = o_sum[c * 16 + i];
+                    for (int i = 0; i < 32; i += 4)
+                        *reinterpret_cast<float4*>(a.out + orow + i) = make_float4(o[i], o[i + 1], o[i + 2], o[i + 3]);
                 } else {
-                    tc_ld16(base + 192 + c * 16, o);
+#pragma unroll
+                    for (int i = 0; i < 32; ++i)
+                        if (i < cols) a.out[orow + i] = o[i];
                 }
+                if (a.out_cast) {
+                    uint16_t* crow = static_cast<uint16_t*>(a.out_cast) + orow;
+                    uint32_t w[16];
 #pragma unroll
-                for (int i = 0; i < 16; ++i) {
-                    const float o1 = m1 == -INFINITY ? 0.0f : merge[(c * 16 + i) * T + r] * f1;
-                    o[i] = (o[i] * f0 + o1) * inv;
-                    bad |= !(fabsf(o[i]) <= 3.4e38f);
-                }
-                if (live && alive) {
-                    if (cols == 64 && (a.Dv & 3) == 0) {
-#pragma unroll
-                        for (int i = 0; i < 16; i += 4)
-                            *reinterpret_cast<float4*>(orow + c * 16 + i) = make_float4(o[i], o[i + 1], o[i + 2], o[i + 3]);
-                    } else {
-                        for (int i = 0; i < 16; ++i)
-                            if (c * 16 + i < cols) orow[c * 16 + i] = o[i];
-                    }
-                    if (a.out_cast) {
-                        uint16_t* crow = static_cast<uint16_t*>(a.out_cast) + ((int64_t)bh * a.L + t) * a.Dv + half * 64 + c * 16;
-                        uint32_t w[8];
-#pragma unroll
-                        for (int i = 0; i < 8; ++i) {
-                            if (a.out_cast_tag == CINN_BF16) {
-                                const __nv_bfloat162 h = __floats2bfloat162_rn(o[2 * i], o[2 * i + 1]);
-                                w[i] = *reinterpret_cast<const uint32_t*>(&h);
-                            } else {
-                                const __half2 h = __floats2half2_rn(o[2 * i], o[2 * i + 1]);
-                                w[i] = *reinterpret_cast<const uint32_t*>(&h);
-                            }
-                        }
-                        if (cols == 64 && (a.Dv & 7) == 0) {
-                            *reinterpret_cast<uint4*>(crow) = make_uint4(w[0], w[1], w[2], w[3]);
-                            *reinterpret_cast<uint4*>(crow + 8) = make_uint4(w[4], w[5], w[6], w[7]);
+                    for (int i = 0; i < 16; ++i) {
+                        if (a.out_cast_tag == CINN_BF16) {
+                            const __nv_bfloat162 x = __floats2bfloat162_rn(o[2 * i], o[2 * i + 1]);
+                            w[i] = *reinterpret_cast<const uint32_t*>(&x);
                         } else {
-                            for (int i = 0; i < 16; ++i)
-                                if (c * 16 + i < cols) crow[i] = (uint16_t)(w[i >> 1] >> (16 * (i & 1)));
+                            const __half2 x = __floats2half2_rn(o[2 * i], o[2 * i + 1]);
+                            w[i] = *reinterpret_cast<const uint32_t*>(&x);
                         }
+                    }
+                    if (cols == 32 && (a.Dv & 7) == 0) {
+#pragma unroll
+                        for (int i = 0; i < 16; i += 4) *reinterpret_cast<uint4*>(crow + 2 * i) = make_uint4(w[i], w[i + 1], w[i + 2], w[i + 3]);
+                    } else {
+#pragma unroll
+                        for (int i = 0; i < 32; ++i)
+                            if (i < cols) crow[i] = (uint16_t)(w[i >> 1] >> (16 * (i & 1)));
                     }
                 }
             }
             if (live && bad) *a.flag = 1;
-            if (live && half == 0) a.lse[(int64_t)bh * a.L + t] = lse;
-        }
-        asm volatile("bar.sync 1, 256;" ::: "memory");
-        // Raw scores by rank -> probabilities by slot.  A warp takes sixteen pieces of 32 slots at a time with all loads in
-        // flight, whole rows of them: every slot of a row is read before any is written.
-        if (half == 0 && alive) {
-            constexpr int U = MAX_SLOTS / 32;
-            const int chunks = (a.K + 31) / 32, per = U / chunks, rows = min(T, a.L - q0);
-            const uint16_t* rank = a.picks.rank + ((int64_t)b * a.L + q0) * a.K;
-            float* attn = a.attn + ((int64_t)bh * a.L + q0) * a.K;
-            for (int k0 = warp; k0 < rows; k0 += 8 * per) {              // rows k0, k0 + 8, ...
-                float v[U];
-                uint32_t c[U];
-                int rr = k0, j = lane;                    // piece u of the batch: its row and this lane's slot
-                auto advance = [&] { if ((j += 32) >= chunks * 32) { j = lane; rr += 8; } };
-                const int end = min(rows, k0 + 8 * per);
-#pragma unroll
-                for (int u = 0; u < U; ++u, advance()) {
-                    // (loads from clamped places and a choice afterwards: behind a condition they would go one by one)
-                    const uint32_t x = rank[min(rr, end - 1) * a.K + min(j, a.K - 1)];
-                    c[u] = rr < end && j < a.K ? x : 0xffffu;
-                }
-                rr = k0; j = lane;
-#pragma unroll
-                for (int u = 0; u < U; ++u, advance()) {
-                    const float x = attn[min(rr, end - 1) * a.K + min((int)c[u], a.K - 1)];
-                    v[u] = c[u] != 0xffffu ? x : -INFINITY;
-                }
-                __syncwarp();
-                rr = k0; j = lane;
-#pragma unroll
-                for (int u = 0; u < U; ++u, advance())
-                    if (rr < end && j < a.K) attn[rr * a.K + j] = exp_fast(v[u] - s_lse[rr]);
+            if (h == 0) {
+                s_lse[r] = lse;
+                if (live && half == 0) a.lse[(int64_t)bh * a.L + t] = lse;
             }
         }
+        asm volatile("bar.sync 1, %0;" ::"n"(256 * PAIRS) : "memory");
+        if (half == 0 && alive)
+            by_slot<8 * PAIRS>(a.picks.rank + ((int64_t)b * a.L + q0) * a.K, a.attn + ((int64_t)bh * a.L + q0) * a.K, s_lse, min(T, a.L - q0), a.K,
+                    a.scale, warp, lane);
     }
     tc_fence_before();
     __syncthreads();
-    if (warp == 9) {
+    if (warp == MMA_WARP) {
         tc_fence_after();
-        tc_dealloc(tmem, 512);
+        tc_dealloc(tmem, 256 * PAIRS);
     }
 }
 
@@ -687,13 +787,15 @@ template <int NS, int ND, int NV> struct QPassShape {
     static constexpr int BYTES = BAR_OFF + 256 + 1024;
 };
 
+constexpr int QUERY_THREADS = 10 * 32;     // two vector warpgroups, TMA warp, MMA warp
+
 // Query pass: one CTA per 128 queries of a head, over their key tiles.  S = q k^T and dP = dO v^T in tensor memory; a
 // thread (a query, half of the tile's keys) turns them into p = exp(scale S - lse) and dS = p (dP - delta) scale, leaves
 // both by rank for the key pass, and writes dS back as an A operand for dq += dS k.  (Collecting a row's values in shared
 // memory to store them together took twice as long as these scattered stores.)  All of tensor memory: 128 columns of
 // S under the second and third parts of dS, 128 of dP, 64 of dS's leading parts, 192 of dq.
 template <int NS, int ND, int NV>
-__global__ void __launch_bounds__(FWD_THREADS, 1)
+__global__ void __launch_bounds__(QUERY_THREADS, 1)
 attn_bwd_query_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                       const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmG,
                       const __grid_constant__ CUtensorMap tmDQ, const BwdArgs a) {
@@ -764,42 +866,27 @@ attn_bwd_query_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
     } else if (warp == 9) {
         if (wait_warp(qfull, 0, abort_flag, (9 << 8) | 2)) {
             constexpr uint32_t id_s = make_idesc_f16(true, T, T), id_o = make_idesc_f16(true, T, 64, false, true);
-            uint32_t it = 0;
-            bool alive = true;
-            auto panel = [&](uint32_t& addr) {
-                const uint32_t s = it % S::RING;
-                if (!alive || !wait_warp(full0 + 8 * s, (it / S::RING) & 1, abort_flag, (9 << 8) | 3)) alive = false;
-                addr = ring + s * PANEL;
-                tc_fence_after();
-            };
-            auto release = [&] {
-                tc_commit(empty0 + 8 * (it % S::RING));
-                ++it;
-            };
+            PanelRing<S::RING> panels(full0, empty0, ring, abort_flag, (9 << 8) | 3);
+            const bool& alive = panels.alive;
             // parts [x_lo, x_hi] of a resident panel (parts `stride` panels apart) against the ring's next panel; with
             // `small`, the panel after it holds the third part, which goes first
             auto product = [&](uint32_t d, uint32_t fixed, int stride, int x_hi, int x_lo, bool small, bool& first) {
-                uint32_t bp, ap;
-                panel(bp);
-                if (!alive) return;
-                const uint64_t bd = panel_desc(bp);
+                uint32_t bp, ap, slot, small_slot;
+                if (!panels.next(bp, slot)) return;
+                const uint32_t bd = panel_desc(bp);
                 if (small) {
-                    const uint32_t held = it++;            // (released below, once every product with it has been issued)
-                    panel(ap);
-                    if (!alive) return;
+                    if (!panels.next(ap, small_slot)) return;
                     mma_panels(d, panel_desc(ap), bd, id_s, first);
                     first = false;
-                    release();
-                    it = held;
+                    panels.release(small_slot);
                 }
-                uint64_t ad = panel_desc(fixed) + (uint64_t)(x_hi * stride * (PANEL >> 4));
+                uint32_t ad = panel_desc(fixed) + x_hi * stride * (PANEL >> 4);
                 for (int x = x_hi; x >= x_lo; --x) {
                     mma_panels(d, ad, bd, id_s, first);
                     first = false;
                     ad -= stride * (PANEL >> 4);
                 }
-                release();
-                if (small) ++it;
+                panels.release(slot);
             };
             for (int j = 0; j < n && alive; ++j) {
                 // (S overwrites the parts of dS that dq of tile j - 1 reads: issued after it, executed after it)
@@ -823,24 +910,22 @@ attn_bwd_query_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
                 }
                 if (!alive) break;
                 tc_commit(sfull);
-                if (!wait_warp(dsready, j & 1, abort_flag, (9 << 8) | 4)) { alive = false; break; }
+                if (!wait_warp(dsready, j & 1, abort_flag, (9 << 8) | 4)) break;
                 const bool fresh = j == 0 || (flush && j % EVERY == 0);
-                if (fresh && j > 0 && !wait_warp(taken, (j / EVERY - 1) & 1, abort_flag, (9 << 8) | 7)) { alive = false; break; }
+                if (fresh && j > 0 && !wait_warp(taken, (j / EVERY - 1) & 1, abort_flag, (9 << 8) | 7)) break;
                 tc_fence_after();
                 for (int c = 0; c < ND && alive; ++c) {
                     first = fresh;
                     for (int p = NS - 1; p >= 0 && alive; --p) {
-                        uint32_t kp;
-                        panel(kp);
-                        if (!alive) break;
-                        const uint64_t kd = panel_desc(kp);
+                        uint32_t kp, slot;
+                        if (!panels.next(kp, slot)) break;
+                        const uint32_t kd = panel_desc(kp);
                         const uint32_t d = t_dq + c * 64;
                         if (p == 0) { mma_part_at<2>(d, t_s, t_lead, kd, id_o, first); first = false; }
                         if (p <= 1) { mma_part_at<1>(d, t_s, t_lead, kd, id_o, first); first = false; }
                         mma_part_at<0>(d, t_s, t_lead, kd, id_o, first);
                         first = false;
-                        tc_commit(empty0 + 8 * (it % S::RING));
-                        ++it;
+                        panels.release(slot);
                     }
                 }
                 if (alive && (j + 1 == n || (flush && (j + 1) % EVERY == 0))) tc_commit(done);
@@ -914,7 +999,8 @@ attn_bwd_query_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
                     at += (bit >> i) & 1u;
                 }
                 at0 += at;
-                store_parts32(t_s + lanes + h * 64 + c * 32, t_lead + lanes + h * 32 + c * 16, p);
+                store_parts16(t_s + lanes + h * 64 + c * 32, t_lead + lanes + h * 32 + c * 16, p);
+                store_parts16(t_s + lanes + h * 64 + c * 32 + 16, t_lead + lanes + h * 32 + c * 16 + 8, p + 16);
             }
             st_wait();
             tc_fence_before();
@@ -973,12 +1059,12 @@ attn_bwd_key_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
     const uint32_t ring = smem_u32(smem);
     uint64_t* bars = reinterpret_cast<uint64_t*>(smem + S::BAR_OFF);
     const uint32_t full0 = smem_u32(bars), empty0 = smem_u32(bars + S::STAGES);
-    const uint32_t ready0 = smem_u32(bars + 2 * S::STAGES), free0 = ready0 + 32;        // [operand][buffer]
-    const uint32_t done = ready0 + 64, taken = ready0 + 72;
+    const uint32_t ready0 = smem_u32(bars + 2 * S::STAGES), free0 = ready0 + 16;        // two each
+    const uint32_t done = ready0 + 32, taken = ready0 + 40;
     constexpr int EVERY = 4;                               // fp32 gradients: chunks between two flushes
     const bool flush = NS > 1 && a.tag == CINN_F32;
-    const uint32_t group0 = ready0 + 80;                   // the four warpgroups' own barriers
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * S::STAGES + 14);
+    const uint32_t group0 = ready0 + 48;                   // the four warpgroups' own barriers
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * S::STAGES + 10);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     int kt, bh;
@@ -988,7 +1074,7 @@ attn_bwd_key_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
     if (tid == 0) {
         *abort_flag = 0;
         for (int i = 0; i < S::STAGES; ++i) { mbar_init(full0 + 8 * i, 1); mbar_init(empty0 + 8 * i, 1); }
-        for (int i = 0; i < 4; ++i) { mbar_init(ready0 + 8 * i, 8); mbar_init(free0 + 8 * i, 1); }
+        for (int i = 0; i < 2; ++i) { mbar_init(ready0 + 8 * i, 8); mbar_init(free0 + 8 * i, 1); }
         mbar_init(done, 1); mbar_init(taken, 16);
         for (int i = 0; i < 4; ++i) mbar_init(group0 + 8 * i, 4);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -1022,34 +1108,34 @@ attn_bwd_key_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
     } else if (warp == 17) {
         constexpr uint32_t id = make_idesc_f16(true, T, 64, false, true);
         bool alive = true;
-        for (int i = 0; i < n && alive; ++i) {
-            const uint32_t s = i % S::STAGES, buf = i & 1;
-            if (!wait_warp(full0 + 8 * s, (i / S::STAGES) & 1, abort_flag, (10 << 8) | 2)) { alive = false; break; }
-            const uint32_t stage = ring + s * S::STAGE;
+        uint32_t s = 0, phase = 0;
+        for (int i = 0; i < n; ++i) {
+            const uint32_t buf = i & 1, stage = ring + s * S::STAGE, empty = empty0 + 8 * s;
+            if (!wait_warp(full0 + 8 * s, phase, abort_flag, (10 << 8) | 2)) { alive = false; break; }
             const bool fresh = i == 0 || (flush && i % EVERY == 0);
             if (fresh && i > 0 && !wait_warp(taken, (i / EVERY - 1) & 1, abort_flag, (10 << 8) | 6)) { alive = false; break; }
+            if (!wait_warp(ready0 + 8 * buf, (i >> 1) & 1, abort_flag, (10 << 8) | 3)) { alive = false; break; }
+            tc_fence_after();
+            if (++s == (uint32_t)S::STAGES) { s = 0; phase ^= 1u; }
 #pragma unroll
             for (int op = 0; op < 2; ++op) {               // dv from p and dO, dk from dS and q
-                if (alive && !wait_warp(ready0 + 8 * (op * 2 + buf), (i >> 1) & 1, abort_flag, (10 << 8) | 3)) alive = false;
-                if (!alive) break;
-                tc_fence_after();
                 const uint32_t at = t_a + (op * 2 + buf) * 48;
                 for (int c = 0; c < (op ? ND : NV); ++c) {
                     const uint32_t d = (op ? t_dk : t_dv) + c * 64;
                     bool first = fresh;
 #pragma unroll
                     for (int p = NS - 1; p >= 0; --p) {
-                        const uint64_t bd = panel_desc(stage + (p * (ND + NV) + (op ? NV : 0) + c) * S::SUB);
+                        const uint32_t bd = panel_desc(stage + (p * (ND + NV) + (op ? NV : 0) + c) * S::SUB);
                         if (p == 0) { mma_part_at<2, 2>(d, at, at + 32, bd, id, first); first = false; }
                         if (p <= 1) { mma_part_at<1, 2>(d, at, at + 32, bd, id, first); first = false; }
                         mma_part_at<0, 2>(d, at, at + 32, bd, id, first);
                         first = false;
                     }
                 }
-                tc_commit(free0 + 8 * (op * 2 + buf));
             }
-            if (alive) tc_commit(empty0 + 8 * s);
-            if (alive && (i + 1 == n || (flush && (i + 1) % EVERY == 0))) tc_commit(done);
+            tc_commit(free0 + 8 * buf);
+            tc_commit(empty);
+            if (i + 1 == n || (flush && (i + 1) % EVERY == 0)) tc_commit(done);
         }
     } else {
         const int half = (warp >> 2) & 1, buf = warp >> 3, quarter = warp & 3, r = quarter * 32 + lane;
@@ -1107,17 +1193,13 @@ attn_bwd_key_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
             // (with this chunk's values already here, the flush costs the tensor core its own time only)
             if (flush && i >= EVERY && i % EVERY == buf && !take()) { alive = false; break; }
             if (!wait_warp(free0 + 8 * buf, ((i >> 1) & 1) ^ 1, abort_flag, (10 << 8) | 4)) { alive = false; break; }
-            if (!wait_warp(free0 + 8 * (2 + buf), ((i >> 1) & 1) ^ 1, abort_flag, (10 << 8) | 4)) { alive = false; break; }
             tc_fence_after();
-            store_parts16(t_a + lanes + buf * 48, t_a + lanes + buf * 48 + 32, half, vp);
-            store_parts16(t_a + lanes + (2 + buf) * 48, t_a + lanes + (2 + buf) * 48 + 32, half, vd);
+            store_parts16(t_a + lanes + buf * 48 + half * 16, t_a + lanes + buf * 48 + 32 + half * 8, vp);
+            store_parts16(t_a + lanes + (2 + buf) * 48 + half * 16, t_a + lanes + (2 + buf) * 48 + 32 + half * 8, vd);
             st_wait();
             tc_fence_before();
             __syncwarp();
-            if (lane == 0) {
-                mbar_arrive(ready0 + 8 * buf);
-                mbar_arrive(ready0 + 8 * (2 + buf));
-            }
+            if (lane == 0) mbar_arrive(ready0 + 8 * buf);
         }
         if (alive && flush) {
             take();
@@ -1275,7 +1357,7 @@ static int launch_fwd(const CUtensorMap& tq, const CUtensorMap& tk, const CUtens
     auto kern = attn_fwd_kernel<NS, ND>;
     CINN_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, FwdShape<NS, ND>::BYTES));
     dim3 grid((unsigned)(p.Lp / T * p.BH), 1, (unsigned)p.nv);
-    kern<<<grid, FWD_THREADS, FwdShape<NS, ND>::BYTES, st>>>(tq, tk, tv, a);
+    kern<<<grid, FwdShape<NS, ND>::THREADS, FwdShape<NS, ND>::BYTES, st>>>(tq, tk, tv, a);
     CINN_CHECK_LAUNCH();
     return CINN_OK;
 }
@@ -1336,7 +1418,7 @@ static int launch_bwd(const CUtensorMap (&m)[9], const BwdArgs& a, const Plan& p
     const unsigned grid = (unsigned)(p.Lp / T * p.BH);
     CINN_CHECK_CUDA(cudaFuncSetAttribute(qk, cudaFuncAttributeMaxDynamicSharedMemorySize, QPassShape<NS, ND, NV>::BYTES));
     CINN_CHECK_CUDA(cudaFuncSetAttribute(kk, cudaFuncAttributeMaxDynamicSharedMemorySize, KPassShape<NS, ND, NV>::BYTES));
-    qk<<<grid, FWD_THREADS, QPassShape<NS, ND, NV>::BYTES, st>>>(m[0], m[1], m[2], m[3], m[6], a);
+    qk<<<grid, QUERY_THREADS, QPassShape<NS, ND, NV>::BYTES, st>>>(m[0], m[1], m[2], m[3], m[6], a);
     CINN_CHECK_LAUNCH();
     kk<<<grid, KEY_THREADS, KPassShape<NS, ND, NV>::BYTES, st>>>(m[4], m[5], m[7], m[8], a);
     CINN_CHECK_LAUNCH();

@@ -31,15 +31,6 @@ struct Picks {
     const int* repeats;                    // (B, tiles): whether a query of the tile picked a key more than once
 };
 
-// D[tmem] (+)= A[tmem] * B[smem desc]
-__device__ __forceinline__ void mma_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
-    asm volatile(
-        "{\n\t.reg .pred p, e;\n\t"
-        "elect.sync _|e, 0xffffffff;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "@e tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
-        ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate) : "memory");
-}
 // 32 lanes x 32 columns, without waiting
 __device__ __forceinline__ void ld32(uint32_t taddr, uint32_t (&r)[32]) {
     asm volatile(
@@ -49,6 +40,14 @@ __device__ __forceinline__ void ld32(uint32_t taddr, uint32_t (&r)[32]) {
           "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]), "=r"(r[17]), "=r"(r[18]),
           "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]),
           "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
+        : "r"(taddr));
+}
+// the same, 16 columns
+__device__ __forceinline__ void ld16(uint32_t taddr, uint32_t (&r)[16]) {
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]),
+          "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
         : "r"(taddr));
 }
 __device__ __forceinline__ void ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
@@ -75,33 +74,67 @@ __device__ __forceinline__ void tma_add_3d(const CUtensorMap* map, uint32_t src,
     asm volatile("cp.reduce.async.bulk.tensor.3d.global.shared::cta.add.bulk_group [%0, {%2, %3, %4}], [%1];"
                  ::"l"(map), "r"(src), "r"(x), "r"(y), "r"(z) : "memory");
 }
+// Two fp32 values in a register pair and one instruction for both.
+__device__ __forceinline__ uint64_t pair2(float a, float b) {
+    uint64_t r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ void unpair2(uint64_t v, float& a, float& b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v)); }
+__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
+    uint64_t r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+__device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) {
+    uint64_t r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
+    uint64_t r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+
 // two fp32 values as three packed bf16 pairs whose sum they are
 __device__ __forceinline__ void split2(float a, float b, uint32_t& hi, uint32_t& mid, uint32_t& lo) {
     auto pack = [](float x, float y) {
         const __nv_bfloat162 t = __floats2bfloat162_rn(x, y);
         return *reinterpret_cast<const uint32_t*>(&t);
     };
+    const uint64_t minus = pair2(-1.0f, -1.0f);
+    auto rest = [&](uint32_t part) {                      // what the part leaves: exact
+        unpair2(fma2(pair2(__uint_as_float(part << 16), __uint_as_float(part & 0xffff0000u)), minus, pair2(a, b)), a, b);
+    };
     hi = pack(a, b);
-    a -= __uint_as_float(hi << 16); b -= __uint_as_float(hi & 0xffff0000u);
+    rest(hi);
     mid = pack(a, b);
-    a -= __uint_as_float(mid << 16); b -= __uint_as_float(mid & 0xffff0000u);
+    rest(mid);
     lo = pack(a, b);
 }
 
-// e^x; a result below 2^-126 is 0
-__device__ __forceinline__ float exp_fast(float x) {
+// 2^x and e^x; a result below 2^-126 is 0
+__device__ __forceinline__ float exp2_fast(float x) {
     float r;
-    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x * 1.4426950408889634f));
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
     return r;
 }
+__device__ __forceinline__ float exp_fast(float x) { return exp2_fast(x * 1.4426950408889634f); }
 
-// if (take) *p = x, as a predicated instruction: as a branch it costs a warp some sixty cycles
-__device__ __forceinline__ void store_if(float* p, float x, uint32_t take) {
+// if (bits & mask) { *(base + at) = x; at += 4; } else p = 0, at in bytes.  As predicated instructions: a branch costs a warp
+// some sixty cycles.
+__device__ __forceinline__ void push_if(uint32_t bits, uint32_t mask, float* base, uint32_t& at, float x, float& p) {
     asm volatile(
-        "{\n\t.reg .pred t;\n\t"
-        "setp.ne.u32 t, %2, 0;\n\t"
-        "@t st.global.f32 [%0], %1;\n\t}"
-        ::"l"(p), "f"(x), "r"(take) : "memory");
+        "{\n\t.reg .pred t;\n\t.reg .b32 m;\n\t.reg .b64 to;\n\t"
+        "and.b32 m, %2, %3;\n\t"
+        "setp.ne.u32 t, m, 0;\n\t"
+        "cvt.u64.u32 to, %0;\n\t"
+        "add.u64 to, to, %4;\n\t"
+        "@t st.global.f32 [to], %5;\n\t"
+        "@t add.u32 %0, %0, 4;\n\t"
+        "selp.f32 %1, %1, 0f00000000, t;\n\t}"
+        : "+r"(at), "+f"(p) : "r"(bits), "r"(mask), "l"(base), "f"(x) : "memory");
 }
 
 // *p = (x, y) if take is not zero, as one predicated instruction
@@ -116,46 +149,72 @@ __device__ __forceinline__ void st8(uint32_t taddr, const uint32_t (&r)[8]) {
     asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%8], {%0, %1, %2, %3, %4, %5, %6, %7};"
                  ::"r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(taddr) : "memory");
 }
-// Writes 32 consecutive reduction positions (keys or queries) of this lane's row as an A operand in tensor memory: the
-// leading parts in 16 columns at `lead`, the second and third in 32 columns at `rest`.
-__device__ __forceinline__ void store_parts32(uint32_t rest, uint32_t lead, const float (&v)[32]) {
-    uint32_t hi[16], mid[16], lo[16];
-#pragma unroll
-    for (int i = 0; i < 16; ++i) split2(v[2 * i], v[2 * i + 1], hi[i], mid[i], lo[i]);
-    st16(lead, hi);
-    st16(rest, mid);
-    st16(rest + 16, lo);
-}
-// A panel used K-major (its 64 columns are the reduction axis; a step of four takes 16 of them) and MN-major (its 128 rows
-// are; a step of eight takes 16 of them): the descriptor of the first step, to which the steps are added.  One thread
-// issues all MMAs, so what it computes between two of them is time the tensor core waits.
-constexpr uint64_t K_STEP = 32 >> 4, MN_STEP = 2048 >> 4;
-__device__ __forceinline__ uint64_t panel_desc(uint32_t panel) { return make_smem_desc(panel, 16, 1024); }
-
-// D (+)= A B over the 64 columns of two K-major panels; the first step overwrites D when `fresh`
-__device__ __forceinline__ void mma_panels(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, bool fresh) {
-    tc_mma_f16(d, a, b, idesc, fresh ? 0u : 1u);
-#pragma unroll
-    for (int s = 1; s < 4; ++s) tc_mma_f16(d, a + s * K_STEP, b + s * K_STEP, idesc, 1u);
-}
-
-// the same for one half (0 or 1) of the 32 positions
-__device__ __forceinline__ void store_parts16(uint32_t rest, uint32_t lead, int half, const float (&v)[16]) {
+// Writes 16 consecutive reduction positions (keys or queries: one step of an MMA) of this lane's row as an A operand in tensor
+// memory: the leading parts in 8 columns at `lead`, the second and third in 8 columns each at `rest`.
+__device__ __forceinline__ void store_parts16(uint32_t rest, uint32_t lead, const float* v) {
     uint32_t hi[8], mid[8], lo[8];
 #pragma unroll
     for (int i = 0; i < 8; ++i) split2(v[2 * i], v[2 * i + 1], hi[i], mid[i], lo[i]);
-    st8(lead + half * 8, hi);
-    st8(rest + half * 8, mid);
-    st8(rest + 16 + half * 8, lo);
+    st8(lead, hi);
+    st8(rest, mid);
+    st8(rest + 8, lo);
+}
+// A panel used K-major (its 64 columns are the reduction axis; a step of four takes 16 of them: 32 bytes) and MN-major (its 128
+// rows are; a step of eight takes 16 of them: 2048 bytes).  Both have one descriptor, of which only the low word (the address in
+// units of 16 bytes) varies.
+constexpr uint32_t DESC_HI = (uint32_t)((((uint64_t)(1024 >> 4) << 32) | (1ull << 46) | (2ull << 61)) >> 32);
+__device__ __forceinline__ uint32_t panel_desc(uint32_t panel) { return ((panel >> 4) & 0x3FFFu) | (1u << 16); }
+
+// One warp issues all MMAs, so what it does between two of them is time the tensor core waits.  A panel's steps are one
+// statement with one election: issued one by one, with 64-bit descriptors, a panel of four cost the warp 350 cycles where
+// the MMAs take 256; like this 257.
+// D (+)= A B over the 64 columns of two K-major panels; the first step overwrites D when `fresh`
+__device__ __forceinline__ void mma_panels(uint32_t d, uint32_t a, uint32_t b, uint32_t idesc, bool fresh) {
+    asm volatile(
+        "{\n\t.reg .pred p, e;\n\t.reg .b64 a, b;\n\t.reg .b32 x, y;\n\t"
+        "elect.sync _|e, 0xffffffff;\n\t"
+        "setp.ne.b32 p, %5, 0;\n\t"
+        "mov.b64 a, {%1, %4};\n\tmov.b64 b, {%2, %4};\n\t"
+        "@e tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %3, p;\n\t"
+        "add.u32 x, %1, 2;\n\tadd.u32 y, %2, 2;\n\tmov.b64 a, {x, %4};\n\tmov.b64 b, {y, %4};\n\t"
+        "@e tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %3, 1;\n\t"
+        "add.u32 x, %1, 4;\n\tadd.u32 y, %2, 4;\n\tmov.b64 a, {x, %4};\n\tmov.b64 b, {y, %4};\n\t"
+        "@e tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %3, 1;\n\t"
+        "add.u32 x, %1, 6;\n\tadd.u32 y, %2, 6;\n\tmov.b64 a, {x, %4};\n\tmov.b64 b, {y, %4};\n\t"
+        "@e tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %3, 1;\n\t}"
+        ::"r"(d), "r"(a), "r"(b), "r"(idesc), "r"(DESC_HI), "r"(fresh ? 0u : 1u) : "memory");
 }
 
-// D (+)= part X of a tensor-memory operand of 16 STEPS positions (store_parts32) times an MN-major panel
+// D (+)= part X of a tensor-memory operand of 16 STEPS positions (store_parts16) times an MN-major panel
 template <int X, int STEPS = 8>
-__device__ __forceinline__ void mma_part_at(uint32_t d, uint32_t rest, uint32_t lead, uint64_t b, uint32_t idesc, bool fresh) {
-    auto column = [&](int s) { return X == 0 ? lead + s * 8 : rest + (s >> 1) * 32 + (X - 1) * 16 + (s & 1) * 8; };
-    mma_ts(d, column(0), b, idesc, fresh ? 0u : 1u);
-#pragma unroll
-    for (int s = 1; s < STEPS; ++s) mma_ts(d, column(s), b + s * MN_STEP, idesc, 1u);
+__device__ __forceinline__ void mma_part_at(uint32_t d, uint32_t rest, uint32_t lead, uint32_t b, uint32_t idesc, bool fresh) {
+    static_assert(STEPS == 8 || STEPS == 2, "the steps are written out");
+    const uint32_t a = X == 0 ? lead : rest + (X - 1) * 8;
+#define CINN_MMA_TS_FIRST                                                                                                           \
+    "{\n\t.reg .pred p, e;\n\t.reg .b64 b;\n\t.reg .b32 x, y;\n\t"                                                                  \
+    "elect.sync _|e, 0xffffffff;\n\t"                                                                                               \
+    "setp.ne.b32 p, %5, 0;\n\t"                                                                                                     \
+    "mov.b64 b, {%2, %4};\n\t"                                                                                                      \
+    "@e tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], b, %3, p;\n\t"
+#define CINN_MMA_TS_STEP(B, A)                                                                                                      \
+    "add.u32 x, %1, " A ";\n\tadd.u32 y, %2, " B ";\n\tmov.b64 b, {y, %4};\n\t"                                                     \
+    "@e tcgen05.mma.cta_group::1.kind::f16 [%0], [x], b, %3, 1;\n\t"
+#define CINN_MMA_TS_ARGS ::"r"(d), "r"(a), "r"(b), "r"(idesc), "r"(DESC_HI), "r"(fresh ? 0u : 1u) : "memory"
+    if constexpr (STEPS == 8 && X == 0)
+        asm volatile(CINN_MMA_TS_FIRST CINN_MMA_TS_STEP("128", "8") CINN_MMA_TS_STEP("256", "16") CINN_MMA_TS_STEP("384", "24")
+                         CINN_MMA_TS_STEP("512", "32") CINN_MMA_TS_STEP("640", "40") CINN_MMA_TS_STEP("768", "48")
+                             CINN_MMA_TS_STEP("896", "56") "}" CINN_MMA_TS_ARGS);
+    else if constexpr (STEPS == 8)
+        asm volatile(CINN_MMA_TS_FIRST CINN_MMA_TS_STEP("128", "16") CINN_MMA_TS_STEP("256", "32") CINN_MMA_TS_STEP("384", "48")
+                         CINN_MMA_TS_STEP("512", "64") CINN_MMA_TS_STEP("640", "80") CINN_MMA_TS_STEP("768", "96")
+                             CINN_MMA_TS_STEP("896", "112") "}" CINN_MMA_TS_ARGS);
+    else if constexpr (X == 0)
+        asm volatile(CINN_MMA_TS_FIRST CINN_MMA_TS_STEP("128", "8") "}" CINN_MMA_TS_ARGS);
+    else
+        asm volatile(CINN_MMA_TS_FIRST CINN_MMA_TS_STEP("128", "16") "}" CINN_MMA_TS_ARGS);
+#undef CINN_MMA_TS_FIRST
+#undef CINN_MMA_TS_STEP
+#undef CINN_MMA_TS_ARGS
 }
 
 }  // namespace atc
