@@ -194,14 +194,15 @@ __device__ __forceinline__ void tile_of_block(int n_tiles, int BH, int group, in
 }
 
 // Shared memory: queries [part][64-column panel] | ring of panels | barriers | row maxima on their way between two warps.
-// With one part two CTAs share an SM, each with one pair of softmax warpgroups: the first loads, the merge and the permutation of
-// one run under the other's tiles (a CTA of two pairs spent 20 000 of its 55 000 cycles on them, at 8 x 8 x 1531 queries of
-// 192).  Three parts of 192 columns need most of an SM's shared memory for the queries alone.
-template <int NS, int ND> struct FwdShape {
-    static constexpr int PAIRS = NS > 1 ? 2 : 1;           // of softmax warpgroups
+// With one part and more blocks than SMs two CTAs share an SM, each with one pair of softmax warpgroups: the first loads, the
+// merge and the permutation of one run under the other's tiles (a CTA of two pairs spends 20 000 of its 55 000 cycles on them, at
+// 8 x 8 x 1531 queries of 192: 195 us, 186 with one pair).  A block that has an SM to itself has two pairs (1 x 4 x 700 queries: 48 -> 45 us a call).
+// Three parts of 192 columns need most of an SM's shared memory for the queries alone.
+template <int NS, int ND, int PAIRS_> struct FwdShape {
+    static constexpr int PAIRS = PAIRS_;                   // of softmax warpgroups
     static constexpr int THREADS = (8 * PAIRS + 2) * 32;   // and a TMA warp, an MMA warp
     static constexpr int Q_PANELS = NS * ND;
-    static constexpr int RING = NS > 1 ? (Q_PANELS > 6 ? 4 : 6) : 6 - Q_PANELS;
+    static constexpr int RING = PAIRS == 1 ? 6 - Q_PANELS : Q_PANELS > 6 ? 4 : 6;
     static constexpr int BAR_OFF = (Q_PANELS + RING) * PANEL;
     static constexpr int PAIR_OFF = BAR_OFF + 512;         // [round & 1][pair][half][row]
     static constexpr int LSE_OFF = PAIR_OFF + 4 * PAIRS * T * 4;
@@ -209,10 +210,10 @@ template <int NS, int ND> struct FwdShape {
 };
 
 // 16 columns of a thread's row: scores to probabilities relative to `m`, left as parts over the scores and beside them.  The
-// picked raw scores go to rows + at (bytes) in passing when PUSH.  (32 columns at a time spilled.)
+// picked raw scores go to `to` in passing when PUSH.  (32 columns at a time spilled.)
 template <bool PUSH>
 __device__ __forceinline__ void softmax_chunk(uint32_t t_s, uint32_t t_lead, uint32_t bit, float scale, float m, bool repeats,
-                                              const uint8_t*& count, float* rows, uint32_t& at, uint64_t (&l)[2]) {
+                                              const uint8_t*& count, float*& to, uint64_t (&l)[2]) {
     uint32_t v[16];
     float p[16];
     ld16(t_s, v);
@@ -224,7 +225,7 @@ __device__ __forceinline__ void softmax_chunk(uint32_t t_s, uint32_t t_lead, uin
 #pragma unroll
         for (int e = i; e < i + 2; ++e) {
             p[e] = exp2_fast(p[e]);
-            if constexpr (PUSH) push_if(bit, 1u << e, rows, at, __uint_as_float(v[e]), p[e]);
+            if constexpr (PUSH) push_if(bit, 1u << e, to, __uint_as_float(v[e]), p[e]);
             else p[e] = bit & (1u << e) ? p[e] : 0.0f;
         }
     }
@@ -307,14 +308,17 @@ __device__ __forceinline__ void by_slot(const uint16_t* rank, float* attn, const
 // which it exchanges with the thread of the other half, and to write exp(score - max) back as three bf16 parts, the A operand
 // of P V, in the columns it has just read and 32 beside them, leaving the raw scores of the picked keys in the probabilities'
 // output (by rank; permuted and normalised at the end).  256 columns per pair: 128 scores, 64 leading parts, 64 of output.
-// Bound by the instructions per score and what hides their latency: FIG
+// Bound by the instructions per score (29, the merge and the permutation among them; they issue in 47 % of the cycles) and, in
+// fp32, by the panels' way into shared memory: the operands of 72 MMAs and the 15 panels of a tile take 7300 cycles of its bandwidth.
+// 8 x 8 x 1531 queries of 192 in bf16: 210 us with two warpgroups per CTA, a thread per row, 168 so; 32 x 8 x 1024 in fp32 655 and 618.  (Skipping
+// chunks that no query of a warp picked from: 2 % slower; the next chunk's scores in flight during this one's: 6 % slower, spills.)
 // NS: bf16 parts of q, k, v; ND: 64-column panels of q and k.
-template <int NS, int ND>
-__global__ void __launch_bounds__(FwdShape<NS, ND>::THREADS, 3 - FwdShape<NS, ND>::PAIRS)
+template <int NS, int ND, int PAIRS>
+__global__ void __launch_bounds__(FwdShape<NS, ND, PAIRS>::THREADS, 3 - PAIRS)
 attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                 const __grid_constant__ CUtensorMap tmV, const FwdArgs a) {
-    using S = FwdShape<NS, ND>;
-    constexpr int PAIRS = S::PAIRS, TMA_WARP = 8 * PAIRS, MMA_WARP = TMA_WARP + 1;
+    using S = FwdShape<NS, ND, PAIRS>;
+    constexpr int TMA_WARP = 8 * PAIRS, MMA_WARP = TMA_WARP + 1;
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
     const uint32_t sq = smem_u32(smem), ring = sq + S::Q_PANELS * PANEL;
@@ -439,8 +443,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         const uint4* bits = reinterpret_cast<const uint4*>(a.picks.bits + qrow * a.words);
         const uint16_t* before = a.picks.before + qrow * a.words + h * 2;
         const bool repeats = a.picks.repeats[b * n_qt + qt] != 0;
-        float* rows = a.attn + (int64_t)bh * a.L * a.K;
-        const uint32_t row_at = (uint32_t)min(t, a.L - 1) * (uint32_t)a.K;
+        float* row = a.attn + ((int64_t)bh * a.L + min(t, a.L - 1)) * a.K;
         const uint8_t* counts = a.picks.count + qrow * a.K;
         float m = -INFINITY;
         uint64_t l2[2] = {0u, 0u};                        // (0, 0) each
@@ -482,7 +485,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         const uint64_t scale2 = pair2(a.scale, a.scale);
         for (int j = pair; j < n; j += PAIRS) {
             const uint4 cur = mine;
-            uint32_t at = (row_at + rank) * 4;
+            float* to = row + rank;                       // the next picked key's raw score goes here
             const uint8_t* count = counts + rank;
             if (j + PAIRS < n) {                          // the next tile's, in flight during this one
                 mine = live ? __ldg(bits + j + PAIRS) : none;
@@ -556,8 +559,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
 #pragma unroll 1
             for (int c = 0; c < 4; ++c) {
                 const uint32_t bit = (c < 2 ? (h ? cur.z : cur.x) : (h ? cur.w : cur.y)) >> (c & 1) * 16;
-                if (half == 0) softmax_chunk<true>(t_s + c * 16, t_lead + c * 8, bit, a.scale, mu, repeats, count, rows, at, l2);
-                else softmax_chunk<false>(t_s + c * 16, t_lead + c * 8, bit, a.scale, mu, repeats, count, rows, at, l2);
+                if (half == 0) softmax_chunk<true>(t_s + c * 16, t_lead + c * 8, bit, a.scale, mu, repeats, count, to, l2);
+                else softmax_chunk<false>(t_s + c * 16, t_lead + c * 8, bit, a.scale, mu, repeats, count, to, l2);
             }
             st_wait();
             tc_fence_before();
@@ -1352,14 +1355,22 @@ static int head_group(const Plan& p) {
     return (int)(want < p.BH ? want : p.BH);
 }
 
-template <int NS, int ND>
-static int launch_fwd(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const FwdArgs& a, const Plan& p, cudaStream_t st) {
-    auto kern = attn_fwd_kernel<NS, ND>;
-    CINN_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, FwdShape<NS, ND>::BYTES));
-    dim3 grid((unsigned)(p.Lp / T * p.BH), 1, (unsigned)p.nv);
-    kern<<<grid, FwdShape<NS, ND>::THREADS, FwdShape<NS, ND>::BYTES, st>>>(tq, tk, tv, a);
+template <int NS, int ND, int PAIRS>
+static int launch_fwd_pairs(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const FwdArgs& a, dim3 grid, cudaStream_t st) {
+    using S = FwdShape<NS, ND, PAIRS>;
+    auto kern = attn_fwd_kernel<NS, ND, PAIRS>;
+    CINN_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, S::BYTES));
+    kern<<<grid, S::THREADS, S::BYTES, st>>>(tq, tk, tv, a);
     CINN_CHECK_LAUNCH();
     return CINN_OK;
+}
+
+template <int NS, int ND>
+static int launch_fwd(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const FwdArgs& a, const Plan& p, cudaStream_t st) {
+    const dim3 grid((unsigned)(p.Lp / T * p.BH), 1, (unsigned)p.nv);
+    if constexpr (NS == 1)
+        if ((int64_t)grid.x * grid.z > sm_count()) return launch_fwd_pairs<NS, ND, 1>(tq, tk, tv, a, grid, st);
+    return launch_fwd_pairs<NS, ND, 2>(tq, tk, tv, a, grid, st);
 }
 
 int64_t forward_workspace_bytes(int64_t B, int64_t H, int64_t L, int64_t K, int64_t Dqk, int64_t Dv, int dtype) {

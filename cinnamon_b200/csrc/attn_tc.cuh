@@ -122,19 +122,16 @@ __device__ __forceinline__ float exp2_fast(float x) {
 }
 __device__ __forceinline__ float exp_fast(float x) { return exp2_fast(x * 1.4426950408889634f); }
 
-// if (bits & mask) { *(base + at) = x; at += 4; } else p = 0, at in bytes.  As predicated instructions: a branch costs a warp
-// some sixty cycles.
-__device__ __forceinline__ void push_if(uint32_t bits, uint32_t mask, float* base, uint32_t& at, float x, float& p) {
+// if (bits & mask) *to++ = x; else p = 0.  As predicated instructions: a branch costs a warp some sixty cycles.
+__device__ __forceinline__ void push_if(uint32_t bits, uint32_t mask, float*& to, float x, float& p) {
     asm volatile(
-        "{\n\t.reg .pred t;\n\t.reg .b32 m;\n\t.reg .b64 to;\n\t"
+        "{\n\t.reg .pred t;\n\t.reg .b32 m;\n\t"
         "and.b32 m, %2, %3;\n\t"
         "setp.ne.u32 t, m, 0;\n\t"
-        "cvt.u64.u32 to, %0;\n\t"
-        "add.u64 to, to, %4;\n\t"
-        "@t st.global.f32 [to], %5;\n\t"
-        "@t add.u32 %0, %0, 4;\n\t"
+        "@t st.global.f32 [%0], %4;\n\t"
+        "@t add.u64 %0, %0, 4;\n\t"
         "selp.f32 %1, %1, 0f00000000, t;\n\t}"
-        : "+r"(at), "+f"(p) : "r"(bits), "r"(mask), "l"(base), "f"(x) : "memory");
+        : "+l"(to), "+f"(p) : "r"(bits), "r"(mask), "f"(x) : "memory");
 }
 
 // *p = (x, y) if take is not zero, as one predicated instruction

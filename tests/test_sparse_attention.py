@@ -199,6 +199,33 @@ def test_tiles_and_gathers(dtype, shape, attention_path):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("shape", [(1, 2, 513, 64, 72, 64), (1, 2, 400, 24, 64, 100), (2, 40, 257, 32, 64, 64), (1, 75, 385, 512, 64, 40)])
+def test_tiles_with_wide_scores(dtype, shape):
+    """Scores of up to some 50, larger for later keys, so that the exponentials' reference point moves in late key tiles; with a
+    block per SM and with two, lists of a power of two of slots (permuted four at a time) and others.  A score of 50 is known
+    to 2^-22 of itself, its exponential to 50 x 2^-22 = 1.2e-5: the bound is three times that."""
+    from cinnamon_b200 import kernels as K
+    B, H, L, Ks, Dqk, Dv = shape
+    g = torch.Generator().manual_seed(sum(shape))
+    q, k = torch.randn(B, H, L, Dqk, generator=g), torch.randn(B, H, L, Dqk, generator=g)
+    q, k = (q * 1.2).to(dtype), (k * (0.2 + torch.arange(L).view(1, 1, L, 1) / L)).to(dtype)
+    v = torch.randn(B, H, L, Dv, generator=g).to(dtype)
+    idx = torch.randint(0, L, (B, L, Ks), generator=g)
+    before = K._L.cinn_set_sparse_attn_dense(1)
+    try:
+        out, attn = K.sparse_attention(q.cuda(), k.cuda(), v.cuda(), idx.cuda(), 1.0)
+    finally:
+        K._L.cinn_set_sparse_attn_dense(before)
+    heads = sorted({0, 1, H // 2, H - 1})
+    ref_out, ref_attn, _ = SO.forward(q[:, heads], k[:, heads], v[:, heads], idx, 1.0)
+    tol = {torch.float32: 4e-5, torch.bfloat16: 8e-3}[dtype]                            # bf16: rounding of the returned output
+    torch.testing.assert_close(out[:, heads].float().cpu().double(), ref_out, rtol=tol, atol=tol)
+    torch.testing.assert_close(attn[:, heads].cpu().double(), ref_attn, rtol=4e-5, atol=1e-7)
+    assert K.device_status() == 0
+
+
+@pytest.mark.gpu
 def test_tiles_fall_back_on_the_device(attention_path):
     """What the tiles cannot express: a key picked more than 255 times, and rows nobody picked that hold NaN or infinity."""
     from cinnamon_b200 import kernels as K
