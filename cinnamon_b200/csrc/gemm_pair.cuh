@@ -9,8 +9,14 @@
 // CTA.  TMA loads are plain per-CTA loads: each CTA fetches only its own halves and reports
 // the bytes to the leader's "operands landed" barrier.
 //
-// Roles per CTA (11 warps): 0-7 promotion/epilogue, 8 TMA producer, 9 TMEM allocation;
-// warps 9 and 10 of the leader issue the MMAs of alternate K blocks.  All waits are bounded exactly as in the one-SM kernel.
+// Roles per CTA (12 warps): 0-7 promotion, 8 TMA producer, 9 TMEM allocation and, in the leader, the MMAs; 10 hands finished
+// tiles to the TMA unit; 11 brings the scales and the tiles' coordinates.  All waits are bounded exactly as in the one-SM kernel.
+//
+// The promotion warps are the bound (a K block took them 840 cycles where its MMAs take 512, a tile 3500 around its K blocks), so
+// they do nothing else: a tile's coordinates cost them 850 cycles of divisions, its stores up to 1000 of waiting for the TMA unit, and
+// the scales registers and a round trip per tile.  The scales' products now arrive through shared memory, on the barrier that reports
+// the MMAs.  16384 x 7168 -> 18432 1915 -> 1708 us, 16384 x 576 -> 7168 102 -> 81, 32768 x 512 -> 1024 32.7 -> 28.3, 32768 rows of 7168 -> 4096 by
+// 32 experts and the way back with it 4.38 -> 4.29 ms, all cool.  (Sixteen warps of 64 columns, to hide more latency: 1957, 89 and 30.)
 #pragma once
 
 namespace pair {
@@ -20,14 +26,21 @@ constexpr int PN = 256;                 // columns of the pair's tile
 constexpr int PSTAGES = 4;               // even (see the one-SM kernel); leaves room for a whole output tile
 constexpr int PA_BYTES = 128 * BK;      // A rows of this CTA: 16 KiB
 constexpr int PB_BYTES = 128 * BK;      // B columns of this CTA: 16 KiB
-constexpr int PTHREADS = 11 * 32;
-// dynamic shared memory: operand stages | two 4 KiB output boxes per promotion warp = the CTA's whole 128 x 256 tile of a
-// 2-byte type (TMA-store boxes; also the 2 KiB-per-warp staging of the non-TMA path) | 256 B of barriers and flags, plus 1 KiB of
-// slack to align the stages to 1024 bytes
+constexpr int PEPI = 8;                 // promotion warps: four TMEM lane quarters x two groups of PCOLS columns
+constexpr int PCOLS = PN / (PEPI / 4);
+constexpr int PTMA = PEPI, PMMA = PEPI + 1, PSTORE = PEPI + 2, PSCALE = PEPI + 3;
+constexpr int PTHREADS = (PEPI + 4) * 32;
+constexpr int PSCALE_SLOTS = 4;         // K blocks whose scale products are in shared memory: [slot][128 columns][row]
+constexpr int PSCALE_BYTES = PSCALE_SLOTS * 2 * 128 * 4;
+constexpr int PTILE_SLOTS = 16;         // coordinates of the next tiles: {m0, n0, one past the last row, expert}
+// dynamic shared memory: operand stages | a 4 KiB output box per promotion warp = the CTA's whole 128 x 256 tile of a
+// 2-byte type (TMA-store boxes; also the 2 KiB-per-warp staging of the non-TMA path) | scale products | tiles | 256 B of barriers and
+// flags, plus 1 KiB of slack to align the stages to 1024 bytes
 constexpr int PSTAGE_OFF = PSTAGES * (PA_BYTES + PB_BYTES);
 constexpr int PBOX_BYTES = STORE_ROWS * 128;  // one TMA-store box
-constexpr int PC_BYTES = 8 * 2 * PBOX_BYTES;
-constexpr size_t PSMEM_BYTES = (size_t)PSTAGE_OFF + PC_BYTES + 256 + 1024;
+constexpr int PBOXES = 16 / PEPI;       // boxes per promotion warp: a round of them all is 64 KiB, a CTA's tile of a 2-byte type
+constexpr int PC_BYTES = PEPI * PBOXES * PBOX_BYTES;
+constexpr size_t PSMEM_BYTES = (size_t)PSTAGE_OFF + PC_BYTES + PSCALE_BYTES + PTILE_SLOTS * 16 + 256 + 1024;
 
 __device__ __forceinline__ uint32_t cluster_ctarank() {
     uint32_t r;
@@ -68,13 +81,22 @@ __device__ __forceinline__ void tc_commit_pair(uint32_t own, uint32_t peer) {
         "@e tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64 [%1];\n\t}"
         ::"r"(own), "r"(peer) : "memory");
 }
-__device__ __forceinline__ void tc_mma_f8_pair(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
+// The four MMAs of a K block, by one election; only the low words of the descriptors vary.  STEP_B: 16-byte units from one step's B to the next
+template <int STEP_B>
+__device__ __forceinline__ void tc_mma_f8_pair(uint32_t d_tmem, uint32_t a_lo, uint32_t b_lo, uint32_t idesc) {
+    constexpr uint32_t hi = (uint32_t)((((uint64_t)(1024 >> 4) << 32) | (1ull << 46) | (2ull << 61)) >> 32);
     asm volatile(
-        "{\n\t.reg .pred p, e;\n\t"
+        "{\n\t.reg .pred e;\n\t.reg .b64 a, b;\n\t.reg .b32 x, y;\n\t"
         "elect.sync _|e, 0xffffffff;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "@e tcgen05.mma.cta_group::2.kind::f8f6f4 [%0], %1, %2, %3, p;\n\t}"
-        ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate) : "memory");
+        "mov.b64 a, {%1, %4};\n\tmov.b64 b, {%2, %4};\n\t"
+        "@e tcgen05.mma.cta_group::2.kind::f8f6f4 [%0], a, b, %3, 0;\n\t"
+        "add.u32 x, %1, 2;\n\tadd.u32 y, %2, %5;\n\tmov.b64 a, {x, %4};\n\tmov.b64 b, {y, %4};\n\t"
+        "@e tcgen05.mma.cta_group::2.kind::f8f6f4 [%0], a, b, %3, 1;\n\t"
+        "add.u32 x, %1, 4;\n\tadd.u32 y, %2, %6;\n\tmov.b64 a, {x, %4};\n\tmov.b64 b, {y, %4};\n\t"
+        "@e tcgen05.mma.cta_group::2.kind::f8f6f4 [%0], a, b, %3, 1;\n\t"
+        "add.u32 x, %1, 6;\n\tadd.u32 y, %2, %7;\n\tmov.b64 a, {x, %4};\n\tmov.b64 b, {y, %4};\n\t"
+        "@e tcgen05.mma.cta_group::2.kind::f8f6f4 [%0], a, b, %3, 1;\n\t}"
+        ::"r"(d_tmem), "r"(a_lo), "r"(b_lo), "r"(idesc), "r"(hi), "n"(STEP_B), "n"(2 * STEP_B), "n"(3 * STEP_B) : "memory");
 }
 __host__ __device__ constexpr uint32_t make_idesc_pair(bool b_mn_major) {
     return (1u << 4) | ((b_mn_major ? 1u : 0u) << 16) | ((uint32_t)(PN >> 3) << 17) | ((uint32_t)(PM >> 4) << 24);
@@ -118,8 +140,11 @@ fp8_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
     uint8_t* smem_a = smem;
     uint8_t* smem_b = smem + PSTAGES * PA_BYTES;
     uint8_t* c_stage = smem + PSTAGE_OFF;
-    uint64_t* bars = reinterpret_cast<uint64_t*>(c_stage + PC_BYTES);
-    // [0, S) full (used in the leader), [S, 2S) empty, [2S, 2S+2) tmem full, [2S+2, 2S+4) tmem empty (leader)
+    float* scales = reinterpret_cast<float*>(c_stage + PC_BYTES);
+    int4* tiles = reinterpret_cast<int4*>(c_stage + PC_BYTES + PSCALE_BYTES);
+    uint64_t* bars = reinterpret_cast<uint64_t*>(tiles + PTILE_SLOTS);
+    // [0, S) full (used in the leader), [S, 2S) empty, [2S, 2S+2) tmem full, [2S+2, 2S+4) tmem empty (leader), then: all boxes of a
+    // round are staged, they have been read
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * PSTAGES + 8);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
     int* cum = reinterpret_cast<int*>(reinterpret_cast<uint8_t*>(bars) + 256);  // GR: E + 1 prefix counts of row tiles
@@ -128,14 +153,17 @@ fp8_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
     const uint32_t rank = cluster_ctarank();           // 0 = leader
     const uint32_t full0 = smem_u32(bars), empty0 = smem_u32(bars + PSTAGES);
     const uint32_t tfull0 = smem_u32(bars + 2 * PSTAGES), tempty0 = smem_u32(bars + 2 * PSTAGES + 2);
+    const uint32_t staged = smem_u32(bars + 2 * PSTAGES + 4), taken = smem_u32(bars + 2 * PSTAGES + 5);
 
     if (threadIdx.x == 0) *abort_flag = 0;
-    if (warp == 8 && lane == 0) {
+    if (warp == PTMA && lane == 0) {
         for (int s = 0; s < PSTAGES; ++s) { mbar_init(full0 + 8 * s, 1); mbar_init(empty0 + 8 * s, 1); }
-        for (int b = 0; b < 2; ++b) { mbar_init(tfull0 + 8 * b, 1); mbar_init(tempty0 + 8 * b, 16); }
+        for (int b = 0; b < 2; ++b) { mbar_init(tfull0 + 8 * b, 2); mbar_init(tempty0 + 8 * b, 2 * PEPI); }
+        mbar_init(staged, PEPI);
+        mbar_init(taken, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    if (warp == 9) {
+    if (warp == PMMA) {
         asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(TMEM_COLS) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
     }
@@ -183,7 +211,7 @@ fp8_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
         }
     };
 
-    if (warp == 8) {
+    if (warp == PTMA) {
         // ------------------------------ TMA producer (both CTAs) ------------------------------
         if (lane == 0) {
             const uint32_t full_leader = mapa(full0, 0);
@@ -211,14 +239,99 @@ fp8_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
                 while (clock64() - t0 < 2000000LL) { }
             }
         }
-    } else if (warp >= 9) {
-        // ------------------ MMA issuers (leader only; whole warps, as in the one-SM kernel) ------------------
+    } else if (warp == PSCALE) {
+        // ------------------ scales (both CTAs): K block `it`'s products sA sB of this CTA's rows, FETCH blocks ahead in registers ------------------
+        constexpr int FETCH = 4;
+        const float* a_ptr[4];
+        const float* b_ptr[2];
+        int t = cluster_id - n_clusters, left = 0;     // K blocks of the tile that are still to be fetched
+        uint32_t entered = 0;
+        uint32_t fetched = 0;
+        float va[FETCH][4], vb[FETCH][2];
+        auto fetch = [&](float (&x)[4], float (&y)[2]) {
+            while (left == 0) {
+                t += n_clusters;
+                if (t >= n_total) { t = n_total; return; }           // (and stays there)
+                PairTile ti; int e, kb0, m_end;
+                locate(t, ti, e, kb0, left, m_end);
+                // (sixteen slots: the slot's last tile has left the promotion warps even when tiles have one K block)
+                if (lane == 0) tiles[entered % PTILE_SLOTS] = make_int4(ti.m0, ti.n0, m_end, e);
+                ++entered;
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    const int row = ti.m0 + 128 * (int)rank + i * 32 + lane;
+                    a_ptr[i] = p.sA + (int64_t)(row < m_end ? row : (GR ? ti.m0 : 0)) * p.sa_stride_m + (int64_t)kb0 * p.sa_stride_k;
+                }
+#pragma unroll
+                for (int c = 0; c < 2; ++c) {
+                    const int col = ti.n0 + c * 128;
+                    b_ptr[c] = p.sB + (int64_t)(col < p.N ? col / 128 : 0) * p.sb_stride_n + (int64_t)kb0 * p.sb_stride_k
+                               + (GR ? (int64_t)e * p.sb_stride_e : 0);
+                }
+            }
+#pragma unroll
+            for (int i = 0; i < 4; ++i) { x[i] = ld_scale(a_ptr[i]); a_ptr[i] += p.sa_stride_k; }
+#pragma unroll
+            for (int c = 0; c < 2; ++c) { y[c] = ld_scale(b_ptr[c]); b_ptr[c] += p.sb_stride_k; }
+            --left;
+            ++fetched;
+        };
+#pragma unroll
+        for (int u = 0; u < FETCH; ++u) fetch(va[u], vb[u]);
+        bool alive = true;
+        for (uint32_t it = 0; alive && it < fetched;) {
+#pragma unroll
+            for (int u = 0; u < FETCH; ++u) {
+                if (alive && it < fetched) {
+                    // (the MMAs of block it - 2 are done, so its buffer had been released by every reader of block it - 4, whose slot
+                    // this is; and that barrier cannot complete again without the arrival below)
+                    if (it >= 2 && !mbar_wait_warp(tfull0 + 8 * (it & 1), ((it - 2) >> 1) & 1, abort_flag, (4 << 8) | 1)) { alive = false; continue; }
+                    float* to = scales + (it % PSCALE_SLOTS) * 256 + lane;
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) { to[i * 32] = va[u][i] * vb[u][0]; to[128 + i * 32] = va[u][i] * vb[u][1]; }
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(tfull0 + 8 * (it & 1));
+                    fetch(va[u], vb[u]);
+                    ++it;
+                }
+            }
+        }
+    } else if (warp == PSTORE) {
+        // ------------------------------ finished tiles to the TMA unit (both CTAs) ------------------------------
+        // A lane sends a box.  A tile's 64 KiB leave the SM in a thousand cycles and an issue blocks until the unit
+        // takes it: promotion warps that issued their own stores stood still for most of that.
+        if (p.tma_out) {
+            constexpr int EPR = 128 / (int)sizeof(typename OutT<OUT>::type);
+            const int w = lane / PBOXES, q = w & 3, h = w >> 2;
+            uint32_t round = 0;
+            bool alive = true;
+            for (int t = cluster_id; t < n_total && alive; t += n_clusters) {
+                PairTile ti; int e, kb0, KB, m_end;
+                locate(t, ti, e, kb0, KB, m_end);
+                const int row = ti.m0 + 128 * (int)rank + q * 32;
+                const int out_row0 = GR ? 0 : e * p.M;
+                for (int r = 0; r < PCOLS / (PBOXES * EPR); ++r, ++round) {
+                    const int col = ti.n0 + h * PCOLS + (r * PBOXES + lane % PBOXES) * EPR;
+                    if (!mbar_wait_warp(staged, round & 1, abort_flag, (5 << 8) | 1)) { alive = false; break; }
+                    if (lane < PEPI * PBOXES) {
+                        if (col < p.N && (!GR || row + 32 <= m_end)) tma_store_2d(&tmC, smem_u32(c_stage) + lane * PBOX_BYTES, col, out_row0 + row);
+                        tma_store_commit();
+                        tma_store_wait_read();
+                    }
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(taken);
+                }
+            }
+            if (lane < PEPI * PBOXES) tma_store_wait_all();     // the boxes have reached global memory
+        }
+    } else if (warp == PMMA) {
+        // ------------------ MMA issuer (leader only; a whole warp, as in the one-SM kernel) ------------------
         if (rank == 0) {
             constexpr uint32_t idesc = make_idesc_pair(B_MN);
             const uint32_t tfull_own = mapa(tfull0, 0), tfull_peer = mapa(tfull0, 1);
             const uint32_t empty_own = mapa(empty0, 0), empty_peer = mapa(empty0, 1);
-            const uint32_t mine = (uint32_t)(warp - 9);
-            uint32_t it = 0, last = 0xffffffffu;
+            const uint32_t a0 = ((smem_u32(smem_a) >> 4) & 0x3FFF) | (1u << 16), b0 = ((smem_u32(smem_b) >> 4) & 0x3FFF) | (1u << 16);
+            uint32_t it = 0;
             bool alive = true;
             for (int t = cluster_id; t < n_total && alive; t += n_clusters) {
                 int KB = KB_dense;
@@ -227,29 +340,17 @@ fp8_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
                     locate(t, ti_, e_, kb0_, KB, end_);
                 }
                 for (int kb = 0; kb < KB; ++kb, ++it) {
-                    if ((it & 1u) != mine) continue;
-                    last = it;
-                    const int s = it % PSTAGES;
-                    const uint32_t ph = (it / PSTAGES) & 1;
+                    const uint32_t s = it % PSTAGES, ph = (it / PSTAGES) & 1;
                     const uint32_t b = it & 1, bph = (it >> 1) & 1;
                     if (!mbar_wait_warp(full0 + 8 * s, ph, abort_flag, (2 << 8) | 1)) { alive = false; break; }
                     if (!mbar_wait_warp(tempty0 + 8 * b, bph ^ 1, abort_flag, (2 << 8) | 2)) { alive = false; break; }
                     tc_fence_after();
-                    const uint32_t a_addr = smem_u32(smem_a + s * PA_BYTES);
-                    const uint32_t b_addr = smem_u32(smem_b + s * PB_BYTES);
-                    const uint32_t d = tmem_base + b * PN;
-#pragma unroll
-                    for (int k = 0; k < BK / 32; ++k) {
-                        const uint64_t ad = make_smem_desc(a_addr + k * 32, 16, 1024);
-                        const uint64_t bd = B_MN ? make_smem_desc(b_addr + k * 32 * 128, 16, 1024)
-                                                 : make_smem_desc(b_addr + k * 32, 16, 1024);
-                        tc_mma_f8_pair(d, ad, bd, idesc, k > 0 ? 1u : 0u);
-                    }
+                    tc_mma_f8_pair<B_MN ? 256 : 2>(tmem_base + b * PN, a0 + s * (PA_BYTES >> 4), b0 + s * (PB_BYTES >> 4), idesc);
                     tc_commit_pair(tfull_own + 8 * b, tfull_peer + 8 * b);
                     tc_commit_pair(empty_own + 8 * s, empty_peer + 8 * s);
                 }
             }
-            if (alive && last != 0xffffffffu) mbar_wait(tfull0 + 8 * (last & 1), (last >> 1) & 1, abort_flag, (2 << 8) | 3);
+            if (alive && it) mbar_wait(tfull0 + 8 * ((it - 1) & 1), ((it - 1) >> 1) & 1, abort_flag, (2 << 8) | 3);
         }
     } else {
         // ------------------------------ promotion / epilogue (both CTAs) ------------------------------
@@ -257,41 +358,26 @@ fp8_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
         const uint32_t tempty_leader = mapa(tempty0, 0);
         uint32_t it = 0;
         bool alive = true;
+        const float* my_scales = scales + (h * PCOLS / 128) * 128 + q * 32 + lane;
         const bool vec_ok = (OUT == CINN_F32 || OUT == CINN_F32_BF16) ? (p.ldc % 4 == 0) : (p.ldc % 8 == 0);
+        uint32_t seen = 0, round = 0;
         for (int t = cluster_id; t < n_total && alive; t += n_clusters) {
-            PairTile ti; int e, kb0, KB, m_end;
-            locate(t, ti, e, kb0, KB, m_end);
-            const int row = ti.m0 + 128 * (int)rank + q * 32 + lane;
-            const bool rvalid = row < m_end;
-            const int col0 = ti.n0 + h * 128;
-            const bool cvalid = col0 < p.N;
-            const float* sa_ptr = p.sA + (int64_t)(rvalid ? row : (GR ? ti.m0 : 0)) * p.sa_stride_m + (int64_t)kb0 * p.sa_stride_k;
-            const float* sb_ptr = p.sB + (int64_t)(cvalid ? col0 / 128 : 0) * p.sb_stride_n + (int64_t)kb0 * p.sb_stride_k
-                                  + (GR ? (int64_t)e * p.sb_stride_e : 0);
-            const int out_row0 = GR ? 0 : e * p.M;                      // GK: the expert's slice of the (E * M, N) output
-            float acc[128];
+            PairTile ti; int e, kb0, KB = KB_dense, m_end;
+            if constexpr (GK) locate(t, ti, e, kb0, KB, m_end);       // (a tile without K blocks does not pass through the scale warp)
+            float acc[PCOLS];
 #pragma unroll
-            for (int i = 0; i < 128; ++i) acc[i] = 0.0f;
-            float sa0 = ld_scale(sa_ptr), sb0 = ld_scale(sb_ptr);
-            float sa1 = 0.f, sb1 = 0.f, sa2 = 0.f, sb2 = 0.f;
-            if (KB > 1) { sa1 = ld_scale(sa_ptr + p.sa_stride_k); sb1 = ld_scale(sb_ptr + p.sb_stride_k); }
-            if (KB > 2) { sa2 = ld_scale(sa_ptr + 2 * p.sa_stride_k); sb2 = ld_scale(sb_ptr + 2 * p.sb_stride_k); }
+            for (int i = 0; i < PCOLS; ++i) acc[i] = 0.0f;
             for (int kb = 0; kb < KB; ++kb, ++it) {
-                const float s = sa0 * sb0;
-                sa0 = sa1; sb0 = sb1; sa1 = sa2; sb1 = sb2;
-                if (kb + 3 < KB) {
-                    sa2 = ld_scale(sa_ptr + (int64_t)(kb + 3) * p.sa_stride_k);
-                    sb2 = ld_scale(sb_ptr + (int64_t)(kb + 3) * p.sb_stride_k);
-                }
                 const uint32_t b = it & 1, bph = (it >> 1) & 1;
                 if (!mbar_wait_warp(tfull0 + 8 * b, bph, abort_flag, (3 << 8) | 1)) { alive = false; break; }
                 tc_fence_after();
-                const uint32_t taddr = tmem_base + ((uint32_t)(q * 32) << 16) + b * PN + h * 128;
-                // packed fp32x2 FMAs: half the issue slots of 128 scalar ones, the same IEEE result in every lane
+                const float s = my_scales[(it % PSCALE_SLOTS) * 256];
+                const uint32_t taddr = tmem_base + ((uint32_t)(q * 32) << 16) + b * PN + h * PCOLS;
+                // packed fp32x2 FMAs: half the issue slots of scalar ones, the same IEEE result in every lane
                 uint64_t s2;
                 asm("mov.b64 %0, {%1, %1};" : "=l"(s2) : "f"(s));
 #pragma unroll
-                for (int c = 0; c < 8; ++c) {
+                for (int c = 0; c < PCOLS / 16; ++c) {
                     float v[16];
                     tc_ld16(taddr + c * 16, v);
 #pragma unroll
@@ -307,66 +393,64 @@ fp8_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
                 __syncwarp();
                 if (lane == 0) mbar_arrive_remote(tempty_leader + 8 * b);
             }
-            if (alive && p.tma_out && (!GR || row - lane + 32 <= m_end)) {
-                // The tile leaves through TMA stores.  Every promotion warp owns 8 KiB of the staging area, two boxes of 32 rows
-                // x 128 bytes (128-byte swizzle): its lanes drop their rows in 16-byte chunks and one lane hands the boxes to
-                // the TMA unit.  A 2-byte output fits the warp's 128 columns in one round; a 4-byte output takes two rounds of
-                // 64 columns.  Nobody waits for the unit until the boxes are needed again, and no warp for another: with boxes
-                // of 128 rows, four warps met at two barriers for each (16384 x 7168 -> 2048: 211 us, where this takes 195;
-                // 32768 x 512 -> 1024: 29.8 and 27.4).
+            if (!alive) break;
+            if constexpr (!GK) {                       // in shared memory since the tile's first scales (the divisions took 850 cycles here)
+                const int4 x = tiles[seen++ % PTILE_SLOTS];
+                ti.m0 = x.x; ti.n0 = x.y; m_end = x.z; e = x.w;
+            }
+            const int row = ti.m0 + 128 * (int)rank + q * 32 + lane;
+            const bool rvalid = row < m_end;
+            const int col0 = ti.n0 + h * PCOLS;
+            const bool cvalid = col0 < p.N;
+            const int out_row0 = GR ? 0 : e * p.M;                      // GK: the expert's slice of the (E * M, N) output
+            if (p.tma_out) {
+                // The tile leaves through TMA stores, which the store warp issues.  Every promotion warp owns a box of 32 rows x 128
+                // bytes (128-byte swizzle) of the staging area, where its lanes drop their rows in 16-byte chunks.  A 2-byte
+                // output fits the warp's 64 columns in one round; a 4-byte output takes two rounds of 32.  Rows of two
+                // owners leave as staged 16-byte stores.
                 using T = typename OutT<OUT>::type;
                 constexpr int EPR = 128 / (int)sizeof(T);          // elements per 128-byte box row
                 constexpr int PER16 = 16 / (int)sizeof(T);
-                constexpr int ROUNDS = 128 / (2 * EPR);
-                const uint32_t slot = smem_u32(c_stage) + warp * 2 * PBOX_BYTES;
+                const uint32_t slot = smem_u32(c_stage) + warp * PBOXES * PBOX_BYTES;
+                const bool whole = !GR || row - lane + 32 <= m_end;
 #pragma unroll
-                for (int r = 0; r < ROUNDS; ++r) {
-                    if (lane == 0) tma_store_wait_read();             // the previous boxes have left the slots
-                    __syncwarp();
+                for (int r = 0; r < PCOLS / (PBOXES * EPR); ++r, ++round) {
+                    if (!mbar_wait_warp(taken, (round & 1) ^ 1, abort_flag, (3 << 8) | 2)) { alive = false; break; }      // the previous boxes have been read
+                    if (whole) {
 #pragma unroll
-                    for (int j = 0; j < 16; ++j) {
-                        const uint4 v = pack16<OUT>(&acc[r * 2 * EPR + (j >> 3) * EPR + (j & 7) * PER16]);
-                        asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};"
-                                     ::"r"(slot + (j >> 3) * PBOX_BYTES + lane * 128 + (((j & 7) ^ (lane & 7)) << 4)),
-                                       "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
-                    }
-                    fence_async_smem();
-                    __syncwarp();
-                    if (lane == 0) {
-#pragma unroll
-                        for (int sl = 0; sl < 2; ++sl) {
-                            const int col = col0 + r * 2 * EPR + sl * EPR;
-                            if (col < p.N) tma_store_2d(&tmC, slot + sl * PBOX_BYTES, col, out_row0 + row);
+                        for (int j = 0; j < PBOXES * 8; ++j) {
+                            const uint4 v = pack16<OUT>(&acc[(r * PBOXES + (j >> 3)) * EPR + (j & 7) * PER16]);
+                            asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};"
+                                         ::"r"(slot + (j >> 3) * PBOX_BYTES + lane * 128 + (((j & 7) ^ (lane & 7)) << 4)), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
                         }
-                        tma_store_commit();
+                        fence_async_smem();
+                    } else if (r == 0 && cvalid) {
+                        store_rows_staged<OUT, PCOLS>(acc, c_stage + warp * PBOXES * PBOX_BYTES, p.C, p.ldc, out_row0 + ti.m0 + 128 * (int)rank + q * 32,
+                                                      out_row0 + m_end, col0, p.N, lane);
                     }
-                    __syncwarp();       // the lane rejoins its warp before the next warp-collective instruction
-                }
-            } else if (alive && vec_ok) {
-                // rows of two owners, or an output that TMA cannot write: staged 16-byte stores
-                if (p.tma_out) {
-                    if (lane == 0) tma_store_wait_read();
                     __syncwarp();
+                    if (lane == 0) mbar_arrive(staged);
                 }
-                if (cvalid) store_rows_staged<OUT, 128>(acc, c_stage + warp * 2 * PBOX_BYTES, p.C, p.ldc,
-                                                        out_row0 + ti.m0 + 128 * (int)rank + q * 32, out_row0 + m_end, col0, p.N, lane);
-            } else if (alive && rvalid && cvalid) {
+            } else if (vec_ok) {
+                // an output that TMA cannot write: staged 16-byte stores
+                if (cvalid) store_rows_staged<OUT, PCOLS>(acc, c_stage + warp * PBOXES * PBOX_BYTES, p.C, p.ldc,
+                                                          out_row0 + ti.m0 + 128 * (int)rank + q * 32, out_row0 + m_end, col0, p.N, lane);
+            } else if (rvalid && cvalid) {
                 const int64_t base = (int64_t)(out_row0 + row) * p.ldc + col0;
 #pragma unroll
-                for (int j = 0; j < 16; ++j) {
+                for (int j = 0; j < PCOLS / 8; ++j) {
                     const int ncols = p.N - (col0 + j * 8);
                     if (ncols > 0) store8<OUT>(p.C, base + j * 8, &acc[j * 8], false, ncols);
                 }
             }
         }
-        if (lane == 0) tma_store_wait_all();                // this warp's boxes have reached global memory
     }
 
     // nobody leaves while the other CTA may still read this CTA's shared memory or signal its barriers
     tc_fence_before();
     __syncthreads();
     cluster_sync();
-    if (warp == 9) {
+    if (warp == PMMA) {
         tc_fence_after();
         asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(TMEM_COLS) : "memory");
     }
