@@ -807,33 +807,38 @@ static int launch_split_sum(const float* part, void* out, int64_t n, int splits,
 struct DensePlan { bool pair; int splits; };
 
 // A K block of a tile costs about 0.45 us in either kernel (a pair of SMs does twice the rows in it), a tile about 3 us
-// around its K blocks.  Splitting adds a pass over the partial sums: about 3 us of launch and the bytes at the rate L2
-// returns them.  The plan with the smallest sum of these wins.  Measured with cold operands, launch included: one tile alone 7.2 /
+// around its K blocks on one SM and 1.6 on a pair.  Splitting adds a pass over the partial sums: about 3 us of launch and the bytes at the
+// rate L2 returns them.  The plan with the smallest sum of these wins.  Measured with cold operands, launch included: one tile alone 7.2 /
 // 12.3 / 34.3 us for 4 / 16 / 64 K blocks, a full wave of pairs 9.2 / 15.4 / 43.0, two waves 12.3 / 24.1 / 71.2; whole -> as
-// planned (M x N x K): 64 x 4096 x 7168 29.7 -> 16.3, 300 x 576 x 7168 29.7 -> 15.4 (B MN-major), 512 x 1024 x 32768 117 -> 31,
-// 16 x 18432 x 7168 38.9 -> 34.3, 128 x 512 x 2560 14.3 -> 12.8.  The demands (12 us, a gain of a tenth) leave the problems whole
-// where the second launch eats what is won: 1024 x 4096 x 4096 (22 us), 64 x 7168 x 2048 (12.8).
+// planned (M x N x K): 64 x 4096 x 7168 29.7 -> 16.3, 300 x 576 x 7168 29.7 -> 15.4 (B MN-major), 512 x 1024 x 32768 117 -> 31 on
+// single SMs and 29 on pairs, 16 x 18432 x 7168 38.9 -> 34.3, 128 x 512 x 2560 14.3 -> 12.8.  The demands (12 us, a gain of a tenth) leave the
+// problems whole where the second launch eats what is won: 1024 x 4096 x 4096 (22 us), 64 x 7168 x 2048 (12.8).
 static DensePlan dense_plan(int64_t M, int64_t N, int64_t K, int b_layout, int64_t workspace_bytes, int sms) {
     const int64_t KB = (K + BK - 1) / BK;
     auto waves = [](int64_t tiles, int64_t slots) { return (double)((tiles + slots - 1) / slots); };
     const int64_t pair_tiles = ((M + pair::PM - 1) / pair::PM) * ((N + pair::PN - 1) / pair::PN);
     const int64_t tiles = ((M + BM - 1) / BM) * ((N + BN - 1) / BN);
-    const double block_us = 0.45, tile_us = 3.0;
+    const double block_us = 0.45, tile_us = 3.0, pair_tile_us = 1.6;
     const int pm = pair_mode();
     // the pair kernel wins with B K-major, the one-SM kernel with B MN-major
     DensePlan best{false, 1};
     double best_us = waves(tiles, sms) * (KB * block_us + tile_us);
     // (128 rows would leave a CTA idle; a pair takes two SMs)
-    if (sms >= 2 && (pm == 2 ? pair_tiles >= sm_count() / 2 : (pm == 1 && b_layout == 0 && M > BM))) {
-        const double us = waves(pair_tiles, sms / 2) * (KB * block_us + tile_us);
+    const bool pairs = sms >= 2 && pm == 1 && b_layout == 0 && M > BM;
+    if (pairs || (sms >= 2 && pm == 2 && pair_tiles >= sm_count() / 2)) {
+        const double us = waves(pair_tiles, sms / 2) * (KB * block_us + pair_tile_us);
         if (us <= best_us * 1.02 || pm == 2) { best = {true, 1}; best_us = us; }
     }
     if (best_us < 12.0 || tiles >= sms) return best;
     for (int s = 2; s <= 32 && s * 2 <= KB; ++s) {
         const int64_t bytes = s * M * N * 4;
         if (bytes > workspace_bytes) break;
-        const double us = waves(tiles * s, sms) * ((double)((KB + s - 1) / s) * block_us + tile_us) + 3.0 + bytes / 4e6;
+        const double blocks_us = (double)((KB + s - 1) / s) * block_us, sum_us = 3.0 + bytes / 4e6;
+        const double us = waves(tiles * s, sms) * (blocks_us + tile_us) + sum_us;
         if (us < 0.9 * best_us) { best = {false, s}; best_us = us; }
+        // (partial sums leave through TMA in rows of 16-byte multiples)
+        const double pair_us = waves(pair_tiles * s, sms / 2) * (blocks_us + pair_tile_us) + sum_us;
+        if (pairs && N % 4 == 0 && s * M < (1LL << 31) && pair_us < 0.9 * best_us) { best = {true, s}; best_us = pair_us; }
     }
     return best;
 }
@@ -875,8 +880,17 @@ int fp8_gemm(const void* A, int64_t lda, const float* sA, int64_t ld_sa, const v
     p.C = C; p.ldc = N; p.M = (int)M; p.N = (int)N; p.K = (int)K;
     p.starts = nullptr; p.ends = nullptr; p.E = 1; p.b_rows_per_expert = 0; p.splits = 1;
     if (plan.pair) {
-        const int64_t pair_tiles = ((M + pair::PM - 1) / pair::PM) * ((N + pair::PN - 1) / pair::PN);
+        const int64_t pair_tiles = ((M + pair::PM - 1) / pair::PM) * ((N + pair::PN - 1) / pair::PN) * plan.splits;
         const int clusters = (int)(pair_tiles < sms / 2 ? pair_tiles : sms / 2);
+        if (plan.splits > 1) {
+            p.C = workspace; p.E = plan.splits;
+            CUtensorMap tc;
+            rc = make_out_map(&tc, ta, p, CINN_F32, plan.splits * M, STORE_ROWS, true);
+            if (rc) return rc;
+            rc = launch_pair<false, CINN_F32, true>(ta, tb, tc, p, clusters, st);
+            if (rc) return rc;
+            return launch_split_sum(static_cast<const float*>(workspace), C, M * N, plan.splits, out_dtype, st);
+        }
         return b_layout == 0 ? launch_pair_out<false>(ta, tb, p, out_dtype, clusters, st)
                              : launch_pair_out<true>(ta, tb, p, out_dtype, clusters, st);
     }
@@ -891,6 +905,28 @@ int fp8_gemm(const void* A, int64_t lda, const float* sA, int64_t ld_sa, const v
     }
     return b_layout == 0 ? launch_out<false, false>(ta, tb, p, out_dtype, grid, st)
                          : launch_out<true, false>(ta, tb, p, out_dtype, grid, st);
+}
+
+// Grouped problems run on pairs of SMs and 256-row tiles from 256 rows per expert on average (how the rows are really spread only
+// the device knows): below that the half-empty tiles cost more than the pair saves.  Both directions; for the input gradient, whose
+// weight is read MN-major, 7168 x 4096 of 32 experts, 32768 rows, 1045 -> 920 us, and 512 x 512
+// of 16 experts, 65536 rows, 67 -> 59.
+static bool grouped_on_pairs(int64_t E, int64_t T, int64_t N, int sms) {
+    return pair_mode() != 0 && sms >= 2 && T >= pair::PM * E && (T + pair::PM - 1) / pair::PM * ((N + pair::PN - 1) / pair::PN) >= sms / 2;
+}
+
+template <bool B_MN>
+static int launch_grouped_pair(const CUtensorMap& ta, const CUtensorMap& tb, GemmParams& p, int out_dtype, int clusters, cudaStream_t st) {
+    CUtensorMap tc;
+    int rc = make_out_map(&tc, ta, p, out_dtype, p.M, STORE_ROWS, true);
+    if (rc) return rc;
+    switch (out_dtype) {
+        case CINN_BF16: return launch_pair<B_MN, CINN_BF16, false, true>(ta, tb, tc, p, clusters, st);
+        case CINN_F16: return launch_pair<B_MN, CINN_F16, false, true>(ta, tb, tc, p, clusters, st);
+        case CINN_F32: return launch_pair<B_MN, CINN_F32, false, true>(ta, tb, tc, p, clusters, st);
+        case CINN_F32_BF16: return launch_pair<B_MN, CINN_F32_BF16, false, true>(ta, tb, tc, p, clusters, st);
+        default: set_error("GEMM: unknown output dtype tag %d", out_dtype); return CINN_ERR_INVALID;
+    }
 }
 
 int fp8_grouped_gemm(const void* A, const float* sA, const void* W, const float* sW, const int64_t* starts,
@@ -909,11 +945,8 @@ int fp8_grouped_gemm(const void* A, const float* sA, const void* W, const float*
     CUtensorMap ta, tb;
     int rc = make_map(&ta, A, (uint64_t)d_in, (uint64_t)T, (uint64_t)d_in, BK, BM);
     if (rc) return rc;
-    // Pairs of SMs on 256-row tiles from 256 rows per expert on average (how the rows are really spread only the device
-    // knows): below that the half-empty tiles cost more than the pair saves.
     const int sms = gemm_sms();
-    const bool use_pair = row_dst == nullptr && pair_mode() != 0 && sms >= 2 && T >= pair::PM * E &&
-                          (T + pair::PM - 1) / pair::PM * ((d_out + pair::PN - 1) / pair::PN) >= sms / 2;
+    const bool use_pair = row_dst == nullptr && grouped_on_pairs(E, T, d_out, sms);
     rc = make_map(&tb, W, (uint64_t)d_in, (uint64_t)(E * d_out), (uint64_t)d_in, BK, use_pair ? 128 : BN);
     if (rc) return rc;
     const int64_t nkb = (d_in + 127) / 128, nnb = (d_out + 127) / 128;
@@ -929,19 +962,7 @@ int fp8_grouped_gemm(const void* A, const float* sA, const void* W, const float*
         return out_dtype == CINN_BF16 ? launch<false, true, CINN_BF16, true>(ta, tb, ta, p, sms, st)
                                       : launch<false, true, CINN_F16, true>(ta, tb, ta, p, sms, st);
     }
-    if (use_pair) {
-        CUtensorMap tc;
-        rc = make_out_map(&tc, ta, p, out_dtype, T, STORE_ROWS, true);
-        if (rc) return rc;
-        const int clusters = sms / 2;
-        switch (out_dtype) {
-            case CINN_BF16: return launch_pair<false, CINN_BF16, false, true>(ta, tb, tc, p, clusters, st);
-            case CINN_F16: return launch_pair<false, CINN_F16, false, true>(ta, tb, tc, p, clusters, st);
-            case CINN_F32: return launch_pair<false, CINN_F32, false, true>(ta, tb, tc, p, clusters, st);
-            case CINN_F32_BF16: return launch_pair<false, CINN_F32_BF16, false, true>(ta, tb, tc, p, clusters, st);
-            default: set_error("GEMM: unknown output dtype tag %d", out_dtype); return CINN_ERR_INVALID;
-        }
-    }
+    if (use_pair) return launch_grouped_pair<false>(ta, tb, p, out_dtype, sms / 2, st);
     return launch_out<false, true>(ta, tb, p, out_dtype, sms, st);
 }
 
@@ -973,7 +994,9 @@ int fp8_grouped_gemm_dgrad(const void* dY, const float* sdY, const void* W, cons
     p.sB = sW; p.sb_stride_k = nkb_in; p.sb_stride_n = 1; p.sb_stride_e = nob * nkb_in;
     p.C = dX; p.ldc = d_in; p.M = (int)T; p.N = (int)d_in; p.K = (int)d_out;
     p.starts = starts; p.ends = ends; p.E = (int)E; p.b_rows_per_expert = (int)d_out;
-    return launch_out<true, true>(ta, tb, p, out_dtype, gemm_sms(), st);
+    const int sms = gemm_sms();
+    if (grouped_on_pairs(E, T, d_in, sms)) return launch_grouped_pair<true>(ta, tb, p, out_dtype, sms / 2, st);
+    return launch_out<true, true>(ta, tb, p, out_dtype, sms, st);
 }
 
 // Weight gradients of all experts in one launch (the GK instantiation of the pair kernel): dW (E, d_out, d_in) with

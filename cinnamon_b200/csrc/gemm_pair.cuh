@@ -125,7 +125,8 @@ __device__ __forceinline__ PairTile pair_tile(const GemmParams& p, int t) {
 // of the experts, dW[e] = dY[rows of e]^T @ x[rows of e].  Both operands are K-major over one padded token axis on
 // which expert e owns the K blocks [kb_start[e], kb_start[e + 1]) (p.starts holds that int array, p.E = E); tile t
 // belongs to expert t / (tiles per expert) and is stored at rows e * M + ... of the (E * M, N) output.  An expert
-// without rows gets zeros.  M and N are multiples of 256 here, so every tile is whole.
+// without rows gets zeros.  Without kb_start (null) the E "experts" are equal pieces of one problem's reduction, whose partial sums
+// split_sum_kernel adds.
 //
 // GR ("grouped rows"): E independent problems of the same N x K over the ragged row ranges [starts[e], ends[e]) of A and C
 // (device arrays), B stacked (E * b_rows_per_expert rows).  The tiles of all experts are one list, found through a prefix sum
@@ -203,8 +204,13 @@ fp8_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
         } else if constexpr (GK) {
             e = t / per_expert;
             ti = pair_tile(p, t - e * per_expert);
-            kb0 = kb_start[e];
-            KB = kb_start[e + 1] - kb0;
+            if (kb_start) {
+                kb0 = kb_start[e];
+                KB = kb_start[e + 1] - kb0;
+            } else {
+                kb0 = (int)((int64_t)KB_dense * e / p.E);
+                KB = (int)((int64_t)KB_dense * (e + 1) / p.E) - kb0;
+            }
         } else {
             e = 0; kb0 = 0; KB = KB_dense;
             ti = pair_tile(p, t);
@@ -314,7 +320,7 @@ fp8_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
                     const int col = ti.n0 + h * PCOLS + (r * PBOXES + lane % PBOXES) * EPR;
                     if (!mbar_wait_warp(staged, round & 1, abort_flag, (5 << 8) | 1)) { alive = false; break; }
                     if (lane < PEPI * PBOXES) {
-                        if (col < p.N && (!GR || row + 32 <= m_end)) tma_store_2d(&tmC, smem_u32(c_stage) + lane * PBOX_BYTES, col, out_row0 + row);
+                        if (col < p.N && (!(GR || GK) || row + 32 <= m_end)) tma_store_2d(&tmC, smem_u32(c_stage) + lane * PBOX_BYTES, col, out_row0 + row);
                         tma_store_commit();
                         tma_store_wait_read();
                     }
@@ -412,7 +418,7 @@ fp8_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
                 constexpr int EPR = 128 / (int)sizeof(T);          // elements per 128-byte box row
                 constexpr int PER16 = 16 / (int)sizeof(T);
                 const uint32_t slot = smem_u32(c_stage) + warp * PBOXES * PBOX_BYTES;
-                const bool whole = !GR || row - lane + 32 <= m_end;
+                const bool whole = !(GR || GK) || row - lane + 32 <= m_end;
 #pragma unroll
                 for (int r = 0; r < PCOLS / (PBOXES * EPR); ++r, ++round) {
                     if (!mbar_wait_warp(taken, (round & 1) ^ 1, abort_flag, (3 << 8) | 2)) { alive = false; break; }      // the previous boxes have been read

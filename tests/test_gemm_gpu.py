@@ -69,7 +69,7 @@ def test_gemm_layout_kn(K, M, N, Kd):
     assert err <= TOL and err <= 2e-5
 
 
-@pytest.mark.parametrize("M,N,Kd", [(128, 256, 8192), (1, 64, 7168), (130, 333, 6032), (1024, 512, 8208)])
+@pytest.mark.parametrize("M,N,Kd", [(128, 256, 8192), (1, 64, 7168), (130, 333, 6032), (1024, 512, 8208), (300, 516, 8208), (257, 260, 12304)])
 @pytest.mark.parametrize("kn", [False, True])
 def test_gemm_cut_along_k(K, M, N, Kd, kn):
     """Few tiles, long reduction: partial sums over pieces of K (the last one short), added in a fixed order."""
@@ -365,6 +365,26 @@ def test_grouped_gemm_on_sm_pairs(K, case):
         got = out.cpu()
         assert torch.all(got[~covered] == 777.0), "rows outside every expert's range were written"
         assert rel_fro(got[covered].float(), ref[covered]) <= {torch.float32: 2e-5, torch.bfloat16: 2e-3, torch.float16: 3e-4}[dtype]
+
+
+@pytest.mark.parametrize("case", [(3, 4096, 384, [700, 0, 900]), (2, 9488, 272, [257, 511]), (2, 4880, 144, [1, 1280]), (1, 5008, 128, [1152])])
+def test_grouped_input_gradient_on_sm_pairs(K, case):
+    """The same edges for the input gradient, whose weight is read with the reduction axis outermost (a reduction that ends
+    inside a block meets the next expert's rows under zeros)."""
+    E, d_in, d_out, counts = case
+    x, w, starts, ends = _grouped_case(E, d_in, d_out, counts, seed=d_in, gap=9)
+    dy = torch.randn(x.shape[0], d_out, generator=torch.Generator().manual_seed(d_in)).bfloat16()
+    ref, _ = O.grouped_gemm_fp8_backward_f64(x, w, starts, ends, dy)
+    gq, gs = K.quantize_fp8_rowwise(dy.cuda())
+    wq, ws = K.quantize_expert_weights(w.cuda())
+    inside = torch.zeros(x.shape[0], dtype=torch.bool)
+    for s, e in zip(starts.tolist(), ends.tolist()):
+        inside[s:e] = True
+    for dtype in (torch.float32, torch.bfloat16):
+        got = K.fp8_grouped_gemm_dgrad(gq, gs, wq, ws, starts.cuda(), ends.cuda(), out_dtype=dtype).cpu()
+        assert torch.all(got[~inside] == 0)
+        assert rel_fro(got[inside].float(), ref[inside]) <= {torch.float32: 2e-5, torch.bfloat16: 2e-3}[dtype]
+    assert K.device_status() == 0
 
 
 def test_gemms_under_a_cap_of_one_sm(K):
