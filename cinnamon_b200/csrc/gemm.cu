@@ -74,14 +74,24 @@ __device__ __forceinline__ float ld_scale(const float* p) {
     return v;
 }
 
-// D[tmem] (+)= A[smem desc] * B[smem desc], e4m3 x e4m3 -> fp32.  Called by a whole warp, issued by one elected lane.
-__device__ __forceinline__ void tc_mma_f8(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
+// D[tmem] = A[smem desc] * B[smem desc], e4m3 x e4m3 -> fp32.  Called by a whole warp, issued by one elected lane.
+// The four MMAs of a K block by one statement with one election: one by one, with 64-bit descriptors, they cost their warp 350
+// cycles, like this 100.  Low words of the descriptors; STEP_B: 16-byte units from one step's B to the next.
+template <int STEP_B>
+__device__ __forceinline__ void tc_mma_f8_block(uint32_t d_tmem, uint32_t a_lo, uint32_t b_lo, uint32_t idesc) {
+    constexpr uint32_t hi = (uint32_t)((((uint64_t)(1024 >> 4) << 32) | (1ull << 46) | (2ull << 61)) >> 32);
     asm volatile(
-        "{\n\t.reg .pred p, e;\n\t"
+        "{\n\t.reg .pred e;\n\t.reg .b64 a, b;\n\t.reg .b32 x, y;\n\t"
         "elect.sync _|e, 0xffffffff;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "@e tcgen05.mma.cta_group::1.kind::f8f6f4 [%0], %1, %2, %3, p;\n\t}"
-        ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate) : "memory");
+        "mov.b64 a, {%1, %4};\n\tmov.b64 b, {%2, %4};\n\t"
+        "@e tcgen05.mma.cta_group::1.kind::f8f6f4 [%0], a, b, %3, 0;\n\t"
+        "add.u32 x, %1, 2;\n\tadd.u32 y, %2, %5;\n\tmov.b64 a, {x, %4};\n\tmov.b64 b, {y, %4};\n\t"
+        "@e tcgen05.mma.cta_group::1.kind::f8f6f4 [%0], a, b, %3, 1;\n\t"
+        "add.u32 x, %1, 4;\n\tadd.u32 y, %2, %6;\n\tmov.b64 a, {x, %4};\n\tmov.b64 b, {y, %4};\n\t"
+        "@e tcgen05.mma.cta_group::1.kind::f8f6f4 [%0], a, b, %3, 1;\n\t"
+        "add.u32 x, %1, 6;\n\tadd.u32 y, %2, %7;\n\tmov.b64 a, {x, %4};\n\tmov.b64 b, {y, %4};\n\t"
+        "@e tcgen05.mma.cta_group::1.kind::f8f6f4 [%0], a, b, %3, 1;\n\t}"
+        ::"r"(d_tmem), "r"(a_lo), "r"(b_lo), "r"(idesc), "r"(hi), "n"(STEP_B), "n"(2 * STEP_B), "n"(3 * STEP_B) : "memory");
 }
 
 // Instruction descriptor for kind::f8f6f4: fp32 accumulate, e4m3 x e4m3, A K-major.
@@ -375,6 +385,8 @@ fp8_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
         {
             constexpr uint32_t idesc = make_idesc(B_MN);
             const uint32_t mine = (uint32_t)(warp - (EPI_WARPS + 1));
+            const uint32_t a0 = ((smem_u32(smem_a) >> 4) & 0x3FFF) | (1u << 16);
+            const uint32_t b0 = ((smem_u32(smem_b) >> 4) & 0x3FFF) | ((B_MN ? (uint32_t)B_BYTES / 2 >> 4 : 1u) << 16);
             uint32_t it = 0, last = 0xffffffffu;
             bool alive = true;
             for (int t = blockIdx.x; t < n_total && alive; t += gridDim.x) {
@@ -391,16 +403,7 @@ fp8_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
                     if (!mbar_wait_warp(full0 + 8 * s, ph, abort_flag, (2 << 8) | 1)) { alive = false; break; }
                     if (!mbar_wait_warp(tempty0 + 8 * b, bph ^ 1, abort_flag, (2 << 8) | 2)) { alive = false; break; }
                     tc_fence_after();
-                    const uint32_t a_addr = smem_u32(smem_a + s * A_BYTES);
-                    const uint32_t b_addr = smem_u32(smem_b + s * B_BYTES);
-                    const uint32_t d = tmem_base + b * BN;
-#pragma unroll
-                    for (int k = 0; k < BK / 32; ++k) {
-                        const uint64_t ad = make_smem_desc(a_addr + k * 32, 16, 1024);
-                        const uint64_t bd = B_MN ? make_smem_desc(b_addr + k * 32 * 128, B_BYTES / 2, 1024)
-                                                 : make_smem_desc(b_addr + k * 32, 16, 1024);
-                        tc_mma_f8(d, ad, bd, idesc, k > 0 ? 1u : 0u);
-                    }
+                    tc_mma_f8_block<B_MN ? 256 : 2>(tmem_base + b * BN, a0 + s * (A_BYTES >> 4), b0 + s * (B_BYTES >> 4), idesc);
                     tc_commit(tfull0 + 8 * b);      // the partial tile is ready for promotion once these MMAs retire
                     tc_commit(empty0 + 8 * s);      // and the stage may be refilled
                 }
@@ -541,6 +544,7 @@ fp8_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
 }
 
 #include "gemm_pair.cuh"
+#include "gemm_rows.cuh"
 #include "gemm16.cuh"
 
 // ---------------------------------------------------------------------------
@@ -804,7 +808,42 @@ static int launch_split_sum(const float* part, void* out, int64_t n, int splits,
     return CINN_OK;
 }
 
-struct DensePlan { bool pair; int splits; };
+struct DensePlan { bool pair; int splits; bool rows; };
+
+template <int ROWS>
+static int launch_rows(const CUtensorMap& ta, const CUtensorMap& tb, const GemmParams& p, int out_dtype, cudaStream_t st) {
+    const dim3 grid((unsigned)((p.N + rows::RN - 1) / rows::RN), (unsigned)((p.M + 127) / 128));
+    auto go = [&](auto kern, int (*allow)(size_t)) {
+        int rc = allow(rows::Shape<ROWS>::BYTES);
+        if (rc) return rc;
+        CINN_CHECK_CUDA(launch_dependent(kern, grid, dim3(rows::RTHREADS), rows::Shape<ROWS>::BYTES, st, ta, tb, p));
+        CINN_CHECK_LAUNCH();
+        return (int)CINN_OK;
+    };
+#define CINN_ROWS(O) case O: return go(rows::fp8_gemm_rows_kernel<ROWS, O>, allow_smem_once<rows::fp8_gemm_rows_kernel<ROWS, O>>)
+    switch (out_dtype) {
+        CINN_ROWS(CINN_BF16);
+        CINN_ROWS(CINN_F32);
+        CINN_ROWS(CINN_F16);
+        CINN_ROWS(CINN_F32_BF16);
+        default: set_error("GEMM: unknown output dtype tag %d", out_dtype); return CINN_ERR_INVALID;
+    }
+#undef CINN_ROWS
+}
+
+// The kernel for few rows: where its CTAs of 32 columns fit on the SMs twice and the reduction is short; without a workspace, that is
+// where the alternative is a handful of long tiles, also where it is long.  us with cold operands, launch included, other kernels ->
+// this one (rows x columns x reduction): 128 x 1024 x 512 12.3 -> 8.2, 512 x 1024 x 512 13.1 -> 8.2, 128 x 512 x 2048 17.2 -> 10.2, 256 x 2560 x
+// 1024 15.2 -> 11.0, 512 of them 14.5 -> 13.1, 64 x 7168 x 2048 18.4 -> 12.3, 64 x 4096 x 7168 whole 36 -> 20.5; on the other side of
+// the line 256 x 7168 x 2048 18.4 -> 20.4, 64 x 18432 x 7168 43.8 and 43.0, 64 x 4096 x 7168 cut 23.6, 64 x 576 x 7168 cut 19.5
+// and 19.3, 64 x 7168 x 18432 cut 46.1 and 47.1.
+static bool rows_pay(int64_t M, int64_t N, int64_t K, int b_layout, int64_t workspace_bytes, int sms) {
+    if (b_layout != 0 || pair_mode() != 1 || sms < sm_count()) return false;
+    const int64_t KB = (K + BK - 1) / BK, blocks = (N + rows::RN - 1) / rows::RN * ((M + 127) / 128);
+    if (blocks > 2 * sms) return false;
+    if (M <= 128 && workspace_bytes == 0) return true;
+    return KB <= 40 && (M <= 128 || blocks * KB <= 16 * sms);
+}
 
 // A K block of a tile costs about 0.45 us in either kernel (a pair of SMs does twice the rows in it), a tile about 3 us
 // around its K blocks on one SM and 1.6 on a pair.  Splitting adds a pass over the partial sums: about 3 us of launch and the bytes at the
@@ -821,13 +860,14 @@ static DensePlan dense_plan(int64_t M, int64_t N, int64_t K, int b_layout, int64
     const double block_us = 0.45, tile_us = 3.0, pair_tile_us = 1.6;
     const int pm = pair_mode();
     // the pair kernel wins with B K-major, the one-SM kernel with B MN-major
-    DensePlan best{false, 1};
+    if (rows_pay(M, N, K, b_layout, workspace_bytes, sms)) return {false, 1, true};
+    DensePlan best{false, 1, false};
     double best_us = waves(tiles, sms) * (KB * block_us + tile_us);
     // (128 rows would leave a CTA idle; a pair takes two SMs)
     const bool pairs = sms >= 2 && pm == 1 && b_layout == 0 && M > BM;
     if (pairs || (sms >= 2 && pm == 2 && pair_tiles >= sm_count() / 2)) {
         const double us = waves(pair_tiles, sms / 2) * (KB * block_us + pair_tile_us);
-        if (us <= best_us * 1.02 || pm == 2) { best = {true, 1}; best_us = us; }
+        if (us <= best_us * 1.02 || pm == 2) { best = {true, 1, false}; best_us = us; }
     }
     if (best_us < 12.0 || tiles >= sms) return best;
     for (int s = 2; s <= 32 && s * 2 <= KB; ++s) {
@@ -835,10 +875,10 @@ static DensePlan dense_plan(int64_t M, int64_t N, int64_t K, int b_layout, int64
         if (bytes > workspace_bytes) break;
         const double blocks_us = (double)((KB + s - 1) / s) * block_us, sum_us = 3.0 + bytes / 4e6;
         const double us = waves(tiles * s, sms) * (blocks_us + tile_us) + sum_us;
-        if (us < 0.9 * best_us) { best = {false, s}; best_us = us; }
+        if (us < 0.9 * best_us) { best = {false, s, false}; best_us = us; }
         // (partial sums leave through TMA in rows of 16-byte multiples)
         const double pair_us = waves(pair_tiles * s, sms / 2) * (blocks_us + pair_tile_us) + sum_us;
-        if (pairs && N % 4 == 0 && s * M < (1LL << 31) && pair_us < 0.9 * best_us) { best = {true, s}; best_us = pair_us; }
+        if (pairs && N % 4 == 0 && s * M < (1LL << 31) && pair_us < 0.9 * best_us) { best = {true, s, false}; best_us = pair_us; }
     }
     return best;
 }
@@ -869,9 +909,9 @@ int fp8_gemm(const void* A, int64_t lda, const float* sA, int64_t ld_sa, const v
     const int sms = gemm_sms();
     const DensePlan plan = dense_plan(M, N, K, b_layout, workspace ? workspace_bytes : 0, sms);
     CUtensorMap ta, tb;
-    int rc = make_map(&ta, A, (uint64_t)K, (uint64_t)M, (uint64_t)lda, BK, BM);
+    int rc = make_map(&ta, A, (uint64_t)K, (uint64_t)M, (uint64_t)lda, BK, plan.rows && M <= 64 ? 64 : BM);
     if (rc) return rc;
-    if (b_layout == 0) rc = make_map(&tb, B, (uint64_t)K, (uint64_t)N, (uint64_t)ldb, BK, plan.pair ? 128 : BN);
+    if (b_layout == 0) rc = make_map(&tb, B, (uint64_t)K, (uint64_t)N, (uint64_t)ldb, BK, plan.rows ? rows::RN : plan.pair ? 128 : BN);
     else rc = make_map(&tb, B, (uint64_t)N, (uint64_t)K, (uint64_t)ldb, 128, BK);
     if (rc) return rc;
     GemmParams p{};
@@ -879,6 +919,7 @@ int fp8_gemm(const void* A, int64_t lda, const float* sA, int64_t ld_sa, const v
     p.sB = sB; p.sb_stride_k = sbk; p.sb_stride_n = sbn; p.sb_stride_e = 0;
     p.C = C; p.ldc = N; p.M = (int)M; p.N = (int)N; p.K = (int)K;
     p.starts = nullptr; p.ends = nullptr; p.E = 1; p.b_rows_per_expert = 0; p.splits = 1;
+    if (plan.rows) return M <= 64 ? launch_rows<64>(ta, tb, p, out_dtype, st) : launch_rows<128>(ta, tb, p, out_dtype, st);
     if (plan.pair) {
         const int64_t pair_tiles = ((M + pair::PM - 1) / pair::PM) * ((N + pair::PN - 1) / pair::PN) * plan.splits;
         const int clusters = (int)(pair_tiles < sms / 2 ? pair_tiles : sms / 2);

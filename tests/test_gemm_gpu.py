@@ -88,6 +88,22 @@ def test_gemm_cut_along_k(K, M, N, Kd, kn):
         assert torch.equal(out, K.fp8_matmul_dsv3(_f8(xq), b, xs.cuda(), ws.cuda().t(), out_dtype=dtype))
 
 
+@pytest.mark.parametrize("N,Kd", [(1024, 512), (333, 144), (576, 2064), (40, 16), (4096, 7168)])
+def test_few_rows_have_the_bits_of_many(K, N, Kd):
+    """The kernel for few rows forms the sums of the others: every row of a small call equals that row of a large one, for one,
+    a part of, all and more than a tile of rows, columns that end inside a block, reductions that end inside a K block."""
+    M = 8192 if N * Kd < 1 << 20 else 4096
+    xq, xs, wq, ws = _operands(M, N, Kd, seed=N + Kd)
+    a, sa, b, sb = _f8(xq), xs.cuda(), _f8(wq), ws.cuda()
+    for dtype in (torch.bfloat16, torch.float32, torch.float16):
+        whole = K.fp8_matmul_dsv3(a, b.t(), sa, sb.t(), out_dtype=dtype)
+        for m in (1, 63, 64, 65, 128, 129, 300):
+            few = K.fp8_matmul_dsv3(a[:m].contiguous(), b.t(), sa[:m].contiguous(), sb.t(), out_dtype=dtype)
+            if K._L.cinn_fp8_gemm_workspace_bytes(m, N, Kd, 0) == 0:       # (a cut reduction adds in another order)
+                assert torch.equal(few, whole[:m]), (m, dtype)
+    assert K.device_status() == 0
+
+
 PAIR_SCRIPT = r"""
 import sys, torch
 sys.path.insert(0, sys.argv[1])
