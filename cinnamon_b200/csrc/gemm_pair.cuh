@@ -179,6 +179,9 @@ fp8_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
 
+    // A 4-byte tile leaves in two rounds: its promotion warps hand over their own boxes, so that each waits for its own to be read
+    // and not for everybody's (32 experts with 127 rows each, 768 x 3584 gradients: FIGT).
+    constexpr bool STORE_WARP = sizeof(typename OutT<OUT>::type) == 2;
     const int KB_dense = (p.K + BK - 1) / BK;
     const int per_expert = pair_total(p);
     const int n_tiles = (p.N + PN - 1) / PN;
@@ -306,7 +309,7 @@ fp8_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
         // ------------------------------ finished tiles to the TMA unit (both CTAs) ------------------------------
         // A lane sends a box.  A tile's 64 KiB leave the SM in a thousand cycles and an issue blocks until the unit
         // takes it: promotion warps that issued their own stores stood still for most of that.
-        if (p.tma_out) {
+        if (STORE_WARP && p.tma_out) {
             constexpr int EPR = 128 / (int)sizeof(typename OutT<OUT>::type);
             const int w = lane / PBOXES, q = w & 3, h = w >> 2;
             uint32_t round = 0;
@@ -410,10 +413,10 @@ fp8_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
             const bool cvalid = col0 < p.N;
             const int out_row0 = GR ? 0 : e * p.M;                      // GK: the expert's slice of the (E * M, N) output
             if (p.tma_out) {
-                // The tile leaves through TMA stores, which the store warp issues.  Every promotion warp owns a box of 32 rows x 128
-                // bytes (128-byte swizzle) of the staging area, where its lanes drop their rows in 16-byte chunks.  A 2-byte
-                // output fits the warp's 64 columns in one round; a 4-byte output takes two rounds of 32.  Rows of two
-                // owners leave as staged 16-byte stores.
+                // The tile leaves through TMA stores.  Every promotion warp owns two boxes of 32 rows x 128 bytes (128-byte swizzle) of the
+                // staging area, where its lanes drop their rows in 16-byte chunks.  A 2-byte output fits the warp's 128 columns in one
+                // round, and the store warp issues it; a 4-byte output takes two rounds of 64.  Rows of two owners leave as
+                // staged 16-byte stores.
                 using T = typename OutT<OUT>::type;
                 constexpr int EPR = 128 / (int)sizeof(T);          // elements per 128-byte box row
                 constexpr int PER16 = 16 / (int)sizeof(T);
@@ -421,7 +424,12 @@ fp8_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
                 const bool whole = !(GR || GK) || row - lane + 32 <= m_end;
 #pragma unroll
                 for (int r = 0; r < PCOLS / (PBOXES * EPR); ++r, ++round) {
-                    if (!mbar_wait_warp(taken, (round & 1) ^ 1, abort_flag, (3 << 8) | 2)) { alive = false; break; }      // the previous boxes have been read
+                    if constexpr (STORE_WARP) {                   // the previous boxes have been read
+                        if (!mbar_wait_warp(taken, (round & 1) ^ 1, abort_flag, (3 << 8) | 2)) { alive = false; break; }
+                    } else {
+                        if (lane == 0) tma_store_wait_read();
+                        __syncwarp();
+                    }
                     if (whole) {
 #pragma unroll
                         for (int j = 0; j < PBOXES * 8; ++j) {
@@ -435,7 +443,19 @@ fp8_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
                                                       out_row0 + m_end, col0, p.N, lane);
                     }
                     __syncwarp();
-                    if (lane == 0) mbar_arrive(staged);
+                    if constexpr (STORE_WARP) {
+                        if (lane == 0) mbar_arrive(staged);
+                    } else {
+                        if (whole && lane == 0) {
+#pragma unroll
+                            for (int b = 0; b < PBOXES; ++b) {
+                                const int col = col0 + (r * PBOXES + b) * EPR;
+                                if (col < p.N) tma_store_2d(&tmC, slot + b * PBOX_BYTES, col, out_row0 + row);
+                            }
+                            tma_store_commit();
+                        }
+                        __syncwarp();   // the lane rejoins its warp before the next warp-collective instruction
+                    }
                 }
             } else if (vec_ok) {
                 // an output that TMA cannot write: staged 16-byte stores
@@ -450,6 +470,7 @@ fp8_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
                 }
             }
         }
+        if (!STORE_WARP && lane == 0) tma_store_wait_all();            // this warp's boxes have reached global memory
     }
 
     // nobody leaves while the other CTA may still read this CTA's shared memory or signal its barriers
