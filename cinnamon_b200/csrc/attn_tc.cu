@@ -243,7 +243,8 @@ __device__ __forceinline__ void softmax_chunk(uint32_t t_s, uint32_t t_lead, uin
 // before any of it is written.
 template <int WARPS>
 __device__ __forceinline__ void by_slot(const uint16_t* rank, float* attn, const float* lse, int rows, int K, float scale, int warp, int lane) {
-    if (K >= 4 && K <= 512 && (K & (K - 1)) == 0) {
+    // (a caller's buffer may start on any 4-byte boundary: rows there go slot by slot)
+    if (K >= 4 && K <= 512 && (K & (K - 1)) == 0 && (reinterpret_cast<uintptr_t>(attn) & 15) == 0) {
         // whole rows in batches of 512 slots, four in a row per lane and load
         const int log_k = 31 - __clz(K), end = rows << log_k;
 #pragma unroll 1

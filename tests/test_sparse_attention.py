@@ -226,6 +226,49 @@ def test_tiles_with_wide_scores(dtype, shape):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("H", [3, 80])                    # a block per SM, two of them
+@pytest.mark.parametrize("Ks", [4, 64, 24])
+def test_tiles_with_probabilities_at_odd_addresses(dtype, H, Ks):
+    """A C caller's probabilities may start on a 4-byte boundary only (a slice of an arena): still the tiles, without their
+    16-byte stores.  The output has the same bits; the probabilities differ by whether score x scale is rounded before
+    the sum of exponentials is taken off it: 2^-24 of a score below 16, so 1e-6 of the probability, and as much for the exponent."""
+    import ctypes
+    from cinnamon_b200 import kernels as K
+    lib = K._lib.lib
+    g = torch.Generator().manual_seed(H + Ks)
+    B, L, dqk, dv = 1, 257, 64, 64
+    tag = {torch.bfloat16: 0, torch.float32: 1}[dtype]
+    q, k = (torch.randn(B, H, L, dqk, generator=g).to(dtype).cuda() for _ in range(2))
+    v = torch.randn(B, H, L, dv, generator=g).to(dtype).cuda()
+    idx = torch.randint(0, L, (B, L, Ks), generator=g).cuda()
+    st = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+    p = lambda t: ctypes.c_void_p(t.data_ptr())                                        # noqa: E731
+    before = K._L.cinn_set_sparse_attn_dense(1)
+    try:
+        need = lib.cinn_sparse_attn_workspace_bytes(B, H, L, Ks, dqk, dv, tag, 0)
+        assert need > 0
+        ws = torch.empty(need, dtype=torch.uint8, device="cuda")
+        results = []
+        for shift in (0, 1, 2, 3):
+            n = B * H * L * Ks
+            arena = torch.full((n + 8,), 7.0, device="cuda")
+            attn = arena[shift:shift + n]
+            assert attn.data_ptr() % 16 == 4 * shift
+            out, lse = torch.empty(B, H, L, dv, device="cuda"), torch.empty(B, H, L, device="cuda")
+            K._lib.check(lib.cinn_sparse_attn_fwd_ws(p(q), p(k), p(v), tag, p(idx), p(out), None, p(lse), p(attn), B, H, L, Ks, dqk, dv,
+                                                     0.125, p(ws), need, st), "fwd")
+            assert torch.all(arena[:shift] == 7) and torch.all(arena[shift + n:] == 7)
+            results.append((out, lse, attn))
+    finally:
+        K._L.cinn_set_sparse_attn_dense(before)
+    for out, lse, attn in results[1:]:
+        assert torch.equal(out, results[0][0]) and torch.equal(lse, results[0][1])
+        torch.testing.assert_close(attn, results[0][2], rtol=3e-6, atol=1e-9)
+    assert K.device_status() == 0
+
+
+@pytest.mark.gpu
 def test_tiles_fall_back_on_the_device(attention_path):
     """What the tiles cannot express: a key picked more than 255 times, and rows nobody picked that hold NaN or infinity."""
     from cinnamon_b200 import kernels as K
