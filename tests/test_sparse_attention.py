@@ -269,6 +269,33 @@ def test_tiles_with_probabilities_at_odd_addresses(dtype, H, Ks):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("H", [2, 160])                   # a block per SM, two of them
+@pytest.mark.parametrize("keys,Ks", [(1, 200), (23, 33), (140, 120), (300, 512)])
+def test_tiles_weigh_repeated_picks(dtype, H, keys, Ks):
+    """Keys picked up to 200 times by a query: one key, a row of consecutive ones (sixteen counts a chunk), some of many; lists whose
+    counts start on every byte of a word, the last query's among them."""
+    from cinnamon_b200 import kernels as K
+    B, L, Dqk, Dv = 1, 300, 64, 64
+    g = torch.Generator().manual_seed(H + Ks)
+    q, k = (torch.randn(B, H, L, Dqk, generator=g).to(dtype) for _ in range(2))
+    v = torch.randn(B, H, L, Dv, generator=g).to(dtype)
+    idx = torch.randint(0, keys, (B, L, Ks), generator=g)
+    idx[0, ::3] += (torch.arange(0, L, 3) - keys).clamp(min=0)[:, None]                # the last keys before a query
+    before = K._L.cinn_set_sparse_attn_dense(1)
+    try:
+        out, attn = K.sparse_attention(q.cuda(), k.cuda(), v.cuda(), idx.cuda())
+    finally:
+        K._L.cinn_set_sparse_attn_dense(before)
+    heads = sorted({0, H // 2, H - 1})
+    ref_out, ref_attn, _ = SO.forward(q[:, heads], k[:, heads], v[:, heads], idx, Dqk ** -0.5)
+    tol = {torch.float32: 1e-5, torch.bfloat16: 8e-3}[dtype]                            # bf16: rounding of the returned output
+    torch.testing.assert_close(out[:, heads].float().cpu().double(), ref_out, rtol=tol, atol=tol)
+    torch.testing.assert_close(attn[:, heads].cpu().double(), ref_attn, rtol=2e-5, atol=1e-7)
+    assert K.device_status() == 0
+
+
+@pytest.mark.gpu
 def test_tiles_fall_back_on_the_device(attention_path):
     """What the tiles cannot express: a key picked more than 255 times, and rows nobody picked that hold NaN or infinity."""
     from cinnamon_b200 import kernels as K
