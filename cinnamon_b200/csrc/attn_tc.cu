@@ -194,9 +194,9 @@ __device__ __forceinline__ void tile_of_block(int n_tiles, int BH, int group, in
 }
 
 // Shared memory: queries [part][64-column panel] | ring of panels | barriers | row maxima on their way between two warps.
-// With one part and more blocks than SMs two CTAs share an SM, each with one pair of softmax warpgroups: the first loads, the
+// With one part and many blocks two CTAs share an SM, each with one pair of softmax warpgroups: the first loads, the
 // merge and the permutation of one run under the other's tiles (a CTA of two pairs spends 20 000 of its 55 000 cycles on them, at
-// 8 x 8 x 1531 queries of 192: 195 us, 186 with one pair).  A block that has an SM to itself has two pairs (1 x 4 x 700 queries: 48 -> 45 us a call).
+// 8 x 8 x 1531 queries of 192).  Where that pays: one_pair.
 // Three parts of 192 columns need most of an SM's shared memory for the queries alone.
 template <int NS, int ND, int PAIRS_> struct FwdShape {
     static constexpr int PAIRS = PAIRS_;                   // of softmax warpgroups
@@ -329,7 +329,8 @@ __device__ __forceinline__ void by_slot(const uint16_t* rank, float* attn, const
 // output (by rank; permuted and normalised at the end).  256 columns per pair: 128 scores, 64 leading parts, 64 of output.
 // Bound by the instructions per score (29, the merge and the permutation among them; they issue in 47 % of the cycles) and, in
 // fp32, by the panels' way into shared memory: the operands of 72 MMAs and the 15 panels of a tile take 7300 cycles of its bandwidth.
-// 8 x 8 x 1531 queries of 192 in bf16: 210 us with two warpgroups per CTA, a thread per row, 168 so; 32 x 8 x 1024 in fp32 655 and 618.  (Skipping
+// The call of 8 x 8 x 1531 queries of 192 in bf16 takes 229 us with two warpgroups per CTA, a thread per row, and 188 so (190 with two pairs);
+// 256 heads of 947 in fp32 831 and 771.  (Skipping
 // chunks that no query of a warp picked from: 2 % slower; the next chunk's scores in flight during this one's: 6 % slower, spills.)
 // NS: bf16 parts of q, k, v; ND: 64-column panels of q and k.
 template <int NS, int ND, int PAIRS>
@@ -1384,11 +1385,35 @@ static int launch_fwd_pairs(const CUtensorMap& tq, const CUtensorMap& tk, const 
     return CINN_OK;
 }
 
+// One pair of softmax warpgroups per CTA and two CTAs per SM, or two pairs in one CTA.  A block of one pair takes 1.4 times as long for
+// its keys, and a call ends no sooner than a block of the last query tile has, so one pair needs more blocks per SM the longer the
+// sequence is.  Up to three rounds of blocks, two rounds of one pair are as long as three of two.  Short blocks that all fit on the
+// SMs at once are the exception, and with two value panels, of which one writes no probabilities, those of two rounds.
+// Call times in us, one pair -> two (heads x queries of 192 | 64, bf16, 128 picks): 11 x 2048 102 -> 74, 18 x 2048 109 -> 94,
+// 25 x 2048 133 -> 125, 38 x 2048 178 -> 176, 50 x 2048 211 -> 217, 85 x 512 92 -> 84, 150 x 512 123 -> 127, 296 x 128 53 -> 57.
+static bool one_pair(int64_t blocks, int64_t n_tiles, int panels, int value_panels, int sms) {
+    if (blocks <= sms) return false;
+    if (blocks <= 2 * sms) return n_tiles <= 2 || (n_tiles <= 6 && panels + value_panels == 2 && 5 * blocks >= 6 * sms);
+    if (blocks <= 3 * sms) return n_tiles <= 6 && value_panels == 2;
+    return 8 * blocks > (24 + (n_tiles > 4 ? n_tiles - 4 : 0)) * sms;
+}
+
+// Heads per group of the forward: groups of one size, so that no small last one ends alone on its long blocks, with about three rounds of
+// blocks each (six of half an SM for long sequences; on short ones that is up to 5 % slower).  Call times, three rounds and
+// the rest in the last group -> this: 31 x 2048 queries of 192 198 -> 152 us with one pair, 62 x 2048 297 -> 256, 19 x 4096 362 -> 268.
+static int forward_group(const Plan& p, bool one) {
+    const int64_t tiles = p.Lp / T, want = ((one && tiles >= 12 ? 6 : 3) * sm_count() + tiles - 1) / tiles;
+    const int64_t groups = (p.BH + want - 1) / want;
+    return (int)((p.BH + groups - 1) / groups);
+}
+
 template <int NS, int ND>
-static int launch_fwd(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const FwdArgs& a, const Plan& p, cudaStream_t st) {
+static int launch_fwd(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, FwdArgs& a, const Plan& p, cudaStream_t st) {
     const dim3 grid((unsigned)(p.Lp / T * p.BH), 1, (unsigned)p.nv);
+    const bool one = NS == 1 && one_pair((int64_t)grid.x * grid.z, p.Lp / T, ND, p.nv, sm_count());
+    a.group = forward_group(p, one);
     if constexpr (NS == 1)
-        if ((int64_t)grid.x * grid.z > sm_count()) return launch_fwd_pairs<NS, ND, 1>(tq, tk, tv, a, grid, st);
+        if (one) return launch_fwd_pairs<NS, ND, 1>(tq, tk, tv, a, grid, st);
     return launch_fwd_pairs<NS, ND, 2>(tq, tk, tv, a, grid, st);
 }
 
@@ -1425,7 +1450,7 @@ int forward(const void* q, const void* k, const void* v, int dtype, const int64_
     a.picks = picks_of(p, ws);
     a.out = out; a.out_cast = out_cast; a.lse = lse; a.attn = attn; a.flag = reinterpret_cast<int*>(ws + p.flag_off);
     a.H = (int)H; a.L = (int)L; a.words = (int)(p.Lp / 32); a.K = (int)K; a.Dv = (int)Dv; a.BH = (int)p.BH; a.scale = scale;
-    a.n_tiles = (int)(p.Lp / T); a.group = head_group(p);
+    a.n_tiles = (int)(p.Lp / T);
     a.out_cast_tag = dtype;
     if (p.ns == 1) {
         switch (p.nd) {

@@ -296,6 +296,65 @@ def test_tiles_weigh_repeated_picks(dtype, H, keys, Ks):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("shape", [(1, 160, 300, 40, 192, 64), (2, 76, 257, 33, 128, 64), (1, 150, 385, 64, 192, 128), (1, 230, 250, 24, 128, 100),
+                                   (4, 37, 400, 16, 64, 128), (1, 45, 2048, 128, 192, 64), (1, 60, 130, 100, 192, 64), (1, 80, 256, 512, 72, 72),
+                                   (1, 37, 1500, 32, 192, 64)])
+def test_tiles_of_many_heads(dtype, shape):
+    """More blocks than SMs: every width of queries and values with one pair of warpgroups per CTA and two CTAs per SM, lists of a power
+    of two of slots and others, heads in one and in several groups, the last of them smaller; and the shapes that keep two pairs."""
+    from cinnamon_b200 import kernels as K
+    B, H, L, Ks, Dqk, Dv = shape
+    g = torch.Generator().manual_seed(sum(shape))
+    q, k = (torch.randn(B, H, L, Dqk, generator=g).to(dtype) for _ in range(2))
+    v = torch.randn(B, H, L, Dv, generator=g).to(dtype)
+    idx = torch.randint(-2, L + 2, (B, L, Ks), generator=g)
+    idx[:, L // 2] = L + 1                                # a query without any valid key
+    before = K._L.cinn_set_sparse_attn_dense(1)
+    try:
+        out, attn = K.sparse_attention(q.cuda(), k.cuda(), v.cuda(), idx.cuda())
+    finally:
+        K._L.cinn_set_sparse_attn_dense(before)
+    heads = sorted({0, H // 2, H - 2, H - 1})
+    ref_out, ref_attn, _ = SO.forward(q[:, heads], k[:, heads], v[:, heads], idx, Dqk ** -0.5)
+    tol = {torch.bfloat16: 8e-3, torch.float16: 1e-3}[dtype]                            # rounding of the returned output
+    torch.testing.assert_close(out[:, heads].float().cpu().double(), ref_out, rtol=tol, atol=tol)
+    torch.testing.assert_close(attn[:, heads].cpu().double(), ref_attn, rtol=2e-5, atol=1e-7)
+    assert K.device_status() == 0
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("H", [2, 160])
+def test_tiles_of_many_heads_fall_back(dtype, H):
+    """A NaN key that some queries picked, a key picked more than 255 times: with a block per SM and with two, the numbers and the NaNs
+    of the gathers."""
+    from cinnamon_b200 import kernels as K
+    g = torch.Generator().manual_seed(H)
+    q, k, v = (torch.randn(1, H, 384, 64, generator=g).to(dtype).cuda() for _ in range(3))
+    idx = torch.randint(0, 100, (1, 384, 264), generator=g).cuda()
+    idx[idx == 17] = 18
+    for nan in (True, False):
+        if nan:
+            k[0, H // 2, 300, 3] = float("nan")
+            idx[0, 301:340, 5] = 300
+        else:
+            k.nan_to_num_(0.0)
+            idx[0, 200, :] = 7
+        got = []
+        for mode in (1, 0):
+            before = K._L.cinn_set_sparse_attn_dense(mode)
+            try:
+                got.append(K.sparse_attention(q, k, v, idx))
+            finally:
+                K._L.cinn_set_sparse_attn_dense(before)
+        assert bool(torch.isnan(got[0][0][0, H // 2, 301:340]).all()) == nan and not torch.isnan(got[0][0][0, 0]).any()
+        for a, b in zip(*got):
+            torch.testing.assert_close(a, b, rtol=1e-5 if dtype == torch.float32 else 8e-3, atol=1e-6, equal_nan=True)
+    assert K.device_status() == 0
+
+
+@pytest.mark.gpu
 def test_tiles_fall_back_on_the_device(attention_path):
     """What the tiles cannot express: a key picked more than 255 times, and rows nobody picked that hold NaN or infinity."""
     from cinnamon_b200 import kernels as K
