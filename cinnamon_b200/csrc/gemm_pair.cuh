@@ -33,14 +33,16 @@ constexpr int PTHREADS = (PEPI + 4) * 32;
 constexpr int PSCALE_SLOTS = 4;         // K blocks whose scale products are in shared memory: [slot][128 columns][row]
 constexpr int PSCALE_BYTES = PSCALE_SLOTS * 2 * 128 * 4;
 constexpr int PTILE_SLOTS = 16;         // coordinates of the next tiles: {m0, n0, one past the last row, expert}
-// dynamic shared memory: operand stages | a 4 KiB output box per promotion warp = the CTA's whole 128 x 256 tile of a
-// 2-byte type (TMA-store boxes; also the 2 KiB-per-warp staging of the non-TMA path) | scale products | tiles | 256 B of barriers and
+// dynamic shared memory: operand stages | two 4 KiB output boxes per promotion warp = the CTA's whole 128 x 256 tile of a
+// 2-byte type (TMA-store boxes; also the 2 KiB-per-warp staging of the non-TMA path) | scale products | scales on their way | tiles | 256 B of barriers and
 // flags, plus 1 KiB of slack to align the stages to 1024 bytes
 constexpr int PSTAGE_OFF = PSTAGES * (PA_BYTES + PB_BYTES);
 constexpr int PBOX_BYTES = STORE_ROWS * 128;  // one TMA-store box
 constexpr int PBOXES = 16 / PEPI;       // boxes per promotion warp: a round of them all is 64 KiB, a CTA's tile of a 2-byte type
 constexpr int PC_BYTES = PEPI * PBOXES * PBOX_BYTES;
-constexpr size_t PSMEM_BYTES = (size_t)PSTAGE_OFF + PC_BYTES + PSCALE_BYTES + PTILE_SLOTS * 16 + 256 + 1024;
+constexpr int PFETCH = 8;               // K blocks whose scales are on their way
+constexpr int PRAW = 128 + 4;           // floats of one: a row's each, two columns'
+constexpr size_t PSMEM_BYTES = (size_t)PSTAGE_OFF + PC_BYTES + PSCALE_BYTES + PFETCH * PRAW * 4 + PTILE_SLOTS * 16 + 256 + 1024;
 
 __device__ __forceinline__ uint32_t cluster_ctarank() {
     uint32_t r;
@@ -142,7 +144,8 @@ fp8_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
     uint8_t* smem_b = smem + PSTAGES * PA_BYTES;
     uint8_t* c_stage = smem + PSTAGE_OFF;
     float* scales = reinterpret_cast<float*>(c_stage + PC_BYTES);
-    int4* tiles = reinterpret_cast<int4*>(c_stage + PC_BYTES + PSCALE_BYTES);
+    float* raw = reinterpret_cast<float*>(c_stage + PC_BYTES + PSCALE_BYTES);
+    int4* tiles = reinterpret_cast<int4*>(raw + PFETCH * PRAW);
     uint64_t* bars = reinterpret_cast<uint64_t*>(tiles + PTILE_SLOTS);
     // [0, S) full (used in the leader), [S, 2S) empty, [2S, 2S+2) tmem full, [2S+2, 2S+4) tmem empty (leader), then: all boxes of a
     // round are staged, they have been read
@@ -249,15 +252,16 @@ fp8_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
             }
         }
     } else if (warp == PSCALE) {
-        // ------------------ scales (both CTAs): K block `it`'s products sA sB of this CTA's rows, FETCH blocks ahead in registers ------------------
-        constexpr int FETCH = 4;
+        // ------------------ scales (both CTAs): K block `it`'s products sA sB of this CTA's rows ------------------
+        // They come PFETCH blocks ahead, copied to shared memory.  Through registers, a block's values waited for the loads issued last, four
+        // blocks on: a miss for every row each eighth block (8837 x 17024 -> 320, one wave of tiles: 101 us so, 69 like this).
         const float* a_ptr[4];
         const float* b_ptr[2];
         int t = cluster_id - n_clusters, left = 0;     // K blocks of the tile that are still to be fetched
         uint32_t entered = 0;
         uint32_t fetched = 0;
-        float va[FETCH][4], vb[FETCH][2];
-        auto fetch = [&](float (&x)[4], float (&y)[2]) {
+        auto copy4 = [](uint32_t dst, const float* src) { asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst), "l"(src) : "memory"); };
+        auto fetch = [&](uint32_t slot) {
             while (left == 0) {
                 t += n_clusters;
                 if (t >= n_total) { t = n_total; return; }           // (and stays there)
@@ -278,33 +282,41 @@ fp8_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
                                + (GR ? (int64_t)e * p.sb_stride_e : 0);
                 }
             }
+            const uint32_t to = smem_u32(raw + slot * PRAW);
 #pragma unroll
-            for (int i = 0; i < 4; ++i) { x[i] = ld_scale(a_ptr[i]); a_ptr[i] += p.sa_stride_k; }
+            for (int i = 0; i < 4; ++i) { copy4(to + (i * 32 + lane) * 4, a_ptr[i]); a_ptr[i] += p.sa_stride_k; }
+            if (lane < 2) copy4(to + (128 + lane) * 4, lane == 0 ? b_ptr[0] : b_ptr[1]);
 #pragma unroll
-            for (int c = 0; c < 2; ++c) { y[c] = ld_scale(b_ptr[c]); b_ptr[c] += p.sb_stride_k; }
+            for (int c = 0; c < 2; ++c) b_ptr[c] += p.sb_stride_k;
             --left;
             ++fetched;
         };
-#pragma unroll
-        for (int u = 0; u < FETCH; ++u) fetch(va[u], vb[u]);
-        bool alive = true;
-        for (uint32_t it = 0; alive && it < fetched;) {
-#pragma unroll
-            for (int u = 0; u < FETCH; ++u) {
-                if (alive && it < fetched) {
-                    // (the MMAs of block it - 2 are done, so its buffer had been released by every reader of block it - 4, whose slot
-                    // this is; and that barrier cannot complete again without the arrival below)
-                    if (it >= 2 && !mbar_wait_warp(tfull0 + 8 * (it & 1), ((it - 2) >> 1) & 1, abort_flag, (4 << 8) | 1)) { alive = false; continue; }
-                    float* to = scales + (it % PSCALE_SLOTS) * 256 + lane;
-#pragma unroll
-                    for (int i = 0; i < 4; ++i) { to[i * 32] = va[u][i] * vb[u][0]; to[128 + i * 32] = va[u][i] * vb[u][1]; }
-                    __syncwarp();
-                    if (lane == 0) mbar_arrive(tfull0 + 8 * (it & 1));
-                    fetch(va[u], vb[u]);
-                    ++it;
-                }
-            }
+#pragma unroll 1
+        for (int u = 0; u < PFETCH; ++u) {
+            fetch(u);
+            asm volatile("cp.async.commit_group;" ::: "memory");
         }
+        for (uint32_t it = 0; it < fetched; ++it) {
+            const uint32_t slot = it % PFETCH;
+            asm volatile("cp.async.wait_group %0;" ::"n"(PFETCH - 1) : "memory");
+            __syncwarp();
+            const float* from = raw + slot * PRAW;
+            const float b0 = from[128], b1 = from[129];
+            float x[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) x[i] = from[i * 32 + lane];
+            // (the MMAs of block it - 2 are done, so its buffer had been released by every reader of block it - 4, whose slot
+            // this is; and that barrier cannot complete again without the arrival below)
+            if (it >= 2 && !mbar_wait_warp(tfull0 + 8 * (it & 1), ((it - 2) >> 1) & 1, abort_flag, (4 << 8) | 1)) break;
+            float* to = scales + (it % PSCALE_SLOTS) * 256 + lane;
+#pragma unroll
+            for (int i = 0; i < 4; ++i) { to[i * 32] = x[i] * b0; to[128 + i * 32] = x[i] * b1; }
+            __syncwarp();
+            if (lane == 0) mbar_arrive(tfull0 + 8 * (it & 1));
+            fetch(slot);
+            asm volatile("cp.async.commit_group;" ::: "memory");
+        }
+        asm volatile("cp.async.wait_all;" ::: "memory");
     } else if (warp == PSTORE) {
         // ------------------------------ finished tiles to the TMA unit (both CTAs) ------------------------------
         // A lane sends a box.  A tile's 64 KiB leave the SM in a thousand cycles and an issue blocks until the unit

@@ -423,6 +423,28 @@ def test_gemms_under_a_cap_of_one_sm(K):
         assert torch.equal(a, b)
 
 
+@pytest.mark.parametrize("M,N,Kd", [(20000, 512, 1168), (20000, 512, 400), (5000, 1024, 2064), (600, 2560, 4112), (9000, 4352, 320), (4500, 2048, 128)])
+def test_kernels_agree_on_every_reduction(K, M, N, Kd):
+    """Reductions of one to 33 blocks, with less in the last one, over several tiles per pair of SMs: the bits of a cap of one SM, which
+    leaves the one-SM kernel only."""
+    xq, xs, wq, ws = _operands(M, N, Kd, seed=M + N + Kd)
+    a, sa, b, sb = _f8(xq), xs.cuda(), _f8(wq), ws.cuda()
+
+    def run(dtype):
+        return K._gemm(a, sa, b, 0, sb, 1, sb.stride(0), M, N, Kd, dtype, whole=True)
+    for dtype in (torch.bfloat16, torch.float32):
+        want = run(dtype)
+        before = K.set_gemm_sm_limit(1)
+        try:
+            got = run(dtype)
+        finally:
+            K.set_gemm_sm_limit(before)
+        assert torch.equal(got, want)
+    rows = torch.arange(0, M, max(1, M // 64))
+    assert rel_fro(want.cpu()[rows], O.fp8_matmul_f64(xq[rows], wq.t(), xs[rows], ws.t())) <= 2e-5
+    assert K.device_status() == 0
+
+
 @pytest.mark.parametrize("name", list(GROUPED))
 @pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
 def test_grouped_gemm_16bit(K, name, dtype):
