@@ -38,6 +38,7 @@ constexpr int WCOLS = BN / (EPI_WARPS / 4);     // accumulator columns per epilo
 constexpr int THREADS = (EPI_WARPS + 3) * 32;     // + TMA producer + two MMA issuers
 constexpr int TMEM_COLS = 512;
 constexpr int MAX_EXPERTS = 384;      // bounded by the shared memory left for the per-expert prefix sums
+constexpr int MAX_SEGMENTS = 1024;    // experts of a grouped weight gradient
 constexpr int GROUP_M = 16;        // rasterisation: m-tiles per L2 group (dense)
 
 // device status word: 0 = fine, otherwise (role << 8) | reason
@@ -690,12 +691,13 @@ static int launch_out(const CUtensorMap& ta, const CUtensorMap& tb, GemmParams& 
     }
 }
 
-template <bool B_MN, int OUT, bool GK = false, bool GR = false>
+template <bool B_MN, int OUT, bool GK = false, bool GR = false, bool OWN = false>
 static int launch_pair(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& tc, const GemmParams& p, int clusters,
                        cudaStream_t st) {
-    constexpr auto kern = pair::fp8_gemm_pair_kernel<B_MN, OUT, GK, GR>;
-    const size_t smem = pair::PSMEM_BYTES + (GR ? 4 * (size_t)(p.E + 2) : 0);
-    int rc = allow_smem_once<kern>(pair::PSMEM_BYTES + (GR ? 4 * (size_t)(MAX_EXPERTS + 2) : 0));
+    constexpr auto kern = pair::fp8_gemm_pair_kernel<B_MN, OUT, GK, GR, OWN>;
+    constexpr int MOST = GR ? MAX_EXPERTS : GK ? MAX_SEGMENTS : -2;              // (counts in shared memory, one per expert and two)
+    const size_t smem = pair::PSMEM_BYTES + (GR || GK ? 4 * (size_t)(p.E + 2) : 0);
+    int rc = allow_smem_once<kern>(pair::PSMEM_BYTES + 4 * (size_t)(MOST + 2));
     if (rc) return rc;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(2 * clusters, 1, 1);
@@ -1045,7 +1047,7 @@ int fp8_grouped_gemm_dgrad(const void* dY, const float* sdY, const void* W, cons
 // transposed, (d_in, max_tiles * 128); kb_start (E + 1 ints, device) gives every expert's K blocks.
 int fp8_gemm_grouped_k(const void* A, const float* sA, const void* B, const float* sB, const int* kb_start, int64_t E,
                        int64_t M, int64_t N, int64_t max_tiles, void* C, int out_dtype, cudaStream_t st) {
-    CINN_CHECK_ARG(E >= 1 && M > 0 && N > 0 && max_tiles >= 1, "grouped-K GEMM: bad shape");
+    CINN_CHECK_ARG(E >= 1 && E <= MAX_SEGMENTS && M > 0 && N > 0 && max_tiles >= 1, "grouped-K GEMM: bad shape");
     CINN_CHECK_ARG(M % pair::PM == 0 && N % pair::PN == 0, "grouped-K GEMM: M (%lld) and N (%lld) must be multiples of 256",
                    (long long)M, (long long)N);
     CINN_CHECK_ARG(A && sA && B && sB && kb_start && C && al16(A) && al16(B) && al16(C), "grouped-K GEMM: null or unaligned pointer");
@@ -1068,10 +1070,16 @@ int fp8_gemm_grouped_k(const void* A, const float* sA, const void* B, const floa
     const int64_t tiles = E * (M / pair::PM) * (N / pair::PN);
     const int sms = gemm_sms(), pairs = sms >= 2 ? sms / 2 : 1;              // (only the two-SM kernel does this: a cap of one SM counts as two)
     const int clusters = (int)(tiles < pairs ? tiles : pairs);
+    // Below two K blocks per expert on average, 4-byte gradients are bound by their stores and by how early a tile's scales are there.  In us with the
+    // quantisers, through the scale warp and OWN: 32 experts of 64 rows, 2048 x 2048 in fp32 142 -> 131, of 192 156 -> 141, of 256 158 and 163,
+    // of 512 207 and 225; 32 of 128 rows, 7168 x 4096 854 -> 777; in bf16, of 128 rows 93 and 101.
+    const bool own = max_tiles - E < 2 * E;
     switch (out_dtype) {
         case CINN_BF16: return launch_pair<false, CINN_BF16, true>(ta, tb, tc, p, clusters, st);
-        case CINN_F32: return launch_pair<false, CINN_F32, true>(ta, tb, tc, p, clusters, st);
-        case CINN_F32_BF16: return launch_pair<false, CINN_F32_BF16, true>(ta, tb, tc, p, clusters, st);
+        case CINN_F32: return own ? launch_pair<false, CINN_F32, true, false, true>(ta, tb, tc, p, clusters, st)
+                                  : launch_pair<false, CINN_F32, true>(ta, tb, tc, p, clusters, st);
+        case CINN_F32_BF16: return own ? launch_pair<false, CINN_F32_BF16, true, false, true>(ta, tb, tc, p, clusters, st)
+                                       : launch_pair<false, CINN_F32_BF16, true>(ta, tb, tc, p, clusters, st);
         default: set_error("grouped-K GEMM: the gradient is fp32 (optionally holding bf16-rounded values) or bf16"); return CINN_ERR_INVALID;
     }
 }

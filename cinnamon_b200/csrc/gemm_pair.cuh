@@ -128,13 +128,15 @@ __device__ __forceinline__ PairTile pair_tile(const GemmParams& p, int t) {
 // which expert e owns the K blocks [kb_start[e], kb_start[e + 1]) (p.starts holds that int array, p.E = E); tile t
 // belongs to expert t / (tiles per expert) and is stored at rows e * M + ... of the (E * M, N) output.  An expert
 // without rows gets zeros.  Without kb_start (null) the E "experts" are equal pieces of one problem's reduction, whose partial sums
-// split_sum_kernel adds.
+// split_sum_kernel adds.  The kernel keeps the array in shared memory: while the stores saturate memory, each role's two loads per
+// tile cost it thousands of cycles (32 experts of 512 rows, 2048 x 2048 in bf16: 182 -> 172 us).
+// OWN: the promotion warps load their scales themselves, for experts of few K blocks: see fp8_gemm_grouped_k.
 //
 // GR ("grouped rows"): E independent problems of the same N x K over the ragged row ranges [starts[e], ends[e]) of A and C
 // (device arrays), B stacked (E * b_rows_per_expert rows).  The tiles of all experts are one list, found through a prefix sum
 // of their tile counts in shared memory behind the barriers; a CTA whose 128 rows are not all its expert's stores them with
 // row predicates.  Worth it from a few tiles of rows per expert on: see fp8_grouped_gemm.
-template <bool B_MN, int OUT, bool GK = false, bool GR = false>
+template <bool B_MN, int OUT, bool GK = false, bool GR = false, bool OWN = false>
 __global__ void __launch_bounds__(PTHREADS, 1)
 fp8_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                      const __grid_constant__ CUtensorMap tmC, const GemmParams p) {
@@ -151,7 +153,7 @@ fp8_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
     // round are staged, they have been read
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * PSTAGES + 8);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
-    int* cum = reinterpret_cast<int*>(reinterpret_cast<uint8_t*>(bars) + 256);  // GR: E + 1 prefix counts of row tiles
+    int* cum = reinterpret_cast<int*>(reinterpret_cast<uint8_t*>(bars) + 256);  // E + 1 prefix counts, GR: of row tiles, GK: of K blocks
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t rank = cluster_ctarank();           // 0 = leader
@@ -162,7 +164,7 @@ fp8_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
     if (threadIdx.x == 0) *abort_flag = 0;
     if (warp == PTMA && lane == 0) {
         for (int s = 0; s < PSTAGES; ++s) { mbar_init(full0 + 8 * s, 1); mbar_init(empty0 + 8 * s, 1); }
-        for (int b = 0; b < 2; ++b) { mbar_init(tfull0 + 8 * b, 2); mbar_init(tempty0 + 8 * b, 2 * PEPI); }
+        for (int b = 0; b < 2; ++b) { mbar_init(tfull0 + 8 * b, OWN ? 1 : 2); mbar_init(tempty0 + 8 * b, 2 * PEPI); }
         mbar_init(staged, PEPI);
         mbar_init(taken, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -176,21 +178,26 @@ fp8_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
     if constexpr (GR) {
         if (warp == 0) tile_prefix_sum(p, cum, PM, lane);
     }
+    if constexpr (GK) {
+        const int* start = reinterpret_cast<const int*>(p.starts);
+        for (int e = threadIdx.x; e <= p.E; e += PTHREADS)
+            cum[e] = start ? start[e] : (int)((int64_t)((p.K + BK - 1) / BK) * e / p.E);
+    }
     tc_fence_before();
     __syncthreads();
     cluster_sync();                                    // both CTAs' barriers exist before anyone signals them
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
 
-    // A 4-byte tile leaves in two rounds: its promotion warps hand over their own boxes, so that each waits for its own to be read
-    // and not for everybody's (32 experts of 127 rows each, 768 x 3584 gradients, forward and backward 197.6 against 191.3 us).
-    constexpr bool STORE_WARP = sizeof(typename OutT<OUT>::type) == 2;
+    // A 4-byte tile leaves in two rounds, and the experts' gradients of either size are bound by their stores: there the promotion warps
+    // hand over their own boxes, so that each waits for its own to be read and not for everybody's (weight gradients of 32 experts
+    // of 64 rows, 2048 x 2048 in bf16, with their quantisers 98 -> 91 us).
+    constexpr bool STORE_WARP = sizeof(typename OutT<OUT>::type) == 2 && !GK;
     const int KB_dense = (p.K + BK - 1) / BK;
     const int per_expert = pair_total(p);
     const int n_tiles = (p.N + PN - 1) / PN;
     const int n_total = GR ? cum[p.E] * n_tiles : (GK ? per_expert * p.E : per_expert);
     const int cluster_id = blockIdx.x >> 1, n_clusters = gridDim.x >> 1;
-    const int* kb_start = reinterpret_cast<const int*>(p.starts);
     // tile t -> its coordinates inside one problem (GR: among all rows), the expert it belongs to, its K blocks, and one past
     // the last row it may write
     auto locate = [&](int t, PairTile& ti, int& e, int& kb0, int& KB, int& m_end) {
@@ -210,13 +217,8 @@ fp8_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
         } else if constexpr (GK) {
             e = t / per_expert;
             ti = pair_tile(p, t - e * per_expert);
-            if (kb_start) {
-                kb0 = kb_start[e];
-                KB = kb_start[e + 1] - kb0;
-            } else {
-                kb0 = (int)((int64_t)KB_dense * e / p.E);
-                KB = (int)((int64_t)KB_dense * (e + 1) / p.E) - kb0;
-            }
+            kb0 = cum[e];
+            KB = cum[e + 1] - kb0;
         } else {
             e = 0; kb0 = 0; KB = KB_dense;
             ti = pair_tile(p, t);
@@ -251,7 +253,7 @@ fp8_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
                 while (clock64() - t0 < 2000000LL) { }
             }
         }
-    } else if (warp == PSCALE) {
+    } else if (!OWN && warp == PSCALE) {
         // ------------------ scales (both CTAs): K block `it`'s products sA sB of this CTA's rows ------------------
         // They come PFETCH blocks ahead, copied to shared memory.  Through registers, a block's values waited for the loads issued last, four
         // blocks on: a miss for every row each eighth block (8837 x 17024 -> 320, one wave of tiles: 101 us so, 69 like this).
@@ -317,11 +319,11 @@ fp8_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
             asm volatile("cp.async.commit_group;" ::: "memory");
         }
         asm volatile("cp.async.wait_all;" ::: "memory");
-    } else if (warp == PSTORE) {
+    } else if (warp == PSTORE || warp == PSCALE) {
         // ------------------------------ finished tiles to the TMA unit (both CTAs) ------------------------------
         // A lane sends a box.  A tile's 64 KiB leave the SM in a thousand cycles and an issue blocks until the unit
         // takes it: promotion warps that issued their own stores stood still for most of that.
-        if (STORE_WARP && p.tma_out) {
+        if (STORE_WARP && warp == PSTORE && p.tma_out) {
             constexpr int EPR = 128 / (int)sizeof(typename OutT<OUT>::type);
             const int w = lane / PBOXES, q = w & 3, h = w >> 2;
             uint32_t round = 0;
@@ -388,11 +390,27 @@ fp8_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
             float acc[PCOLS];
 #pragma unroll
             for (int i = 0; i < PCOLS; ++i) acc[i] = 0.0f;
+            // OWN: the warp's own scales, three blocks ahead
+            const float *sa_ptr = nullptr, *sb_ptr = nullptr;
+            float sa[3], sb[3];
+            if constexpr (OWN) {
+                sa_ptr = p.sA + (int64_t)(ti.m0 + 128 * (int)rank + q * 32 + lane) * p.sa_stride_m + (int64_t)kb0 * p.sa_stride_k;
+                sb_ptr = p.sB + (int64_t)(ti.n0 / 128 + h) * p.sb_stride_n + (int64_t)kb0 * p.sb_stride_k;
+#pragma unroll
+                for (int i = 0; i < 3; ++i)
+                    if (i < KB) { sa[i] = ld_scale(sa_ptr + i * p.sa_stride_k); sb[i] = ld_scale(sb_ptr + i * p.sb_stride_k); }
+            }
             for (int kb = 0; kb < KB; ++kb, ++it) {
                 const uint32_t b = it & 1, bph = (it >> 1) & 1;
+                float s;
+                if constexpr (OWN) {
+                    s = sa[0] * sb[0];
+                    sa[0] = sa[1]; sb[0] = sb[1]; sa[1] = sa[2]; sb[1] = sb[2];
+                    if (kb + 3 < KB) { sa[2] = ld_scale(sa_ptr + (kb + 3) * p.sa_stride_k); sb[2] = ld_scale(sb_ptr + (kb + 3) * p.sb_stride_k); }
+                }
                 if (!mbar_wait_warp(tfull0 + 8 * b, bph, abort_flag, (3 << 8) | 1)) { alive = false; break; }
                 tc_fence_after();
-                const float s = my_scales[(it % PSCALE_SLOTS) * 256];
+                if constexpr (!OWN) s = my_scales[(it % PSCALE_SLOTS) * 256];
                 const uint32_t taddr = tmem_base + ((uint32_t)(q * 32) << 16) + b * PN + h * PCOLS;
                 // packed fp32x2 FMAs: half the issue slots of scalar ones, the same IEEE result in every lane
                 uint64_t s2;

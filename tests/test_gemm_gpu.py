@@ -671,6 +671,35 @@ FUSED_WGRAD = {
 }
 
 
+@pytest.mark.parametrize("counts", [[255, 256, 256, 128], [256, 256, 256, 129], [0, 1, 128, 129, 127, 0, 200], [130, 600, 0, 20], [1300, 700]])
+def test_grouped_weight_gradients_of_short_and_long_experts(K, counts):
+    """None, one, two and more K blocks per expert, on both sides of two on average, several tiles per pair of SMs: the bits of the per-expert
+    loop in every type of the gradient."""
+    E, d_in, d_out = len(counts), 1792, 1536
+    x, w, starts, ends = _grouped_case(E, d_in, d_out, counts, seed=sum(counts), gap=5)
+    dy = torch.randn(x.shape[0], d_out, generator=torch.Generator().manual_seed(E)).bfloat16()
+    xq, xs = K.quantize_fp8_rowwise(x.cuda())
+    args = (dy.cuda(), xq, xs, starts.cuda(), ends.cuda(), E, d_in, d_out)
+    loop = K.fp8_grouped_wgrad(*args, w_dtype=torch.float32, fused=False)
+    assert torch.equal(K.fp8_grouped_wgrad(*args, w_dtype=torch.float32, fused=True), loop)
+    assert torch.equal(K.fp8_grouped_wgrad(*args, w_dtype=torch.bfloat16, fused=True), K.fp8_grouped_wgrad(*args, w_dtype=torch.bfloat16, fused=False))
+    assert all(bool((loop[e] == 0).all()) == (c == 0) for e, c in enumerate(counts))
+    assert K.device_status() == 0
+
+
+def test_grouped_weight_gradient_of_a_thousand_experts(K):
+    """The largest number of experts of one call, most of them empty."""
+    E, d = 1024, 256
+    counts = [(e % 7 == 0) * (e % 5) for e in range(E)]
+    x, w, starts, ends = _grouped_case(E, d, d, counts, seed=3, gap=2)
+    dy = torch.randn(x.shape[0], d, generator=torch.Generator().manual_seed(4)).bfloat16()
+    xq, xs = K.quantize_fp8_rowwise(x.cuda())
+    args = (dy.cuda(), xq, xs, starts.cuda(), ends.cuda(), E, d, d)
+    for dtype in (torch.float32, torch.bfloat16):
+        assert torch.equal(K.fp8_grouped_wgrad(*args, w_dtype=dtype, fused=True), K.fp8_grouped_wgrad(*args, w_dtype=dtype, fused=False))
+    assert K.device_status() == 0
+
+
 @pytest.mark.parametrize("name", list(FUSED_WGRAD))
 def test_grouped_weight_gradient_in_one_gemm(K, name):
     """cinn_fp8_grouped_wgrad_fused (segments padded to tiles on the device, two quantiser launches, one grouped-K
