@@ -19,6 +19,7 @@
 #include <cuda.h>
 #include <mutex>
 #include <atomic>
+#include <cmath>
 #include <cstdlib>
 
 namespace cinn {
@@ -810,6 +811,13 @@ static int launch_split_sum(const float* part, void* out, int64_t n, int splits,
     return CINN_OK;
 }
 
+// us that a wave of tiles of a reduction over K takes on single SMs and on pairs, fitted to 130 calls of both kernels one after
+// another (M 256 ... 16384, N 256 ... 8192, K 128 ... 16384; 4 % off on average)
+static double tile_cost(int64_t K, bool pair) {
+    const double KB = (double)((K + BK - 1) / BK);
+    return pair ? KB * 0.44 + 1.75 : KB * 0.50 + 1.6;
+}
+
 struct DensePlan { bool pair; int splits; bool rows; };
 
 template <int ROWS>
@@ -953,9 +961,14 @@ int fp8_gemm(const void* A, int64_t lda, const float* sA, int64_t ld_sa, const v
 // Grouped problems run on pairs of SMs and 256-row tiles from 256 rows per expert on average (how the rows are really spread only
 // the device knows): below that the half-empty tiles cost more than the pair saves.  Both directions; for the input gradient, whose
 // weight is read MN-major, 7168 x 4096 of 32 experts, 32768 rows, 1045 -> 920 us, and 512 x 512
-// of 16 experts, 65536 rows, 67 -> 59.
-static bool grouped_on_pairs(int64_t E, int64_t T, int64_t N, int sms) {
-    return pair_mode() != 0 && sms >= 2 && T >= pair::PM * E && (T + pair::PM - 1) / pair::PM * ((N + pair::PN - 1) / pair::PN) >= sms / 2;
+// of 16 experts, 65536 rows, 67 -> 59.  Not where the pairs' last wave is nearly empty and the single SMs' is not, with half a tile
+// too many per expert: 8 experts, 3045 rows, 3328 -> 2560 53 us on pairs (three waves) and 43 (two), 32 of 9123, 1024 -> 768 25.6 and 21.5.
+static bool grouped_on_pairs(int64_t E, int64_t T, int64_t N, int64_t K, int sms) {
+    if (pair_mode() == 0 || sms < 2 || T < pair::PM * E) return false;
+    const int64_t n_tiles = (N + pair::PN - 1) / pair::PN;
+    if ((T + pair::PM - 1) / pair::PM * n_tiles < sms / 2) return false;
+    auto waves = [&](int64_t rows, int slots) { return std::ceil((double)(2 * T + rows * E) / (double)(2 * rows) * (double)n_tiles / slots); };
+    return waves(pair::PM, sms / 2) * tile_cost(K, true) <= 1.25 * waves(BM, sms) * tile_cost(K, false);
 }
 
 template <bool B_MN>
@@ -989,7 +1002,7 @@ int fp8_grouped_gemm(const void* A, const float* sA, const void* W, const float*
     int rc = make_map(&ta, A, (uint64_t)d_in, (uint64_t)T, (uint64_t)d_in, BK, BM);
     if (rc) return rc;
     const int sms = gemm_sms();
-    const bool use_pair = row_dst == nullptr && grouped_on_pairs(E, T, d_out, sms);
+    const bool use_pair = row_dst == nullptr && grouped_on_pairs(E, T, d_out, d_in, sms);
     rc = make_map(&tb, W, (uint64_t)d_in, (uint64_t)(E * d_out), (uint64_t)d_in, BK, use_pair ? 128 : BN);
     if (rc) return rc;
     const int64_t nkb = (d_in + 127) / 128, nnb = (d_out + 127) / 128;
@@ -1038,7 +1051,7 @@ int fp8_grouped_gemm_dgrad(const void* dY, const float* sdY, const void* W, cons
     p.C = dX; p.ldc = d_in; p.M = (int)T; p.N = (int)d_in; p.K = (int)d_out;
     p.starts = starts; p.ends = ends; p.E = (int)E; p.b_rows_per_expert = (int)d_out;
     const int sms = gemm_sms();
-    if (grouped_on_pairs(E, T, d_in, sms)) return launch_grouped_pair<true>(ta, tb, p, out_dtype, sms / 2, st);
+    if (grouped_on_pairs(E, T, d_in, d_out, sms)) return launch_grouped_pair<true>(ta, tb, p, out_dtype, sms / 2, st);
     return launch_out<true, true>(ta, tb, p, out_dtype, sms, st);
 }
 

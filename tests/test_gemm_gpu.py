@@ -445,6 +445,31 @@ def test_kernels_agree_on_every_reduction(K, M, N, Kd):
     assert K.device_status() == 0
 
 
+@pytest.mark.parametrize("case", [(8, 2560, 640, 380), (32, 768, 512, 285), (4, 1536, 384, 1200), (16, 512, 1024, 600)])
+def test_grouped_kernels_agree(K, case):
+    """Both directions at shapes that run on pairs of SMs and at shapes that do not for their waves: the bits of a cap of one SM."""
+    E, d_in, d_out, rows = case
+    counts = [rows + 37 * ((e * 5) % 9 - 4) for e in range(E)]
+    x, w, starts, ends = _grouped_case(E, d_in, d_out, counts, seed=E + rows, gap=3)
+    xq, xs = K.quantize_fp8_rowwise(x.cuda())
+    wq, ws = K.quantize_expert_weights(w.cuda())
+    gq, gs = K.quantize_fp8_rowwise(torch.randn(x.shape[0], d_out, generator=torch.Generator().manual_seed(E)).bfloat16().cuda())
+    range_ = (starts.cuda(), ends.cuda())
+
+    def run():
+        return (K.fp8_grouped_gemm_dgrad(gq, gs, wq, ws, *range_, out_dtype=torch.bfloat16),
+                K.moe_grouped_gemm(x.cuda(), w.cuda(), *range_, dtype=torch.bfloat16))
+    want = run()
+    before = K.set_gemm_sm_limit(1)
+    try:
+        got = run()
+    finally:
+        K.set_gemm_sm_limit(before)
+    for a, b in zip(got, want):
+        assert torch.equal(a[:int(ends[-1])], b[:int(ends[-1])])
+    assert K.device_status() == 0
+
+
 @pytest.mark.parametrize("name", list(GROUPED))
 @pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
 def test_grouped_gemm_16bit(K, name, dtype):
