@@ -855,13 +855,13 @@ static bool rows_pay(int64_t M, int64_t N, int64_t K, int b_layout, int64_t work
     return KB <= 40 && (M <= 128 || blocks * KB <= 16 * sms);
 }
 
-// A K block of a tile costs about 0.45 us in either kernel (a pair of SMs does twice the rows in it), a tile about 3 us
+// Whole, by waves of tiles (tile_cost).  2155 x 320 -> 4352 takes 10.6 us on single SMs (two waves) and 12.3 on pairs (three), 4498 x 128 -> 8128
+// 19.1 and 23.2 (one K block), 10646 x 512 -> 1472 18.8 and 16.0.
+// Cut along K, with cold operands and the launch: a K block of a tile costs about 0.45 us in either kernel, a tile about 3 us
 // around its K blocks on one SM and 1.6 on a pair.  Splitting adds a pass over the partial sums: about 3 us of launch and the bytes at the
-// rate L2 returns them.  The plan with the smallest sum of these wins.  Measured with cold operands, launch included: one tile alone 7.2 /
-// 12.3 / 34.3 us for 4 / 16 / 64 K blocks, a full wave of pairs 9.2 / 15.4 / 43.0, two waves 12.3 / 24.1 / 71.2; whole -> as
-// planned (M x N x K): 64 x 4096 x 7168 29.7 -> 16.3, 300 x 576 x 7168 29.7 -> 15.4 (B MN-major), 512 x 1024 x 32768 117 -> 31 on
-// single SMs and 29 on pairs, 16 x 18432 x 7168 38.9 -> 34.3, 128 x 512 x 2560 14.3 -> 12.8.  The demands (12 us, a gain of a tenth) leave the
-// problems whole where the second launch eats what is won: 1024 x 4096 x 4096 (22 us), 64 x 7168 x 2048 (12.8).
+// rate L2 returns them.  The plan with the smallest sum of these wins.  Whole -> as planned (M x N x K): 300 x 576 x 7168 29.7 -> 15.4 (B
+// MN-major), 512 x 1024 x 32768 117 -> 31 on single SMs and 29 on pairs, 16 x 18432 x 7168 38.9 -> 34.3.  The demands (12 us, a gain of a
+// tenth) leave the problems whole where the second launch eats what is won: 1024 x 4096 x 4096 (22 us).
 static DensePlan dense_plan(int64_t M, int64_t N, int64_t K, int b_layout, int64_t workspace_bytes, int sms) {
     const int64_t KB = (K + BK - 1) / BK;
     auto waves = [](int64_t tiles, int64_t slots) { return (double)((tiles + slots - 1) / slots); };
@@ -876,8 +876,10 @@ static DensePlan dense_plan(int64_t M, int64_t N, int64_t K, int b_layout, int64
     // (128 rows would leave a CTA idle; a pair takes two SMs)
     const bool pairs = sms >= 2 && pm == 1 && b_layout == 0 && M > BM;
     if (pairs || (sms >= 2 && pm == 2 && pair_tiles >= sm_count() / 2)) {
-        const double us = waves(pair_tiles, sms / 2) * (KB * block_us + pair_tile_us);
-        if (us <= best_us * 1.02 || pm == 2) { best = {true, 1, false}; best_us = us; }
+        if (pm == 2 || waves(pair_tiles, sms / 2) * tile_cost(K, true) <= waves(tiles, sms) * tile_cost(K, false)) {
+            best = {true, 1, false};
+            best_us = waves(pair_tiles, sms / 2) * (KB * block_us + pair_tile_us);
+        }
     }
     if (best_us < 12.0 || tiles >= sms) return best;
     for (int s = 2; s <= 32 && s * 2 <= KB; ++s) {
