@@ -104,6 +104,24 @@ def test_few_rows_have_the_bits_of_many(K, N, Kd):
     assert K.device_status() == 0
 
 
+@pytest.mark.parametrize("N,Kd,rows", [(40, 16, 20000), (96, 272, 8192), (4096, 7168, 4096), (7168, 5136, 2048)])
+def test_few_rows_without_a_cut(K, N, Kd, rows):
+    """Calls that are never cut along K (the experts' and the shared expert's): the kernel for few rows, also over a long reduction, gives
+    every row the bits of a call of many rows, which is too large for it, and both are the float64 oracle's."""
+    xq, xs, wq, ws = _operands(rows, N, Kd, seed=N + Kd)
+    a, sa, b, sb = _f8(xq), xs.cuda(), _f8(wq), ws.cuda()
+
+    def run(m, dtype):
+        return K._gemm(a[:m].contiguous(), sa[:m].contiguous(), b, 0, sb, 1, sb.stride(0), m, N, Kd, dtype, whole=True)
+    for dtype in (torch.bfloat16, torch.float32, torch.float16):
+        many = run(rows, dtype)
+        for m in (1, 63, 64, 65, 128):
+            assert torch.equal(run(m, dtype), many[:m]), (m, dtype)
+        if dtype == torch.float32:
+            assert rel_fro(many[:128], O.fp8_matmul_f64(xq[:128], wq.t(), xs[:128], ws.t())) <= 2e-5
+    assert K.device_status() == 0
+
+
 PAIR_SCRIPT = r"""
 import sys, torch
 sys.path.insert(0, sys.argv[1])
