@@ -19,8 +19,8 @@ constexpr int RTHREADS = 6 * 32;
 constexpr int RTMEM_COLS = 2 * BATCH * RN;
 constexpr int RB_BYTES = RN * BK;
 
-// ROWS: rows of A that are staged, 64 or 128.  The MMAs take 128 rows: with 64 the rest are bytes of other stages, whose products
-// nobody reads.
+// ROWS: rows of A that a stage has room for, 64 or 128; p.box_rows of them are copied.  The MMAs take 128 rows: the rest are whatever
+// lies there and bytes of other stages, whose products nobody reads.
 template <int ROWS> struct Shape {
     static constexpr int STAGES = ROWS == 64 ? 8 : 5;
     static constexpr int A_BYTES = ROWS * BK;
@@ -67,7 +67,7 @@ fp8_gemm_rows_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
             uint32_t s = 0, ph = 0;
             for (int kb = 0; kb < KB; ++kb) {
                 if (!mbar_wait(empty0 + 8 * s, ph ^ 1, abort_flag, (6 << 8) | 1)) { alive = false; break; }
-                mbar_expect_tx(full0 + 8 * s, S::A_BYTES + RB_BYTES);
+                mbar_expect_tx(full0 + 8 * s, p.box_rows * BK + RB_BYTES);
                 tma_load_2d(&tmB, full0 + 8 * s, smem_b + s * RB_BYTES, kb * BK, n0);
                 tma_load_2d(&tmA, full0 + 8 * s, smem_a + s * S::A_BYTES, kb * BK, m0);
                 if (++s == S::STAGES) { s = 0; ph ^= 1; }

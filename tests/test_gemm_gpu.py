@@ -20,6 +20,7 @@ def K():
     yield kernels
     assert kernels.device_status() == 0, "a kernel gave up on a bounded wait"
     kernels.set_div_mode("full")
+    torch.cuda.empty_cache()            # (what is allocated next does not keep this module's large segments)
 
 
 def _operands(M, N, Kd, seed):
@@ -115,7 +116,7 @@ def test_few_rows_without_a_cut(K, N, Kd, rows):
         return K._gemm(a[:m].contiguous(), sa[:m].contiguous(), b, 0, sb, 1, sb.stride(0), m, N, Kd, dtype, whole=True)
     for dtype in (torch.bfloat16, torch.float32, torch.float16):
         many = run(rows, dtype)
-        for m in (1, 63, 64, 65, 128):
+        for m in (1, 5, 16, 63, 64, 65, 100, 128):
             assert torch.equal(run(m, dtype), many[:m]), (m, dtype)
         if dtype == torch.float32:
             assert rel_fro(many[:128], O.fp8_matmul_f64(xq[:128], wq.t(), xs[:128], ws.t())) <= 2e-5

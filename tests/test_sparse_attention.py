@@ -225,7 +225,15 @@ def test_tiles_with_wide_scores(dtype, shape):
     assert K.device_status() == 0
 
 
+@pytest.fixture
+def released():
+    """Gives the test's memory back: a later test counts what the allocator holds."""
+    yield
+    torch.cuda.empty_cache()
+
+
 @pytest.mark.gpu
+@pytest.mark.usefixtures("released")
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
 @pytest.mark.parametrize("H", [3, 80])                    # a block per SM, two of them
 @pytest.mark.parametrize("Ks", [4, 64, 24])
@@ -269,6 +277,7 @@ def test_tiles_with_probabilities_at_odd_addresses(dtype, H, Ks):
 
 
 @pytest.mark.gpu
+@pytest.mark.usefixtures("released")
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
 @pytest.mark.parametrize("H", [2, 160])                   # a block per SM, two of them
 @pytest.mark.parametrize("keys,Ks", [(1, 200), (23, 33), (140, 120), (300, 512)])
@@ -296,6 +305,7 @@ def test_tiles_weigh_repeated_picks(dtype, H, keys, Ks):
 
 
 @pytest.mark.gpu
+@pytest.mark.usefixtures("released")
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 @pytest.mark.parametrize("shape", [(1, 160, 300, 40, 192, 64), (2, 76, 257, 33, 128, 64), (1, 150, 385, 64, 192, 128), (1, 230, 250, 24, 128, 100),
                                    (4, 37, 400, 16, 64, 128), (1, 45, 2048, 128, 192, 64), (1, 60, 130, 100, 192, 64), (1, 80, 256, 512, 72, 72),
@@ -324,6 +334,7 @@ def test_tiles_of_many_heads(dtype, shape):
 
 
 @pytest.mark.gpu
+@pytest.mark.usefixtures("released")
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
 @pytest.mark.parametrize("H", [2, 160])
 def test_tiles_of_many_heads_fall_back(dtype, H):
