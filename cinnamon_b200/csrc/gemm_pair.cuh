@@ -14,7 +14,7 @@
 //
 // The promotion warps are the bound (a K block took them 840 cycles where its MMAs take 512, a tile 3500 around its K blocks), so
 // they do nothing else: a tile's coordinates cost them 850 cycles of divisions, its stores up to 1000 of waiting for the TMA unit, and
-// the scales registers and a round trip per tile.  The scales' products now arrive through shared memory, on the barrier that reports
+// the scales registers and a round trip per tile.  The scales now arrive through shared memory, on the barrier that reports
 // the MMAs.  16384 x 7168 -> 18432 1915 -> 1708 us, 16384 x 576 -> 7168 102 -> 81, 32768 x 512 -> 1024 32.7 -> 28.3, 32768 rows of 7168 -> 4096 by
 // 32 experts and the way back with it 4.38 -> 4.29 ms, all cool.  (Sixteen warps of 64 columns, to hide more latency: 1957, 89 and 30.)
 #pragma once
@@ -30,19 +30,19 @@ constexpr int PEPI = 8;                 // promotion warps: four TMEM lane quart
 constexpr int PCOLS = PN / (PEPI / 4);
 constexpr int PTMA = PEPI, PMMA = PEPI + 1, PSTORE = PEPI + 2, PSCALE = PEPI + 3;
 constexpr int PTHREADS = (PEPI + 4) * 32;
-constexpr int PSCALE_SLOTS = 4;         // K blocks whose scale products are in shared memory: [slot][128 columns][row]
-constexpr int PSCALE_BYTES = PSCALE_SLOTS * 2 * 128 * 4;
+constexpr int PFETCH = 8;               // K blocks whose scales are on their way
+constexpr int PSCALE_SLOTS = 16;        // K blocks whose scales have a place: one per row, two columns'
+constexpr int PSCALES = 128 + 4;
+constexpr int PSCALE_BYTES = PSCALE_SLOTS * PSCALES * 4;
 constexpr int PTILE_SLOTS = 16;         // coordinates of the next tiles: {m0, n0, one past the last row, expert}
 // dynamic shared memory: operand stages | two 4 KiB output boxes per promotion warp = the CTA's whole 128 x 256 tile of a
-// 2-byte type (TMA-store boxes; also the 2 KiB-per-warp staging of the non-TMA path) | scale products | scales on their way | tiles | 256 B of barriers and
+// 2-byte type (TMA-store boxes; also the 2 KiB-per-warp staging of the non-TMA path) | scales | tiles | 256 B of barriers and
 // flags, plus 1 KiB of slack to align the stages to 1024 bytes
 constexpr int PSTAGE_OFF = PSTAGES * (PA_BYTES + PB_BYTES);
 constexpr int PBOX_BYTES = STORE_ROWS * 128;  // one TMA-store box
 constexpr int PBOXES = 16 / PEPI;       // boxes per promotion warp: a round of them all is 64 KiB, a CTA's tile of a 2-byte type
 constexpr int PC_BYTES = PEPI * PBOXES * PBOX_BYTES;
-constexpr int PFETCH = 8;               // K blocks whose scales are on their way
-constexpr int PRAW = 128 + 4;           // floats of one: a row's each, two columns'
-constexpr size_t PSMEM_BYTES = (size_t)PSTAGE_OFF + PC_BYTES + PSCALE_BYTES + PFETCH * PRAW * 4 + PTILE_SLOTS * 16 + 256 + 1024;
+constexpr size_t PSMEM_BYTES = (size_t)PSTAGE_OFF + PC_BYTES + PSCALE_BYTES + PTILE_SLOTS * 16 + 256 + 1024;
 
 __device__ __forceinline__ uint32_t cluster_ctarank() {
     uint32_t r;
@@ -146,8 +146,7 @@ fp8_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
     uint8_t* smem_b = smem + PSTAGES * PA_BYTES;
     uint8_t* c_stage = smem + PSTAGE_OFF;
     float* scales = reinterpret_cast<float*>(c_stage + PC_BYTES);
-    float* raw = reinterpret_cast<float*>(c_stage + PC_BYTES + PSCALE_BYTES);
-    int4* tiles = reinterpret_cast<int4*>(raw + PFETCH * PRAW);
+    int4* tiles = reinterpret_cast<int4*>(c_stage + PC_BYTES + PSCALE_BYTES);
     uint64_t* bars = reinterpret_cast<uint64_t*>(tiles + PTILE_SLOTS);
     // [0, S) full (used in the leader), [S, 2S) empty, [2S, 2S+2) tmem full, [2S+2, 2S+4) tmem empty (leader), then: all boxes of a
     // round are staged, they have been read
@@ -192,7 +191,7 @@ fp8_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
     // A 4-byte tile leaves in two rounds, and the experts' gradients of either size are bound by their stores: there the promotion warps
     // hand over their own boxes, so that each waits for its own to be read and not for everybody's (weight gradients of 32 experts
     // of 64 rows, 2048 x 2048 in bf16, with their quantisers 98 -> 91 us).
-    constexpr bool STORE_WARP = sizeof(typename OutT<OUT>::type) == 2 && !GK;
+    constexpr bool TWO_BYTE = sizeof(typename OutT<OUT>::type) == 2, STORE_WARP = TWO_BYTE && !GK;
     const int KB_dense = (p.K + BK - 1) / BK;
     const int per_expert = pair_total(p);
     const int n_tiles = (p.N + PN - 1) / PN;
@@ -254,16 +253,17 @@ fp8_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
             }
         }
     } else if (!OWN && warp == PSCALE) {
-        // ------------------ scales (both CTAs): K block `it`'s products sA sB of this CTA's rows ------------------
-        // They come PFETCH blocks ahead, copied to shared memory.  Through registers, a block's values waited for the loads issued last, four
-        // blocks on: a miss for every row each eighth block (8837 x 17024 -> 320, one wave of tiles: 101 us so, 69 like this).
+        // ------------------ scales (both CTAs): this CTA's rows' and both column blocks', K block by K block ------------------
+        // Copied to where they are read, PFETCH blocks ahead.  Through registers, a block's values waited for the loads issued last, four
+        // blocks on: a miss for every row each eighth block (8837 x 17024 -> 320, one wave of tiles: 125 us so, 96 like this).  Multiplied here
+        // and not by their readers: 1 to 2 % slower on long reductions (the warp takes issue slots of two promotion warps).
         const float* a_ptr[4];
         const float* b_ptr[2];
         int t = cluster_id - n_clusters, left = 0;     // K blocks of the tile that are still to be fetched
         uint32_t entered = 0;
         uint32_t fetched = 0;
         auto copy4 = [](uint32_t dst, const float* src) { asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst), "l"(src) : "memory"); };
-        auto fetch = [&](uint32_t slot) {
+        auto fetch = [&](uint32_t block) {
             while (left == 0) {
                 t += n_clusters;
                 if (t >= n_total) { t = n_total; return; }           // (and stays there)
@@ -284,7 +284,7 @@ fp8_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
                                + (GR ? (int64_t)e * p.sb_stride_e : 0);
                 }
             }
-            const uint32_t to = smem_u32(raw + slot * PRAW);
+            const uint32_t to = smem_u32(scales + block % PSCALE_SLOTS * PSCALES);
 #pragma unroll
             for (int i = 0; i < 4; ++i) { copy4(to + (i * 32 + lane) * 4, a_ptr[i]); a_ptr[i] += p.sa_stride_k; }
             if (lane < 2) copy4(to + (128 + lane) * 4, lane == 0 ? b_ptr[0] : b_ptr[1]);
@@ -299,23 +299,13 @@ fp8_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
             asm volatile("cp.async.commit_group;" ::: "memory");
         }
         for (uint32_t it = 0; it < fetched; ++it) {
-            const uint32_t slot = it % PFETCH;
             asm volatile("cp.async.wait_group %0;" ::"n"(PFETCH - 1) : "memory");
             __syncwarp();
-            const float* from = raw + slot * PRAW;
-            const float b0 = from[128], b1 = from[129];
-            float x[4];
-#pragma unroll
-            for (int i = 0; i < 4; ++i) x[i] = from[i * 32 + lane];
-            // (the MMAs of block it - 2 are done, so its buffer had been released by every reader of block it - 4, whose slot
-            // this is; and that barrier cannot complete again without the arrival below)
+            // (that barrier cannot complete again without the arrival below; and once the MMAs of block it - 2 are done, every reader of
+            // block it - 4 has released its buffer, so that the slot of block it - 8 may be filled again)
             if (it >= 2 && !mbar_wait_warp(tfull0 + 8 * (it & 1), ((it - 2) >> 1) & 1, abort_flag, (4 << 8) | 1)) break;
-            float* to = scales + (it % PSCALE_SLOTS) * 256 + lane;
-#pragma unroll
-            for (int i = 0; i < 4; ++i) { to[i * 32] = x[i] * b0; to[128 + i * 32] = x[i] * b1; }
-            __syncwarp();
             if (lane == 0) mbar_arrive(tfull0 + 8 * (it & 1));
-            fetch(slot);
+            fetch(it + PFETCH);
             asm volatile("cp.async.commit_group;" ::: "memory");
         }
         asm volatile("cp.async.wait_all;" ::: "memory");
@@ -381,7 +371,8 @@ fp8_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
         const uint32_t tempty_leader = mapa(tempty0, 0);
         uint32_t it = 0;
         bool alive = true;
-        const float* my_scales = scales + (h * PCOLS / 128) * 128 + q * 32 + lane;
+        const float* my_scales = scales + q * 32 + lane;
+        const float* column_scale = scales + 128 + h * PCOLS / 128;
         const bool vec_ok = (OUT == CINN_F32 || OUT == CINN_F32_BF16) ? (p.ldc % 4 == 0) : (p.ldc % 8 == 0);
         uint32_t seen = 0, round = 0;
         for (int t = cluster_id; t < n_total && alive; t += n_clusters) {
@@ -410,7 +401,7 @@ fp8_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
                 }
                 if (!mbar_wait_warp(tfull0 + 8 * b, bph, abort_flag, (3 << 8) | 1)) { alive = false; break; }
                 tc_fence_after();
-                if constexpr (!OWN) s = my_scales[(it % PSCALE_SLOTS) * 256];
+                if constexpr (!OWN) s = my_scales[(it % PSCALE_SLOTS) * PSCALES] * column_scale[(it % PSCALE_SLOTS) * PSCALES];
                 const uint32_t taddr = tmem_base + ((uint32_t)(q * 32) << 16) + b * PN + h * PCOLS;
                 // packed fp32x2 FMAs: half the issue slots of scalar ones, the same IEEE result in every lane
                 uint64_t s2;
@@ -442,7 +433,7 @@ fp8_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
             const int col0 = ti.n0 + h * PCOLS;
             const bool cvalid = col0 < p.N;
             const int out_row0 = GR ? 0 : e * p.M;                      // GK: the expert's slice of the (E * M, N) output
-            if (p.tma_out) {
+            if (GK || p.tma_out) {                                      // (what GK writes always goes through TMA)
                 // The tile leaves through TMA stores.  Every promotion warp owns two boxes of 32 rows x 128 bytes (128-byte swizzle) of the
                 // staging area, where its lanes drop their rows in 16-byte chunks.  A 2-byte output fits the warp's 128 columns in one
                 // round, and the store warp issues it; a 4-byte output takes two rounds of 64.  Rows of two owners leave as
@@ -451,7 +442,7 @@ fp8_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
                 constexpr int EPR = 128 / (int)sizeof(T);          // elements per 128-byte box row
                 constexpr int PER16 = 16 / (int)sizeof(T);
                 const uint32_t slot = smem_u32(c_stage) + warp * PBOXES * PBOX_BYTES;
-                const bool whole = !(GR || GK) || row - lane + 32 <= m_end;
+                const bool whole = !(GR || (GK && !TWO_BYTE)) || row - lane + 32 <= m_end;
 #pragma unroll
                 for (int r = 0; r < PCOLS / (PBOXES * EPR); ++r, ++round) {
                     if constexpr (STORE_WARP) {                   // the previous boxes have been read
