@@ -8,6 +8,7 @@
 // by one query, or results that are not finite (a NaN in a row nobody picked must not reach anyone, and 0 * NaN on a
 // tensor core would let it) set the flag, and the gather kernel, launched behind with that flag as its condition,
 // computes the whole call again.
+#include <type_traits>
 #include "attn_tc.cuh"
 #include <atomic>
 #include <cmath>
@@ -233,8 +234,8 @@ __device__ __forceinline__ void times_counts(float (&p)[16], uint32_t bit, const
 
 // 16 columns of a thread's row: scores to probabilities relative to `m`, left as parts over the scores and beside them.  The
 // picked raw scores go to `to` in passing when PUSH.  (32 columns at a time spilled.)
-template <bool PUSH>
-__device__ __forceinline__ void softmax_chunk(uint32_t t_s, uint32_t t_lead, uint32_t bit, float scale, float m, bool repeats,
+template <bool PUSH, bool REPEATS>
+__device__ __forceinline__ void softmax_chunk(uint32_t t_s, uint32_t t_lead, uint32_t bit, float scale, float m,
                                               const uint8_t*& count, float*& to, uint64_t (&l)[2]) {
     uint32_t v[16];
     float p[16];
@@ -251,7 +252,7 @@ __device__ __forceinline__ void softmax_chunk(uint32_t t_s, uint32_t t_lead, uin
             else p[e] = bit & (1u << e) ? p[e] : 0.0f;
         }
     }
-    if (repeats) times_counts(p, bit, count);
+    if constexpr (REPEATS) times_counts(p, bit, count);
 #pragma unroll
     for (int i = 0; i < 16; i += 2) l[(i >> 1) & 1] = add2(l[(i >> 1) & 1], pair2(p[i], p[i + 1]));
     store_parts16(t_s, t_lead, p);
@@ -576,12 +577,19 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
                 }
             }
             const float mu = m == -INFINITY ? 0.0f : m;
+            // (repeats are known per tile: inside a chunk, the choice cost the calls without any 1 %)
+            auto chunks = [&](auto push, auto repeated) {
 #pragma unroll 1
-            for (int c = 0; c < 4; ++c) {
-                const uint32_t bit = (c < 2 ? (h ? cur.z : cur.x) : (h ? cur.w : cur.y)) >> (c & 1) * 16;
-                if (half == 0) softmax_chunk<true>(t_s + c * 16, t_lead + c * 8, bit, a.scale, mu, repeats, count, to, l2);
-                else softmax_chunk<false>(t_s + c * 16, t_lead + c * 8, bit, a.scale, mu, repeats, count, to, l2);
-            }
+                for (int c = 0; c < 4; ++c) {
+                    const uint32_t bit = (c < 2 ? (h ? cur.z : cur.x) : (h ? cur.w : cur.y)) >> (c & 1) * 16;
+                    softmax_chunk<push.value, repeated.value>(t_s + c * 16, t_lead + c * 8, bit, a.scale, mu, count, to, l2);
+                }
+            };
+            constexpr std::true_type yes;
+            constexpr std::false_type no;
+            if (half == 0) { if (repeats) chunks(yes, yes); else chunks(yes, no); }
+            else if (repeats) chunks(no, yes);
+            else chunks(no, no);
             st_wait();
             tc_fence_before();
             __syncwarp();
