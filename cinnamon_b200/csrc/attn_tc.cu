@@ -1303,8 +1303,10 @@ static Plan make_plan(int64_t B, int64_t H, int64_t L, int64_t K, int64_t Dqk, i
 
 // Whether the dense tiles are worth it: their time (the causal half of the tiles is visited, a constant number of cycles
 // each that grows with the widths) against the gathers' (K rows of Dqk + Dv elements per query).  The constants are fitted
-// to measurements over L = 500 ... 4096, K = 32 ... 128, widths 64 ... 192; at 2 x 8 x 4096 queries the line lies between
-// K = 32 (gathers 0.21 ms, tiles 0.29 ms forward in bf16) and K = 128 (0.49 ms against 0.40 ms in fp32).
+// to measurements over L = 500 ... 4096, K = 32 ... 128, widths 64 ... 192, the forward's with a forward that took a quarter longer in bf16.
+// The forward's calls as they are now, gathers against tiles, at 2 x 8 x 4096 queries of 192: in bf16 131 and 207 us for K = 16, 207 and 205
+// for 32, 369 and 203 for 64; in fp32 240 and 457 for 32, 424 and 455 for 64, 774 and 461 for 128; at 1 x 8 x 2048 of 64 in bf16 49 and 66 for
+// 32, 80 and 66 for 64.
 static std::atomic<int> g_mode{-1};         // -1: by the estimate; 0 / 1: never / wherever the tiles can (tests, measurements)
 int set_mode(int mode) { return g_mode.exchange(mode); }
 

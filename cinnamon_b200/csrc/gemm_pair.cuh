@@ -255,7 +255,7 @@ fp8_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
     } else if (!OWN && warp == PSCALE) {
         // ------------------ scales (both CTAs): this CTA's rows' and both column blocks', K block by K block ------------------
         // Copied to where they are read, PFETCH blocks ahead.  Through registers, a block's values waited for the loads issued last, four
-        // blocks on: a miss for every row each eighth block (8837 x 17024 -> 320, one wave of tiles: 125 us so, 96 like this).  Multiplied here
+        // blocks on: a miss for every row each eighth block (8837 x 17024 -> 320, one wave of tiles: 101 us so, 69 like this).  Multiplied here
         // and not by their readers: 1 to 2 % slower on long reductions (the warp takes issue slots of two promotion warps).
         const float* a_ptr[4];
         const float* b_ptr[2];
