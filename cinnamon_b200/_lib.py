@@ -23,9 +23,11 @@ SIGNATURES = {
     "cinn_last_error": [],
     "cinn_quant_rowwise": [_vp, _i32, _i64, _i64, _i64, _i64, _vp, _vp, _i32, _i32, _i32, _vp],
     "cinn_quant_rowwise_dual": [_vp, _i32, _i64, _i64, _i64, _vp, _vp, _vp, _vp, _i32, _i32, _vp],
+    "cinn_quant_rowwise_dual_padded": [_vp, _i32, _i64, _i64, _i64, _vp, _vp, _vp, _vp, _i32, _i32, _vp],
     "cinn_selfcheck_division": [_vp, _vp],
     "cinn_quant_rowwise_with_block": [_vp, _i32, _i64, _i64, _i64, _vp, _vp, _vp, _vp, _i32, _i32, _vp],
     "cinn_quant_rowwise_with_block_t": [_vp, _i32, _i64, _i64, _i64, _vp, _vp, _vp, _vp, _i32, _i32, _vp],
+    "cinn_quant_rowwise_with_block_t_padded": [_vp, _i32, _i64, _i64, _i64, _vp, _vp, _vp, _vp, _i32, _i32, _vp],
     "cinn_set_wait_limit_cycles": [ctypes.c_longlong],
     "cinn_quant_blockwise_t": [_vp, _i32, _i64, _i64, _i64, _vp, _vp, _vp, _i32, _i32, _vp],
     "cinn_quant_linear": [_vp, _i32, _i64, _i64, _vp, _vp, _i32, _vp, _i32, _i64, _i64, _vp, _vp, _i64, _i64, _i64, _i32, _vp],

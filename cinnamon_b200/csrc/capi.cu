@@ -33,7 +33,7 @@ int sm_count() {
 int quantize(bool blockwise, const void* x, int dtype, int64_t M, int64_t N, int64_t ld_m, int64_t ld_n, void* q,
              float* scales, int bm, int bn, int round_scale, int div_mode, cudaStream_t st);
 int quantize_dual(const void* x, int dtype, int64_t M, int64_t N, int64_t ld, void* q_row, float* s_row, void* q_col,
-                  float* s_col, int round_scale, int div_mode, cudaStream_t st);
+                  float* s_col, int round_scale, int div_mode, cudaStream_t st, bool padded);
 int selfcheck_division(unsigned long long* mismatches, cudaStream_t st);
 int requant_row_to_block(const void* xq, const float* xs, int64_t M, int64_t K, void* out, float* scales,
                          int transpose_out, int div_mode, cudaStream_t st);
@@ -115,7 +115,7 @@ int fp8_grouped_wgrad(const void* dY, int dy_dtype, const void* x_q, const float
                       const int64_t* ends_host, int64_t E, int64_t T, int64_t d_in, int64_t d_out, void* scratch,
                       int64_t scratch_bytes, void* dW, int out_dtype, int div_mode, cudaStream_t st);
 int quantize_row_block(const void* x, int dtype, int64_t M, int64_t N, int64_t ld, void* q_row, float* s_row, void* q_blk,
-                       float* s_blk, int round_scale, int div_mode, cudaStream_t st, int transpose_block);
+                       float* s_blk, int round_scale, int div_mode, cudaStream_t st, int transpose_block, bool padded);
 int quantize_block_t(const void* x, int dtype, int64_t M, int64_t N, int64_t ld, void* q, void* q_t, float* scales,
                      int round_scale, int div_mode, cudaStream_t st);
 int swiglu(const void* h12, const void* dh, void* out, int dtype, int64_t T_rows, int64_t I, int backward, int round, cudaStream_t st);
@@ -178,7 +178,12 @@ int cinn_quant_block_beside(const void* x, int x_dtype, int64_t M, int64_t N, in
 
 int cinn_quant_rowwise_dual(const void* x, int x_dtype, int64_t M, int64_t N, int64_t ld, void* q_row, float* s_row,
                             void* q_col, float* s_col, int round_scale, int div_mode, void* stream) {
-    return cinn::quantize_dual(x, x_dtype, M, N, ld, q_row, s_row, q_col, s_col, round_scale, div_mode, (cudaStream_t)stream);
+    return cinn::quantize_dual(x, x_dtype, M, N, ld, q_row, s_row, q_col, s_col, round_scale, div_mode, (cudaStream_t)stream, false);
+}
+
+int cinn_quant_rowwise_dual_padded(const void* x, int x_dtype, int64_t M, int64_t N, int64_t ld, void* q_row, float* s_row,
+                                   void* q_col, float* s_col, int round_scale, int div_mode, void* stream) {
+    return cinn::quantize_dual(x, x_dtype, M, N, ld, q_row, s_row, q_col, s_col, round_scale, div_mode, (cudaStream_t)stream, true);
 }
 
 int cinn_selfcheck_division(unsigned long long* mismatches, void* stream) {
@@ -188,13 +193,19 @@ int cinn_selfcheck_division(unsigned long long* mismatches, void* stream) {
 int cinn_quant_rowwise_with_block(const void* x, int x_dtype, int64_t M, int64_t N, int64_t ld, void* q_row, float* s_row,
                                   void* q_block, float* s_block, int round_scale, int div_mode, void* stream) {
     return cinn::quantize_row_block(x, x_dtype, M, N, ld, q_row, s_row, q_block, s_block, round_scale, div_mode,
-                                    (cudaStream_t)stream, 0);
+                                    (cudaStream_t)stream, 0, false);
 }
 
 int cinn_quant_rowwise_with_block_t(const void* x, int x_dtype, int64_t M, int64_t N, int64_t ld, void* q_row, float* s_row,
                                     void* q_block_t, float* s_block, int round_scale, int div_mode, void* stream) {
     return cinn::quantize_row_block(x, x_dtype, M, N, ld, q_row, s_row, q_block_t, s_block, round_scale, div_mode,
-                                    (cudaStream_t)stream, 1);
+                                    (cudaStream_t)stream, 1, false);
+}
+
+int cinn_quant_rowwise_with_block_t_padded(const void* x, int x_dtype, int64_t M, int64_t N, int64_t ld, void* q_row, float* s_row,
+                                           void* q_block_t, float* s_block, int round_scale, int div_mode, void* stream) {
+    return cinn::quantize_row_block(x, x_dtype, M, N, ld, q_row, s_row, q_block_t, s_block, round_scale, div_mode,
+                                    (cudaStream_t)stream, 1, true);
 }
 
 int cinn_requant_row_to_block(const void* xq, const float* xs, int64_t M, int64_t K, void* out, float* scales,

@@ -22,7 +22,7 @@ using at::Tensor;
 
 #define CINN_HOST_API(X)                                                                                            \
     X(cinn_last_error) X(cinn_quant_rowwise) X(cinn_quant_rowwise_dual) X(cinn_quant_rowwise_with_block)             \
-    X(cinn_quant_rowwise_with_block_t) X(cinn_quant_blockwise) X(cinn_quant_block_beside) X(cinn_quant_linear) X(cinn_transpose_bytes)     \
+    X(cinn_quant_rowwise_with_block_t) X(cinn_quant_rowwise_dual_padded) X(cinn_quant_rowwise_with_block_t_padded) X(cinn_quant_blockwise) X(cinn_quant_block_beside) X(cinn_quant_linear) X(cinn_transpose_bytes)     \
     X(cinn_requant_row_to_block) X(cinn_fp8_gemm_ws) X(cinn_fp8_gemm_pitched) X(cinn_fp8_gemm_workspace_bytes) \
     X(cinn_sparse_attn_workspace_bytes) X(cinn_sparse_attn_fwd_ws) X(cinn_sparse_attn_bwd) X(cinn_sparse_attn_bwd_ws)                  \
     X(cinn_moe_route_workspace_ints) X(cinn_moe_route_ranges) X(cinn_spread_rows) X(cinn_fp8_grouped_gemm)                \
@@ -92,6 +92,11 @@ bool takes_node(const T&... t) {
     return (at::GradMode::is_enabled() && (t.requires_grad() || ...)) || (t._fw_grad(/*level=*/0).defined() || ...);
 }
 inline int64_t up(int64_t a, int64_t b) { return (a + b - 1) / b; }
+constexpr int64_t MAX_PADDED_ROWS = 65535 * 128;          // of the padded quantisers: row blocks that a launch takes
+// Whether they read a matrix in place, in 16-byte pieces
+inline bool padded_in_place(const Tensor& t) {
+    return t.stride(1) == 1 && t.stride(0) >= t.size(1) && t.stride(0) % 8 == 0 && (reinterpret_cast<uintptr_t>(t.data_ptr()) & 15) == 0;
+}
 inline void* stream() { return at::cuda::getCurrentCUDAStream().stream(); }
 inline float* f32(const Tensor& t);
 Tensor gemm(const Tensor& a, const Tensor& sa, const Tensor& b, int layout, const Tensor& sb, int64_t sbk, int64_t sbn, int64_t M,

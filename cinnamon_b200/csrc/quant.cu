@@ -367,6 +367,7 @@ __device__ __forceinline__ bool dual_tile(float (&v)[8][8], float (*s_amax)[128]
     const int n = n0 + sub * 8;
     const int mt = SEG ? src0 + hw * 8 : m0 + hw * 8;          // first row of this thread's row-wise outputs
     const int m_rows = SEG ? src0 + cnt : M;                    // one past the last row that is written row-wise
+    const int pitch = (M + 15) & ~15;                           // of the transposed rows, zeros behind M (whole 16-byte stores)
     if constexpr (SEG) {
 #pragma unroll
         for (int i = 0; i < 8; ++i)
@@ -455,9 +456,9 @@ __device__ __forceinline__ bool dual_tile(float (&v)[8][8], float (*s_amax)[128]
         const int idx = threadIdx.x + rep * 256;
         const int nl = idx >> 3, ch = idx & 7;
         const int nn = n0 + nl, mm = m0 + ch * 16;
-        if (nn < N && mm < M) {
+        if (nn < N && mm < pitch) {
             const uint4 val = *reinterpret_cast<const uint4*>(&s_out[nl * 128 + (((ch ^ (nl >> 3)) & 7) << 4)]);
-            __stcs(reinterpret_cast<uint4*>(q_col + (int64_t)nn * M + mm), val);
+            __stcs(reinterpret_cast<uint4*>(q_col + (int64_t)nn * pitch + mm), val);
         }
     }
     return true;
@@ -552,15 +553,15 @@ __device__ __forceinline__ bool row_block_tile(float (&v)[8][8], float* s_red, u
             *reinterpret_cast<uint2*>(&s_out[nl * 128 + ((((hw >> 1) ^ sub) & 7) << 4) + ((hw & 1) << 3)]) = o2;
         }
         __syncthreads();
-        const int m0 = bm * 128, n0 = bn * 128;
+        const int m0 = bm * 128, n0 = bn * 128, pitch = (M + 15) & ~15;
 #pragma unroll
         for (int rep = 0; rep < 4; ++rep) {
             const int idx = threadIdx.x + rep * 256;
             const int nl = idx >> 3, ch = idx & 7;
             const int nn = n0 + nl, mm = m0 + ch * 16;
-            if (nn < N && mm < M) {
+            if (nn < N && mm < pitch) {
                 const uint4 val = *reinterpret_cast<const uint4*>(&s_out[nl * 128 + (((ch ^ (nl >> 3)) & 7) << 4)]);
-                __stcs(reinterpret_cast<uint4*>(q_blk + (int64_t)nn * M + mm), val);
+                __stcs(reinterpret_cast<uint4*>(q_blk + (int64_t)nn * pitch + mm), val);
             }
         }
         // the staging tile and s_red are next written after the next piece's block-wide barrier
@@ -1480,11 +1481,12 @@ int quantize(bool blockwise, const void* x, int dtype, int64_t M, int64_t N, int
 
 template <typename T>
 static int dispatch_dual(const T* x, int64_t M, int64_t N, int64_t ld, uint8_t* q_row, float* s_row, uint8_t* q_col,
-                         float* s_col, int round_scale, int div_mode, cudaStream_t st) {
+                         float* s_col, int round_scale, int div_mode, cudaStream_t st, bool padded) {
     const int nb_n = (int)((N + 127) / 128), nb_m = (int)((M + 127) / 128);
-    const bool fused = M % 16 == 0 && N % 8 == 0 && ld % 8 == 0 && nb_m <= 65535 && aligned16(x) && aligned16(q_row) &&
+    const bool fused = (M % 16 == 0 || padded) && N % 8 == 0 && ld % 8 == 0 && nb_m <= 65535 && aligned16(x) && aligned16(q_row) &&
                        aligned16(q_col);
     if (!fused) {
+        CINN_CHECK_ARG(!padded || M % 16 == 0, "dual quantiser: padded rows need N %% 8 == 0, aligned rows and M <= 8388480");
         // ragged shapes: the two single-output quantisers, reading x twice
         int rc = dispatch_quant(false, x, M, N, ld, (int64_t)1, q_row, s_row, 1, 128, round_scale, div_mode, st);
         if (rc) return rc;
@@ -1530,10 +1532,11 @@ int requant_row_to_block(const void* xq, const float* xs, int64_t M, int64_t K, 
 // Row-wise 1x128 quantisation plus the 128x128 re-quantisation of its result, one pass over x.
 template <typename T>
 static int dispatch_row_block(const T* x, int64_t M, int64_t N, int64_t ld, uint8_t* q_row, float* s_row, uint8_t* q_blk,
-                              float* s_blk, int round_scale, int div_mode, cudaStream_t st, int transpose_block = 0) {
+                              float* s_blk, int round_scale, int div_mode, cudaStream_t st, int transpose_block) {
     const int nb_n = (int)((N + 127) / 128), nb_m = (int)((M + 127) / 128);
     const bool fused = N % 16 == 0 && ld % 8 == 0 && nb_m <= 65535 && aligned16(x) && aligned16(q_row) && aligned16(q_blk);
     if (!fused) {
+        CINN_CHECK_ARG(!transpose_block || M % 16 == 0, "row + block quantiser: padded rows need aligned rows and M <= 8388480");
         int rc = dispatch_quant(false, x, M, N, ld, (int64_t)1, q_row, s_row, 1, 128, round_scale, div_mode, st);
         if (rc) return rc;
         return requant_row_to_block(q_row, s_row, M, N, q_blk, s_blk, transpose_block, div_mode, st);
@@ -1578,8 +1581,8 @@ static int dispatch_row_block(const T* x, int64_t M, int64_t N, int64_t ld, uint
 }
 
 int quantize_row_block(const void* x, int dtype, int64_t M, int64_t N, int64_t ld, void* q_row, float* s_row, void* q_blk,
-                       float* s_blk, int round_scale, int div_mode, cudaStream_t st, int transpose_block) {
-    CINN_CHECK_ARG(!transpose_block || M % 16 == 0,
+                       float* s_blk, int round_scale, int div_mode, cudaStream_t st, int transpose_block, bool padded) {
+    CINN_CHECK_ARG(!transpose_block || padded || M % 16 == 0,
                    "row + block quantiser: a transposed block copy needs a row count (%lld) that is a multiple of 16", (long long)M);
     CINN_CHECK_ARG(M >= 0 && N >= 0, "row + block quantiser: negative shape (%lld, %lld)", (long long)M, (long long)N);
     if (M == 0 || N == 0) return CINN_OK;
@@ -1848,8 +1851,9 @@ int read_quant_status(int* out, int reset) {
     return CINN_OK;
 }
 
+// padded: the rows of q_col are M rounded up to 16 long, with zeros behind M
 int quantize_dual(const void* x, int dtype, int64_t M, int64_t N, int64_t ld, void* q_row, float* s_row, void* q_col,
-                  float* s_col, int round_scale, int div_mode, cudaStream_t st) {
+                  float* s_col, int round_scale, int div_mode, cudaStream_t st, bool padded) {
     CINN_CHECK_ARG(M >= 0 && N >= 0, "dual quantiser: negative shape (%lld, %lld)", (long long)M, (long long)N);
     if (M == 0 || N == 0) return CINN_OK;
     CINN_CHECK_ARG(x && q_row && s_row && q_col && s_col, "dual quantiser: null pointer");
@@ -1857,9 +1861,9 @@ int quantize_dual(const void* x, int dtype, int64_t M, int64_t N, int64_t ld, vo
     CINN_CHECK_ARG(ld >= N, "dual quantiser: row pitch %lld below the row length %lld", (long long)ld, (long long)N);
     CINN_CHECK_ARG(div_mode == CINN_DIV_FULL || div_mode == CINN_DIV_RN, "dual quantiser: unknown div_mode %d", div_mode);
     switch (dtype) {
-        case CINN_BF16: return dispatch_dual((const __nv_bfloat16*)x, M, N, ld, (uint8_t*)q_row, s_row, (uint8_t*)q_col, s_col, round_scale, div_mode, st);
-        case CINN_F16:  return dispatch_dual((const __half*)x, M, N, ld, (uint8_t*)q_row, s_row, (uint8_t*)q_col, s_col, round_scale, div_mode, st);
-        case CINN_F32:  return dispatch_dual((const float*)x, M, N, ld, (uint8_t*)q_row, s_row, (uint8_t*)q_col, s_col, round_scale, div_mode, st);
+        case CINN_BF16: return dispatch_dual((const __nv_bfloat16*)x, M, N, ld, (uint8_t*)q_row, s_row, (uint8_t*)q_col, s_col, round_scale, div_mode, st, padded);
+        case CINN_F16:  return dispatch_dual((const __half*)x, M, N, ld, (uint8_t*)q_row, s_row, (uint8_t*)q_col, s_col, round_scale, div_mode, st, padded);
+        case CINN_F32:  return dispatch_dual((const float*)x, M, N, ld, (uint8_t*)q_row, s_row, (uint8_t*)q_col, s_col, round_scale, div_mode, st, padded);
         default: set_error("dual quantiser: unknown dtype tag %d", dtype); return CINN_ERR_INVALID;
     }
 }

@@ -33,6 +33,7 @@ from .sparse_attention import SparseAttentionFunction, sparse_attention  # noqa:
 _L = _lib.lib
 _host = _lib.host
 FP8_E4M3_MAX = 448.0
+_MAX_PADDED_ROWS = 65535 * 128              # of the quantisers that pad a ragged number of rows: row blocks a launch takes
 
 _DTYPE_TAG = {torch.bfloat16: _lib.BF16, torch.float32: _lib.F32, torch.float16: _lib.F16}
 _DIV_MODE = {"full": _lib.DIV_FULL, "rn": _lib.DIV_RN}[os.environ.get("CINN_DIV_MODE", "full")]
@@ -158,7 +159,28 @@ def quantize_fp8_rowwise_dual(x: torch.Tensor, round_scale: bool = False):
     return q_row, s_row, q_col, s_col
 
 
-def quantize_fp8_rowwise_with_block(x: torch.Tensor, round_scale: bool = False, transpose_block: bool = False):
+def _padded_in_place(t: torch.Tensor) -> bool:
+    return t.stride(1) == 1 and t.stride(0) >= t.shape[1] and t.stride(0) % 8 == 0 and t.data_ptr() % 16 == 0
+
+
+def _quantize_dual_padded(x: torch.Tensor, round_scale: bool):
+    """``quantize_fp8_rowwise_dual`` with ``q_col`` (N, M rounded up to 16), zeros behind the first M of its rows."""
+    x = _as_quant_input(x)
+    if not _padded_in_place(x):
+        x = x.clone(memory_format=torch.contiguous_format)
+    M, N = x.shape
+    with torch.cuda.device(x.device):
+        q_row = torch.empty((M, N), dtype=torch.float8_e4m3fn, device=x.device)
+        s_row = torch.empty((M, (N + 127) // 128), dtype=torch.float32, device=x.device)
+        q_col = torch.empty((N, (M + 15) // 16 * 16), dtype=torch.float8_e4m3fn, device=x.device)
+        s_col = torch.empty((N, (M + 127) // 128), dtype=torch.float32, device=x.device)
+        _lib.check(_L.cinn_quant_rowwise_dual_padded(_ptr(x), _DTYPE_TAG[x.dtype], M, N, x.stride(0), _ptr(q_row), _ptr(s_row),
+                                                     _ptr(q_col), _ptr(s_col), int(bool(round_scale)), _DIV_MODE, _stream(x)),
+                   "cinn_quant_rowwise_dual")
+    return q_row, s_row, q_col, s_col
+
+
+def quantize_fp8_rowwise_with_block(x: torch.Tensor, round_scale: bool = False, transpose_block: bool = False, _padded: bool = False):
     """``quantize_fp8_rowwise(x)`` together with ``quantize_fp8_blockwise(dequantize_fp8_rowwise(q, s))`` of its result
     (what ``FP8MatmulFunction`` computes in its forward, reference src/kernels.py:746, and on the saved activations in
     its backward, :784-787) from one pass over ``x``.  Returns ``(q_row, s_row, q_block, s_block)``; bit-identical to
@@ -172,12 +194,16 @@ def quantize_fp8_rowwise_with_block(x: torch.Tensor, round_scale: bool = False, 
         x = x.contiguous()
     M, N = x.shape
     nb = (N + 127) // 128
+    Mp = (M + 15) // 16 * 16 if _padded else M            # rows of the transposed copy, zeros behind the first M
+    if Mp != M and x.stride(0) >= N and not _padded_in_place(x):
+        x = x.clone(memory_format=torch.contiguous_format)
     with torch.cuda.device(x.device):
         q_row = torch.empty((M, N), dtype=torch.float8_e4m3fn, device=x.device)
         s_row = torch.empty((M, nb), dtype=torch.float32, device=x.device)
-        q_blk = torch.empty((N, M) if transpose_block else (M, N), dtype=torch.float8_e4m3fn, device=x.device)
+        q_blk = torch.empty((N, Mp) if transpose_block else (M, N), dtype=torch.float8_e4m3fn, device=x.device)
         s_blk = torch.empty(((M + 127) // 128, nb), dtype=torch.float32, device=x.device)
-        fn = _L.cinn_quant_rowwise_with_block_t if transpose_block else _L.cinn_quant_rowwise_with_block
+        fn = _L.cinn_quant_rowwise_with_block if not transpose_block else (
+            _L.cinn_quant_rowwise_with_block_t_padded if _padded else _L.cinn_quant_rowwise_with_block_t)
         _lib.check(fn(_ptr(x), _DTYPE_TAG[x.dtype], M, N, x.stride(0), _ptr(q_row), _ptr(s_row),
                       _ptr(q_blk), _ptr(s_blk), int(bool(round_scale)), _DIV_MODE, _stream(x)),
                    "cinn_quant_rowwise_with_block")
@@ -383,11 +409,12 @@ class FP8MatmulFunction(torch.autograd.Function):
         # backward needs (:784-787) comes out of the same pass over x and is what gets saved
         want_wgrad = ctx.needs_input_grad[1] and K % 16 == 0
         # the block copy is written with the token axis contiguous: the weight gradient reduces over tokens, and both
-        # of its operands are then K-major like the forward's (tensor-core operand reads are fastest that way)
-        x_blk_t = want_wgrad and M % 16 == 0 and _KMAJOR_BACKWARD
+        # of its operands are then K-major like the forward's (tensor-core operand reads are fastest that way); a ragged
+        # number of tokens is padded to a multiple of 16 with zeros
+        x_blk_t = want_wgrad and _KMAJOR_BACKWARD and (M % 16 == 0 or M <= _MAX_PADDED_ROWS)
         if want_wgrad:
             x_fp8, x_scale, x_blk, x_blk_scale = quantize_fp8_rowwise_with_block(x_flat, round_scale=round_scale,
-                                                                                 transpose_block=x_blk_t)
+                                                                                 transpose_block=x_blk_t, _padded=x_blk_t)
         else:
             x_fp8, x_scale = quantize_fp8_rowwise(x_flat, block_size=128, round_scale=round_scale)
         ctx.w_fp8_t = None
@@ -430,15 +457,19 @@ class FP8MatmulFunction(torch.autograd.Function):
             grad_flat = grad_flat.contiguous()
         M = grad_flat.shape[0]
         # The token axis is the reduction axis of the weight gradient; the GEMM wants it in multiples
-        # of 16, so a ragged token count is padded with zero rows (they change neither an amax nor a sum).
+        # of 16, so a ragged token count is padded with zeros (they change neither an amax nor a sum), by the quantiser
+        # where it can.
         Mp = (M + 15) // 16 * 16
-        if Mp != M:                                        # (never with a transposed block copy: that needs M % 16 == 0)
+        in_pass = Mp != M and N % 8 == 0 and M <= _MAX_PADDED_ROWS
+        if Mp != M and not in_pass:
             grad_flat = torch.nn.functional.pad(grad_flat, (0, 0, 0, Mp - M))
+        if Mp != M and not ctx.x_is_block_t:
             x_fp8 = torch.nn.functional.pad(x_fp8.view(torch.uint8), (0, 0, 0, Mp - M)).view(torch.float8_e4m3fn)
             if not ctx.x_is_block:                         # block scales: zero rows stay inside the last row block
                 x_scale = torch.nn.functional.pad(x_scale, (0, 0, 0, Mp - M), value=1.0)
         # dy quantised along features for dgrad (:771) and along tokens for wgrad (:781-783), one pass over dy
-        grad_fp8, grad_scale, grad_fp8_t, grad_scale_t = quantize_fp8_rowwise_dual(grad_flat, round_scale=round_scale)
+        dual = _quantize_dual_padded if in_pass else quantize_fp8_rowwise_dual
+        grad_fp8, grad_scale, grad_fp8_t, grad_scale_t = dual(grad_flat, round_scale=round_scale)
         # dgrad (:771-774): dy (M, N) @ W (N, K).  W is the B operand with the reduction axis N; a byte-transposed
         # copy (K, N) puts that axis innermost (the block scales are shared, indices swapped), otherwise the stored
         # bytes are read (reduction, output)

@@ -62,7 +62,7 @@ def _linear_layout(x_shape, w_shape, w_stride, w_dtype, need_dgrad: bool, need_w
         M *= s
     N = w_shape[0]
     want_wgrad = need_wgrad and Kd % 16 == 0
-    x_blk_t = want_wgrad and M % 16 == 0 and K._KMAJOR_BACKWARD
+    x_blk_t = want_wgrad and K._KMAJOR_BACKWARD and (M % 16 == 0 or M <= K._MAX_PADDED_ROWS)
     w_contig = (w_stride[1] == 1 and w_stride[0] % 4 == 0) or w_dtype not in K._DTYPE_TAG
     w_t = K._KMAJOR_BACKWARD and need_dgrad and N % 16 == 0 and Kd % 4 == 0 and w_contig
     return M, Kd, N, want_wgrad, x_blk_t, w_t
@@ -82,7 +82,7 @@ def fp8_linear_fwd(x: Tensor, weight: Tensor, round_scale: bool, need_dgrad: boo
 def _(x, weight, round_scale, need_dgrad, need_wgrad):
     M, Kd, N, want_wgrad, x_blk_t, w_t = _linear_layout(x.shape, weight.shape, weight.stride(), weight.dtype, need_dgrad, need_wgrad)
     e = lambda shape, dt: torch.empty(shape, dtype=dt, device=x.device)                         # noqa: E731
-    return (e(tuple(x.shape[:-1]) + (N,), torch.bfloat16), e((Kd, M) if x_blk_t else (M, Kd), F8),
+    return (e(tuple(x.shape[:-1]) + (N,), torch.bfloat16), e((Kd, (M + 15) // 16 * 16) if x_blk_t else (M, Kd), F8),
             e((_nb(M) if want_wgrad else M, _nb(Kd)), torch.float32), e((N, Kd), F8), e((_nb(N), _nb(Kd)), torch.float32),
             e((Kd, N) if w_t else (0,), F8))
 

@@ -60,6 +60,12 @@ int cinn_quant_rowwise(const void* x, int x_dtype, int64_t M, int64_t N, int64_t
 int cinn_quant_rowwise_dual(const void* x, int x_dtype, int64_t M, int64_t N, int64_t ld, void* q_row, float* s_row,
                             void* q_col, float* s_col, int round_scale, int div_mode, void* stream);
 
+/* The same for any M: q_col is (N, M rounded up to 16) with zero bytes behind the first M of a row, the form in which the
+ * weight-gradient GEMM takes a ragged number of tokens as its reduction axis.  N and ld must be multiples of 8, x, q_row
+ * and q_col 16-byte aligned and M at most 8388480 (without these, M a multiple of 16). */
+int cinn_quant_rowwise_dual_padded(const void* x, int x_dtype, int64_t M, int64_t N, int64_t ld, void* q_row, float* s_row,
+                                   void* q_col, float* s_col, int round_scale, int div_mode, void* stream);
+
 /* Diagnostic (no reference counterpart).  With CINN_DIV_FULL the quantisers form x / scale as
  * x * rcp.approx(scale), the reciprocal taken once per scale.  This call checks on the current GPU that the
  * product has the bits of div.full.f32(x, scale) - the instruction Triton emits for the reference kernels

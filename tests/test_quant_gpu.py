@@ -295,3 +295,40 @@ def test_rowwise_with_transposed_block_copy(K, shape, dtype, rs):
     assert q_blk_t.shape == (N, M) and torch.equal(q_blk_t.view(torch.uint8), q_blk.view(torch.uint8).t())
     ref_q, ref_s = O.requantize_row_to_block(*O.quantize_rowwise(x.cpu(), 128, rs))
     assert_quant_equal(q_blk, s_blk, ref_q, ref_s, what="block copy")
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("M,N,rs", [(1, 128, False), (15, 264, True), (17, 128, False), (127, 640, True), (143, 200, False), (2049, 384, True)])
+def test_padded_quantisers_on_a_ragged_number_of_rows(K, M, N, rs, dtype):
+    """Rows of the transposed copies are M rounded up to 16 long: the bytes and scales of the separate calls, zeros behind them."""
+    x = torch.randn(M, N, device="cuda", generator=torch.Generator(device="cuda").manual_seed(M)).mul_(3).to(dtype)
+    Mp = (M + 15) // 16 * 16
+    q, s, qt, st = K._quantize_dual_padded(x, rs)
+    rq, r_s = K.quantize_fp8_rowwise(x, 128, rs)
+    cq, c_s = K.quantize_fp8_rowwise(x.t(), 128, rs)
+    assert qt.shape == (N, Mp) and torch.equal(s, r_s) and torch.equal(st, c_s)
+    assert torch.equal(q.view(torch.uint8), rq.view(torch.uint8)) and torch.equal(qt[:, :M].view(torch.uint8), cq.view(torch.uint8))
+    assert int(qt[:, M:].view(torch.uint8).sum()) == 0
+    if N % 16 == 0:
+        q2, s2, blk, bs = K.quantize_fp8_rowwise_with_block(x, rs, transpose_block=True, _padded=True)
+        bq, b_s = K.requantize_rowwise_to_blockwise(rq, r_s)
+        assert blk.shape == (N, Mp) and torch.equal(s2, r_s) and torch.equal(bs, b_s)
+        assert torch.equal(q2.view(torch.uint8), rq.view(torch.uint8)) and int(blk[:, M:].view(torch.uint8).sum()) == 0
+        assert torch.equal(blk[:, :M].view(torch.uint8), bq.view(torch.uint8).t())
+
+
+@pytest.mark.parametrize("M,off", [(33, 0), (33, 8), (1001, 4)])
+def test_linear_gradients_of_ragged_and_unaligned_tokens(K, M, off):
+    """A ragged number of tokens, rows at any alignment: the gradients of the same tokens padded with zero rows by hand."""
+    g = torch.Generator(device="cuda").manual_seed(M + off)
+    lin = K.FP8Linear(256, 384).cuda()
+    buf, dbuf = (torch.randn(M * n + off, device="cuda", generator=g, dtype=torch.float32).to(torch.bfloat16) for n in (256, 384))
+    x, dy = buf[off:].view(M, 256), dbuf[off:].view(M, 384)
+    Mp = (M + 15) // 16 * 16
+    grads = []
+    for rows in (M, Mp):
+        xs, ds = (torch.nn.functional.pad(t, (0, 0, 0, rows - M)) if rows > M else t for t in (x, dy))
+        xs = xs.detach().requires_grad_(True)
+        gx, gw = torch.autograd.grad(lin(xs), [xs, lin.weight], ds)
+        grads.append((gx[:M], gw))
+    assert torch.equal(grads[0][0], grads[1][0]) and torch.equal(grads[0][1], grads[1][1])
