@@ -91,6 +91,11 @@ int cinn_quant_rowwise_with_block(const void* x, int x_dtype, int64_t M, int64_t
 int cinn_quant_rowwise_with_block_t(const void* x, int x_dtype, int64_t M, int64_t N, int64_t ld, void* q_row, float* s_row,
                                     void* q_block_t, float* s_block, int round_scale, int div_mode, void* stream);
 
+/* The same for any M, with rows of q_block_t M rounded up to 16 long and zero bytes behind the first M; ld a multiple of 8,
+ * x, q_row and q_block_t 16-byte aligned and M at most 8388480 (without these, M a multiple of 16). */
+int cinn_quant_rowwise_with_block_t_padded(const void* x, int x_dtype, int64_t M, int64_t N, int64_t ld, void* q_row, float* s_row,
+                                           void* q_block_t, float* s_block, int round_scale, int div_mode, void* stream);
+
 /* Block-wise block_m x block_n quantisation.
  * Replaces quantize_fp8_blockwise_kernel + quantize_fp8_blockwise (src/kernels.py:74-132, 219-259).
  * scales: (ceil(M/block_m), ceil(N/block_n)). */
