@@ -30,6 +30,8 @@ SIGNATURES = {
     "cinn_quant_rowwise_with_block_t_padded": [_vp, _i32, _i64, _i64, _i64, _vp, _vp, _vp, _vp, _i32, _i32, _vp],
     "cinn_set_wait_limit_cycles": [ctypes.c_longlong],
     "cinn_quant_blockwise_t": [_vp, _i32, _i64, _i64, _i64, _vp, _vp, _vp, _i32, _i32, _vp],
+    "cinn_fp8_linear_few_takes": [_vp, _i32, _i64, _i64, _vp, _i32, _i64, _i64, _i64, _i64, _i64],
+    "cinn_fp8_linear_few": [_vp, _i32, _i64, _i32, _vp, _i64, _vp, _i64, _i64, _i64, _i32, _vp],
     "cinn_quant_linear": [_vp, _i32, _i64, _i64, _vp, _vp, _i32, _vp, _i32, _i64, _i64, _vp, _vp, _i64, _i64, _i64, _i32, _vp],
     "cinn_quant_block_beside": [_vp, _i32, _i64, _i64, _i64, _i64, _vp, _vp, _vp, _i32, _i32, _vp],
     "cinn_quant_blockwise": [_vp, _i32, _i64, _i64, _i64, _i64, _vp, _vp, _i32, _i32, _i32, _i32, _vp],

@@ -16,7 +16,7 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 LIB_DIR = os.path.join(HERE, "lib")
 LIB_PATH = os.path.join(LIB_DIR, "libcinnamon_b200.so")
-SOURCES = ["quant.cu", "gemm.cu", "moe.cu", "moe_train.cu", "route.cu", "sparse_attn.cu", "attn_tc.cu", "indexer.cu", "wgrad.cu", "capi.cu"]
+SOURCES = ["quant.cu", "gemm.cu", "linear_few.cu", "moe.cu", "moe_train.cu", "route.cu", "sparse_attn.cu", "attn_tc.cu", "indexer.cu", "wgrad.cu", "capi.cu"]
 HOST_DIR = os.path.join(CSRC, "host")
 HOST_PATH = os.path.join(LIB_DIR, "_host.so")
 HOST_SOURCES = ["linear.cpp", "attention.cpp", "moe.cpp", "moe_train.cpp", "module.cpp"]

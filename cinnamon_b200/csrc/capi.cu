@@ -57,6 +57,10 @@ int fp8_grouped_gemm(const void* A, const float* sA, const void* W, const float*
 int p2p_row_table(const int64_t* seg_start, const int64_t* home_base, const int64_t* peer_home, int64_t n_rows, int64_t row_bytes,
                   int n_segments, int n_ranks, int64_t capacity, long long* row_dst, cudaStream_t st);   // rows past seg_start[n_segments] get 0
 
+bool linear_few_takes(const void* x, int x_dtype, int64_t ldx_m, int64_t ldx_k, const void* w, int w_dtype, int64_t ldw_n, int64_t ldw_k,
+                      int64_t M, int64_t N, int64_t K);
+int linear_few(const void* x, int x_dtype, int64_t ldx, int round_scale, const float* w, int64_t ldw, void* out, int64_t M, int64_t N,
+               int64_t K, int div_mode, cudaStream_t st);
 int read_device_status(int* out, int reset);
 int fp8_grouped_gemm_dgrad(const void* dY, const float* sdY, const void* W, const float* sW, const int64_t* starts,
                            const int64_t* ends, int64_t E, int64_t T, int64_t d_in, int64_t d_out, void* dX, int out_dtype,
@@ -169,6 +173,16 @@ int cinn_quant_linear(const void* x, int x_dtype, int64_t ldx_m, int64_t ldx_k, 
                       void* stream) {
     return cinn::quantize_linear(x, x_dtype, ldx_m, ldx_k, xq, xs, round_scale, w, w_dtype, ldw_n, ldw_k, wq, ws, M, N, K, div_mode,
                                  (cudaStream_t)stream);
+}
+
+int cinn_fp8_linear_few_takes(const void* x, int x_dtype, int64_t ldx_m, int64_t ldx_k, const void* w, int w_dtype, int64_t ldw_n,
+                              int64_t ldw_k, int64_t M, int64_t N, int64_t K) {
+    return cinn::linear_few_takes(x, x_dtype, ldx_m, ldx_k, w, w_dtype, ldw_n, ldw_k, M, N, K);
+}
+
+int cinn_fp8_linear_few(const void* x, int x_dtype, int64_t ldx, int round_scale, const float* w, int64_t ldw, void* out, int64_t M,
+                        int64_t N, int64_t K, int div_mode, void* stream) {
+    return cinn::linear_few(x, x_dtype, ldx, round_scale, w, ldw, out, M, N, K, div_mode, (cudaStream_t)stream);
 }
 
 int cinn_quant_block_beside(const void* x, int x_dtype, int64_t M, int64_t N, int64_t ld_m, int64_t ld_n, void* q, void* q_t,

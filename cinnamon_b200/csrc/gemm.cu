@@ -77,26 +77,6 @@ __device__ __forceinline__ float ld_scale(const float* p) {
     return v;
 }
 
-// D[tmem] = A[smem desc] * B[smem desc], e4m3 x e4m3 -> fp32.  Called by a whole warp, issued by one elected lane.
-// The four MMAs of a K block by one statement with one election: one by one, with 64-bit descriptors, they cost their warp 350
-// cycles, like this 100.  Low words of the descriptors; STEP_B: 16-byte units from one step's B to the next.
-template <int STEP_B>
-__device__ __forceinline__ void tc_mma_f8_block(uint32_t d_tmem, uint32_t a_lo, uint32_t b_lo, uint32_t idesc) {
-    constexpr uint32_t hi = (uint32_t)((((uint64_t)(1024 >> 4) << 32) | (1ull << 46) | (2ull << 61)) >> 32);
-    asm volatile(
-        "{\n\t.reg .pred e;\n\t.reg .b64 a, b;\n\t.reg .b32 x, y;\n\t"
-        "elect.sync _|e, 0xffffffff;\n\t"
-        "mov.b64 a, {%1, %4};\n\tmov.b64 b, {%2, %4};\n\t"
-        "@e tcgen05.mma.cta_group::1.kind::f8f6f4 [%0], a, b, %3, 0;\n\t"
-        "add.u32 x, %1, 2;\n\tadd.u32 y, %2, %5;\n\tmov.b64 a, {x, %4};\n\tmov.b64 b, {y, %4};\n\t"
-        "@e tcgen05.mma.cta_group::1.kind::f8f6f4 [%0], a, b, %3, 1;\n\t"
-        "add.u32 x, %1, 4;\n\tadd.u32 y, %2, %6;\n\tmov.b64 a, {x, %4};\n\tmov.b64 b, {y, %4};\n\t"
-        "@e tcgen05.mma.cta_group::1.kind::f8f6f4 [%0], a, b, %3, 1;\n\t"
-        "add.u32 x, %1, 6;\n\tadd.u32 y, %2, %7;\n\tmov.b64 a, {x, %4};\n\tmov.b64 b, {y, %4};\n\t"
-        "@e tcgen05.mma.cta_group::1.kind::f8f6f4 [%0], a, b, %3, 1;\n\t}"
-        ::"r"(d_tmem), "r"(a_lo), "r"(b_lo), "r"(idesc), "r"(hi), "n"(STEP_B), "n"(2 * STEP_B), "n"(3 * STEP_B) : "memory");
-}
-
 // Instruction descriptor for kind::f8f6f4: fp32 accumulate, e4m3 x e4m3, A K-major.
 __host__ __device__ constexpr uint32_t make_idesc(bool b_mn_major) {
     return (1u << 4)                              // D format: fp32
@@ -754,6 +734,7 @@ static inline int gemm_sms() {
     const int lim = g_gemm_sm_limit.load(std::memory_order_relaxed), all = sm_count();
     return (lim > 0 && lim < all) ? lim : all;
 }
+bool gemm_sms_capped() { return gemm_sms() < sm_count(); }
 int set_gemm_sm_limit(int n) { return g_gemm_sm_limit.exchange(n < 0 ? 0 : n); }
 
 static inline bool al16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
@@ -1165,11 +1146,12 @@ int read_quant_status(int* out, int reset);
 int read_moe_status(int* out, int reset);
 int read_indexer_status(int* out, int reset);
 int read_attn_status(int* out, int reset);
+int read_linear_few_status(int* out, int reset);
 
 // One word for the caller: the GEMM's code if it has one, else the quantisers', the exchange kernels', the indexer's,
-// the attention's.
+// the attention's, the few-row linear's.
 int read_device_status(int* out, int reset) {
-    int v = 0, q = 0, m = 0, x = 0, a = 0;
+    int v = 0, q = 0, m = 0, x = 0, a = 0, f = 0;
     CINN_CHECK_CUDA(cudaMemcpyFromSymbol(&v, g_device_status, sizeof(int)));
     if (reset && v != 0) {
         int z = 0;
@@ -1183,7 +1165,9 @@ int read_device_status(int* out, int reset) {
     if (rc) return rc;
     rc = read_attn_status(&a, reset);
     if (rc) return rc;
-    *out = v != 0 ? v : (q != 0 ? q : (m != 0 ? m : (x != 0 ? x : a)));
+    rc = read_linear_few_status(&f, reset);
+    if (rc) return rc;
+    *out = v != 0 ? v : (q != 0 ? q : (m != 0 ? m : (x != 0 ? x : (a != 0 ? a : f))));
     return CINN_OK;
 }
 

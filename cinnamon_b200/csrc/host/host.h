@@ -25,6 +25,7 @@ using at::Tensor;
     X(cinn_quant_rowwise_with_block_t) X(cinn_quant_rowwise_dual_padded) X(cinn_quant_rowwise_with_block_t_padded) X(cinn_quant_blockwise) X(cinn_quant_block_beside) X(cinn_quant_linear) X(cinn_transpose_bytes)     \
     X(cinn_requant_row_to_block) X(cinn_fp8_gemm_ws) X(cinn_fp8_gemm_pitched) X(cinn_fp8_gemm_workspace_bytes) \
     X(cinn_sparse_attn_workspace_bytes) X(cinn_sparse_attn_fwd_ws) X(cinn_sparse_attn_bwd) X(cinn_sparse_attn_bwd_ws)                  \
+    X(cinn_fp8_linear_few_takes) X(cinn_fp8_linear_few)                                                                   \
     X(cinn_moe_route_workspace_ints) X(cinn_moe_route_ranges) X(cinn_spread_rows) X(cinn_fp8_grouped_gemm)                \
     X(cinn_swiglu_quant_rowwise) X(cinn_moe_combine) X(cinn_moe_combine_add) X(cinn_moe_sum_add)                \
     X(cinn_swiglu_rounded) X(cinn_swiglu_rounded_backward) X(cinn_moe_balance_workspace_bytes) X(cinn_moe_balance_loss)     \
@@ -108,7 +109,10 @@ struct Linear {                                 // what an FP8 linear's forward 
 };
 Linear linear_forward(const Tensor& x, const Tensor& weight, bool round_scale, bool need_dgrad, bool need_wgrad, bool kmajor, int div,
                       const Tensor& w_q, const Tensor& w_s, const Tensor& w_qt);
-Tensor linear_inference(const Tensor& x, const Tensor& weight, bool round_scale, int div);
+// the rest of linear_forward once x is quantised: weight, product (into r.out)
+void linear_multiply(Linear& r, const Tensor& xq, const Tensor& xs, const Tensor& wf, bool need_dgrad, bool kmajor, int div, const Tensor& w_q,
+                     const Tensor& w_s, const Tensor& w_qt);
+Tensor linear_inference(const Tensor& x, const Tensor& weight, bool round_scale, int div, bool one_kernel);
 // (input gradients, weight gradient).  `parts` > 1: the weight is that many layers of equally many rows (a multiple of 128)
 // stacked, and every layer's input gradient is returned by itself.
 std::tuple<std::vector<Tensor>, Tensor> linear_backward(const Tensor& grad_out, Tensor x, Tensor x_scale, const Tensor& w,

@@ -160,8 +160,9 @@ std::tuple<std::vector<Tensor>, Tensor> linear_backward(const Tensor& grad_out, 
 }
 
 
-// Without gradients nothing but the result outlives the call: one scratch buffer, one launch for both quantisers.
-Tensor linear_inference(const Tensor& x, const Tensor& weight, bool round_scale, int div) {
+// Without gradients nothing but the result outlives the call: one launch for few rows (one_kernel), else one scratch buffer and one
+// launch for both quantisers.
+Tensor linear_inference(const Tensor& x, const Tensor& weight, bool round_scale, int div, bool one_kernel) {
     check_operands(x, weight, Tensor(), Tensor());
     c10::cuda::CUDAGuard guard(x.device());
     const int64_t K = x.size(-1), N = weight.size(0), nkb = up(K, 128);
@@ -170,6 +171,12 @@ Tensor linear_inference(const Tensor& x, const Tensor& weight, bool round_scale,
     auto shape = x.sizes().vec();
     shape.back() = N;
     Tensor out = empty(shape, at::kBFloat16, x.device());
+    if (one_kernel && api.cinn_fp8_linear_few_takes(xf.data_ptr(), tag_of(xf.scalar_type()), xf.stride(0), xf.stride(1), wf.data_ptr(),
+                                      tag_of(wf.scalar_type()), wf.stride(0), wf.stride(1), M, N, K)) {
+        check(api.cinn_fp8_linear_few(xf.data_ptr(), tag_of(xf.scalar_type()), xf.stride(0), round_scale, f32(wf), wf.stride(0),
+                                      out.data_ptr(), M, N, K, div, stream()), "cinn_fp8_linear_few");
+        return out;
+    }
     const auto room = [](int64_t bytes) { return (bytes + 255) / 256 * 256; };
     const int64_t o_xs = room(M * K), o_wq = o_xs + room(4 * M * nkb), o_ws = o_wq + room(N * K), o_part = o_ws + room(4 * up(N, 128) * nkb);
     const int64_t need = api.cinn_fp8_gemm_workspace_bytes(M, N, K, 0);            // few tiles, long reduction: cut along K
@@ -239,7 +246,7 @@ void bind_linear(pybind11::module_& m) {
         const CachedWeight cached{or_none(wq), or_none(ws), or_none(wqt)};
         if (takes_node(x, w))
             return LinearNode::apply(x, w, round_scale, kmajor, (int64_t)div, &cached);
-        if (!cached.q.defined()) return linear_inference(x, w, round_scale, div);
+        if (!cached.q.defined()) return linear_inference(x, w, round_scale, div, true);
         return linear_forward(x, w, round_scale, false, false, kmajor, div, cached.q, cached.s, cached.q_t).out;
     });
 }

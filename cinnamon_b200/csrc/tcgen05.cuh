@@ -59,6 +59,26 @@ __device__ __forceinline__ void tc_mma_f16(uint32_t d_tmem, uint64_t a_desc, uin
         ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate) : "memory");
 }
 
+// D[tmem] = A[smem desc] * B[smem desc], e4m3 x e4m3 -> fp32.  Called by a whole warp, issued by one elected lane.
+// The four MMAs of a K block by one statement with one election: one by one, with 64-bit descriptors, they cost their warp 350
+// cycles, like this 100.  Low words of the descriptors; STEP_B: 16-byte units from one step's B to the next.
+template <int STEP_B>
+__device__ __forceinline__ void tc_mma_f8_block(uint32_t d_tmem, uint32_t a_lo, uint32_t b_lo, uint32_t idesc) {
+    constexpr uint32_t hi = (uint32_t)((((uint64_t)(1024 >> 4) << 32) | (1ull << 46) | (2ull << 61)) >> 32);
+    asm volatile(
+        "{\n\t.reg .pred e;\n\t.reg .b64 a, b;\n\t.reg .b32 x, y;\n\t"
+        "elect.sync _|e, 0xffffffff;\n\t"
+        "mov.b64 a, {%1, %4};\n\tmov.b64 b, {%2, %4};\n\t"
+        "@e tcgen05.mma.cta_group::1.kind::f8f6f4 [%0], a, b, %3, 0;\n\t"
+        "add.u32 x, %1, 2;\n\tadd.u32 y, %2, %5;\n\tmov.b64 a, {x, %4};\n\tmov.b64 b, {y, %4};\n\t"
+        "@e tcgen05.mma.cta_group::1.kind::f8f6f4 [%0], a, b, %3, 1;\n\t"
+        "add.u32 x, %1, 4;\n\tadd.u32 y, %2, %6;\n\tmov.b64 a, {x, %4};\n\tmov.b64 b, {y, %4};\n\t"
+        "@e tcgen05.mma.cta_group::1.kind::f8f6f4 [%0], a, b, %3, 1;\n\t"
+        "add.u32 x, %1, 6;\n\tadd.u32 y, %2, %7;\n\tmov.b64 a, {x, %4};\n\tmov.b64 b, {y, %4};\n\t"
+        "@e tcgen05.mma.cta_group::1.kind::f8f6f4 [%0], a, b, %3, 1;\n\t}"
+        ::"r"(d_tmem), "r"(a_lo), "r"(b_lo), "r"(idesc), "r"(hi), "n"(STEP_B), "n"(2 * STEP_B), "n"(3 * STEP_B) : "memory");
+}
+
 // kind::f16 instruction descriptor: fp32 accumulate, A and B of the same 16-bit type; *_mn: that operand is MN-major
 __host__ __device__ constexpr uint32_t make_idesc_f16(bool bf16, int m, int n, bool a_mn = false, bool b_mn = false) {
     return (1u << 4)                                   // D format: fp32

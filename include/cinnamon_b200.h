@@ -96,6 +96,16 @@ int cinn_quant_rowwise_with_block_t(const void* x, int x_dtype, int64_t M, int64
 int cinn_quant_rowwise_with_block_t_padded(const void* x, int x_dtype, int64_t M, int64_t N, int64_t ld, void* q_row, float* s_row,
                                            void* q_block_t, float* s_block, int round_scale, int div_mode, void* stream);
 
+/* A linear without gradients on up to 128 rows in one kernel: x (M, K) quantised row-wise (cinn_quant_rowwise) times the fp32
+ * weight w (N, K) quantised in 128 x 128 blocks (cinn_quant_blockwise), scales as in cinn_fp8_gemm, out (M, N) bf16, contiguous.
+ * Replaces the forward of FP8MatmulFunction (src/kernels.py:746-752) where nothing is kept for a backward.
+ * cinn_fp8_linear_few_takes: whether it can take these operands and pays (1) or not (0).  K a multiple of 16, rows of x and w contiguous
+ * with 16-byte pitches, pointers 16-byte aligned; anything else is refused. */
+int cinn_fp8_linear_few_takes(const void* x, int x_dtype, int64_t ldx_m, int64_t ldx_k, const void* w, int w_dtype, int64_t ldw_n,
+                              int64_t ldw_k, int64_t M, int64_t N, int64_t K);
+int cinn_fp8_linear_few(const void* x, int x_dtype, int64_t ldx, int round_scale, const float* w, int64_t ldw, void* out, int64_t M,
+                        int64_t N, int64_t K, int div_mode, void* stream);
+
 /* Block-wise block_m x block_n quantisation.
  * Replaces quantize_fp8_blockwise_kernel + quantize_fp8_blockwise (src/kernels.py:74-132, 219-259).
  * scales: (ceil(M/block_m), ceil(N/block_n)). */

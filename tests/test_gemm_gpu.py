@@ -813,3 +813,56 @@ def test_zero_rows_outside_ranges(K):
     dx = K.fp8_grouped_gemm_dgrad(dq, dsc, wq, wsc, starts, ends)
     assert torch.count_nonzero(dx[:10]) == 0 and torch.count_nonzero(dx[200:300]) == 0 and torch.count_nonzero(dx[650:]) == 0
     assert torch.count_nonzero(dx[10:200]) > 0 and torch.isfinite(dx.float()).all()
+
+
+@pytest.mark.parametrize("M,N,Kd", [(1, 128, 128), (1, 4, 16), (33, 200, 144), (97, 1000, 1040), (128, 1024, 512), (64, 130, 2048),
+                                    (128, 8320, 256), (5, 19072, 384), (31, 8192, 1152)])
+@pytest.mark.parametrize("dtype,rs,div", [(torch.bfloat16, False, "full"), (torch.float32, True, "full"), (torch.float16, False, "rn")])
+def test_linear_on_few_rows_in_one_kernel(K, M, N, Kd, dtype, rs, div):
+    """Quantising and multiplying in one kernel (one to eight CTAs per column tile) against the product of what the quantisers give,
+    in 64 bits: fp32 sums over K blocks (2^-23 per addition of partial products) and one rounding to bf16."""
+    g = torch.Generator(device="cuda").manual_seed(M + N + Kd)
+    x = torch.randn(M, Kd, device="cuda", generator=g).mul_(3).to(dtype)
+    w = torch.randn(N, Kd, device="cuda", generator=g).mul_(0.02)
+    mode = K.get_div_mode()
+    K.set_div_mode(div)
+    try:
+        out = torch.empty(M, N, device="cuda", dtype=torch.bfloat16)
+        assert K._L.cinn_fp8_linear_few(K._ptr(x), K._DTYPE_TAG[dtype], Kd, int(rs), K._ptr(w), Kd, K._ptr(out), M, N, Kd, K._DIV_MODE, K._stream(x)) == 0
+        xq, xs = K.quantize_fp8_rowwise(x, 128, rs)
+        wq, ws = K.quantize_fp8_blockwise(w)
+        whole = K._gemm(xq, xs, wq, 0, ws, ws.stride(1), ws.stride(0), M, N, Kd, torch.bfloat16, whole=True)
+    finally:
+        K.set_div_mode(mode)
+    a = xq.double() * xs.double().repeat_interleave(128, 1)[:, :Kd]
+    b = wq.double() * ws.double().repeat_interleave(128, 0)[:N].repeat_interleave(128, 1)[:, :Kd]
+    ref, size = a @ b.t(), a.abs() @ b.abs().t()
+    assert bool(((out.double() - ref).abs() <= ref.abs() * 2.0 ** -8 + size * (Kd + 64) * 2.0 ** -23).all())
+    if N > 16384 or Kd <= 128:                          # one CTA per column tile: the sums of the separate kernels, in their order
+        assert torch.equal(out, whole)
+    else:
+        assert float((out.double() - whole.double()).norm() / whole.double().norm()) < 2.0 ** -9
+
+
+def test_linear_on_few_rows_any_alignment(K):
+    """One launch for rows that fit, two for those that do not (rows off 16-byte boundaries, strides, a reduction too long for it to
+    pay); the same result."""
+    g = torch.Generator(device="cuda").manual_seed(5)
+    lin = K.FP8Linear(272, 384).cuda()
+    x = torch.randn(20, 272, device="cuda", generator=g, dtype=torch.float32).to(torch.bfloat16)
+    with torch.no_grad():
+        n = K.launch_count
+        ref = lin(x)
+        assert K.launch_count - n == 1
+        odd = torch.empty(20 * 272 + 3, device="cuda", dtype=torch.bfloat16)[3:].view(20, 272).copy_(x)
+        wide = torch.empty(20, 300, device="cuda", dtype=torch.bfloat16)[:, 4:276].copy_(x)
+        turned = x.t().contiguous().t()
+        for other, few in ((odd, 2), (wide, 2), (turned, 2), (x.view(4, 5, 272), 1)):
+            n = K.launch_count
+            y = lin(other).reshape(20, 384)
+            assert K.launch_count - n >= 2 if few == 2 else K.launch_count - n == 1
+            assert float((y.double() - ref.double()).norm() / ref.double().norm()) < 2.0 ** -9
+        long = K.FP8Linear(7168, 2048).cuda()
+        n = K.launch_count
+        long(torch.randn(4, 7168, device="cuda"))
+        assert K.launch_count - n >= 2
