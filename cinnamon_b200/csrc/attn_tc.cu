@@ -1302,11 +1302,12 @@ static Plan make_plan(int64_t B, int64_t H, int64_t L, int64_t K, int64_t Dqk, i
 }
 
 // Whether the dense tiles are worth it: their time (the causal half of the tiles is visited, a constant number of cycles
-// each that grows with the widths) against the gathers' (K rows of Dqk + Dv elements per query).  The constants are fitted
-// to measurements over L = 500 ... 4096, K = 32 ... 128, widths 64 ... 192, the forward's with a forward that took a quarter longer in bf16.
-// The forward's calls as they are now, gathers against tiles, at 2 x 8 x 4096 queries of 192: in bf16 131 and 207 us for K = 16, 207 and 205
-// for 32, 369 and 203 for 64; in fp32 240 and 457 for 32, 424 and 455 for 64, 774 and 461 for 128; at 1 x 8 x 2048 of 64 in bf16 49 and 66 for
-// 32, 80 and 66 for 64.
+// each that grows with the widths, and every query tile costs its start and its probabilities; what was picked and the parts come
+// first) against the gathers' (K rows of Dqk + Dv elements per query and a constant per row).  The constants are fitted to 70 calls of each, forward and
+// backward, over B = 1 ... 32, L = 257 ... 4062, K = 32 ... 256, widths 64 ... 192, bf16 and fp32: 9 to 16 % off on average, and the way that
+// is taken costs 0.3 (forward) and 0.7 % (backward) more than the faster one would.  With the constants of a forward that was slower in
+// bf16 and of fewer lengths it was 4.5 and 3 %: gathers against tiles, 16 x 4 x 2286 queries, 64 picks of 64 / 128 in bf16 838 and 403 us
+// (it took the gathers), 4 x 8 x 3965, 64 of 192 / 128 861 and 581, 1 x 4 x 1105 in fp32 backward 72 and 199 (it took the tiles).
 static std::atomic<int> g_mode{-1};         // -1: by the estimate; 0 / 1: never / wherever the tiles can (tests, measurements)
 int set_mode(int mode) { return g_mode.exchange(mode); }
 
@@ -1318,15 +1319,17 @@ static bool dense_pays(const Plan& p, bool backward) {
     const double queries = (double)p.BH * p.L, row = (double)(p.Dqk + p.Dv), widths = p.dp + 64.0 * p.nv;
     const double gathered = queries * p.K * row * (wide ? 4 : 2), split = parts ? queries * (row + p.Dqk) * (wide ? 10 : 8) / 6.2e6 : 0.0;
     const double picks = 15.0 + 5.5e-6 * p.B * p.L * p.K;
-    double cycles, gather_us;
+    double cycles, tiles_us, gather_us;
     if (!backward) {
-        cycles = tiles * p.nv * (parts ? 8800.0 + 48.0 * p.dp : 7500.0 + 8.0 * p.dp) + q_tiles * p.nv * (6000.0 + 100.0 * p.K);
-        gather_us = 8.0 + gathered / (wide ? 9.5e6 : 5.3e6);
+        cycles = p.nv * (parts ? tiles * (2800.0 + 43.0 * p.dp) + q_tiles * (11100.0 + 68.0 * p.K) : tiles * (3600.0 + 3.4 * p.dp) + q_tiles * (3000.0 + 84.0 * p.K));
+        tiles_us = picks * (parts ? 2.3 : 2.15) + split;
+        gather_us = wide ? 9.0 + gathered / 15.3e6 + queries * p.K / 39e3 : 21.0 + gathered / 11.2e6 + queries * p.K / 26e3;
     } else {
-        cycles = tiles * (parts ? 27000.0 + 130.0 * widths : 12000.0 + 55.0 * widths) + q_tiles * 20000.0;
-        gather_us = 30.0 + gathered / (wide ? 3.7e6 : 2.0e6);
+        cycles = parts ? tiles * (3300.0 + 170.0 * widths) + q_tiles * (10000.0 + 937.0 * p.K) : tiles * (8800.0 + 41.6 * widths) + q_tiles * (13100.0 + 363.0 * p.K);
+        tiles_us = parts ? picks * 1.3 + 75.0 + split : picks * 3.75;
+        gather_us = wide ? 27.0 + gathered / 4.46e6 + queries * p.K / 71e3 : 60.0 + gathered / 2.79e6 + queries * p.K / 28.5e3;
     }
-    return (picks + split + (backward ? 20.0 : 0.0) + cycles / (148.0 * 1900.0)) < 0.9 * gather_us;
+    return tiles_us + cycles / (148.0 * 1900.0) < 0.95 * gather_us;
 }
 
 static bool supported(int64_t B, int64_t H, int64_t L, int64_t K, int64_t Dqk, int64_t Dv) {
