@@ -86,6 +86,14 @@ SIGNATURES = {
     "cinn_fp8_grouped_wgrad_scratch_bytes": [_i64, _i64, _i64],
     "cinn_fp8_grouped_wgrad_fused_scratch_bytes": [_i64, _i64, _i64, _i64],
     "cinn_fp8_grouped_wgrad_fused": [_vp, _i32, _vp, _vp, _vp, _vp, _i64, _i64, _i64, _i64, _vp, _i64, _vp, _i32, _i32, _vp, _vp, _vp],
+    "cinn_quant_segments_bytes": [_i64, _i64, _i64],
+    "cinn_quant_rowwise_segments": [_vp, _i32, _i64, _i64, _vp, _vp, _i64, _vp, _vp, _vp, _i64, _i32, _vp],
+    "cinn_fp8_grouped_wgrad_segments_scratch_bytes": [_i64, _i64, _i64],
+    "cinn_swiglu_rounded_quant_block_t": [_vp, _i32, _i64, _i64, _vp, _vp, _vp, _vp, _i32, _vp],
+    "cinn_swiglu_rounded_backward_quant_dual": [_vp, _vp, _i32, _i64, _i64, _vp, _vp, _vp, _vp, _i32, _vp],
+    "cinn_swiglu_quant_segments": [_vp, _i32, _i64, _i64, _vp, _vp, _i64, _vp, _vp, _vp, _i64, _vp],
+    "cinn_fp8_grouped_wgrad_swiglu": [_vp, _vp, _i32, _vp, _vp, _vp, _vp, _i64, _i64, _i64, _i64, _vp, _i64, _vp, _i32, _vp, _vp, _vp],
+    "cinn_fp8_grouped_wgrad_segments": [_vp, _i32, _vp, _i64, _i64, _i64, _i64, _vp, _i64, _vp, _i32, _i32, _vp, _vp, _vp],
     "cinn_fp8_grouped_wgrad": [_vp, _i32, _vp, _vp, _vp, _vp, _i64, _i64, _i64, _i64, _vp, _i64, _vp, _i32, _i32, _vp],
     "cinn_swiglu": [_vp, _vp, _i32, _i64, _i64, _vp],
     "cinn_swiglu_backward": [_vp, _vp, _vp, _i32, _i64, _i64, _vp],
@@ -115,7 +123,8 @@ def _load() -> ctypes.CDLL:
                       else ctypes.c_longlong if name == "cinn_set_wait_limit_cycles"
                       else ctypes.c_int64 if name in ("cinn_moe_route_workspace_ints", "cinn_moe_route_static_max_ints", "cinn_fp8_gemm_workspace_bytes", "cinn_moe_balance_workspace_bytes",
                                                  "cinn_sparse_attn_workspace_bytes", "cinn_launch_count",
-                                                 "cinn_fp8_grouped_wgrad_scratch_bytes", "cinn_fp8_grouped_wgrad_fused_scratch_bytes")
+                                                 "cinn_fp8_grouped_wgrad_scratch_bytes", "cinn_fp8_grouped_wgrad_fused_scratch_bytes",
+                                                 "cinn_quant_segments_bytes", "cinn_fp8_grouped_wgrad_segments_scratch_bytes")
                       else ctypes.c_int)
     return lib
 

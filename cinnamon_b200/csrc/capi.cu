@@ -96,7 +96,7 @@ int64_t grouped_wgrad_fused_scratch_bytes(int64_t T, int64_t E, int64_t d_in, in
 int fp8_grouped_wgrad_fused(const void* dY, int dy_dtype, const void* x_q, const float* x_s, const int64_t* starts_dev,
                             const int64_t* ends_dev, int64_t E, int64_t T, int64_t d_in, int64_t d_out, void* scratch,
                             int64_t scratch_bytes, void* dW, int out_dtype, int div_mode, void* dy_q_row, float* dy_s_row,
-                            cudaStream_t st);
+                            const void* h12, cudaStream_t st);
 int grouped_gemm_16bit(const void* A, const void* W, int in_dtype, const int64_t* starts, const int64_t* ends, int64_t E,
                        int64_t T, int64_t d_in, int64_t d_out, void* C, int out_dtype, cudaStream_t st);
 int zero_rows_outside(void* buf, int64_t T, int64_t row_bytes, const int64_t* starts, const int64_t* ends, int64_t E,
@@ -114,6 +114,18 @@ int p2p_dispatch_signal(const void* q, const float* s, const int64_t* token_indi
 int p2p_row_table_wait(const int64_t* seg_start, const int64_t* home_base, const int64_t* peer_home, int64_t n_rows,
                        int64_t row_bytes, int n_segments, int n_ranks, int64_t capacity, long long* row_dst,
                        const int64_t* peer_flags, int me, int flag_slot, unsigned epoch, cudaStream_t st);
+int64_t quant_segments_bytes(int64_t T, int64_t E, int64_t d);
+int quantize_row_segments(const void* x, int dtype, int64_t T, int64_t d, const int64_t* starts_dev, const int64_t* ends_dev, int64_t E,
+                          void* q_row, float* s_row, void* segments, int64_t segments_bytes, int div_mode, bool swiglu, cudaStream_t st);
+struct SegmentTiles;
+int swiglu_quant_block(const void* h12, int dtype, int64_t T, int64_t I, void* q_row, float* s_row, void* q_blk, float* s_blk, int round_scale,
+                       const SegmentTiles* seg, cudaStream_t st);
+int swiglu_backward_quant_dual(const void* h12, const void* dh, int dtype, int64_t T, int64_t I, void* q_row, float* s_row, void* q_col,
+                               float* s_col, int round_scale, const SegmentTiles* seg, cudaStream_t st);
+int64_t grouped_wgrad_segments_scratch_bytes(int64_t T, int64_t E, int64_t d_out);
+int fp8_grouped_wgrad_segments(const void* dY, int dy_dtype, const void* segments, int64_t E, int64_t T, int64_t d_in, int64_t d_out,
+                               void* scratch, int64_t scratch_bytes, void* dW, int out_dtype, int div_mode, void* dy_q_row, float* dy_s_row,
+                               cudaStream_t st);
 int64_t grouped_wgrad_scratch_bytes(int64_t max_rows, int64_t d_in, int64_t d_out);
 int fp8_grouped_wgrad(const void* dY, int dy_dtype, const void* x_q, const float* x_s, const int64_t* starts_host,
                       const int64_t* ends_host, int64_t E, int64_t T, int64_t d_in, int64_t d_out, void* scratch,
@@ -438,6 +450,24 @@ int cinn_p2p_barrier(const int64_t* peer_flags, int rank, int n_ranks, unsigned 
 
 long long cinn_set_wait_limit_cycles(long long cycles) { return cinn::set_p2p_wait_limit(cycles); }
 
+int64_t cinn_quant_segments_bytes(int64_t T, int64_t E, int64_t d) { return cinn::quant_segments_bytes(T, E, d); }
+
+int cinn_quant_rowwise_segments(const void* x, int x_dtype, int64_t T, int64_t d, const int64_t* starts, const int64_t* ends, int64_t E,
+                                void* q_row, float* s_row, void* segments, int64_t segments_bytes, int div_mode, void* stream) {
+    return cinn::quantize_row_segments(x, x_dtype, T, d, starts, ends, E, q_row, s_row, segments, segments_bytes, div_mode, false, (cudaStream_t)stream);
+}
+
+int64_t cinn_fp8_grouped_wgrad_segments_scratch_bytes(int64_t T, int64_t E, int64_t d_out) {
+    return cinn::grouped_wgrad_segments_scratch_bytes(T, E, d_out);
+}
+
+int cinn_fp8_grouped_wgrad_segments(const void* dY, int dy_dtype, const void* segments, int64_t E, int64_t T, int64_t d_in, int64_t d_out,
+                                    void* scratch, int64_t scratch_bytes, void* dW, int out_dtype, int div_mode, void* dy_q_row,
+                                    float* dy_s_row, void* stream) {
+    return cinn::fp8_grouped_wgrad_segments(dY, dy_dtype, segments, E, T, d_in, d_out, scratch, scratch_bytes, dW, out_dtype, div_mode, dy_q_row,
+                                            dy_s_row, (cudaStream_t)stream);
+}
+
 int64_t cinn_fp8_grouped_wgrad_fused_scratch_bytes(int64_t total_rows, int64_t n_experts, int64_t d_in, int64_t d_out) {
     return cinn::grouped_wgrad_fused_scratch_bytes(total_rows, n_experts, d_in, d_out);
 }
@@ -448,7 +478,32 @@ int cinn_fp8_grouped_wgrad_fused(const void* dY, int dy_dtype, const void* x_q, 
                                  float* dy_row_scales, void* stream) {
     return cinn::fp8_grouped_wgrad_fused(dY, dy_dtype, x_q, x_scales, expert_starts, expert_ends, n_experts, total_rows, d_in, d_out,
                                          scratch, scratch_bytes, dW, out_dtype, div_mode, dy_q_row, dy_row_scales,
-                                         (cudaStream_t)stream);
+                                         nullptr, (cudaStream_t)stream);
+}
+
+int cinn_fp8_grouped_wgrad_swiglu(const void* h12, const void* dh, int dtype, const void* x_q, const float* x_scales,
+                                  const int64_t* expert_starts, const int64_t* expert_ends, int64_t n_experts, int64_t total_rows, int64_t d_in,
+                                  int64_t I, void* scratch, int64_t scratch_bytes, void* dW, int out_dtype, void* q_row, float* row_scales,
+                                  void* stream) {
+    if (h12 == nullptr) { cinn::set_error("grouped_wgrad_swiglu: null pointer"); return CINN_ERR_INVALID; }
+    return cinn::fp8_grouped_wgrad_fused(dh, dtype, x_q, x_scales, expert_starts, expert_ends, n_experts, total_rows, d_in, 2 * I, scratch,
+                                         scratch_bytes, dW, out_dtype, CINN_DIV_FULL, q_row, row_scales, h12, (cudaStream_t)stream);
+}
+
+int cinn_swiglu_quant_segments(const void* h12, int dtype, int64_t T, int64_t I, const int64_t* starts, const int64_t* ends, int64_t E,
+                               void* q_row, float* s_row, void* segments, int64_t segments_bytes, void* stream) {
+    return cinn::quantize_row_segments(h12, dtype, T, I, starts, ends, E, q_row, s_row, segments, segments_bytes, CINN_DIV_FULL, true,
+                                       (cudaStream_t)stream);
+}
+
+int cinn_swiglu_rounded_quant_block_t(const void* h12, int dtype, int64_t T, int64_t I, void* q_row, float* s_row, void* q_block_t,
+                                      float* s_block, int round_scale, void* stream) {
+    return cinn::swiglu_quant_block(h12, dtype, T, I, q_row, s_row, q_block_t, s_block, round_scale, nullptr, (cudaStream_t)stream);
+}
+
+int cinn_swiglu_rounded_backward_quant_dual(const void* h12, const void* dh, int dtype, int64_t T, int64_t I, void* q_row, float* s_row,
+                                            void* q_col, float* s_col, int round_scale, void* stream) {
+    return cinn::swiglu_backward_quant_dual(h12, dh, dtype, T, I, q_row, s_row, q_col, s_col, round_scale, nullptr, (cudaStream_t)stream);
 }
 
 int cinn_grouped_gemm_16bit(const void* A, const void* W, int in_dtype, const int64_t* expert_starts, const int64_t* expert_ends,

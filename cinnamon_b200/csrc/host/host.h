@@ -30,7 +30,9 @@ using at::Tensor;
     X(cinn_swiglu_quant_rowwise) X(cinn_moe_combine) X(cinn_moe_combine_add) X(cinn_moe_sum_add)                \
     X(cinn_swiglu_rounded) X(cinn_swiglu_rounded_backward) X(cinn_moe_balance_workspace_bytes) X(cinn_moe_balance_loss)     \
     X(cinn_moe_gates_backward) X(cinn_moe_update_bias) X(cinn_moe_combine_backward) X(cinn_swiglu_backward)                 \
-    X(cinn_fp8_grouped_wgrad_fused_scratch_bytes) X(cinn_fp8_grouped_wgrad_fused) X(cinn_fp8_grouped_gemm_dgrad) X(cinn_zero_rows_outside)
+    X(cinn_fp8_grouped_wgrad_fused_scratch_bytes) X(cinn_fp8_grouped_wgrad_fused) X(cinn_quant_segments_bytes) X(cinn_quant_rowwise_segments)             \
+    X(cinn_fp8_grouped_wgrad_segments_scratch_bytes) X(cinn_fp8_grouped_wgrad_segments)                          \
+    X(cinn_swiglu_rounded_quant_block_t) X(cinn_swiglu_rounded_backward_quant_dual) X(cinn_swiglu_quant_segments) X(cinn_fp8_grouped_wgrad_swiglu) X(cinn_fp8_grouped_gemm_dgrad) X(cinn_zero_rows_outside)
 
 struct Api {
 #define CINN_DECL(name) decltype(&::name) name = nullptr;
@@ -103,6 +105,7 @@ inline float* f32(const Tensor& t);
 Tensor gemm(const Tensor& a, const Tensor& sa, const Tensor& b, int layout, const Tensor& sb, int64_t sbk, int64_t sbn, int64_t M,
             int64_t N, int64_t K, at::ScalarType type, int tag);               // linear.cpp
 
+struct Quantised { Tensor q, s; };
 struct Linear {                                 // what an FP8 linear's forward leaves for its backward
     Tensor out, x, x_scale, w, w_scale, w_t;
     bool x_is_block = false, x_is_block_t = false;
@@ -120,8 +123,13 @@ std::tuple<std::vector<Tensor>, Tensor> linear_backward(const Tensor& grad_out, 
                                                         bool round_scale, bool x_is_block, bool x_is_block_t,
                                                         at::ScalarType weight_dtype, bool kmajor, int div, bool want_gx,
                                                         bool want_gw, at::ScalarType gx_type, int parts = 1);
+// the rest of it once the output gradient is quantised
+std::tuple<std::vector<Tensor>, Tensor> linear_backward_quantised(const Quantised& g, const Quantised& g_t, int64_t M, Tensor x, Tensor x_scale,
+                                                                  const Tensor& w, const Tensor& w_scale, const Tensor& w_t,
+                                                                  at::IntArrayRef x_shape, bool x_is_block, bool x_is_block_t,
+                                                                  at::ScalarType weight_dtype, bool kmajor, int div, bool want_gx,
+                                                                  bool want_gw, at::ScalarType gx_type, int parts);
 
-struct Quantised { Tensor q, s; };
 Quantised rowwise(const Tensor& x, bool round_scale, int div);                 // moe.cpp
 Quantised swiglu_quantised(const Tensor& h12, int div);
 Tensor grouped(const Quantised& x, const Quantised& w, const Tensor& starts, const Tensor& ends, at::ScalarType type = at::kBFloat16);

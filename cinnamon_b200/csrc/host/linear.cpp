@@ -62,13 +62,27 @@ Linear linear_forward(const Tensor& x, const Tensor& weight, bool round_scale, b
         r.x = xq;
         r.x_scale = xs;
     }
+    linear_multiply(r, xq, xs, wf, need_dgrad, kmajor, div, w_q, w_s, w_qt);
+    if (x.dim() != 2) {
+        auto shape = x.sizes().vec();
+        shape.back() = N;
+        r.out = r.out.view(shape);
+    }
+    return r;
+}
+
+// wf: the weight in a type the quantiser reads (undefined with w_q)
+void linear_multiply(Linear& r, const Tensor& xq, const Tensor& xs, const Tensor& wf, bool need_dgrad, bool kmajor, int div, const Tensor& w_q,
+                     const Tensor& w_s, const Tensor& w_qt) {
+    const at::Device dev = xq.device();
+    const int64_t M = xq.size(0), K = xq.size(1), N = (w_q.defined() ? w_q : wf).size(0);
     if (w_q.defined()) {
         r.w = w_q;
         r.w_scale = w_s;
         r.w_t = w_qt;
     } else {
         r.w = empty({N, K}, F8, dev);
-        r.w_scale = empty({up(N, 128), nkb}, at::kFloat, dev);
+        r.w_scale = empty({up(N, 128), up(K, 128)}, at::kFloat, dev);
         // the input gradient multiplies by the weight with N as the reduction axis: the byte-transposed copy it reads
         // comes out of the same pass
         if (kmajor && need_dgrad && N % 16 == 0 && K % 4 == 0 && wf.stride(1) == 1 && wf.stride(0) % 4 == 0) {
@@ -80,12 +94,6 @@ Linear linear_forward(const Tensor& x, const Tensor& weight, bool round_scale, b
               "cinn_quant_blockwise");
     }
     r.out = gemm(xq, xs, r.w, 0, r.w_scale, r.w_scale.stride(1), r.w_scale.stride(0), M, N, K, at::kBFloat16, TAG_BF16);
-    if (x.dim() != 2) {
-        auto shape = x.sizes().vec();
-        shape.back() = N;
-        r.out = r.out.view(shape);
-    }
-    return r;
 }
 
 std::tuple<std::vector<Tensor>, Tensor> linear_backward(const Tensor& grad_out, Tensor x, Tensor x_scale, const Tensor& w,
@@ -95,7 +103,7 @@ std::tuple<std::vector<Tensor>, Tensor> linear_backward(const Tensor& grad_out, 
                                                         bool want_gw, at::ScalarType gx_type, int parts) {
     c10::cuda::CUDAGuard guard(w.device());
     const at::Device dev = w.device();
-    const int64_t N = w.size(0), K = w.size(1);
+    const int64_t N = w.size(0);
     Tensor g = readable(grad_out.dim() == 2 ? grad_out : grad_out.reshape({-1, grad_out.size(-1)}));
     if (g.stride(1) != 1) g = g.contiguous();
     int64_t M = g.size(0);
@@ -119,6 +127,19 @@ std::tuple<std::vector<Tensor>, Tensor> linear_backward(const Tensor& grad_out, 
     check((rows == Mp ? api.cinn_quant_rowwise_dual : api.cinn_quant_rowwise_dual_padded)(
               g.data_ptr(), tag_of(g.scalar_type()), rows, N, g.stride(0), gq.data_ptr(), f32(gs), gqt.data_ptr(), f32(gst), round_scale, div,
               stream()), "cinn_quant_rowwise_dual");
+    return linear_backward_quantised({gq, gs}, {gqt, gst}, M, x, x_scale, w, w_scale, w_t, x_shape, x_is_block, x_is_block_t, weight_dtype, kmajor,
+                                     div, want_gx, want_gw, gx_type, parts);
+}
+
+// g: the output gradient quantised along its features (M rows at least), g_t: along the tokens, (N, M rounded up to 16)
+std::tuple<std::vector<Tensor>, Tensor> linear_backward_quantised(const Quantised& g, const Quantised& g_t, int64_t M, Tensor x, Tensor x_scale,
+                                                                  const Tensor& w, const Tensor& w_scale, const Tensor& w_t,
+                                                                  at::IntArrayRef x_shape, bool x_is_block, bool x_is_block_t,
+                                                                  at::ScalarType weight_dtype, bool kmajor, int div, bool want_gx,
+                                                                  bool want_gw, at::ScalarType gx_type, int parts) {
+    const at::Device dev = w.device();
+    const int64_t N = w.size(0), K = w.size(1), Mp = g_t.q.size(1);
+    const Tensor &gq = g.q, &gs = g.s, &gqt = g_t.q, &gst = g_t.s;
     // (the reference's input gradient is bf16 and autograd casts it to the input's type: fp32 holds those values)
     const int gx_tag = gx_type == at::kFloat ? TAG_F32_BF16 : TAG_BF16;
     std::vector<Tensor> gx(parts);

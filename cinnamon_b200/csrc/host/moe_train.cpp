@@ -28,6 +28,29 @@ Tensor swiglu_rounded(const Tensor& h12) {
     return h;
 }
 
+// Whether SwiGLU can be part of the quantisers next to it
+bool swiglu_in_quantisers(const Tensor& h12, bool kmajor, int div) {
+    const int64_t T = h12.size(0), I = h12.size(1) / 2;
+    return kmajor && div == CINN_DIV_FULL && h12.element_size() == 2 && tag_of(h12.scalar_type()) >= 0 && T >= 1 && T <= MAX_PADDED_ROWS &&
+           I >= 128 && I % 128 == 0 && (reinterpret_cast<uintptr_t>(h12.data_ptr()) & 15) == 0;
+}
+
+// linear_forward(swiglu_rounded(h12), w, ...) of a weight that wants its gradient
+Linear swiglu_linear_forward(const Tensor& h12, const Tensor& w, bool round_scale, bool need_dgrad, int div) {
+    const at::Device dev = h12.device();
+    const int64_t T = h12.size(0), I = h12.size(1) / 2;
+    const Tensor wf = readable(w);
+    Linear r;
+    r.x_is_block = r.x_is_block_t = true;
+    r.x = empty({I, up(T, 16) * 16}, F8, dev);
+    r.x_scale = empty({up(T, 128), I / 128}, at::kFloat, dev);
+    const Tensor xq = empty({T, I}, F8, dev), xs = empty({T, I / 128}, at::kFloat, dev);
+    check(api.cinn_swiglu_rounded_quant_block_t(h12.data_ptr(), tag_of(h12.scalar_type()), T, I, xq.data_ptr(), f32(xs), r.x.data_ptr(),
+                                                f32(r.x_scale), round_scale, stream()), "cinn_swiglu_rounded_quant_block_t");
+    linear_multiply(r, xq, xs, wf, need_dgrad, true, div, Tensor(), Tensor(), Tensor());
+    return r;
+}
+
 // x comes in twice, once for w2 and once for w1: each of the two layers returns an input gradient of its own, rounded to bf16
 // as the layer by itself rounds it, and autograd adds them up in the order in which it would for two layers.  (One product over
 // [dh1 dh2] [w1; w2] rounds once and is 20 us faster at 32768 tokens, but then the block's gradient depends on whether a
@@ -39,7 +62,9 @@ struct SwiGLUNode : public torch::autograd::Function<SwiGLUNode> {
         const bool gx = x.requires_grad(), g12 = w1.requires_grad() || w2.requires_grad(), g3 = w3.requires_grad(), any = gx || g12;
         const Linear a = linear_forward(x, at::cat({w1, w2}), o->round12, gx, g12, o->kmajor, o->div, Tensor(), Tensor(), Tensor());
         const Tensor h12 = a.out.view({-1, a.out.size(-1)});
-        const Linear b = linear_forward(swiglu_rounded(h12), w3, o->round3, any, g3, o->kmajor, o->div, Tensor(), Tensor(), Tensor());
+        const Linear b = g3 && swiglu_in_quantisers(h12, o->kmajor, o->div)
+            ? swiglu_linear_forward(h12, w3, o->round3, any, o->div)
+            : linear_forward(swiglu_rounded(h12), w3, o->round3, any, g3, o->kmajor, o->div, Tensor(), Tensor(), Tensor());
         ctx->set_materialize_grads(false);
         if (any || g3) {
             ctx->save_for_backward({a.x, a.x_scale, a.w, a.w_scale, a.w_t, h12, b.x, b.x_scale, b.w, b.w_scale, b.w_t});
@@ -72,19 +97,34 @@ struct SwiGLUNode : public torch::autograd::Function<SwiGLUNode> {
             };
             const Tensor& h12 = s[5];
             const int64_t T = h12.size(0), I = h12.size(1) / 2;
-            std::tie(dh, d3) = back(ctx->saved_data["b"].toInt(), grads[0], 6, {T, I}, gx || g12, g3, at::kBFloat16, 1);
-            if (!(gx || g12)) return;
-            c10::cuda::CUDAGuard guard(h12.device());
-            Tensor dh12 = empty({T, 2 * I}, h12.scalar_type(), h12.device()), d12;
-            check(api.cinn_swiglu_rounded_backward(h12.data_ptr(), dh[0].data_ptr(), dh12.data_ptr(), tag_of(h12.scalar_type()), T, I, stream()),
-                  "cinn_swiglu_backward");
-            std::tie(dx, d12) = back(ctx->saved_data["a"].toInt(), dh12, 0, ctx->saved_data["x_shape"].toIntVector(), gx, g12,
-                                     ctx->saved_data["x32"].toBool() ? at::kFloat : at::kBFloat16, 2);
-            if (g12) {
+            auto split = [&](const Tensor& d12) {
+                if (!g12) return;
                 const auto halves = at::unsafe_split(d12, I, 0);
                 d1 = halves[0];
                 d2 = halves[1];
+            };
+            std::tie(dh, d3) = back(ctx->saved_data["b"].toInt(), grads[0], 6, {T, I}, gx || g12, g3, at::kBFloat16, 1);
+            if (!(gx || g12)) return;
+            c10::cuda::CUDAGuard guard(h12.device());
+            const int64_t f = ctx->saved_data["a"].toInt();
+            const auto x_type = ctx->saved_data["x32"].toBool() ? at::kFloat : at::kBFloat16;
+            Tensor d12;
+            if (swiglu_in_quantisers(h12, f & 8, (int)(f >> 4 & 15)) && (!g12 || f & 4)) {
+                const Quantised g{empty({T, 2 * I}, F8, h12.device()), empty({T, 2 * I / 128}, at::kFloat, h12.device())};
+                const Quantised g_t{empty({2 * I, up(T, 16) * 16}, F8, h12.device()), empty({2 * I, up(T, 128)}, at::kFloat, h12.device())};
+                check(api.cinn_swiglu_rounded_backward_quant_dual(h12.data_ptr(), dh[0].data_ptr(), tag_of(h12.scalar_type()), T, I, g.q.data_ptr(),
+                                                                  f32(g.s), g_t.q.data_ptr(), f32(g_t.s), f & 1, stream()),
+                      "cinn_swiglu_rounded_backward_quant_dual");
+                std::tie(dx, d12) = linear_backward_quantised(g, g_t, T, s[0], s[1], s[2], s[3], s[4], ctx->saved_data["x_shape"].toIntVector(), f & 2,
+                                                              f & 4, (at::ScalarType)(f >> 8 & 255), f & 8, (int)(f >> 4 & 15), gx, g12, x_type, 2);
+                split(d12);
+                return;
             }
+            Tensor dh12 = empty({T, 2 * I}, h12.scalar_type(), h12.device());
+            check(api.cinn_swiglu_rounded_backward(h12.data_ptr(), dh[0].data_ptr(), dh12.data_ptr(), tag_of(h12.scalar_type()), T, I, stream()),
+                  "cinn_swiglu_backward");
+            std::tie(dx, d12) = back(f, dh12, 0, ctx->saved_data["x_shape"].toIntVector(), gx, g12, x_type, 2);
+            split(d12);
         });
         return {dx[1], dx[0], d1, d2, d3, Tensor()};
     }
@@ -103,20 +143,34 @@ struct BlockOptions {
     Tensor counts;                             // out: rows per expert
 };
 
-// gradients of grouped(x, w) given dy; `covered`: the experts' ranges cover every row (else the others' gradients are zero)
+// gradients of grouped(x, w) given dy; `covered`: the experts' ranges cover every row (else the others' gradients are zero).
+// xs undefined: xq holds the segments that the forward's quantiser left.  h12: dy is the gradient of SwiGLU's result, not of the product
 std::tuple<Tensor, Tensor> grouped_backward(const Tensor& dy, const Tensor& xq, const Tensor& xs, const Tensor& wq, const Tensor& ws,
                                             const Tensor& starts, const Tensor& ends, at::ScalarType w_type, bool want_x,
-                                            at::ScalarType x_type, int div, bool covered = true) {
+                                            at::ScalarType x_type, int div, bool covered = true, const Tensor& h12 = Tensor()) {
     const int64_t R = dy.size(0), E = wq.size(0), d_out = wq.size(1), d_in = wq.size(2);
     const at::Device dev = dy.device();
     const int64_t *st = starts.data_ptr<int64_t>(), *en = ends.data_ptr<int64_t>();
-    const int64_t need = api.cinn_fp8_grouped_wgrad_fused_scratch_bytes(R, E, d_in, d_out);
+    const bool segments = !xs.defined();
+    const int64_t need = segments ? api.cinn_fp8_grouped_wgrad_segments_scratch_bytes(R, E, d_out)
+                                  : api.cinn_fp8_grouped_wgrad_fused_scratch_bytes(R, E, d_in, d_out);
     Tensor scratch = empty({need}, at::kByte, dev), dw = empty({E, d_out, d_in}, w_type, dev);
     Tensor gq = empty({R, d_out}, F8, dev), gs = empty({R, d_out / 128}, at::kFloat, dev);
     const bool one_pass = dy.scalar_type() != at::kFloat;          // both quantisations of dy from one pass: 2-byte gradients
-    check(api.cinn_fp8_grouped_wgrad_fused(dy.data_ptr(), tag_of(dy.scalar_type()), xq.data_ptr(), f32(xs), st, en, E, R, d_in, d_out,
-                                           scratch.data_ptr(), need, dw.data_ptr(), w_type == at::kFloat ? TAG_F32_BF16 : TAG_BF16, div,
-                                           one_pass ? gq.data_ptr() : nullptr, one_pass ? f32(gs) : nullptr, stream()), "cinn_fp8_grouped_wgrad_fused");
+    void* rows_q = one_pass ? gq.data_ptr() : nullptr;
+    float* rows_s = one_pass ? f32(gs) : nullptr;
+    const int dw_tag = w_type == at::kFloat ? TAG_F32_BF16 : TAG_BF16;
+    if (h12.defined())
+        check(api.cinn_fp8_grouped_wgrad_swiglu(h12.data_ptr(), dy.data_ptr(), tag_of(dy.scalar_type()), xq.data_ptr(), f32(xs), st, en, E, R, d_in,
+                                                d_out / 2, scratch.data_ptr(), need, dw.data_ptr(), dw_tag, rows_q, rows_s, stream()),
+              "cinn_fp8_grouped_wgrad_swiglu");
+    else if (segments)
+        check(api.cinn_fp8_grouped_wgrad_segments(dy.data_ptr(), tag_of(dy.scalar_type()), xq.data_ptr(), E, R, d_in, d_out, scratch.data_ptr(),
+                                                  need, dw.data_ptr(), dw_tag, div, rows_q, rows_s, stream()), "cinn_fp8_grouped_wgrad_segments");
+    else
+        check(api.cinn_fp8_grouped_wgrad_fused(dy.data_ptr(), tag_of(dy.scalar_type()), xq.data_ptr(), f32(xs), st, en, E, R, d_in, d_out,
+                                               scratch.data_ptr(), need, dw.data_ptr(), dw_tag, div, rows_q, rows_s, stream()),
+              "cinn_fp8_grouped_wgrad_fused");
     Tensor dx;
     if (want_x) {
         if (!one_pass) {
@@ -147,8 +201,24 @@ struct BlockNode : public torch::autograd::Function<BlockNode> {
         const Tensor starts = r.starts(), ends = r.ends();
         const Quantised rows = spread(rowwise(x, false, o->div), r, k);
         const Tensor h12 = grouped(rows, o->w12, starts, ends);
-        const Quantised h = swiglu_quantised(h12, o->div);
-        const Tensor out = grouped(h, o->w3, starts, ends);
+        // Where a backward will come, the weight gradient's copy of the activations comes out of the same pass; it is kept in place of
+        // the row-wise bytes (h.s undefined: h.q holds the segments).
+        Quantised h;
+        Tensor out;
+        const bool segments = (w12.requires_grad() || w3.requires_grad() || x.requires_grad()) && swiglu_in_quantisers(h12, true, o->div) &&
+                              r.pairs > 0 && h12.size(1) % 512 == 0 && d % 256 == 0 && E <= 1024 && up(r.pairs, 128) + E <= 65535;
+        if (segments) {
+            const int64_t I = h12.size(1) / 2, bytes = api.cinn_quant_segments_bytes(r.pairs, E, I);
+            const Quantised hq{empty({r.pairs, I}, F8, dev), empty({r.pairs, I / 128}, at::kFloat, dev)};
+            h.q = empty({bytes}, at::kByte, dev);
+            check(api.cinn_swiglu_quant_segments(h12.data_ptr(), tag_of(h12.scalar_type()), r.pairs, I, starts.data_ptr<int64_t>(),
+                                                 ends.data_ptr<int64_t>(), E, hq.q.data_ptr(), f32(hq.s), h.q.data_ptr(), bytes, stream()),
+                  "cinn_swiglu_quant_segments");
+            out = grouped(hq, o->w3, starts, ends);
+        } else {
+            h = swiglu_quantised(h12, o->div);
+            out = grouped(h, o->w3, starts, ends);
+        }
         Tensor y = empty({T, d}, at::kFloat, dev);
         check(api.cinn_moe_combine_add(out.data_ptr(), TAG_BF16, r.pos(), r.gates(), addend.data_ptr(), tag_of(addend.scalar_type()), f32(y),
                                        T, r.pairs, (int)k, d, stream()), "cinn_moe_combine_add");
@@ -204,11 +274,16 @@ struct BlockNode : public torch::autograd::Function<BlockNode> {
                     d_out.reset();
                     if (below) {
                         const int64_t I = h12.size(1) / 2;
-                        Tensor dh12 = empty({r.pairs, 2 * I}, at::kBFloat16, dev);
-                        check(api.cinn_swiglu_backward(h12.data_ptr(), dh.data_ptr(), dh12.data_ptr(), TAG_BF16, r.pairs, I, stream()),
-                              "cinn_swiglu_backward");
-                        std::tie(d_rows, dw12) = grouped_backward(dh12, s[5], s[6], s[11], s[12], starts, ends, type(5), want_x,
-                                                                  type(3), div);
+                        if (!s[9].defined()) {             // the widths and the division flavour were found to fit in the forward
+                            std::tie(d_rows, dw12) = grouped_backward(dh, s[5], s[6], s[11], s[12], starts, ends, type(5), want_x, type(3), div,
+                                                                      true, h12);
+                        } else {
+                            Tensor dh12 = empty({r.pairs, 2 * I}, at::kBFloat16, dev);
+                            check(api.cinn_swiglu_backward(h12.data_ptr(), dh.data_ptr(), dh12.data_ptr(), TAG_BF16, r.pairs, I, stream()),
+                                  "cinn_swiglu_backward");
+                            std::tie(d_rows, dw12) = grouped_backward(dh12, s[5], s[6], s[11], s[12], starts, ends, type(5), want_x,
+                                                                      type(3), div);
+                        }
                     }
                 }
             }
@@ -246,8 +321,24 @@ struct GroupedNode : public torch::autograd::Function<GroupedNode> {
         c10::cuda::CUDAGuard guard(x_in.device());
         at::AutoDispatchBelowAutograd below;
         const Tensor x = readable(x_in), starts = starts_in.to(at::kLong).contiguous(), ends = ends_in.to(at::kLong).contiguous();
-        const Quantised xq = rowwise(x, false, (int)div);
-        ctx->save_for_backward({xq.q, xq.s, wq->q, wq->s, starts, ends});
+        const int64_t R = x.size(0), E = wq->q.size(0), d = x.dim() == 2 ? x.size(1) : 0;
+        // Where the weight gradient can be had (its widths are multiples of 256) its copy of x comes out of the forward's pass.
+        const bool segments = w.requires_grad() && x.dim() == 2 && x.element_size() == 2 && x.is_contiguous() && R > 0 && d == wq->q.size(2) &&
+                              d % 256 == 0 && wq->q.size(1) % 256 == 0 && E >= 1 && E <= 1024 && up(R, 128) + E <= 65535 &&
+                              starts.numel() == E && ends.numel() == E && (reinterpret_cast<uintptr_t>(x.data_ptr()) & 15) == 0;
+        Quantised xq;
+        if (segments) {
+            const int64_t bytes = api.cinn_quant_segments_bytes(R, E, d);
+            Tensor seg = empty({bytes}, at::kByte, x.device());
+            xq = {empty({R, d}, F8, x.device()), empty({R, d / 128}, at::kFloat, x.device())};
+            check(api.cinn_quant_rowwise_segments(x.data_ptr(), tag_of(x.scalar_type()), R, d, starts.data_ptr<int64_t>(), ends.data_ptr<int64_t>(),
+                                                  E, xq.q.data_ptr(), f32(xq.s), seg.data_ptr(), bytes, (int)div, stream()),
+                  "cinn_quant_rowwise_segments");
+            ctx->save_for_backward({seg, Tensor(), wq->q, wq->s, starts, ends});
+        } else {
+            xq = rowwise(x, false, (int)div);
+            ctx->save_for_backward({xq.q, xq.s, wq->q, wq->s, starts, ends});
+        }
         ctx->saved_data["n"] = std::vector<int64_t>{(int64_t)x_in.scalar_type(), (int64_t)w.scalar_type(), div};
         return grouped(xq, *wq, starts, ends, type);
     }
@@ -256,7 +347,7 @@ struct GroupedNode : public torch::autograd::Function<GroupedNode> {
         const auto n = ctx->saved_data["n"].toIntVector();
         Tensor dx, dw;
         as_python_error([&] {
-            c10::cuda::CUDAGuard guard(s[0].device());
+            c10::cuda::CUDAGuard guard(s[2].device());
             const Tensor dy = readable(grads[0]).contiguous();
             const auto x_type = (at::ScalarType)n[0], w_type = (at::ScalarType)n[1];
             const auto dx_type = tag_of(x_type) < 0 ? at::kFloat : x_type;

@@ -384,17 +384,19 @@ __device__ __forceinline__ bool dual_tile(float (&v)[8][8], float (*s_amax)[128]
 // written; the thread then decodes its own bytes, multiplies by the row scale (exactly what
 // dequantize_fp8_rowwise yields), and the block's amax is one shuffle tree + shared memory.  Bit-identical to
 // quantize_fp8_rowwise followed by the row-to-block re-quantiser, with x read once and its e4m3 copy never re-read.
-// TRANS: the block-scaled bytes are written transposed, (N, M) with M contiguous (M a multiple of 16): the layout in
-// which the weight-gradient GEMM reads them K-major.  They leave through the staging tile of dual_tile.
-template <int DIV, bool ROUND, bool TRANS, typename AfterSync>
+// TRANS: the block-scaled bytes are written transposed, (N, M) with M contiguous and rounded up to 16 (zeros behind it): the
+// layout in which the weight-gradient GEMM reads them K-major.  They leave through the staging tile of dual_tile.
+// SEG: as in dual_tile (TRANS only).
+template <int DIV, bool ROUND, bool TRANS, bool SEG = false, typename AfterSync>
 __device__ __forceinline__ bool row_block_tile(float (&v)[8][8], float* s_red, uint8_t* s_out, bool ok,
                                                uint8_t* __restrict__ q_row,
                                                float* __restrict__ s_row, uint8_t* __restrict__ q_blk,
                                                float* __restrict__ s_blk, int M, int N, int nb_n, int bm, int bn,
-                                               AfterSync&& after_sync) {
+                                               AfterSync&& after_sync, int src0 = 0, int cnt = 128) {
     const int sub = threadIdx.x & 15, hw = threadIdx.x >> 4, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int n = bn * 128 + sub * 8;
-    const int mt = bm * 128 + hw * 8;
+    const int mt = SEG ? src0 + hw * 8 : bm * 128 + hw * 8;    // first row of this thread's row-wise outputs
+    const int m_rows = SEG ? src0 + cnt : M;                    // one past the last of them
     float bmax = 0.0f;
     float m[8];
 #pragma unroll
@@ -405,7 +407,7 @@ __device__ __forceinline__ bool row_block_tile(float (&v)[8][8], float* s_red, u
     }
     const float mine = scale_from_amax<DIV, ROUND>(half_warp_rows_max(m, sub));
     const int own = mt + half_warp_row(sub);
-    if ((sub & 1) == 0 && own < M) s_row[(int64_t)own * nb_n + bn] = mine;
+    if ((sub & 1) == 0 && own < m_rows) s_row[(int64_t)own * nb_n + bn] = mine;
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
         const float s = __shfl_sync(0xffffffffu, mine, half_warp_lane(i), 16);
@@ -415,7 +417,7 @@ __device__ __forceinline__ bool row_block_tile(float (&v)[8][8], float* s_red, u
                           scaled_clamped<DIV>(v[i][2], d), scaled_clamped<DIV>(v[i][3], d));
         o2.y = cvt_e4m3x4(scaled_clamped<DIV>(v[i][4], d), scaled_clamped<DIV>(v[i][5], d),
                           scaled_clamped<DIV>(v[i][6], d), scaled_clamped<DIV>(v[i][7], d));
-        const bool inb = mt + i < M && n < N;
+        const bool inb = mt + i < m_rows && n < N;
         if (inb) __stcs(reinterpret_cast<uint2*>(q_row + (int64_t)(mt + i) * N + n), o2);
         // what the backward would read back: e4m3 value times the row scale (zero outside the matrix)
         const uint32_t w[2] = {o2.x, o2.y};
@@ -481,6 +483,297 @@ __device__ __forceinline__ bool row_block_tile(float (&v)[8][8], float* s_red, u
         // the staging tile and s_red are next written after the next piece's block-wide barrier
     }
     return true;
+}
+
+// ---------------------------------------------------------------------------
+// The same two passes on a piece of a 2-byte type as it is stored, with the products of div.full (x times the scale's reciprocal).
+// They are bound by their instructions, so those that only matter for NaN and infinity go: amaxes are taken of packed pairs with a
+// maximum that hands NaN on, and where that finds every element finite nothing has to be clamped (the conversion saturates), a
+// row tile's largest decoded value is its amax converted (conversion and products are monotone), and products come in pairs.
+// A piece with any other element takes the passes above.
+// ---------------------------------------------------------------------------
+template <typename T> struct Pair;
+template <> struct Pair<__nv_bfloat16> {
+    static constexpr uint32_t EXP = 0x7f807f80u;          // exponent of infinity and NaN
+    static __device__ __forceinline__ uint32_t max_nan(uint32_t a, uint32_t b) {
+        const __nv_bfloat162 r = __hmax2_nan(*reinterpret_cast<const __nv_bfloat162*>(&a), *reinterpret_cast<const __nv_bfloat162*>(&b));
+        return *reinterpret_cast<const uint32_t*>(&r);
+    }
+    static __device__ __forceinline__ float lo(uint32_t w) { return __uint_as_float(w << 16); }
+    static __device__ __forceinline__ float hi(uint32_t w) { return __uint_as_float(w & 0xffff0000u); }
+    static __device__ __forceinline__ float2 both(uint32_t w) { return make_float2(lo(w), hi(w)); }
+};
+template <> struct Pair<__half> {
+    static constexpr uint32_t EXP = 0x7c007c00u;
+    static __device__ __forceinline__ uint32_t max_nan(uint32_t a, uint32_t b) {
+        const __half2 r = __hmax2_nan(*reinterpret_cast<const __half2*>(&a), *reinterpret_cast<const __half2*>(&b));
+        return *reinterpret_cast<const uint32_t*>(&r);
+    }
+    static __device__ __forceinline__ float2 both(uint32_t w) { return __half22float2(*reinterpret_cast<const __half2*>(&w)); }
+    static __device__ __forceinline__ float lo(uint32_t w) { return both(w).x; }
+    static __device__ __forceinline__ float hi(uint32_t w) { return both(w).y; }
+};
+template <typename T>
+__device__ __forceinline__ bool not_finite(uint32_t w) {          // either half infinite or NaN
+    constexpr uint32_t E = Pair<T>::EXP;
+    return (w & E & 0xffffu) == (E & 0xffffu) || (w & E & 0xffff0000u) == (E & 0xffff0000u);
+}
+
+struct Raw8x8 { uint32_t w[8][4]; };                       // rows hw * 8 + i, columns sub * 8 + 2 * k and + 1 of the piece
+
+// half_warp_rows_max of packed candidates: m[i] holds two of row i.  The result, of row half_warp_row(sub), in both halves.
+template <typename T>
+__device__ __forceinline__ uint32_t half_warp_rows_max_packed(const uint32_t (&m)[8], int sub) {
+    uint32_t r[4], a[2];
+    const bool up8 = sub & 8, up4 = sub & 4, up2 = sub & 2;
+#pragma unroll
+    for (int i = 0; i < 4; ++i)                            // rows 2i | 2i + 1
+        r[i] = Pair<T>::max_nan(__byte_perm(m[2 * i], m[2 * i + 1], 0x5410), __byte_perm(m[2 * i], m[2 * i + 1], 0x7632));
+#pragma unroll
+    for (int i = 0; i < 2; ++i)
+        a[i] = Pair<T>::max_nan(up8 ? r[i + 2] : r[i], __shfl_xor_sync(0xffffffffu, up8 ? r[i] : r[i + 2], 8));
+    uint32_t b = Pair<T>::max_nan(up4 ? a[1] : a[0], __shfl_xor_sync(0xffffffffu, up4 ? a[0] : a[1], 4));
+    b = Pair<T>::max_nan(b, __shfl_xor_sync(0xffffffffu, b, 2));
+    b = Pair<T>::max_nan(b, __shfl_xor_sync(0xffffffffu, b, 1));
+    return __byte_perm(b, 0, up2 ? 0x3232 : 0x1010);
+}
+// two products by one factor each
+__device__ __forceinline__ float2 mul2(float2 x, float2 d) {
+    float2 y;
+    asm("{\n\t.reg .b64 a, b;\n\tmov.b64 a, {%2, %3};\n\tmov.b64 b, {%4, %5};\n\tmul.rn.f32x2 a, a, b;\n\tmov.b64 {%0, %1}, a;\n\t}"
+        : "=f"(y.x), "=f"(y.y) : "f"(x.x), "f"(x.y), "f"(d.x), "f"(d.y));
+    return y;
+}
+__device__ __forceinline__ uint32_t cvt_pairs(float2 a, float2 b) { return cvt_e4m3x4(a.x, a.y, b.x, b.y); }
+
+template <typename T, bool ROUND, bool SEG = false, typename AfterSync>
+__device__ __forceinline__ bool dual_tile16(const Raw8x8& in, float (*s_amax)[128], uint8_t* s_out, bool ok,
+                                            uint8_t* __restrict__ q_row, float* __restrict__ s_row,
+                                            uint8_t* __restrict__ q_col, float* __restrict__ s_col, int M, int N, int nb_n,
+                                            int nb_m, int bm, int bn, AfterSync&& after_sync, int src0 = 0, int cnt = 128) {
+    using P = Pair<T>;
+    constexpr int DIV = CINN_DIV_FULL;
+    const int sub = threadIdx.x & 15, hw = threadIdx.x >> 4, warp = threadIdx.x >> 5;
+    const int m0 = bm * 128, n0 = bn * 128;
+    const int n = n0 + sub * 8;
+    const int mt = SEG ? src0 + hw * 8 : m0 + hw * 8;
+    const int m_rows = SEG ? src0 + cnt : M;
+    const int pitch = (M + 15) & ~15;
+    Raw8x8 r = in;
+    if constexpr (SEG) {
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+            if (hw * 8 + i >= cnt) {
+#pragma unroll
+                for (int k = 0; k < 4; ++k) r.w[i][k] = 0u;
+            }
+    }
+    uint32_t rmax[8], cmax[4] = {0u, 0u, 0u, 0u};
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        uint32_t m = 0u;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const uint32_t a = r.w[i][k] & 0x7fff7fffu;
+            m = P::max_nan(m, a);
+            cmax[k] = P::max_nan(cmax[k], a);
+        }
+        rmax[i] = m;
+    }
+    bool odd = false;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        odd |= not_finite<T>(cmax[k]);
+        cmax[k] = P::max_nan(cmax[k], __shfl_xor_sync(0xffffffffu, cmax[k], 16));
+    }
+    uint32_t (*s_packed)[64] = reinterpret_cast<uint32_t (*)[64]>(s_amax + 1);       // (row 0 is for the columns' divisors)
+    if ((threadIdx.x & 31) < 16) *reinterpret_cast<uint4*>(&s_packed[warp][sub * 4]) = make_uint4(cmax[0], cmax[1], cmax[2], cmax[3]);
+    if (!__syncthreads_and(ok && !odd)) {
+        float v[8][8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+#pragma unroll
+            for (int k = 0; k < 4; ++k) { const float2 f = P::both(in.w[i][k]); v[i][2 * k] = f.x; v[i][2 * k + 1] = f.y; }
+        return dual_tile<DIV, ROUND, SEG>(v, s_amax, s_out, ok, q_row, s_row, q_col, s_col, M, N, nb_n, nb_m, bm, bn, after_sync, src0, cnt);
+    }
+    after_sync();
+    if ((threadIdx.x & 31) < 8) {
+        const int c = warp * 8 + (threadIdx.x & 7);        // two columns
+        uint32_t a = s_packed[0][c];
+#pragma unroll
+        for (int w = 1; w < 8; ++w) a = P::max_nan(a, s_packed[w][c]);
+        const float2 am = P::both(a);
+        const float lo = scale_from_amax<DIV, ROUND>(am.x), hi = scale_from_amax<DIV, ROUND>(am.y);
+        *reinterpret_cast<float2*>(&s_amax[0][2 * c]) = make_float2(divisor_of<DIV>(lo), divisor_of<DIV>(hi));
+        if (n0 + 2 * c < N) s_col[(int64_t)(n0 + 2 * c) * nb_m + bm] = lo;
+        if (n0 + 2 * c + 1 < N) s_col[(int64_t)(n0 + 2 * c + 1) * nb_m + bm] = hi;
+    }
+    float2 v[8][4];
+    {
+        const float s = scale_from_amax<DIV, ROUND>(P::lo(half_warp_rows_max_packed<T>(rmax, sub)));
+        const float mine = divisor_of<DIV>(s);
+        const int own = mt + half_warp_row(sub);
+        if ((sub & 1) == 0 && own < m_rows && n0 < N) s_row[(int64_t)own * nb_n + bn] = s;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            const float d = __shfl_sync(0xffffffffu, mine, half_warp_lane(i), 16);
+            const float2 d2 = make_float2(d, d);
+#pragma unroll
+            for (int k = 0; k < 4; ++k) v[i][k] = P::both(r.w[i][k]);
+            if (mt + i < m_rows && n < N) {
+                uint2 o2;
+                o2.x = cvt_pairs(mul2(v[i][0], d2), mul2(v[i][1], d2));
+                o2.y = cvt_pairs(mul2(v[i][2], d2), mul2(v[i][3], d2));
+                __stcs(reinterpret_cast<uint2*>(q_row + (int64_t)(mt + i) * N + n), o2);
+            }
+        }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        const float2 d2 = *reinterpret_cast<const float2*>(&s_amax[0][sub * 8 + 2 * k]);
+        float2 y[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) y[i] = mul2(v[i][k], d2);
+        const uint32_t at = ((((hw >> 1) ^ sub) & 7) << 4) + ((hw & 1) << 3);
+        uint8_t* col = &s_out[(sub * 8 + 2 * k) * 128 + at];
+        *reinterpret_cast<uint2*>(col) = make_uint2(cvt_e4m3x4(y[0].x, y[1].x, y[2].x, y[3].x), cvt_e4m3x4(y[4].x, y[5].x, y[6].x, y[7].x));
+        *reinterpret_cast<uint2*>(col + 128) = make_uint2(cvt_e4m3x4(y[0].y, y[1].y, y[2].y, y[3].y), cvt_e4m3x4(y[4].y, y[5].y, y[6].y, y[7].y));
+    }
+    __syncthreads();
+#pragma unroll
+    for (int rep = 0; rep < 4; ++rep) {
+        const int idx = threadIdx.x + rep * 256;
+        const int nl = idx >> 3, ch = idx & 7;
+        const int nn = n0 + nl, mm = m0 + ch * 16;
+        if (nn < N && mm < pitch) {
+            const uint4 val = *reinterpret_cast<const uint4*>(&s_out[nl * 128 + (((ch ^ (nl >> 3)) & 7) << 4)]);
+            __stcs(reinterpret_cast<uint4*>(q_col + (int64_t)nn * pitch + mm), val);
+        }
+    }
+    return true;
+}
+
+template <typename T, bool ROUND, bool TRANS, bool SEG = false, typename AfterSync>
+__device__ __forceinline__ bool row_block_tile16(const Raw8x8& in, float* s_red, uint8_t* s_out, bool ok, uint8_t* __restrict__ q_row,
+                                                 float* __restrict__ s_row, uint8_t* __restrict__ q_blk, float* __restrict__ s_blk, int M,
+                                                 int N, int nb_n, int bm, int bn, AfterSync&& after_sync, int src0 = 0, int cnt = 128) {
+    using P = Pair<T>;
+    constexpr int DIV = CINN_DIV_FULL;
+    const int sub = threadIdx.x & 15, hw = threadIdx.x >> 4, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int n = bn * 128 + sub * 8;
+    const int mt = SEG ? src0 + hw * 8 : bm * 128 + hw * 8;
+    const int m_rows = SEG ? src0 + cnt : M;
+    uint32_t rmax[8];
+    bool odd = false;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        uint32_t m = 0u;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) m = P::max_nan(m, in.w[i][k] & 0x7fff7fffu);
+        rmax[i] = m;
+        odd |= not_finite<T>(m);
+    }
+    const float amax = P::lo(half_warp_rows_max_packed<T>(rmax, sub));
+    const float mine = scale_from_amax<DIV, ROUND>(amax);
+    const int own = mt + half_warp_row(sub);
+    // the row tile's largest decoded value; rows of other pieces and past the end count as zeros
+    float bmax = own < m_rows ? __fmul_rn(e4m3x2_to_float2(cvt_e4m3x2(__fmul_rn(amax, divisor_of<DIV>(mine)), 0.0f)).x, mine) : 0.0f;
+    bmax = warp_max(bmax);
+    if (lane == 0) s_red[warp] = bmax;
+    const bool finite = __syncthreads_and(ok && !odd);
+    bmax = s_red[0];
+#pragma unroll
+    for (int w8 = 1; w8 < 8; ++w8) bmax = fmaxf(bmax, s_red[w8]);
+    if (!finite || !(bmax <= 3.4e38f)) {                   // (a power-of-two scale can take a decoded value past the largest float)
+        __syncthreads();
+        float v[8][8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+#pragma unroll
+            for (int k = 0; k < 4; ++k) { const float2 f = P::both(in.w[i][k]); v[i][2 * k] = f.x; v[i][2 * k + 1] = f.y; }
+        return row_block_tile<DIV, ROUND, TRANS, SEG>(v, s_red, s_out, ok, q_row, s_row, q_blk, s_blk, M, N, nb_n, bm, bn, after_sync, src0, cnt);
+    }
+    after_sync();
+    if ((sub & 1) == 0 && own < m_rows) s_row[(int64_t)own * nb_n + bn] = mine;
+    const float sb = scale_from_amax<DIV, false>(bmax), db = divisor_of<DIV>(sb);
+    const float2 db2 = make_float2(db, db);
+    if (threadIdx.x == 0) s_blk[(int64_t)bm * nb_n + bn] = sb;
+    float2 v[8][4];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        const float s = __shfl_sync(0xffffffffu, mine, half_warp_lane(i), 16);
+        const float d = divisor_of<DIV>(s);
+        const float2 d2 = make_float2(d, d), s2 = make_float2(s, s);
+        uint2 o2;
+        o2.x = cvt_pairs(mul2(P::both(in.w[i][0]), d2), mul2(P::both(in.w[i][1]), d2));
+        o2.y = cvt_pairs(mul2(P::both(in.w[i][2]), d2), mul2(P::both(in.w[i][3]), d2));
+        const bool inb = mt + i < m_rows && n < N;
+        if (inb) __stcs(reinterpret_cast<uint2*>(q_row + (int64_t)(mt + i) * N + n), o2);
+        if (SEG && mt + i >= m_rows) o2 = make_uint2(0u, 0u);          // (past the end of the matrix everything is zero already)
+        v[i][0] = mul2(mul2(e4m3x2_to_float2((uint16_t)(o2.x & 0xffff)), s2), db2);
+        v[i][1] = mul2(mul2(e4m3x2_to_float2((uint16_t)(o2.x >> 16)), s2), db2);
+        v[i][2] = mul2(mul2(e4m3x2_to_float2((uint16_t)(o2.y & 0xffff)), s2), db2);
+        v[i][3] = mul2(mul2(e4m3x2_to_float2((uint16_t)(o2.y >> 16)), s2), db2);
+        if constexpr (!TRANS) {
+            if (inb) __stcs(reinterpret_cast<uint2*>(q_blk + (int64_t)(mt + i) * N + n), make_uint2(cvt_pairs(v[i][0], v[i][1]), cvt_pairs(v[i][2], v[i][3])));
+        }
+    }
+    if constexpr (!TRANS) {
+        __syncthreads();                      // s_red is free for the next piece
+    } else {
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const uint32_t at = ((((hw >> 1) ^ sub) & 7) << 4) + ((hw & 1) << 3);
+            uint8_t* col = &s_out[(sub * 8 + 2 * k) * 128 + at];
+            *reinterpret_cast<uint2*>(col) = make_uint2(cvt_e4m3x4(v[0][k].x, v[1][k].x, v[2][k].x, v[3][k].x), cvt_e4m3x4(v[4][k].x, v[5][k].x, v[6][k].x, v[7][k].x));
+            *reinterpret_cast<uint2*>(col + 128) = make_uint2(cvt_e4m3x4(v[0][k].y, v[1][k].y, v[2][k].y, v[3][k].y), cvt_e4m3x4(v[4][k].y, v[5][k].y, v[6][k].y, v[7][k].y));
+        }
+        __syncthreads();
+        const int m0 = bm * 128, n0 = bn * 128, pitch = (M + 15) & ~15;
+#pragma unroll
+        for (int rep = 0; rep < 4; ++rep) {
+            const int idx = threadIdx.x + rep * 256;
+            const int nl = idx >> 3, ch = idx & 7;
+            const int nn = n0 + nl, mm = m0 + ch * 16;
+            if (nn < N && mm < pitch) {
+                const uint4 val = *reinterpret_cast<const uint4*>(&s_out[nl * 128 + (((ch ^ (nl >> 3)) & 7) << 4)]);
+                __stcs(reinterpret_cast<uint4*>(q_blk + (int64_t)nn * pitch + mm), val);
+            }
+        }
+    }
+    return true;
+}
+
+// One piece of a 2-byte type out of its stage, by the passes that its division flavour allows.  MODE as in the kernels below.
+template <typename T, int DIV, bool ROUND, int MODE, bool SEG = false, typename AfterSync>
+__device__ __forceinline__ bool piece_from_stage(const uint8_t* src, float (*s_amax)[128], uint8_t* s_out, bool ok, uint8_t* q_row, float* s_row,
+                                                 uint8_t* q_col, float* s_col, int M, int N, int nb_n, int nb_m, int bm, int bn,
+                                                 AfterSync&& after_sync, int src0 = 0, int cnt = 128) {
+    Raw8x8 raw;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        const uint4 a = *reinterpret_cast<const uint4*>(src + i * 256);
+        raw.w[i][0] = a.x; raw.w[i][1] = a.y; raw.w[i][2] = a.z; raw.w[i][3] = a.w;
+    }
+    if constexpr (DIV == CINN_DIV_FULL) {
+        if constexpr (MODE == 0)
+            return dual_tile16<T, ROUND, SEG>(raw, s_amax, s_out, ok, q_row, s_row, q_col, s_col, M, N, nb_n, nb_m, bm, bn, after_sync, src0, cnt);
+        else
+            return row_block_tile16<T, ROUND, MODE == 2, SEG>(raw, &s_amax[0][0], s_out, ok, q_row, s_row, q_col, s_col, M, N, nb_n, bm, bn,
+                                                              after_sync, src0, cnt);
+    } else {
+        float v[8][8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+#pragma unroll
+            for (int k = 0; k < 4; ++k) { const float2 f = Pair<T>::both(raw.w[i][k]); v[i][2 * k] = f.x; v[i][2 * k + 1] = f.y; }
+        if constexpr (MODE == 0)
+            return dual_tile<DIV, ROUND, SEG>(v, s_amax, s_out, ok, q_row, s_row, q_col, s_col, M, N, nb_n, nb_m, bm, bn, after_sync, src0, cnt);
+        else
+            return row_block_tile<DIV, ROUND, MODE == 2, SEG>(v, &s_amax[0][0], s_out, ok, q_row, s_row, q_col, s_col, M, N, nb_n, bm, bn,
+                                                              after_sync, src0, cnt);
+    }
 }
 
 // One CTA per piece, loads straight into registers (4-byte inputs, and rows whose pitch a tensor map cannot take).
@@ -579,23 +872,12 @@ quant_row_dual_tma_kernel(const __grid_constant__ CUtensorMap tmX, uint8_t* __re
     for (; t < total; t += stride, ++k) {
         const int s = k % DUAL_STAGES;
         const bool ok = mbar_wait_bounded(full0 + 8 * s, (k / DUAL_STAGES) & 1);
-        const uint8_t* src = stages + s * DUAL_STAGE_BYTES + (hw * 8) * 256 + sub * 16;
-        float v[8][8];
-#pragma unroll
-        for (int i = 0; i < 8; ++i) {
-            Raw8<T> r;
-            r.a = *reinterpret_cast<const uint4*>(src + i * 256);
-            unpack_raw8<T>(r, v[i]);
-        }
         const int tn = t + DUAL_STAGES * stride;
         int bm, bn;
         coords(t, bm, bn);
-        if constexpr (MODE == 0)
-            alive = dual_tile<DIV, ROUND>(v, s_amax, s_out, ok, q_row, s_row, q_col, s_col, M, N, nb_n, nb_m, bm, bn,
-                                          [&] { if (threadIdx.x == 0 && tn < total) issue(tn, s); });
-        else
-            alive = row_block_tile<DIV, ROUND, MODE == 2>(v, &s_amax[0][0], s_out, ok, q_row, s_row, q_col, s_col, M, N, nb_n,
-                                                          bm, bn, [&] { if (threadIdx.x == 0 && tn < total) issue(tn, s); });
+        alive = piece_from_stage<T, DIV, ROUND, MODE>(stages + s * DUAL_STAGE_BYTES + (hw * 8) * 256 + sub * 16, s_amax, s_out, ok, q_row, s_row,
+                                                      q_col, s_col, M, N, nb_n, nb_m, bm, bn,
+                                                      [&] { if (threadIdx.x == 0 && tn < total) issue(tn, s); });
         if (!alive) break;
     }
     if (!alive && threadIdx.x == 0) {
@@ -606,12 +888,14 @@ quant_row_dual_tma_kernel(const __grid_constant__ CUtensorMap tmX, uint8_t* __re
     }
 }
 
-// The dual quantiser over a token axis cut into per-expert segments (the backward of the grouped expert GEMM): one
+// The dual quantiser (MODE 0) over a token axis cut into per-expert segments (the backward of the grouped expert GEMM): one
 // pass over dY yields its row-wise quantisation (what the grouped input gradient reads, in place of the rows) and the
 // quantisation of dY^T along the tokens of each segment, padded to whole tiles (what the grouped weight gradient
 // reads).  Tile y of the padded axis holds tile_cnt[y] rows from tile_src[y] on; only the first *n_tiles tiles exist.
 // Same TMA ring as the dense kernel; the elected thread leaves each stage's (first row, row count) beside the barriers.
-template <typename T, int DIV>
+// MODE 2: the row + block pass with its block copy transposed, segment by segment (the forward's x, whose block copy the weight
+// gradient reads: one pass of 195 us over 32768 x 7168 in place of the row-wise one and a re-quantisation of its bytes, 165 + 157).
+template <typename T, int DIV, int MODE>
 __global__ void __launch_bounds__(256, 2)
 quant_row_dual_seg_kernel(const __grid_constant__ CUtensorMap tmX, uint8_t* __restrict__ q_row, float* __restrict__ s_row,
                           uint8_t* __restrict__ q_col, float* __restrict__ s_col, int M_pad, int N, int nb_n, int nb_m,
@@ -652,24 +936,150 @@ quant_row_dual_seg_kernel(const __grid_constant__ CUtensorMap tmX, uint8_t* __re
         const int s = k % DUAL_STAGES;
         const bool ok = mbar_wait_bounded(full0 + 8 * s, (k / DUAL_STAGES) & 1);
         const int src0 = s_meta[2 * s], cnt = s_meta[2 * s + 1];
-        const uint8_t* src = stages + s * DUAL_STAGE_BYTES + (hw * 8) * 256 + sub * 16;
-        float v[8][8];
-#pragma unroll
-        for (int i = 0; i < 8; ++i) {
-            Raw8<T> r;
-            r.a = *reinterpret_cast<const uint4*>(src + i * 256);
-            unpack_raw8<T>(r, v[i]);
-        }
         const int tn = t + DUAL_STAGES * stride;
         const int bm = t / nb_n, bn = t - bm * nb_n;
-        alive = dual_tile<DIV, false, true>(v, s_amax, s_out, ok, q_row, s_row, q_col, s_col, M_pad, N, nb_n, nb_m, bm, bn,
-                                            [&] { if (threadIdx.x == 0 && tn < total) issue(tn, s); }, src0, cnt);
+        alive = piece_from_stage<T, DIV, false, MODE, true>(stages + s * DUAL_STAGE_BYTES + (hw * 8) * 256 + sub * 16, s_amax, s_out, ok, q_row,
+                                                            s_row, q_col, s_col, M_pad, N, nb_n, nb_m, bm, bn,
+                                                            [&] { if (threadIdx.x == 0 && tn < total) issue(tn, s); }, src0, cnt);
         if (!alive) break;
     }
     if (!alive && threadIdx.x == 0) {
         atomicCAS(&g_quant_status, 0, (4 << 8) | 1);
         for (int j = 1; j < DUAL_STAGES; ++j)
             if (t + j * stride < total) mbar_wait_bounded(full0 + 8 * ((k + j) % DUAL_STAGES), ((k + j) / DUAL_STAGES) & 1);
+    }
+}
+
+// ---------------------------------------------------------------------------
+// SwiGLU inside the quantisers that follow it (16-bit activations, products of div.full): its result does not go to memory in
+// between.  h12 is (rows, 2 * I), the gate half first.
+//   swiglu_row_block_kernel     forward: h = silu(h1) * h2, row-wise and, in blocks, transposed (row_block_tile16).
+//                               32768 x 2 x 1024: 46 us of SwiGLU and 29 of the quantiser, as one pass %FWD%
+//   swiglu_backward_dual_kernel backward: both halves of dh12 from h12 and dh, along both axes (dual_tile16).  56 and 52 us, so %BWD%
+// Values are rounded to the activation type where the separate kernels round them, so the bytes are theirs.
+// EXACT: silu by the exact sequences, rounded by itself before the product (the shared expert's layers); else a few fp32 ulp off, not
+// rounded by itself (the routed experts': see swiglu_quant_row_kernel) in the forward, exact and unrounded in the backward.
+// SEG: pieces are tiles of the experts' segments, as in quant_row_dual_seg_kernel.
+// Bound by memory with the loads of a piece, 32 or 48 KiB of a CTA, in registers; two CTAs per SM load and convert in turn.
+// ---------------------------------------------------------------------------
+template <typename T> __device__ __forceinline__ uint32_t pack2(float lo, float hi);
+template <> __device__ __forceinline__ uint32_t pack2<__nv_bfloat16>(float lo, float hi) {
+    const __nv_bfloat162 h = __floats2bfloat162_rn(lo, hi);
+    return *reinterpret_cast<const uint32_t*>(&h);
+}
+template <> __device__ __forceinline__ uint32_t pack2<__half>(float lo, float hi) {
+    const __half2 h = __floats2half2_rn(lo, hi);
+    return *reinterpret_cast<const uint32_t*>(&h);
+}
+template <typename T> __device__ __forceinline__ float rounded(float v) { return Pair<T>::lo(pack2<T>(v, v)); }
+
+// the pieces of a launch, in bands of DUAL_GROUP_M row blocks or, SEG, the experts' tiles one after the other
+template <bool SEG>
+__device__ __forceinline__ void piece_coords(int t, int nb_n, int nb_m, int& bm, int& bn) {
+    if constexpr (SEG) {
+        bm = t / nb_n;
+        bn = t - bm * nb_n;
+    } else {
+        const int band = t / (DUAL_GROUP_M * nb_n), r = t - band * (DUAL_GROUP_M * nb_n), rows = min(DUAL_GROUP_M, nb_m - band * DUAL_GROUP_M);
+        bn = r / rows;
+        bm = band * DUAL_GROUP_M + (r - bn * rows);
+    }
+}
+
+template <typename T, bool ROUND, bool EXACT, bool SEG>
+__global__ void __launch_bounds__(256, 2)
+swiglu_row_block_kernel(const T* __restrict__ h12, uint8_t* __restrict__ q_row, float* __restrict__ s_row, uint8_t* __restrict__ q_blk,
+                        float* __restrict__ s_blk, int M, int I, int nb_n, int nb_m, int total, const int* __restrict__ tile_src,
+                        const int* __restrict__ tile_cnt, const int* __restrict__ n_tiles) {
+    __shared__ __align__(16) float s_red[8];
+    __shared__ __align__(16) uint8_t s_out[128 * 128];
+    const int sub = threadIdx.x & 15, hw = threadIdx.x >> 4;
+    pdl_trigger();
+    if constexpr (SEG) total = *n_tiles * nb_n;
+    for (int t = blockIdx.x; t < total; t += gridDim.x) {
+        int bm, bn;
+        piece_coords<SEG>(t, nb_n, nb_m, bm, bn);
+        const int src0 = SEG ? tile_src[bm] : bm * 128, cnt = SEG ? tile_cnt[bm] : min(128, M - bm * 128);
+        const T* p = h12 + (int64_t)(src0 + hw * 8) * (2 * (int64_t)I) + bn * 128 + sub * 8;
+        uint4 a[8], b[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            const bool live = hw * 8 + i < cnt;
+            a[i] = live ? __ldcs(reinterpret_cast<const uint4*>(p + i * 2 * (int64_t)I)) : make_uint4(0u, 0u, 0u, 0u);
+            b[i] = live ? __ldcs(reinterpret_cast<const uint4*>(p + i * 2 * (int64_t)I + I)) : make_uint4(0u, 0u, 0u, 0u);
+        }
+        Raw8x8 raw;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            const uint32_t aw[4] = {a[i].x, a[i].y, a[i].z, a[i].w}, bw[4] = {b[i].x, b[i].y, b[i].z, b[i].w};
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                const float2 x = Pair<T>::both(aw[k]), y = Pair<T>::both(bw[k]);
+                if constexpr (EXACT)
+                    raw.w[i][k] = pack2<T>(rounded<T>(x.x / (1.0f + expf(-x.x))) * y.x, rounded<T>(x.y / (1.0f + expf(-x.y))) * y.y);
+                else
+                    raw.w[i][k] = pack2<T>(__fdividef(x.x, 1.0f + __expf(-x.x)) * y.x, __fdividef(x.y, 1.0f + __expf(-x.y)) * y.y);
+            }
+        }
+        row_block_tile16<T, ROUND, true, SEG>(raw, s_red, s_out, true, q_row, s_row, q_blk, s_blk, M, I, nb_n, bm, bn, [] {}, src0, cnt);
+    }
+}
+
+template <typename T, bool ROUND, bool EXACT, bool SEG>
+__global__ void __launch_bounds__(256, 2)
+swiglu_backward_dual_kernel(const T* __restrict__ h12, const T* __restrict__ dh, uint8_t* __restrict__ q_row, float* __restrict__ s_row,
+                            uint8_t* __restrict__ q_col, float* __restrict__ s_col, int M, int I, int nb_i, int nb_m, int total,
+                            const int* __restrict__ tile_src, const int* __restrict__ tile_cnt, const int* __restrict__ n_tiles) {
+    __shared__ __align__(16) float s_amax[8][128];
+    __shared__ __align__(16) uint8_t s_out[128 * 128];
+    const int sub = threadIdx.x & 15, hw = threadIdx.x >> 4;
+    pdl_trigger();
+    if constexpr (SEG) total = *n_tiles * nb_i;
+    for (int t = blockIdx.x; t < total; t += gridDim.x) {
+        int bm, bn;
+        piece_coords<SEG>(t, nb_i, nb_m, bm, bn);
+        const int src0 = SEG ? tile_src[bm] : bm * 128, cnt = SEG ? tile_cnt[bm] : min(128, M - bm * 128);
+        const int64_t row0 = src0 + hw * 8;
+        const T* p = h12 + row0 * (2 * (int64_t)I) + bn * 128 + sub * 8;
+        const T* pg = dh + row0 * (int64_t)I + bn * 128 + sub * 8;
+        Raw8x8 d1, d2;
+#pragma unroll
+        for (int half = 0; half < 2; ++half) {
+            uint4 a[4], b[4], g[4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const int i = half * 4 + j;
+                const bool live = hw * 8 + i < cnt;
+                a[j] = live ? __ldcs(reinterpret_cast<const uint4*>(p + i * 2 * (int64_t)I)) : make_uint4(0u, 0u, 0u, 0u);
+                b[j] = live ? __ldcs(reinterpret_cast<const uint4*>(p + i * 2 * (int64_t)I + I)) : make_uint4(0u, 0u, 0u, 0u);
+                g[j] = live ? __ldcs(reinterpret_cast<const uint4*>(pg + i * (int64_t)I)) : make_uint4(0u, 0u, 0u, 0u);
+            }
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const uint32_t aw[4] = {a[j].x, a[j].y, a[j].z, a[j].w}, bw[4] = {b[j].x, b[j].y, b[j].z, b[j].w}, gw[4] = {g[j].x, g[j].y, g[j].z, g[j].w};
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    const float2 x = Pair<T>::both(aw[k]), y = Pair<T>::both(bw[k]), z = Pair<T>::both(gw[k]);
+                    float e1[2], e2[2];
+                    const float xs[2] = {x.x, x.y}, ys[2] = {y.x, y.y}, zs[2] = {z.x, z.y};
+#pragma unroll
+                    for (int u = 0; u < 2; ++u) {
+                        const float sig = 1.0f / (1.0f + expf(-xs[u]));
+                        if constexpr (EXACT) {
+                            e1[u] = rounded<T>(zs[u] * ys[u]) * sig * (1.0f + xs[u] * (1.0f - sig));
+                            e2[u] = zs[u] * rounded<T>(xs[u] * sig);
+                        } else {
+                            e1[u] = zs[u] * ys[u] * sig * (1.0f + xs[u] * (1.0f - sig));
+                            e2[u] = zs[u] * xs[u] * sig;
+                        }
+                    }
+                    d1.w[half * 4 + j][k] = pack2<T>(e1[0], e1[1]);
+                    d2.w[half * 4 + j][k] = pack2<T>(e2[0], e2[1]);
+                }
+            }
+        }
+        dual_tile16<T, ROUND, SEG>(d1, s_amax, s_out, true, q_row, s_row, q_col, s_col, M, 2 * I, 2 * nb_i, nb_m, bm, bn, [] {}, src0, cnt);
+        dual_tile16<T, ROUND, SEG>(d2, s_amax, s_out, true, q_row, s_row, q_col, s_col, M, 2 * I, 2 * nb_i, nb_m, bm, bn + nb_i, [] {}, src0, cnt);
     }
 }
 
@@ -1616,41 +2026,65 @@ int requant_row_to_block_padded(const void* xq, const float* xs, int64_t M_in, i
 // row ranges, kb_start[e] = first tile of expert e (kb_start[E] = number of tiles), and per tile its first source row
 // and its number of valid rows.  One CTA.
 // ---------------------------------------------------------------------------
+// All ranges are loaded at once and summed by a scan: one thread adding them up was a chain of loads (32 experts 13 us, so 3).
+constexpr int MAX_SEGMENT_EXPERTS = 1024;
 __global__ void __launch_bounds__(256)
 segment_tiles_kernel(const int64_t* __restrict__ starts, const int64_t* __restrict__ ends, int E, int64_t T,
                      int* __restrict__ kb_start, int* __restrict__ tile_src, int* __restrict__ tile_cnt, int max_tiles) {
-    __shared__ int s_first[1025];
-    if (threadIdx.x == 0) {
-        int run = 0;
-        for (int e = 0; e < E; ++e) {
+    constexpr int PER = MAX_SEGMENT_EXPERTS / 256;         // consecutive experts of a thread
+    __shared__ int s_first[MAX_SEGMENT_EXPERTS + 1], s_src[MAX_SEGMENT_EXPERTS], s_rows[MAX_SEGMENT_EXPERTS];
+    __shared__ long long s_warp[8];
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int per = (E + 255) / 256;                       // at most PER
+    int tiles[PER];
+    long long sum = 0;
+#pragma unroll
+    for (int i = 0; i < PER; ++i) {
+        const int e = tid * per + i;
+        tiles[i] = 0;
+        if (i < per && e < E) {
             long long s = starts[e], t = ends[e];
             if (s < 0) s = 0;
             if (t > T) t = T;
             const int n = t > s ? (int)(t - s) : 0;
-            s_first[e] = run;
-            run += (n + 127) / 128;
-            if (run > max_tiles) run = max_tiles;           // cannot happen for disjoint ranges; keeps every index in range
+            s_src[e] = (int)s;
+            s_rows[e] = n;
+            tiles[i] = (n + 127) / 128;
         }
-        s_first[E] = run;
+        sum += tiles[i];
+    }
+    long long incl = sum;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const long long v = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += v;
+    }
+    if (lane == 31) s_warp[warp] = incl;
+    __syncthreads();
+    long long run = incl - sum;
+    for (int w = 0; w < warp; ++w) run += s_warp[w];
+    // (capped: cannot happen for disjoint ranges; keeps every index in range)
+#pragma unroll
+    for (int i = 0; i < PER; ++i) {
+        const int e = tid * per + i;
+        if (i < per && e < E) s_first[e] = (int)min(run, (long long)max_tiles);
+        run += tiles[i];
+        if (i < per && e == E - 1) s_first[E] = (int)min(run, (long long)max_tiles);
     }
     __syncthreads();
-    for (int e = threadIdx.x; e <= E; e += 256) kb_start[e] = s_first[e];
-    for (int e = 0; e < E; ++e) {
-        long long s = starts[e], t = ends[e];
-        if (s < 0) s = 0;
-        if (t > T) t = T;
-        const int n = t > s ? (int)(t - s) : 0;
+    for (int e = tid; e <= E; e += 256) kb_start[e] = s_first[e];
+    for (int e = warp; e < E; e += 8) {
         const int first = s_first[e], cnt = s_first[e + 1] - first;
-        for (int g = threadIdx.x; g < cnt; g += 256) {
-            tile_src[first + g] = (int)s + g * 128;
-            tile_cnt[first + g] = min(128, n - g * 128);
+        for (int g = lane; g < cnt; g += 32) {
+            tile_src[first + g] = s_src[e] + g * 128;
+            tile_cnt[first + g] = min(128, s_rows[e] - g * 128);
         }
     }
 }
 
 int segment_tiles(const int64_t* starts, const int64_t* ends, int E, int64_t T, int* kb_start, int* tile_src, int* tile_cnt,
                   int max_tiles, cudaStream_t st) {
-    CINN_CHECK_ARG(E >= 1 && E <= 1024 && T >= 0 && T < (1LL << 31) && max_tiles >= 1, "segment_tiles: 1 <= experts <= 1024");
+    CINN_CHECK_ARG(E >= 1 && E <= MAX_SEGMENT_EXPERTS && T >= 0 && T < (1LL << 31) && max_tiles >= 1, "segment_tiles: 1 <= experts <= 1024");
     segment_tiles_kernel<<<1, 256, 0, st>>>(starts, ends, E, T, kb_start, tile_src, tile_cnt, max_tiles);
     CINN_CHECK_LAUNCH();
     return CINN_OK;
@@ -1691,9 +2125,10 @@ int quantize_transposed_segmented(const void* x, int dtype, int64_t M, int64_t L
 
 // dY (T, N) of a 2-byte type -> q_row (T, N) + s_row (T, N / 128) for the rows inside segments, and the transposed,
 // segment-padded quantisation q_col (N, max_tiles * 128) + s_col (N, max_tiles); one pass (quant_row_dual_seg_kernel).
+// block: q_col is the block-scaled copy of the row-wise result instead, s_col (max_tiles, N / 128).
 int quantize_dual_segmented(const void* x, int dtype, int64_t T, int64_t N, void* q_row, float* s_row, void* q_col, float* s_col,
                             int max_tiles, const int* tile_src, const int* tile_cnt, const int* n_tiles, int div_mode,
-                            cudaStream_t st) {
+                            cudaStream_t st, bool block) {
     CINN_CHECK_ARG((dtype == CINN_BF16 || dtype == CINN_F16) && T >= 1 && T < (1LL << 31) && N >= 128 && N % 128 == 0 &&
                    max_tiles >= 1 && max_tiles <= 65535, "segmented dual quantiser: 2-byte input, N a multiple of 128");
     CINN_CHECK_ARG(x && q_row && s_row && q_col && s_col && tile_src && tile_cnt && n_tiles && aligned16(x) && aligned16(q_row) &&
@@ -1705,9 +2140,9 @@ int quantize_dual_segmented(const void* x, int dtype, int64_t T, int64_t N, void
     const int nb_n = (int)(N / 128);
     const int64_t total = (int64_t)nb_n * max_tiles;
     const int grid = (int)(total < 2 * (int64_t)sm_count() ? total : 2 * (int64_t)sm_count());
-#define CINN_DS(TT, DIV)                                                                                              \
+#define CINN_DSM(TT, DIV, MODE)                                                                                              \
     do {                                                                                                              \
-        auto kern = quant_row_dual_seg_kernel<TT, DIV>;                                                               \
+        auto kern = quant_row_dual_seg_kernel<TT, DIV, MODE>;                                                         \
         static std::once_flag once;                                                                                   \
         static cudaError_t attr_err = cudaSuccess;                                                                    \
         std::call_once(once, [&] {                                                                                    \
@@ -1717,9 +2152,11 @@ int quantize_dual_segmented(const void* x, int dtype, int64_t T, int64_t N, void
         kern<<<grid, 256, DUAL_SMEM_BYTES, st>>>(tm, (uint8_t*)q_row, s_row, (uint8_t*)q_col, s_col, max_tiles * 128, (int)N, \
                                                  nb_n, max_tiles, tile_src, tile_cnt, n_tiles);                       \
     } while (0)
+#define CINN_DS(TT, DIV) do { if (block) CINN_DSM(TT, DIV, 2); else CINN_DSM(TT, DIV, 0); } while (0)
     if (dtype == CINN_BF16) { if (div_mode == CINN_DIV_FULL) CINN_DS(__nv_bfloat16, CINN_DIV_FULL); else CINN_DS(__nv_bfloat16, CINN_DIV_RN); }
     else                    { if (div_mode == CINN_DIV_FULL) CINN_DS(__half, CINN_DIV_FULL);        else CINN_DS(__half, CINN_DIV_RN); }
 #undef CINN_DS
+#undef CINN_DSM
     CINN_CHECK_LAUNCH();
     return CINN_OK;
 }
@@ -1750,6 +2187,59 @@ int requant_row_to_block_segmented(const void* xq, const float* xs, int64_t K, v
     else
         requant_row_to_block_kernel<CINN_DIV_RN, true, true><<<grid, 256, 0, st>>>((const uint8_t*)xq, xs, nb, (uint8_t*)out, scales, M, (int)K, nb, M,
                                                                                   tile_src, tile_cnt, n_tiles);
+    CINN_CHECK_LAUNCH();
+    return CINN_OK;
+}
+
+// SwiGLU with the quantisers that follow it: see the kernels.  seg: the experts' tiles (null: one range of all T rows); M is the length of
+// the transposed copies' rows before their rounding up to 16.
+struct SegmentTiles { const int *src, *cnt, *n; int max; };
+
+static int check_swiglu(const void* h12, int dtype, int64_t T, int64_t I, const void* q_row, const void* q_t, const char* what) {
+    CINN_CHECK_ARG(dtype == CINN_BF16 || dtype == CINN_F16, "%s: 2-byte activations", what);
+    CINN_CHECK_ARG(T >= 1 && T <= 65535 * 128 && I >= 128 && I % 128 == 0 && I < (1LL << 30), "%s: rows %lld, hidden width %lld (a multiple of 128)",
+                   what, (long long)T, (long long)I);
+    CINN_CHECK_ARG(h12 && q_row && q_t && aligned16(h12) && aligned16(q_row) && aligned16(q_t), "%s: null or unaligned pointer", what);
+    return CINN_OK;
+}
+
+int swiglu_quant_block(const void* h12, int dtype, int64_t T, int64_t I, void* q_row, float* s_row, void* q_blk, float* s_blk, int round_scale,
+                       const SegmentTiles* seg, cudaStream_t st) {
+    int rc = check_swiglu(h12, dtype, T, I, q_row, q_blk, "swiglu + row + block quantiser");
+    if (rc) return rc;
+    const int nb_n = (int)(I / 128), nb_m = seg ? seg->max : (int)((T + 127) / 128);
+    const int64_t total = (int64_t)nb_n * nb_m, cap = 2 * (int64_t)sm_count();
+    CINN_CHECK_ARG(total < (1LL << 31) && s_row && s_blk && !(seg && round_scale), "swiglu + row + block quantiser: bad arguments");
+    const int grid = (int)(total < cap ? total : cap);
+#define CINN_SB(T_, RND, EXACT, SEG)                                                                                              \
+    swiglu_row_block_kernel<T_, RND, EXACT, SEG><<<grid, 256, 0, st>>>((const T_*)h12, (uint8_t*)q_row, s_row, (uint8_t*)q_blk, s_blk,  \
+        seg ? seg->max * 128 : (int)T, (int)I, nb_n, nb_m, (int)total, seg ? seg->src : nullptr, seg ? seg->cnt : nullptr, seg ? seg->n : nullptr)
+#define CINN_SBT(T_) do { if (seg) CINN_SB(T_, false, false, true); else if (round_scale) CINN_SB(T_, true, true, false); else CINN_SB(T_, false, true, false); } while (0)
+    if (dtype == CINN_BF16) CINN_SBT(__nv_bfloat16);
+    else CINN_SBT(__half);
+#undef CINN_SBT
+#undef CINN_SB
+    CINN_CHECK_LAUNCH();
+    return CINN_OK;
+}
+
+int swiglu_backward_quant_dual(const void* h12, const void* dh, int dtype, int64_t T, int64_t I, void* q_row, float* s_row, void* q_col,
+                               float* s_col, int round_scale, const SegmentTiles* seg, cudaStream_t st) {
+    int rc = check_swiglu(h12, dtype, T, I, q_row, q_col, "swiglu backward + dual quantiser");
+    if (rc) return rc;
+    const int nb_i = (int)(I / 128), nb_m = seg ? seg->max : (int)((T + 127) / 128);
+    const int64_t total = (int64_t)nb_i * nb_m, cap = 2 * (int64_t)sm_count();
+    CINN_CHECK_ARG(total < (1LL << 31) && dh && aligned16(dh) && s_row && s_col && !(seg && round_scale), "swiglu backward + dual quantiser: bad arguments");
+    const int grid = (int)(total < cap ? total : cap);
+#define CINN_SD(T_, RND, EXACT, SEG)                                                                                              \
+    swiglu_backward_dual_kernel<T_, RND, EXACT, SEG><<<grid, 256, 0, st>>>((const T_*)h12, (const T_*)dh, (uint8_t*)q_row, s_row,       \
+        (uint8_t*)q_col, s_col, seg ? seg->max * 128 : (int)T, (int)I, nb_i, nb_m, (int)total, seg ? seg->src : nullptr,               \
+        seg ? seg->cnt : nullptr, seg ? seg->n : nullptr)
+#define CINN_SDT(T_) do { if (seg) CINN_SD(T_, false, false, true); else if (round_scale) CINN_SD(T_, true, true, false); else CINN_SD(T_, false, true, false); } while (0)
+    if (dtype == CINN_BF16) CINN_SDT(__nv_bfloat16);
+    else CINN_SDT(__half);
+#undef CINN_SDT
+#undef CINN_SD
     CINN_CHECK_LAUNCH();
     return CINN_OK;
 }

@@ -91,11 +91,17 @@ int quantize_transposed_segmented(const void* x, int dtype, int64_t M, int64_t L
                                   const int* tile_src, const int* tile_cnt, const int* n_tiles, int div_mode, cudaStream_t st);
 int quantize_dual_segmented(const void* x, int dtype, int64_t T, int64_t N, void* q_row, float* s_row, void* q_col, float* s_col,
                             int max_tiles, const int* tile_src, const int* tile_cnt, const int* n_tiles, int div_mode,
-                            cudaStream_t st);
+                            cudaStream_t st, bool block);
 int requant_row_to_block_segmented(const void* xq, const float* xs, int64_t K, void* out, float* scales, int max_tiles,
                                    const int* tile_src, const int* tile_cnt, const int* n_tiles, int div_mode, cudaStream_t st);
 int fp8_gemm_grouped_k(const void* A, const float* sA, const void* B, const float* sB, const int* kb_start, int64_t E,
                        int64_t M, int64_t N, int64_t max_tiles, void* C, int out_dtype, cudaStream_t st);
+
+struct SegmentTiles { const int *src, *cnt, *n; int max; };      // as in quant.cu
+int swiglu_quant_block(const void* h12, int dtype, int64_t T, int64_t I, void* q_row, float* s_row, void* q_blk, float* s_blk, int round_scale,
+                       const SegmentTiles* seg, cudaStream_t st);
+int swiglu_backward_quant_dual(const void* h12, const void* dh, int dtype, int64_t T, int64_t I, void* q_row, float* s_row, void* q_col,
+                               float* s_col, int round_scale, const SegmentTiles* seg, cudaStream_t st);
 
 static inline int64_t fused_max_tiles(int64_t T, int64_t E) { return (T + 127) / 128 + E; }
 
@@ -105,10 +111,11 @@ int64_t grouped_wgrad_fused_scratch_bytes(int64_t T, int64_t E, int64_t d_in, in
            up(mt * nkb * 4, 256);
 }
 
+// h12: null, or dY is the gradient of silu(h12[:, :I]) * h12[:, I:] (I = d_out / 2) and the derivative of that is taken on the way
 int fp8_grouped_wgrad_fused(const void* dY, int dy_dtype, const void* x_q, const float* x_s, const int64_t* starts_dev,
                             const int64_t* ends_dev, int64_t E, int64_t T, int64_t d_in, int64_t d_out, void* scratch,
                             int64_t scratch_bytes, void* dW, int out_dtype, int div_mode, void* dy_q_row, float* dy_s_row,
-                            cudaStream_t st) {
+                            const void* h12, cudaStream_t st) {
     CINN_CHECK_ARG(E >= 1 && E <= 1024 && T >= 0 && d_in > 0 && d_out > 0, "grouped_wgrad_fused: bad shape");
     CINN_CHECK_ARG((dy_q_row == nullptr) == (dy_s_row == nullptr), "grouped_wgrad_fused: pass both row-wise outputs or neither");
     CINN_CHECK_ARG(dy_q_row == nullptr || dy_dtype == CINN_BF16 || dy_dtype == CINN_F16,
@@ -130,14 +137,84 @@ int fp8_grouped_wgrad_fused(const void* dY, int dy_dtype, const void* x_q, const
     float* b_s = reinterpret_cast<float*>(b_q + up(d_in * mt * 128, 256));
     int rc = segment_tiles(starts_dev, ends_dev, (int)E, T, kb_start, tile_src, tile_cnt, (int)mt, st);
     if (rc) return rc;
-    if (dy_q_row != nullptr)
+    if (h12 != nullptr) {
+        CINN_CHECK_ARG(dy_q_row != nullptr && div_mode == CINN_DIV_FULL && mt <= 65535, "grouped_wgrad_swiglu: needs the row-wise outputs and div.full");
+        const SegmentTiles seg{tile_src, tile_cnt, kb_start + E, (int)mt};
+        rc = swiglu_backward_quant_dual(h12, dY, dy_dtype, T, d_out / 2, dy_q_row, dy_s_row, a_q, a_s, 0, &seg, st);
+    } else if (dy_q_row != nullptr)
         // both quantisations of dY in one pass: the caller's grouped input gradient reads the row-wise one
         rc = quantize_dual_segmented(dY, dy_dtype, T, d_out, dy_q_row, dy_s_row, a_q, a_s, (int)mt, tile_src, tile_cnt, kb_start + E,
-                                     div_mode, st);
+                                     div_mode, st, false);
     else
         rc = quantize_transposed_segmented(dY, dy_dtype, d_out, d_out, a_q, a_s, (int)mt, tile_src, tile_cnt, kb_start + E, div_mode, st);
     if (rc) return rc;
     rc = requant_row_to_block_segmented(x_q, x_s, d_in, b_q, b_s, (int)mt, tile_src, tile_cnt, kb_start + E, div_mode, st);
+    if (rc) return rc;
+    return fp8_gemm_grouped_k(a_q, a_s, b_q, b_s, kb_start, E, d_out, d_in, mt, dW, out_dtype, st);
+}
+
+// ---------------------------------------------------------------------------
+// The same with x's part made by the forward: one pass over x writes its row-wise quantisation (what the forward's GEMM reads) and, into
+// `segments`, the experts' tiles and the block-scaled, transposed copy of that result; the backward keeps `segments` in place
+// of the row-wise bytes.  Same bytes as the calls above.  Layout of `segments`: tiles (ints) | bytes | scales.
+// ---------------------------------------------------------------------------
+static int64_t segment_ints_bytes(int64_t E, int64_t mt) { return up((E + 1 + 2 * mt) * 4, 256); }
+
+int64_t quant_segments_bytes(int64_t T, int64_t E, int64_t d) {
+    const int64_t mt = fused_max_tiles(T < 0 ? 0 : T, E < 0 ? 0 : E);
+    return segment_ints_bytes(E, mt) + up(d * mt * 128, 256) + up(mt * ((d + 127) / 128) * 4, 256);
+}
+
+// swiglu: x is (T, 2 * d) and what is quantised is silu(x[:, :d]) * x[:, d:]
+int quantize_row_segments(const void* x, int dtype, int64_t T, int64_t d, const int64_t* starts_dev, const int64_t* ends_dev, int64_t E,
+                          void* q_row, float* s_row, void* segments, int64_t segments_bytes, int div_mode, bool swiglu, cudaStream_t st) {
+    CINN_CHECK_ARG(E >= 1 && E <= 1024 && T >= 1 && T < (1LL << 31) && d > 0, "quant_rowwise_segments: bad shape");
+    CINN_CHECK_ARG(starts_dev && ends_dev && segments && (reinterpret_cast<uintptr_t>(segments) & 255) == 0 &&
+                   segments_bytes >= quant_segments_bytes(T, E, d), "quant_rowwise_segments: null, unaligned or short buffer");
+    CINN_CHECK_ARG(div_mode == CINN_DIV_FULL || div_mode == CINN_DIV_RN, "quant_rowwise_segments: unknown div_mode %d", div_mode);
+    const int64_t mt = fused_max_tiles(T, E);
+    CINN_CHECK_ARG(mt <= 65535, "quant_rowwise_segments: too many rows");
+    int* kb_start = static_cast<int*>(segments);
+    int *tile_src = kb_start + (E + 1), *tile_cnt = tile_src + mt;
+    uint8_t* b_q = static_cast<uint8_t*>(segments) + segment_ints_bytes(E, mt);
+    int rc = segment_tiles(starts_dev, ends_dev, (int)E, T, kb_start, tile_src, tile_cnt, (int)mt, st);
+    if (rc) return rc;
+    if (swiglu) {
+        CINN_CHECK_ARG(div_mode == CINN_DIV_FULL, "swiglu_quant_segments: div.full only");
+        const SegmentTiles seg{tile_src, tile_cnt, kb_start + E, (int)mt};
+        return swiglu_quant_block(x, dtype, T, d, q_row, s_row, b_q, reinterpret_cast<float*>(b_q + up(d * mt * 128, 256)), 0, &seg, st);
+    }
+    return quantize_dual_segmented(x, dtype, T, d, q_row, s_row, b_q, reinterpret_cast<float*>(b_q + up(d * mt * 128, 256)), (int)mt, tile_src,
+                                   tile_cnt, kb_start + E, div_mode, st, true);
+}
+
+int64_t grouped_wgrad_segments_scratch_bytes(int64_t T, int64_t E, int64_t d_out) {
+    const int64_t mt = fused_max_tiles(T < 0 ? 0 : T, E < 0 ? 0 : E);
+    return up(d_out * mt * 128, 256) + up(d_out * mt * 4, 256);
+}
+
+int fp8_grouped_wgrad_segments(const void* dY, int dy_dtype, const void* segments, int64_t E, int64_t T, int64_t d_in, int64_t d_out,
+                               void* scratch, int64_t scratch_bytes, void* dW, int out_dtype, int div_mode, void* dy_q_row, float* dy_s_row,
+                               cudaStream_t st) {
+    CINN_CHECK_ARG(E >= 1 && E <= 1024 && T >= 1 && d_in > 0 && d_out > 0, "grouped_wgrad_segments: bad shape");
+    CINN_CHECK_ARG((dy_q_row == nullptr) == (dy_s_row == nullptr), "grouped_wgrad_segments: pass both row-wise outputs or neither");
+    CINN_CHECK_ARG(dy_q_row == nullptr || dy_dtype == CINN_BF16 || dy_dtype == CINN_F16,
+                   "grouped_wgrad_segments: the row-wise quantisation of dY comes with 2-byte gradients only");
+    CINN_CHECK_ARG(d_in % 256 == 0 && d_out % 256 == 0, "grouped_wgrad_segments: d_in (%lld) and d_out (%lld) must be multiples of 256",
+                   (long long)d_in, (long long)d_out);
+    CINN_CHECK_ARG(dY && segments && scratch && dW && (reinterpret_cast<uintptr_t>(segments) & 255) == 0 &&
+                   (reinterpret_cast<uintptr_t>(scratch) & 255) == 0 && scratch_bytes >= grouped_wgrad_segments_scratch_bytes(T, E, d_out),
+                   "grouped_wgrad_segments: null, unaligned or short buffer");
+    const int64_t mt = fused_max_tiles(T, E);
+    const int* kb_start = static_cast<const int*>(segments);
+    const int *tile_src = kb_start + (E + 1), *tile_cnt = tile_src + mt;
+    const uint8_t* b_q = static_cast<const uint8_t*>(segments) + segment_ints_bytes(E, mt);
+    const float* b_s = reinterpret_cast<const float*>(b_q + up(d_in * mt * 128, 256));
+    uint8_t* a_q = static_cast<uint8_t*>(scratch);
+    float* a_s = reinterpret_cast<float*>(a_q + up(d_out * mt * 128, 256));
+    const int rc = dy_q_row != nullptr
+        ? quantize_dual_segmented(dY, dy_dtype, T, d_out, dy_q_row, dy_s_row, a_q, a_s, (int)mt, tile_src, tile_cnt, kb_start + E, div_mode, st, false)
+        : quantize_transposed_segmented(dY, dy_dtype, d_out, d_out, a_q, a_s, (int)mt, tile_src, tile_cnt, kb_start + E, div_mode, st);
     if (rc) return rc;
     return fp8_gemm_grouped_k(a_q, a_s, b_q, b_s, kb_start, E, d_out, d_in, mt, dW, out_dtype, st);
 }

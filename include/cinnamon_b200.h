@@ -248,6 +248,39 @@ int cinn_fp8_grouped_wgrad_fused(const void* dY, int dy_dtype, const void* x_q, 
                                  void* scratch, int64_t scratch_bytes, void* dW, int out_dtype, int div_mode, void* dy_q_row,
                                  float* dy_row_scales, void* stream);
 
+/* The same with x's part made by the forward.  cinn_quant_rowwise_segments quantises x (T, d) of a 2-byte type (d a multiple of 128)
+ * row-wise for the rows inside expert ranges - q_row (T, d), s_row (T, d / 128), other rows are left alone - and writes into
+ * `segments` what the weight gradient reads of x (the experts' tiles and the block-scaled, transposed copy of that result);
+ * cinn_fp8_grouped_wgrad_segments takes it in place of x_q, x_scales and the ranges.  Same bytes as cinn_quant_rowwise and
+ * cinn_fp8_grouped_wgrad_fused.  T + 127 * E at most about 8 million rows; segments and scratch 256-byte aligned. */
+int64_t cinn_quant_segments_bytes(int64_t T, int64_t E, int64_t d);
+int cinn_quant_rowwise_segments(const void* x, int x_dtype, int64_t T, int64_t d, const int64_t* starts, const int64_t* ends, int64_t E,
+                                void* q_row, float* s_row, void* segments, int64_t segments_bytes, int div_mode, void* stream);
+int64_t cinn_fp8_grouped_wgrad_segments_scratch_bytes(int64_t T, int64_t E, int64_t d_out);
+int cinn_fp8_grouped_wgrad_segments(const void* dY, int dy_dtype, const void* segments, int64_t E, int64_t T, int64_t d_in, int64_t d_out,
+                                    void* scratch, int64_t scratch_bytes, void* dW, int out_dtype, int div_mode, void* dy_q_row,
+                                    float* dy_s_row, void* stream);
+
+/* SwiGLU inside the quantisers around it (bf16 or fp16 activations, CINN_DIV_FULL): the bytes of the separate calls, without the
+ * activations going through memory in between.  h12 is (T, 2 * I) with the gate half first, I a multiple of 128, T at most 8388480; the
+ * transposed copies' rows are T rounded up to 16 long with zeros behind T.
+ *   cinn_swiglu_rounded_quant_block_t:       cinn_swiglu_rounded, then cinn_quant_rowwise_with_block_t_padded (src/layers.py:15-31)
+ *   cinn_swiglu_rounded_backward_quant_dual: cinn_swiglu_rounded_backward, then cinn_quant_rowwise_dual_padded of its (T, 2 * I) result
+ *   cinn_swiglu_quant_segments:              cinn_swiglu_quant_rowwise, with `segments` of its result as cinn_quant_rowwise_segments
+ *                                            leaves them (src/layers.py:71-74)
+ *   cinn_fp8_grouped_wgrad_swiglu:           cinn_swiglu_backward, then cinn_fp8_grouped_wgrad_fused of its result (d_out = 2 * I);
+ *                                            q_row (total_rows, 2 * I) and row_scales are not optional */
+int cinn_swiglu_rounded_quant_block_t(const void* h12, int dtype, int64_t T, int64_t I, void* q_row, float* s_row, void* q_block_t,
+                                      float* s_block, int round_scale, void* stream);
+int cinn_swiglu_rounded_backward_quant_dual(const void* h12, const void* dh, int dtype, int64_t T, int64_t I, void* q_row, float* s_row,
+                                            void* q_col, float* s_col, int round_scale, void* stream);
+int cinn_swiglu_quant_segments(const void* h12, int dtype, int64_t T, int64_t I, const int64_t* starts, const int64_t* ends, int64_t E,
+                               void* q_row, float* s_row, void* segments, int64_t segments_bytes, void* stream);
+int cinn_fp8_grouped_wgrad_swiglu(const void* h12, const void* dh, int dtype, const void* x_q, const float* x_scales,
+                                  const int64_t* expert_starts, const int64_t* expert_ends, int64_t n_experts, int64_t total_rows, int64_t d_in,
+                                  int64_t I, void* scratch, int64_t scratch_bytes, void* dW, int out_dtype, void* q_row, float* row_scales,
+                                  void* stream);
+
 /* y[t, :] = sum_j gates[t, j] * rows[pos[t, j], :]  for t < n_tokens, j < top_k; fp32 result, no atomics.
  * Replaces the gate multiply, torch.zeros and scatter_add_ at the end of MoE.forward (src/layers.py:157-160).
  * rows: (n_rows, d) bf16 / fp16 / fp32.  pos: (n_tokens, top_k) int64 row indices (negative = skip), ascending per

@@ -332,3 +332,157 @@ def test_linear_gradients_of_ragged_and_unaligned_tokens(K, M, off):
         gx, gw = torch.autograd.grad(lin(xs), [xs, lin.weight], ds)
         grads.append((gx[:M], gw))
     assert torch.equal(grads[0][0], grads[1][0]) and torch.equal(grads[0][1], grads[1][1])
+
+
+def _pieces(M, N, kind, dtype, seed):
+    x = torch.randn(M, N, device="cuda", generator=torch.Generator(device="cuda").manual_seed(seed)).mul_(3)
+    if kind == "special":
+        x[M // 3, N // 2], x[M // 2, 5], x[0, N - 1] = float("nan"), float("inf"), -float("inf")
+    elif kind == "huge":
+        x.mul_(6e4 if dtype == torch.float16 else 1e38).clamp_(-6.5e4 if dtype == torch.float16 else -3.38e38, 6.5e4 if dtype == torch.float16 else 3.38e38)
+    elif kind == "tiny":
+        x.mul_(1e-7)
+    return x.to(dtype)
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("kind", ["normal", "special", "huge", "tiny"])
+@pytest.mark.parametrize("M,N,rs", [(144, 272, False), (400, 640, True), (128, 128, True)])
+def test_packed_passes_against_the_separate_quantisers(K, M, N, rs, kind, dtype):
+    """The dual and the row + block pass on 2-byte inputs with div.full, also where a piece holds NaN or infinity or its decoded
+    values overflow: the bytes and scales of the separate quantisers."""
+    x, mode = _pieces(M, N, kind, dtype, M + N), K.get_div_mode()
+    K.set_div_mode("full")
+    try:
+        q, s, qt, st = K.quantize_fp8_rowwise_dual(x, rs)
+        rq, r_s = K.quantize_fp8_rowwise(x, 128, rs)
+        cq, c_s = K.quantize_fp8_rowwise(x.t().contiguous(), 128, rs)
+        b8 = lambda t: t.contiguous().view(torch.uint8)                                       # noqa: E731
+        assert torch.equal(b8(q), b8(rq)) and torch.equal(s, r_s) and torch.equal(b8(qt), b8(cq)) and torch.equal(st, c_s)
+        bq, b_s = K.requantize_rowwise_to_blockwise(rq, r_s)
+        for t in (False, True):
+            q2, s2, blk, bs = K.quantize_fp8_rowwise_with_block(x, rs, transpose_block=t)
+            assert torch.equal(b8(q2), b8(rq)) and torch.equal(s2, r_s) and torch.equal(bs, b_s)
+            assert torch.equal(b8(blk.t() if t else blk), b8(bq))
+    finally:
+        K.set_div_mode(mode)
+
+
+def _ranges(counts):
+    ends = torch.tensor(counts, device="cuda").cumsum(0)
+    return ends - torch.tensor(counts, device="cuda"), ends
+
+
+def _segment_parts(K, buf, T, E, d):
+    mt = (T + 127) // 128 + E
+    up = lambda n: (n + 255) // 256 * 256                                                     # noqa: E731
+    o = up((E + 1 + 2 * mt) * 4)
+    n = int(buf[:4 * (E + 1)].view(torch.int32)[E])                                           # tiles that exist
+    q = buf[o:o + d * mt * 128].view(d, mt * 128)[:, :n * 128]
+    s = buf[o + up(d * mt * 128):][:4 * mt * (d // 128)].view(torch.float32).view(mt, d // 128)[:n]
+    return buf[:4 * (E + 1)].view(torch.int32), q, s
+
+
+def _segment_reference(K, q, s, starts, ends, d):
+    cols, scales = [], []
+    for a, b in zip(starts.tolist(), ends.tolist()):
+        if b <= a:
+            continue
+        pad = -(b - a) % 128
+        qe = torch.nn.functional.pad(q[a:b].view(torch.uint8), (0, 0, 0, pad)).view(torch.float8_e4m3fn)
+        se = torch.nn.functional.pad(s[a:b], (0, 0, 0, pad), value=1.0)
+        bq, bs = K.requantize_rowwise_to_blockwise(qe, se)
+        cols.append(bq.view(torch.uint8).t())
+        scales.append(bs)
+    return torch.cat(cols, 1), torch.cat(scales)
+
+
+@pytest.mark.parametrize("counts", [[5, 0, 128, 129, 300], [1], [0, 0, 640], [40] * 33])
+@pytest.mark.parametrize("swiglu,kind", [(False, "normal"), (False, "special"), (True, "normal")])
+def test_row_quantiser_with_segments(K, counts, swiglu, kind):
+    """x, or SwiGLU of it, quantised row-wise with the experts' block copies from one pass: the separate calls' bytes, scales and tiles."""
+    T, d, E, mode = sum(counts), 256, len(counts), K.get_div_mode()
+    x = _pieces(T, 2 * d if swiglu else d, kind if T > 10 else "normal", torch.bfloat16, T)
+    starts, ends = _ranges(counts)
+    K.set_div_mode("full")
+    try:
+        q, s = torch.zeros(T, d, device="cuda", dtype=torch.float8_e4m3fn), torch.zeros(T, d // 128, device="cuda")
+        buf = torch.empty(K._L.cinn_quant_segments_bytes(T, E, d), device="cuda", dtype=torch.uint8)
+        common = (T, d, K._ptr(starts), K._ptr(ends), E, K._ptr(q), K._ptr(s), K._ptr(buf), buf.numel())
+        if swiglu:
+            assert K._L.cinn_swiglu_quant_segments(K._ptr(x), 0, *common, K._stream(x)) == 0
+            rq, r_s = K.swiglu_quantize_rowwise(x)
+        else:
+            assert K._L.cinn_quant_rowwise_segments(K._ptr(x), 0, *common, K._DIV_MODE, K._stream(x)) == 0
+            rq, r_s = K.quantize_fp8_rowwise(x)
+        first, bq, bs = _segment_parts(K, buf, T, E, d)
+        ref_q, ref_s = _segment_reference(K, rq, r_s, starts, ends, d)
+    finally:
+        K.set_div_mode(mode)
+    tiles = (torch.tensor(counts, device="cuda") + 127) // 128
+    assert first.tolist() == [0] + tiles.cumsum(0).tolist()
+    assert torch.equal(q.view(torch.uint8), rq.view(torch.uint8)) and torch.equal(s, r_s)
+    assert torch.equal(bq, ref_q) and torch.equal(bs, ref_s)
+
+
+@pytest.mark.parametrize("T,I,rs", [(1, 128, False), (130, 256, True), (517, 384, False)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_swiglu_inside_the_quantisers(K, T, I, rs, dtype):
+    """SwiGLU with the quantisers of a linear around it, forward and backward, against the separate calls: the same bytes."""
+    g = torch.Generator(device="cuda").manual_seed(T)
+    h12, dh = (torch.randn(T, n, device="cuda", generator=g).mul_(2).to(dtype) for n in (2 * I, I))
+    tag, mode, Tp = K._DTYPE_TAG[dtype], K.get_div_mode(), (T + 15) // 16 * 16
+    e8 = lambda *n: torch.empty(*n, device="cuda", dtype=torch.float8_e4m3fn)                 # noqa: E731
+    e4 = lambda *n: torch.empty(*n, device="cuda")                                            # noqa: E731
+    nb, nbi = (T + 127) // 128, I // 128
+    K.set_div_mode("full")
+    try:
+        h, dh12 = torch.empty(T, I, device="cuda", dtype=dtype), torch.empty(T, 2 * I, device="cuda", dtype=dtype)
+        assert K._L.cinn_swiglu_rounded(K._ptr(h12), K._ptr(h), tag, T, I, K._stream(h)) == 0
+        want = K.quantize_fp8_rowwise_with_block(h, rs, transpose_block=True, _padded=True)
+        got = (e8(T, I), e4(T, nbi), e8(I, Tp), e4(nb, nbi))
+        assert K._L.cinn_swiglu_rounded_quant_block_t(K._ptr(h12), tag, T, I, *map(K._ptr, got), int(rs), K._stream(h)) == 0
+        for a, b in zip(got, want):
+            assert torch.equal(a.view(torch.uint8), b.view(torch.uint8))
+        assert K._L.cinn_swiglu_rounded_backward(K._ptr(h12), K._ptr(dh), K._ptr(dh12), tag, T, I, K._stream(h)) == 0
+        want = K._quantize_dual_padded(dh12, rs)
+        got = (e8(T, 2 * I), e4(T, 2 * nbi), e8(2 * I, Tp), e4(2 * I, nb))
+        assert K._L.cinn_swiglu_rounded_backward_quant_dual(K._ptr(h12), K._ptr(dh), tag, T, I, *map(K._ptr, got), int(rs), K._stream(h)) == 0
+        for a, b in zip(got, want):
+            assert torch.equal(a.view(torch.uint8), b.view(torch.uint8))
+    finally:
+        K.set_div_mode(mode)
+
+
+@pytest.mark.parametrize("counts", [[5, 0, 128, 129, 300], [64] * 9])
+def test_grouped_weight_gradient_with_swiglu(K, counts):
+    """The experts' weight gradient and the row-wise operand of the input gradient with SwiGLU's derivative on the way: as after the
+    separate kernel."""
+    T, E, d, I, mode = sum(counts), len(counts), 256, 256, K.get_div_mode()
+    g = torch.Generator(device="cuda").manual_seed(T)
+    h12, dh, x = (torch.randn(T, n, device="cuda", generator=g).to(torch.bfloat16) for n in (2 * I, I, d))
+    starts, ends = _ranges(counts)
+    K.set_div_mode("full")
+    try:
+        xq, xs = K.quantize_fp8_rowwise(x)
+        need = K._L.cinn_fp8_grouped_wgrad_fused_scratch_bytes(T, E, d, 2 * I)
+        ws = torch.empty(need, device="cuda", dtype=torch.uint8)
+        dh12 = torch.empty_like(h12)
+        assert K._L.cinn_swiglu_backward(K._ptr(h12), K._ptr(dh), K._ptr(dh12), 0, T, I, K._stream(x)) == 0
+        res = []
+        for fused in (False, True):
+            q, s = torch.zeros(T, 2 * I, device="cuda", dtype=torch.uint8), torch.zeros(T, 2 * I // 128, device="cuda")
+            dw = torch.empty(E, 2 * I, d, device="cuda")
+            tail = (K._ptr(xq), K._ptr(xs), K._ptr(starts), K._ptr(ends), E, T, d)
+            if fused:
+                rc = K._L.cinn_fp8_grouped_wgrad_swiglu(K._ptr(h12), K._ptr(dh), 0, *tail, I, K._ptr(ws), need, K._ptr(dw), 1, K._ptr(q), K._ptr(s),
+                                                        K._stream(x))
+            else:
+                rc = K._L.cinn_fp8_grouped_wgrad_fused(K._ptr(dh12), 0, *tail, 2 * I, K._ptr(ws), need, K._ptr(dw), 1, K._DIV_MODE, K._ptr(q), K._ptr(s),
+                                                       K._stream(x))
+            assert rc == 0
+            res.append((q, s, dw))
+    finally:
+        K.set_div_mode(mode)
+    for a, b in zip(*res):
+        assert torch.equal(a, b)
