@@ -159,28 +159,6 @@ __device__ __forceinline__ void store_parts16(uint32_t rest, uint32_t lead, cons
 // A panel used K-major (its 64 columns are the reduction axis; a step of four takes 16 of them: 32 bytes) and MN-major (its 128
 // rows are; a step of eight takes 16 of them: 2048 bytes).  Both have one descriptor, of which only the low word (the address in
 // units of 16 bytes) varies.
-constexpr uint32_t DESC_HI = (uint32_t)((((uint64_t)(1024 >> 4) << 32) | (1ull << 46) | (2ull << 61)) >> 32);
-__device__ __forceinline__ uint32_t panel_desc(uint32_t panel) { return ((panel >> 4) & 0x3FFFu) | (1u << 16); }
-
-// One warp issues all MMAs, so what it does between two of them is time the tensor core waits.  A panel's steps are one
-// statement with one election: issued one by one, with 64-bit descriptors, a panel of four cost the warp 350 cycles where
-// the MMAs take 256; like this 257.
-// D (+)= A B over the 64 columns of two K-major panels; the first step overwrites D when `fresh`
-__device__ __forceinline__ void mma_panels(uint32_t d, uint32_t a, uint32_t b, uint32_t idesc, bool fresh) {
-    asm volatile(
-        "{\n\t.reg .pred p, e;\n\t.reg .b64 a, b;\n\t.reg .b32 x, y;\n\t"
-        "elect.sync _|e, 0xffffffff;\n\t"
-        "setp.ne.b32 p, %5, 0;\n\t"
-        "mov.b64 a, {%1, %4};\n\tmov.b64 b, {%2, %4};\n\t"
-        "@e tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %3, p;\n\t"
-        "add.u32 x, %1, 2;\n\tadd.u32 y, %2, 2;\n\tmov.b64 a, {x, %4};\n\tmov.b64 b, {y, %4};\n\t"
-        "@e tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %3, 1;\n\t"
-        "add.u32 x, %1, 4;\n\tadd.u32 y, %2, 4;\n\tmov.b64 a, {x, %4};\n\tmov.b64 b, {y, %4};\n\t"
-        "@e tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %3, 1;\n\t"
-        "add.u32 x, %1, 6;\n\tadd.u32 y, %2, 6;\n\tmov.b64 a, {x, %4};\n\tmov.b64 b, {y, %4};\n\t"
-        "@e tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %3, 1;\n\t}"
-        ::"r"(d), "r"(a), "r"(b), "r"(idesc), "r"(DESC_HI), "r"(fresh ? 0u : 1u) : "memory");
-}
 
 // D (+)= part X of a tensor-memory operand of 16 STEPS positions (store_parts16) times an MN-major panel
 template <int X, int STEPS = 8>

@@ -577,6 +577,27 @@ int encode_map_2d(CUtensorMap* map, const void* base, uint64_t inner, uint64_t r
 
 // 3-D map: `planes` matrices of (rows, inner), boxes of box_inner columns x box_rows of one matrix; rows past a matrix's end
 // read as zeros instead of its neighbour's, and are not written
+int encode_map(CUtensorMap* map, const void* base, uint32_t rank, const uint64_t* dims, const uint64_t* strides, const uint32_t* box,
+               CUtensorMapDataType dtype, CUtensorMapSwizzle swizzle) {
+    EncodeFn enc = get_encode();
+    if (!enc) { set_error("cuTensorMapEncodeTiled is not available from the CUDA driver"); return CINN_ERR_CUDA; }
+    const cuuint32_t ones[5] = {1, 1, 1, 1, 1};
+    cuuint64_t d[5], st[4];
+    cuuint32_t bx[5];
+    for (uint32_t i = 0; i < rank; ++i) { d[i] = dims[i]; bx[i] = box[i]; if (i) st[i - 1] = strides[i - 1]; }
+    auto go = [&] {
+        return enc(map, dtype, rank, const_cast<void*>(base), d, st, bx, ones, CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle,
+                   CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    };
+    CUresult r = go();
+    if (r == CUDA_ERROR_INVALID_CONTEXT || r == CUDA_ERROR_NOT_INITIALIZED) { cudaFree(nullptr); r = go(); }
+    if (r != CUDA_SUCCESS) {
+        set_error("cuTensorMapEncodeTiled failed with CUresult %d (base %p, %u dimensions)", (int)r, base, rank);
+        return CINN_ERR_CUDA;
+    }
+    return CINN_OK;
+}
+
 int encode_map_3d(CUtensorMap* map, const void* base, uint64_t inner, uint64_t rows, uint64_t planes, uint64_t pitch_bytes,
                   uint32_t box_rows, CUtensorMapDataType dtype, uint32_t box_inner, CUtensorMapSwizzle swizzle) {
     EncodeFn enc = get_encode();

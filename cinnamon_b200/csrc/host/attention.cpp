@@ -73,6 +73,19 @@ std::tuple<Tensor, Tensor, Tensor> backward(const Tensor& grad_out, const Tensor
     return {gq.to(in), gk.to(in), gv.to(in)};
 }
 
+// Lightning indexer logits (reference src/kernels.py:392-433); q (B, Lq, H, d), k (B, Lk, d), w (B, Lq, H), any strides
+Tensor indexer(const Tensor& q_in, const Tensor& k_in, const Tensor& w_in) {
+    require(q_in.is_cuda() && k_in.is_cuda() && w_in.is_cuda(), "Inputs must be on CUDA");
+    c10::cuda::CUDAGuard guard(q_in.device());
+    const at::ScalarType in = q_in.scalar_type(), work = tag_of(in) < 0 ? at::kFloat : in;
+    const Tensor q = q_in.to(work), k = k_in.to(work), w = w_in.to(work);
+    Tensor out = empty({q.size(0), q.size(1), k.size(1)}, at::kHalf, q.device());
+    check(api.cinn_lightning_indexer(q.data_ptr(), k.data_ptr(), w.data_ptr(), tag_of(work), out.data_ptr(), q.size(0), q.size(1), k.size(1),
+                                     q.size(2), q.size(3), q.strides().data(), k.strides().data(), w.strides().data(), stream()),
+          "cinn_lightning_indexer");
+    return out;
+}
+
 class AttentionNode : public torch::autograd::Function<AttentionNode> {
 public:
     static torch::autograd::variable_list forward(torch::autograd::AutogradContext* ctx, const Tensor& q, const Tensor& k, const Tensor& v,
@@ -98,6 +111,7 @@ public:
 }  // namespace
 
 void bind_attention(pybind11::module_& m) {
+    m.def("indexer", &indexer);
     // (out, attention weights, then what the backward takes: q, k, v, idx, out in fp32, lse)
     m.def("attention_forward", [](const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& idx, double scale) {
         Attention r = forward(q, k, v, idx, scale);

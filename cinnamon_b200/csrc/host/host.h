@@ -24,6 +24,7 @@ using at::Tensor;
     X(cinn_last_error) X(cinn_quant_rowwise) X(cinn_quant_rowwise_dual) X(cinn_quant_rowwise_with_block)             \
     X(cinn_quant_rowwise_with_block_t) X(cinn_quant_rowwise_dual_padded) X(cinn_quant_rowwise_with_block_t_padded) X(cinn_quant_blockwise) X(cinn_quant_block_beside) X(cinn_quant_linear) X(cinn_transpose_bytes)     \
     X(cinn_requant_row_to_block) X(cinn_fp8_gemm_ws) X(cinn_fp8_gemm_pitched) X(cinn_fp8_gemm_workspace_bytes) \
+    X(cinn_lightning_indexer)                                                                                           \
     X(cinn_sparse_attn_workspace_bytes) X(cinn_sparse_attn_fwd_ws) X(cinn_sparse_attn_bwd) X(cinn_sparse_attn_bwd_ws)                  \
     X(cinn_fp8_linear_few_takes) X(cinn_fp8_linear_few)                                                                   \
     X(cinn_moe_route_workspace_ints) X(cinn_moe_route_ranges) X(cinn_spread_rows) X(cinn_fp8_grouped_gemm)                \

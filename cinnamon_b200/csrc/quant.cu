@@ -954,13 +954,15 @@ quant_row_dual_seg_kernel(const __grid_constant__ CUtensorMap tmX, uint8_t* __re
 // SwiGLU inside the quantisers that follow it (16-bit activations, products of div.full): its result does not go to memory in
 // between.  h12 is (rows, 2 * I), the gate half first.
 //   swiglu_row_block_kernel     forward: h = silu(h1) * h2, row-wise and, in blocks, transposed (row_block_tile16).
-//                               32768 x 2 x 1024: 46 us of SwiGLU and 29 of the quantiser, as one pass %FWD%
-//   swiglu_backward_dual_kernel backward: both halves of dh12 from h12 and dh, along both axes (dual_tile16).  56 and 52 us, so %BWD%
+//                               32768 x 2 x 1024: 46 us of SwiGLU and 29 of the quantiser, as one pass 67
+//   swiglu_backward_dual_kernel backward: both halves of dh12 from h12 and dh, along both axes (dual_tile16).  56 and 52 us, so 106, with a launch
+//                               and 268 MB less
 // Values are rounded to the activation type where the separate kernels round them, so the bytes are theirs.
 // EXACT: silu by the exact sequences, rounded by itself before the product (the shared expert's layers); else a few fp32 ulp off, not
 // rounded by itself (the routed experts': see swiglu_quant_row_kernel) in the forward, exact and unrounded in the backward.
 // SEG: pieces are tiles of the experts' segments, as in quant_row_dual_seg_kernel.
-// Bound by memory with the loads of a piece, 32 or 48 KiB of a CTA, in registers; two CTAs per SM load and convert in turn.
+// Bound by the exact exponentials and quotients, 40 instructions per element, with the loads of a piece, 32 or 48 KiB of a CTA, in
+// registers; two CTAs per SM load and convert in turn (three, of 80 registers: no faster, nor the dual quantisers so).
 // ---------------------------------------------------------------------------
 template <typename T> __device__ __forceinline__ uint32_t pack2(float lo, float hi);
 template <> __device__ __forceinline__ uint32_t pack2<__nv_bfloat16>(float lo, float hi) {

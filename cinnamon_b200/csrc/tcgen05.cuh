@@ -87,6 +87,31 @@ __host__ __device__ constexpr uint32_t make_idesc_f16(bool bf16, int m, int n, b
            | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(m >> 4) << 24);
 }
 
+// Operands in panels: 128 rows (or as many as the other side has) of 128 bytes, 128-byte swizzle.  The low word of a panel's descriptor;
+// the high one is the same for all.
+constexpr uint32_t DESC_HI = (uint32_t)((((uint64_t)(1024 >> 4) << 32) | (1ull << 46) | (2ull << 61)) >> 32);
+__device__ __forceinline__ uint32_t panel_desc(uint32_t panel) { return ((panel >> 4) & 0x3FFFu) | (1u << 16); }
+
+// One warp issues all MMAs, so what it does between two of them is time the tensor core waits.  A panel's steps are one
+// statement with one election: issued one by one, with 64-bit descriptors, a panel of four cost the warp 350 cycles where
+// the MMAs take 256; like this 257.
+// D (+)= A B over the 64 columns of two K-major panels; the first step overwrites D when `fresh`
+__device__ __forceinline__ void mma_panels(uint32_t d, uint32_t a, uint32_t b, uint32_t idesc, bool fresh) {
+    asm volatile(
+        "{\n\t.reg .pred p, e;\n\t.reg .b64 a, b;\n\t.reg .b32 x, y;\n\t"
+        "elect.sync _|e, 0xffffffff;\n\t"
+        "setp.ne.b32 p, %5, 0;\n\t"
+        "mov.b64 a, {%1, %4};\n\tmov.b64 b, {%2, %4};\n\t"
+        "@e tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %3, p;\n\t"
+        "add.u32 x, %1, 2;\n\tadd.u32 y, %2, 2;\n\tmov.b64 a, {x, %4};\n\tmov.b64 b, {y, %4};\n\t"
+        "@e tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %3, 1;\n\t"
+        "add.u32 x, %1, 4;\n\tadd.u32 y, %2, 4;\n\tmov.b64 a, {x, %4};\n\tmov.b64 b, {y, %4};\n\t"
+        "@e tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %3, 1;\n\t"
+        "add.u32 x, %1, 6;\n\tadd.u32 y, %2, 6;\n\tmov.b64 a, {x, %4};\n\tmov.b64 b, {y, %4};\n\t"
+        "@e tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %3, 1;\n\t}"
+        ::"r"(d), "r"(a), "r"(b), "r"(idesc), "r"(DESC_HI), "r"(fresh ? 0u : 1u) : "memory");
+}
+
 // 32 lanes x 16 consecutive fp32 columns: thread i receives TMEM lane (base lane + i)
 __device__ __forceinline__ void tc_ld16(uint32_t taddr, float (&v)[16]) {
     uint32_t r[16];

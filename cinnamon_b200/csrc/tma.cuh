@@ -51,4 +51,8 @@ int encode_map_3d(CUtensorMap* map, const void* base, uint64_t inner, uint64_t r
                   uint32_t box_rows, CUtensorMapDataType dtype, uint32_t box_inner = 64,
                   CUtensorMapSwizzle swizzle = CU_TENSOR_MAP_SWIZZLE_128B);
 
+// any rank: `strides` in bytes, of the dimensions after the first
+int encode_map(CUtensorMap* map, const void* base, uint32_t rank, const uint64_t* dims, const uint64_t* strides, const uint32_t* box,
+               CUtensorMapDataType dtype, CUtensorMapSwizzle swizzle);
+
 }  // namespace cinn

@@ -76,3 +76,42 @@ def test_tile_edges(shape, dtype):
     got = K.lightning_indexer_fused(q.cuda(), k.cuda(), w.cuda())
     _close_fp16(got.cpu(), SO.lightning_indexer(q, k, w))
     assert K.device_status() == 0
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("shape", [(1, 1, 1, 1, 8), (2, 300, 517, 9, 64), (3, 129, 1000, 4, 128), (20, 260, 391, 2, 64), (1, 2000, 1537, 3, 72),
+                                   (4, 200, 136, 10, 64)])
+def test_runs_of_tiles(shape, dtype):
+    """CTAs with several tiles: runs that cross query tiles, rings that go round, odd and even rows, one head more than the ring has room
+    for; values past fp16's range turn into infinities as the reference's do."""
+    from cinnamon_b200 import kernels as K
+    B, Lq, Lk, H, d = shape
+    g = torch.Generator(device="cuda").manual_seed(sum(shape))
+    q, k = torch.randn(B, Lq, H, d, device="cuda", generator=g).to(dtype), torch.randn(B, Lk, d, device="cuda", generator=g).to(dtype)
+    w = torch.rand(B, Lq, H, device="cuda", generator=g).to(dtype)
+    for _ in range(2):
+        got = K.lightning_indexer_fused(q, k, w)
+    want = torch.zeros(B, Lq, Lk, device="cuda", dtype=torch.float64)
+    for h in range(H):
+        want += (q[:, :, h].half().double() @ k.half().double().transpose(1, 2)).clamp_min(0) * w[:, :, h, None].double()
+    _close_fp16(got, want)
+    if dtype == torch.bfloat16:
+        q[0, 0], k[0, 0] = 0, 0
+        q[0, 0, :, 0], k[0, 0, 0], w[0, 0] = 1e5, 2.0, 1.0
+        got = K.lightning_indexer_fused(q, k, w)
+        assert float(got[0, 0, 0]) == float("inf")
+    assert K.device_status() == 0
+
+
+@pytest.mark.gpu
+def test_strided_queries_and_one_of_a_dimension():
+    """Views that TMA reads (heads innermost but one, batch and rows of one) and one it does not (an expanded batch)."""
+    from cinnamon_b200 import kernels as K
+    g = torch.Generator(device="cuda").manual_seed(3)
+    r = lambda *s: torch.randn(*s, device="cuda", generator=g).bfloat16()                     # noqa: E731
+    for q, k in ((r(2, 4, 150, 64).transpose(1, 2), r(2, 150, 128)[:, :, 64:]), (r(1, 1, 1, 64), r(1, 1, 64)),
+                 (r(150, 3, 2, 64).permute(2, 0, 1, 3), r(200, 2, 64).transpose(0, 1)), (r(1, 150, 4, 64).expand(2, -1, -1, -1), r(2, 33, 64))):
+        w = torch.rand(q.shape[:3], device="cuda", generator=g).bfloat16()
+        want = torch.einsum("bqhd,bkd->bqhk", q.double(), k.double()).clamp_min(0).mul(w.double()[..., None]).sum(2)
+        _close_fp16(K.lightning_indexer_fused(q, k, w), want)
