@@ -19,8 +19,9 @@
 // General form (fp32, any strides, many heads): one CTA per tile.  All threads read the inputs (16 bytes at a time where the layout allows),
 // round to fp16 and write the swizzled tiles; one warp issues the MMAs into one of two buffers while eight warps fold the previous
 // head's (64 registers per thread).  Queries of up to 64 KiB of heads are resident at a time, so two CTAs share an SM and one loads
-// while the other computes.
-// (439 us on the scalar kernel.)
+// while the other computes.  Its weights stay a load per head and its odd rows are stored element by element: brought into shared
+// memory ahead the weights cost 183 us for 171 (8 x 2753, 4 heads of 64 in fp32), stores of words from the odd rows' first boundary 180 for 171.  One
+// statement per panel of MMAs gives 167.
 //
 // Scalar kernel (wider rows): 16 queries x 64 keys per CTA.  The key tile is kept transposed in shared memory as fp16
 // ([d][key], so the 16 lanes that share a query read 16 consecutive keys), the queries of all heads as fp16
@@ -179,36 +180,6 @@ __device__ __forceinline__ void load_tile(uint8_t* dst, const T* src, int rows, 
     }
 }
 
-// 32 rows of COLS logits from a warp's staging (rows of COLS * 2 bytes, 16-byte chunks XOR-ed with the row) to rows at any 2-byte boundary:
-// words from a row's first 4-byte boundary on, and an element at each end of a row that is off one.  Rows of the same alignment are
-// taken together, so that it is worked out once (element by element, or with a division of work per row, the stores of an odd
-// row length took longer than everything else).
-template <int COLS>
-__device__ __forceinline__ void store_any(const uint8_t* stage, __half* out, int64_t ld, int rows, int cols, int lane) {
-    constexpr int WORDS = COLS / 2, TOGETHER = 32 / WORDS;         // words of a row; rows of an instruction
-    constexpr int CHUNKS = COLS / 8, SHIFT = CHUNKS == 4 ? 1 : 0;
-    const int p = lane % WORDS, up = lane / WORDS;
-    const int c0 = p >> 2, c1 = ((p + 1) % WORDS) >> 2, o0 = (p & 3) * 4, o1 = ((p + 1) & 3) * 4;
-#pragma unroll
-    for (int u = 0; u < 2 / TOGETHER; ++u) {
-        const int r0 = u + up;                                     // rows r0, r0 + 2, ...
-        __half* row = out + r0 * ld;
-        const int odd = (int)(reinterpret_cast<uintptr_t>(row) >> 1) & 1, s = 2 * p + odd;
-        const bool two = s + 1 < cols, one = s + 1 == cols, head = odd && p == 0 && cols > 0;
-#pragma unroll
-        for (int i = 0; i < 16; ++i, row += 2 * ld) {
-            const int r = 2 * i + r0, x = (r >> SHIFT) & (CHUNKS - 1);
-            const uint32_t w0 = *reinterpret_cast<const uint32_t*>(stage + r * (COLS * 2) + ((c0 ^ x) << 4) + o0);
-            const uint32_t w1 = *reinterpret_cast<const uint32_t*>(stage + r * (COLS * 2) + ((c1 ^ x) << 4) + o1);
-            if (r < rows) {
-                if (two) *reinterpret_cast<uint32_t*>(row + s) = odd ? __funnelshift_r(w0, w1, 16) : w0;
-                if (one) row[s] = __ushort_as_half((uint16_t)(odd ? w0 >> 16 : w0));
-                if (head) row[0] = __ushort_as_half((uint16_t)w0);
-            }
-        }
-    }
-}
-
 template <typename T>
 __global__ void __launch_bounds__(ITC_THREADS, 2)
 indexer_tc_kernel(const T* __restrict__ q, const T* __restrict__ k, const T* __restrict__ w, __half* __restrict__ out,
@@ -218,8 +189,7 @@ indexer_tc_kernel(const T* __restrict__ q, const T* __restrict__ k, const T* __r
     const int head_bytes = (a.dpad / 64) * ITC_PANEL;
     uint8_t* sQ = smem;                                            // [head of the chunk][panel][row][128 B]
     uint8_t* sK = smem + (size_t)a.heads_per_chunk * head_bytes;   // [panel][row][128 B]
-    float* sW = reinterpret_cast<float*>(sK + head_bytes);          // [head of the chunk][query]: a load per head was a round trip per head
-    uint64_t* bars = reinterpret_cast<uint64_t*>(sW + a.heads_per_chunk * ITC_T); // two "dot products ready", two "buffer free"
+    uint64_t* bars = reinterpret_cast<uint64_t*>(sK + head_bytes); // two "dot products ready", two "buffer free"
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 4);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -235,6 +205,7 @@ indexer_tc_kernel(const T* __restrict__ q, const T* __restrict__ k, const T* __r
     const T* qb = q + b * a.sqb;
     load_tile<T>(sK, kb + k0 * a.skk, a.Lk - k0, a.skk, a.skd, a.d, a.dpad, a.vec_k);
     const int quarter = warp & 3, group = warp >> 2;                // TMEM lane quarter, column group of 64 keys
+    const int t = q0 + quarter * 32 + lane;
     float acc[64];
 #pragma unroll
     for (int i = 0; i < 64; ++i) acc[i] = 0.0f;
@@ -245,10 +216,6 @@ indexer_tc_kernel(const T* __restrict__ q, const T* __restrict__ k, const T* __r
         const int nh = min(a.heads_per_chunk, a.H - h0);
         for (int h = 0; h < nh; ++h)
             load_tile<T>(sQ + h * head_bytes, qb + q0 * a.sqq + (h0 + h) * a.sqh, a.Lq - q0, a.sqq, a.sqd, a.d, a.dpad, a.vec_q);
-        for (int e = tid; e < nh * ITC_T; e += ITC_THREADS) {
-            const int h = e >> 7, r = q0 + (e & (ITC_T - 1));
-            sW[e] = r < a.Lq ? w_to_float<T>(w[b * a.swb + r * a.swq + (h0 + h) * a.swh]) : 0.0f;
-        }
         fence_async_smem();
         tc_fence_before();
         __syncthreads();
@@ -271,7 +238,7 @@ indexer_tc_kernel(const T* __restrict__ q, const T* __restrict__ k, const T* __r
         }
         for (int h = 0; h < nh && alive; ++h) {
             const uint32_t n = it0 + h, buf = n & 1;
-            const float wh = sW[h * ITC_T + quarter * 32 + lane];
+            const float wh = t < a.Lq ? w_to_float<T>(w[b * a.swb + t * a.swq + (h0 + h) * a.swh]) : 0.0f;
             const bool ok = mbar_wait_bounded(full0 + 8 * buf, (n >> 1) & 1, abort_flag, (7 << 8) | 2, &g_indexer_status);
             if (!__all_sync(0xffffffffu, ok)) { alive = false; break; }
             tc_fence_after();
@@ -313,7 +280,14 @@ indexer_tc_kernel(const T* __restrict__ q, const T* __restrict__ k, const T* __r
                         *reinterpret_cast<const uint4*>(stage + r * 128 + ((c ^ (r & 7)) << 4));
             }
         } else {
-            store_any<64>(stage, ob, a.Lk, min(32, a.Lq - t0), min(64, a.Lk - s0), lane);
+            for (int r = 0; r < 32 && t0 + r < a.Lq; ++r) {
+#pragma unroll
+                for (int i = 0; i < 2; ++i) {
+                    const int s = lane + 32 * i;
+                    if (s0 + s < a.Lk)
+                        ob[(int64_t)r * a.Lk + s] = *reinterpret_cast<const __half*>(stage + r * 128 + (((s >> 3) ^ (r & 7)) << 4) + (s & 7) * 2);
+                }
+            }
         }
     }
     tc_fence_before();
@@ -676,10 +650,10 @@ static int indexer_tc_typed(const T* q, const T* k, const T* w, __half* out, int
     auto on16 = [](int64_t stride) { return (stride * (int64_t)sizeof(T)) % 16 == 0; };
     a.vec_q = d % 8 == 0 && sq[3] == 1 && on16(sq[0]) && on16(sq[1]) && on16(sq[2]) && (reinterpret_cast<uintptr_t>(q) & 15) == 0;
     a.vec_k = d % 8 == 0 && sk[2] == 1 && on16(sk[0]) && on16(sk[1]) && (reinterpret_cast<uintptr_t>(k) & 15) == 0;
-    const size_t smem = (size_t)(a.heads_per_chunk + 1) * head_bytes + (size_t)a.heads_per_chunk * ITC_T * 4 + 1024 + 64;
+    const size_t smem = (size_t)(a.heads_per_chunk + 1) * head_bytes + 1024 + 64;
     dim3 grid((unsigned)((Lk + ITC_T - 1) / ITC_T), (unsigned)((Lq + ITC_T - 1) / ITC_T), (unsigned)B);
     CINN_CHECK_ARG(grid.y <= 65535 && grid.z <= 65535, "lightning_indexer: too many queries or batches");
-    CINN_CHECK_CUDA(cudaFuncSetAttribute(indexer_tc_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, 102 * 1024));
+    CINN_CHECK_CUDA(cudaFuncSetAttribute(indexer_tc_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, 100 * 1024));
     indexer_tc_kernel<T><<<grid, ITC_THREADS, smem, st>>>(q, k, w, out, a);
     CINN_CHECK_LAUNCH();
     return CINN_OK;
