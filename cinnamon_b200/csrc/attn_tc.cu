@@ -1303,11 +1303,13 @@ static Plan make_plan(int64_t B, int64_t H, int64_t L, int64_t K, int64_t Dqk, i
 
 // Whether the dense tiles are worth it: their time (the causal half of the tiles is visited, a constant number of cycles
 // each that grows with the widths, and every query tile costs its start and its probabilities; what was picked and the parts come
-// first) against the gathers' (K rows of Dqk + Dv elements per query and a constant per row).  The constants are fitted to 70 calls of each, forward and
-// backward, over B = 1 ... 32, L = 257 ... 4062, K = 32 ... 256, widths 64 ... 192, bf16 and fp32: 9 to 16 % off on average, and the way that
-// is taken costs 0.3 (forward) and 0.7 % (backward) more than the faster one would.  With the constants of a forward that was slower in
-// bf16 and of fewer lengths it was 4.5 and 3 %: gathers against tiles, 16 x 4 x 2286 queries, 64 picks of 64 / 128 in bf16 838 and 403 us
-// (it took the gathers), 4 x 8 x 3965, 64 of 192 / 128 861 and 581, 1 x 4 x 1105 in fp32 backward 72 and 199 (it took the tiles).
+// first) against the gathers' (K rows of Dqk + Dv elements per query and a constant per row).  The tiles take the larger of their number over
+// the SMs and of the longest query tile's chain: with the sum of both, or the first alone, the estimate was 11 % off on average, with the
+// larger 5 (backward).  Fitted to 420 calls, B = 1 ... 32, L = 257 ... 4081, K = 32 ... 256, widths 64 ... 192, bf16 and fp32.  On 170 others the way
+// that is taken costs more than the faster one would by 0.3 (forward) and 0.1 % (backward) in bf16, 0.2 and 0.1 in fp32, at worst 1.12 times;
+// without the chain, fitted to 70 calls, by 0.4, 0.5, 0.7 and 2.4, at worst 1.74; with constants of a slower forward and fewer lengths by 3.0, 0.5,
+// 3.4 and 3.5, at worst 1.9.  Gathers against tiles: 16 x 4 x 2286 queries, 64 picks of 64 / 128 in bf16 838 and 403 us, 4 x 8 x 3965,
+// 64 of 192 / 128 861 and 581; backward 4 x 4 x 2033, 64 of 128 / 128 in fp32 549 and 428, 1 x 8 x 1965, 32 of 128 / 64 in bf16 131 and 176.
 static std::atomic<int> g_mode{-1};         // -1: by the estimate; 0 / 1: never / wherever the tiles can (tests, measurements)
 int set_mode(int mode) { return g_mode.exchange(mode); }
 
@@ -1318,18 +1320,25 @@ static bool dense_pays(const Plan& p, bool backward) {
     const bool parts = p.ns > 1, wide = p.dtype == CINN_F32;
     const double queries = (double)p.BH * p.L, row = (double)(p.Dqk + p.Dv), widths = p.dp + 64.0 * p.nv;
     const double gathered = queries * p.K * row * (wide ? 4 : 2), split = parts ? queries * (row + p.Dqk) * (wide ? 10 : 8) / 6.2e6 : 0.0;
-    const double picks = 15.0 + 5.5e-6 * p.B * p.L * p.K;
-    double cycles, tiles_us, gather_us;
+    const double picked = 5.5e-6 * p.B * p.L * p.K;
+    // cycles of a tile, how much of the longest query tile's chain counts, cycles of a query tile, microseconds before the tiles
+    double tile, chain, query_tile, first, gather_us;
     if (!backward) {
-        cycles = p.nv * (parts ? tiles * (2800.0 + 43.0 * p.dp) + q_tiles * (11100.0 + 68.0 * p.K) : tiles * (3600.0 + 3.4 * p.dp) + q_tiles * (3000.0 + 84.0 * p.K));
-        tiles_us = picks * (parts ? 2.3 : 2.15) + split;
-        gather_us = wide ? 9.0 + gathered / 15.3e6 + queries * p.K / 39e3 : 21.0 + gathered / 11.2e6 + queries * p.K / 26e3;
+        tile = parts ? 3870.0 + 35.6 * p.dp : 3590.0 + 5.97 * p.dp;
+        chain = parts ? 0.81 : 0.85;
+        query_tile = parts ? 2570.0 + 49.7 * p.K : 4810.0 + 57.6 * p.K;
+        first = parts ? 21.3 + 2.02 * picked + 1.91 * split : 20.0 + 3.27 * picked;
+        gather_us = wide ? 10.1 + gathered / 14.44e6 + queries * p.K / 44.3e3 : 11.8 + gathered / 9.85e6 + queries * p.K / 27.9e3;
     } else {
-        cycles = parts ? tiles * (3300.0 + 170.0 * widths) + q_tiles * (10000.0 + 937.0 * p.K) : tiles * (8800.0 + 41.6 * widths) + q_tiles * (13100.0 + 363.0 * p.K);
-        tiles_us = parts ? picks * 1.3 + 75.0 + split : picks * 3.75;
-        gather_us = wide ? 27.0 + gathered / 4.46e6 + queries * p.K / 71e3 : 60.0 + gathered / 2.79e6 + queries * p.K / 28.5e3;
+        tile = parts ? 10530.0 + 126.2 * widths : 9120.0 + 40.4 * widths;
+        chain = parts ? 0.89 : 0.85;
+        query_tile = parts ? 53.8 * p.K : 19000.0 + 95.3 * p.K;
+        first = parts ? 31.8 + 1.95 * picked + 2.97 * split : 29.9 + 1.19 * picked;
+        gather_us = wide ? 24.1 + gathered / 4.47e6 + queries * p.K / 65.9e3 : 40.6 + gathered / 2.71e6 + queries * p.K / 26.3e3;
     }
-    return tiles_us + cycles / (148.0 * 1900.0) < 0.95 * gather_us;
+    const double ctas = backward ? 1.0 : (double)p.nv;      // a forward CTA computes 64 columns of the output
+    const double all = ctas * tiles * tile / 148.0, longest = chain * (double)(p.Lp / T) * tile;
+    return first + ((all > longest ? all : longest) + ctas * q_tiles * query_tile / 148.0) / 1900.0 < gather_us;
 }
 
 static bool supported(int64_t B, int64_t H, int64_t L, int64_t K, int64_t Dqk, int64_t Dv) {
