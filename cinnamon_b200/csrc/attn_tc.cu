@@ -65,6 +65,8 @@ struct WarpgroupBarrier {
 __global__ void __launch_bounds__(128)
 picks_kernel(const int64_t* __restrict__ idx, uint32_t* __restrict__ bits, uint16_t* __restrict__ rank, uint8_t* __restrict__ count,
              uint16_t* __restrict__ before_out, int* __restrict__ repeats, int* __restrict__ flag, int64_t n_rows, int L, int words, int K, int warps) {
+    pdl_wait();
+    pdl_trigger();
     extern __shared__ __align__(16) uint32_t sm[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if (warp >= warps) return;
@@ -138,6 +140,8 @@ struct SplitJobs { SplitJob job[4]; int n; };
 template <typename U, int NS>
 __global__ void __launch_bounds__(256)
 split_parts_kernel(const SplitJobs jobs) {
+    pdl_wait();
+    pdl_trigger();
     for (int n = 0; n < jobs.n; ++n) {
         const SplitJob jb = jobs.job[n];
         const U* src = static_cast<const U*>(jb.src);
@@ -338,6 +342,8 @@ template <int NS, int ND, int PAIRS>
 __global__ void __launch_bounds__(FwdShape<NS, ND, PAIRS>::THREADS, 3 - PAIRS)
 attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                 const __grid_constant__ CUtensorMap tmV, const FwdArgs a) {
+    pdl_wait();
+    pdl_trigger();
     using S = FwdShape<NS, ND, PAIRS>;
     constexpr int TMA_WARP = 8 * PAIRS, MMA_WARP = TMA_WARP + 1;
     extern __shared__ uint8_t smem_raw[];
@@ -707,6 +713,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
 template <typename U>
 __global__ void __launch_bounds__(256)
 delta_kernel(const U* __restrict__ d_out, const float* __restrict__ out, float* __restrict__ delta, int64_t rows, int Dv) {
+    pdl_wait();
+    pdl_trigger();
     const int lane = threadIdx.x & 31;
     for (int64_t w = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5); w < rows; w += (int64_t)gridDim.x * 8) {
         float s = 0.0f;
@@ -830,6 +838,8 @@ __global__ void __launch_bounds__(QUERY_THREADS, 1)
 attn_bwd_query_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                       const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmG,
                       const __grid_constant__ CUtensorMap tmDQ, const BwdArgs a) {
+    pdl_wait();
+    pdl_trigger();
     using S = QPassShape<NS, ND, NV>;
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
@@ -1084,6 +1094,8 @@ template <int NS, int ND, int NV>
 __global__ void __launch_bounds__(KEY_THREADS, 1)
 attn_bwd_key_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmG,
                     const __grid_constant__ CUtensorMap tmDK, const __grid_constant__ CUtensorMap tmDV, const BwdArgs a) {
+    pdl_wait();
+    pdl_trigger();
     using S = KPassShape<NS, ND, NV>;
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
@@ -1363,7 +1375,7 @@ static int make_picks(const Plan& p, const int64_t* idx, uint8_t* ws, cudaStream
     const int64_t want = (rows + warps - 1) / warps, cap = (int64_t)sm_count() * 16;
     const unsigned grid = (unsigned)(want < cap ? want : cap);
     int* flag = reinterpret_cast<int*>(ws + p.flag_off);
-    picks_kernel<<<grid, 32 * warps, smem, st>>>(idx, reinterpret_cast<uint32_t*>(ws + p.bits_off),
+    launch_dependent(picks_kernel, dim3(grid), dim3(32 * warps), smem, st, idx, reinterpret_cast<uint32_t*>(ws + p.bits_off),
                                                  reinterpret_cast<uint16_t*>(ws + p.rank_off), ws + p.count_off,
                                                  reinterpret_cast<uint16_t*>(ws + p.before_off), flag + 1, flag, rows,
                                                  (int)p.L, words, (int)p.K, warps);
@@ -1374,9 +1386,9 @@ static int make_picks(const Plan& p, const int64_t* idx, uint8_t* ws, cudaStream
 static int split_parts(const SplitJobs& jobs, int dtype, cudaStream_t st) {
     const unsigned grid = (unsigned)sm_count() * 16;
     switch (dtype) {
-        case CINN_F32: split_parts_kernel<float, 3><<<grid, 256, 0, st>>>(jobs); break;
-        case CINN_F16: split_parts_kernel<__half, 3><<<grid, 256, 0, st>>>(jobs); break;
-        default: split_parts_kernel<__nv_bfloat16, 1><<<grid, 256, 0, st>>>(jobs); break;
+        case CINN_F32: launch_dependent(split_parts_kernel<float, 3>, dim3(grid), dim3(256), 0, st, jobs); break;
+        case CINN_F16: launch_dependent(split_parts_kernel<__half, 3>, dim3(grid), dim3(256), 0, st, jobs); break;
+        default: launch_dependent(split_parts_kernel<__nv_bfloat16, 1>, dim3(grid), dim3(256), 0, st, jobs); break;
     }
     CINN_CHECK_LAUNCH();
     return CINN_OK;
@@ -1402,7 +1414,7 @@ static int launch_fwd_pairs(const CUtensorMap& tq, const CUtensorMap& tk, const 
     using S = FwdShape<NS, ND, PAIRS>;
     auto kern = attn_fwd_kernel<NS, ND, PAIRS>;
     CINN_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, S::BYTES));
-    kern<<<grid, S::THREADS, S::BYTES, st>>>(tq, tk, tv, a);
+    launch_dependent(kern, dim3(grid), dim3(S::THREADS), S::BYTES, st, tq, tk, tv, a);
     CINN_CHECK_LAUNCH();
     return CINN_OK;
 }
@@ -1495,9 +1507,9 @@ static int launch_bwd(const CUtensorMap (&m)[9], const BwdArgs& a, const Plan& p
     const unsigned grid = (unsigned)(p.Lp / T * p.BH);
     CINN_CHECK_CUDA(cudaFuncSetAttribute(qk, cudaFuncAttributeMaxDynamicSharedMemorySize, QPassShape<NS, ND, NV>::BYTES));
     CINN_CHECK_CUDA(cudaFuncSetAttribute(kk, cudaFuncAttributeMaxDynamicSharedMemorySize, KPassShape<NS, ND, NV>::BYTES));
-    qk<<<grid, QUERY_THREADS, QPassShape<NS, ND, NV>::BYTES, st>>>(m[0], m[1], m[2], m[3], m[6], a);
+    launch_dependent(qk, dim3(grid), dim3(QUERY_THREADS), QPassShape<NS, ND, NV>::BYTES, st, m[0], m[1], m[2], m[3], m[6], a);
     CINN_CHECK_LAUNCH();
-    kk<<<grid, KEY_THREADS, KPassShape<NS, ND, NV>::BYTES, st>>>(m[4], m[5], m[7], m[8], a);
+    launch_dependent(kk, dim3(grid), dim3(KEY_THREADS), KPassShape<NS, ND, NV>::BYTES, st, m[4], m[5], m[7], m[8], a);
     CINN_CHECK_LAUNCH();
     return CINN_OK;
 }
@@ -1533,9 +1545,9 @@ int backward(const void* d_out, const float* out, const float* lse, const void* 
     const int64_t rows = p.BH * L, want = (rows + 7) / 8, cap = (int64_t)sm_count() * 32;
     const unsigned dgrid = (unsigned)(want < cap ? want : cap);
     switch (dtype) {
-        case CINN_F32: delta_kernel<float><<<dgrid, 256, 0, st>>>((const float*)d_out, out, delta, rows, (int)Dv); break;
-        case CINN_F16: delta_kernel<__half><<<dgrid, 256, 0, st>>>((const __half*)d_out, out, delta, rows, (int)Dv); break;
-        default: delta_kernel<__nv_bfloat16><<<dgrid, 256, 0, st>>>((const __nv_bfloat16*)d_out, out, delta, rows, (int)Dv); break;
+        case CINN_F32: launch_dependent(delta_kernel<float>, dim3(dgrid), dim3(256), 0, st, (const float*)d_out, out, delta, rows, (int)Dv); break;
+        case CINN_F16: launch_dependent(delta_kernel<__half>, dim3(dgrid), dim3(256), 0, st, (const __half*)d_out, out, delta, rows, (int)Dv); break;
+        default: launch_dependent(delta_kernel<__nv_bfloat16>, dim3(dgrid), dim3(256), 0, st, (const __nv_bfloat16*)d_out, out, delta, rows, (int)Dv); break;
     }
     CINN_CHECK_LAUNCH();
     CUtensorMap m[9];                                      // q, k, v, dO in boxes of 128 rows; q, dO in boxes of 32; dq, dk, dv

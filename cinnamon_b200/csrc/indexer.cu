@@ -21,7 +21,7 @@
 // head's (64 registers per thread).  Queries of up to 64 KiB of heads are resident at a time, so two CTAs share an SM and one loads
 // while the other computes.  Its weights stay a load per head and its odd rows are stored element by element: brought into shared
 // memory ahead the weights cost 183 us for 171 (8 x 2753, 4 heads of 64 in fp32), stores of words from the odd rows' first boundary 180 for 171.  One
-// statement per panel of MMAs gives 167.
+// statement per panel of MMAs gives 167, an early start 168, both 164; 8 x 1024 24.4 -> 20.9.
 //
 // Scalar kernel (wider rows): 16 queries x 64 keys per CTA.  The key tile is kept transposed in shared memory as fp16
 // ([d][key], so the 16 lanes that share a query read 16 consecutive keys), the queries of all heads as fp16
@@ -201,6 +201,8 @@ indexer_tc_kernel(const T* __restrict__ q, const T* __restrict__ k, const T* __r
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 0) tc_alloc(smem_u32(tmem_slot), 2 * ITC_T);
+    pdl_wait();
+    pdl_trigger();
     const T* kb = k + b * a.skb;
     const T* qb = q + b * a.sqb;
     load_tile<T>(sK, kb + k0 * a.skk, a.Lk - k0, a.skk, a.skd, a.d, a.dpad, a.vec_k);
@@ -654,7 +656,7 @@ static int indexer_tc_typed(const T* q, const T* k, const T* w, __half* out, int
     dim3 grid((unsigned)((Lk + ITC_T - 1) / ITC_T), (unsigned)((Lq + ITC_T - 1) / ITC_T), (unsigned)B);
     CINN_CHECK_ARG(grid.y <= 65535 && grid.z <= 65535, "lightning_indexer: too many queries or batches");
     CINN_CHECK_CUDA(cudaFuncSetAttribute(indexer_tc_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, 100 * 1024));
-    indexer_tc_kernel<T><<<grid, ITC_THREADS, smem, st>>>(q, k, w, out, a);
+    launch_dependent(indexer_tc_kernel<T>, grid, dim3(ITC_THREADS), smem, st, q, k, w, out, a);
     CINN_CHECK_LAUNCH();
     return CINN_OK;
 }

@@ -55,6 +55,8 @@ fp8_linear_few_kernel(const TX* __restrict__ x, int64_t ldx, const float* __rest
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 0) tc_alloc(smem_u32(&tmem_slot), TMEM_COLS);
+    pdl_wait();
+    pdl_trigger();
     const int slices = gridDim.x, slice = blockIdx.x, n0 = blockIdx.y * TILE;
     const int KB = (K + TILE - 1) / TILE, kb0 = KB * slice / slices, kb1 = KB * (slice + 1) / slices;
 
@@ -257,13 +259,15 @@ static int launch(const TX* x, int64_t ldx, const float* w, int64_t ldw, __nv_bf
     cfg.blockDim = dim3(THREADS, 1, 1);
     cfg.dynamicSmemBytes = SMEM_BYTES;
     cfg.stream = st;
-    cudaLaunchAttribute attr[1];
+    cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = slices;
     attr[0].val.clusterDim.y = 1;
     attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = 2;
     CINN_CHECK_CUDA(cudaLaunchKernelEx(&cfg, kern, x, ldx, w, ldw, out, M, N, K));
     CINN_CHECK_LAUNCH();
     return CINN_OK;

@@ -56,6 +56,8 @@ __global__ void __launch_bounds__(256)
 moe_combine_kernel(const T* __restrict__ rows, const int64_t* __restrict__ pos, const float* __restrict__ gates,
                    const void* __restrict__ addend, int addend_dtype, float* __restrict__ y, int64_t n_tokens, int64_t n_rows,
                    int top_k, int d, int per_token) {
+    pdl_wait();
+    pdl_trigger();
     constexpr int SLOTS = 256;                         // (token, slot) pairs of a CTA kept in shared memory
     __shared__ int64_t s_pos[SLOTS];
     __shared__ float s_gate[SLOTS];
@@ -114,8 +116,8 @@ static void launch_combine(const T* rows, const int64_t* pos, const float* gates
     const int64_t tokens = 256 / per;
     const bool few = n_tokens < 4 * sm_count() && d <= 32768;
     const dim3 grid((unsigned)((n_tokens + tokens - 1) / tokens), few ? (unsigned)((d + per * 8 - 1) / (per * 8)) : 1u);
-    if (top_k <= 2) moe_combine_kernel<T, 2><<<grid, 256, 0, st>>>(rows, pos, gates, addend, addend_dtype, y, n_tokens, n_rows, top_k, d, per);
-    else moe_combine_kernel<T, 4><<<grid, 256, 0, st>>>(rows, pos, gates, addend, addend_dtype, y, n_tokens, n_rows, top_k, d, per);
+    if (top_k <= 2) launch_dependent(moe_combine_kernel<T, 2>, dim3(grid), dim3(256), 0, st, rows, pos, gates, addend, addend_dtype, y, n_tokens, n_rows, top_k, d, per);
+    else launch_dependent(moe_combine_kernel<T, 4>, dim3(grid), dim3(256), 0, st, rows, pos, gates, addend, addend_dtype, y, n_tokens, n_rows, top_k, d, per);
 }
 
 // gates null: every gate is one (the entry points that take gates refuse a null)
@@ -179,6 +181,8 @@ __global__ void __launch_bounds__(256)
 moe_combine_backward_kernel(const T* __restrict__ rows, const int64_t* __restrict__ pos, const float* __restrict__ gates,
                             const float* __restrict__ dy, T* __restrict__ d_rows, float* __restrict__ d_gates,
                             int64_t n_pairs, int64_t n_rows, int top_k, int d) {
+    pdl_wait();
+    pdl_trigger();
     const int lane = threadIdx.x & 31;
     const int64_t warp = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5);
     const int64_t n_warps = (int64_t)gridDim.x * 8;
@@ -210,6 +214,8 @@ moe_combine_backward_kernel(const T* __restrict__ rows, const int64_t* __restric
 template <typename T, bool BACKWARD, bool ROUND = false>
 __global__ void __launch_bounds__(256)
 swiglu_kernel(const T* __restrict__ h12, const T* __restrict__ dh, T* __restrict__ out, int64_t T_rows, int I) {
+    pdl_wait();
+    pdl_trigger();
     const int per_row = I >> 3;
     const int64_t total = T_rows * per_row;
     for (int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x; i < total; i += (int64_t)gridDim.x * 256) {
@@ -252,10 +258,10 @@ static int swiglu_typed(const T* h12, const T* dh, T* out, int64_t T_rows, int64
     int64_t blocks = (T_rows * (I / 8) + 255) / 256;
     const int64_t cap = (int64_t)sm_count() * 16;
     if (blocks > cap) blocks = cap;
-    if (backward && round) swiglu_kernel<T, true, true><<<(unsigned)blocks, 256, 0, st>>>(h12, dh, out, T_rows, (int)I);
-    else if (backward) swiglu_kernel<T, true><<<(unsigned)blocks, 256, 0, st>>>(h12, dh, out, T_rows, (int)I);
-    else if (round) swiglu_kernel<T, false, true><<<(unsigned)blocks, 256, 0, st>>>(h12, dh, out, T_rows, (int)I);
-    else swiglu_kernel<T, false><<<(unsigned)blocks, 256, 0, st>>>(h12, dh, out, T_rows, (int)I);
+    if (backward && round) launch_dependent(swiglu_kernel<T, true, true>, dim3((unsigned)blocks), dim3(256), 0, st, h12, dh, out, T_rows, (int)I);
+    else if (backward) launch_dependent(swiglu_kernel<T, true>, dim3((unsigned)blocks), dim3(256), 0, st, h12, dh, out, T_rows, (int)I);
+    else if (round) launch_dependent(swiglu_kernel<T, false, true>, dim3((unsigned)blocks), dim3(256), 0, st, h12, dh, out, T_rows, (int)I);
+    else launch_dependent(swiglu_kernel<T, false>, dim3((unsigned)blocks), dim3(256), 0, st, h12, dh, out, T_rows, (int)I);
     CINN_CHECK_LAUNCH();
     return CINN_OK;
 }
@@ -322,6 +328,8 @@ int gather_rows(const void* q, const float* s, const int64_t* idx, void* out_q, 
 __global__ void __launch_bounds__(256)
 spread_rows_kernel(const uint8_t* __restrict__ q, const float* __restrict__ s, const int64_t* __restrict__ pos,
                    uint8_t* __restrict__ out_q, float* __restrict__ out_s, int64_t n_rows, int top_k, int d, int ns) {
+    pdl_wait();
+    pdl_trigger();
     const int64_t t = blockIdx.x;
     const int vecs = d >> 4;
     const uint4* in = reinterpret_cast<const uint4*>(q + t * d);
@@ -349,7 +357,7 @@ int spread_rows(const void* q, const float* s, const int64_t* pos, void* out_q, 
                    "spread_rows: the row width (%lld) must be a multiple of 16", (long long)d);
     CINN_CHECK_ARG((reinterpret_cast<uintptr_t>(q) & 15) == 0 && (reinterpret_cast<uintptr_t>(out_q) & 15) == 0,
                    "spread_rows: byte buffers must be 16-byte aligned");
-    spread_rows_kernel<<<(unsigned)n_tokens, 256, 0, st>>>((const uint8_t*)q, s, pos, (uint8_t*)out_q, out_s, n_rows, top_k, (int)d, (int)ns);
+    launch_dependent(spread_rows_kernel, dim3((unsigned)n_tokens), dim3(256), 0, st, (const uint8_t*)q, s, pos, (uint8_t*)out_q, out_s, n_rows, top_k, (int)d, (int)ns);
     CINN_CHECK_LAUNCH();
     return CINN_OK;
 }
@@ -848,6 +856,8 @@ int p2p_return(const void* rows, const int64_t* seg_start, const int64_t* home_b
 __global__ void __launch_bounds__(256)
 zero_rows_outside_kernel(uint8_t* __restrict__ buf, int64_t T, int64_t row_bytes, const int64_t* __restrict__ starts,
                          const int64_t* __restrict__ ends, int E) {
+    pdl_wait();
+    pdl_trigger();
     __shared__ int covered[128];
     const int64_t r0 = (int64_t)blockIdx.x * 128;
     if (threadIdx.x < 128) covered[threadIdx.x] = 0;
@@ -879,7 +889,7 @@ int zero_rows_outside(void* buf, int64_t T, int64_t row_bytes, const int64_t* st
     CINN_CHECK_ARG(buf && (E == 0 || (starts && ends)), "zero_rows_outside: null pointer");
     const int64_t blocks = (T + 127) / 128;
     CINN_CHECK_ARG(blocks < (1LL << 31), "zero_rows_outside: too many rows");
-    zero_rows_outside_kernel<<<(unsigned)blocks, 256, 0, st>>>((uint8_t*)buf, T, row_bytes, starts, ends, (int)E);
+    launch_dependent(zero_rows_outside_kernel, dim3((unsigned)blocks), dim3(256), 0, st, (uint8_t*)buf, T, row_bytes, starts, ends, (int)E);
     CINN_CHECK_LAUNCH();
     return CINN_OK;
 }
@@ -898,9 +908,9 @@ int moe_combine_backward(const void* rows, int dtype, const int64_t* pos, const 
     const int64_t cap = (int64_t)sm_count() * 16;
     if (blocks > cap) blocks = cap;
     switch (dtype) {
-        case CINN_BF16: moe_combine_backward_kernel<__nv_bfloat16><<<(unsigned)blocks, 256, 0, st>>>((const __nv_bfloat16*)rows, pos, gates, dy, (__nv_bfloat16*)d_rows, d_gates, n_pairs, n_rows, top_k, (int)d); break;
-        case CINN_F16: moe_combine_backward_kernel<__half><<<(unsigned)blocks, 256, 0, st>>>((const __half*)rows, pos, gates, dy, (__half*)d_rows, d_gates, n_pairs, n_rows, top_k, (int)d); break;
-        case CINN_F32: moe_combine_backward_kernel<float><<<(unsigned)blocks, 256, 0, st>>>((const float*)rows, pos, gates, dy, (float*)d_rows, d_gates, n_pairs, n_rows, top_k, (int)d); break;
+        case CINN_BF16: launch_dependent(moe_combine_backward_kernel<__nv_bfloat16>, dim3((unsigned)blocks), dim3(256), 0, st, (const __nv_bfloat16*)rows, pos, gates, dy, (__nv_bfloat16*)d_rows, d_gates, n_pairs, n_rows, top_k, (int)d); break;
+        case CINN_F16: launch_dependent(moe_combine_backward_kernel<__half>, dim3((unsigned)blocks), dim3(256), 0, st, (const __half*)rows, pos, gates, dy, (__half*)d_rows, d_gates, n_pairs, n_rows, top_k, (int)d); break;
+        case CINN_F32: launch_dependent(moe_combine_backward_kernel<float>, dim3((unsigned)blocks), dim3(256), 0, st, (const float*)rows, pos, gates, dy, (float*)d_rows, d_gates, n_pairs, n_rows, top_k, (int)d); break;
         default: set_error("moe_combine_backward: unknown dtype tag %d", dtype); return CINN_ERR_INVALID;
     }
     CINN_CHECK_LAUNCH();

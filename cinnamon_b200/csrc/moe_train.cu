@@ -36,6 +36,8 @@ template <int VPL, typename L>                 // scores per lane, E <= 32 * VPL
 __global__ void __launch_bounds__(256)
 balance_partial_kernel(const L* __restrict__ logits, const int* __restrict__ top_experts, float* __restrict__ part_p,
                        int* __restrict__ part_c, int seq, int chunks, int E, int top_k) {
+    pdl_wait();
+    pdl_trigger();
     __shared__ float s_p[MAX_E];
     __shared__ int s_c[MAX_E];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -77,6 +79,8 @@ balance_partial_kernel(const L* __restrict__ logits, const int* __restrict__ top
 __global__ void __launch_bounds__(1024)
 balance_finish_kernel(const float* __restrict__ part_p, const int* __restrict__ part_c, float* __restrict__ share,
                       float* __restrict__ loss, int batch, int seq, int chunks, int E, int top_k, float alpha) {
+    pdl_wait();
+    pdl_trigger();
     __shared__ float s_sum[32];
     float sum = 0.0f;
     for (int64_t i = threadIdx.x; i < (int64_t)batch * E; i += 1024) {
@@ -109,6 +113,8 @@ __global__ void __launch_bounds__(256)
 gates_backward_kernel(const L* __restrict__ logits, const int64_t* __restrict__ sorted_experts, const int64_t* __restrict__ pair_pos,
                       const float* __restrict__ d_gates, const float* __restrict__ share, const float* __restrict__ d_loss, float coef,
                       L* __restrict__ d_logits, int64_t T, int seq, int E, int top_k) {
+    pdl_wait();
+    pdl_trigger();
     const int lane = threadIdx.x & 31;
     for (int64_t t = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5); t < T; t += (int64_t)gridDim.x * 8) {
         float s[VPL], ds[VPL], sum = 0.0f;
@@ -160,6 +166,8 @@ gates_backward_kernel(const L* __restrict__ logits, const int64_t* __restrict__ 
 
 // bias of over-used experts down by gamma, of the others up, clamped to [-1, 1] (src/layers.py:111-116)
 __global__ void update_bias_kernel(const int64_t* __restrict__ counts, float* __restrict__ bias, int E, float expected, float gamma) {
+    pdl_wait();
+    pdl_trigger();
     for (int e = threadIdx.x; e < E; e += blockDim.x) {
         const float b = bias[e] + ((float)counts[e] > expected ? -gamma : gamma);
         bias[e] = fminf(fmaxf(b, -1.0f), 1.0f);
@@ -182,7 +190,7 @@ int64_t balance_workspace_bytes(int64_t batch, int64_t seq, int E) { return batc
 
 template <typename L>
 static void launch_balance(const L* logits, const int* top, float* pp, int* pc, int batch, int seq, int chunks, int E, int top_k, cudaStream_t st) {
-#define CINN_CALL(V) balance_partial_kernel<V, L><<<batch * chunks, 256, 0, st>>>(logits, top, pp, pc, seq, chunks, E, top_k)
+#define CINN_CALL(V) launch_dependent(balance_partial_kernel<V, L>, dim3(batch * chunks), dim3(256), 0, st, logits, top, pp, pc, seq, chunks, E, top_k)
     CINN_VPL(CINN_CALL);
 #undef CINN_CALL
 }
@@ -200,7 +208,7 @@ int balance_loss(const void* logits, int dtype, const int* top_experts, int64_t 
     else if (dtype == CINN_BF16) launch_balance((const __nv_bfloat16*)logits, top_experts, pp, pc, (int)batch, (int)seq, (int)chunks, E, top_k, st);
     else launch_balance((const __half*)logits, top_experts, pp, pc, (int)batch, (int)seq, (int)chunks, E, top_k, st);
     CINN_CHECK_LAUNCH();
-    balance_finish_kernel<<<1, 1024, 0, st>>>(pp, pc, share, loss, (int)batch, (int)seq, (int)chunks, E, top_k, alpha);
+    launch_dependent(balance_finish_kernel, dim3(1), dim3(1024), 0, st, pp, pc, share, loss, (int)batch, (int)seq, (int)chunks, E, top_k, alpha);
     CINN_CHECK_LAUNCH();
     return CINN_OK;
 }
@@ -210,7 +218,7 @@ static void launch_gates(const L* logits, const int64_t* se, const int64_t* pos,
                          float coef, L* out, int64_t T, int seq, int E, int top_k, cudaStream_t st) {
     const int64_t want = (T + 7) / 8, cap = (int64_t)sm_count() * 16;
     const unsigned grid = (unsigned)(want < cap ? want : cap);
-#define CINN_CALL(V) gates_backward_kernel<V, L><<<grid, 256, 0, st>>>(logits, se, pos, dg, share, dl, coef, out, T, seq, E, top_k)
+#define CINN_CALL(V) launch_dependent(gates_backward_kernel<V, L>, dim3(grid), dim3(256), 0, st, logits, se, pos, dg, share, dl, coef, out, T, seq, E, top_k)
     CINN_VPL(CINN_CALL);
 #undef CINN_CALL
 }
@@ -233,7 +241,7 @@ int gates_backward(const void* logits, int dtype, const int64_t* sorted_experts,
 
 int update_bias(const int64_t* counts, float* bias, int E, float expected, float gamma, cudaStream_t st) {
     CINN_CHECK_ARG(counts && bias && E >= 1, "update_bias: bad arguments");
-    update_bias_kernel<<<1, 256, 0, st>>>(counts, bias, E, expected, gamma);
+    launch_dependent(update_bias_kernel, dim3(1), dim3(256), 0, st, counts, bias, E, expected, gamma);
     CINN_CHECK_LAUNCH();
     return CINN_OK;
 }

@@ -88,6 +88,7 @@ template <typename T, int DIV, bool ROUND, int UNROLL>
 __global__ void __launch_bounds__(256)
 quant_row_vec_kernel(const T* __restrict__ x, int64_t ld, uint8_t* __restrict__ q, float* __restrict__ scales,
                      int N, int nb, int64_t total_tiles, int step_rows, int step_cols) {
+    pdl_wait();
     pdl_trigger();
     quant_rows<T, DIV, ROUND, UNROLL>(x, ld, q, scales, N, nb, total_tiles, step_rows, step_cols, blockIdx.x, gridDim.x);
 }
@@ -783,9 +784,10 @@ template <typename T, int DIV, bool ROUND, int MODE = 0>
 __global__ void __launch_bounds__(256, 2)
 quant_row_dual_kernel(const T* __restrict__ x, int64_t ld, uint8_t* __restrict__ q_row, float* __restrict__ s_row,
                       uint8_t* __restrict__ q_col, float* __restrict__ s_col, int M, int N, int nb_n, int nb_m) {
+    pdl_wait();
+    pdl_trigger();
     __shared__ __align__(16) float s_amax[8][128];
     __shared__ __align__(16) uint8_t s_out[128 * 128];
-    pdl_trigger();
     const int sub = threadIdx.x & 15, hw = threadIdx.x >> 4;
     const int n = blockIdx.x * 128 + sub * 8;
     const int mt = blockIdx.y * 128 + hw * 8;
@@ -830,6 +832,8 @@ __global__ void __launch_bounds__(256, 2)
 quant_row_dual_tma_kernel(const __grid_constant__ CUtensorMap tmX, uint8_t* __restrict__ q_row, float* __restrict__ s_row,
                           uint8_t* __restrict__ q_col, float* __restrict__ s_col, int M, int N, int nb_n, int nb_m,
                           int total) {
+    pdl_wait();
+    pdl_trigger();
     static_assert(sizeof(T) == 2, "the TMA-fed path takes 2-byte inputs");
     extern __shared__ __align__(128) uint8_t dsm[];
     uint8_t* stages = dsm;
@@ -840,7 +844,6 @@ quant_row_dual_tma_kernel(const __grid_constant__ CUtensorMap tmX, uint8_t* __re
     const int sub = threadIdx.x & 15, hw = threadIdx.x >> 4;
     const int stride = gridDim.x;
 
-    pdl_trigger();
     if (threadIdx.x == 0) {
         for (int s = 0; s < DUAL_STAGES; ++s) mbar_init(full0 + 8 * s, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -900,6 +903,8 @@ __global__ void __launch_bounds__(256, 2)
 quant_row_dual_seg_kernel(const __grid_constant__ CUtensorMap tmX, uint8_t* __restrict__ q_row, float* __restrict__ s_row,
                           uint8_t* __restrict__ q_col, float* __restrict__ s_col, int M_pad, int N, int nb_n, int nb_m,
                           const int* __restrict__ tile_src, const int* __restrict__ tile_cnt, const int* __restrict__ n_tiles) {
+    pdl_wait();
+    pdl_trigger();
     static_assert(sizeof(T) == 2, "the TMA-fed path takes 2-byte inputs");
     extern __shared__ __align__(128) uint8_t dsm[];
     uint8_t* stages = dsm;
@@ -993,10 +998,11 @@ __global__ void __launch_bounds__(256, 2)
 swiglu_row_block_kernel(const T* __restrict__ h12, uint8_t* __restrict__ q_row, float* __restrict__ s_row, uint8_t* __restrict__ q_blk,
                         float* __restrict__ s_blk, int M, int I, int nb_n, int nb_m, int total, const int* __restrict__ tile_src,
                         const int* __restrict__ tile_cnt, const int* __restrict__ n_tiles) {
+    pdl_wait();
+    pdl_trigger();
     __shared__ __align__(16) float s_red[8];
     __shared__ __align__(16) uint8_t s_out[128 * 128];
     const int sub = threadIdx.x & 15, hw = threadIdx.x >> 4;
-    pdl_trigger();
     if constexpr (SEG) total = *n_tiles * nb_n;
     for (int t = blockIdx.x; t < total; t += gridDim.x) {
         int bm, bn;
@@ -1032,10 +1038,11 @@ __global__ void __launch_bounds__(256, 2)
 swiglu_backward_dual_kernel(const T* __restrict__ h12, const T* __restrict__ dh, uint8_t* __restrict__ q_row, float* __restrict__ s_row,
                             uint8_t* __restrict__ q_col, float* __restrict__ s_col, int M, int I, int nb_i, int nb_m, int total,
                             const int* __restrict__ tile_src, const int* __restrict__ tile_cnt, const int* __restrict__ n_tiles) {
+    pdl_wait();
+    pdl_trigger();
     __shared__ __align__(16) float s_amax[8][128];
     __shared__ __align__(16) uint8_t s_out[128 * 128];
     const int sub = threadIdx.x & 15, hw = threadIdx.x >> 4;
-    pdl_trigger();
     if constexpr (SEG) total = *n_tiles * nb_i;
     for (int t = blockIdx.x; t < total; t += gridDim.x) {
         int bm, bn;
@@ -1135,6 +1142,7 @@ template <typename T, int DIV, bool ROUND>
 __global__ void __launch_bounds__(256)
 quant_block_vec_kernel(const T* __restrict__ x, int64_t ld, uint8_t* __restrict__ q, float* __restrict__ scales,
                        int M, int N, int nb, int beside) {
+    if (!beside) pdl_wait();
     pdl_trigger();
     quant_block<T, DIV, ROUND>(x, ld, q, scales, M, N, nb, blockIdx.x, blockIdx.y);
     if (beside) pdl_wait();
@@ -1147,6 +1155,7 @@ __global__ void __launch_bounds__(256)
 quant_linear_kernel(const TX* __restrict__ x, int64_t ldx, uint8_t* __restrict__ xq, float* __restrict__ xs, int64_t total_tiles,
                     int step_rows, int step_cols, const TW* __restrict__ w, int64_t ldw, uint8_t* __restrict__ wq,
                     float* __restrict__ ws, int N, int K, int nb_k, int w_blocks) {
+    pdl_wait();
     pdl_trigger();
     if ((int)blockIdx.x < w_blocks)
         quant_block<TW, DIV, false>(w, ldw, wq, ws, N, K, nb_k, blockIdx.x % nb_k, blockIdx.x / nb_k);
@@ -1194,9 +1203,10 @@ template <typename T, int DIV, bool ROUND>
 __global__ void __launch_bounds__(256)
 quant_block_vec_t_kernel(const T* __restrict__ x, int64_t ld, uint8_t* __restrict__ q, uint8_t* __restrict__ q_t,
                          float* __restrict__ scales, int M, int N, int nb, int beside) {
+    if (!beside) pdl_wait();
+    pdl_trigger();
     __shared__ float s_red[8];
     __shared__ uint32_t s_t[128 * 32];
-    pdl_trigger();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int r0 = blockIdx.y * 128, c = blockIdx.x * 128 + lane * 4;
     float v[16][4];
@@ -1385,6 +1395,8 @@ __global__ void __launch_bounds__(256, 2)
 requant_seg_t_kernel(const uint8_t* __restrict__ xq, const float* __restrict__ xs, uint8_t* __restrict__ out,
                      float* __restrict__ scales, int M, int K, int nb, const int* __restrict__ tile_src,
                      const int* __restrict__ tile_cnt, const int* __restrict__ n_tiles) {
+    pdl_wait();
+    pdl_trigger();
     __shared__ __align__(16) uint8_t s_raw[2][128 * 128];
     __shared__ float s_rs[2][128];
     __shared__ float s_red[8];
@@ -1477,9 +1489,10 @@ __global__ void __launch_bounds__(256)
 swiglu_quant_row_kernel(const T* __restrict__ h12, uint8_t* __restrict__ q, float* __restrict__ scales,
                         int I, int nb, int64_t total_tiles, int step_rows, int step_cols,
                         const int64_t* __restrict__ n_rows_dev) {
+    pdl_wait();
+    pdl_trigger();
     // optional row count that only the device knows (an expert-parallel rank's received rows): rows past it are skipped
     if (n_rows_dev != nullptr) total_tiles = min(total_tiles, max(n_rows_dev[0], (int64_t)0) * nb);
-    pdl_trigger();
     // the n-th tile of this half-warp is hw + n * n_hw; (step_rows, step_cols) = divmod(n_hw, nb): tile
     // coordinates advance without a division in the loop
     const int sub = threadIdx.x & 15;
@@ -1644,7 +1657,7 @@ static int launch_rowwise(const T* x, int64_t M, int64_t N, int64_t ld_m, int64_
         const int64_t cap = (int64_t)sms * 8;
         if (blocks > cap) blocks = cap;
         const int64_t n_hw = blocks * 16;
-        quant_row_vec_kernel<T, DIV, ROUND, UNROLL><<<(unsigned)blocks, 256, 0, st>>>(
+        launch_early_if(quantise_early(M, N), quant_row_vec_kernel<T, DIV, ROUND, UNROLL>, dim3((unsigned)blocks), dim3(256), 0, st,
             x, ld_m, q, scales, (int)N, nb, tiles, (int)(n_hw / nb), (int)(n_hw % nb));
     } else if (block == 128 && ld_m == 1 && ld_n >= M && M % 8 == 0 && ld_n % 8 == 0 && N % 16 == 0 && aligned16(x) &&
                aligned16(q) && M > 1) {
@@ -1675,7 +1688,7 @@ static int launch_blockwise(const T* x, int64_t M, int64_t N, int64_t ld_m, int6
     const bool a = sizeof(T) == 4 ? aligned16(x) : ((reinterpret_cast<uintptr_t>(x) & 7) == 0);
     if (bm == 128 && bn == 128 && ld_n == 1 && N % 4 == 0 && ld_m % 4 == 0 && a && (reinterpret_cast<uintptr_t>(q) & 3) == 0) {
         if (t_beside) CINN_CHECK_CUDA(launch_dependent(quant_block_vec_kernel<T, DIV, ROUND>, grid, 256, 0, st, x, ld_m, q, scales, (int)M, (int)N, nb, 1));
-        else quant_block_vec_kernel<T, DIV, ROUND><<<grid, 256, 0, st>>>(x, ld_m, q, scales, (int)M, (int)N, nb, 0);
+        else launch_early_if(quantise_early(M, N), quant_block_vec_kernel<T, DIV, ROUND>, dim3(grid), dim3(256), 0, st, x, ld_m, q, scales, (int)M, (int)N, nb, 0);
     } else {
         quant_block_generic_kernel<T, DIV, ROUND><<<grid, 256, 0, st>>>(x, ld_m, ld_n, q, scales, (int)M, (int)N, bm, bn, nb);
     }
@@ -1692,7 +1705,7 @@ static int dispatch_block_t(const T* x, int64_t M, int64_t N, int64_t ld, uint8_
 #define CINN_B(DIV, RND) \
     do { \
         if (t_beside) CINN_CHECK_CUDA(launch_dependent(quant_block_vec_t_kernel<T, DIV, RND>, grid, 256, 0, st, x, ld, q, q_t, scales, (int)M, (int)N, nb, 1)); \
-        else quant_block_vec_t_kernel<T, DIV, RND><<<grid, 256, 0, st>>>(x, ld, q, q_t, scales, (int)M, (int)N, nb, 0); \
+        else launch_early_if(quantise_early(M, N), quant_block_vec_t_kernel<T, DIV, RND>, dim3(grid), dim3(256), 0, st, x, ld, q, q_t, scales, (int)M, (int)N, nb, 0); \
     } while (0)
     if (div_mode == CINN_DIV_FULL) { if (round_scale) CINN_B(CINN_DIV_FULL, true); else CINN_B(CINN_DIV_FULL, false); }
     else                           { if (round_scale) CINN_B(CINN_DIV_RN, true);   else CINN_B(CINN_DIV_RN, false); }
@@ -1730,7 +1743,10 @@ static int launch_quant_linear(const TX* x, int64_t ldx, uint8_t* xq, float* xs,
     if (blocks > cap) blocks = cap;
     const int64_t n_hw = blocks * 16;
     const unsigned grid = (unsigned)(w_blocks + blocks);
-#define CINN_Q(DIV, RND) quant_linear_kernel<TX, TW, DIV, RND><<<grid, 256, 0, st>>>(x, ldx, xq, xs, tiles, (int)(n_hw / nb), (int)(n_hw % nb), w, ldw, wq, ws, (int)N, (int)K, nb, (int)w_blocks)
+    // As in quantise_early, and only a grid that fits on the SMs at once (eight blocks each): 403 x 2048 -> 12928 47 -> 53 us.  Few rows are not
+    // multiplied in long tiles and gain up to 3072 columns (12 x 2368 -> 1856 12.4 -> 11.6, 100 x 3072 -> 2048 16.4 -> 13.9), not at 4096 (40 x 4096
+    // -> 4096 26.7 -> 27.5).
+#define CINN_Q(DIV, RND) launch_early_if((int64_t)grid <= 8 * (int64_t)sm_count() && (K <= 2048 || (M <= 128 && K <= 3072)), quant_linear_kernel<TX, TW, DIV, RND>, dim3(grid), dim3(256), 0, st, x, ldx, xq, xs, tiles, (int)(n_hw / nb), (int)(n_hw % nb), w, ldw, wq, ws, (int)N, (int)K, nb, (int)w_blocks)
     if (div_mode == CINN_DIV_FULL) { if (round_scale) CINN_Q(CINN_DIV_FULL, true); else CINN_Q(CINN_DIV_FULL, false); }
     else                           { if (round_scale) CINN_Q(CINN_DIV_RN, true);   else CINN_Q(CINN_DIV_RN, false); }
 #undef CINN_Q
@@ -1836,14 +1852,14 @@ static int dispatch_dual(const T* x, int64_t M, int64_t N, int64_t ld, uint8_t* 
             attr_err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, DUAL_SMEM_BYTES);      \
         });                                                                                                           \
         CINN_CHECK_CUDA(attr_err);                                                                                    \
-        kern<<<grid, 256, DUAL_SMEM_BYTES, st>>>(tm, q_row, s_row, q_col, s_col, (int)M, (int)N, nb_n, nb_m, (int)total); \
+        launch_early_if(quantise_early(M, N), kern, dim3(grid), dim3(256), DUAL_SMEM_BYTES, st, tm, q_row, s_row, q_col, s_col, (int)M, (int)N, nb_n, nb_m, (int)total); \
     } while (0)
         if (div_mode == CINN_DIV_FULL) { if (round_scale) CINN_D(CINN_DIV_FULL, true); else CINN_D(CINN_DIV_FULL, false); }
         else                           { if (round_scale) CINN_D(CINN_DIV_RN, true);   else CINN_D(CINN_DIV_RN, false); }
 #undef CINN_D
     } else {
         dim3 grid((unsigned)nb_n, (unsigned)nb_m);
-#define CINN_D(DIV, RND) quant_row_dual_kernel<T, DIV, RND><<<grid, 256, 0, st>>>(x, ld, q_row, s_row, q_col, s_col, (int)M, (int)N, nb_n, nb_m)
+#define CINN_D(DIV, RND) launch_early_if(quantise_early(M, N), quant_row_dual_kernel<T, DIV, RND>, dim3(grid), dim3(256), 0, st, x, ld, q_row, s_row, q_col, s_col, (int)M, (int)N, nb_n, nb_m)
         if (div_mode == CINN_DIV_FULL) { if (round_scale) CINN_D(CINN_DIV_FULL, true); else CINN_D(CINN_DIV_FULL, false); }
         else                           { if (round_scale) CINN_D(CINN_DIV_RN, true);   else CINN_D(CINN_DIV_RN, false); }
 #undef CINN_D
@@ -1886,7 +1902,7 @@ static int dispatch_row_block(const T* x, int64_t M, int64_t N, int64_t ld, uint
                 attr_err = cudaFuncSetAttribute(quant_row_dual_tma_kernel<T, DIV, RND, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, DUAL_SMEM_BYTES); \
         });                                                                                                           \
         CINN_CHECK_CUDA(attr_err);                                                                                    \
-        kern<<<grid, 256, DUAL_SMEM_BYTES, st>>>(tm, q_row, s_row, q_blk, s_blk, (int)M, (int)N, nb_n, nb_m, (int)total); \
+        launch_early_if(quantise_early(M, N), kern, dim3(grid), dim3(256), DUAL_SMEM_BYTES, st, tm, q_row, s_row, q_blk, s_blk, (int)M, (int)N, nb_n, nb_m, (int)total); \
     } while (0)
         if (div_mode == CINN_DIV_FULL) { if (round_scale) CINN_D(CINN_DIV_FULL, true); else CINN_D(CINN_DIV_FULL, false); }
         else                           { if (round_scale) CINN_D(CINN_DIV_RN, true);   else CINN_D(CINN_DIV_RN, false); }
@@ -1895,8 +1911,8 @@ static int dispatch_row_block(const T* x, int64_t M, int64_t N, int64_t ld, uint
         dim3 grid((unsigned)nb_n, (unsigned)nb_m);
 #define CINN_D(DIV, RND)                                                                                              \
     do {                                                                                                              \
-        if (transpose_block) quant_row_dual_kernel<T, DIV, RND, 2><<<grid, 256, 0, st>>>(x, ld, q_row, s_row, q_blk, s_blk, (int)M, (int)N, nb_n, nb_m); \
-        else quant_row_dual_kernel<T, DIV, RND, 1><<<grid, 256, 0, st>>>(x, ld, q_row, s_row, q_blk, s_blk, (int)M, (int)N, nb_n, nb_m); \
+        if (transpose_block) launch_early_if(quantise_early(M, N), quant_row_dual_kernel<T, DIV, RND, 2>, dim3(grid), dim3(256), 0, st, x, ld, q_row, s_row, q_blk, s_blk, (int)M, (int)N, nb_n, nb_m); \
+        else launch_early_if(quantise_early(M, N), quant_row_dual_kernel<T, DIV, RND, 1>, dim3(grid), dim3(256), 0, st, x, ld, q_row, s_row, q_blk, s_blk, (int)M, (int)N, nb_n, nb_m); \
     } while (0)
         if (div_mode == CINN_DIV_FULL) { if (round_scale) CINN_D(CINN_DIV_FULL, true); else CINN_D(CINN_DIV_FULL, false); }
         else                           { if (round_scale) CINN_D(CINN_DIV_RN, true);   else CINN_D(CINN_DIV_RN, false); }
@@ -2033,6 +2049,8 @@ constexpr int MAX_SEGMENT_EXPERTS = 1024;
 __global__ void __launch_bounds__(256)
 segment_tiles_kernel(const int64_t* __restrict__ starts, const int64_t* __restrict__ ends, int E, int64_t T,
                      int* __restrict__ kb_start, int* __restrict__ tile_src, int* __restrict__ tile_cnt, int max_tiles) {
+    pdl_wait();
+    pdl_trigger();
     constexpr int PER = MAX_SEGMENT_EXPERTS / 256;         // consecutive experts of a thread
     __shared__ int s_first[MAX_SEGMENT_EXPERTS + 1], s_src[MAX_SEGMENT_EXPERTS], s_rows[MAX_SEGMENT_EXPERTS];
     __shared__ long long s_warp[8];
@@ -2087,7 +2105,7 @@ segment_tiles_kernel(const int64_t* __restrict__ starts, const int64_t* __restri
 int segment_tiles(const int64_t* starts, const int64_t* ends, int E, int64_t T, int* kb_start, int* tile_src, int* tile_cnt,
                   int max_tiles, cudaStream_t st) {
     CINN_CHECK_ARG(E >= 1 && E <= MAX_SEGMENT_EXPERTS && T >= 0 && T < (1LL << 31) && max_tiles >= 1, "segment_tiles: 1 <= experts <= 1024");
-    segment_tiles_kernel<<<1, 256, 0, st>>>(starts, ends, E, T, kb_start, tile_src, tile_cnt, max_tiles);
+    launch_dependent(segment_tiles_kernel, dim3(1), dim3(256), 0, st, starts, ends, E, T, kb_start, tile_src, tile_cnt, max_tiles);
     CINN_CHECK_LAUNCH();
     return CINN_OK;
 }
@@ -2151,7 +2169,7 @@ int quantize_dual_segmented(const void* x, int dtype, int64_t T, int64_t N, void
             attr_err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, DUAL_SMEM_BYTES);      \
         });                                                                                                           \
         CINN_CHECK_CUDA(attr_err);                                                                                    \
-        kern<<<grid, 256, DUAL_SMEM_BYTES, st>>>(tm, (uint8_t*)q_row, s_row, (uint8_t*)q_col, s_col, max_tiles * 128, (int)N, \
+        launch_early_if(quantise_early(T, N), kern, dim3(grid), dim3(256), DUAL_SMEM_BYTES, st, tm, (uint8_t*)q_row, s_row, (uint8_t*)q_col, s_col, max_tiles * 128, (int)N, \
                                                  nb_n, max_tiles, tile_src, tile_cnt, n_tiles);                       \
     } while (0)
 #define CINN_DS(TT, DIV) do { if (block) CINN_DSM(TT, DIV, 2); else CINN_DSM(TT, DIV, 0); } while (0)
@@ -2176,9 +2194,9 @@ int requant_row_to_block_segmented(const void* xq, const float* xs, int64_t K, v
         const int64_t tiles = (int64_t)nb * max_tiles;
         const int grid = (int)(tiles < (int64_t)sm_count() * 2 ? tiles : (int64_t)sm_count() * 2);
         if (div_mode == CINN_DIV_FULL)
-            requant_seg_t_kernel<CINN_DIV_FULL><<<grid, 256, 0, st>>>((const uint8_t*)xq, xs, (uint8_t*)out, scales, M, (int)K, nb, tile_src, tile_cnt, n_tiles);
+            launch_early_if(quantise_early(M, K), requant_seg_t_kernel<CINN_DIV_FULL>, dim3(grid), dim3(256), 0, st, (const uint8_t*)xq, xs, (uint8_t*)out, scales, M, (int)K, nb, tile_src, tile_cnt, n_tiles);
         else
-            requant_seg_t_kernel<CINN_DIV_RN><<<grid, 256, 0, st>>>((const uint8_t*)xq, xs, (uint8_t*)out, scales, M, (int)K, nb, tile_src, tile_cnt, n_tiles);
+            launch_early_if(quantise_early(M, K), requant_seg_t_kernel<CINN_DIV_RN>, dim3(grid), dim3(256), 0, st, (const uint8_t*)xq, xs, (uint8_t*)out, scales, M, (int)K, nb, tile_src, tile_cnt, n_tiles);
         CINN_CHECK_LAUNCH();
         return CINN_OK;
     }
@@ -2214,7 +2232,7 @@ int swiglu_quant_block(const void* h12, int dtype, int64_t T, int64_t I, void* q
     CINN_CHECK_ARG(total < (1LL << 31) && s_row && s_blk && !(seg && round_scale), "swiglu + row + block quantiser: bad arguments");
     const int grid = (int)(total < cap ? total : cap);
 #define CINN_SB(T_, RND, EXACT, SEG)                                                                                              \
-    swiglu_row_block_kernel<T_, RND, EXACT, SEG><<<grid, 256, 0, st>>>((const T_*)h12, (uint8_t*)q_row, s_row, (uint8_t*)q_blk, s_blk,  \
+    launch_early_if(quantise_early(T, I), swiglu_row_block_kernel<T_, RND, EXACT, SEG>, dim3(grid), dim3(256), 0, st, (const T_*)h12, (uint8_t*)q_row, s_row, (uint8_t*)q_blk, s_blk,  \
         seg ? seg->max * 128 : (int)T, (int)I, nb_n, nb_m, (int)total, seg ? seg->src : nullptr, seg ? seg->cnt : nullptr, seg ? seg->n : nullptr)
 #define CINN_SBT(T_) do { if (seg) CINN_SB(T_, false, false, true); else if (round_scale) CINN_SB(T_, true, true, false); else CINN_SB(T_, false, true, false); } while (0)
     if (dtype == CINN_BF16) CINN_SBT(__nv_bfloat16);
@@ -2234,7 +2252,7 @@ int swiglu_backward_quant_dual(const void* h12, const void* dh, int dtype, int64
     CINN_CHECK_ARG(total < (1LL << 31) && dh && aligned16(dh) && s_row && s_col && !(seg && round_scale), "swiglu backward + dual quantiser: bad arguments");
     const int grid = (int)(total < cap ? total : cap);
 #define CINN_SD(T_, RND, EXACT, SEG)                                                                                              \
-    swiglu_backward_dual_kernel<T_, RND, EXACT, SEG><<<grid, 256, 0, st>>>((const T_*)h12, (const T_*)dh, (uint8_t*)q_row, s_row,       \
+    launch_early_if(quantise_early(T, I), swiglu_backward_dual_kernel<T_, RND, EXACT, SEG>, dim3(grid), dim3(256), 0, st, (const T_*)h12, (const T_*)dh, (uint8_t*)q_row, s_row,       \
         (uint8_t*)q_col, s_col, seg ? seg->max * 128 : (int)T, (int)I, nb_i, nb_m, (int)total, seg ? seg->src : nullptr,               \
         seg ? seg->cnt : nullptr, seg ? seg->n : nullptr)
 #define CINN_SDT(T_) do { if (seg) CINN_SD(T_, false, false, true); else if (round_scale) CINN_SD(T_, true, true, false); else CINN_SD(T_, false, true, false); } while (0)
@@ -2328,8 +2346,8 @@ static int launch_swiglu(const T* h12, int64_t T_rows, int64_t I, uint8_t* q, fl
     if (blocks > cap) blocks = cap;
     const int64_t n_hw = blocks * 16;
     const int sr = (int)(n_hw / nb), sc = (int)(n_hw % nb);
-    if (div_mode == CINN_DIV_FULL) swiglu_quant_row_kernel<T, CINN_DIV_FULL><<<(unsigned)blocks, 256, 0, st>>>(h12, q, scales, (int)I, nb, tiles, sr, sc, n_rows_dev);
-    else swiglu_quant_row_kernel<T, CINN_DIV_RN><<<(unsigned)blocks, 256, 0, st>>>(h12, q, scales, (int)I, nb, tiles, sr, sc, n_rows_dev);
+    if (div_mode == CINN_DIV_FULL) launch_early_if(quantise_early(T_rows, I), swiglu_quant_row_kernel<T, CINN_DIV_FULL>, dim3((unsigned)blocks), dim3(256), 0, st, h12, q, scales, (int)I, nb, tiles, sr, sc, n_rows_dev);
+    else launch_early_if(quantise_early(T_rows, I), swiglu_quant_row_kernel<T, CINN_DIV_RN>, dim3((unsigned)blocks), dim3(256), 0, st, h12, q, scales, (int)I, nb, tiles, sr, sc, n_rows_dev);
     CINN_CHECK_LAUNCH();
     return CINN_OK;
 }

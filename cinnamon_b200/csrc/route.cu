@@ -50,6 +50,8 @@ template <int VPL, typename L>      // expert values per lane, E <= 32 * VPL
 __global__ void __launch_bounds__(256)
 route_topk_kernel(const L* __restrict__ logits, const float* __restrict__ bias, int T, int E, int top_k, int tokens_per_cta,
                   int* __restrict__ top_experts, float* __restrict__ top_gates, int* __restrict__ hist) {
+    pdl_wait();
+    pdl_trigger();
     __shared__ int s_hist[ROUTE_MAX_EXPERTS];
     for (int e = threadIdx.x; e < E; e += 256) s_hist[e] = 0;
     __syncthreads();
@@ -113,6 +115,8 @@ route_topk_kernel(const L* __restrict__ logits, const float* __restrict__ bias, 
 
 __global__ void __launch_bounds__(256)
 route_scan_kernel(int* __restrict__ hist, int n_ctas, int E, int* __restrict__ totals) {
+    pdl_wait();
+    pdl_trigger();
     const int lane = threadIdx.x & 31, e = blockIdx.x * 8 + (threadIdx.x >> 5);
     if (e >= E) return;
     int carry = 0;
@@ -146,6 +150,8 @@ route_scatter_kernel(const int* __restrict__ top_experts, const float* __restric
                      float* __restrict__ sorted_scores, int64_t* __restrict__ sorted_experts, int64_t* __restrict__ counts,
                      int64_t* __restrict__ starts, int64_t* __restrict__ ends, int64_t* __restrict__ pair_pos,
                      float* __restrict__ pair_gate) {
+    pdl_wait();
+    pdl_trigger();
     __shared__ int s_next[ROUTE_MAX_EXPERTS];                                  // next free row of every expert
     __shared__ int s_warp[8];
     __shared__ int s_pos[ROUTE_MAX_TOKENS_PER_CTA * ROUTE_MAX_TOPK];
@@ -252,7 +258,7 @@ int64_t moe_route_workspace_ints(int64_t T, int E) {
 template <typename L>
 static void launch_topk(const L* logits, const float* bias, int T, int E, int top_k, int per, int n_ctas, int* top_experts,
                         float* top_gates, int* hist, cudaStream_t st) {
-#define CINN_TOPK(V) route_topk_kernel<V, L><<<n_ctas, 256, 0, st>>>(logits, bias, T, E, top_k, per, top_experts, top_gates, hist)
+#define CINN_TOPK(V) launch_dependent(route_topk_kernel<V, L>, dim3(n_ctas), dim3(256), 0, st, logits, bias, T, E, top_k, per, top_experts, top_gates, hist)
     if (E <= 32) CINN_TOPK(1);
     else if (E <= 64) CINN_TOPK(2);
     else if (E <= 128) CINN_TOPK(4);
@@ -291,10 +297,10 @@ int moe_route(const void* logits, int logits_dtype, const float* bias, int64_t T
     else launch_topk((const __half*)logits, bias, (int)T, E, top_k, per, n_ctas, top_experts, top_gates, hist, st);
     CINN_CHECK_LAUNCH();
     if (totals) {
-        route_scan_kernel<<<(E + 7) / 8, 256, 0, st>>>(hist, n_ctas, E, totals);
+        launch_dependent(route_scan_kernel, dim3((E + 7) / 8), dim3(256), 0, st, hist, n_ctas, E, totals);
         CINN_CHECK_LAUNCH();
     }
-    route_scatter_kernel<<<n_ctas, 256, 0, st>>>(top_experts, top_gates, hist, totals, (int)T, E, top_k, per, token_indices, sorted_scores,
+    launch_dependent(route_scatter_kernel, dim3(n_ctas), dim3(256), 0, st, top_experts, top_gates, hist, totals, (int)T, E, top_k, per, token_indices, sorted_scores,
                                                  sorted_experts, counts, starts, ends, pair_pos, pair_gate);
     CINN_CHECK_LAUNCH();
     return CINN_OK;
