@@ -844,6 +844,22 @@ def test_linear_on_few_rows_in_one_kernel(K, M, N, Kd, dtype, rs, div):
         assert float((out.double() - whole.double()).norm() / whole.double().norm()) < 2.0 ** -9
 
 
+@pytest.mark.parametrize("M,N,Kd", [(1, 128, 256), (128, 1024, 512), (82, 3776, 512), (4, 1344, 1024), (33, 200, 144), (17, 1000, 656)])
+@pytest.mark.parametrize("dtype,rs", [(torch.bfloat16, True), (torch.float32, False)])
+def test_linear_on_few_rows_has_the_bits_of_two_kernels(K, M, N, Kd, dtype, rs):
+    """One K block per CTA: the cluster scales and adds the products in one step, in the order of the separate kernels."""
+    g = torch.Generator(device="cuda").manual_seed(M * 7 + N + Kd)
+    layer = K.FP8Linear(Kd, N, round_scale=rs).cuda()
+    x = torch.randn(M, Kd, device="cuda", generator=g).mul_(3).to(dtype)
+    n = K.launch_count
+    with torch.no_grad():
+        out = layer(x)
+    assert K.launch_count - n == 1
+    xq, xs = K.quantize_fp8_rowwise(x, 128, rs)
+    wq, ws = K.quantize_fp8_blockwise(layer.weight.detach())
+    assert torch.equal(out, K._gemm(xq, xs, wq, 0, ws, ws.stride(1), ws.stride(0), M, N, Kd, torch.bfloat16, whole=True))
+
+
 def test_linear_on_few_rows_any_alignment(K):
     """One launch for rows that fit, two for those that do not (rows off 16-byte boundaries, strides, a reduction too long for it to
     pay); the same result."""
