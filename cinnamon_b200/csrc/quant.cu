@@ -1743,10 +1743,11 @@ static int launch_quant_linear(const TX* x, int64_t ldx, uint8_t* xq, float* xs,
     if (blocks > cap) blocks = cap;
     const int64_t n_hw = blocks * 16;
     const unsigned grid = (unsigned)(w_blocks + blocks);
-    // As in quantise_early, and only a grid that fits on the SMs at once (eight blocks each): 403 x 2048 -> 12928 47 -> 53 us.  Few rows are not
-    // multiplied in long tiles and gain up to 3072 columns (12 x 2368 -> 1856 12.4 -> 11.6, 100 x 3072 -> 2048 16.4 -> 13.9), not at 4096 (40 x 4096
-    // -> 4096 26.7 -> 27.5).
-#define CINN_Q(DIV, RND) launch_early_if((int64_t)grid <= 8 * (int64_t)sm_count() && (K <= 2048 || (M <= 128 && K <= 3072)), quant_linear_kernel<TX, TW, DIV, RND>, dim3(grid), dim3(256), 0, st, x, ldx, xq, xs, tiles, (int)(n_hw / nb), (int)(n_hw % nb), w, ldw, wq, ws, (int)N, (int)K, nb, (int)w_blocks)
+    // As in quantise_early, and only where the grid fits on the SMs at once (eight blocks each) and the weight's blocks take half of that at most:
+    // 332 x 1408 -> 11712 (1012 of them) 26.8 -> 29.2 us, 40 x 1600 -> 7000 (715) 18.5 -> 19.0, but 800 x 768 -> 9000 (426) 20.5 -> 19.6, 2595 x
+    // 512 -> 7104 24.6 -> 23.0, 8000 x 512 -> 1024 17.4 -> 15.5.  Few rows are not multiplied in long tiles and gain up to 3072 columns (12 x 2368 ->
+    // 1856 12.3 -> 11.3, 100 x 3072 -> 2048 16.1 -> 13.8), not at 4096 (40 x 4096 -> 4096 26.7 -> 27.5).
+#define CINN_Q(DIV, RND) launch_early_if((int64_t)grid <= cap && 2 * w_blocks <= cap && (K <= 2048 || (M <= 128 && K <= 3072)), quant_linear_kernel<TX, TW, DIV, RND>, dim3(grid), dim3(256), 0, st, x, ldx, xq, xs, tiles, (int)(n_hw / nb), (int)(n_hw % nb), w, ldw, wq, ws, (int)N, (int)K, nb, (int)w_blocks)
     if (div_mode == CINN_DIV_FULL) { if (round_scale) CINN_Q(CINN_DIV_FULL, true); else CINN_Q(CINN_DIV_FULL, false); }
     else                           { if (round_scale) CINN_Q(CINN_DIV_RN, true);   else CINN_Q(CINN_DIV_RN, false); }
 #undef CINN_Q
