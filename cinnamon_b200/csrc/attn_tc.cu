@@ -1317,10 +1317,10 @@ static Plan make_plan(int64_t B, int64_t H, int64_t L, int64_t K, int64_t Dqk, i
 // each that grows with the widths, and every query tile costs its start and its probabilities; what was picked and the parts come
 // first) against the gathers' (K rows of Dqk + Dv elements per query and a constant per row).  The tiles take the larger of their number over
 // the SMs and of the longest query tile's chain: with the sum of both, or the first alone, the estimate was 11 % off on average, with the
-// larger 5 (backward).  Fitted to 420 calls, B = 1 ... 32, L = 257 ... 4081, K = 32 ... 256, widths 64 ... 192, bf16 and fp32.  On 170 others the way
-// that is taken costs more than the faster one would by 0.3 (forward) and 0.1 % (backward) in bf16, 0.2 and 0.1 in fp32, at worst 1.12 times;
-// without the chain, fitted to 70 calls, by 0.4, 0.5, 0.7 and 2.4, at worst 1.74; with constants of a slower forward and fewer lengths by 3.0, 0.5,
-// 3.4 and 3.5, at worst 1.9.  Gathers against tiles: 16 x 4 x 2286 queries, 64 picks of 64 / 128 in bf16 838 and 403 us, 4 x 8 x 3965,
+// larger 5 (backward).  Fitted to 420 calls, B = 1 ... 32, L = 256 ... 4052, K = 32 ... 256, widths 64 ... 192, bf16 and fp32.  On 400 others the way
+// that is taken costs more than the faster one would by 0.1 (forward) and 0.2 % (backward) in bf16, 0.2 and 0.2 in fp32, at worst 1.17 times;
+// with constants of a slower forward, fewer lengths and no chain by 7, 2, 3.4 and 4.4, at worst 2.5.  Gathers against tiles:
+// 16 x 4 x 2286 queries, 64 picks of 64 / 128 in bf16 838 and 403 us, 4 x 8 x 3965,
 // 64 of 192 / 128 861 and 581; backward 4 x 4 x 2033, 64 of 128 / 128 in fp32 549 and 428, 1 x 8 x 1965, 32 of 128 / 64 in bf16 131 and 176.
 static std::atomic<int> g_mode{-1};         // -1: by the estimate; 0 / 1: never / wherever the tiles can (tests, measurements)
 int set_mode(int mode) { return g_mode.exchange(mode); }
@@ -1336,17 +1336,17 @@ static bool dense_pays(const Plan& p, bool backward) {
     // cycles of a tile, how much of the longest query tile's chain counts, cycles of a query tile, microseconds before the tiles
     double tile, chain, query_tile, first, gather_us;
     if (!backward) {
-        tile = parts ? 3870.0 + 35.6 * p.dp : 3590.0 + 5.97 * p.dp;
-        chain = parts ? 0.81 : 0.85;
-        query_tile = parts ? 2570.0 + 49.7 * p.K : 4810.0 + 57.6 * p.K;
-        first = parts ? 21.3 + 2.02 * picked + 1.91 * split : 20.0 + 3.27 * picked;
-        gather_us = wide ? 10.1 + gathered / 14.44e6 + queries * p.K / 44.3e3 : 11.8 + gathered / 9.85e6 + queries * p.K / 27.9e3;
+        tile = parts ? 3740.0 + 34.2 * p.dp : 3610.0 + 4.28 * p.dp;
+        chain = parts ? 0.81 : 0.76;
+        query_tile = parts ? 3850.0 + 67.0 * p.K : 4900.0 + 50.1 * p.K;
+        first = parts ? 17.7 + 1.75 * picked + 1.80 * split : 20.6 + 3.01 * picked;
+        gather_us = wide ? 9.8 + gathered / 14.95e6 + queries * p.K / 43.8e3 : 12.1 + gathered / 10.15e6 + queries * p.K / 26.6e3;
     } else {
-        tile = parts ? 10530.0 + 126.2 * widths : 9120.0 + 40.4 * widths;
-        chain = parts ? 0.89 : 0.85;
-        query_tile = parts ? 53.8 * p.K : 19000.0 + 95.3 * p.K;
-        first = parts ? 31.8 + 1.95 * picked + 2.97 * split : 29.9 + 1.19 * picked;
-        gather_us = wide ? 24.1 + gathered / 4.47e6 + queries * p.K / 65.9e3 : 40.6 + gathered / 2.71e6 + queries * p.K / 26.3e3;
+        tile = parts ? 9190.0 + 126.6 * widths : 9510.0 + 39.2 * widths;
+        chain = parts ? 0.905 : 0.814;
+        query_tile = parts ? 112.0 * p.K : 15160.0 + 117.6 * p.K;
+        first = parts ? 26.8 + 0.84 * picked + 2.93 * split : 24.9 + 0.46 * picked;
+        gather_us = wide ? 28.6 + gathered / 4.40e6 + queries * p.K / 76.2e3 : 42.6 + gathered / 2.76e6 + queries * p.K / 23.5e3;
     }
     const double ctas = backward ? 1.0 : (double)p.nv;      // a forward CTA computes 64 columns of the output
     const double all = ctas * tiles * tile / 148.0, longest = chain * (double)(p.Lp / T) * tile;
