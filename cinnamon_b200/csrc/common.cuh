@@ -75,12 +75,13 @@ inline cudaError_t launch_dependent(void (*kern)(P...), dim3 grid, dim3 block, s
 
 int sm_count();   // SMs of the current device (cached per device)
 
-// launch_dependent if `early`, else a plain launch: the kernel starts when the one before it has ended
+// launch_dependent if `early`, else a plain launch: the kernel starts when the one before it has ended.  Both leave an error
+// where CINN_CHECK_LAUNCH finds it.
 template <typename... P, typename... A>
 inline cudaError_t launch_early_if(bool early, void (*kern)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A&&... args) {
     if (early) return launch_dependent(kern, grid, block, smem, st, static_cast<A&&>(args)...);
     kern<<<grid, block, smem, st>>>(static_cast<P>(args)...);
-    return cudaGetLastError();
+    return cudaPeekAtLastError();
 }
 // Whether a quantiser of so many rows starts early.  Short ones gain the launch.  In front of a GEMM of long tiles an early start costs more than it
 // wins, up to a tile's time: 403 x 4032 -> 12928 80 -> 96 us, 1824 x 6976 -> 8832 forward and backward 458 -> 470, 16384 x 7168 -> 18432 7020 ->

@@ -120,3 +120,56 @@ def test_convert_to_fp8_selection_rules(built):
     assert isinstance(b.w3, K.FP8Linear) and not b.w3.round_scale and b.w3.bias is not None
     assert type(b.attn_proj) is torch.nn.Linear and type(b.router) is torch.nn.Linear and type(b.tiny) is torch.nn.Linear
     assert sorted(n for n, _ in b.w1.named_parameters()) == ["weight"]
+
+
+def test_a_launch_that_fails_is_reported(built, tmp_path):
+    """Early or plain, a launch that the CUDA runtime refuses is an error of the call and counts as none: the launch helpers over a
+    runtime of this test's own, whose launches fail and whose last error is cleared when it is read."""
+    import subprocess
+    from cinnamon_b200 import build as B
+    exe, runtime, calls = tmp_path / "launch", tmp_path / "runtime.cpp", tmp_path / "calls.cu"
+    runtime.write_text("""
+int last = 0, next = 0;                                       // errors: what is pending, what the next launch ends with
+static int launched() { if (next != 0) last = next; return next; }
+extern "C" {
+int cudaGetLastError() { const int e = last; last = 0; return e; }
+int cudaPeekAtLastError() { return last; }
+const char* cudaGetErrorString(int) { return "refused"; }
+int cudaLaunchKernel() { return launched(); }
+int cudaLaunchKernelExC() { return launched(); }
+unsigned __cudaPushCallConfiguration() { return 0; }
+int __cudaPopCallConfiguration() { return 0; }
+void** __cudaRegisterFatBinary(void*) { static void* h; return &h; }
+void __cudaRegisterFatBinaryEnd(void**) {}
+void __cudaUnregisterFatBinary(void**) {}
+void __cudaRegisterFunction() {}
+char __cudaInitModule(void**) { return 0; }
+}
+""")
+    calls.write_text("""
+#include "common.cuh"
+extern int last, next;
+namespace cinn {
+std::atomic<int64_t> g_launches{0};
+void set_error(const char*, ...) {}
+}
+__global__ void kernel(int) {}
+static int call(bool early) {
+    cinn::launch_early_if(early, kernel, dim3(1), dim3(32), 0, nullptr, 1);
+    CINN_CHECK_LAUNCH();
+    return CINN_OK;
+}
+int main() {
+    for (int early = 0; early < 2; ++early) {
+        next = 0;
+        if (call(early) != CINN_OK || cinn::g_launches != early + 1) return 10 + early;
+        next = cudaErrorInvalidConfiguration;
+        if (call(early) != CINN_ERR_CUDA || cinn::g_launches != early + 1 || last != 0) return 20 + early;
+    }
+    return 0;
+}
+""")
+    p = subprocess.run([B._nvcc(), *B.NVCC_FLAGS, "-cudart", "none", "-I" + B.CSRC, str(calls), str(runtime), "-o", str(exe)],
+                       capture_output=True, text=True, timeout=300)
+    assert p.returncode == 0, p.stderr
+    assert subprocess.run([str(exe)], timeout=60).returncode == 0
