@@ -73,6 +73,19 @@ inline cudaError_t launch_dependent(void (*kern)(P...), dim3 grid, dim3 block, s
     return cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...);
 }
 
+// Lets a kernel use up to `bytes` of dynamic shared memory, once per device.  The limit belongs to the function, not to a
+// launch or a thread: it is set to the most any launch can ask for, so that no thread lowers it under another one.
+template <auto KERN>
+inline int allow_smem_once(size_t bytes) {
+    static std::atomic<uint64_t> done{0};
+    int dev = 0;
+    CINN_CHECK_CUDA(cudaGetDevice(&dev));
+    if (dev >= 0 && dev < 64 && (done.load(std::memory_order_acquire) >> dev & 1)) return CINN_OK;
+    CINN_CHECK_CUDA(cudaFuncSetAttribute(KERN, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+    if (dev >= 0 && dev < 64) done.fetch_or(1ULL << dev, std::memory_order_release);
+    return CINN_OK;
+}
+
 int sm_count();   // SMs of the current device (cached per device)
 
 // launch_dependent if `early`, else a plain launch: the kernel starts when the one before it has ended.  Both leave an error

@@ -631,19 +631,6 @@ static size_t smem_bytes(int E) {
     return n;
 }
 
-// Lets a kernel use up to `bytes` of dynamic shared memory, once per device.  The limit belongs to the function, not to a
-// launch or a thread: it is set to the most any launch can ask for, so that no thread lowers it under another one.
-template <auto KERN>
-static int allow_smem_once(size_t bytes) {
-    static std::atomic<uint64_t> done{0};
-    int dev = 0;
-    CINN_CHECK_CUDA(cudaGetDevice(&dev));
-    if (dev >= 0 && dev < 64 && (done.load(std::memory_order_acquire) >> dev & 1)) return CINN_OK;
-    CINN_CHECK_CUDA(cudaFuncSetAttribute(KERN, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
-    if (dev >= 0 && dev < 64) done.fetch_or(1ULL << dev, std::memory_order_release);
-    return CINN_OK;
-}
-
 // Output map for the TMA-store epilogue: (rows, N) of a 2-byte type, boxes of 64 columns x 128 rows, 128-byte swizzle.
 // Sets p.tma_out; when the output cannot go through TMA the (unused) operand map is passed in its place.
 static int make_out_map(CUtensorMap* tc, const CUtensorMap& fallback, GemmParams& p, int out_dtype, int64_t rows,

@@ -625,13 +625,7 @@ static int indexer_run(const T* q, const T* k, const T* w, __half* out, int B, i
     const uint32_t qbox[4] = {64, 1, ITC_T, 1}, kbox[3] = {64, ITC_T, 1};
     if (encode_map(&tq, q, 4, qd, qst, qbox, type, CU_TENSOR_MAP_SWIZZLE_128B) || encode_map(&tk, k, 3, kd, kst, kbox, type, CU_TENSOR_MAP_SWIZZLE_128B))
         return -1;                                                  // (strides that the driver does not take)
-    static std::atomic<uint64_t> allowed{0};                        // devices on which the kernel may use its shared memory
-    int dev = 0;
-    CINN_CHECK_CUDA(cudaGetDevice(&dev));
-    if (dev >= 64 || !(allowed.load(std::memory_order_acquire) >> dev & 1)) {
-        CINN_CHECK_CUDA(cudaFuncSetAttribute(indexer_run_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, IRUN_SMEM_BYTES));
-        if (dev < 64) allowed.fetch_or(1ULL << dev, std::memory_order_release);
-    }
+    if (const int failed = allow_smem_once<indexer_run_kernel<T>>(IRUN_SMEM_BYTES)) return failed;
     const int grid = a.tiles < sm_count() ? a.tiles : sm_count();
     CINN_CHECK_CUDA(launch_dependent(indexer_run_kernel<T>, dim3(grid), dim3(IRUN_THREADS), IRUN_SMEM_BYTES, st, tq, tk, w, out, a));
     CINN_CHECK_LAUNCH();

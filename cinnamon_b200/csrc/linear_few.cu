@@ -256,13 +256,7 @@ static int slices_of(int64_t N, int64_t K) {
 template <typename TX, int DIV, bool ROUND>
 static int launch(const TX* x, int64_t ldx, const float* w, int64_t ldw, __nv_bfloat16* out, int M, int N, int K, cudaStream_t st) {
     constexpr auto kern = fp8_linear_few_kernel<TX, DIV, ROUND>;
-    static std::atomic<uint64_t> allowed{0};               // devices on which the kernel may use its shared memory
-    int dev = 0;
-    CINN_CHECK_CUDA(cudaGetDevice(&dev));
-    if (dev >= 64 || !(allowed.load(std::memory_order_acquire) >> dev & 1)) {
-        CINN_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));
-        if (dev < 64) allowed.fetch_or(1ULL << dev, std::memory_order_release);
-    }
+    if (const int failed = allow_smem_once<kern>(SMEM_BYTES)) return failed;
     const int slices = slices_of(N, K);
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)slices, (unsigned)((N + TILE - 1) / TILE), 1);

@@ -11,7 +11,6 @@
 // reduces amax with warp shuffles, and writes packed e4m3 (4-16 bytes per lane).
 #include "elements.cuh"
 #include "tma.cuh"
-#include <mutex>
 
 namespace cinn {
 
@@ -1846,13 +1845,8 @@ static int dispatch_dual(const T* x, int64_t M, int64_t N, int64_t ld, uint8_t* 
         const int grid = (int)(total < 2 * (int64_t)sm_count() ? total : 2 * (int64_t)sm_count());
 #define CINN_D(DIV, RND)                                                                                              \
     do {                                                                                                              \
-        auto kern = quant_row_dual_tma_kernel<T, DIV, RND>;                                                           \
-        static std::once_flag once;                                                                                   \
-        static cudaError_t attr_err = cudaSuccess;                                                                    \
-        std::call_once(once, [&] {                                                                                    \
-            attr_err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, DUAL_SMEM_BYTES);      \
-        });                                                                                                           \
-        CINN_CHECK_CUDA(attr_err);                                                                                    \
+        constexpr auto kern = quant_row_dual_tma_kernel<T, DIV, RND>;                                                 \
+        if (const int failed = allow_smem_once<kern>(DUAL_SMEM_BYTES)) return failed;                                 \
         launch_early_if(quantise_early(M, N), kern, dim3(grid), dim3(256), DUAL_SMEM_BYTES, st, tm, q_row, s_row, q_col, s_col, (int)M, (int)N, nb_n, nb_m, (int)total); \
     } while (0)
         if (div_mode == CINN_DIV_FULL) { if (round_scale) CINN_D(CINN_DIV_FULL, true); else CINN_D(CINN_DIV_FULL, false); }
@@ -1894,15 +1888,10 @@ static int dispatch_row_block(const T* x, int64_t M, int64_t N, int64_t ld, uint
         const int grid = (int)(total < 2 * (int64_t)sm_count() ? total : 2 * (int64_t)sm_count());
 #define CINN_D(DIV, RND)                                                                                              \
     do {                                                                                                              \
-        auto kern = transpose_block ? quant_row_dual_tma_kernel<T, DIV, RND, 2> : quant_row_dual_tma_kernel<T, DIV, RND, 1>; \
-        static std::once_flag once;                                                                                   \
-        static cudaError_t attr_err = cudaSuccess;                                                                    \
-        std::call_once(once, [&] {                                                                                    \
-            attr_err = cudaFuncSetAttribute(quant_row_dual_tma_kernel<T, DIV, RND, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, DUAL_SMEM_BYTES); \
-            if (attr_err == cudaSuccess)                                                                              \
-                attr_err = cudaFuncSetAttribute(quant_row_dual_tma_kernel<T, DIV, RND, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, DUAL_SMEM_BYTES); \
-        });                                                                                                           \
-        CINN_CHECK_CUDA(attr_err);                                                                                    \
+        constexpr auto turned = quant_row_dual_tma_kernel<T, DIV, RND, 2>, straight = quant_row_dual_tma_kernel<T, DIV, RND, 1>;\
+        const int failed = transpose_block ? allow_smem_once<turned>(DUAL_SMEM_BYTES) : allow_smem_once<straight>(DUAL_SMEM_BYTES);\
+        if (failed) return failed;                                                                                    \
+        const auto kern = transpose_block ? turned : straight;                                                        \
         launch_early_if(quantise_early(M, N), kern, dim3(grid), dim3(256), DUAL_SMEM_BYTES, st, tm, q_row, s_row, q_blk, s_blk, (int)M, (int)N, nb_n, nb_m, (int)total); \
     } while (0)
         if (div_mode == CINN_DIV_FULL) { if (round_scale) CINN_D(CINN_DIV_FULL, true); else CINN_D(CINN_DIV_FULL, false); }
@@ -2163,13 +2152,8 @@ int quantize_dual_segmented(const void* x, int dtype, int64_t T, int64_t N, void
     const int grid = (int)(total < 2 * (int64_t)sm_count() ? total : 2 * (int64_t)sm_count());
 #define CINN_DSM(TT, DIV, MODE)                                                                                              \
     do {                                                                                                              \
-        auto kern = quant_row_dual_seg_kernel<TT, DIV, MODE>;                                                         \
-        static std::once_flag once;                                                                                   \
-        static cudaError_t attr_err = cudaSuccess;                                                                    \
-        std::call_once(once, [&] {                                                                                    \
-            attr_err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, DUAL_SMEM_BYTES);      \
-        });                                                                                                           \
-        CINN_CHECK_CUDA(attr_err);                                                                                    \
+        constexpr auto kern = quant_row_dual_seg_kernel<TT, DIV, MODE>;                                               \
+        if (const int failed = allow_smem_once<kern>(DUAL_SMEM_BYTES)) return failed;                                 \
         launch_early_if(quantise_early(T, N), kern, dim3(grid), dim3(256), DUAL_SMEM_BYTES, st, tm, (uint8_t*)q_row, s_row, (uint8_t*)q_col, s_col, max_tiles * 128, (int)N, \
                                                  nb_n, max_tiles, tile_src, tile_cnt, n_tiles);                       \
     } while (0)
