@@ -343,7 +343,6 @@ __global__ void __launch_bounds__(FwdShape<NS, ND, PAIRS>::THREADS, 3 - PAIRS)
 attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                 const __grid_constant__ CUtensorMap tmV, const FwdArgs a) {
     pdl_wait();
-    pdl_trigger();
     using S = FwdShape<NS, ND, PAIRS>;
     constexpr int TMA_WARP = 8 * PAIRS, MMA_WARP = TMA_WARP + 1;
     extern __shared__ uint8_t smem_raw[];
@@ -370,7 +369,10 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         for (int i = 0; i < 8; ++i) mbar_init(pair0 + 8 * i, 2);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    if (warp == MMA_WARP) tc_alloc(smem_u32(tmem_slot), 256 * PAIRS);
+    if (warp == MMA_WARP) {
+        tc_alloc(smem_u32(tmem_slot), 256 * PAIRS);
+        pdl_trigger();
+    }
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
@@ -839,7 +841,6 @@ attn_bwd_query_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
                       const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmG,
                       const __grid_constant__ CUtensorMap tmDQ, const BwdArgs a) {
     pdl_wait();
-    pdl_trigger();
     using S = QPassShape<NS, ND, NV>;
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
@@ -863,7 +864,10 @@ attn_bwd_query_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
         for (int i = 0; i < 2; ++i) mbar_init(group0 + 8 * i, 4);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    if (warp == 9) tc_alloc(smem_u32(tmem_slot), 512);
+    if (warp == 9) {
+        tc_alloc(smem_u32(tmem_slot), 512);
+        pdl_trigger();
+    }
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
@@ -1095,7 +1099,6 @@ __global__ void __launch_bounds__(KEY_THREADS, 1)
 attn_bwd_key_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmG,
                     const __grid_constant__ CUtensorMap tmDK, const __grid_constant__ CUtensorMap tmDV, const BwdArgs a) {
     pdl_wait();
-    pdl_trigger();
     using S = KPassShape<NS, ND, NV>;
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
@@ -1122,7 +1125,10 @@ attn_bwd_key_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
         for (int i = 0; i < 4; ++i) mbar_init(group0 + 8 * i, 4);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    if (warp == 17) tc_alloc(smem_u32(tmem_slot), 512);
+    if (warp == 17) {
+        tc_alloc(smem_u32(tmem_slot), 512);
+        pdl_trigger();
+    }
     tc_fence_before();
     __syncthreads();
     tc_fence_after();

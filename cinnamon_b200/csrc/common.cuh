@@ -59,6 +59,11 @@ extern std::atomic<int64_t> g_launches;
 // still running, as soon as every block of that one has called pdl_trigger (or has ended); nothing it reads or writes in
 // global memory may come before its pdl_wait, which returns when the kernel before has finished and its writes are visible.
 // What is won is the launch latency and the prologue, which between kernels of 3 - 10 us are a quarter of the time.
+// Two conditions on every kernel that triggers:
+//   - It triggers after its own pdl_wait.  Whatever starts behind it then finds all that came before it done, which the quantisers that
+//     work beside the kernel ahead of them build on: they read and write before they wait, and wait before they end.
+//   - With tensor memory it triggers from the warp that allocates, after the allocation.  The kernels behind allocate before they wait: a block
+//     that triggered first could find its columns taken by one that waits for its end, and neither would get on.
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 

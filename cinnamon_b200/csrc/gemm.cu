@@ -297,7 +297,7 @@ fp8_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
     pdl_wait();                                    // (all of the above is this block's own; from here on, memory is read)
-    pdl_trigger();
+    if (warp == EPI_WARPS + 1) pdl_trigger();
     if constexpr (GROUPED) {
         if (warp == 0) tile_prefix_sum(p, cum, BM, lane);
     }

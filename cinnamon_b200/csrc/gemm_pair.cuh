@@ -173,7 +173,7 @@ fp8_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
     }
     pdl_wait();                                        // (all of the above is this block's own; from here on, memory is read)
-    pdl_trigger();
+    if (warp == PMMA) pdl_trigger();
     if constexpr (GR) {
         if (warp == 0) tile_prefix_sum(p, cum, PM, lane);
     }

@@ -53,7 +53,7 @@ fp8_gemm_rows_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
     }
     if (warp == 5) tc_alloc(smem_u32(tmem_slot), RTMEM_COLS);
     pdl_wait();                                        // (all of the above is this block's own; from here on, memory is read)
-    pdl_trigger();
+    if (warp == 5) pdl_trigger();
     tc_fence_before();
     __syncthreads();
     tc_fence_after();

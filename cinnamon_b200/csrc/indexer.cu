@@ -202,7 +202,7 @@ indexer_tc_kernel(const T* __restrict__ q, const T* __restrict__ k, const T* __r
     }
     if (warp == 0) tc_alloc(smem_u32(tmem_slot), 2 * ITC_T);
     pdl_wait();
-    pdl_trigger();
+    if (warp == 0) pdl_trigger();
     const T* kb = k + b * a.skb;
     const T* qb = q + b * a.sqb;
     load_tile<T>(sK, kb + k0 * a.skk, a.Lk - k0, a.skk, a.skd, a.d, a.dpad, a.vec_k);
@@ -383,7 +383,7 @@ indexer_run_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
     }
     if (warp == IRUN_MMA) tc_alloc(smem_u32(tmem_slot), IRUN_BUFS * ITC_T);
     pdl_wait();
-    pdl_trigger();
+    if (warp == IRUN_MMA) pdl_trigger();
     tc_fence_before();
     __syncthreads();
     tc_fence_after();

@@ -57,9 +57,9 @@ fp8_linear_few_kernel(const TX* __restrict__ x, int64_t ldx, const float* __rest
         for (int i = 0; i < 2; ++i) mbar_init(done0 + 8 * i, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    if (warp == 0) tc_alloc(smem_u32(&tmem_slot), TMEM_COLS);
+    if (warp == 1) tc_alloc(smem_u32(&tmem_slot), TMEM_COLS);        // (warp 0 has the barriers to set up)
     pdl_wait();
-    pdl_trigger();
+    if (warp == 1) pdl_trigger();
     const int slices = gridDim.x, slice = blockIdx.x, n0 = blockIdx.y * TILE;
     const int KB = (K + TILE - 1) / TILE, kb0 = KB * slice / slices, kb1 = KB * (slice + 1) / slices;
     const bool one = slices > 1 && slices == KB;           // a K block per CTA: its products stay unscaled until they are added
@@ -189,7 +189,7 @@ fp8_linear_few_kernel(const TX* __restrict__ x, int64_t ldx, const float* __rest
     if (kb1 > kb0) promote(kb1 - kb0 - 1, sb_old);
     tc_fence_before();
     __syncthreads();
-    if (warp == 0) {
+    if (warp == 1) {
         tc_fence_after();
         tc_dealloc(tmem, TMEM_COLS);
     }
