@@ -5,12 +5,14 @@
 // What has to move is the weight, once.  Quantised by a kernel of its own it moves 1.5 times (4 bytes read, 1 written, 1 read again),
 // and both kernels of a small layer are launch latency.  A CTA takes 128 columns over a part of the reduction; the parts of a
 // column tile are a cluster and add up through distributed shared memory, in order.  Per K block of 128 all 16 warps hold the
-// block of the weight in registers (8 rows of a warp, 16 bytes per lane) with the next one's loads in flight, agree on its
-// amax, write e4m3 into the 128-byte-swizzled B tile, the rows of x into the A tile, and one warp issues the MMAs; the product of
-// the K block before is scaled and added meanwhile.  Every sum runs over whole K blocks in their order.  A CTA with one K block hands over its
+// block of the weight in registers (8 rows of a warp, 16 bytes per lane), agree on its amax, write e4m3 into the 128-byte-swizzled B tile,
+// the rows of x into the A tile, and one warp issues the MMAs.  A CTA with one K block hands over its
 // products as they are, with its rows' scales, and the cluster scales and adds in one step as the separate kernels do: the same bits.
 // (Scaled before, each product was rounded once more: 0.0054 % of the results were not the exact sum in bf16, 0.0045 of the separate
-// kernels'; 120 calls, 1 ... 128 rows, 256 ... 1024 columns.)
+// kernels'; 120 calls, 1 ... 128 rows, 256 ... 1024 columns.)  Without the loop over K blocks, the passes over the rows of x in step and the sums of
+// the other CTAs asked for together: 1 x 512 -> 1024 5.8 -> 4.5 us and 128 x 512 -> 1024 8.5 -> 7.4 (back to back from a graph).  That is the form that linear_few_takes chooses.  A call of the entry point that has
+// more K blocks than CTAs runs the other one: the next block's loads are in flight while one is converted, the product of the block
+// before is scaled and added meanwhile, and every sum runs over whole K blocks in their order.
 //
 // All waits are bounded; cluster barriers are reached by every thread whatever a wait said.
 #include "elements.cuh"
@@ -30,7 +32,6 @@ constexpr int TILE = 128;                  // rows, columns and reduction of an 
 constexpr int TILE_BYTES = TILE * TILE;
 constexpr int SMEM_BYTES = 4 * TILE_BYTES + 1024;      // two A and two B tiles; later 128 x 128 fp32 partial sums
 constexpr int COLS = TILE / (WARPS / 4);   // columns of a promotion warp
-constexpr int TMEM_COLS = 2 * TILE;
 constexpr int MAX_SLICES = 8;              // CTAs of a cluster: the portable limit
 
 constexpr uint32_t IDESC = (1u << 4) | ((uint32_t)(TILE >> 3) << 17) | ((uint32_t)(TILE >> 4) << 24);
@@ -38,10 +39,12 @@ constexpr uint32_t IDESC = (1u << 4) | ((uint32_t)(TILE >> 3) << 17) | ((uint32_
 // byte `b` of row r of an operand tile: 128-byte rows, 16-byte chunks XOR-ed with the row
 __device__ __forceinline__ uint32_t tile_off(int r, int b) { return (uint32_t)(r * 128 + ((((b >> 4) ^ r) & 7) << 4) + (b & 15)); }
 
-template <typename TX, int DIV, bool ROUND>
+// ONE: a K block per CTA, the form that linear_few_takes chooses; otherwise a run of them
+template <typename TX, int DIV, bool ROUND, bool ONE>
 __global__ void __launch_bounds__(THREADS, 1)
 fp8_linear_few_kernel(const TX* __restrict__ x, int64_t ldx, const float* __restrict__ w, int64_t ldw, __nv_bfloat16* __restrict__ out,
                       int M, int N, int K) {
+    constexpr int TMEM_COLS = (ONE ? 1 : 2) * TILE;
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
     __shared__ __align__(8) uint64_t bars[2];
@@ -61,14 +64,14 @@ fp8_linear_few_kernel(const TX* __restrict__ x, int64_t ldx, const float* __rest
     pdl_wait();
     if (warp == 1) pdl_trigger();
     const int slices = gridDim.x, slice = blockIdx.x, n0 = blockIdx.y * TILE;
-    const int KB = (K + TILE - 1) / TILE, kb0 = KB * slice / slices, kb1 = KB * (slice + 1) / slices;
-    const bool one = slices > 1 && slices == KB;           // a K block per CTA: its products stay unscaled until they are added
-    if (tid < TILE) s_row[tid] = 1.0f;
+    const int KB = (K + TILE - 1) / TILE, kb0 = ONE ? slice : KB * slice / slices, kb1 = ONE ? slice + 1 : KB * (slice + 1) / slices;
+    const bool unscaled = ONE && slices > 1;               // products that stay as they are until they are added
+    if (!ONE && tid < TILE) s_row[tid] = 1.0f;
 
     // the K block's piece of the weight: rows warp * 8 + i of the tile, 16 bytes per lane
     const float* wp = w + (int64_t)(n0 + warp * 8) * ldw + lane * 4;
     const int w_rows = min(8, N - n0 - warp * 8);
-    float4 cur[8], nxt[8];
+    float4 cur[8], nxt[ONE ? 1 : 8];
     auto fetch = [&](int kb, float4 (&r)[8]) {
         const bool live = kb < kb1 && kb * TILE + lane * 4 < K;
 #pragma unroll
@@ -94,7 +97,7 @@ fp8_linear_few_kernel(const TX* __restrict__ x, int64_t ldx, const float* __rest
         if (!alive || quarter * 32 >= M) return;
         tc_fence_after();
         float s = s_a[buf][quarter * 32 + lane] * sb;
-        if (one) {
+        if (unscaled) {
             if (group == 0) s_row[quarter * 32 + lane] = s;
             s = 1.0f;
         }
@@ -120,7 +123,7 @@ fp8_linear_few_kernel(const TX* __restrict__ x, int64_t ldx, const float* __rest
         const int buf = it & 1;
         uint8_t* sA = smem + buf * TILE_BYTES;
         uint8_t* sB = smem + (2 + buf) * TILE_BYTES;
-        fetch(kb + 1, nxt);
+        if constexpr (!ONE) fetch(kb + 1, nxt);
         // the rows of x, a half-warp per 1 x 128 tile: 2-byte types are asked for here, so that they are there when the block is scaled
         const int sub = tid & 15, col = kb * TILE + sub * 8;
         constexpr bool EARLY = sizeof(TX) == 2;
@@ -148,29 +151,52 @@ fp8_linear_few_kernel(const TX* __restrict__ x, int64_t ldx, const float* __rest
             *reinterpret_cast<uint32_t*>(sB + tile_off(warp * 8 + i, lane * 4)) =
                 cvt_e4m3x4(scaled_clamped<DIV>(cur[i].x, db), scaled_clamped<DIV>(cur[i].y, db), scaled_clamped<DIV>(cur[i].z, db),
                            scaled_clamped<DIV>(cur[i].w, db));
+        // `passes` of 32 rows in step, so that one's shuffles and quotients run under another's
+        auto quantise_rows = [&](int first, auto passes) {
+            constexpr int P = decltype(passes)::value;
+            float a[P], v[P][8];
 #pragma unroll
-        for (int p = 0; p < TILE * 16 / THREADS; ++p) {
-            if (p * (THREADS / 16) >= M) break;
-            const int r = p * (THREADS / 16) + (tid >> 4);
-            float v[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-            if constexpr (EARLY) {
-                Raw8<TX> raw;
-                raw.a = xr[p];
-                unpack_raw8<TX>(raw, v);
-            } else if (r < M && col < K) {
-                Elem<TX>::load8(x + (int64_t)r * ldx + col, v);
+            for (int p = 0; p < P; ++p) {
+                const int r = (first + p) * (THREADS / 16) + (tid >> 4);
+                if constexpr (EARLY) {
+                    Raw8<TX> raw;
+                    raw.a = xr[first + p];
+                    unpack_raw8<TX>(raw, v[p]);
+                } else {
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) v[p][i] = 0.0f;
+                    if (r < M && col < K) Elem<TX>::load8(x + (int64_t)r * ldx + col, v[p]);
+                }
+                a[p] = 0.0f;
+#pragma unroll
+                for (int i = 0; i < 8; ++i) a[p] = fmaxf(a[p], fabsf(v[p][i]));
             }
-            float a = 0.0f;
 #pragma unroll
-            for (int i = 0; i < 8; ++i) a = fmaxf(a, fabsf(v[i]));
+            for (int o = 8; o > 0; o >>= 1)
 #pragma unroll
-            for (int o = 8; o > 0; o >>= 1) a = fmaxf(a, __shfl_xor_sync(0xffffffffu, a, o));
-            const float s = scale_from_amax<DIV, ROUND>(a), d = divisor_of<DIV>(s);
-            uint2 o2;
-            o2.x = cvt_e4m3x4(scaled_clamped<DIV>(v[0], d), scaled_clamped<DIV>(v[1], d), scaled_clamped<DIV>(v[2], d), scaled_clamped<DIV>(v[3], d));
-            o2.y = cvt_e4m3x4(scaled_clamped<DIV>(v[4], d), scaled_clamped<DIV>(v[5], d), scaled_clamped<DIV>(v[6], d), scaled_clamped<DIV>(v[7], d));
-            *reinterpret_cast<uint2*>(sA + tile_off(r, sub * 8)) = o2;
-            if (sub == 0) s_a[buf][r] = s;
+                for (int p = 0; p < P; ++p) a[p] = fmaxf(a[p], __shfl_xor_sync(0xffffffffu, a[p], o));
+#pragma unroll
+            for (int p = 0; p < P; ++p) {
+                const int r = (first + p) * (THREADS / 16) + (tid >> 4);
+                const float s = scale_from_amax<DIV, ROUND>(a[p]), d = divisor_of<DIV>(s);
+                uint2 o2;
+                o2.x = cvt_e4m3x4(scaled_clamped<DIV>(v[p][0], d), scaled_clamped<DIV>(v[p][1], d), scaled_clamped<DIV>(v[p][2], d),
+                                  scaled_clamped<DIV>(v[p][3], d));
+                o2.y = cvt_e4m3x4(scaled_clamped<DIV>(v[p][4], d), scaled_clamped<DIV>(v[p][5], d), scaled_clamped<DIV>(v[p][6], d),
+                                  scaled_clamped<DIV>(v[p][7], d));
+                *reinterpret_cast<uint2*>(sA + tile_off(r, sub * 8)) = o2;
+                if (sub == 0) s_a[buf][r] = s;
+            }
+        };
+        constexpr int PASSES = TILE * 16 / THREADS;
+        if (!ONE || M <= THREADS / 16) {
+#pragma unroll
+            for (int p = 0; p < (ONE ? 1 : PASSES); ++p)
+                if (p * (THREADS / 16) < M) quantise_rows(p, std::integral_constant<int, 1>{});
+        } else if (M <= 2 * (THREADS / 16)) {
+            quantise_rows(0, std::integral_constant<int, 2>{});
+        } else {
+            quantise_rows(0, std::integral_constant<int, PASSES>{});
         }
         fence_async_smem();
         tc_fence_before();
@@ -181,10 +207,12 @@ fp8_linear_few_kernel(const TX* __restrict__ x, int64_t ldx, const float* __rest
             tc_mma_f8_block<2>(tmem + buf * TILE, ((smem_u32(sA) >> 4) & 0x3FFF) | lo, ((smem_u32(sB) >> 4) & 0x3FFF) | lo, IDESC);
             tc_commit(done0 + 8 * buf);
         }
-        if (it > 0) promote(it - 1, sb_old);
+        if (!ONE && it > 0) promote(it - 1, sb_old);
         sb_old = sb;
+        if constexpr (!ONE) {
 #pragma unroll
-        for (int i = 0; i < 8; ++i) cur[i] = nxt[i];
+            for (int i = 0; i < 8; ++i) cur[i] = nxt[i];
+        }
     }
     if (kb1 > kb0) promote(kb1 - kb0 - 1, sb_old);
     tc_fence_before();
@@ -225,11 +253,21 @@ fp8_linear_few_kernel(const TX* __restrict__ x, int64_t ldx, const float* __rest
     cluster.sync();
     for (int e = slice * THREADS + tid; e < M * 32; e += slices * THREADS) {
         const int r = e >> 5, c = e & 31, n = n0 + c * 4;
+        // all of them asked for before the first is added: one round trip to the other SMs, not one after the other
+        float4 part[MAX_SLICES];
+        float f[MAX_SLICES];
+#pragma unroll
+        for (int s = 0; s < MAX_SLICES; ++s) {
+            if (s >= slices) break;
+            part[s] = *reinterpret_cast<const float4*>(cluster.map_shared_rank(smem, s) + r * 512 + ((c ^ (r & 7)) << 4));
+            f[s] = *cluster.map_shared_rank(&s_row[r], s);
+        }
         float4 sum = make_float4(0.f, 0.f, 0.f, 0.f);
-        for (int s = 0; s < slices; ++s) {
-            const float4 v = *reinterpret_cast<const float4*>(cluster.map_shared_rank(smem, s) + r * 512 + ((c ^ (r & 7)) << 4));
-            const float f = *cluster.map_shared_rank(&s_row[r], s);
-            sum.x = fmaf(v.x, f, sum.x); sum.y = fmaf(v.y, f, sum.y); sum.z = fmaf(v.z, f, sum.z); sum.w = fmaf(v.w, f, sum.w);
+#pragma unroll
+        for (int s = 0; s < MAX_SLICES; ++s) {
+            if (s >= slices) break;
+            sum.x = fmaf(part[s].x, f[s], sum.x); sum.y = fmaf(part[s].y, f[s], sum.y);
+            sum.z = fmaf(part[s].z, f[s], sum.z); sum.w = fmaf(part[s].w, f[s], sum.w);
         }
         __nv_bfloat162 h[2] = {__floats2bfloat162_rn(sum.x, sum.y), __floats2bfloat162_rn(sum.z, sum.w)};
         __nv_bfloat16* o = out + (int64_t)r * N + n;
@@ -244,20 +282,46 @@ fp8_linear_few_kernel(const TX* __restrict__ x, int64_t ldx, const float* __rest
     cluster.sync();                                        // nobody leaves while its sums are being read
 }
 
-// CTAs that share a column tile's reduction: one per K block if there are SMs for them all at once, in clusters that the GPCs hold (of 16
-// SMs or more: sizes that do not divide 16 leave some idle)
+// Clusters of so many CTAs that run at once: a GPC holds whole ones only, and GPCs differ in their SMs.  Asked of the driver once per device.
+static int clusters_at_once(int slices) {
+    static std::atomic<int> known[64][MAX_SLICES + 1];
+    constexpr auto kern = fp8_linear_few_kernel<__nv_bfloat16, CINN_DIV_FULL, false, true>;
+    int dev = 0, n = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) dev = 0;
+    if ((n = known[dev][slices].load(std::memory_order_relaxed)) > 0) return n;
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute attr[1];
+    cfg.gridDim = dim3((unsigned)slices, (unsigned)sm_count(), 1);
+    cfg.blockDim = dim3(THREADS, 1, 1);
+    cfg.dynamicSmemBytes = SMEM_BYTES;
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = slices;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    if (allow_smem_once<kern>(SMEM_BYTES) != CINN_OK || cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess) {
+        cudaGetLastError();
+        return 0;
+    }
+    known[dev][slices].store(n, std::memory_order_relaxed);
+    return n;
+}
+
+// CTAs that share a column tile's reduction: one per K block if their clusters all run at once and leave an eighth of the SMs (sizes that do
+// not divide 16: a quarter) to what runs beside.  Sixteen clusters of eight were 128 CTAs of 148 and ran in two turns: 8 x 1024 -> 2048 12.5 us
+// where the two kernels take 7.5.
 static int slices_of(int64_t N, int64_t K) {
     const int64_t tiles = (N + TILE - 1) / TILE, KB = (K + TILE - 1) / TILE;
     for (int s = (int)(KB < MAX_SLICES ? KB : MAX_SLICES); s > 1; --s)
-        if (tiles * s <= sm_count() * (16 % s == 0 ? 7 : 6) / 8) return s;
+        if (tiles * s <= sm_count() * (16 % s == 0 ? 7 : 6) / 8 && tiles <= clusters_at_once(s)) return s;
     return 1;
 }
 
-template <typename TX, int DIV, bool ROUND>
-static int launch(const TX* x, int64_t ldx, const float* w, int64_t ldw, __nv_bfloat16* out, int M, int N, int K, cudaStream_t st) {
-    constexpr auto kern = fp8_linear_few_kernel<TX, DIV, ROUND>;
+template <typename TX, int DIV, bool ROUND, bool ONE>
+static int launch_form(const TX* x, int64_t ldx, const float* w, int64_t ldw, __nv_bfloat16* out, int M, int N, int K, int slices,
+                       cudaStream_t st) {
+    constexpr auto kern = fp8_linear_few_kernel<TX, DIV, ROUND, ONE>;
     if (const int failed = allow_smem_once<kern>(SMEM_BYTES)) return failed;
-    const int slices = slices_of(N, K);
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)slices, (unsigned)((N + TILE - 1) / TILE), 1);
     cfg.blockDim = dim3(THREADS, 1, 1);
@@ -277,6 +341,13 @@ static int launch(const TX* x, int64_t ldx, const float* w, int64_t ldw, __nv_bf
     return CINN_OK;
 }
 
+template <typename TX, int DIV, bool ROUND>
+static int launch(const TX* x, int64_t ldx, const float* w, int64_t ldw, __nv_bfloat16* out, int M, int N, int K, cudaStream_t st) {
+    const int slices = slices_of(N, K);
+    return (K + TILE - 1) / TILE == slices ? launch_form<TX, DIV, ROUND, true>(x, ldx, w, ldw, out, M, N, K, slices, st)
+                                           : launch_form<TX, DIV, ROUND, false>(x, ldx, w, ldw, out, M, N, K, slices, st);
+}
+
 }  // namespace few
 
 bool gemm_sms_capped();                                    // gemm.cu: other kernels are to run beside the multiplications
@@ -292,9 +363,12 @@ static bool fits(const void* x, int x_dtype, int64_t ldx_m, int64_t ldx_k, const
 }
 
 // Worth it where every CTA has one K block, for then the launch that it saves is what counts; with more, each block waits for its
-// piece of the weight, where the quantiser's many CTAs stream them.  us a call, two kernels against this one: one block, 4 x 1024 -> 1344
-// 11.9 and 8.6, 82 x 512 -> 3776 12.0 and 10.3; two, 7 x 2048 -> 1472 11.9 and 12.3, 99 x 1472 -> 1600 12.1 and 14.4; three, 117 x
-// 2368 -> 768 12.0 and 18.5.
+// piece of the weight, where the quantiser's many CTAs stream them.  us a call, two kernels against this one, one block: weights that stay in
+// L2, 4 x 1024 -> 1344 9.9 and 6.7, 128 x 512 -> 1024 9.7 and 8.1; every call another weight, 10.0 and 6.7, 9.7 and 8.4.  Two blocks, 7 x 2048 -> 1472
+// 11.9 and 12.3, 99 x 1472 -> 1600 12.1 and 14.4; three, 117 x 2368 -> 768 12.0 and 18.5.
+// Replayed from a CUDA graph the launch costs next to nothing and the exchange between the CTAs counts, which grows with the rows: 128 x 512 -> 1024
+// 5.8 and 7.4, 64 5.7 and 5.8, 32 5.7 and 5.3, 128 x 1024 -> 1344 7.0 and 9.0, 32 6.6 and 6.3; without an exchange, 128 x 128 -> 8192, 6.0 and 5.3.
+// So callers under capture take it for up to 32 rows, or for one K block in all (csrc/host/linear.cpp).
 bool linear_few_takes(const void* x, int x_dtype, int64_t ldx_m, int64_t ldx_k, const void* w, int w_dtype, int64_t ldw_n, int64_t ldw_k,
                       int64_t M, int64_t N, int64_t K) {
     return fits(x, x_dtype, ldx_m, ldx_k, w, w_dtype, ldw_n, ldw_k, M, N, K) && !gemm_sms_capped() &&

@@ -882,3 +882,47 @@ def test_linear_on_few_rows_any_alignment(K):
         n = K.launch_count
         long(torch.randn(4, 7168, device="cuda"))
         assert K.launch_count - n >= 2
+
+
+@pytest.mark.parametrize("M,Kd,kernels", [(8, 512, 1), (33, 512, 2), (128, 128, 1), (128, 512, 2)])
+def test_linear_on_few_rows_under_capture(K, M, Kd, kernels):
+    """Outside a capture one kernel; inside one, where a launch costs next to nothing, two for many rows with an exchange between CTAs: the
+    same bits."""
+    lin = K.FP8Linear(Kd, 1024).cuda()
+    x = torch.randn(M, Kd, device="cuda", generator=torch.Generator(device="cuda").manual_seed(M)).to(torch.bfloat16)
+    with torch.no_grad():
+        n = K.launch_count
+        ref = lin(x)
+        assert K.launch_count - n == 1
+        torch.cuda.synchronize()
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g):
+            n = K.launch_count
+            out = lin(x)
+            assert K.launch_count - n == kernels
+        g.replay()
+    assert torch.equal(out, ref)
+    del g
+
+
+@pytest.mark.parametrize("M", [1, 31, 32, 33, 64, 65, 97, 128])
+@pytest.mark.parametrize("dtype,special", [(torch.bfloat16, False), (torch.bfloat16, True), (torch.float32, True)])
+def test_linear_on_few_rows_in_passes_of_32(K, M, dtype, special):
+    """One, two or four passes over the rows of x, also with NaN and infinity in x and in the weight: the bits of two kernels."""
+    g = torch.Generator(device="cuda").manual_seed(M)
+    lin = K.FP8Linear(400, 264).cuda()
+    x = torch.randn(M, 400, device="cuda", generator=g).mul_(3)
+    if special:
+        x[0, 7], x[M // 2, 130], x[M - 1, 399] = float("nan"), float("inf"), -float("inf")
+        with torch.no_grad():
+            lin.weight[5, 9], lin.weight[200, 300], lin.weight[263, 399] = float("nan"), float("inf"), -float("inf")
+    x = x.to(dtype)
+    with torch.no_grad():
+        n = K.launch_count
+        out = lin(x)
+    assert K.launch_count - n == 1
+    xq, xs = K.quantize_fp8_rowwise(x, 128, lin.round_scale)
+    wq, ws = K.quantize_fp8_blockwise(lin.weight.detach())
+    ref = K._gemm(xq, xs, wq, 0, ws, ws.stride(1), ws.stride(0), M, 264, 400, torch.bfloat16, whole=True)
+    assert torch.equal(out.isnan(), ref.isnan()) and torch.equal(out.nan_to_num(7.0), ref.nan_to_num(7.0))
+    assert not special or (bool(ref.isnan().any()) and (M == 1 or bool(ref.isfinite().any())))       # (one row has them all)
