@@ -118,7 +118,7 @@ static void launch_combine(const T* rows, const int64_t* pos, const float* gates
     const dim3 grid((unsigned)((n_tokens + tokens - 1) / tokens), few ? (unsigned)((d + per * 8 - 1) / (per * 8)) : 1u);
     // early for a few tokens, where the launch counts (a serving layer of 397: 118 -> 105 us with all its kernels).  32768 tokens of 7168, both this
     // kernel and the row spread early 15.48 ms, neither 15.34 (medians of five processes each, which overlap: 15.42 - 15.58, 15.30 - 15.55).
-    const bool early = n_tokens <= 8 * (int64_t)sm_count();
+    const bool early = n_tokens <= 8 * (int64_t)sm_count() && !captured(st);
     if (top_k <= 2) launch_early_if(early, moe_combine_kernel<T, 2>, dim3(grid), dim3(256), 0, st, rows, pos, gates, addend, addend_dtype, y, n_tokens, n_rows, top_k, d, per);
     else launch_early_if(early, moe_combine_kernel<T, 4>, dim3(grid), dim3(256), 0, st, rows, pos, gates, addend, addend_dtype, y, n_tokens, n_rows, top_k, d, per);
 }
@@ -360,7 +360,7 @@ int spread_rows(const void* q, const float* s, const int64_t* pos, void* out_q, 
                    "spread_rows: the row width (%lld) must be a multiple of 16", (long long)d);
     CINN_CHECK_ARG((reinterpret_cast<uintptr_t>(q) & 15) == 0 && (reinterpret_cast<uintptr_t>(out_q) & 15) == 0,
                    "spread_rows: byte buffers must be 16-byte aligned");
-    launch_early_if(n_tokens <= 8 * (int64_t)sm_count(), spread_rows_kernel, dim3((unsigned)n_tokens), dim3(256), 0, st, (const uint8_t*)q, s, pos, (uint8_t*)out_q, out_s, n_rows, top_k, (int)d, (int)ns);
+    launch_early_if(n_tokens <= 8 * (int64_t)sm_count() && !captured(st), spread_rows_kernel, dim3((unsigned)n_tokens), dim3(256), 0, st, (const uint8_t*)q, s, pos, (uint8_t*)out_q, out_s, n_rows, top_k, (int)d, (int)ns);
     CINN_CHECK_LAUNCH();
     return CINN_OK;
 }

@@ -1656,7 +1656,7 @@ static int launch_rowwise(const T* x, int64_t M, int64_t N, int64_t ld_m, int64_
         const int64_t cap = (int64_t)sms * 8;
         if (blocks > cap) blocks = cap;
         const int64_t n_hw = blocks * 16;
-        launch_early_if(quantise_early(M, N), quant_row_vec_kernel<T, DIV, ROUND, UNROLL>, dim3((unsigned)blocks), dim3(256), 0, st,
+        launch_early_if(quantise_early(M, N, st), quant_row_vec_kernel<T, DIV, ROUND, UNROLL>, dim3((unsigned)blocks), dim3(256), 0, st,
             x, ld_m, q, scales, (int)N, nb, tiles, (int)(n_hw / nb), (int)(n_hw % nb));
     } else if (block == 128 && ld_m == 1 && ld_n >= M && M % 8 == 0 && ld_n % 8 == 0 && N % 16 == 0 && aligned16(x) &&
                aligned16(q) && M > 1) {
@@ -1687,7 +1687,7 @@ static int launch_blockwise(const T* x, int64_t M, int64_t N, int64_t ld_m, int6
     const bool a = sizeof(T) == 4 ? aligned16(x) : ((reinterpret_cast<uintptr_t>(x) & 7) == 0);
     if (bm == 128 && bn == 128 && ld_n == 1 && N % 4 == 0 && ld_m % 4 == 0 && a && (reinterpret_cast<uintptr_t>(q) & 3) == 0) {
         if (t_beside) CINN_CHECK_CUDA(launch_dependent(quant_block_vec_kernel<T, DIV, ROUND>, grid, 256, 0, st, x, ld_m, q, scales, (int)M, (int)N, nb, 1));
-        else launch_early_if(quantise_early(M, N), quant_block_vec_kernel<T, DIV, ROUND>, dim3(grid), dim3(256), 0, st, x, ld_m, q, scales, (int)M, (int)N, nb, 0);
+        else launch_early_if(quantise_early(M, N, st), quant_block_vec_kernel<T, DIV, ROUND>, dim3(grid), dim3(256), 0, st, x, ld_m, q, scales, (int)M, (int)N, nb, 0);
     } else {
         quant_block_generic_kernel<T, DIV, ROUND><<<grid, 256, 0, st>>>(x, ld_m, ld_n, q, scales, (int)M, (int)N, bm, bn, nb);
     }
@@ -1704,7 +1704,7 @@ static int dispatch_block_t(const T* x, int64_t M, int64_t N, int64_t ld, uint8_
 #define CINN_B(DIV, RND) \
     do { \
         if (t_beside) CINN_CHECK_CUDA(launch_dependent(quant_block_vec_t_kernel<T, DIV, RND>, grid, 256, 0, st, x, ld, q, q_t, scales, (int)M, (int)N, nb, 1)); \
-        else launch_early_if(quantise_early(M, N), quant_block_vec_t_kernel<T, DIV, RND>, dim3(grid), dim3(256), 0, st, x, ld, q, q_t, scales, (int)M, (int)N, nb, 0); \
+        else launch_early_if(quantise_early(M, N, st), quant_block_vec_t_kernel<T, DIV, RND>, dim3(grid), dim3(256), 0, st, x, ld, q, q_t, scales, (int)M, (int)N, nb, 0); \
     } while (0)
     if (div_mode == CINN_DIV_FULL) { if (round_scale) CINN_B(CINN_DIV_FULL, true); else CINN_B(CINN_DIV_FULL, false); }
     else                           { if (round_scale) CINN_B(CINN_DIV_RN, true);   else CINN_B(CINN_DIV_RN, false); }
@@ -1746,7 +1746,7 @@ static int launch_quant_linear(const TX* x, int64_t ldx, uint8_t* xq, float* xs,
     // 332 x 1408 -> 11712 (1012 of them) 26.8 -> 29.2 us, 40 x 1600 -> 7000 (715) 18.5 -> 19.0, but 800 x 768 -> 9000 (426) 20.5 -> 19.6, 2595 x
     // 512 -> 7104 24.6 -> 23.0, 8000 x 512 -> 1024 17.4 -> 15.5.  Few rows are not multiplied in long tiles and gain up to 3072 columns (12 x 2368 ->
     // 1856 12.3 -> 11.3, 100 x 3072 -> 2048 16.1 -> 13.8), not at 4096 (40 x 4096 -> 4096 26.7 -> 27.5).
-#define CINN_Q(DIV, RND) launch_early_if((int64_t)grid <= cap && 2 * w_blocks <= cap && (K <= 2048 || (M <= 128 && K <= 3072)), quant_linear_kernel<TX, TW, DIV, RND>, dim3(grid), dim3(256), 0, st, x, ldx, xq, xs, tiles, (int)(n_hw / nb), (int)(n_hw % nb), w, ldw, wq, ws, (int)N, (int)K, nb, (int)w_blocks)
+#define CINN_Q(DIV, RND) launch_early_if((int64_t)grid <= cap && 2 * w_blocks <= cap && (K <= 2048 || (M <= 128 && K <= 3072)) && !captured(st), quant_linear_kernel<TX, TW, DIV, RND>, dim3(grid), dim3(256), 0, st, x, ldx, xq, xs, tiles, (int)(n_hw / nb), (int)(n_hw % nb), w, ldw, wq, ws, (int)N, (int)K, nb, (int)w_blocks)
     if (div_mode == CINN_DIV_FULL) { if (round_scale) CINN_Q(CINN_DIV_FULL, true); else CINN_Q(CINN_DIV_FULL, false); }
     else                           { if (round_scale) CINN_Q(CINN_DIV_RN, true);   else CINN_Q(CINN_DIV_RN, false); }
 #undef CINN_Q
@@ -1847,14 +1847,14 @@ static int dispatch_dual(const T* x, int64_t M, int64_t N, int64_t ld, uint8_t* 
     do {                                                                                                              \
         constexpr auto kern = quant_row_dual_tma_kernel<T, DIV, RND>;                                                 \
         if (const int failed = allow_smem_once<kern>(DUAL_SMEM_BYTES)) return failed;                                 \
-        launch_early_if(quantise_early(M, N), kern, dim3(grid), dim3(256), DUAL_SMEM_BYTES, st, tm, q_row, s_row, q_col, s_col, (int)M, (int)N, nb_n, nb_m, (int)total); \
+        launch_early_if(quantise_early(M, N, st), kern, dim3(grid), dim3(256), DUAL_SMEM_BYTES, st, tm, q_row, s_row, q_col, s_col, (int)M, (int)N, nb_n, nb_m, (int)total); \
     } while (0)
         if (div_mode == CINN_DIV_FULL) { if (round_scale) CINN_D(CINN_DIV_FULL, true); else CINN_D(CINN_DIV_FULL, false); }
         else                           { if (round_scale) CINN_D(CINN_DIV_RN, true);   else CINN_D(CINN_DIV_RN, false); }
 #undef CINN_D
     } else {
         dim3 grid((unsigned)nb_n, (unsigned)nb_m);
-#define CINN_D(DIV, RND) launch_early_if(quantise_early(M, N), quant_row_dual_kernel<T, DIV, RND>, dim3(grid), dim3(256), 0, st, x, ld, q_row, s_row, q_col, s_col, (int)M, (int)N, nb_n, nb_m)
+#define CINN_D(DIV, RND) launch_early_if(quantise_early(M, N, st), quant_row_dual_kernel<T, DIV, RND>, dim3(grid), dim3(256), 0, st, x, ld, q_row, s_row, q_col, s_col, (int)M, (int)N, nb_n, nb_m)
         if (div_mode == CINN_DIV_FULL) { if (round_scale) CINN_D(CINN_DIV_FULL, true); else CINN_D(CINN_DIV_FULL, false); }
         else                           { if (round_scale) CINN_D(CINN_DIV_RN, true);   else CINN_D(CINN_DIV_RN, false); }
 #undef CINN_D
@@ -1892,7 +1892,7 @@ static int dispatch_row_block(const T* x, int64_t M, int64_t N, int64_t ld, uint
         const int failed = transpose_block ? allow_smem_once<turned>(DUAL_SMEM_BYTES) : allow_smem_once<straight>(DUAL_SMEM_BYTES);\
         if (failed) return failed;                                                                                    \
         const auto kern = transpose_block ? turned : straight;                                                        \
-        launch_early_if(quantise_early(M, N), kern, dim3(grid), dim3(256), DUAL_SMEM_BYTES, st, tm, q_row, s_row, q_blk, s_blk, (int)M, (int)N, nb_n, nb_m, (int)total); \
+        launch_early_if(quantise_early(M, N, st), kern, dim3(grid), dim3(256), DUAL_SMEM_BYTES, st, tm, q_row, s_row, q_blk, s_blk, (int)M, (int)N, nb_n, nb_m, (int)total); \
     } while (0)
         if (div_mode == CINN_DIV_FULL) { if (round_scale) CINN_D(CINN_DIV_FULL, true); else CINN_D(CINN_DIV_FULL, false); }
         else                           { if (round_scale) CINN_D(CINN_DIV_RN, true);   else CINN_D(CINN_DIV_RN, false); }
@@ -1901,8 +1901,8 @@ static int dispatch_row_block(const T* x, int64_t M, int64_t N, int64_t ld, uint
         dim3 grid((unsigned)nb_n, (unsigned)nb_m);
 #define CINN_D(DIV, RND)                                                                                              \
     do {                                                                                                              \
-        if (transpose_block) launch_early_if(quantise_early(M, N), quant_row_dual_kernel<T, DIV, RND, 2>, dim3(grid), dim3(256), 0, st, x, ld, q_row, s_row, q_blk, s_blk, (int)M, (int)N, nb_n, nb_m); \
-        else launch_early_if(quantise_early(M, N), quant_row_dual_kernel<T, DIV, RND, 1>, dim3(grid), dim3(256), 0, st, x, ld, q_row, s_row, q_blk, s_blk, (int)M, (int)N, nb_n, nb_m); \
+        if (transpose_block) launch_early_if(quantise_early(M, N, st), quant_row_dual_kernel<T, DIV, RND, 2>, dim3(grid), dim3(256), 0, st, x, ld, q_row, s_row, q_blk, s_blk, (int)M, (int)N, nb_n, nb_m); \
+        else launch_early_if(quantise_early(M, N, st), quant_row_dual_kernel<T, DIV, RND, 1>, dim3(grid), dim3(256), 0, st, x, ld, q_row, s_row, q_blk, s_blk, (int)M, (int)N, nb_n, nb_m); \
     } while (0)
         if (div_mode == CINN_DIV_FULL) { if (round_scale) CINN_D(CINN_DIV_FULL, true); else CINN_D(CINN_DIV_FULL, false); }
         else                           { if (round_scale) CINN_D(CINN_DIV_RN, true);   else CINN_D(CINN_DIV_RN, false); }
@@ -2154,7 +2154,7 @@ int quantize_dual_segmented(const void* x, int dtype, int64_t T, int64_t N, void
     do {                                                                                                              \
         constexpr auto kern = quant_row_dual_seg_kernel<TT, DIV, MODE>;                                               \
         if (const int failed = allow_smem_once<kern>(DUAL_SMEM_BYTES)) return failed;                                 \
-        launch_early_if(quantise_early(T, N), kern, dim3(grid), dim3(256), DUAL_SMEM_BYTES, st, tm, (uint8_t*)q_row, s_row, (uint8_t*)q_col, s_col, max_tiles * 128, (int)N, \
+        launch_early_if(quantise_early(T, N, st), kern, dim3(grid), dim3(256), DUAL_SMEM_BYTES, st, tm, (uint8_t*)q_row, s_row, (uint8_t*)q_col, s_col, max_tiles * 128, (int)N, \
                                                  nb_n, max_tiles, tile_src, tile_cnt, n_tiles);                       \
     } while (0)
 #define CINN_DS(TT, DIV) do { if (block) CINN_DSM(TT, DIV, 2); else CINN_DSM(TT, DIV, 0); } while (0)
@@ -2179,9 +2179,9 @@ int requant_row_to_block_segmented(const void* xq, const float* xs, int64_t K, v
         const int64_t tiles = (int64_t)nb * max_tiles;
         const int grid = (int)(tiles < (int64_t)sm_count() * 2 ? tiles : (int64_t)sm_count() * 2);
         if (div_mode == CINN_DIV_FULL)
-            launch_early_if(quantise_early(M, K), requant_seg_t_kernel<CINN_DIV_FULL>, dim3(grid), dim3(256), 0, st, (const uint8_t*)xq, xs, (uint8_t*)out, scales, M, (int)K, nb, tile_src, tile_cnt, n_tiles);
+            launch_early_if(quantise_early(M, K, st), requant_seg_t_kernel<CINN_DIV_FULL>, dim3(grid), dim3(256), 0, st, (const uint8_t*)xq, xs, (uint8_t*)out, scales, M, (int)K, nb, tile_src, tile_cnt, n_tiles);
         else
-            launch_early_if(quantise_early(M, K), requant_seg_t_kernel<CINN_DIV_RN>, dim3(grid), dim3(256), 0, st, (const uint8_t*)xq, xs, (uint8_t*)out, scales, M, (int)K, nb, tile_src, tile_cnt, n_tiles);
+            launch_early_if(quantise_early(M, K, st), requant_seg_t_kernel<CINN_DIV_RN>, dim3(grid), dim3(256), 0, st, (const uint8_t*)xq, xs, (uint8_t*)out, scales, M, (int)K, nb, tile_src, tile_cnt, n_tiles);
         CINN_CHECK_LAUNCH();
         return CINN_OK;
     }
@@ -2217,7 +2217,7 @@ int swiglu_quant_block(const void* h12, int dtype, int64_t T, int64_t I, void* q
     CINN_CHECK_ARG(total < (1LL << 31) && s_row && s_blk && !(seg && round_scale), "swiglu + row + block quantiser: bad arguments");
     const int grid = (int)(total < cap ? total : cap);
 #define CINN_SB(T_, RND, EXACT, SEG)                                                                                              \
-    launch_early_if(quantise_early(T, I), swiglu_row_block_kernel<T_, RND, EXACT, SEG>, dim3(grid), dim3(256), 0, st, (const T_*)h12, (uint8_t*)q_row, s_row, (uint8_t*)q_blk, s_blk,  \
+    launch_early_if(quantise_early(T, I, st), swiglu_row_block_kernel<T_, RND, EXACT, SEG>, dim3(grid), dim3(256), 0, st, (const T_*)h12, (uint8_t*)q_row, s_row, (uint8_t*)q_blk, s_blk,  \
         seg ? seg->max * 128 : (int)T, (int)I, nb_n, nb_m, (int)total, seg ? seg->src : nullptr, seg ? seg->cnt : nullptr, seg ? seg->n : nullptr)
 #define CINN_SBT(T_) do { if (seg) CINN_SB(T_, false, false, true); else if (round_scale) CINN_SB(T_, true, true, false); else CINN_SB(T_, false, true, false); } while (0)
     if (dtype == CINN_BF16) CINN_SBT(__nv_bfloat16);
@@ -2237,7 +2237,7 @@ int swiglu_backward_quant_dual(const void* h12, const void* dh, int dtype, int64
     CINN_CHECK_ARG(total < (1LL << 31) && dh && aligned16(dh) && s_row && s_col && !(seg && round_scale), "swiglu backward + dual quantiser: bad arguments");
     const int grid = (int)(total < cap ? total : cap);
 #define CINN_SD(T_, RND, EXACT, SEG)                                                                                              \
-    launch_early_if(quantise_early(T, I), swiglu_backward_dual_kernel<T_, RND, EXACT, SEG>, dim3(grid), dim3(256), 0, st, (const T_*)h12, (const T_*)dh, (uint8_t*)q_row, s_row,       \
+    launch_early_if(quantise_early(T, I, st), swiglu_backward_dual_kernel<T_, RND, EXACT, SEG>, dim3(grid), dim3(256), 0, st, (const T_*)h12, (const T_*)dh, (uint8_t*)q_row, s_row,       \
         (uint8_t*)q_col, s_col, seg ? seg->max * 128 : (int)T, (int)I, nb_i, nb_m, (int)total, seg ? seg->src : nullptr,               \
         seg ? seg->cnt : nullptr, seg ? seg->n : nullptr)
 #define CINN_SDT(T_) do { if (seg) CINN_SD(T_, false, false, true); else if (round_scale) CINN_SD(T_, true, true, false); else CINN_SD(T_, false, true, false); } while (0)
@@ -2331,8 +2331,8 @@ static int launch_swiglu(const T* h12, int64_t T_rows, int64_t I, uint8_t* q, fl
     if (blocks > cap) blocks = cap;
     const int64_t n_hw = blocks * 16;
     const int sr = (int)(n_hw / nb), sc = (int)(n_hw % nb);
-    if (div_mode == CINN_DIV_FULL) launch_early_if(quantise_early(T_rows, I), swiglu_quant_row_kernel<T, CINN_DIV_FULL>, dim3((unsigned)blocks), dim3(256), 0, st, h12, q, scales, (int)I, nb, tiles, sr, sc, n_rows_dev);
-    else launch_early_if(quantise_early(T_rows, I), swiglu_quant_row_kernel<T, CINN_DIV_RN>, dim3((unsigned)blocks), dim3(256), 0, st, h12, q, scales, (int)I, nb, tiles, sr, sc, n_rows_dev);
+    if (div_mode == CINN_DIV_FULL) launch_early_if(quantise_early(T_rows, I, st), swiglu_quant_row_kernel<T, CINN_DIV_FULL>, dim3((unsigned)blocks), dim3(256), 0, st, h12, q, scales, (int)I, nb, tiles, sr, sc, n_rows_dev);
+    else launch_early_if(quantise_early(T_rows, I, st), swiglu_quant_row_kernel<T, CINN_DIV_RN>, dim3((unsigned)blocks), dim3(256), 0, st, h12, q, scales, (int)I, nb, tiles, sr, sc, n_rows_dev);
     CINN_CHECK_LAUNCH();
     return CINN_OK;
 }

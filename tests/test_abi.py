@@ -122,14 +122,9 @@ def test_convert_to_fp8_selection_rules(built):
     assert sorted(n for n, _ in b.w1.named_parameters()) == ["weight"]
 
 
-def test_a_launch_that_fails_is_reported(built, tmp_path):
-    """Early or plain, a launch that the CUDA runtime refuses is an error of the call and counts as none: the launch helpers over a
-    runtime of this test's own, whose launches fail and whose last error is cleared when it is read."""
-    import subprocess
-    from cinnamon_b200 import build as B
-    exe, runtime, calls = tmp_path / "launch", tmp_path / "runtime.cpp", tmp_path / "calls.cu"
-    runtime.write_text("""
-int last = 0, next = 0;                                       // errors: what is pending, what the next launch ends with
+# a CUDA runtime whose launches end as they are told and whose last error is cleared when it is read
+RUNTIME = """
+int last = 0, next = 0, capturing = 0;                        // errors: what is pending, what the next launch ends with
 static int launched() { if (next != 0) last = next; return next; }
 extern "C" {
 int cudaGetLastError() { const int e = last; last = 0; return e; }
@@ -137,6 +132,7 @@ int cudaPeekAtLastError() { return last; }
 const char* cudaGetErrorString(int) { return "refused"; }
 int cudaLaunchKernel() { return launched(); }
 int cudaLaunchKernelExC() { return launched(); }
+int cudaStreamIsCapturing(void*, int* status) { *status = capturing; return 0; }
 unsigned __cudaPushCallConfiguration() { return 0; }
 int __cudaPopCallConfiguration() { return 0; }
 void** __cudaRegisterFatBinary(void*) { static void* h; return &h; }
@@ -145,14 +141,31 @@ void __cudaUnregisterFatBinary(void**) {}
 void __cudaRegisterFunction() {}
 char __cudaInitModule(void**) { return 0; }
 }
-""")
+"""
+
+
+def _run_over_runtime(tmp_path, program):
+    import subprocess
+    from cinnamon_b200 import build as B
+    exe, runtime, calls = tmp_path / "launch", tmp_path / "runtime.cpp", tmp_path / "calls.cu"
+    runtime.write_text(RUNTIME)
     calls.write_text("""
 #include "common.cuh"
-extern int last, next;
+extern int last, next, capturing;
 namespace cinn {
 std::atomic<int64_t> g_launches{0};
 void set_error(const char*, ...) {}
 }
+""" + program)
+    p = subprocess.run([B._nvcc(), *B.NVCC_FLAGS, "-cudart", "none", "-I" + B.CSRC, str(calls), str(runtime), "-o", str(exe)],
+                       capture_output=True, text=True, timeout=300)
+    assert p.returncode == 0, p.stderr
+    return subprocess.run([str(exe)], timeout=60).returncode
+
+
+def test_a_launch_that_fails_is_reported(built, tmp_path):
+    """Early or plain, a launch that the CUDA runtime refuses is an error of the call and counts as none."""
+    assert _run_over_runtime(tmp_path, """
 __global__ void kernel(int) {}
 static int call(bool early) {
     cinn::launch_early_if(early, kernel, dim3(1), dim3(32), 0, nullptr, 1);
@@ -168,8 +181,16 @@ int main() {
     }
     return 0;
 }
-""")
-    p = subprocess.run([B._nvcc(), *B.NVCC_FLAGS, "-cudart", "none", "-I" + B.CSRC, str(calls), str(runtime), "-o", str(exe)],
-                       capture_output=True, text=True, timeout=300)
-    assert p.returncode == 0, p.stderr
-    assert subprocess.run([str(exe)], timeout=60).returncode == 0
+""") == 0
+
+
+def test_quantisers_start_early_for_short_rows_and_outside_a_capture(built, tmp_path):
+    assert _run_over_runtime(tmp_path, """
+int main() {
+    using cinn::quantise_early;
+    if (!quantise_early(4096, 512, nullptr) || quantise_early(4096, 4096, nullptr) || quantise_early(1 << 20, 1024, nullptr)) return 1;
+    capturing = cudaStreamCaptureStatusActive;
+    if (quantise_early(4096, 512, nullptr) || !cinn::captured(nullptr)) return 2;
+    return 0;
+}
+""") == 0
