@@ -1871,6 +1871,10 @@ template <typename T>
 static int dispatch_row_block(const T* x, int64_t M, int64_t N, int64_t ld, uint8_t* q_row, float* s_row, uint8_t* q_blk,
                               float* s_blk, int round_scale, int div_mode, cudaStream_t st, int transpose_block) {
     const int nb_n = (int)((N + 127) / 128), nb_m = (int)((M + 127) / 128);
+    // The weight's quantiser works beside this one, and a GEMM follows: long rows gain only while there are few of them.  us forward and backward, early
+    // and plain: 1024 x 2048 -> 8832 121.8 and 123.6, 1824 x 1280 -> 8832 132.2 and 134.2, but 1824 x 2048 -> 8832 165.3 and 163.0, 4096 x 2048 ->
+    // 8832 276.8 and 270.8, 8192 x 1536 -> 8832 398.0 and 393.4, 30000 x 2048 -> 2048 451.8 and 446.5
+    const bool early = quantise_early(M, N, st) && (N <= 1024 || M * N <= 3 << 20);
     const bool fused = N % 16 == 0 && ld % 8 == 0 && nb_m <= 65535 && aligned16(x) && aligned16(q_row) && aligned16(q_blk);
     if (!fused) {
         CINN_CHECK_ARG(!transpose_block || M % 16 == 0, "row + block quantiser: padded rows need aligned rows and M <= 8388480");
@@ -1892,7 +1896,7 @@ static int dispatch_row_block(const T* x, int64_t M, int64_t N, int64_t ld, uint
         const int failed = transpose_block ? allow_smem_once<turned>(DUAL_SMEM_BYTES) : allow_smem_once<straight>(DUAL_SMEM_BYTES);\
         if (failed) return failed;                                                                                    \
         const auto kern = transpose_block ? turned : straight;                                                        \
-        launch_early_if(quantise_early(M, N, st), kern, dim3(grid), dim3(256), DUAL_SMEM_BYTES, st, tm, q_row, s_row, q_blk, s_blk, (int)M, (int)N, nb_n, nb_m, (int)total); \
+        launch_early_if(early, kern, dim3(grid), dim3(256), DUAL_SMEM_BYTES, st, tm, q_row, s_row, q_blk, s_blk, (int)M, (int)N, nb_n, nb_m, (int)total); \
     } while (0)
         if (div_mode == CINN_DIV_FULL) { if (round_scale) CINN_D(CINN_DIV_FULL, true); else CINN_D(CINN_DIV_FULL, false); }
         else                           { if (round_scale) CINN_D(CINN_DIV_RN, true);   else CINN_D(CINN_DIV_RN, false); }
@@ -1901,8 +1905,8 @@ static int dispatch_row_block(const T* x, int64_t M, int64_t N, int64_t ld, uint
         dim3 grid((unsigned)nb_n, (unsigned)nb_m);
 #define CINN_D(DIV, RND)                                                                                              \
     do {                                                                                                              \
-        if (transpose_block) launch_early_if(quantise_early(M, N, st), quant_row_dual_kernel<T, DIV, RND, 2>, dim3(grid), dim3(256), 0, st, x, ld, q_row, s_row, q_blk, s_blk, (int)M, (int)N, nb_n, nb_m); \
-        else launch_early_if(quantise_early(M, N, st), quant_row_dual_kernel<T, DIV, RND, 1>, dim3(grid), dim3(256), 0, st, x, ld, q_row, s_row, q_blk, s_blk, (int)M, (int)N, nb_n, nb_m); \
+        if (transpose_block) launch_early_if(early, quant_row_dual_kernel<T, DIV, RND, 2>, dim3(grid), dim3(256), 0, st, x, ld, q_row, s_row, q_blk, s_blk, (int)M, (int)N, nb_n, nb_m); \
+        else launch_early_if(early, quant_row_dual_kernel<T, DIV, RND, 1>, dim3(grid), dim3(256), 0, st, x, ld, q_row, s_row, q_blk, s_blk, (int)M, (int)N, nb_n, nb_m); \
     } while (0)
         if (div_mode == CINN_DIV_FULL) { if (round_scale) CINN_D(CINN_DIV_FULL, true); else CINN_D(CINN_DIV_FULL, false); }
         else                           { if (round_scale) CINN_D(CINN_DIV_RN, true);   else CINN_D(CINN_DIV_RN, false); }
