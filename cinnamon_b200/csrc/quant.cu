@@ -896,12 +896,14 @@ quant_row_dual_tma_kernel(const __grid_constant__ CUtensorMap tmX, uint8_t* __re
 // reads).  Tile y of the padded axis holds tile_cnt[y] rows from tile_src[y] on; only the first *n_tiles tiles exist.
 // Same TMA ring as the dense kernel; the elected thread leaves each stage's (first row, row count) beside the barriers.
 // MODE 2: the row + block pass with its block copy transposed, segment by segment (the forward's x, whose block copy the weight
-// gradient reads: one pass of 195 us over 32768 x 7168 in place of the row-wise one and a re-quantisation of its bytes, 165 + 157).
+// gradient reads: one pass of 195 us over 32768 x 7168 in place of the row-wise one and a re-quantisation of its bytes, 165 + 157).  Where tiles
+// had to be dropped (overlapping ranges) it quantises all rows row-wise behind its tiles, for the forward reads every range's.
 template <typename T, int DIV, int MODE>
 __global__ void __launch_bounds__(256, 2)
 quant_row_dual_seg_kernel(const __grid_constant__ CUtensorMap tmX, uint8_t* __restrict__ q_row, float* __restrict__ s_row,
                           uint8_t* __restrict__ q_col, float* __restrict__ s_col, int M_pad, int N, int nb_n, int nb_m,
-                          const int* __restrict__ tile_src, const int* __restrict__ tile_cnt, const int* __restrict__ n_tiles) {
+                          const int* __restrict__ tile_src, const int* __restrict__ tile_cnt, const int* __restrict__ n_tiles,
+                          const T* __restrict__ x, int64_t rows, const int* __restrict__ dropped) {
     pdl_wait();
     pdl_trigger();
     static_assert(sizeof(T) == 2, "the TMA-fed path takes 2-byte inputs");
@@ -951,6 +953,10 @@ quant_row_dual_seg_kernel(const __grid_constant__ CUtensorMap tmX, uint8_t* __re
         atomicCAS(&g_quant_status, 0, (4 << 8) | 1);
         for (int j = 1; j < DUAL_STAGES; ++j)
             if (t + j * stride < total) mbar_wait_bounded(full0 + 8 * ((k + j) % DUAL_STAGES), ((k + j) / DUAL_STAGES) & 1);
+    }
+    if constexpr (MODE == 2) {
+        if (alive && *dropped)
+            quant_rows<T, DIV, false, 1>(x, N, q_row, s_row, N, nb_n, rows * nb_n, stride * 16 / nb_n, stride * 16 % nb_n, blockIdx.x, stride);
     }
 }
 
@@ -2042,7 +2048,8 @@ int requant_row_to_block_padded(const void* xq, const float* xs, int64_t M_in, i
 constexpr int MAX_SEGMENT_EXPERTS = 1024;
 __global__ void __launch_bounds__(256)
 segment_tiles_kernel(const int64_t* __restrict__ starts, const int64_t* __restrict__ ends, int E, int64_t T,
-                     int* __restrict__ kb_start, int* __restrict__ tile_src, int* __restrict__ tile_cnt, int max_tiles) {
+                     int* __restrict__ kb_start, int* __restrict__ tile_src, int* __restrict__ tile_cnt, int max_tiles,
+                     int* __restrict__ dropped) {
     pdl_wait();
     pdl_trigger();
     constexpr int PER = MAX_SEGMENT_EXPERTS / 256;         // consecutive experts of a thread
@@ -2077,13 +2084,16 @@ segment_tiles_kernel(const int64_t* __restrict__ starts, const int64_t* __restri
     __syncthreads();
     long long run = incl - sum;
     for (int w = 0; w < warp; ++w) run += s_warp[w];
-    // (capped: cannot happen for disjoint ranges; keeps every index in range)
+    // (capped: cannot happen for disjoint ranges; keeps every index in range, and the tiles past the cap are left out)
 #pragma unroll
     for (int i = 0; i < PER; ++i) {
         const int e = tid * per + i;
         if (i < per && e < E) s_first[e] = (int)min(run, (long long)max_tiles);
         run += tiles[i];
-        if (i < per && e == E - 1) s_first[E] = (int)min(run, (long long)max_tiles);
+        if (i < per && e == E - 1) {
+            s_first[E] = (int)min(run, (long long)max_tiles);
+            if (dropped) *dropped = run > max_tiles;
+        }
     }
     __syncthreads();
     for (int e = tid; e <= E; e += 256) kb_start[e] = s_first[e];
@@ -2097,9 +2107,9 @@ segment_tiles_kernel(const int64_t* __restrict__ starts, const int64_t* __restri
 }
 
 int segment_tiles(const int64_t* starts, const int64_t* ends, int E, int64_t T, int* kb_start, int* tile_src, int* tile_cnt,
-                  int max_tiles, cudaStream_t st) {
+                  int max_tiles, int* dropped, cudaStream_t st) {
     CINN_CHECK_ARG(E >= 1 && E <= MAX_SEGMENT_EXPERTS && T >= 0 && T < (1LL << 31) && max_tiles >= 1, "segment_tiles: 1 <= experts <= 1024");
-    launch_dependent(segment_tiles_kernel, dim3(1), dim3(256), 0, st, starts, ends, E, T, kb_start, tile_src, tile_cnt, max_tiles);
+    launch_dependent(segment_tiles_kernel, dim3(1), dim3(256), 0, st, starts, ends, E, T, kb_start, tile_src, tile_cnt, max_tiles, dropped);
     CINN_CHECK_LAUNCH();
     return CINN_OK;
 }
@@ -2139,12 +2149,12 @@ int quantize_transposed_segmented(const void* x, int dtype, int64_t M, int64_t L
 
 // dY (T, N) of a 2-byte type -> q_row (T, N) + s_row (T, N / 128) for the rows inside segments, and the transposed,
 // segment-padded quantisation q_col (N, max_tiles * 128) + s_col (N, max_tiles); one pass (quant_row_dual_seg_kernel).
-// block: q_col is the block-scaled copy of the row-wise result instead, s_col (max_tiles, N / 128).
+// block: q_col is the block-scaled copy of the row-wise result instead, s_col (max_tiles, N / 128), and `dropped` says whether tiles are missing.
 int quantize_dual_segmented(const void* x, int dtype, int64_t T, int64_t N, void* q_row, float* s_row, void* q_col, float* s_col,
                             int max_tiles, const int* tile_src, const int* tile_cnt, const int* n_tiles, int div_mode,
-                            cudaStream_t st, bool block) {
+                            cudaStream_t st, bool block, const int* dropped) {
     CINN_CHECK_ARG((dtype == CINN_BF16 || dtype == CINN_F16) && T >= 1 && T < (1LL << 31) && N >= 128 && N % 128 == 0 &&
-                   max_tiles >= 1 && max_tiles <= 65535, "segmented dual quantiser: 2-byte input, N a multiple of 128");
+                   max_tiles >= 1 && max_tiles <= 65535 && (!block || dropped), "segmented dual quantiser: 2-byte input, N a multiple of 128");
     CINN_CHECK_ARG(x && q_row && s_row && q_col && s_col && tile_src && tile_cnt && n_tiles && aligned16(x) && aligned16(q_row) &&
                    aligned16(q_col), "segmented dual quantiser: null or unaligned pointer");
     CUtensorMap tm;
@@ -2159,7 +2169,7 @@ int quantize_dual_segmented(const void* x, int dtype, int64_t T, int64_t N, void
         constexpr auto kern = quant_row_dual_seg_kernel<TT, DIV, MODE>;                                               \
         if (const int failed = allow_smem_once<kern>(DUAL_SMEM_BYTES)) return failed;                                 \
         launch_early_if(quantise_early(T, N, st), kern, dim3(grid), dim3(256), DUAL_SMEM_BYTES, st, tm, (uint8_t*)q_row, s_row, (uint8_t*)q_col, s_col, max_tiles * 128, (int)N, \
-                                                 nb_n, max_tiles, tile_src, tile_cnt, n_tiles);                       \
+                                                 nb_n, max_tiles, tile_src, tile_cnt, n_tiles, (const TT*)x, T, dropped); \
     } while (0)
 #define CINN_DS(TT, DIV) do { if (block) CINN_DSM(TT, DIV, 2); else CINN_DSM(TT, DIV, 0); } while (0)
     if (dtype == CINN_BF16) { if (div_mode == CINN_DIV_FULL) CINN_DS(__nv_bfloat16, CINN_DIV_FULL); else CINN_DS(__nv_bfloat16, CINN_DIV_RN); }

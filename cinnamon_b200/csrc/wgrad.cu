@@ -86,12 +86,12 @@ int fp8_grouped_wgrad(const void* dY, int dy_dtype, const void* x_q, const float
 // Needs d_out and d_in multiples of 256; starts / ends are DEVICE arrays here.
 // ---------------------------------------------------------------------------
 int segment_tiles(const int64_t* starts, const int64_t* ends, int E, int64_t T, int* kb_start, int* tile_src, int* tile_cnt,
-                  int max_tiles, cudaStream_t st);
+                  int max_tiles, int* dropped, cudaStream_t st);
 int quantize_transposed_segmented(const void* x, int dtype, int64_t M, int64_t L, void* q, float* scales, int max_tiles,
                                   const int* tile_src, const int* tile_cnt, const int* n_tiles, int div_mode, cudaStream_t st);
 int quantize_dual_segmented(const void* x, int dtype, int64_t T, int64_t N, void* q_row, float* s_row, void* q_col, float* s_col,
                             int max_tiles, const int* tile_src, const int* tile_cnt, const int* n_tiles, int div_mode,
-                            cudaStream_t st, bool block);
+                            cudaStream_t st, bool block, const int* dropped);
 int requant_row_to_block_segmented(const void* xq, const float* xs, int64_t K, void* out, float* scales, int max_tiles,
                                    const int* tile_src, const int* tile_cnt, const int* n_tiles, int div_mode, cudaStream_t st);
 int fp8_gemm_grouped_k(const void* A, const float* sA, const void* B, const float* sB, const int* kb_start, int64_t E,
@@ -135,7 +135,7 @@ int fp8_grouped_wgrad_fused(const void* dY, int dy_dtype, const void* x_q, const
     float* a_s = reinterpret_cast<float*>(a_q + up(d_out * mt * 128, 256));
     uint8_t* b_q = reinterpret_cast<uint8_t*>(a_s) + up(d_out * mt * 4, 256);
     float* b_s = reinterpret_cast<float*>(b_q + up(d_in * mt * 128, 256));
-    int rc = segment_tiles(starts_dev, ends_dev, (int)E, T, kb_start, tile_src, tile_cnt, (int)mt, st);
+    int rc = segment_tiles(starts_dev, ends_dev, (int)E, T, kb_start, tile_src, tile_cnt, (int)mt, nullptr, st);
     if (rc) return rc;
     if (h12 != nullptr) {
         CINN_CHECK_ARG(dy_q_row != nullptr && div_mode == CINN_DIV_FULL && mt <= 65535, "grouped_wgrad_swiglu: needs the row-wise outputs and div.full");
@@ -144,7 +144,7 @@ int fp8_grouped_wgrad_fused(const void* dY, int dy_dtype, const void* x_q, const
     } else if (dy_q_row != nullptr)
         // both quantisations of dY in one pass: the caller's grouped input gradient reads the row-wise one
         rc = quantize_dual_segmented(dY, dy_dtype, T, d_out, dy_q_row, dy_s_row, a_q, a_s, (int)mt, tile_src, tile_cnt, kb_start + E,
-                                     div_mode, st, false);
+                                     div_mode, st, false, nullptr);
     else
         rc = quantize_transposed_segmented(dY, dy_dtype, d_out, d_out, a_q, a_s, (int)mt, tile_src, tile_cnt, kb_start + E, div_mode, st);
     if (rc) return rc;
@@ -156,13 +156,13 @@ int fp8_grouped_wgrad_fused(const void* dY, int dy_dtype, const void* x_q, const
 // ---------------------------------------------------------------------------
 // The same with x's part made by the forward: one pass over x writes its row-wise quantisation (what the forward's GEMM reads) and, into
 // `segments`, the experts' tiles and the block-scaled, transposed copy of that result; the backward keeps `segments` in place
-// of the row-wise bytes.  Same bytes as the calls above.  Layout of `segments`: tiles (ints) | bytes | scales.
+// of the row-wise bytes.  Same bytes as the calls above.  Layout of `segments`: tiles (ints) | bytes | scales | whether tiles were dropped.
 // ---------------------------------------------------------------------------
 static int64_t segment_ints_bytes(int64_t E, int64_t mt) { return up((E + 1 + 2 * mt) * 4, 256); }
 
 int64_t quant_segments_bytes(int64_t T, int64_t E, int64_t d) {
     const int64_t mt = fused_max_tiles(T < 0 ? 0 : T, E < 0 ? 0 : E);
-    return segment_ints_bytes(E, mt) + up(d * mt * 128, 256) + up(mt * ((d + 127) / 128) * 4, 256);
+    return segment_ints_bytes(E, mt) + up(d * mt * 128, 256) + up(mt * ((d + 127) / 128) * 4, 256) + 256;
 }
 
 // swiglu: x is (T, 2 * d) and what is quantised is silu(x[:, :d]) * x[:, d:]
@@ -177,7 +177,8 @@ int quantize_row_segments(const void* x, int dtype, int64_t T, int64_t d, const 
     int* kb_start = static_cast<int*>(segments);
     int *tile_src = kb_start + (E + 1), *tile_cnt = tile_src + mt;
     uint8_t* b_q = static_cast<uint8_t*>(segments) + segment_ints_bytes(E, mt);
-    int rc = segment_tiles(starts_dev, ends_dev, (int)E, T, kb_start, tile_src, tile_cnt, (int)mt, st);
+    int* dropped = reinterpret_cast<int*>(static_cast<uint8_t*>(segments) + quant_segments_bytes(T, E, d) - 256);
+    int rc = segment_tiles(starts_dev, ends_dev, (int)E, T, kb_start, tile_src, tile_cnt, (int)mt, dropped, st);
     if (rc) return rc;
     if (swiglu) {
         CINN_CHECK_ARG(div_mode == CINN_DIV_FULL, "swiglu_quant_segments: div.full only");
@@ -185,7 +186,7 @@ int quantize_row_segments(const void* x, int dtype, int64_t T, int64_t d, const 
         return swiglu_quant_block(x, dtype, T, d, q_row, s_row, b_q, reinterpret_cast<float*>(b_q + up(d * mt * 128, 256)), 0, &seg, st);
     }
     return quantize_dual_segmented(x, dtype, T, d, q_row, s_row, b_q, reinterpret_cast<float*>(b_q + up(d * mt * 128, 256)), (int)mt, tile_src,
-                                   tile_cnt, kb_start + E, div_mode, st, true);
+                                   tile_cnt, kb_start + E, div_mode, st, true, dropped);
 }
 
 int64_t grouped_wgrad_segments_scratch_bytes(int64_t T, int64_t E, int64_t d_out) {
@@ -213,7 +214,7 @@ int fp8_grouped_wgrad_segments(const void* dY, int dy_dtype, const void* segment
     uint8_t* a_q = static_cast<uint8_t*>(scratch);
     float* a_s = reinterpret_cast<float*>(a_q + up(d_out * mt * 128, 256));
     const int rc = dy_q_row != nullptr
-        ? quantize_dual_segmented(dY, dy_dtype, T, d_out, dy_q_row, dy_s_row, a_q, a_s, (int)mt, tile_src, tile_cnt, kb_start + E, div_mode, st, false)
+        ? quantize_dual_segmented(dY, dy_dtype, T, d_out, dy_q_row, dy_s_row, a_q, a_s, (int)mt, tile_src, tile_cnt, kb_start + E, div_mode, st, false, nullptr)
         : quantize_transposed_segmented(dY, dy_dtype, d_out, d_out, a_q, a_s, (int)mt, tile_src, tile_cnt, kb_start + E, div_mode, st);
     if (rc) return rc;
     return fp8_gemm_grouped_k(a_q, a_s, b_q, b_s, kb_start, E, d_out, d_in, mt, dW, out_dtype, st);

@@ -252,7 +252,9 @@ int cinn_fp8_grouped_wgrad_fused(const void* dY, int dy_dtype, const void* x_q, 
  * row-wise for the rows inside expert ranges - q_row (T, d), s_row (T, d / 128), other rows are left alone - and writes into
  * `segments` what the weight gradient reads of x (the experts' tiles and the block-scaled, transposed copy of that result);
  * cinn_fp8_grouped_wgrad_segments takes it in place of x_q, x_scales and the ranges.  Same bytes as cinn_quant_rowwise and
- * cinn_fp8_grouped_wgrad_fused.  T + 127 * E at most about 8 million rows; segments and scratch 256-byte aligned. */
+ * cinn_fp8_grouped_wgrad_fused.  T + 127 * E at most about 8 million rows; segments and scratch 256-byte aligned.  `segments` holds
+ * T rounded up to 128 and 128 * E rows: ranges that overlap can need more, and then all rows are quantised row-wise, but the weight
+ * gradient leaves rows out, as cinn_fp8_grouped_wgrad_fused does (cinn_swiglu_quant_segments takes disjoint ranges only). */
 int64_t cinn_quant_segments_bytes(int64_t T, int64_t E, int64_t d);
 int cinn_quant_rowwise_segments(const void* x, int x_dtype, int64_t T, int64_t d, const int64_t* starts, const int64_t* ends, int64_t E,
                                 void* q_row, float* s_row, void* segments, int64_t segments_bytes, int div_mode, void* stream);

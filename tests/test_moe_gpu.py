@@ -528,3 +528,19 @@ def test_dispatch_signal_by_expert_ranges(K):
     for i in range(G):
         assert torch.equal(bufs[0][i], bufs[1][i]) and torch.equal(scs[0][i], scs[1][i])
     assert call(2, 2, 160) != 0 and call(0, e_local + 1, 160) != 0   # empty / out-of-range expert ranges are refused
+
+
+def test_grouped_forward_with_overlapping_ranges_and_a_gradient_to_come(K):
+    """Overlapping ranges can need more padded tiles than there are: the rows of an expert behind them are quantised all the same, so that
+    the result does not depend on whether the weight wants a gradient."""
+    g = torch.Generator(device="cuda").manual_seed(11)
+    R, d_in, d_out = 1000, 512, 256
+    x = torch.randn(R, d_in, device="cuda", generator=g).to(torch.bfloat16)
+    w = torch.randn(3, d_out, d_in, device="cuda", generator=g).mul_(0.02).requires_grad_(True)
+    starts, ends = (torch.tensor(v, device="cuda") for v in ([0, 0, 900], [900, 900, R]))
+    poison = torch.full((4 << 20,), 0x7f, dtype=torch.uint8, device="cuda")             # whatever is not written reads as NaN
+    del poison
+    y = K.moe_grouped_gemm(x, w, starts, ends, dtype=torch.bfloat16)
+    with torch.no_grad():
+        ref = K.moe_grouped_gemm(x, w, starts, ends, dtype=torch.bfloat16)
+    assert torch.equal(y[900:], ref[900:])
