@@ -35,6 +35,13 @@ bool swiglu_in_quantisers(const Tensor& h12, bool kmajor, int div) {
            I >= 128 && I % 128 == 0 && (reinterpret_cast<uintptr_t>(h12.data_ptr()) & 15) == 0;
 }
 
+// Whether the copy of the activations in the experts' tiles may be kept for the backward in place of the row-wise bytes.  It holds up to
+// 128 rows more per expert: no more than there are rows, or than an eighth of the experts' e4m3 weights, which are kept as well.  (2048 rows of
+// 7168 over 64 experts of 4096 outputs: 73 MB in place of 15, beside weights of 1.9 GB; over 64 of 512, 2048 rows stay row-wise.)
+bool segments_fit(int64_t rows, int64_t experts, int64_t d_out) {
+    return experts >= 1 && experts <= 1024 && up(rows, 128) + experts <= 65535 && (128 * experts <= rows || 8 * 128 <= d_out);
+}
+
 // linear_forward(swiglu_rounded(h12), w, ...) of a weight that wants its gradient
 Linear swiglu_linear_forward(const Tensor& h12, const Tensor& w, bool round_scale, bool need_dgrad, int div) {
     const at::Device dev = h12.device();
@@ -206,7 +213,7 @@ struct BlockNode : public torch::autograd::Function<BlockNode> {
         Quantised h;
         Tensor out;
         const bool segments = (w12.requires_grad() || w3.requires_grad() || x.requires_grad()) && swiglu_in_quantisers(h12, true, o->div) &&
-                              r.pairs > 0 && h12.size(1) % 512 == 0 && d % 256 == 0 && E <= 1024 && up(r.pairs, 128) + E <= 65535;
+                              r.pairs > 0 && h12.size(1) % 512 == 0 && d % 256 == 0 && segments_fit(r.pairs, E, d);
         if (segments) {
             const int64_t I = h12.size(1) / 2, bytes = api.cinn_quant_segments_bytes(r.pairs, E, I);
             const Quantised hq{empty({r.pairs, I}, F8, dev), empty({r.pairs, I / 128}, at::kFloat, dev)};
@@ -324,7 +331,7 @@ struct GroupedNode : public torch::autograd::Function<GroupedNode> {
         const int64_t R = x.size(0), E = wq->q.size(0), d = x.dim() == 2 ? x.size(1) : 0;
         // Where the weight gradient can be had (its widths are multiples of 256) its copy of x comes out of the forward's pass.
         const bool segments = w.requires_grad() && x.dim() == 2 && x.element_size() == 2 && x.is_contiguous() && R > 0 && d == wq->q.size(2) &&
-                              d % 256 == 0 && wq->q.size(1) % 256 == 0 && E >= 1 && E <= 1024 && up(R, 128) + E <= 65535 &&
+                              d % 256 == 0 && wq->q.size(1) % 256 == 0 && segments_fit(R, E, wq->q.size(1)) &&
                               starts.numel() == E && ends.numel() == E && (reinterpret_cast<uintptr_t>(x.data_ptr()) & 15) == 0;
         Quantised xq;
         if (segments) {

@@ -544,3 +544,31 @@ def test_grouped_forward_with_overlapping_ranges_and_a_gradient_to_come(K):
     with torch.no_grad():
         ref = K.moe_grouped_gemm(x, w, starts, ends, dtype=torch.bfloat16)
     assert torch.equal(y[900:], ref[900:])
+
+
+@pytest.mark.parametrize("E,R,d_out", [(64, 300, 512), (8, 2048, 512), (16, 40, 1024)])
+def test_what_a_grouped_gemm_keeps_for_its_backward(K, E, R, d_out):
+    """The copy of x that is kept holds at most as many rows again as x, or an eighth of the weights' bytes; the gradients are the same
+    either way."""
+    g = torch.Generator(device="cuda").manual_seed(E)
+    d_in = 512
+    x = torch.randn(R, d_in, device="cuda", generator=g).to(torch.bfloat16)
+    w = torch.randn(E, d_out, d_in, device="cuda", generator=g).mul_(0.02).requires_grad_(True)
+    ends = torch.arange(1, E + 1, device="cuda") * R // E
+    starts = torch.cat([ends.new_zeros(1), ends[:-1]])
+    dy = torch.randn(R, d_out, device="cuda", generator=g).to(torch.bfloat16)
+    K.moe_grouped_gemm(x, w, starts, ends, dtype=torch.bfloat16)                         # (the weight's e4m3 copy may be kept between calls)
+    before = torch.cuda.memory_allocated()
+    y = K.moe_grouped_gemm(x, w, starts, ends, dtype=torch.bfloat16)
+    held = torch.cuda.memory_allocated() - before - y.numel() * 2
+    weights, rows = E * d_out * d_in, -(-R // 128) * 128 * d_in
+    held -= weights if held >= weights else 0                                            # (where it is not kept)
+    assert held <= max(2 * rows, rows + weights // 8) * 1.05 + weights // 1024 + (1 << 20)     # (blocks of the allocator: up to 1 MiB more)
+    gw, = torch.autograd.grad(y, [w], dy)
+    q, s = K.quantize_fp8_rowwise(x)
+    ref = torch.zeros_like(w)
+    for e in range(E):
+        a, b = int(starts[e]), int(ends[e])
+        if b > a:
+            ref[e] = dy[a:b].float().t() @ (q[a:b].float() * s[a:b].repeat_interleave(128, 1))
+    assert float((gw - ref).norm() / ref.norm()) < 0.06
