@@ -486,3 +486,47 @@ def test_grouped_weight_gradient_with_swiglu(K, counts):
         K.set_div_mode(mode)
     for a, b in zip(*res):
         assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("kind", ["special", "huge", "tiny"])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_swiglu_inside_the_quantisers_on_special_values(K, kind, dtype):
+    """NaN and infinity in the activations and the gradient, and values whose products overflow or vanish: the bytes and scales of the
+    separate calls, in the dense and the segmented passes."""
+    T, I, mode = 300, 256, K.get_div_mode()
+    h12, dh = _pieces(T, 2 * I, kind, dtype, 5), _pieces(T, I, kind, dtype, 6)
+    tag, Tp, nb, nbi = K._DTYPE_TAG[dtype], (T + 15) // 16 * 16, (T + 127) // 128, I // 128
+    e8 = lambda *n: torch.empty(*n, device="cuda", dtype=torch.float8_e4m3fn)                 # noqa: E731
+    e4 = lambda *n: torch.empty(*n, device="cuda")                                            # noqa: E731
+
+    def same(got, want):
+        for a, b in zip(got, want):
+            if a.dtype == torch.float32:
+                assert torch.equal(a.nan_to_num(-1.0), b.nan_to_num(-1.0)) and torch.equal(a.isnan(), b.isnan())
+            else:
+                assert torch.equal(a.view(torch.uint8) & 0x7f, b.view(torch.uint8) & 0x7f)     # (a NaN may have either sign)
+                assert torch.equal(a.float().nan_to_num(0.0), b.float().nan_to_num(0.0))
+
+    K.set_div_mode("full")
+    try:
+        h, dh12 = torch.empty(T, I, device="cuda", dtype=dtype), torch.empty(T, 2 * I, device="cuda", dtype=dtype)
+        assert K._L.cinn_swiglu_rounded(K._ptr(h12), K._ptr(h), tag, T, I, K._stream(h)) == 0
+        got = (e8(T, I), e4(T, nbi), e8(I, Tp), e4(nb, nbi))
+        assert K._L.cinn_swiglu_rounded_quant_block_t(K._ptr(h12), tag, T, I, *map(K._ptr, got), 0, K._stream(h)) == 0
+        same(got, K.quantize_fp8_rowwise_with_block(h, False, transpose_block=True, _padded=True))
+        assert K._L.cinn_swiglu_rounded_backward(K._ptr(h12), K._ptr(dh), K._ptr(dh12), tag, T, I, K._stream(h)) == 0
+        got = (e8(T, 2 * I), e4(T, 2 * nbi), e8(2 * I, Tp), e4(2 * I, nb))
+        assert K._L.cinn_swiglu_rounded_backward_quant_dual(K._ptr(h12), K._ptr(dh), tag, T, I, *map(K._ptr, got), 0, K._stream(h)) == 0
+        same(got, K._quantize_dual_padded(dh12, False))
+        starts, ends = _ranges([100, 7, 193])
+        q, s = e8(T, I), e4(T, nbi)
+        buf = torch.empty(K._L.cinn_quant_segments_bytes(T, 3, I), device="cuda", dtype=torch.uint8)
+        assert K._L.cinn_swiglu_quant_segments(K._ptr(h12), tag, T, I, K._ptr(starts), K._ptr(ends), 3, K._ptr(q), K._ptr(s), K._ptr(buf),
+                                               buf.numel(), K._stream(h)) == 0
+        rq, r_s = K.swiglu_quantize_rowwise(h12)
+        same((q, s), (rq, r_s))
+        _, bq, bs = _segment_parts(K, buf, T, 3, I)
+        want_q, want_s = _segment_reference(K, rq, r_s, starts, ends, I)
+        same((bq.contiguous().view(torch.float8_e4m3fn), bs.contiguous()), (want_q.contiguous().view(torch.float8_e4m3fn), want_s))
+    finally:
+        K.set_div_mode(mode)
