@@ -156,9 +156,6 @@ __device__ __forceinline__ void store_parts16(uint32_t rest, uint32_t lead, cons
     st8(rest, mid);
     st8(rest + 8, lo);
 }
-// A panel used K-major (its 64 columns are the reduction axis; a step of four takes 16 of them: 32 bytes) and MN-major (its 128
-// rows are; a step of eight takes 16 of them: 2048 bytes).  Both have one descriptor, of which only the low word (the address in
-// units of 16 bytes) varies.
 
 // D (+)= part X of a tensor-memory operand of 16 STEPS positions (store_parts16) times an MN-major panel
 template <int X, int STEPS = 8>

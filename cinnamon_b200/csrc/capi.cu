@@ -117,7 +117,6 @@ int p2p_row_table_wait(const int64_t* seg_start, const int64_t* home_base, const
 int64_t quant_segments_bytes(int64_t T, int64_t E, int64_t d);
 int quantize_row_segments(const void* x, int dtype, int64_t T, int64_t d, const int64_t* starts_dev, const int64_t* ends_dev, int64_t E,
                           void* q_row, float* s_row, void* segments, int64_t segments_bytes, int div_mode, bool swiglu, cudaStream_t st);
-struct SegmentTiles;
 int swiglu_quant_block(const void* h12, int dtype, int64_t T, int64_t I, void* q_row, float* s_row, void* q_blk, float* s_blk, int round_scale,
                        const SegmentTiles* seg, cudaStream_t st);
 int swiglu_backward_quant_dual(const void* h12, const void* dh, int dtype, int64_t T, int64_t I, void* q_row, float* s_row, void* q_col,

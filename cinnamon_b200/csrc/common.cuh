@@ -93,6 +93,9 @@ inline int allow_smem_once(size_t bytes) {
 
 int sm_count();   // SMs of the current device (cached per device)
 
+// The tiles of the experts' row ranges, on the device: first row and rows of each, how many there are; at most `max`
+struct SegmentTiles { const int *src, *cnt, *n; int max; };
+
 // launch_dependent if `early`, else a plain launch: the kernel starts when the one before it has ended.  Both leave an error
 // where CINN_CHECK_LAUNCH finds it.
 template <typename... P, typename... A>

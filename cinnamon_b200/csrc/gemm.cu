@@ -575,8 +575,6 @@ int encode_map_2d(CUtensorMap* map, const void* base, uint64_t inner, uint64_t r
     return CINN_OK;
 }
 
-// 3-D map: `planes` matrices of (rows, inner), boxes of box_inner columns x box_rows of one matrix; rows past a matrix's end
-// read as zeros instead of its neighbour's, and are not written
 int encode_map(CUtensorMap* map, const void* base, uint32_t rank, const uint64_t* dims, const uint64_t* strides, const uint32_t* box,
                CUtensorMapDataType dtype, CUtensorMapSwizzle swizzle) {
     EncodeFn enc = get_encode();
@@ -598,6 +596,8 @@ int encode_map(CUtensorMap* map, const void* base, uint32_t rank, const uint64_t
     return CINN_OK;
 }
 
+// 3-D map: `planes` matrices of (rows, inner), boxes of box_inner columns x box_rows of one matrix; rows past a matrix's end
+// read as zeros instead of its neighbour's, and are not written
 int encode_map_3d(CUtensorMap* map, const void* base, uint64_t inner, uint64_t rows, uint64_t planes, uint64_t pitch_bytes,
                   uint32_t box_rows, CUtensorMapDataType dtype, uint32_t box_inner, CUtensorMapSwizzle swizzle) {
     EncodeFn enc = get_encode();

@@ -373,7 +373,9 @@ struct GroupedNode : public torch::autograd::Function<GroupedNode> {
 void bind_moe_train(pybind11::module_& m) {
     m.def("swiglu_block", [](const Tensor& x, const Tensor& w1, const Tensor& w2, const Tensor& w3, bool round12, bool round3, bool kmajor,
                              int div) {
-        if (!takes_node(x, w1, w2, w3)) {          // nothing is kept for a backward; with gradients or without, the same numbers
+        // Nothing is kept for a backward; with gradients or without, the same numbers.  Its linears quantise and multiply in two launches on any
+        // number of rows: the one-kernel form has the same bits, but this call's five launches are part of what it promises.
+        if (!takes_node(x, w1, w2, w3)) {
             const Tensor h12 = linear_inference(x, at::cat({w1, w2}), round12, div, false);
             c10::cuda::CUDAGuard guard(x.device());
             Tensor y = linear_inference(swiglu_rounded(h12.view({-1, h12.size(-1)})), w3, round3, div, false);

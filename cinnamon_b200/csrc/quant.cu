@@ -2212,8 +2212,6 @@ int requant_row_to_block_segmented(const void* xq, const float* xs, int64_t K, v
 
 // SwiGLU with the quantisers that follow it: see the kernels.  seg: the experts' tiles (null: one range of all T rows); M is the length of
 // the transposed copies' rows before their rounding up to 16.
-struct SegmentTiles { const int *src, *cnt, *n; int max; };
-
 static int check_swiglu(const void* h12, int dtype, int64_t T, int64_t I, const void* q_row, const void* q_t, const char* what) {
     CINN_CHECK_ARG(dtype == CINN_BF16 || dtype == CINN_F16, "%s: 2-byte activations", what);
     CINN_CHECK_ARG(T >= 1 && T <= 65535 * 128 && I >= 128 && I % 128 == 0 && I < (1LL << 30), "%s: rows %lld, hidden width %lld (a multiple of 128)",

@@ -87,8 +87,9 @@ __host__ __device__ constexpr uint32_t make_idesc_f16(bool bf16, int m, int n, b
            | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(m >> 4) << 24);
 }
 
-// Operands in panels: 128 rows (or as many as the other side has) of 128 bytes, 128-byte swizzle.  The low word of a panel's descriptor;
-// the high one is the same for all.
+// Operands in panels: 128 rows (or as many as the other side has) of 128 bytes, 128-byte swizzle.  A panel is used K-major (its 64 columns
+// are the reduction axis; a step of four takes 16 of them: 32 bytes) and MN-major (its 128 rows are; a step of eight takes 16 of them: 2048
+// bytes).  Both have one descriptor, of which only the low word (the address in units of 16 bytes) varies.
 constexpr uint32_t DESC_HI = (uint32_t)((((uint64_t)(1024 >> 4) << 32) | (1ull << 46) | (2ull << 61)) >> 32);
 __device__ __forceinline__ uint32_t panel_desc(uint32_t panel) { return ((panel >> 4) & 0x3FFFu) | (1u << 16); }
 

@@ -97,7 +97,6 @@ int requant_row_to_block_segmented(const void* xq, const float* xs, int64_t K, v
 int fp8_gemm_grouped_k(const void* A, const float* sA, const void* B, const float* sB, const int* kb_start, int64_t E,
                        int64_t M, int64_t N, int64_t max_tiles, void* C, int out_dtype, cudaStream_t st);
 
-struct SegmentTiles { const int *src, *cnt, *n; int max; };      // as in quant.cu
 int swiglu_quant_block(const void* h12, int dtype, int64_t T, int64_t I, void* q_row, float* s_row, void* q_blk, float* s_blk, int round_scale,
                        const SegmentTiles* seg, cudaStream_t st);
 int swiglu_backward_quant_dual(const void* h12, const void* dh, int dtype, int64_t T, int64_t I, void* q_row, float* s_row, void* q_col,
