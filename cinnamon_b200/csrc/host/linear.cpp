@@ -193,9 +193,9 @@ Tensor linear_inference(const Tensor& x, const Tensor& weight, bool round_scale,
     shape.back() = N;
     Tensor out = empty(shape, at::kBFloat16, x.device());
     // under capture the launch that the one kernel saves costs next to nothing, and with many rows the two are shorter (csrc/linear_few.cu)
-    const auto pays = [&] { return M <= 32 || K <= 128 || c10::cuda::currentStreamCaptureStatusMayInitCtx() == c10::cuda::CaptureStatus::None; };
-    if (one_kernel && M <= 128 && pays() && api.cinn_fp8_linear_few_takes(xf.data_ptr(), tag_of(xf.scalar_type()), xf.stride(0), xf.stride(1), wf.data_ptr(),
-                                      tag_of(wf.scalar_type()), wf.stride(0), wf.stride(1), M, N, K)) {
+    const auto pays = [&] { return M <= 32 || K <= 128 || !capturing(); };
+    if (one_kernel && M <= 128 && K <= 1024 && api.cinn_fp8_linear_few_takes(xf.data_ptr(), tag_of(xf.scalar_type()), xf.stride(0), xf.stride(1), wf.data_ptr(),
+                                      tag_of(wf.scalar_type()), wf.stride(0), wf.stride(1), M, N, K) && pays()) {
         check(api.cinn_fp8_linear_few(xf.data_ptr(), tag_of(xf.scalar_type()), xf.stride(0), round_scale, f32(wf), wf.stride(0),
                                       out.data_ptr(), M, N, K, div, stream()), "cinn_fp8_linear_few");
         return out;

@@ -310,11 +310,14 @@ static int clusters_at_once(int slices) {
 // CTAs that share a column tile's reduction: one per K block if their clusters all run at once and leave an eighth of the SMs (sizes that do
 // not divide 16: a quarter) to what runs beside.  Sixteen clusters of eight were 128 CTAs of 148 and ran in two turns: 8 x 1024 -> 2048 12.5 us
 // where the two kernels take 7.5.
+static bool fits_at_once(int64_t tiles, int s) {
+    return s == 1 || (tiles * s <= sm_count() * (16 % s == 0 ? 7 : 6) / 8 && tiles <= clusters_at_once(s));
+}
 static int slices_of(int64_t N, int64_t K) {
     const int64_t tiles = (N + TILE - 1) / TILE, KB = (K + TILE - 1) / TILE;
-    for (int s = (int)(KB < MAX_SLICES ? KB : MAX_SLICES); s > 1; --s)
-        if (tiles * s <= sm_count() * (16 % s == 0 ? 7 : 6) / 8 && tiles <= clusters_at_once(s)) return s;
-    return 1;
+    int s = (int)(KB < MAX_SLICES ? KB : MAX_SLICES);
+    while (!fits_at_once(tiles, s)) --s;
+    return s;
 }
 
 template <typename TX, int DIV, bool ROUND, bool ONE>
@@ -371,8 +374,9 @@ static bool fits(const void* x, int x_dtype, int64_t ldx_m, int64_t ldx_k, const
 // So callers under capture take it for up to 32 rows, or for one K block in all (csrc/host/linear.cpp).
 bool linear_few_takes(const void* x, int x_dtype, int64_t ldx_m, int64_t ldx_k, const void* w, int w_dtype, int64_t ldw_n, int64_t ldw_k,
                       int64_t M, int64_t N, int64_t K) {
-    return fits(x, x_dtype, ldx_m, ldx_k, w, w_dtype, ldw_n, ldw_k, M, N, K) && !gemm_sms_capped() &&
-           (K + few::TILE - 1) / few::TILE <= few::slices_of(N, K);
+    const int64_t KB = (K + few::TILE - 1) / few::TILE;
+    return KB <= few::MAX_SLICES && fits(x, x_dtype, ldx_m, ldx_k, w, w_dtype, ldw_n, ldw_k, M, N, K) && !gemm_sms_capped() &&
+           few::fits_at_once((N + few::TILE - 1) / few::TILE, (int)KB);
 }
 
 int linear_few(const void* x, int x_dtype, int64_t ldx, int round_scale, const float* w, int64_t ldw, void* out, int64_t M, int64_t N,
