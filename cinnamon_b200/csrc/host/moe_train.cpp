@@ -28,9 +28,16 @@ Tensor swiglu_rounded(const Tensor& h12) {
     return h;
 }
 
-// Whether SwiGLU can be part of the quantisers next to it
+// Whether SwiGLU can be part of the quantisers next to it, and pays.  It saves a launch and a pass over memory, but a piece of 128 x 128 takes a CTA
+// 8 - 10 us, two to an SM at a time: where the pieces do not fill a turn, or just begin a second, the separate passes are shorter.  us from a graph, in
+// the quantisers and by itself, forward, dense and routed backward (with its product): 32 pieces 7.6 and 6.1, 10.0 and 6.1, 25.1 and 21.8; 192 10.3
+// and 10.2, 14.0 and 12.5, 30.1 and 28.8; 256 10.8 and 11.4, 14.7 and 14.9, 31.5 and 33.2; 384 17.4 and 15.7, 23.5 and 21.3, 48.5 and 48.1; 512 20.9 and
+// 19.3, 27.7 and 28.8, 54.7 and 57.3; 2048 67 and 71, 96 and 105, 155 and 166.  Outside a graph a block so small waits for the host, which has a launch
+// less to make.
 bool swiglu_in_quantisers(const Tensor& h12, bool kmajor, int div) {
-    const int64_t T = h12.size(0), I = h12.size(1) / 2;
+    const int64_t T = h12.size(0), I = h12.size(1) / 2, pieces = up(T, 128) * (I / 128);
+    const int64_t sms = at::cuda::getCurrentDeviceProperties()->multiProcessorCount;
+    if (!(pieces > 3 * sms || (pieces >= 192 && pieces <= 2 * sms)) && capturing()) return false;
     return kmajor && div == CINN_DIV_FULL && h12.element_size() == 2 && tag_of(h12.scalar_type()) >= 0 && T >= 1 && T <= MAX_PADDED_ROWS &&
            I >= 128 && I % 128 == 0 && (reinterpret_cast<uintptr_t>(h12.data_ptr()) & 15) == 0;
 }

@@ -335,3 +335,30 @@ def test_launch_count_is_what_the_profiler_sees(K):
             torch.cuda.synchronize()
         seen = [e.name for e in prof.events() if e.device_type.name == "CUDA" and "cinn::" in e.name]
         assert K.launch_count - n == len(seen), (i, seen)
+
+
+@pytest.mark.parametrize("T", [40, 3100])
+def test_swiglu_in_training_under_capture(K, T):
+    """A few tokens under capture take SwiGLU as passes of its own, many take it inside the quantisers: the numbers of the call outside."""
+    from cinnamon_b200 import layers
+    torch.manual_seed(T)
+    with torch.device("cuda"):
+        block = K.convert_to_fp8(layers.SwiGLU(256, 1024))
+    x = torch.randn(T, 256, device="cuda").to(torch.bfloat16).requires_grad_(True)
+    dy = torch.randn(T, 256, device="cuda").to(torch.bfloat16)
+
+    def run():
+        n = K.launch_count
+        y = block(x)
+        g = torch.autograd.grad(y, [x, *block.parameters()], dy)
+        return [y.detach(), *g], K.launch_count - n
+
+    (want, outside), _ = run(), torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        got, inside = run()
+    graph.replay()
+    assert inside - outside == (2 if T == 40 else 0)          # SwiGLU by itself, forward and backward
+    for a, b in zip(got, want):
+        assert torch.equal(a, b)
+    del graph
