@@ -1,7 +1,6 @@
 // extern "C" surface of the library: argument marshalling only.
 #include "common.cuh"
 #include "../../include/cinnamon_b200.h"
-#include <mutex>
 
 namespace cinn {
 
@@ -17,17 +16,14 @@ void set_error(const char* fmt, ...) {
 std::atomic<int64_t> g_launches{0};
 
 int sm_count() {
-    static int cached[64];
-    static std::mutex mu;
-    int dev = 0;
+    static std::atomic<int> cached[64];
+    int dev = 0, n = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 148;
-    std::lock_guard<std::mutex> lk(mu);
-    if (cached[dev] == 0) {
-        int n = 0;
+    if ((n = cached[dev].load(std::memory_order_relaxed)) == 0) {
         if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) n = 148;
-        cached[dev] = n;
+        cached[dev].store(n, std::memory_order_relaxed);
     }
-    return cached[dev];
+    return n;
 }
 
 int quantize(bool blockwise, const void* x, int dtype, int64_t M, int64_t N, int64_t ld_m, int64_t ld_n, void* q,

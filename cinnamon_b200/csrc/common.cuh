@@ -104,14 +104,14 @@ inline cudaError_t launch_early_if(bool early, void (*kern)(P...), dim3 grid, di
     kern<<<grid, block, smem, st>>>(static_cast<P>(args)...);
     return cudaPeekAtLastError();
 }
-// Whether a launch on this stream becomes a node of a graph.  What an early start wins is the gap between two launches, and between a
+// Whether a launch on this stream becomes a node of a graph (never on the null stream).  What an early start wins is the gap between two launches, and between a
 // graph's nodes there is little of one.  us a replayed pass, quantisers, combine and row spread early and plain: linear forward and backward
 // 4096 x 512 -> 2048 55.6 and 53.9, 512 x 512 -> 2048 23.8 and 22.9, 2048 x 2048 -> 8192 158.1 and 156.1, forward 100 x 768 -> 2688 8.0 and 7.5,
 // serving layer of 64 tokens 79.5 and 77.1; the other way 300 x 512 -> 512 17.6 and 18.0, forward 4096 x 512 -> 2048 13.7 and 14.1, serving one
 // token 46.3 and 47.1.
 inline bool captured(cudaStream_t st) {
     cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
-    return cudaStreamIsCapturing(st, &status) == cudaSuccess && status != cudaStreamCaptureStatusNone;
+    return st != nullptr && cudaStreamIsCapturing(st, &status) == cudaSuccess && status != cudaStreamCaptureStatusNone;
 }
 // Whether a quantiser of so many rows starts early.  Short ones gain the launch.  In front of a GEMM of long tiles an early start costs more than it
 // wins, up to a tile's time: 403 x 4032 -> 12928 80 -> 96 us, 1824 x 6976 -> 8832 forward and backward 458 -> 470, 16384 x 7168 -> 18432 7020 ->

@@ -742,7 +742,7 @@ static inline int gemm_sms() {
     const int lim = g_gemm_sm_limit.load(std::memory_order_relaxed), all = sm_count();
     return (lim > 0 && lim < all) ? lim : all;
 }
-bool gemm_sms_capped() { return gemm_sms() < sm_count(); }
+bool gemm_sms_capped() { return g_gemm_sm_limit.load(std::memory_order_relaxed) > 0 && gemm_sms() < sm_count(); }
 int set_gemm_sm_limit(int n) { return g_gemm_sm_limit.exchange(n < 0 ? 0 : n); }
 
 static inline bool al16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }

@@ -188,9 +188,10 @@ def test_quantisers_start_early_for_short_rows_and_outside_a_capture(built, tmp_
     assert _run_over_runtime(tmp_path, """
 int main() {
     using cinn::quantise_early;
-    if (!quantise_early(4096, 512, nullptr) || quantise_early(4096, 4096, nullptr) || quantise_early(1 << 20, 1024, nullptr)) return 1;
+    const cudaStream_t s = reinterpret_cast<cudaStream_t>(0x1000);
+    if (!quantise_early(4096, 512, s) || quantise_early(4096, 4096, s) || quantise_early(1 << 20, 1024, s)) return 1;
     capturing = cudaStreamCaptureStatusActive;
-    if (quantise_early(4096, 512, nullptr) || !cinn::captured(nullptr)) return 2;
+    if (quantise_early(4096, 512, s) || !cinn::captured(s) || cinn::captured(nullptr)) return 2;
     return 0;
 }
 """) == 0
