@@ -271,11 +271,13 @@ __device__ __forceinline__ float half_warp_rows_max(const float (&m)[8], int sub
 // are the `cnt` source rows from `src0` on (the row-wise bytes and scales go to those rows; the rest of the piece
 // counts as zeros), while the transposed bytes and their scales go to the padded position `bm` of an output whose
 // token axis is `M` long (`nb_m` tiles).
-template <int DIV, bool ROUND, bool SEG = false, typename AfterSync>
+// ROLLED: in loops, for pieces that are rare (see unpack_piece).
+template <int DIV, bool ROUND, bool SEG = false, bool ROLLED = false, typename AfterSync>
 __device__ __forceinline__ bool dual_tile(float (&v)[8][8], float (*s_amax)[128], uint8_t* s_out, bool ok,
                                           uint8_t* __restrict__ q_row, float* __restrict__ s_row,
                                           uint8_t* __restrict__ q_col, float* __restrict__ s_col, int M, int N, int nb_n,
                                           int nb_m, int bm, int bn, AfterSync&& after_sync, int src0 = 0, int cnt = 128) {
+    constexpr int UNROLL = ROLLED ? 1 : 8;
     const int sub = threadIdx.x & 15, hw = threadIdx.x >> 4, warp = threadIdx.x >> 5;
     const int m0 = bm * 128, n0 = bn * 128;
     const int n = n0 + sub * 8;
@@ -283,20 +285,20 @@ __device__ __forceinline__ bool dual_tile(float (&v)[8][8], float (*s_amax)[128]
     const int m_rows = SEG ? src0 + cnt : M;                    // one past the last row that is written row-wise
     const int pitch = (M + 15) & ~15;                           // of the transposed rows, zeros behind M (whole 16-byte stores)
     if constexpr (SEG) {
-#pragma unroll
+#pragma unroll UNROLL
         for (int i = 0; i < 8; ++i)
             if (hw * 8 + i >= cnt) {
-#pragma unroll
+#pragma unroll UNROLL
                 for (int j = 0; j < 8; ++j) v[i][j] = 0.0f;
             }
     }
 
     // column tiles first: their reduction needs the barrier, the row tiles fill the wait
     float cam[8];
-#pragma unroll
+#pragma unroll UNROLL
     for (int j = 0; j < 8; ++j) {
         float a = 0.0f;
-#pragma unroll
+#pragma unroll UNROLL
         for (int i = 0; i < 8; ++i) a = fmaxf(a, fabsf(v[i][j]));
         cam[j] = fmaxf(a, __shfl_xor_sync(0xffffffffu, a, 16));
     }
@@ -311,7 +313,7 @@ __device__ __forceinline__ bool dual_tile(float (&v)[8][8], float (*s_amax)[128]
     if ((threadIdx.x & 31) < 16) {
         const int c = warp * 16 + sub;
         float a = s_amax[0][c];
-#pragma unroll
+#pragma unroll UNROLL
         for (int w = 1; w < 8; ++w) a = fmaxf(a, s_amax[w][c]);
         const float sc = scale_from_amax<DIV, ROUND>(a);
         s_amax[0][c] = divisor_of<DIV>(sc);
@@ -321,17 +323,17 @@ __device__ __forceinline__ bool dual_tile(float (&v)[8][8], float (*s_amax)[128]
     // row tiles: amax inside the half-warp, bytes straight to global memory
     {
         float m[8];
-#pragma unroll
+#pragma unroll UNROLL
         for (int i = 0; i < 8; ++i) {
             m[i] = 0.0f;
-#pragma unroll
+#pragma unroll UNROLL
             for (int j = 0; j < 8; ++j) m[i] = fmaxf(m[i], fabsf(v[i][j]));
         }
         const float s = scale_from_amax<DIV, ROUND>(half_warp_rows_max(m, sub));
         const float mine = divisor_of<DIV>(s);
         const int own = mt + half_warp_row(sub);
         if ((sub & 1) == 0 && own < m_rows && n0 < N) s_row[(int64_t)own * nb_n + bn] = s;
-#pragma unroll
+#pragma unroll UNROLL
         for (int i = 0; i < 8; ++i) {
             const float d = __shfl_sync(0xffffffffu, mine, half_warp_lane(i), 16);
             if (mt + i < m_rows && n < N) {
@@ -353,7 +355,7 @@ __device__ __forceinline__ bool dual_tile(float (&v)[8][8], float (*s_amax)[128]
         const float4 hi = *reinterpret_cast<const float4*>(&s_amax[0][sub * 8 + 4]);
         dv[0] = lo.x; dv[1] = lo.y; dv[2] = lo.z; dv[3] = lo.w; dv[4] = hi.x; dv[5] = hi.y; dv[6] = hi.z; dv[7] = hi.w;
     }
-#pragma unroll
+#pragma unroll UNROLL
     for (int j = 0; j < 8; ++j) {
         uint2 o2;
         o2.x = cvt_e4m3x4(scaled_clamped<DIV>(v[0][j], dv[j]), scaled_clamped<DIV>(v[1][j], dv[j]),
@@ -365,7 +367,7 @@ __device__ __forceinline__ bool dual_tile(float (&v)[8][8], float (*s_amax)[128]
     }
     __syncthreads();
     // 128 transposed rows x 8 chunks of 16 bytes (16 consecutive m)
-#pragma unroll
+#pragma unroll UNROLL
     for (int rep = 0; rep < 4; ++rep) {
         const int idx = threadIdx.x + rep * 256;
         const int nl = idx >> 3, ch = idx & 7;
@@ -387,28 +389,29 @@ __device__ __forceinline__ bool dual_tile(float (&v)[8][8], float (*s_amax)[128]
 // TRANS: the block-scaled bytes are written transposed, (N, M) with M contiguous and rounded up to 16 (zeros behind it): the
 // layout in which the weight-gradient GEMM reads them K-major.  They leave through the staging tile of dual_tile.
 // SEG: as in dual_tile (TRANS only).
-template <int DIV, bool ROUND, bool TRANS, bool SEG = false, typename AfterSync>
+template <int DIV, bool ROUND, bool TRANS, bool SEG = false, bool ROLLED = false, typename AfterSync>
 __device__ __forceinline__ bool row_block_tile(float (&v)[8][8], float* s_red, uint8_t* s_out, bool ok,
                                                uint8_t* __restrict__ q_row,
                                                float* __restrict__ s_row, uint8_t* __restrict__ q_blk,
                                                float* __restrict__ s_blk, int M, int N, int nb_n, int bm, int bn,
                                                AfterSync&& after_sync, int src0 = 0, int cnt = 128) {
+    constexpr int UNROLL = ROLLED ? 1 : 8;
     const int sub = threadIdx.x & 15, hw = threadIdx.x >> 4, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int n = bn * 128 + sub * 8;
     const int mt = SEG ? src0 + hw * 8 : bm * 128 + hw * 8;    // first row of this thread's row-wise outputs
     const int m_rows = SEG ? src0 + cnt : M;                    // one past the last of them
     float bmax = 0.0f;
     float m[8];
-#pragma unroll
+#pragma unroll UNROLL
     for (int i = 0; i < 8; ++i) {
         m[i] = 0.0f;
-#pragma unroll
+#pragma unroll UNROLL
         for (int j = 0; j < 8; ++j) m[i] = fmaxf(m[i], fabsf(v[i][j]));
     }
     const float mine = scale_from_amax<DIV, ROUND>(half_warp_rows_max(m, sub));
     const int own = mt + half_warp_row(sub);
     if ((sub & 1) == 0 && own < m_rows) s_row[(int64_t)own * nb_n + bn] = mine;
-#pragma unroll
+#pragma unroll UNROLL
     for (int i = 0; i < 8; ++i) {
         const float s = __shfl_sync(0xffffffffu, mine, half_warp_lane(i), 16);
         const float d = divisor_of<DIV>(s);
@@ -421,7 +424,7 @@ __device__ __forceinline__ bool row_block_tile(float (&v)[8][8], float* s_red, u
         if (inb) __stcs(reinterpret_cast<uint2*>(q_row + (int64_t)(mt + i) * N + n), o2);
         // what the backward would read back: e4m3 value times the row scale (zero outside the matrix)
         const uint32_t w[2] = {o2.x, o2.y};
-#pragma unroll
+#pragma unroll UNROLL
         for (int h = 0; h < 2; ++h) {
             const float2 lo = e4m3x2_to_float2((uint16_t)(w[h] & 0xffff));
             const float2 hi = e4m3x2_to_float2((uint16_t)(w[h] >> 16));
@@ -430,7 +433,7 @@ __device__ __forceinline__ bool row_block_tile(float (&v)[8][8], float* s_red, u
             v[i][4 * h + 2] = inb ? __fmul_rn(hi.x, s) : 0.0f;
             v[i][4 * h + 3] = inb ? __fmul_rn(hi.y, s) : 0.0f;
         }
-#pragma unroll
+#pragma unroll UNROLL
         for (int j = 0; j < 8; ++j) bmax = fmaxf(bmax, fabsf(v[i][j]));
     }
     bmax = warp_max(bmax);
@@ -438,13 +441,13 @@ __device__ __forceinline__ bool row_block_tile(float (&v)[8][8], float* s_red, u
     if (!__syncthreads_and(ok)) return false;
     after_sync();
     bmax = s_red[0];
-#pragma unroll
+#pragma unroll UNROLL
     for (int w8 = 1; w8 < 8; ++w8) bmax = fmaxf(bmax, s_red[w8]);
     const float sb = scale_from_amax<DIV, false>(bmax);
     const float db = divisor_of<DIV>(sb);
     if (threadIdx.x == 0) s_blk[(int64_t)bm * nb_n + bn] = sb;
     if constexpr (!TRANS) {
-#pragma unroll
+#pragma unroll UNROLL
         for (int i = 0; i < 8; ++i) {
             if (mt + i < M && n < N) {
                 uint2 o2;
@@ -458,7 +461,7 @@ __device__ __forceinline__ bool row_block_tile(float (&v)[8][8], float* s_red, u
         __syncthreads();                      // s_red is free for the next piece
     } else {
         // eight rows of one column per 8-byte store into the staging tile (elements outside the matrix are zeros)
-#pragma unroll
+#pragma unroll UNROLL
         for (int j = 0; j < 8; ++j) {
             uint2 o2;
             o2.x = cvt_e4m3x4(scaled_clamped<DIV>(v[0][j], db), scaled_clamped<DIV>(v[1][j], db),
@@ -470,7 +473,7 @@ __device__ __forceinline__ bool row_block_tile(float (&v)[8][8], float* s_red, u
         }
         __syncthreads();
         const int m0 = bm * 128, n0 = bn * 128, pitch = (M + 15) & ~15;
-#pragma unroll
+#pragma unroll UNROLL
         for (int rep = 0; rep < 4; ++rep) {
             const int idx = threadIdx.x + rep * 256;
             const int nl = idx >> 3, ch = idx & 7;
@@ -520,6 +523,17 @@ __device__ __forceinline__ bool not_finite(uint32_t w) {          // either half
 }
 
 struct Raw8x8 { uint32_t w[8][4]; };                       // rows hw * 8 + i, columns sub * 8 + 2 * k and + 1 of the piece
+
+// A piece with other elements takes the passes above in loops (ROLLED).  Unrolled, never taken, they doubled the kernels' code, and the GEMM behind
+// a dual quantiser took 16.5 us for 14.0: forward and backward, from a graph, 640 x 2048 -> 4096 72 us for 62, 2000 x 4096 -> 4096 155 for 152.  (The
+// unpacking stays unrolled: an index into `in` would put every piece into local memory, 32768 x 512 -> 1024 forward and backward 132 -> 141 us.)
+template <typename T>
+__device__ __forceinline__ void unpack_piece(const Raw8x8& in, float (&v)[8][8]) {
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+#pragma unroll
+        for (int k = 0; k < 4; ++k) { const float2 f = Pair<T>::both(in.w[i][k]); v[i][2 * k] = f.x; v[i][2 * k + 1] = f.y; }
+}
 
 // half_warp_rows_max of packed candidates: m[i] holds two of row i.  The result, of row half_warp_row(sub), in both halves.
 template <typename T>
@@ -590,11 +604,8 @@ __device__ __forceinline__ bool dual_tile16(const Raw8x8& in, float (*s_amax)[12
     if ((threadIdx.x & 31) < 16) *reinterpret_cast<uint4*>(&s_packed[warp][sub * 4]) = make_uint4(cmax[0], cmax[1], cmax[2], cmax[3]);
     if (!__syncthreads_and(ok && !odd)) {
         float v[8][8];
-#pragma unroll
-        for (int i = 0; i < 8; ++i)
-#pragma unroll
-            for (int k = 0; k < 4; ++k) { const float2 f = P::both(in.w[i][k]); v[i][2 * k] = f.x; v[i][2 * k + 1] = f.y; }
-        return dual_tile<DIV, ROUND, SEG>(v, s_amax, s_out, ok, q_row, s_row, q_col, s_col, M, N, nb_n, nb_m, bm, bn, after_sync, src0, cnt);
+        unpack_piece<T>(in, v);
+        return dual_tile<DIV, ROUND, SEG, true>(v, s_amax, s_out, ok, q_row, s_row, q_col, s_col, M, N, nb_n, nb_m, bm, bn, after_sync, src0, cnt);
     }
     after_sync();
     if ((threadIdx.x & 31) < 8) {
@@ -654,7 +665,7 @@ __device__ __forceinline__ bool dual_tile16(const Raw8x8& in, float (*s_amax)[12
     return true;
 }
 
-template <typename T, bool ROUND, bool TRANS, bool SEG = false, typename AfterSync>
+template <typename T, bool ROUND, bool TRANS, bool SEG = false, bool ROLLED = true, typename AfterSync>
 __device__ __forceinline__ bool row_block_tile16(const Raw8x8& in, float* s_red, uint8_t* s_out, bool ok, uint8_t* __restrict__ q_row,
                                                  float* __restrict__ s_row, uint8_t* __restrict__ q_blk, float* __restrict__ s_blk, int M,
                                                  int N, int nb_n, int bm, int bn, AfterSync&& after_sync, int src0 = 0, int cnt = 128) {
@@ -688,11 +699,8 @@ __device__ __forceinline__ bool row_block_tile16(const Raw8x8& in, float* s_red,
     if (!finite || !(bmax <= 3.4e38f)) {                   // (a power-of-two scale can take a decoded value past the largest float)
         __syncthreads();
         float v[8][8];
-#pragma unroll
-        for (int i = 0; i < 8; ++i)
-#pragma unroll
-            for (int k = 0; k < 4; ++k) { const float2 f = P::both(in.w[i][k]); v[i][2 * k] = f.x; v[i][2 * k + 1] = f.y; }
-        return row_block_tile<DIV, ROUND, TRANS, SEG>(v, s_red, s_out, ok, q_row, s_row, q_blk, s_blk, M, N, nb_n, bm, bn, after_sync, src0, cnt);
+        unpack_piece<T>(in, v);
+        return row_block_tile<DIV, ROUND, TRANS, SEG, ROLLED>(v, s_red, s_out, ok, q_row, s_row, q_blk, s_blk, M, N, nb_n, bm, bn, after_sync, src0, cnt);
     }
     after_sync();
     if ((sub & 1) == 0 && own < m_rows) s_row[(int64_t)own * nb_n + bn] = mine;
@@ -1034,7 +1042,8 @@ swiglu_row_block_kernel(const T* __restrict__ h12, uint8_t* __restrict__ q_row, 
                     raw.w[i][k] = pack2<T>(__fdividef(x.x, 1.0f + __expf(-x.x)) * y.x, __fdividef(x.y, 1.0f + __expf(-x.y)) * y.y);
             }
         }
-        row_block_tile16<T, ROUND, true, SEG>(raw, s_red, s_out, true, q_row, s_row, q_blk, s_blk, M, I, nb_n, bm, bn, [] {}, src0, cnt);
+        // (not ROLLED: 32768 x 1024 in segments 55 us, 57.5 with the loops)
+        row_block_tile16<T, ROUND, true, SEG, false>(raw, s_red, s_out, true, q_row, s_row, q_blk, s_blk, M, I, nb_n, bm, bn, [] {}, src0, cnt);
     }
 }
 
