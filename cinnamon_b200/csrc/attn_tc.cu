@@ -1356,7 +1356,20 @@ static bool dense_pays(const Plan& p, bool backward) {
     }
     const double ctas = backward ? 1.0 : (double)p.nv;      // a forward CTA computes 64 columns of the output
     const double all = ctas * tiles * tile / 148.0, longest = chain * (double)(p.Lp / T) * tile;
-    return first + ((all > longest ? all : longest) + ctas * q_tiles * query_tile / 148.0) / 1900.0 < gather_us;
+    double cycles = (all > longest ? all : longest) + ctas * q_tiles * query_tile / 148.0;
+    if (!backward) {
+        // With few queries a forward is one of them after the other: a query's picks on the gathers' side, and on the tiles' side, with CTAs for less
+        // than half the SMs, the longest chain and its query tile.  Fitted to 280 calls of one sequence, 1 ... 8 heads, L = 256 ... 640, K = 32 ... 256: the way
+        // taken costs 0.6 % more than the faster one, at worst 1.14 times (without this 5.8 %, 1.9 times); on 250 others of every size 0.65 %, 1.19 times
+        // (0.86 %, 1.43).  us, gathers and tiles: 2 x 313 queries, 256 picks of 192 / 128 in fp32 101 and 53, 4 x 313, 128 picks 52 and 40, in bf16 39
+        // and 29; 1 x 512, 128 picks of 192 / 64 39 and 46.
+        const double one_query = 6.0 + p.K * row * (wide ? 4 : 2) / 4100.0 + (wide ? 0.0 : 0.055 * p.K) + gathered / (wide ? 14.95e6 : 10.15e6);
+        if (one_query > gather_us) gather_us = one_query;
+        if (ctas * q_tiles < 74.0)
+            cycles = parts ? 0.664 * (double)(p.Lp / T) * tile + 1200.0 + 191.0 * p.K : 0.515 * (double)(p.Lp / T) * tile - 3980.0 + 117.0 * p.K;
+        if (cycles < 0.0) cycles = 0.0;
+    }
+    return first + cycles / 1900.0 < gather_us;
 }
 
 static bool supported(int64_t B, int64_t H, int64_t L, int64_t K, int64_t Dqk, int64_t Dv) {
